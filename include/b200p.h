@@ -182,9 +182,12 @@ size_t b200p_attn_workspace_bytes(int64_t B, int64_t L, int Hq, int D);
 int b200p_attn_decode_static(const void* q, const void* kcache, const void* vcache, const int32_t* lengths,
                              void* out, int64_t B, int Hq, int Hkv, int D, int64_t Tcap,
                              float scale, int dtype, int flags, void* stream);
-/* 0 = auto, 1 = generic CUDA-core kernel only, 2 = tensor (mma) kernels only: split-K decode for L == 1, causal flash
- * prefill for L > 1 (16-bit, head_dim 128) */
+/* 0 = auto, 1 = generic CUDA-core kernel only, 2 = tensor kernels only: split-K decode for L == 1, causal flash prefill for
+ * L > 1 (16-bit, head_dim 128: tcgen05, mma.sync for the smallest calls), 3 = tcgen05 for every such prefill */
 int b200p_attn_set_path(int path);
+/* 0, or 1 + the role (0 loader, 1 MMA issuer, 2 / 3 softmax) whose bounded barrier wait ran out in a tcgen05 prefill attention
+ * since the last call (which clears it).  Synchronises the device. */
+int b200p_attn_tc_fault(void);
 
 /* mx.argmax(logits, axis=-1, keepdims=True)                         [utils.py:350-352,363]
  * logits float [B, V] (ldl floats between rows) -> tokens int32 [B]; lowest index among ties.

@@ -5,6 +5,7 @@
 
 namespace b200p {
 
+int sm_count();
 // implemented in the kernel translation units
 int qmv_launch(const void* x, const uint32_t* w, const void* s, const void* b, void* y, int64_t M, int64_t N,
                int64_t K, int64_t ldx, int64_t ldy, int gs, int bits, int dtype, int epi, int flags, cudaStream_t st);
@@ -32,6 +33,9 @@ int attn_decode_launch(const void* q, const void* kc, const void* vc, const int3
                        int out_perm, void* ws, size_t ws_bytes, cudaStream_t st);
 size_t attn_decode_workspace_bytes(int64_t B, int64_t L, int Hq, int D);
 bool attn_prefill_supported(int64_t L, int Hq, int Hkv, int D, int dtype);
+bool attn_prefill_tc_supported(int64_t L, int Hq, int Hkv, int D, int dtype);
+int attn_prefill_tc_launch(const void* q, const void* kc, const void* vc, const int32_t* lengths, void* out, int64_t B, int64_t L,
+                           int Hq, int Hkv, int D, int64_t Tcap, float scale, int dtype, int out_perm, cudaStream_t st);
 int attn_prefill_launch(const void* q, const void* kc, const void* vc, const int32_t* lengths, void* out, int64_t B, int64_t L,
                         int Hq, int Hkv, int D, int64_t Tcap, float scale, int dtype, int out_perm, cudaStream_t st);
 
@@ -163,6 +167,14 @@ extern "C" int b200p_attn(const void* q, const void* kcache, const void* vcache,
   const bool tc_ok = attn_decode_supported(L, Hq, Hkv, D, dtype);
   const bool pf_ok = attn_prefill_supported(L, Hq, Hkv, D, dtype);
   if (g_attn_path == 2) B200P_REQUIRE(tc_ok || pf_ok, B200P_ERR_ARG, "tensor attention forced but unsupported for this call");
+  // Prompts run on tcgen05 except the smallest: a call of at most 64 new tokens over a cache of at most 256 positions that fills
+  // the SMs at most twice with mma.sync CTAs (64 queries of one head each) is shorter than the tcgen05 kernel's set-up (32 / 8
+  // heads, B=1, empty cache, L=2 / 16 / 64: 4.1 / 4.4 / 4.9 against 6.9 / 6.9 / 9.0 us).  Beyond it tcgen05 wins at every size: 1000
+  // cached positions 18.6 against 27.7 us (L=2, B=1), L=200 at B=8 19.6 against 33.5 us, L=777 at 8000 cached 125 against 568 us.
+  // (Its softmax takes the maximum before the scale, so negative scales stay on the mma.sync kernel.)
+  const bool pf_small = L <= 64 && Tcap <= 256 && B * Hq <= 2 * (int64_t)sm_count();
+  if (g_attn_path != 1 && scale >= 0.f && (g_attn_path == 3 || !pf_small) && attn_prefill_tc_supported(L, Hq, Hkv, D, dtype))
+    return attn_prefill_tc_launch(q, kcache, vcache, lengths, out, B, L, Hq, Hkv, D, Tcap, scale, dtype, out_perm, st);
   if (pf_ok && g_attn_path != 1)
     return attn_prefill_launch(q, kcache, vcache, lengths, out, B, L, Hq, Hkv, D, Tcap, scale, dtype, out_perm, st);
   if (tc_ok && g_attn_path != 1) {

@@ -314,6 +314,49 @@ def test_attention_tensor_prefill_causal(ops, dtype, B, L, Hq, Hkv, lengths):
     assert rel_err(got, gen) < {"float16": 2e-3, "bfloat16": 1.2e-2}[dtype]
 
 
+@pytest.mark.parametrize("dtype,B,L,Hq,Hkv,lengths", [
+    ("float16", 1, 2, 4, 1, [0]),                 # the smallest call: two queries, one key tile
+    ("float16", 2, 31, 8, 2, [97, 96]),           # keys end at / one short of a tile edge (128)
+    ("bfloat16", 2, 33, 8, 2, [96, 230]),         # one key past a tile edge; a second, nearly empty query tile
+    ("float16", 1, 129, 4, 4, [0]),               # one head per key head: 128 queries per tile, one in the second
+    ("bfloat16", 1, 26, 10, 2, [127]),            # five heads per key head: 125 of 128 rows of a tile
+    ("float16", 3, 70, 16, 1, [0, 300, 700]),     # sixteen heads per key head, more key tiles than ring slots
+    ("bfloat16", 1, 300, 6, 2, [40]),             # three heads per key head, several query tiles
+])
+@pytest.mark.parametrize("perm", [False, True])
+def test_attention_tcgen05_prefill(ops, dtype, B, L, Hq, Hkv, lengths, perm):
+    """attn_prefill_tc.cu against the oracle's SDPA at the edges of its tiles.  The cache holds NaN behind the last key, scores reach
+    far apart (rows dominated by one key).  Tolerances as for the mma.sync kernel: the same roundings (probabilities, output)."""
+    from mlx_parallm_b200 import _lib
+    D, dt, scale = 128, TD[dtype], 128 ** -0.5
+    rng = np.random.default_rng(L)
+    Tcap = max(lengths) + L + 3
+    q = (rng.standard_normal((B, L, Hq, D)) * 3).astype(np.float32)
+    k = rng.standard_normal((B, Hkv, Tcap, D)).astype(np.float32)
+    v = rng.standard_normal((B, Hkv, Tcap, D)).astype(np.float32)
+    qt, kt, vt = (torch.from_numpy(a).to(dt).cuda() for a in (q, k, v))
+    exp = np.zeros((B, L, Hq * D))
+    for b in range(B):
+        n = lengths[b] + L
+        kt[b, :, n:], vt[b, :, n:] = float("nan"), float("nan")
+        kb, vb = (t[b, :, :n].double().cpu().repeat_interleave(Hq // Hkv, 0) for t in (kt, vt))
+        s = torch.einsum("lhd,htd->hlt", qt[b].double().cpu(), kb) * scale
+        s.masked_fill_(torch.arange(n)[None, None] > (lengths[b] + torch.arange(L))[None, :, None], -float("inf"))
+        exp[b] = torch.einsum("hlt,htd->lhd", s.softmax(-1), vb).reshape(L, Hq * D).numpy()
+    out = torch.full((B, L, Hq * D), 7.0, dtype=dt, device="cuda")
+    ws = torch.empty((max(ops.attn_workspace_bytes(B, L, Hq, D), 16),), dtype=torch.uint8, device="cuda")
+    _lib.check(_lib.lib().b200p_attn_set_path(3))
+    try:
+        ops.attn(qt, kt, vt, torch.tensor(lengths, dtype=torch.int32, device="cuda"), out, B, L, Hq, Hkv, D, scale, workspace=ws, out_perm=perm)
+    finally:
+        _lib.lib().b200p_attn_set_path(0)
+    assert _lib.lib().b200p_attn_tc_fault() == 0
+    got = out.float().cpu().numpy()
+    if perm:                                              # undo [0,4,1,5,2,6,3,7] inside every group of 8
+        got = got.reshape(B, L, -1, 8)[..., [0, 2, 4, 6, 1, 3, 5, 7]].reshape(B, L, Hq * D)
+    assert rel_err(got, exp) < {"float16": 2e-3, "bfloat16": 1.2e-2}[dtype]
+
+
 # ---------------------------------------------------------------- samplers
 def test_argmax_ties_and_probs(ops):
     rng = np.random.default_rng(6)
