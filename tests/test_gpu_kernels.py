@@ -265,6 +265,42 @@ def test_rope_kv_append_counts_rows_beyond_capacity(ops, D):
     assert ops.kv_overflow_count() == 0                       # nothing dropped: the counter stays clear
 
 
+@pytest.mark.parametrize("dtype,B,L,Hq,Hkv,norm", [
+    ("float16", 1, 256, 4, 2, False),             # the smallest call of the row kernel: one token per CTA
+    ("bfloat16", 3, 211, 5, 1, True),             # 633 tokens: two per CTA, the last CTA half empty
+    ("float16", 2, 601, 3, 3, True),              # 1202 tokens: four per CTA
+    ("bfloat16", 1, 2371, 40, 8, True),           # eight per CTA, more heads than walkers
+])
+def test_rope_kv_append_prompt_rows(ops, dtype, B, L, Hq, Hkv, norm):
+    """Calls of 256 tokens and more (16-byte accesses, angles shared by the heads) against the per-head kernel fed the same tokens in
+    smaller portions.  Without norms bit for bit; with them the sum of squares runs in another order: one rounding of the result."""
+    D, dt = 128, TD[dtype]
+    g = torch.Generator(device="cuda").manual_seed(L)
+    qkv = torch.randn((B, L, (Hq + 2 * Hkv) * D), generator=g, device="cuda").to(dt)
+    wq, wk = ((1 + 0.1 * torch.randn(D, generator=g, device="cuda")).to(dt) if norm else None for _ in range(2))
+    lengths = torch.tensor([3 * b for b in range(B)], dtype=torch.int32, device="cuda")
+    cap = L + 3 * (B - 1) - 1                     # the last row's last token does not fit
+    res = []
+    for portion in (L, 200 // B):
+        q = torch.zeros((B, L, Hq, D), dtype=dt, device="cuda")
+        kc, vc = (torch.zeros((B, Hkv, cap, D), dtype=dt, device="cuda") for _ in range(2))
+        ops.kv_overflow_count(reset=True)
+        for l in range(0, L, portion):
+            n = min(portion, L - l)
+            qo = torch.zeros((B, n, Hq, D), dtype=dt, device="cuda")
+            ops.rope_kv_append(qkv[:, l:l + n].contiguous(), qo, kc, vc, lengths + l, B, n, Hq, Hkv, D, 10000.0, 1.0, wq, wk, 1e-6)
+            q[:, l:l + n] = qo
+        res.append((q, kc, vc, ops.kv_overflow_count(reset=True)))
+    (q, kc, vc, n), (q2, kc2, vc2, n2) = res
+    assert n == n2 == Hkv and torch.equal(vc, vc2)
+    for a, b in ((q, q2), (kc, kc2)):
+        if not norm:
+            assert torch.equal(a, b)
+        else:
+            ulp = 2.0 ** (-10 if dtype == "float16" else -7)
+            assert (a.float() - b.float()).abs().max() <= 2 * ulp * b.float().abs().max() and (a != b).float().mean() < 1e-2
+
+
 def attn_case(ops, B, L, Hq, Hkv, D, lengths, dtype, path, seed=5):
     from mlx_parallm_b200 import _lib
     rng = np.random.default_rng(seed)
