@@ -108,9 +108,12 @@ size_t b200p_qmm_workspace_bytes(int64_t M, int64_t N, int64_t K);
 int b200p_qmm_tensor_supported(int64_t M, int64_t N, int64_t K, int group_size, int bits, int dtype,
                                int epilogue);
 /* force a path for tests/benchmarks: 0 = auto, 1 = CUDA-core GEMV only, 2 = tcgen05 tile kernels only, 3 = mma.sync
- * GEMV only, 4 = mma.sync small-matrix GEMM only (csrc/qmm_mma.cu: ADD_RESIDUAL, M <= 64, N % 128 == 0, K % 256 == 0)
- * (2, 3 and 4: error if the call is unsupported on that path) */
+ * GEMV only, 4 = mma.sync small-matrix GEMM only (csrc/qmm_mma.cu: ADD_RESIDUAL, M <= 64, N % 128 == 0, K % 256 == 0),
+ * 6 = TMA-ring GEMV only (csrc/qmv_ring.cu: M <= 16, K % 512 == 0, N % 16 == 0)
+ * (2, 3, 4 and 6: error if the call is unsupported on that path) */
 int b200p_qmm_set_path(int path);
+/* 1 if a bounded wait of the TMA-ring GEMV ran out since the last call (which clears it), else 0.  Synchronises the device. */
+int b200p_qmv_fault(void);
 /* smallest M routed to the tensor path in auto mode (default 1: measured, scripts/qmm_sweep.py, profiles/r1_run11_qmm_sweep_gemv_vs_tensor.txt) */
 int b200p_qmm_set_min_tensor_m(int m);
 

@@ -22,6 +22,9 @@ bool qmv_mma_supported(int64_t M, int64_t N, int64_t K, int gs, int bits, int dt
 bool qmm_mma_supported(int64_t M, int64_t N, int64_t K, int gs, int bits, int dtype, int epi, const void* y, int64_t ldy);
 int qmm_mma_launch(const void* x, const uint32_t* w, const void* s, const void* b, void* y, int64_t M, int64_t N, int64_t K,
                    int64_t ldx, int64_t ldy, int dtype, int flags, cudaStream_t st);
+bool qmv_ring_supported(int64_t M, int64_t N, int64_t K, int gs, int bits, int dtype, int epi);
+int qmv_ring_launch(const void* x, const uint32_t* w, const void* s, const void* b, void* y, int64_t M, int64_t N, int64_t K, int64_t ldx,
+                    int64_t ldy, int bits, int dtype, int epi, int flags, cudaStream_t st);
 int qmv_mma_launch(const void* x, const uint32_t* w, const void* s, const void* b, void* y, int64_t M, int64_t N, int64_t K,
                    int64_t ldx, int64_t ldy, int dtype, int epi, int flags, cudaStream_t st);
 int attn_generic_launch(const void* q, const void* kc, const void* vc, const int32_t* lengths, void* out,
@@ -55,6 +58,16 @@ static int g_mma_max_m = [] { const char* e = getenv("B200P_MMA_MAX_M"); return 
 // grows (its activation loads are per 16-row warp, not shared through shared memory).  The CUDA-core GEMV loses everywhere.
 static int g_gemv_max_m = [] { const char* e = getenv("B200P_GEMV_MAX_M"); return e ? atoi(e) : 4; }();
 static long long g_gemv_max_weights = [] { const char* e = getenv("B200P_GEMV_MAX_WEIGHTS"); return e ? atoll(e) : (1ll << 25); }();
+// The TMA-ring GEMV (qmv_ring.cu), measured against the kernels it replaces (us per launch in a CUDA graph over weight copies larger than
+// L2): whole-tile epilogues gate|up 28672 x 4096 f16 16.2 against 21.7 at M = 1, 18.5 against 22.1 at M = 6 (bf16 19.0 / 25.9, 21.3 /
+// 26.1); 57344 x 8192 8-bit 82 against 92; accumulating o_proj 4096 x 4096 5.2 against 6.0 at M = 1, 5.8 against 6.9 at M = 4, down_proj
+// 4096 x 14336 11.2 against 13.2 at M = 1, 12.2 against 13.9 at M = 2 but 13.2 against 12.1 at M = 3; in 8 bits it loses there (62 against
+// 53 us, 8192 x 28672 bf16).  Matrices under 8 M weights stay on the kernels without rings.
+static bool qmv_ring_preferred(int64_t M, int64_t N, int64_t K, int bits, int epi) {
+  if (N * K < (1ll << 23)) return false;
+  if (epi != B200P_EPI_ADD_RESIDUAL) return M <= (bits == 4 ? 6 : 8);
+  return bits == 4 && M <= 4 && N * K <= (M <= 2 ? 2 : 1) * g_gemv_max_weights;
+}
 static int g_attn_path = 0;  // 0 auto, 1 generic, 2 tensor
 }  // namespace b200p
 
@@ -67,7 +80,7 @@ extern "C" int b200p_qmm_set_min_tensor_m(int m) {
 }
 
 extern "C" int b200p_qmm_set_path(int path) {
-  B200P_REQUIRE(path >= 0 && path <= 4, B200P_ERR_ARG, "path must be 0..4");
+  B200P_REQUIRE(path >= 0 && path <= 6 && path != 5, B200P_ERR_ARG, "path must be 0..4 or 6");
   g_qmm_path = path;
   return B200P_OK;
 }
@@ -113,6 +126,14 @@ extern "C" int b200p_qmm(const void* x, const uint32_t* w, const void* scales, c
   if (M == 0) return B200P_OK;
   PdlClass pdl_cls(64);
   cudaStream_t st = (cudaStream_t)stream;
+  const bool ring_ok = qmv_ring_supported(M, N, K, group_size, bits, dtype, epilogue) && aligned(scales, 16) && aligned(biases, 16) &&
+                       aligned(y, epilogue == B200P_EPI_STORE || epilogue == B200P_EPI_SILU_MUL ? 2 : 4);
+  if (g_qmm_path == 6) B200P_REQUIRE(ring_ok, B200P_ERR_ARG, "ring GEMV forced but unsupported for this call");
+  if (ring_ok && (g_qmm_path == 6 || (g_qmm_path == 0 && qmv_ring_preferred(M, N, K, bits, epilogue)))) {
+    const int rc = qmv_ring_launch(x, w, scales, biases, y, M, N, K, ldx, ldy, bits, dtype, epilogue, flags, st);
+    if (rc <= 0) return rc;                      // 1: x does not fit beside the rings
+    B200P_REQUIRE(g_qmm_path != 6, B200P_ERR_ARG, "ring GEMV forced but x does not fit");
+  }
   // (SILU_MUL through the GEMV: 16-bit output, PERM8 allowed; the other GEMV epilogues write fp32 in the natural order)
   const bool mma_ok = qmv_mma_supported(M, N, K, group_size, bits, dtype, epilogue) && aligned(w, 32) &&
                       (epilogue == B200P_EPI_SILU_MUL ? aligned(y, 2) : (aligned(y, 4) && !(flags & B200P_Y_PERM8)));

@@ -619,6 +619,29 @@ def test_qmm_small_scale_dequant_is_bit_identical(ops, M, N, K, bits, epi):
         assert rel_err(a, f) < 2e-5          # operands below 2^-10 round as subnormals at 1/16: absolute error <= 2^-21
 
 
+# ---------------------------------------------------------------- TMA-ring GEMV of b200p_qmm (M <= 16)
+@pytest.mark.parametrize("M,N,K,bits,dtype,epi,small", [
+    (1, 16, 512, 4, "float16", 1, True),          # one unit: seven of eight warps have nothing to do
+    (2, 48, 1024, 4, "bfloat16", 3, False),       # two units per tile: runs end inside a tile, idle warps in between
+    (3, 2400, 1536, 4, "float16", 0, False),      # three chunks per tile against eight warps, 16-bit store
+    (4, 4096, 4096, 4, "float16", 2, True),       # accumulate: tiles shared by two CTAs
+    (5, 96, 17408, 4, "bfloat16", 2, False),      # accumulate: several panels of k, few tiles
+    (8, 1024, 5120, 4, "float16", 3, True),       # 16-warp CTAs
+    (9, 256, 2048, 4, "bfloat16", 1, False),      # second n-tile, one token in it
+    (16, 512, 2048, 4, "float16", 2, False),
+    (1, 512, 2048, 8, "float16", 3, True),
+    (7, 80, 1024, 8, "bfloat16", 0, False),
+    (13, 64, 4096, 8, "float16", 2, False),
+])
+def test_qmm_ring_gemv(ops, M, N, K, bits, dtype, epi, small):
+    """csrc/qmv_ring.cu against the oracle at the edges of its schedule.  Tolerances as for the other 16-bit paths: A is q*s+b rounded to
+    the storage type, sums are fp32, 16-bit epilogues round once more."""
+    from mlx_parallm_b200 import _lib
+    got, exp = qmm_case(ops, M, N, K, bits, dtype, epi, seed=M + N, path=6, ragged_ld=(M in (3, 9)), small_scale=small)
+    assert _lib.lib().b200p_qmv_fault() == 0
+    assert rel_err(got, exp) < {"float16": 3e-3, "bfloat16": 2e-2}[dtype]
+
+
 # ---------------------------------------------------------------- mma.sync register GEMV of b200p_qmm (M <= 16)
 MMA_CASES = [  # M, N, K, dtype, epilogue (1 = fp32 store, 2 = += into fp32, split-K with red.add)
     (1, 256, 256, "float16", 1), (3, 512, 1024, "float16", 2), (8, 96, 512, "bfloat16", 1), (9, 1024, 4096, "float16", 2),
