@@ -114,6 +114,8 @@ int b200p_qmm_tensor_supported(int64_t M, int64_t N, int64_t K, int group_size, 
 int b200p_qmm_set_path(int path);
 /* 1 if a bounded wait of the TMA-ring GEMV ran out since the last call (which clears it), else 0.  Synchronises the device. */
 int b200p_qmv_fault(void);
+/* the same for the wide tiles of more than 128 tokens (csrc/qmm_wide.cu): 0, or 1 + the role that gave up */
+int b200p_qmm_wide_fault(void);
 /* smallest M routed to the tensor path in auto mode (default 1: measured, scripts/qmm_sweep.py, profiles/r1_run11_qmm_sweep_gemv_vs_tensor.txt) */
 int b200p_qmm_set_min_tensor_m(int m);
 

@@ -69,6 +69,7 @@ SIGNATURES = {
     "b200p_gemm_tc_fault": (_i32, []),
     "b200p_attn_tc_fault": (_i32, []),
     "b200p_qmv_fault": (_i32, []),
+    "b200p_qmm_wide_fault": (_i32, []),
     "b200p_ragged_plan": (_i32, [_vp, _vp, _vp, _vp, _vp, _vp, _i32, _i64, _vp]),
     "b200p_ragged_advance": (_i32, [_vp, _vp, _vp, _vp, _vp, _i32, _vp]),
     "b200p_embed_hashed": (_i32, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _f32, _i64, _i64, _i64, _i32, _vp]),

@@ -22,6 +22,9 @@ bool qmv_mma_supported(int64_t M, int64_t N, int64_t K, int gs, int bits, int dt
 bool qmm_mma_supported(int64_t M, int64_t N, int64_t K, int gs, int bits, int dtype, int epi, const void* y, int64_t ldy);
 int qmm_mma_launch(const void* x, const uint32_t* w, const void* s, const void* b, void* y, int64_t M, int64_t N, int64_t K,
                    int64_t ldx, int64_t ldy, int dtype, int flags, cudaStream_t st);
+bool qmm_wide_supported(int64_t M, int64_t N, int64_t K, int bits, int epi, const void* s, const void* b, const void* y, int64_t ldy);
+int qmm_wide_launch(const void* x, const uint32_t* w, const void* s, const void* b, void* y, int64_t M, int64_t N, int64_t K, int64_t ldx,
+                    int64_t ldy, int bits, int dtype, int epi, int flags, cudaStream_t st);
 bool qmv_ring_supported(int64_t M, int64_t N, int64_t K, int gs, int bits, int dtype, int epi);
 int qmv_ring_launch(const void* x, const uint32_t* w, const void* s, const void* b, void* y, int64_t M, int64_t N, int64_t K, int64_t ldx,
                     int64_t ldy, int bits, int dtype, int epi, int flags, cudaStream_t st);
@@ -155,6 +158,9 @@ extern "C" int b200p_qmm(const void* x, const uint32_t* w, const void* scales, c
   if (g_qmm_path == 2) {
     B200P_REQUIRE(tc_ok, B200P_ERR_ARG, "tensor path forced but unsupported for this call");
   }
+  // more than 128 tokens: one 128-row weight block against up to 256 tokens (the rule and its figures: qmm_wide.cu)
+  if (tc_ok && g_qmm_path != 1 && qmm_wide_supported(M, N, K, bits, epilogue, scales, biases, y, ldy))
+    return qmm_wide_launch(x, w, scales, biases, y, M, N, K, ldx, ldy, bits, dtype, epilogue, flags, st);
   // fp32 accumulate epilogue: the stream-K kernel (partial tiles summed by TMA reduce-adds, no workspace, no tail);
   // B200P_QMM_SK=0 keeps everything on the whole-tile kernel (A/B measurements)
   if (tc_ok && g_qmm_path != 1 && g_use_sk && qmm_sk_supported(M, N, K, bits, epilogue, y, ldy))

@@ -619,6 +619,26 @@ def test_qmm_small_scale_dequant_is_bit_identical(ops, M, N, K, bits, epi):
         assert rel_err(a, f) < 2e-5          # operands below 2^-10 round as subnormals at 1/16: absolute error <= 2^-21
 
 
+# ---------------------------------------------------------------- wide tiles of b200p_qmm (M > 128)
+@pytest.mark.parametrize("M,N,K,bits,dtype,epi,small", [
+    (129, 128, 512, 4, "float16", 1, True),       # one tile, the shortest K: two stages
+    (201, 1000, 1024, 4, "bfloat16", 0, False),   # rows past N in the last block, tokens past M in the tile
+    (256, 208, 1536, 4, "float16", 3, False),     # gated: a block whose last gate rows do not exist, a full token tile
+    (257, 2000, 512, 4, "bfloat16", 3, False),    # two token tiles, one row of the second in use by one token less than half
+    (300, 264, 4096, 4, "float16", 2, True),      # accumulate: K ranges of one tile on several CTAs
+    (1100, 5120, 512, 4, "float16", 2, False),    # accumulate: a whole round of tiles, the rest cut along K
+    (140, 512, 2048, 8, "float16", 1, True),      # 8 bits: two k-blocks per stage
+    (333, 384, 1024, 8, "bfloat16", 3, False),
+    (205, 260 * 4, 512, 8, "bfloat16", 2, False),
+])
+def test_qmm_wide_tiles(ops, M, N, K, bits, dtype, epi, small):
+    """csrc/qmm_wide.cu against the oracle.  Tolerances as for the other 16-bit paths (A rounded to the storage type, fp32 sums)."""
+    from mlx_parallm_b200 import _lib
+    got, exp = qmm_case(ops, M, N, K, bits, dtype, epi, seed=M + N, path=2, ragged_ld=(M in (201, 300)), small_scale=small)
+    assert _lib.lib().b200p_qmm_wide_fault() == 0
+    assert rel_err(got, exp) < {"float16": 3e-3, "bfloat16": 2e-2}[dtype]
+
+
 # ---------------------------------------------------------------- TMA-ring GEMV of b200p_qmm (M <= 16)
 @pytest.mark.parametrize("M,N,K,bits,dtype,epi,small", [
     (1, 16, 512, 4, "float16", 1, True),          # one unit: seven of eight warps have nothing to do
