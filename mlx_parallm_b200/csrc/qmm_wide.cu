@@ -22,7 +22,7 @@
 // ranges of (tile, K stage) and adds its sums with cp.reduce.async.bulk.tensor (as qmm_sk.cu does).  Every mbarrier wait is bounded (g_qmm_wide_fault).
 //
 // Measured (bf16 or f16, us, before / after): gate|up 28672 x 4096 4-bit 62 / 51 at 201 tokens, 64 / 57 at 256, 235 / 208 at 1000, 500 / 390 at
-// 2048, 1261 / 780 at 4096 (1.2 PFLOP/s); 57344 x 8192 8-bit 356 / 221 at 201, 1280 / 820 at 1000; down 4096 x 14336 405 / 359 at 4096.
+// 2048, 1261 / 780 at 4096 (1.2 PFLOP/s); 57344 x 8192 8-bit (bf16, with the fp32 dequantisation of dequant.cuh) 356 / 214 at 201, 1201 / 790 at 1000; down 4096 x 14336 405 / 359 at 4096.
 //
 // warp roles (768 threads): 0..15 dequantisers (group g = 4 warps takes k-blocks g, g + 4, ...; thread = weight row), 16..19 epilogue,
 // 20 TMA producer of weights, scales and biases, 21 TMA producer of X, 22 / 23 MMA issuers.
@@ -539,8 +539,8 @@ bool qmm_wide_supported(int64_t M, int64_t N, int64_t K, int bits, int epi, cons
     if (N % 4 != 0 || !aligned(y, 16) || (ldy * 4) % 16 != 0) return false;
     // 4-bit sums of up to 1024 tokens: the stream-K kernel's 128-token tiles are as fast where they hold the tokens as tightly (4096 x
     // 14336, us, wide / stream-K: 26.3 / 27.4 at 201 tokens, 29.0 / 27.9 at 256, 43.1 / 44.0 at 400, 90.0 / 89.7 at 1000; 4096 x 4096: 14.1 /
-    // 15.3, 16.2 / 15.6, 18.8 / 19.8, 30.8 / 29.5); above, 177 / 190 at 2048 and 359 / 405 at 4096.  8-bit codes: 98 / 127 at 201
-    // tokens, 107 / 128 at 256, 412 / 546 at 1000 (8192 x 28672, bf16).
+    // 15.3, 16.2 / 15.6, 18.8 / 19.8, 30.8 / 29.5); above, 177 / 190 at 2048 and 359 / 405 at 4096.  8-bit codes: 94 / 127 at 201
+    // tokens, 105 / 128 at 256, 400 / 510 at 1000 (8192 x 28672, bf16).
     const int64_t tm = (M + MAX_TOKENS - 1) / MAX_TOKENS, padded = tm * (((M + tm - 1) / tm + 15) / 16 * 16);
     return bits == 8 || M > 1024 || (M + 127) / 128 * 128 * 100 >= 108 * padded;
   }
