@@ -69,7 +69,7 @@ class QuantizedLinear:
 
     def __call__(self, x, epilogue=EPI_STORE, out=None, workspace=None, x_perm=False, y_perm=False):
         lead = x.shape[:-1]
-        y = ops.qmm(x.reshape(-1, x.shape[-1]), self.weight, self.scales, self.biases, self.group_size,
+        y = ops.qmm(x if len(lead) == 1 else x.reshape(-1, x.shape[-1]), self.weight, self.scales, self.biases, self.group_size,
                     self.bits, epilogue, out, workspace, x_perm=x_perm, y_perm=y_perm, small_scale=self.small_scale)
         return y if out is not None else y.reshape(*lead, -1)
 
