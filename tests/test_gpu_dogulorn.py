@@ -623,3 +623,35 @@ def test_delta_scan_key_and_value_sizes(dk, dv, H, KH):
     assert (o.double().cpu().view(M, H, dv) - want_o).abs().max() < 1e-4
     assert (dev[5].double().cpu()[[0, 2]] - want_s[[0, 2]]).abs().max() < 1e-4
     assert torch.equal(dev[5].cpu()[1], state0[1])               # a row that no entry names is not touched
+
+
+@pytest.mark.parametrize("lens,H,KH,dv,channel", [([257], 1, 1, 128, False), ([1, 300, 2], 3, 1, 256, True), ([130, 3, 129, 9], 4, 2, 128, True)])
+def test_delta_prep_rows_equals_the_per_token_kernel(lens, H, KH, dv, channel):
+    """Prompts of more than 256 tokens with 128-channel heads (one warp per 128 channels and 8 tokens) against the per-token kernel fed
+    the same portions in two halves: bit for bit, entries that begin inside a warp's tokens and carried inputs among them."""
+    from mlx_parallm_b200 import ops
+    dk, taps, M, nb = 128, 4, sum(lens), len(lens)
+    C, f32, i32 = 2 * KH * dk + H * dv, torch.float32, torch.int32
+    g = torch.Generator(device="cuda").manual_seed(M)
+    rnd = lambda *s: torch.randn(s, generator=g, device="cuda")        # noqa: E731
+    n_dec = H * (dk if channel else 1)
+    proj, a, conv_w, state = rnd(M, C + H + 3), rnd(M, n_dec), rnd(C, taps), rnd(nb, taps - 1, C)
+    A_log, dt_bias = rnd(H), rnd(n_dec)
+    cu = torch.tensor([0] + np.cumsum(lens).tolist(), dtype=i32, device="cuda")
+    rows = torch.arange(nb, dtype=i32, device="cuda").flip(0).contiguous()
+    lengths = torch.tensor([0, 2, 1, 7][:nb], dtype=i32, device="cuda")  # nothing carried, fewer than taps - 1 inputs, all of them
+    t = [torch.zeros(M, dtype=i32, device="cuda") for _ in range(3)]
+    ops.ragged_plan(cu, rows, lengths, *t, nb, M)
+
+    def run(parts):
+        out = [torch.zeros((M, n), dtype=f32, device="cuda") for n in (KH * dk, KH * dk, H * dv, H, n_dec)]
+        for lo, hi in parts:
+            # the per-token kernel reads earlier inputs of a portion from the rows before its own: give it the whole tensors' slices
+            ops.delta_prep(proj[lo:hi], C, a[lo:hi], conv_w, state, A_log, dt_bias, *(x[lo:hi].contiguous() for x in t), *(o[lo:hi] for o in out),
+                           H, KH, dk, dv, taps)
+        return out
+
+    whole = run([(0, M)])
+    cuts = list(range(0, M, 200)) + [M]
+    for w, p in zip(whole, run(list(zip(cuts[:-1], cuts[1:])))):
+        assert torch.equal(w, p)
