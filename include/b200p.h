@@ -60,8 +60,8 @@ enum {
 #define B200P_OUT_PERM8 0x1     /* flags of b200p_rmsnorm / b200p_attn: write the 16-bit output PERM8 */
 /* Caller's promise about the weights of a b200p_qmm call, OR-ed into `epilogue` like the layout flags: every scale of the
  * matrix satisfies |s| < 0.0625 (checked once at load time by the host: mlx_parallm_b200/models/_transformer.py).  F16
- * calls then dequantise with ONE half2 FMA per code pair on subnormal operands (csrc/dequant.cuh) -- same rounding of
- * q*s+b, two thirds of the instructions.  Ignored for BF16 / F32. */
+ * and BF16 calls then dequantise with ONE packed FMA per code pair on subnormal operands (csrc/dequant.cuh) -- same rounding of
+ * q*s+b, half to two thirds of the instructions.  (BF16 needs no more than |s| < 256.)  Ignored for F32. */
 #define B200P_W_SMALLSCALE 0x400
 
 const char* b200p_version(void);

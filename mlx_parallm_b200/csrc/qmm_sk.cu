@@ -75,7 +75,7 @@ struct TcParams {
 };
 
 
-// FAST: the small-scale dequant of dequant.cuh (f16, caller promised B200P_W_SMALLSCALE): A and D are produced at 1/16.
+// FAST: the small-scale dequant of dequant.cuh (caller promised B200P_W_SMALLSCALE): A and D are produced at 1 / SmallScaleOut<T>.
 template <typename T, int BITS, bool XPERM, bool FAST>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 qmm_sk_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x,
@@ -261,9 +261,9 @@ qmm_sk_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
       uint32_t o[32];
       const uint32_t* pw = reinterpret_cast<const uint32_t*>(pk + j2 * CPK);
       if constexpr (FAST) {
-        const SmallScale sc = small_scale_prep(s2, b2);
+        const SmallScale sc = small_scale_prep<T>(s2, b2);
 #pragma unroll
-        for (int c = 0; c < 8; ++c) dequant8_small<BITS, XPERM>(pw + c * (BITS / 4), sc, o + 4 * c);
+        for (int c = 0; c < 8; ++c) dequant8_small<T, BITS, XPERM>(pw + c * (BITS / 4), sc, o + 4 * c);
       } else {
 #pragma unroll
         for (int c = 0; c < 8; ++c) dequant8<T, BITS, XPERM>(pw + c * (BITS / 4), s2, b2, o + 4 * c);
@@ -345,7 +345,7 @@ qmm_sk_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
     const int r = e * 32 + lane;                     // output row (weight row) within the 128-row block
     const uint32_t lane_base = tmem_base + ((uint32_t)(e * 32) << 16);
     const int et = threadIdx.x - DQ_THREADS;         // 0..127
-    constexpr float DSCALE = FAST ? 16.f : 1.f;      // FAST: A (hence D) was produced at 1/16
+    constexpr float DSCALE = FAST ? SmallScaleOut<T>::value : 1.f;      // A (hence D) was produced at a power of two below
     pdl_wait();                                      // y belongs to the previous kernels until here
     int seg = 0;
     uint32_t nchunk = 0;
@@ -473,7 +473,7 @@ int qmm_sk_launch(const void* x, const uint32_t* w, const void* s, const void* b
   B200P_REQUIRE((flags & B200P_Y_PERM8) == 0, B200P_ERR_ARG, "B200P_Y_PERM8 applies to 16-bit outputs only");
   const int num_kb = (int)(K / 64);
   const bool sb_tma = (num_kb % 8) == 0 && aligned(s, 16) && aligned(b, 16);
-  const bool fast = (flags & B200P_W_SMALLSCALE) != 0 && dtype == B200P_F16;
+  const bool fast = (flags & B200P_W_SMALLSCALE) != 0;
   const CUtensorMapDataType dt16 = dtype == B200P_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
   CUtensorMap tms[5];
   int rc = tc_encode_2d(enc, &tms[0], CU_TENSOR_MAP_DATA_TYPE_UINT8, w, (uint64_t)(K * bits / 8), (uint64_t)N,
@@ -509,7 +509,8 @@ int qmm_sk_launch(const void* x, const uint32_t* w, const void* s, const void* b
     if (fast) return x_perm ? launch_sk<__half, 4, true, true>(tms, p, pl, st) : launch_sk<__half, 4, false, true>(tms, p, pl, st);
     return x_perm ? launch_sk<__half, 4, true, false>(tms, p, pl, st) : launch_sk<__half, 4, false, false>(tms, p, pl, st);
   }
-  if (bits == 8) return launch_sk<__nv_bfloat16, 8, false, false>(tms, p, pl, st);
+  if (bits == 8) return fast ? launch_sk<__nv_bfloat16, 8, false, true>(tms, p, pl, st) : launch_sk<__nv_bfloat16, 8, false, false>(tms, p, pl, st);
+  if (fast) return x_perm ? launch_sk<__nv_bfloat16, 4, true, true>(tms, p, pl, st) : launch_sk<__nv_bfloat16, 4, false, true>(tms, p, pl, st);
   return x_perm ? launch_sk<__nv_bfloat16, 4, true, false>(tms, p, pl, st) : launch_sk<__nv_bfloat16, 4, false, false>(tms, p, pl, st);
 }
 

@@ -235,7 +235,7 @@ __device__ __forceinline__ void tc_emit(const TcParams& p, bool silu, int r, con
 template <typename T, bool FAST>
 __device__ __forceinline__ void tc_drain_tile(const TcParams& p, bool silu, int r, uint32_t dA, uint32_t dB, int TN, int rowA0,
                                               int rowB0, int tok0, int worker, int nworkers) {
-  constexpr float DSCALE = FAST ? 16.f : 1.f;        // FAST: A (hence D) was produced at 1/16
+  constexpr float DSCALE = FAST ? SmallScaleOut<T>::value : 1.f;        // A (hence D) was produced at a power of two below
   for (int t0 = worker * EPI_TOK; t0 < TN; t0 += nworkers * EPI_TOK) {
     if (tok0 + t0 >= p.M_tok) break;                 // padding tokens of the last token tile
     float a[EPI_TOK], b[EPI_TOK];
@@ -250,12 +250,11 @@ __device__ __forceinline__ void tc_drain_tile(const TcParams& p, bool silu, int 
   }
 }
 
-// FAST: the small-scale dequant of dequant.cuh (f16, caller promised B200P_W_SMALLSCALE): A and D are produced at 1/16.
+// FAST: the small-scale dequant of dequant.cuh (caller promised B200P_W_SMALLSCALE): A and D are produced at 1 / SmallScaleOut<T>.
 template <typename T, int BITS, bool XPERM, bool FAST>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 qmm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x,
               const __grid_constant__ CUtensorMap tm_s, const __grid_constant__ CUtensorMap tm_b, const TcParams p) {
-  static_assert(!FAST || std::is_same<T, __half>::value, "the subnormal-operand dequant is an f16 trick");
   constexpr int PKB = 64 * BITS / 8;            // packed bytes per row per k-block
   constexpr int KPS = 128 / PKB;                // k-blocks per stage (a stage row is one 128-byte line)
   constexpr int SPG = 8 / KPS;                  // stages per scale/bias group of 8 k-blocks
@@ -468,9 +467,9 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
       TSEC_BEGIN();
       const uint32_t* pw = reinterpret_cast<const uint32_t*>(pk + j2 * CPK);
       if constexpr (FAST) {
-        const SmallScale sc = small_scale_prep(s2, b2);
+        const SmallScale sc = small_scale_prep<T>(s2, b2);
 #pragma unroll
-        for (int c = 0; c < 8; ++c) dequant8_small<BITS, XPERM>(pw + c * (BITS / 4), sc, o + 4 * c);
+        for (int c = 0; c < 8; ++c) dequant8_small<T, BITS, XPERM>(pw + c * (BITS / 4), sc, o + 4 * c);
       } else {
 #pragma unroll
         for (int c = 0; c < 8; ++c) dequant8<T, BITS, XPERM>(pw + c * (BITS / 4), s2, b2, o + 4 * c);
@@ -598,7 +597,7 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
     const int r = e * 32 + lane;                     // output row (weight row) within the 128-row block
     const uint32_t lane_base = tmem_base + ((uint32_t)(e * 32) << 16);
     const int et = threadIdx.x - DQ_THREADS;         // 0..127
-    constexpr float DSCALE = FAST ? 16.f : 1.f;      // FAST: A (hence D) was produced at 1/16
+    constexpr float DSCALE = FAST ? SmallScaleOut<T>::value : 1.f;      // A (hence D) was produced at a power of two below
     const int64_t slot_elems = (int64_t)2 * TN * 128;   // one partial tile: [2 blocks][TN tokens][128 rows] fp32
 
     pdl_wait();                                      // y and the workspace belong to the previous kernels until here
@@ -911,7 +910,7 @@ int qmm_tc_launch(const void* x, const uint32_t* w, const void* s, const void* b
   const int num_kb = (int)(K / 64);
   const bool sb_tma = (num_kb % 8) == 0 && aligned(s, 16) && aligned(b, 16);
   const CUtensorMapDataType dt16 = dtype == B200P_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
-  const bool fast = (flags & B200P_W_SMALLSCALE) != 0 && dtype == B200P_F16;
+  const bool fast = (flags & B200P_W_SMALLSCALE) != 0;
   CUtensorMap tms[4];
   int rc = tc_encode_2d(enc, &tms[0], CU_TENSOR_MAP_DATA_TYPE_UINT8, w, (uint64_t)(K * bits / 8), (uint64_t)N,
                      (uint64_t)(K * bits / 8), 128u, (uint32_t)pl.R, CU_TENSOR_MAP_SWIZZLE_128B, "weights");
@@ -953,7 +952,8 @@ int qmm_tc_launch(const void* x, const uint32_t* w, const void* s, const void* b
     if (fast) return x_perm ? launch_tc<__half, 4, true, true>(tms, p, pl, st) : launch_tc<__half, 4, false, true>(tms, p, pl, st);
     return x_perm ? launch_tc<__half, 4, true, false>(tms, p, pl, st) : launch_tc<__half, 4, false, false>(tms, p, pl, st);
   } else {
-    if (bits == 8) return launch_tc<__nv_bfloat16, 8, false, false>(tms, p, pl, st);
+    if (bits == 8) return fast ? launch_tc<__nv_bfloat16, 8, false, true>(tms, p, pl, st) : launch_tc<__nv_bfloat16, 8, false, false>(tms, p, pl, st);
+    if (fast) return x_perm ? launch_tc<__nv_bfloat16, 4, true, true>(tms, p, pl, st) : launch_tc<__nv_bfloat16, 4, false, true>(tms, p, pl, st);
     return x_perm ? launch_tc<__nv_bfloat16, 4, true, false>(tms, p, pl, st) : launch_tc<__nv_bfloat16, 4, false, false>(tms, p, pl, st);
   }
 }

@@ -193,7 +193,7 @@ __device__ __forceinline__ bool all_of(int id, int threads, bool v) {
 template <typename T, bool FAST, bool ADD>
 __device__ __forceinline__ bool drain(const Params& p, const CUtensorMap* tm_y, Shared* sh, uint32_t tmem, int tile, uint32_t parity, int worker,
                                       int q, int lane, uint32_t stage) {
-  constexpr float DSCALE = FAST ? 16.f : 1.f;
+  constexpr float DSCALE = FAST ? SmallScaleOut<T>::value : 1.f;
   constexpr int TOK = ADD ? ADD_TOK : 16;
   int rb, tm;
   tile_of(p, tile, rb, tm);
@@ -237,7 +237,7 @@ __device__ __forceinline__ bool drain(const Params& p, const CUtensorMap* tm_y, 
   return true;
 }
 
-// FAST: the small-scale dequant of dequant.cuh (f16, caller promised B200P_W_SMALLSCALE): A and D are produced at 1/16.
+// FAST: the small-scale dequant of dequant.cuh (caller promised B200P_W_SMALLSCALE): A and D are produced at 1 / SmallScaleOut<T>.
 template <typename T, int BITS, bool XPERM, bool FAST, bool ADD>
 __global__ void __launch_bounds__(THREADS, 1)
 qmm_wide_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x,
@@ -423,9 +423,9 @@ qmm_wide_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
           uint32_t o[32];
           const uint32_t* pw = reinterpret_cast<const uint32_t*>(pk);
           if constexpr (FAST) {
-            const SmallScale sc = small_scale_prep(s2, b2);
+            const SmallScale sc = small_scale_prep<T>(s2, b2);
 #pragma unroll
-            for (int c = 0; c < 8; ++c) dequant8_small<BITS, XPERM>(pw + c * (BITS / 4), sc, o + 4 * c);
+            for (int c = 0; c < 8; ++c) dequant8_small<T, BITS, XPERM>(pw + c * (BITS / 4), sc, o + 4 * c);
           } else {
 #pragma unroll
             for (int c = 0; c < 8; ++c) dequant8<T, BITS, XPERM>(pw + c * (BITS / 4), s2, b2, o + 4 * c);
@@ -553,7 +553,7 @@ int qmm_wide_launch(const void* x, const uint32_t* w, const void* s, const void*
   TcEncodeFn enc = tc_get_encode();
   B200P_REQUIRE(enc != nullptr, B200P_ERR_CUDA, "cuTensorMapEncodeTiled entry point not available");
   const bool x_perm = (flags & B200P_X_PERM8) != 0, add = epi == B200P_EPI_ADD_RESIDUAL;
-  const bool fast = (flags & B200P_W_SMALLSCALE) != 0 && dtype == B200P_F16;
+  const bool fast = (flags & B200P_W_SMALLSCALE) != 0;
   const Plan pl = make_plan(M, N, K, bits, epi);
   B200P_REQUIRE(pl.w_stages >= 2, B200P_ERR_ARG, "shared memory too small for the tensor path");
   const CUtensorMapDataType dt16 = dtype == B200P_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
@@ -580,7 +580,8 @@ int qmm_wide_launch(const void* x, const uint32_t* w, const void* s, const void*
     if (fast) return x_perm ? GO(__half, 4, true, true) : GO(__half, 4, false, true);
     return x_perm ? GO(__half, 4, true, false) : GO(__half, 4, false, false);
   }
-  if (bits == 8) return GO(__nv_bfloat16, 8, false, false);
+  if (bits == 8) return fast ? GO(__nv_bfloat16, 8, false, true) : GO(__nv_bfloat16, 8, false, false);
+  if (fast) return x_perm ? GO(__nv_bfloat16, 4, true, true) : GO(__nv_bfloat16, 4, false, true);
   return x_perm ? GO(__nv_bfloat16, 4, true, false) : GO(__nv_bfloat16, 4, false, false);
 #undef GO
 }

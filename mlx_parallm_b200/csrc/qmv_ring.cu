@@ -159,8 +159,8 @@ __device__ __forceinline__ void qr_emit(const QrParams& p, int tile, int g, int 
   }
 }
 
-// NW warps; FAST: the small-scale dequant of dequant.cuh (f16, caller promised B200P_W_SMALLSCALE): A and the sums are produced at
-// 1/16; NT: n-tiles of 8 tokens.
+// NW warps; FAST: the small-scale dequant of dequant.cuh (caller promised B200P_W_SMALLSCALE): A and the sums are produced at
+// 1 / SmallScaleOut<T>; NT: n-tiles of 8 tokens.
 template <typename T, int BITS, bool FAST, int NT, int NW>
 __global__ void __launch_bounds__(NW * 32, 16 / NW)
 qmv_ring_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_s,
@@ -297,13 +297,13 @@ qmv_ring_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
         const uint32_t* pa = reinterpret_cast<const uint32_t*>(qa[c2]);
         const uint32_t* pb = reinterpret_cast<const uint32_t*>(qb[c2]);
         SmallScale ca, cb;
-        if constexpr (FAST) { ca = small_scale_prep(s2a, b2a); cb = small_scale_prep(s2b, b2b); }
+        if constexpr (FAST) { ca = small_scale_prep<T>(s2a, b2a); cb = small_scale_prep<T>(s2b, b2b); }
 #pragma unroll
         for (int i = 0; i < PIECES; ++i) {
           uint32_t da[4], db[4];
           if constexpr (FAST) {
-            dequant8_small<BITS, true>(pa + i * (BITS / 4), ca, da);
-            dequant8_small<BITS, true>(pb + i * (BITS / 4), cb, db);
+            dequant8_small<T, BITS, true>(pa + i * (BITS / 4), ca, da);
+            dequant8_small<T, BITS, true>(pb + i * (BITS / 4), cb, db);
           } else {
             dequant8<T, BITS, true>(pa + i * (BITS / 4), s2a, b2a, da);
             dequant8<T, BITS, true>(pb + i * (BITS / 4), s2b, b2b, db);
@@ -323,7 +323,7 @@ qmv_ring_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
     // ---- end of the tile, of the panel or of this warp's run: the sums leave the accumulators
     const bool tile_ends = at.ch + 1 == at.ch1;
     if (tile_ends || u + 1 == u1) {
-      constexpr float D = FAST ? 16.f : 1.f;
+      constexpr float D = FAST ? SmallScaleOut<T>::value : 1.f;
 #pragma unroll
       for (int n = 0; n < NT; ++n)
 #pragma unroll
@@ -454,14 +454,15 @@ int qmv_ring_launch(const void* x, const uint32_t* w, const void* s, const void*
                      CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     B200P_REQUIRE(r == CUDA_SUCCESS, B200P_ERR_CUDA, "cuTensorMapEncodeTiled(scales) failed: %d", (int)r);
   }
-  const bool fast = (flags & B200P_W_SMALLSCALE) != 0 && dtype == B200P_F16;
+  const bool fast = (flags & B200P_W_SMALLSCALE) != 0;
 #define GO2(T_, B_, F_, N_) (pl.nw == 8 ? qr_run<T_, B_, F_, N_, 8>(tm, p, pl, st) : qr_run<T_, B_, F_, N_, 16>(tm, p, pl, st))
 #define GO(T_, B_, F_) (M <= 8 ? GO2(T_, B_, F_, 1) : GO2(T_, B_, F_, 2))
   if (dtype == B200P_F16) {
     if (bits == 4) return fast ? GO(__half, 4, true) : GO(__half, 4, false);
     return fast ? GO(__half, 8, true) : GO(__half, 8, false);
   }
-  return bits == 4 ? GO(__nv_bfloat16, 4, false) : GO(__nv_bfloat16, 8, false);
+  if (bits == 4) return fast ? GO(__nv_bfloat16, 4, true) : GO(__nv_bfloat16, 4, false);
+  return fast ? GO(__nv_bfloat16, 8, true) : GO(__nv_bfloat16, 8, false);
 #undef GO
 #undef GO2
 }

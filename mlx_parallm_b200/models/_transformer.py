@@ -44,8 +44,8 @@ ACC32_MAX_ROWS = 128
 # 14.9 + 4.2 vs 23.5 us, TP=4 10.8 + 3.5 vs 17.3, TP=8 7.4 + 3.1 vs 13.7).
 GATE_UP_ACC32_MAX_WEIGHTS = 100 * 1000 * 1000
 USE_PERM8 = True                  # 4-bit 16-bit models: GEMM inputs in the PERM8 column order (include/b200p.h)
-# |scale| bound under which an f16 matrix may take the subnormal-operand dequant (B200P_W_SMALLSCALE, csrc/dequant.cuh):
-# the kernel needs s * 2^20 finite in half precision, i.e. |s| < 0.0625; checked once per matrix at load time.
+# |scale| bound under which an f16 or bf16 matrix may take the subnormal-operand dequant (B200P_W_SMALLSCALE, csrc/dequant.cuh):
+# the kernel needs s * 2^20 finite in half precision, i.e. |s| < 0.0625 (bf16: s * 2^120); checked once per matrix at load time.
 SMALL_SCALE_BOUND = 0.06
 
 
@@ -63,7 +63,7 @@ class QuantizedLinear:
         self.out_features = weight.shape[0]
         self.in_features = weight.shape[1] * 32 // self.bits
         if small_scale is None:      # one reduction + host read per matrix, at load time only
-            small_scale = (scales.dtype == torch.float16 and scales.is_cuda and scales.numel() > 0
+            small_scale = (scales.dtype in (torch.float16, torch.bfloat16) and scales.is_cuda and scales.numel() > 0
                            and float(scales.abs().max()) < SMALL_SCALE_BOUND)
         self.small_scale = bool(small_scale)
 

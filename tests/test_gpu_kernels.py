@@ -619,6 +619,22 @@ def test_qmm_small_scale_dequant_is_bit_identical(ops, M, N, K, bits, epi):
         assert rel_err(a, f) < 2e-5          # operands below 2^-10 round as subnormals at 1/16: absolute error <= 2^-21
 
 
+@pytest.mark.parametrize("M,N,K,bits,epi,path", [(1, 1024, 1024, 4, 3, 6), (2, 512, 2048, 8, 2, 6), (5, 1000, 192, 4, 1, 2), (64, 2048, 1024, 4, 3, 2),
+                                                 (64, 4096, 1024, 4, 2, 2), (24, 512, 2048, 8, 1, 2), (60, 512, 320, 8, 2, 0), (200, 512, 512, 4, 0, 0),
+                                                 (300, 264, 1536, 4, 2, 0), (201, 1000, 1024, 8, 3, 0)])
+def test_qmm_small_scale_dequant_of_bf16(ops, M, N, K, bits, epi, path):
+    """bf16: codes as integers times 2^-133, scales times 2^120, operands at 2^-13: every step but the one rounding of q*s+b is exact, so
+    4-bit products equal the direct form's where the order of the sums is fixed (whole tiles, or one CTA per K range); 8-bit operands,
+    which go through fp32 and a rounded constant otherwise, are no farther from the 64-bit result."""
+    a, exp = qmm_case(ops, M, N, K, bits, "bfloat16", epi, seed=M, path=path, small_scale=False)
+    f, _ = qmm_case(ops, M, N, K, bits, "bfloat16", epi, seed=M, path=path, small_scale=True)
+    if bits == 4 and epi != 2:
+        assert np.array_equal(a, f)
+    elif bits == 4:
+        assert rel_err(f, a) < 1e-6                              # fp32 sums in another order
+    assert rel_err(f, exp) < rel_err(a, exp) * 1.05 + 1e-6
+
+
 # ---------------------------------------------------------------- wide tiles of b200p_qmm (M > 128)
 @pytest.mark.parametrize("M,N,K,bits,dtype,epi,small", [
     (129, 128, 512, 4, "float16", 1, True),       # one tile, the shortest K: two stages
