@@ -131,8 +131,14 @@ extern "C" int b200p_qmm(const void* x, const uint32_t* w, const void* scales, c
   cudaStream_t st = (cudaStream_t)stream;
   const bool ring_ok = qmv_ring_supported(M, N, K, group_size, bits, dtype, epilogue) && aligned(scales, 16) && aligned(biases, 16) &&
                        aligned(y, epilogue == B200P_EPI_STORE || epilogue == B200P_EPI_SILU_MUL ? 2 : 4);
+  // The ring and the wide kernel need neither a workspace nor y rows of whole words; a call that the kernels they stand in for would
+  // refuse goes on to those, and is refused there.
+  const bool f32out = epilogue == B200P_EPI_STORE_F32 || epilogue == B200P_EPI_ADD_RESIDUAL;
+  const bool tile_args = workspace && workspace_bytes >= qmm_tc_workspace_bytes(M, N, K) && aligned(workspace, 16) && aligned(y, 4) &&
+                         (f32out || ldy % 2 == 0);
+  const bool sk_args = g_use_sk && qmm_sk_supported(M, N, K, bits, epilogue, y, ldy);
   if (g_qmm_path == 6) B200P_REQUIRE(ring_ok, B200P_ERR_ARG, "ring GEMV forced but unsupported for this call");
-  if (ring_ok && (g_qmm_path == 6 || (g_qmm_path == 0 && qmv_ring_preferred(M, N, K, bits, epilogue)))) {
+  if (ring_ok && (g_qmm_path == 6 || (g_qmm_path == 0 && (tile_args || sk_args) && qmv_ring_preferred(M, N, K, bits, epilogue)))) {
     const int rc = qmv_ring_launch(x, w, scales, biases, y, M, N, K, ldx, ldy, bits, dtype, epilogue, flags, st);
     if (rc <= 0) return rc;                      // 1: x does not fit beside the rings
     B200P_REQUIRE(g_qmm_path != 6, B200P_ERR_ARG, "ring GEMV forced but x does not fit");
@@ -159,11 +165,11 @@ extern "C" int b200p_qmm(const void* x, const uint32_t* w, const void* scales, c
     B200P_REQUIRE(tc_ok, B200P_ERR_ARG, "tensor path forced but unsupported for this call");
   }
   // more than 128 tokens: one 128-row weight block against up to 256 tokens (the rule and its figures: qmm_wide.cu)
-  if (tc_ok && g_qmm_path != 1 && qmm_wide_supported(M, N, K, bits, epilogue, scales, biases, y, ldy))
+  if (tc_ok && g_qmm_path != 1 && (tile_args || sk_args) && qmm_wide_supported(M, N, K, bits, epilogue, scales, biases, y, ldy))
     return qmm_wide_launch(x, w, scales, biases, y, M, N, K, ldx, ldy, bits, dtype, epilogue, flags, st);
   // fp32 accumulate epilogue: the stream-K kernel (partial tiles summed by TMA reduce-adds, no workspace, no tail);
   // B200P_QMM_SK=0 keeps everything on the whole-tile kernel (A/B measurements)
-  if (tc_ok && g_qmm_path != 1 && g_use_sk && qmm_sk_supported(M, N, K, bits, epilogue, y, ldy))
+  if (tc_ok && g_qmm_path != 1 && sk_args)
     return qmm_sk_launch(x, w, scales, biases, y, M, N, K, ldx, ldy, bits, dtype, flags, st);
   if (tc_ok && g_qmm_path != 1) {
     B200P_REQUIRE(workspace && workspace_bytes >= qmm_tc_workspace_bytes(M, N, K), B200P_ERR_ARG,
@@ -200,7 +206,9 @@ extern "C" int b200p_attn(const void* q, const void* kcache, const void* vcache,
   // cached positions 18.6 against 27.7 us (L=2, B=1), L=200 at B=8 19.6 against 33.5 us, L=777 at 8000 cached 125 against 568 us.
   // (Its softmax takes the maximum before the scale, so negative scales stay on the mma.sync kernel.)
   const bool pf_small = L <= 64 && Tcap <= 256 && B * Hq <= 2 * (int64_t)sm_count();
-  if (g_attn_path != 1 && scale >= 0.f && (g_attn_path == 3 || !pf_small) && attn_prefill_tc_supported(L, Hq, Hkv, D, dtype))
+  // (What does not fit its 32-bit row numbers stays there too, to be run or refused as it is.)
+  const bool pf_fits = L < (1ll << 30) && Tcap < (1ll << 31) - 128 && B < 65536 && Hq < 65536;
+  if (g_attn_path != 1 && scale >= 0.f && pf_fits && (g_attn_path == 3 || !pf_small) && attn_prefill_tc_supported(L, Hq, Hkv, D, dtype))
     return attn_prefill_tc_launch(q, kcache, vcache, lengths, out, B, L, Hq, Hkv, D, Tcap, scale, dtype, out_perm, st);
   if (pf_ok && g_attn_path != 1)
     return attn_prefill_launch(q, kcache, vcache, lengths, out, B, L, Hq, Hkv, D, Tcap, scale, dtype, out_perm, st);

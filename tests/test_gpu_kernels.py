@@ -635,6 +635,24 @@ def test_qmm_small_scale_dequant_of_bf16(ops, M, N, K, bits, epi, path):
     assert rel_err(f, exp) < rel_err(a, exp) * 1.05 + 1e-6
 
 
+@pytest.mark.parametrize("M,N,K,bits,epi", [(2, 8192, 1024, 4, 3), (201, 512, 512, 4, 0), (300, 512, 1024, 8, 1)])
+def test_qmm_arguments_of_the_tile_kernel_stay_required(ops, M, N, K, bits, epi):
+    """The ring and wide kernels use no workspace, but a call without one, or with 16-bit rows of odd length, is refused as on any size."""
+    from mlx_parallm_b200 import _lib
+    wq, s = torch.zeros((N, K * bits // 32), dtype=torch.int32, device="cuda"), torch.zeros((N, K // 64), dtype=torch.float16, device="cuda")
+    x, ws = torch.zeros((M, K), dtype=torch.float16, device="cuda"), torch.zeros(ops.qmm_workspace_bytes(M, N, K), dtype=torch.uint8, device="cuda")
+    n = N // 2 if epi == 3 else N
+    out = torch.empty((M, n + 1), dtype=torch.float32 if epi == 1 else torch.float16, device="cuda")
+
+    def call(ld, work, nbytes):
+        return _lib.lib().b200p_qmm(x.data_ptr(), wq.data_ptr(), s.data_ptr(), s.data_ptr(), out.data_ptr(), M, N, K, K, ld, 64, bits, _lib.F16, epi,
+                                    work, nbytes, torch.cuda.current_stream().cuda_stream)
+    assert call(n, ws.data_ptr(), ws.numel()) == 0
+    assert call(n, None, 0) < 0 and call(n, ws.data_ptr(), ws.numel() - 1) < 0
+    assert (call(n + 1, ws.data_ptr(), ws.numel()) == 0) == (epi == 1)
+    torch.cuda.synchronize()
+
+
 # ---------------------------------------------------------------- wide tiles of b200p_qmm (M > 128)
 @pytest.mark.parametrize("M,N,K,bits,dtype,epi,small", [
     (129, 128, 512, 4, "float16", 1, True),       # one tile, the shortest K: two stages
