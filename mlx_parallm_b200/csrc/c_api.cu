@@ -62,9 +62,9 @@ static int g_mma_max_m = [] { const char* e = getenv("B200P_MMA_MAX_M"); return 
 static int g_gemv_max_m = [] { const char* e = getenv("B200P_GEMV_MAX_M"); return e ? atoi(e) : 4; }();
 static long long g_gemv_max_weights = [] { const char* e = getenv("B200P_GEMV_MAX_WEIGHTS"); return e ? atoll(e) : (1ll << 25); }();
 // The TMA-ring GEMV (qmv_ring.cu), measured against the kernels it replaces (us per launch in a CUDA graph over weight copies larger than
-// L2): whole-tile epilogues gate|up 28672 x 4096 f16 16.2 against 21.7 at M = 1, 18.5 against 22.1 at M = 6 (bf16 19.0 / 25.9, 21.3 /
+// L2): whole-tile epilogues gate|up 28672 x 4096 f16 16.2 against 21.7 at M = 1, 18.5 against 22.1 at M = 6 (bf16, direct dequantisation on both sides, 19.0 / 25.9, 21.3 /
 // 26.1); 57344 x 8192 8-bit 82 against 92; accumulating o_proj 4096 x 4096 5.2 against 6.0 at M = 1, 5.8 against 6.9 at M = 4, down_proj
-// 4096 x 14336 11.2 against 13.2 at M = 1, 12.2 against 13.9 at M = 2 but 13.2 against 12.1 at M = 3; in 8 bits it loses there (62 against
+// 4096 x 14336 11.2 against 13.2 at M = 1, 12.2 against 13.9 at M = 2 but 13.2 against 12.1 at M = 3; in 8 bits it loses there (direct dequantisation: 62 against
 // 53 us, 8192 x 28672 bf16).  Matrices under 8 M weights stay on the kernels without rings.
 static bool qmv_ring_preferred(int64_t M, int64_t N, int64_t K, int bits, int epi) {
   if (N * K < (1ll << 23)) return false;

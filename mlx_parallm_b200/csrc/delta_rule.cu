@@ -13,6 +13,8 @@
 
 namespace b200p {
 
+int sm_count();
+
 __device__ __forceinline__ float silu_f(float z) { return z / (1.f + __expf(-z)); }
 __device__ __forceinline__ float softplus_f(float z) { return z > 20.f ? z : log1pf(expf(z)); }
 
@@ -249,8 +251,8 @@ __device__ __forceinline__ float2 ds_reduce2(float x0, float y0, float x1, float
 
 // MODE 0: delta rule, one decay per head and token; 1: delta rule, one decay per head, key channel and token (decay
 // [M, H, dk]); 2: no correction, S <- g S + k v^T (one decay per head and token; beta unused).
-template <int DKP, int MODE>
-__global__ void __launch_bounds__(ds_threads(DKP))
+template <int DKP, int MODE, int PER_SM = 1>
+__global__ void __launch_bounds__(ds_threads(DKP), PER_SM)
 delta_scan_kernel(const float* __restrict__ qn, const float* __restrict__ kn, const float* __restrict__ v,
                   const float* __restrict__ beta, const float* __restrict__ decay, float* __restrict__ state,
                   const int32_t* __restrict__ cu, const int32_t* __restrict__ rows, const int32_t* __restrict__ lengths,
@@ -514,7 +516,15 @@ static void delta_scan_launch(dim3 grid, cudaStream_t st, const float* qn, const
                               float* o, int H, int KH, int dk, int dv) {
   if (dk <= 32) delta_scan_kernel<32, MODE><<<grid, ds_threads(32), 0, st>>>(qn, kn, v, beta, decay, state, cu, rows, lengths, o, H, KH, dk, dv);
   else if (dk <= 64) delta_scan_kernel<64, MODE><<<grid, ds_threads(64), 0, st>>>(qn, kn, v, beta, decay, state, cu, rows, lengths, o, H, KH, dk, dv);
-  else if (dk <= 128) delta_scan_kernel<128, MODE><<<grid, ds_threads(128), 0, st>>>(qn, kn, v, beta, decay, state, cu, rows, lengths, o, H, KH, dk, dv);
+  else if (dk <= 128) {
+    // One CTA per SM may have 170 registers a thread and the shortest chain.  More CTAs than SMs are better run in pairs of 128
+    // registers (a few words spilled): a whole layer pass at 16 sequences of 16 tokens 139 -> 134 us with 16 heads and 193 -> 185 with
+    // 32, of 250 tokens 636 -> 583 and 1185 -> 1054.  The instances share their source and so the order of every sum.
+    if ((int64_t)grid.x * grid.y * grid.z > sm_count())
+      delta_scan_kernel<128, MODE, 2><<<grid, ds_threads(128), 0, st>>>(qn, kn, v, beta, decay, state, cu, rows, lengths, o, H, KH, dk, dv);
+    else
+      delta_scan_kernel<128, MODE><<<grid, ds_threads(128), 0, st>>>(qn, kn, v, beta, decay, state, cu, rows, lengths, o, H, KH, dk, dv);
+  }
   else if (dk <= 256) delta_scan_kernel<256, MODE><<<grid, ds_threads(256), 0, st>>>(qn, kn, v, beta, decay, state, cu, rows, lengths, o, H, KH, dk, dv);
   else delta_scan_kernel<512, MODE><<<grid, ds_threads(512), 0, st>>>(qn, kn, v, beta, decay, state, cu, rows, lengths, o, H, KH, dk, dv);
 }

@@ -625,6 +625,28 @@ def test_delta_scan_key_and_value_sizes(dk, dv, H, KH):
     assert torch.equal(dev[5].cpu()[1], state0[1])               # a row that no entry names is not touched
 
 
+@pytest.mark.parametrize("mode,dk", [(0, 128), (1, 128), (1, 100), (2, 128)])
+def test_delta_scan_of_more_ctas_than_sms_equals_its_parts(mode, dk):
+    """12 entries x 16 heads of 128 value columns are 384 CTAs, run two per SM; the same entries four at a time are 128, run one per SM:
+    one summation order, bit for bit, partial chunks and decode entries among them."""
+    from mlx_parallm_b200 import ops
+    H, KH, dv, lens = 16, 8, 128, [1, 9, 17, 8, 2, 30, 1, 16, 3, 24, 7, 11]
+    g, nb, M = torch.Generator(device="cuda").manual_seed(mode), len(lens), sum(lens)
+    rnd = lambda *sh: torch.randn(*sh, generator=g, device="cuda")
+    qn, kn, v = rnd(M, KH * dk) / dk, torch.nn.functional.normalize(rnd(M, KH, dk), dim=-1).reshape(M, -1), rnd(M, H * dv)
+    beta, decay = torch.rand(M, H, generator=g, device="cuda"), 0.5 + 0.5 * torch.rand(M, H * (dk if mode == 1 else 1), generator=g, device="cuda")
+    states = [(rnd(nb, H, dk, dv) * 0.3)]
+    states.append(states[0].clone())
+    i32, off = dict(dtype=torch.int32, device="cuda"), [0]
+    for n in lens:
+        off.append(off[-1] + n)
+    rows, lengths, o = torch.arange(nb, **i32), torch.tensor([3] * nb, **i32), [torch.zeros(M, H * dv, device="cuda") for _ in range(2)]
+    ops.delta_scan(qn, kn, v, beta, decay, states[0], torch.tensor(off, **i32), rows, lengths, o[0], nb, H, KH, dk, dv, mode)
+    for e in range(0, nb, 4):
+        ops.delta_scan(qn, kn, v, beta, decay, states[1], torch.tensor(off[e:e + 5], **i32), rows[e:e + 4].contiguous(), lengths, o[1], 4, H, KH, dk, dv, mode)
+    assert torch.equal(o[0], o[1]) and torch.equal(states[0], states[1])
+
+
 @pytest.mark.parametrize("lens,H,KH,dv,channel", [([257], 1, 1, 128, False), ([1, 300, 2], 3, 1, 256, True), ([130, 3, 129, 9], 4, 2, 128, True)])
 def test_delta_prep_rows_equals_the_per_token_kernel(lens, H, KH, dv, channel):
     """Prompts of more than 256 tokens with 128-channel heads (one warp per 128 channels and 8 tokens) against the per-token kernel fed
