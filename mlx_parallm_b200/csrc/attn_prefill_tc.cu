@@ -58,34 +58,9 @@ struct AttnTcShared {
 };
 
 __device__ __forceinline__ bool ft_wait(uint32_t bar, uint32_t parity, AttnTcShared* sh, int role) {
-  const long long t0 = clock64();
-  for (;;) {
-    uint32_t ok;
-    asm volatile(
-        "{\n"
-        ".reg .pred p;\n"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-        "selp.b32 %0, 1, 0, p;\n"
-        "}\n"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    if (ok) return true;
-    if (sh->abort) return false;
-    if (clock64() - t0 > 2000000000ll) {
-      sh->abort = 1;
-      atomicCAS(&g_attn_tc_fault, 0, 1 + role);
-      return false;
-    }
-  }
+  return mbar_wait_warp(bar, parity, &sh->abort, &g_attn_tc_fault, role);
 }
 
-__device__ __forceinline__ void ft_tma_3d(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2, uint32_t bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(dst),
-      "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(bar)
-      : "memory");
-}
 __device__ __forceinline__ void ft_tma_5d(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2, int c3, int c4, uint32_t bar) {
   asm volatile(
       "cp.async.bulk.tensor.5d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5, %6}], [%7];" ::"r"(dst),
@@ -193,25 +168,14 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_con
       int slot = 0;
       uint32_t ph = 0;
       const int z = b * p.Hkv + kvh;
-      int issued = 0;
-      for (; issued < 2 * n_tiles; ++issued) {             // K0 V0 K1 V1 ...
-        if (!ft_wait(smem_u32(&sh->kv_empty[slot]), ph ^ 1u, sh, 0)) break;
+      for (int issued = 0; issued < 2 * n_tiles; ++issued) {                         // K0 V0 K1 V1 ...
+        if (!mbar_wait_lane(smem_u32(&sh->kv_empty[slot]), ph ^ 1u, &sh->abort, &g_attn_tc_fault, 0)) break;
         const uint32_t bar = smem_u32(&sh->kv_full[slot]), dst = ring + slot * FT_TILE_BYTES;
         mbar_arrive_expect_tx(bar, FT_TILE_BYTES);
         const CUtensorMap* m = (issued & 1) ? &tmv : &tmk;
-        ft_tma_3d(dst, m, 0, (issued >> 1) * FT_KEYS, z, bar);
-        ft_tma_3d(dst + FT_HALF, m, 64, (issued >> 1) * FT_KEYS, z, bar);
+        tma_load_3d(dst, m, 0, (issued >> 1) * FT_KEYS, z, bar);
+        tma_load_3d(dst + FT_HALF, m, 64, (issued >> 1) * FT_KEYS, z, bar);
         if (++slot == FT_RING) { slot = 0; ph ^= 1u; }
-      }
-      if (issued < 2 * n_tiles) {                          // gave up: the copies in flight land before the CTA goes
-        for (int k = max(0, issued - FT_RING); k < issued; ++k) {
-          const uint32_t bar = smem_u32(&sh->kv_full[k % FT_RING]);
-          const long long t0 = clock64();
-          uint32_t ok = 0;
-          while (!ok && clock64() - t0 < 100000000ll)
-            asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.b32 %0, 1, 0, p;\n}\n"
-                         : "=r"(ok) : "r"(bar), "r"((uint32_t)((k / FT_RING) & 1)) : "memory");
-        }
       }
     }
    } else if (warp == 8) {
@@ -397,6 +361,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_con
       }
     }
   }
+  if (sh->abort) wait_settle();
   tc_fence_before();
   __syncthreads();
   if (warp == 8) {

@@ -54,13 +54,6 @@ struct GemmTcParams {
 };
 constexpr int GT_MAX_GROUPS = 1024;
 
-__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2, uint32_t bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(dst),
-      "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(bar)
-      : "memory");
-}
-
 // D[tmem] (+)= A[smem desc] * B[smem desc]^T, 16-bit inputs, fp32 accumulation
 __device__ __forceinline__ void umma_f16_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accum) {
   asm volatile(
@@ -233,30 +226,6 @@ __device__ __forceinline__ GemmTcTile gemm_tc_tile(const GemmTcParams& p, const 
   return r;
 }
 
-// bounded wait: gives up after about a second, or as soon as another role of the CTA has given up
-__device__ __forceinline__ bool gemm_tc_wait(uint32_t bar, uint32_t parity, GemmTcShared* sh, int role) {
-  const long long t0 = clock64();
-  for (;;) {
-    uint32_t ok;
-    asm volatile(
-        "{\n"
-        ".reg .pred p;\n"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-        "selp.b32 %0, 1, 0, p;\n"
-        "}\n"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    if (ok) return true;
-    if (sh->abort) return false;
-    if (clock64() - t0 > 2000000000ll) {
-      sh->abort = 1;
-      atomicCAS(&g_gemm_tc_fault, 0, 1 + role);
-      return false;
-    }
-  }
-}
-
 template <typename T, int BN, int STAGES>
 __global__ void __launch_bounds__(GT_THREADS, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constant__ CUtensorMap tmw, const GemmTcParams p) {
@@ -322,7 +291,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constant__ 
         const GemmTcTile tl = gemm_tc_tile(p, sh, t);
         const int z = tl.z, nt = tl.nt, mt = tl.mt, first = tl.first;
         for (int kb = kb0; kb < kb1; ++kb) {
-          if (!(ok = gemm_tc_wait(smem_u32(&sh->empty[stage]), phase ^ 1u, sh, 0))) break;
+          if (!(ok = mbar_wait_lane(smem_u32(&sh->empty[stage]), phase ^ 1u, &sh->abort, &g_gemm_tc_fault, 0))) break;
           const uint32_t bar = smem_u32(&sh->full[stage]);
           const uint32_t dst = base + stage * STAGE_BYTES;
           mbar_arrive_expect_tx(bar, STAGE_BYTES);
@@ -345,12 +314,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constant__ 
       uint32_t phase = 0, acc_phase = 0;
       bool ok = true;
       for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
-        if (!(ok = gemm_tc_wait(smem_u32(&sh->acc_empty[acc]), acc_phase ^ 1u, sh, 1))) break;
+        if (!(ok = mbar_wait_lane(smem_u32(&sh->acc_empty[acc]), acc_phase ^ 1u, &sh->abort, &g_gemm_tc_fault, 1))) break;
         tc_fence_after();
         const uint32_t d = tmem_base + (uint32_t)(acc * BN);
         const int kb0 = (t % p.splits) * p.kb_per_split, kb1 = min(p.num_kb, kb0 + p.kb_per_split);
         for (int kb = kb0; kb < kb1; ++kb) {
-          if (!(ok = gemm_tc_wait(smem_u32(&sh->full[stage]), phase, sh, 1))) break;
+          if (!(ok = mbar_wait_lane(smem_u32(&sh->full[stage]), phase, &sh->abort, &g_gemm_tc_fault, 1))) break;
           tc_fence_after();
           const uint64_t ad = make_desc_sw128(base + stage * STAGE_BYTES);
           const uint64_t bd = make_desc_sw128(base + stage * STAGE_BYTES + GT_A_BYTES);
@@ -372,7 +341,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constant__ 
     for (int t = blockIdx.x; t < num_tiles; t += gridDim.x) {
       const GemmTcTile tl = gemm_tc_tile(p, sh, t);
       const int z = tl.z, nt = tl.nt, mt = tl.mt, first = tl.first, len = tl.len;
-      if (!gemm_tc_wait(smem_u32(&sh->acc_full[acc]), acc_phase, sh, 2)) break;
+      if (!mbar_wait_warp(smem_u32(&sh->acc_full[acc]), acc_phase, &sh->abort, &g_gemm_tc_fault, 2)) break;
       tc_fence_after();
       const int64_t row = (int64_t)mt * GT_BM + lg * 32 + lane;               // within the batch index's (group's) rows
       const int64_t row_off = p.seg ? (first + row) * p.ldy : (int64_t)z * p.sy + row * p.ldy;
@@ -394,6 +363,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constant__ 
       if (++acc == 2) { acc = 0; acc_phase ^= 1u; }
     }
   }
+  if (sh->abort) wait_settle();
   tc_fence_before();
   __syncthreads();
   if (warp == 1) {

@@ -116,27 +116,7 @@ __device__ __forceinline__ void tile_of(const Params& p, int tile, int& rb, int&
 }
 
 __device__ __forceinline__ bool wait(uint64_t* bar, uint32_t parity, Shared* sh, int role) {
-  const uint32_t a = smem_u32(bar);
-  const long long t0 = clock64();
-  for (;;) {
-    uint32_t ok;
-    asm volatile(
-        "{\n"
-        ".reg .pred p;\n"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-        "selp.b32 %0, 1, 0, p;\n"
-        "}\n"
-        : "=r"(ok)
-        : "r"(a), "r"(parity)
-        : "memory");
-    if (ok) return true;
-    if (sh->abort) return false;
-    if (clock64() - t0 > 2000000000ll) {
-      sh->abort = 1;
-      atomicCAS(&g_qmm_wide_fault, 0, 1 + role);
-      return false;
-    }
-  }
+  return mbar_wait_warp(smem_u32(bar), parity, &sh->abort, &g_qmm_wide_fault, role);
 }
 
 // 16 tokens of one thread's output column
@@ -459,10 +439,7 @@ qmm_wide_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
       ok = drain<T, FAST, ADD>(p, &tm_y, sh, tmem, tile, seg & 1u, 0, q, lane, epi_ring);
     if (ADD && lane == 0) bulk_wait_all();
   }
-  if (sh->abort) {                                           // gave up: copies in flight land before the CTA goes
-    const long long t0 = clock64();
-    while (clock64() - t0 < 100000000ll) {}
-  }
+  if (sh->abort) wait_settle();
   tc_fence_before();
   __syncthreads();
   if (warp == WARP_MMA) {

@@ -83,32 +83,6 @@ __device__ __forceinline__ void qr_next(const QrParams& p, QrPos& r) {
   r.ch = r.ch0;
 }
 
-__device__ __forceinline__ void qr_tma_3d(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2, uint32_t bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(dst),
-      "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(bar)
-      : "memory");
-}
-__device__ __forceinline__ bool qr_wait(uint32_t bar, uint32_t parity) {
-  const long long t0 = clock64();
-  for (;;) {
-    uint32_t ok;
-    asm volatile(
-        "{\n"
-        ".reg .pred p;\n"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-        "selp.b32 %0, 1, 0, p;\n"
-        "}\n"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    if (ok) return true;
-    if (clock64() - t0 > 2000000000ll) {
-      g_qmv_ring_fault = 1;
-      return false;
-    }
-  }
-}
 __device__ __forceinline__ uint32_t lds_u16(uint32_t addr) {
   uint16_t v;
   asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(addr));
@@ -211,8 +185,8 @@ qmv_ring_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
       const uint32_t bar = my_bar + 8 * stage, dst = my_ring + stage * CODE_BYTES, sdst = my_scales + stage * SCALE_BYTES;
       const int ra = silu ? pr.tile * 8 : pr.tile * 16, rb = silu ? p.N / 2 + ra : ra + 8;
       mbar_arrive_expect_tx(bar, CODE_BYTES + SCALE_BYTES);
-      qr_tma_3d(dst, &tm_w, 0, ra, pr.ch * STEPS, bar);
-      qr_tma_3d(dst + CODE_BYTES / 2, &tm_w, 0, rb, pr.ch * STEPS, bar);
+      tma_load_3d(dst, &tm_w, 0, ra, pr.ch * STEPS, bar);
+      tma_load_3d(dst + CODE_BYTES / 2, &tm_w, 0, rb, pr.ch * STEPS, bar);
       tma_load_2d(sdst, &tm_s, pr.ch * 8, ra, bar);
       tma_load_2d(sdst + 128, &tm_b, pr.ch * 8, ra, bar);
       tma_load_2d(sdst + 256, &tm_s, pr.ch * 8, rb, bar);
@@ -263,7 +237,7 @@ qmv_ring_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
   int seg_start = u0;                                      // first unit of the current tile that this warp computed
   bool ok = true;
   for (int u = u0; u < u1; ++u) {
-    if (!(ok = qr_wait(my_bar + 8 * stage, ph))) break;
+    if (!(ok = mbar_wait_warp(my_bar + 8 * stage, ph, nullptr, &g_qmv_ring_fault, 0))) break;      // (a warp's stages are its own: it gives up alone)
     const uint32_t sb = my_ring + stage * CODE_BYTES + g * 128, ss = my_scales + stage * SCALE_BYTES + g * 16;
     const uint8_t* xs = x_mine + ((at.ch * QR_UNIT_K - k0) / STEP_K) * x_step;
 #pragma unroll
@@ -352,10 +326,7 @@ qmv_ring_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
     }
     if (u + 1 < u1) qr_next(p, at);
   }
-  if (!ok) {                                               // gave up: copies in flight land before the CTA goes
-    const long long t0 = clock64();
-    while (clock64() - t0 < 100000000ll) {}
-  }
+  if (!ok) wait_settle();
   // ---- tiles shared by several warps of the CTA: the warp that opened a tile adds the others' pieces in warp order
   if (lane == 0) seg_of[warp] = parked0;
   __syncthreads();

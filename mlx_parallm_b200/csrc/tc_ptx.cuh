@@ -32,6 +32,57 @@ __device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity) {
       "r"(parity)
       : "memory");
 }
+// ---- bounded waits: they give up after about a second, or as soon as another role of the CTA has (abort; null: the waiter is on its own),
+// and then return false.  A role that gives up leaves through the kernel's common exit.
+__device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+      "selp.b32 %0, 1, 0, p;\n"
+      "}\n"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+constexpr long long WAIT_CYCLES = 2000000000ll;
+__device__ __forceinline__ void wait_gave_up(volatile int* abort, int* word, int role) {
+  if (abort) *abort = 1;
+  atomicCAS(word, 0, 1 + role);
+}
+// One thread:
+__device__ __forceinline__ bool mbar_wait_lane(uint32_t bar, uint32_t parity, volatile int* abort, int* word, int role) {
+  const long long t0 = clock64();
+  for (;;) {
+    if (mbar_try_wait(bar, parity)) return true;
+    if (abort && *abort) return false;
+    if (clock64() - t0 > WAIT_CYCLES) {
+      wait_gave_up(abort, word, role);
+      return false;
+    }
+  }
+}
+// A whole warp, by vote.  Lanes on their own may see the barrier's phase end at different polls, and a loop with two ways out brings them
+// together only where both meet again, but what follows (tcgen05.ld / .st, mma.sync) is for all lanes at once.  Voting at every poll also keeps
+// the loop's branches uniform: one vote after a loop of lanes is 5 to 12 % slower in the wide products (28672 x 4096 at 4096 tokens 930 / 820 us).
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort, int* word, int role) {
+  const long long t0 = clock64();
+  for (;;) {
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+    if (__any_sync(0xffffffffu, clock64() - t0 > WAIT_CYCLES)) {
+      wait_gave_up(abort, word, role);
+      return false;
+    }
+    if (abort && __any_sync(0xffffffffu, *abort != 0)) return false;
+  }
+}
+// after giving up: the CTA's copies and MMAs in flight come to their end (microseconds) before its memory is another's
+__device__ __forceinline__ void wait_settle() {
+  const long long t0 = clock64();
+  while (clock64() - t0 < 100000000ll) {}
+}
 // one lane of a CONVERGED warp; unlike `lane == 0` the compiler knows the guarded code is warp-uniform, so tcgen05 /
 // TMA operands go straight to uniform registers (no per-instruction uniformisation loop)
 __device__ __forceinline__ bool elect_one() {
@@ -53,6 +104,12 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
       "l"(map), "r"(c0), "r"(c1), "r"(bar)
+      : "memory");
+}
+__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(dst),
+      "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(bar)
       : "memory");
 }
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* map) {

@@ -673,6 +673,24 @@ def test_qmm_wide_tiles(ops, M, N, K, bits, dtype, epi, small):
     assert rel_err(got, exp) < {"float16": 3e-3, "bfloat16": 2e-2}[dtype]
 
 
+@pytest.mark.parametrize("M,N,K,bits,dtype", [(201, 2048, 4096, 8, "bfloat16"), (250, 18944, 1024, 8, "bfloat16"), (300, 4096, 2048, 4, "float16")])
+def test_qmm_wide_tiles_repeat_bit_for_bit(ops, M, N, K, bits, dtype):
+    """Whole tiles are summed in a fixed order: hundreds of launches over the same operands agree in every bit.  (A k-block of one row that is
+    lost on its way to the tensor core shows as a column that differs.)"""
+    g = torch.Generator(device="cuda")
+    g.manual_seed(M)
+    dt = TD[dtype]
+    w = torch.randint(-2 ** 31, 2 ** 31, (N, K * bits // 32), generator=g, device="cuda", dtype=torch.int64).to(torch.int32)
+    s = ((torch.rand((N, K // 64), generator=g, device="cuda") + 0.5) * 2 / (2 ** bits - 1) / K ** 0.5).to(dt)
+    b = (-s.float() * (2 ** bits - 1) / 2).to(dt)
+    x, ws = torch.randn((M, K), generator=g, device="cuda").to(dt), torch.zeros(ops.qmm_workspace_bytes(M, N, K), dtype=torch.uint8, device="cuda")
+    first = ops.qmm(x, w, s, b, 64, bits, 1, workspace=ws, small_scale=True)
+    bad = torch.zeros((), dtype=torch.int64, device="cuda")
+    for _ in range(300):
+        bad += (ops.qmm(x, w, s, b, 64, bits, 1, workspace=ws, small_scale=True) != first).sum()
+    assert int(bad) == 0
+
+
 # ---------------------------------------------------------------- TMA-ring GEMV of b200p_qmm (M <= 16)
 @pytest.mark.parametrize("M,N,K,bits,dtype,epi,small", [
     (1, 16, 512, 4, "float16", 1, True),          # one unit: seven of eight warps have nothing to do
