@@ -476,6 +476,9 @@ static Plan make_plan(int64_t M, int64_t N, int64_t K, int bits, int epi) {
   const int fixed = 1024 + NSB * 2 * SB_TILE_BYTES + (add ? WORKERS * STAGE_OUT_BYTES : 0) + (int)sizeof(Shared);
   int st = (SMEM_BUDGET - fixed - X_SLOTS * pl.TN * 128) / W_STAGE_BYTES;
   pl.w_stages = st > MAX_STAGES ? MAX_STAGES : st;
+  // 8 bits: a group of dequantisers takes every second stage.  With an odd ring it would come to each slot every second time round, and
+  // a wait for a slot's phase does not tell the fill before last from one that is still on its way.
+  if (bits == 8) pl.w_stages &= ~1;
   pl.smem = fixed + X_SLOTS * pl.TN * 128 + pl.w_stages * W_STAGE_BYTES;
   return pl;
 }

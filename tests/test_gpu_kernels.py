@@ -664,6 +664,8 @@ def test_qmm_arguments_of_the_tile_kernel_stay_required(ops, M, N, K, bits, epi)
     (140, 512, 2048, 8, "float16", 1, True),      # 8 bits: two k-blocks per stage
     (333, 384, 1024, 8, "bfloat16", 3, False),
     (205, 260 * 4, 512, 8, "bfloat16", 2, False),
+    (201, 264, 8192, 8, "bfloat16", 2, True),     # accumulate: token tiles of 208, beside which an odd number of weight stages would fit
+    (256, 512, 8192, 8, "float16", 0, False),     # the same of 256
 ])
 def test_qmm_wide_tiles(ops, M, N, K, bits, dtype, epi, small):
     """csrc/qmm_wide.cu against the oracle.  Tolerances as for the other 16-bit paths (A rounded to the storage type, fp32 sums)."""
