@@ -10,8 +10,8 @@
 // global -> shared with cp.async (two stages, XOR-swizzled 16-byte chunks, shared by the four warps); S = Q K^T and O += P V
 // run on mma.sync m16n8k16 with an fp32 online softmax in registers -- the same fragment plumbing as the decode kernel
 // (attn_decode.cu).  No barrier, TMEM or tensor-map set-up: the kernel of the smallest calls (at most 64 new tokens over at most 256
-// positions: 4 to 5 us against 7 to 9 us on tcgen05) and of negative scales; attn_prefill_tc.cu takes everything else, the rule is in
-// c_api.cu.
+// positions: 4 to 5 us against 7 to 9 us on tcgen05) and of scales that are no normal positive number; attn_prefill_tc.cu takes
+// everything else, the rule is in c_api.cu.
 #include "common.cuh"
 #include "mma_util.cuh"
 

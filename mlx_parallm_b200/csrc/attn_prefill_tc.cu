@@ -287,7 +287,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_con
       }
       t0 = max3(t0, s[124], s[125]);
       t1 = max3(t1, s[126], s[127]);
-      const float mt = fmaxf(fmaxf(t0, t1), fmaxf(t2, t3)) * p.scale_log2e;          // (the scale is positive)
+      const float mt = fmaxf(fmaxf(t0, t1), fmaxf(t2, t3)) * p.scale_log2e;          // (the scale is normal and positive)
       // the first tile holds key 0, which every row sees: m is finite from then on.  O(j - 1) is complete: S(j) was issued behind it
       if (__any_sync(0xffffffffu, mt > m + 8.f)) {
         const float mn = fmaxf(m, mt);

@@ -1,4 +1,5 @@
 // C-ABI glue: the path dispatchers of b200p_qmm / b200p_attn (error plumbing and device checks: runtime.cu).
+#include <float.h>
 #include <stdlib.h>
 
 #include "common.cuh"
@@ -204,11 +205,14 @@ extern "C" int b200p_attn(const void* q, const void* kcache, const void* vcache,
   // the SMs at most twice with mma.sync CTAs (64 queries of one head each) is shorter than the tcgen05 kernel's set-up (32 / 8
   // heads, B=1, empty cache, L=2 / 16 / 64: 4.1 / 4.4 / 4.9 against 6.9 / 6.9 / 9.0 us).  Beyond it tcgen05 wins at every size: 1000
   // cached positions 18.6 against 27.7 us (L=2, B=1), L=200 at B=8 19.6 against 33.5 us, L=777 at 8000 cached 125 against 568 us.
-  // (Its softmax takes the maximum before the scale, so negative scales stay on the mma.sync kernel.)
+  // (Its softmax masks and takes the maximum before it scales, so a scale that is no normal positive number -- negative, zero, or so
+  // small that a masked score's -inf would be lost -- stays on the mma.sync kernel, which scales first.)
+  const float scale_log2e = scale * 1.4426950408889634f;
+  const bool pf_scale = scale_log2e >= FLT_MIN && scale_log2e <= FLT_MAX;
   const bool pf_small = L <= 64 && Tcap <= 256 && B * Hq <= 2 * (int64_t)sm_count();
   // (What does not fit its 32-bit row numbers stays there too, to be run or refused as it is.)
   const bool pf_fits = L < (1ll << 30) && Tcap < (1ll << 31) - 128 && B < 65536 && Hq < 65536;
-  if (g_attn_path != 1 && scale >= 0.f && pf_fits && (g_attn_path == 3 || !pf_small) && attn_prefill_tc_supported(L, Hq, Hkv, D, dtype))
+  if (g_attn_path != 1 && pf_scale && pf_fits && (g_attn_path == 3 || !pf_small) && attn_prefill_tc_supported(L, Hq, Hkv, D, dtype))
     return attn_prefill_tc_launch(q, kcache, vcache, lengths, out, B, L, Hq, Hkv, D, Tcap, scale, dtype, out_perm, st);
   if (pf_ok && g_attn_path != 1)
     return attn_prefill_launch(q, kcache, vcache, lengths, out, B, L, Hq, Hkv, D, Tcap, scale, dtype, out_perm, st);

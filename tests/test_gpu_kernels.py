@@ -393,6 +393,56 @@ def test_attention_tcgen05_prefill(ops, dtype, B, L, Hq, Hkv, lengths, perm):
     assert rel_err(got, exp) < {"float16": 2e-3, "bfloat16": 1.2e-2}[dtype]
 
 
+def prefill(ops, q, k, v, lengths, scale, path=0):
+    """ops.attn over prompts: q [B, L, Hq, D], k / v [B, Hkv, Tcap, D] -> [B, L, Hq, D]."""
+    from mlx_parallm_b200 import _lib
+    B, L, Hq, D = q.shape
+    out = torch.full((B, L, Hq * D), 7.0, dtype=q.dtype, device="cuda")
+    ws = torch.empty((max(ops.attn_workspace_bytes(B, L, Hq, D), 16),), dtype=torch.uint8, device="cuda")
+    _lib.check(_lib.lib().b200p_attn_set_path(path))
+    try:
+        ops.attn(q, k, v, torch.tensor(lengths, dtype=torch.int32, device="cuda"), out, B, L, Hq, k.shape[1], D, scale, workspace=ws)
+    finally:
+        _lib.lib().b200p_attn_set_path(0)
+    assert _lib.lib().b200p_attn_tc_fault() == 0
+    return out.view(B, L, Hq, D)
+
+
+def prefill_exact(q, k, v, lengths, scale):
+    """The same in 64 bits."""
+    B, L, Hq, D = q.shape
+    out = torch.empty((B, L, Hq, D), dtype=torch.float64, device="cuda")
+    for b in range(B):
+        n = lengths[b] + L
+        kb, vb = (t[b, :, :n].double().repeat_interleave(Hq // k.shape[1], 0) for t in (k, v))
+        s = torch.einsum("lhd,htd->hlt", q[b].double(), kb) * scale
+        s.masked_fill_(torch.arange(n, device="cuda")[None, None] > (lengths[b] + torch.arange(L, device="cuda"))[None, :, None], -float("inf"))
+        out[b] = torch.einsum("hlt,htd->lhd", s.softmax(-1), vb)
+    return out
+
+
+def prefill_inputs(dtype, B, L, Hq, Hkv, Tcap, seed, spread=1.0):
+    """Queries, keys, values; scores q.k / sqrt(128) have standard deviation ``spread``."""
+    g = torch.Generator(device="cuda")
+    g.manual_seed(seed)
+    r = lambda *shape: torch.randn(shape, generator=g, device="cuda")
+    return (r(B, L, Hq, 128) * spread).to(TD[dtype]), r(B, Hkv, Tcap, 128).to(TD[dtype]), r(B, Hkv, Tcap, 128).to(TD[dtype])
+
+
+@pytest.mark.parametrize("dtype", ["float16", "bfloat16"])
+@pytest.mark.parametrize("scale", [0.0, 1e-44, 1e-39, -0.11, 2e-38])
+@pytest.mark.parametrize("path", [0, 3])
+def test_attention_prefill_of_scales_that_are_not_normal_positive_numbers(ops, dtype, scale, path):
+    """Scale 0 is the mean of the visible values (masked scores stay masked), as are scales below the normal numbers; 2e-38 is the
+    smallest kind that the tcgen05 kernel takes; negative scales prefer the least similar keys.  70 tokens over up to 370 positions: beyond the rule for
+    the smallest calls.  Tolerances as for the other prefill tests."""
+    q, k, v = prefill_inputs(dtype, 2, 70, 8, 2, 400, seed=3)
+    got = prefill(ops, q, k, v, [0, 300], scale, path)
+    exp = prefill_exact(q, k, v, [0, 300], scale)
+    assert torch.isfinite(got).all()
+    assert rel_err(got.float().cpu().numpy(), exp.cpu().numpy()) < {"float16": 2e-3, "bfloat16": 1.2e-2}[dtype]
+
+
 # ---------------------------------------------------------------- samplers
 def test_argmax_ties_and_probs(ops):
     rng = np.random.default_rng(6)
