@@ -189,7 +189,7 @@ int b200p_attn_decode_static(const void* q, const void* kcache, const void* vcac
                              float scale, int dtype, int flags, void* stream);
 /* 0 = auto, 1 = generic CUDA-core kernel only, 2 = tensor kernels only: split-K decode for L == 1, causal flash prefill for
  * L > 1 (16-bit, head_dim 128: tcgen05, mma.sync for the smallest calls and for scales that are no normal positive number),
- * 3 = tcgen05 for the smallest calls too */
+ * 3 = tcgen05 for the smallest calls too, 4 = mma.sync for every such prefill */
 int b200p_attn_set_path(int path);
 /* 0, or 1 + the role (0 loader, 1 MMA issuer, 2 / 3 softmax) whose bounded barrier wait ran out in a tcgen05 prefill attention
  * since the last call (which clears it).  Synchronises the device. */

@@ -72,7 +72,7 @@ static bool qmv_ring_preferred(int64_t M, int64_t N, int64_t K, int bits, int ep
   if (epi != B200P_EPI_ADD_RESIDUAL) return M <= (bits == 4 ? 6 : 8);
   return bits == 4 && M <= 4 && N * K <= (M <= 2 ? 2 : 1) * g_gemv_max_weights;
 }
-static int g_attn_path = 0;  // 0 auto, 1 generic, 2 tensor
+static int g_attn_path = 0;  // 0 auto, 1 generic, 2 tensor, 3 tcgen05 prefill at any size, 4 mma.sync prefill at any size
 }  // namespace b200p
 
 using namespace b200p;
@@ -90,7 +90,7 @@ extern "C" int b200p_qmm_set_path(int path) {
 }
 
 extern "C" int b200p_attn_set_path(int path) {
-  B200P_REQUIRE(path >= 0 && path <= 3, B200P_ERR_ARG, "path must be 0..3");
+  B200P_REQUIRE(path >= 0 && path <= 4, B200P_ERR_ARG, "path must be 0..4");
   g_attn_path = path;
   return B200P_OK;
 }
@@ -212,7 +212,7 @@ extern "C" int b200p_attn(const void* q, const void* kcache, const void* vcache,
   const bool pf_small = L <= 64 && Tcap <= 256 && B * Hq <= 2 * (int64_t)sm_count();
   // (What does not fit its 32-bit row numbers stays there too, to be run or refused as it is.)
   const bool pf_fits = L < (1ll << 30) && Tcap < (1ll << 31) - 128 && B < 65536 && Hq < 65536;
-  if (g_attn_path != 1 && pf_scale && pf_fits && (g_attn_path == 3 || !pf_small) && attn_prefill_tc_supported(L, Hq, Hkv, D, dtype))
+  if (g_attn_path != 1 && g_attn_path != 4 && pf_scale && pf_fits && (g_attn_path == 3 || !pf_small) && attn_prefill_tc_supported(L, Hq, Hkv, D, dtype))
     return attn_prefill_tc_launch(q, kcache, vcache, lengths, out, B, L, Hq, Hkv, D, Tcap, scale, dtype, out_perm, st);
   if (pf_ok && g_attn_path != 1)
     return attn_prefill_launch(q, kcache, vcache, lengths, out, B, L, Hq, Hkv, D, Tcap, scale, dtype, out_perm, st);

@@ -342,9 +342,11 @@ def test_attention_generic_prefill_causal(ops):
     ("float16", 1, 200, 4, 4, [64]),              # several key tiles, MHA
     ("float16", 2, 64, 8, 8, [0, 0]),             # exactly one query tile, pure causal
 ])
-def test_attention_tensor_prefill_causal(ops, dtype, B, L, Hq, Hkv, lengths):
-    """mma.sync flash prefill (attn_prefill.cu) against the oracle's SDPA with the additive causal mask."""
-    got, exp = attn_case(ops, B, L, Hq, Hkv, 128, lengths, dtype, path=2)
+@pytest.mark.parametrize("path", [2, 4])
+def test_attention_tensor_prefill_causal(ops, dtype, B, L, Hq, Hkv, lengths, path):
+    """Tensor prefill against the oracle's SDPA with the additive causal mask: as dispatched (the second and the last case on mma.sync,
+    attn_prefill.cu, the others on tcgen05) and all of it on mma.sync."""
+    got, exp = attn_case(ops, B, L, Hq, Hkv, 128, lengths, dtype, path=path)
     assert rel_err(got, exp) < {"float16": 2e-3, "bfloat16": 1.2e-2}[dtype]
     gen, _ = attn_case(ops, B, L, Hq, Hkv, 128, lengths, dtype, path=1)
     assert rel_err(got, gen) < {"float16": 2e-3, "bfloat16": 1.2e-2}[dtype]
