@@ -289,8 +289,11 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_con
       t1 = max3(t1, s[126], s[127]);
       const float mt = fmaxf(fmaxf(t0, t1), fmaxf(t2, t3)) * p.scale_log2e;          // (the scale is normal and positive)
       // the first tile holds key 0, which every row sees: m is finite from then on.  O(j - 1) is complete: S(j) was issued behind it
-      if (__any_sync(0xffffffffu, mt > m + 8.f)) {
-        const float mn = fmaxf(m, mt);
+      // Each row decides for itself (the vote only skips the work where no row wants it): a row's bits depend on its own scores, not on
+      // which tokens and heads share its warp.
+      const bool grow = mt > m + 8.f;
+      if (__any_sync(0xffffffffu, grow)) {
+        const float mn = grow ? mt : m;
         if (j > 0) {
           const float f = ex2(m - mn);
           sum *= f;

@@ -445,6 +445,26 @@ def test_attention_prefill_of_scales_that_are_not_normal_positive_numbers(ops, d
     assert rel_err(got.float().cpu().numpy(), exp.cpu().numpy()) < {"float16": 2e-3, "bfloat16": 1.2e-2}[dtype]
 
 
+@pytest.mark.parametrize("dtype", ["float16", "bfloat16"])
+@pytest.mark.parametrize("path", [3, 4])
+def test_attention_prefill_rows_do_not_depend_on_their_neighbours(ops, dtype, path):
+    """A token's output is a function of its own query and the keys before it, bit for bit: other tokens' and heads' scores grow at other
+    tiles, and a prompt cut into two portions puts a token into another tile row beside other tokens."""
+    q, k, v = prefill_inputs(dtype, 1, 150, 8, 2, 1300, seed=11, spread=2.0)
+    one = prefill(ops, q, k, v, [1100], 128 ** -0.5, path)
+    other = q.clone()
+    other[:, 1::2] *= 3
+    other[:, :, ::4] = 0
+    keep = torch.zeros((1, 150, 8, 1), dtype=torch.bool, device="cuda")
+    keep[:, ::2] = True
+    keep[:, :, ::4] = False
+    two = prefill(ops, other, k, v, [1100], 128 ** -0.5, path)
+    assert torch.equal(one.masked_fill(~keep, 0), two.masked_fill(~keep, 0))
+    for cut in (37, 90):
+        parts = [prefill(ops, q[:, a:b].contiguous(), k, v, [1100 + a], 128 ** -0.5, path) for a, b in ((0, cut), (cut, 150))]
+        assert torch.equal(one, torch.cat(parts, 1))
+
+
 # ---------------------------------------------------------------- samplers
 def test_argmax_ties_and_probs(ops):
     rng = np.random.default_rng(6)
