@@ -465,6 +465,17 @@ def test_attention_prefill_rows_do_not_depend_on_their_neighbours(ops, dtype, pa
         assert torch.equal(one, torch.cat(parts, 1))
 
 
+@pytest.mark.parametrize("dtype", ["float16", "bfloat16"])
+@pytest.mark.parametrize("spread", [1.0, 2.0, 4.0])
+def test_attention_tcgen05_prefill_is_as_exact_as_the_mma_sync_kernel(ops, dtype, spread):
+    """Error against 64 bits over 6000 keys, from flat rows to rows that one key dominates.  Both kernels round the probabilities and the
+    output to 16 bits; over half a million outputs their errors agree to better than a percent if nothing else is rounded."""
+    q, k, v = prefill_inputs(dtype, 1, 64, 64, 8, 6064, seed=int(spread), spread=spread)
+    exp = prefill_exact(q, k, v, [6000], 128 ** -0.5)
+    err = {path: float((prefill(ops, q, k, v, [6000], 128 ** -0.5, path).double() - exp).norm() / exp.norm()) for path in (3, 4)}
+    assert err[3] < 1.01 * err[4], err
+
+
 # ---------------------------------------------------------------- samplers
 def test_argmax_ties_and_probs(ops):
     rng = np.random.default_rng(6)
