@@ -152,7 +152,9 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_con
   const int l0 = pair * 2 * p.qpt;
   pdl_wait();
   const int len_b = p.lengths[b];
-  const int kend = (int)min((int64_t)len_b + min(p.L, l0 + 2 * p.qpt), p.Tcap);      // keys any row of this CTA may see
+  // keys any row of this CTA may see; at least one, so that rows that see none (negative lengths) come out as NaN from one masked tile
+  // instead of waiting for a tile that nobody fetches
+  const int kend = max(1, (int)min((int64_t)len_b + min(p.L, l0 + 2 * p.qpt), p.Tcap));
   const int n_tiles = (kend + FT_KEYS - 1) / FT_KEYS;
 
   if (warp >= 8) {

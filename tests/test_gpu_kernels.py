@@ -476,6 +476,17 @@ def test_attention_tcgen05_prefill_is_as_exact_as_the_mma_sync_kernel(ops, dtype
     assert err[3] < 1.01 * err[4], err
 
 
+def test_attention_prefill_of_rows_that_see_no_key(ops):
+    """Negative cache lengths: tokens without a visible key are NaN on both kernels, the others are as usual; no wait runs out."""
+    q, k, v = prefill_inputs("float16", 3, 70, 8, 2, 400, seed=5)
+    lengths = [-500, -30, 200]
+    for path in (3, 4):
+        got = prefill(ops, q, k, v, lengths, 128 ** -0.5, path)
+        assert torch.isnan(got[0]).all() and torch.isnan(got[1, :30]).all()
+        exp = prefill_exact(q[1:, 30:].contiguous(), k[1:], v[1:], [0, 230], 128 ** -0.5)
+        assert rel_err(got[1:, 30:].float().cpu().numpy(), exp.cpu().numpy()) < 2e-3
+
+
 # ---------------------------------------------------------------- samplers
 def test_argmax_ties_and_probs(ops):
     rng = np.random.default_rng(6)
