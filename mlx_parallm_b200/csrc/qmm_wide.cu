@@ -365,9 +365,11 @@ qmm_wide_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
     const uint32_t out_stage = epi_ring + (uint32_t)((1 + grp) * STAGE_OUT_BYTES);
     int pending = -1;                                       // the previous segment's tile, still to be drained
     uint32_t drained = 0;                                   // segments drained so far
+    bool voted = false;                                     // (ADD) left by the vote that drain() begins with
     auto drain_pending = [&]() {
       pdl_wait();                                           // y belongs to the previous kernels until here
       ok = drain<T, FAST, ADD>(p, &tm_y, sh, tmem, pending, drained & 1u, 1 + grp, q, lane, out_stage);
+      voted = !ok;
       pending = -1;
       ++drained;
     };
@@ -429,6 +431,8 @@ qmm_wide_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
       pending = tile;
     }
     if (ok && pending >= 0) drain_pending();
+    // A warp that gave up outside a drain still owes its group one vote: the others come to it at their next drain, or here.
+    if (ADD && !ok && !voted) all_of(2 + grp, 128, false);
     if (ADD && lane == 0) bulk_wait_all();                  // staging memory and outputs are settled before the CTA retires
   } else {
     // ===================================== epilogue =========================================
