@@ -35,6 +35,8 @@ extern "C" {
 #define B200P_ERR_ALIGN  -2   /* pointer or leading dimension not aligned as required */
 #define B200P_ERR_ARCH   -3   /* device is not sm_100 */
 #define B200P_ERR_CUDA   -4   /* CUDA runtime error (message in b200p_last_error) */
+#define B200P_ERR_TIMEOUT -5  /* a bounded wait inside an earlier launch gave up: outputs since then are incomplete.  Calls that would
+                               * launch a kernel with such waits return it until the kernel's b200p_*_fault function has been called */
 
 enum { B200P_F32 = 0, B200P_F16 = 1, B200P_BF16 = 2 };
 
@@ -112,6 +114,11 @@ int b200p_qmm_tensor_supported(int64_t M, int64_t N, int64_t K, int group_size, 
  * 6 = TMA-ring GEMV only (csrc/qmv_ring.cu: M <= 16, K % 512 == 0, N % 16 == 0)
  * (2, 3, 4 and 6: error if the call is unsupported on that path) */
 int b200p_qmm_set_path(int path);
+/* 0, or 256 * (1 + kernel) + 1 + role once a bounded wait has given up (kernels: 0 dense GEMM, 1 prefill attention, 2 TMA-ring GEMV,
+ * 3 wide tiles).  A load from host memory, no synchronisation, clears nothing; replays of captured launches report there too. */
+int b200p_wait_fault(void);
+/* launches one warp that waits a millisecond for nothing and reports as the TMA-ring GEMV would (test of the report's way) */
+int b200p_wait_probe(void* stream);
 /* 1 if a bounded wait of the TMA-ring GEMV ran out since the last call (which clears it), else 0.  Synchronises the device. */
 int b200p_qmv_fault(void);
 /* the same for the wide tiles of more than 128 tokens (csrc/qmm_wide.cu): 0, or 1 + the role that gave up */

@@ -68,6 +68,8 @@ SIGNATURES = {
     "b200p_gemm_set_path": (_i32, [_i32]),
     "b200p_gemm_tc_fault": (_i32, []),
     "b200p_attn_tc_fault": (_i32, []),
+    "b200p_wait_fault": (_i32, []),
+    "b200p_wait_probe": (_i32, [_vp]),
     "b200p_qmv_fault": (_i32, []),
     "b200p_qmm_wide_fault": (_i32, []),
     "b200p_ragged_plan": (_i32, [_vp, _vp, _vp, _vp, _vp, _vp, _i32, _i64, _vp]),

@@ -20,7 +20,7 @@
 //
 // warp roles (384 threads): warps 0..3 / 4..7 softmax and output of tile 0 / 1 (thread = row), warp 8 MMA issuer (owns TMEM),
 // warp 9 TMA producer, warps 10 and 11 only give their registers away.  Shared memory: Q 2 x 32 KB, a ring of five 32 KB slots that alternate K and V tiles.
-// Every mbarrier wait is bounded; one that runs out raises g_attn_tc_fault and every role leaves through the common exit.
+// Every mbarrier wait is bounded; one that runs out is reported and every role leaves through the common exit.
 #include <cuda.h>
 
 #include <type_traits>
@@ -39,8 +39,6 @@ constexpr int FT_THREADS = 384;
 constexpr int FT_REGS_SOFTMAX = 216, FT_REGS_OTHER = 72;
 constexpr int FT_SMEM = 1024 + (2 + FT_RING) * FT_TILE_BYTES + 256;
 
-__device__ int g_attn_tc_fault;                            // 0, or 1 + the role that gave up waiting
-
 struct AttnTcParams {
   const int32_t* lengths;
   void* out;
@@ -49,6 +47,7 @@ struct AttnTcParams {
   int64_t Tcap;
   float scale_log2e;
   int out_perm, out_vec;
+  int* wait_word;               // where a wait that gives up reports
 };
 
 struct AttnTcShared {
@@ -57,8 +56,8 @@ struct AttnTcShared {
   volatile int abort;
 };
 
-__device__ __forceinline__ bool ft_wait(uint32_t bar, uint32_t parity, AttnTcShared* sh, int role) {
-  return mbar_wait_warp(bar, parity, &sh->abort, &g_attn_tc_fault, role);
+__device__ __forceinline__ bool ft_wait(uint32_t bar, uint32_t parity, AttnTcShared* sh, const AttnTcParams& p, int role) {
+  return mbar_wait_warp(bar, parity, &sh->abort, p.wait_word, role);
 }
 
 __device__ __forceinline__ void ft_tma_5d(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2, int c3, int c4, uint32_t bar) {
@@ -171,7 +170,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_con
       uint32_t ph = 0;
       const int z = b * p.Hkv + kvh;
       for (int issued = 0; issued < 2 * n_tiles; ++issued) {                         // K0 V0 K1 V1 ...
-        if (!mbar_wait_lane(smem_u32(&sh->kv_empty[slot]), ph ^ 1u, &sh->abort, &g_attn_tc_fault, 0)) break;
+        if (!mbar_wait_lane(smem_u32(&sh->kv_empty[slot]), ph ^ 1u, &sh->abort, p.wait_word, 0)) break;
         const uint32_t bar = smem_u32(&sh->kv_full[slot]), dst = ring + slot * FT_TILE_BYTES;
         mbar_arrive_expect_tx(bar, FT_TILE_BYTES);
         const CUtensorMap* m = (issued & 1) ? &tmv : &tmk;
@@ -199,7 +198,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_con
       for (int k = 0; k < 8; ++k)                          // 16 keys = 2048 bytes; P: 8 columns
         umma_f16_ts(tmem + 256 + 128 * i, tmem + 128 * i + 8 * k, bd + (uint64_t)(k * (2048 >> 4)), idesc_pv, (k || acc) ? 1u : 0u);
     };
-    bool ok = ft_wait(smem_u32(&sh->q_full), 0, sh, 1) && ft_wait(smem_u32(&sh->kv_full[0]), 0, sh, 1);
+    bool ok = ft_wait(smem_u32(&sh->q_full), 0, sh, p, 1) && ft_wait(smem_u32(&sh->kv_full[0]), 0, sh, p, 1);
     if (ok) {
       tc_fence_after();
       if (elect_one()) {
@@ -215,7 +214,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_con
     uint32_t ph = 0;                                       // phase of `slot`
     for (int j = 0; j < n_tiles && ok; ++j) {
       const int vslot = slot;
-      if (!(ok = ft_wait(smem_u32(&sh->kv_full[vslot]), ph, sh, 1))) break;
+      if (!(ok = ft_wait(smem_u32(&sh->kv_full[vslot]), ph, sh, p, 1))) break;
       if (++slot == FT_RING) { slot = 0; ph ^= 1u; }
       if (j == n_tiles - 1 && kend < n_tiles * FT_KEYS) {
         // the probabilities of keys past kend are zero, but what the cache holds there may not be finite: zero those rows of V
@@ -230,11 +229,11 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_con
       const bool more = j + 1 < n_tiles;
       const int kslot = slot;
       if (more) {
-        if (!(ok = ft_wait(smem_u32(&sh->kv_full[kslot]), ph, sh, 1))) break;
+        if (!(ok = ft_wait(smem_u32(&sh->kv_full[kslot]), ph, sh, p, 1))) break;
         if (++slot == FT_RING) { slot = 0; ph ^= 1u; }
       }
       for (int i = 0; i < 2; ++i) {
-        if (!(ok = ft_wait(smem_u32(&sh->p_full[i]), (uint32_t)(j & 1), sh, 1))) break;
+        if (!(ok = ft_wait(smem_u32(&sh->p_full[i]), (uint32_t)(j & 1), sh, p, 1))) break;
         tc_fence_after();
         if (elect_one()) {
           pv(i, vslot, j > 0 ? 1u : 0u);
@@ -268,7 +267,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_con
     const float2 sc2 = make_float2(p.scale_log2e, p.scale_log2e);
     bool ok = true;
     for (int j = 0; j < n_tiles; ++j) {
-      if (!(ok = ft_wait(smem_u32(&sh->s_full[i]), (uint32_t)(j & 1), sh, 2 + i))) break;
+      if (!(ok = ft_wait(smem_u32(&sh->s_full[i]), (uint32_t)(j & 1), sh, p, 2 + i))) break;
       tc_fence_after();
       float s[128];
 #pragma unroll
@@ -337,7 +336,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_con
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&sh->p_full[i]));
     }
-    if (ok) ok = ft_wait(smem_u32(&sh->o_full[i]), 0, sh, 2 + i);
+    if (ok) ok = ft_wait(smem_u32(&sh->o_full[i]), 0, sh, p, 2 + i);
     pdl_launch_dependents();
     if (ok) {
       tc_fence_after();
@@ -408,6 +407,7 @@ int attn_prefill_tc_launch(const void* q, const void* kc, const void* vc, const 
   TcEncodeFn enc = tc_get_encode();
   B200P_REQUIRE(enc != nullptr, B200P_ERR_CUDA, "cuTensorMapEncodeTiled entry point not available");
   AttnTcParams p;
+  if (const int rc = wait_word(WAIT_ATTN_TC, &p.wait_word)) return rc;
   p.lengths = lengths; p.out = out; p.L = (int)L; p.Hq = Hq; p.Hkv = Hkv; p.G = Hq / Hkv; p.qpt = FT_ROWS / p.G;
   p.pairs = (int)((L + 2 * p.qpt - 1) / (2 * p.qpt));
   p.Tcap = Tcap; p.scale_log2e = scale * 1.4426950408889634f; p.out_perm = out_perm; p.out_vec = aligned(out, 16) ? 1 : 0;
@@ -439,9 +439,4 @@ int attn_prefill_tc_launch(const void* q, const void* kc, const void* vc, const 
 
 // 0, or 1 + the role (0 loader, 1 MMA issuer, 2 / 3 softmax) of the first wait of a tcgen05 prefill attention that ran out;
 // reading clears it.  Synchronises the device.
-extern "C" int b200p_attn_tc_fault(void) {
-  int v = 0, zero = 0;
-  if (cudaMemcpyFromSymbol(&v, b200p::g_attn_tc_fault, sizeof(int)) != cudaSuccess) return -1;
-  if (v) cudaMemcpyToSymbol(b200p::g_attn_tc_fault, &zero, sizeof(int));
-  return v;
-}
+extern "C" int b200p_attn_tc_fault(void) { return b200p::wait_take(b200p::WAIT_ATTN_TC); }

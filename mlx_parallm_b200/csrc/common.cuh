@@ -30,6 +30,12 @@ int cuda_fail(cudaError_t e, const char* what);
     if (e__ != cudaSuccess) return ::b200p::cuda_fail(e__, what);  \
   } while (0)
 
+// ---- bounded device waits (tc_ptx.cuh): each kind of kernel has a word in page-locked host memory, which a wait that gives up writes.
+// Reading it costs the host a load and no synchronisation (runtime.cu).
+enum WaitKind { WAIT_GEMM_TC, WAIT_ATTN_TC, WAIT_QMV_RING, WAIT_QMM_WIDE, WAIT_KINDS };
+int wait_word(WaitKind kind, int** word);      // where the kernel reports; an error once any launch's wait has given up
+int wait_take(WaitKind kind);                  // synchronises the device, returns the word and clears it; -1: the device failed
+
 static inline bool aligned(const void* p, size_t a) { return (reinterpret_cast<uintptr_t>(p) % a) == 0; }
 
 // ---- storage-type traits ---------------------------------------------------------------------

@@ -37,8 +37,6 @@ int sm_count();
 constexpr int GT_BM = 128, GT_BK = 64, GT_THREADS = 192, GT_EPI_WARP0 = 2;
 constexpr int GT_A_BYTES = GT_BM * GT_BK * 2;
 
-__device__ int g_gemm_tc_fault;                   // 0, or 1 + the role that gave up waiting
-
 struct GemmTcParams {
   void* y;
   int64_t M, N, K, ldy, sy;
@@ -51,6 +49,7 @@ struct GemmTcParams {
   // memory first, every CTA counts the groups' tiles there
   const int32_t* seg;
   int groups;
+  int* wait_word;                // where a wait that gives up reports
 };
 constexpr int GT_MAX_GROUPS = 1024;
 
@@ -291,7 +290,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constant__ 
         const GemmTcTile tl = gemm_tc_tile(p, sh, t);
         const int z = tl.z, nt = tl.nt, mt = tl.mt, first = tl.first;
         for (int kb = kb0; kb < kb1; ++kb) {
-          if (!(ok = mbar_wait_lane(smem_u32(&sh->empty[stage]), phase ^ 1u, &sh->abort, &g_gemm_tc_fault, 0))) break;
+          if (!(ok = mbar_wait_lane(smem_u32(&sh->empty[stage]), phase ^ 1u, &sh->abort, p.wait_word, 0))) break;
           const uint32_t bar = smem_u32(&sh->full[stage]);
           const uint32_t dst = base + stage * STAGE_BYTES;
           mbar_arrive_expect_tx(bar, STAGE_BYTES);
@@ -314,12 +313,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constant__ 
       uint32_t phase = 0, acc_phase = 0;
       bool ok = true;
       for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
-        if (!(ok = mbar_wait_lane(smem_u32(&sh->acc_empty[acc]), acc_phase ^ 1u, &sh->abort, &g_gemm_tc_fault, 1))) break;
+        if (!(ok = mbar_wait_lane(smem_u32(&sh->acc_empty[acc]), acc_phase ^ 1u, &sh->abort, p.wait_word, 1))) break;
         tc_fence_after();
         const uint32_t d = tmem_base + (uint32_t)(acc * BN);
         const int kb0 = (t % p.splits) * p.kb_per_split, kb1 = min(p.num_kb, kb0 + p.kb_per_split);
         for (int kb = kb0; kb < kb1; ++kb) {
-          if (!(ok = mbar_wait_lane(smem_u32(&sh->full[stage]), phase, &sh->abort, &g_gemm_tc_fault, 1))) break;
+          if (!(ok = mbar_wait_lane(smem_u32(&sh->full[stage]), phase, &sh->abort, p.wait_word, 1))) break;
           tc_fence_after();
           const uint64_t ad = make_desc_sw128(base + stage * STAGE_BYTES);
           const uint64_t bd = make_desc_sw128(base + stage * STAGE_BYTES + GT_A_BYTES);
@@ -341,7 +340,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constant__ 
     for (int t = blockIdx.x; t < num_tiles; t += gridDim.x) {
       const GemmTcTile tl = gemm_tc_tile(p, sh, t);
       const int z = tl.z, nt = tl.nt, mt = tl.mt, first = tl.first, len = tl.len;
-      if (!mbar_wait_warp(smem_u32(&sh->acc_full[acc]), acc_phase, &sh->abort, &g_gemm_tc_fault, 2)) break;
+      if (!mbar_wait_warp(smem_u32(&sh->acc_full[acc]), acc_phase, &sh->abort, p.wait_word, 2)) break;
       tc_fence_after();
       const int64_t row = (int64_t)mt * GT_BM + lg * 32 + lane;               // within the batch index's (group's) rows
       const int64_t row_off = p.seg ? (first + row) * p.ldy : (int64_t)z * p.sy + row * p.ldy;
@@ -405,6 +404,7 @@ static int gemm_tc_run(const CUtensorMap& tmx, const CUtensorMap& tmw, GemmTcPar
     if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(gemm_tc_kernel)");
     attr_set = true;
   }
+  if (const int rc = wait_word(WAIT_GEMM_TC, &p.wait_word)) return rc;
   const int grid = p.num_tiles < sm_count() ? p.num_tiles : sm_count();
   kern<<<grid, GT_THREADS, smem, st>>>(tmx, tmw, p);
   B200P_LAUNCH_CHECK("gemm_tc_kernel");
@@ -547,9 +547,4 @@ template int gemm_tc_launch<__nv_bfloat16>(const __nv_bfloat16*, const __nv_bflo
 
 // 0, or 1 + the role (0 loader, 1 MMA issuer, 2 epilogue) of the first wait of a tcgen05 dense GEMM that ran out; reading
 // clears it.  Synchronises the device.
-extern "C" int b200p_gemm_tc_fault(void) {
-  int v = 0, zero = 0;
-  if (cudaMemcpyFromSymbol(&v, b200p::g_gemm_tc_fault, sizeof(int)) != cudaSuccess) return -1;
-  if (v) cudaMemcpyToSymbol(b200p::g_gemm_tc_fault, &zero, sizeof(int));
-  return v;
-}
+extern "C" int b200p_gemm_tc_fault(void) { return b200p::wait_take(b200p::WAIT_GEMM_TC); }

@@ -19,7 +19,7 @@
 //
 // Schedule: epilogues that need whole sums take whole tiles round robin (CTAs running at one time share
 // the larger operand through L2); the accumulating epilogue does the same as far as whole rounds go, cuts what is left into equal
-// ranges of (tile, K stage) and adds its sums with cp.reduce.async.bulk.tensor (as qmm_sk.cu does).  Every mbarrier wait is bounded (g_qmm_wide_fault).
+// ranges of (tile, K stage) and adds its sums with cp.reduce.async.bulk.tensor (as qmm_sk.cu does).  Every mbarrier wait is bounded; one that runs out is reported.
 //
 // Measured (bf16 or f16, us, before / after): gate|up 28672 x 4096 4-bit 62 / 51 at 201 tokens, 64 / 57 at 256, 235 / 208 at 1000, 500 / 390 at
 // 2048, 1261 / 780 at 4096 (1.2 PFLOP/s); 57344 x 8192 8-bit (bf16, with the fp32 dequantisation of dequant.cuh) 356 / 214 at 201, 1201 / 790 at 1000; down 4096 x 14336 405 / 359 at 4096.
@@ -55,8 +55,6 @@ constexpr int WORKERS = 1 + DQ_WARPS / 4;         // warps per lane quarter that
 constexpr int ADD_TOK = 8, STAGE_OUT_BYTES = ADD_TOK * 128 * 4;      // staging of four warps' partial sums: 8 tokens x 128 rows
 constexpr int SMEM_BUDGET = 227 * 1024;
 
-__device__ int g_qmm_wide_fault;                  // 0, or 1 + the role that gave up waiting
-
 struct Params {
   void* y;
   int M_tok, N, epi, y_perm;
@@ -65,6 +63,7 @@ struct Params {
   int num_st;                                     // stages along K
   int tiles_m, row_blocks, items, row_fast;       // token tiles, row blocks, all tiles and their order (tile_of)
   int w_stages;
+  int* wait_word;                                 // where a wait that gives up reports
 };
 struct Shared {
   uint64_t full_w[MAX_STAGES], empty_w[MAX_STAGES], full_x[X_SLOTS], empty_x[X_SLOTS], full_a[A_SLOTS], empty_a[A_SLOTS];
@@ -115,8 +114,8 @@ __device__ __forceinline__ void tile_of(const Params& p, int tile, int& rb, int&
   }
 }
 
-__device__ __forceinline__ bool wait(uint64_t* bar, uint32_t parity, Shared* sh, int role) {
-  return mbar_wait_warp(smem_u32(bar), parity, &sh->abort, &g_qmm_wide_fault, role);
+__device__ __forceinline__ bool wait(uint64_t* bar, uint32_t parity, Shared* sh, const Params& p, int role) {
+  return mbar_wait_warp(smem_u32(bar), parity, &sh->abort, p.wait_word, role);
 }
 
 // 16 tokens of one thread's output column
@@ -179,7 +178,7 @@ __device__ __forceinline__ bool drain(const Params& p, const CUtensorMap* tm_y, 
   tile_of(p, tile, rb, tm);
   const int tok0 = tm * p.TN;
   const uint32_t d = tmem + ((uint32_t)(q * 32) << 16);
-  bool ok = wait(&sh->acc_full[0], parity, sh, 4) && wait(&sh->acc_full[1], parity, sh, 4);
+  bool ok = wait(&sh->acc_full[0], parity, sh, p, 4) && wait(&sh->acc_full[1], parity, sh, p, 4);
   if (ADD) ok = all_of(1 + worker, 128, ok);                 // (the four warps meet at barriers below: one mind)
   if (!ok) return false;
   tc_fence_after();
@@ -270,7 +269,7 @@ qmm_wide_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
       tile_of(p, tile, rb, tm);
       for (int st = s0; st < s0 + ns; ++st) {
         if (st == s0 || st % SPG == 0) {                    // a new group of 8 k-blocks
-          if (!(ok = wait(&sh->sb_empty[sbi], sbph ^ 1u, sh, 0))) break;
+          if (!(ok = wait(&sh->sb_empty[sbi], sbph ^ 1u, sh, p, 0))) break;
           if (elect_one()) {
             const uint32_t dst = sb_ring + sbi * 2 * SB_TILE_BYTES, bar = smem_u32(&sh->sb_full[sbi]);
             const int kb0 = st / SPG * 8;
@@ -289,7 +288,7 @@ qmm_wide_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
           __syncwarp();
           if (++sbi == NSB) { sbi = 0; sbph ^= 1u; }
         }
-        if (!(ok = wait(&sh->empty_w[si], ph ^ 1u, sh, 0))) break;
+        if (!(ok = wait(&sh->empty_w[si], ph ^ 1u, sh, p, 0))) break;
         if (elect_one()) {
           const uint32_t dst = w_ring + si * W_STAGE_BYTES, bar = smem_u32(&sh->full_w[si]);
           mbar_arrive_expect_tx(bar, W_STAGE_BYTES);
@@ -313,7 +312,7 @@ qmm_wide_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
       tile_of(p, tile, rb, tm);
       const int tok0 = tm * p.TN;
       for (int kb = s0 * KPS; kb < (s0 + ns) * KPS; ++kb) {
-        if (!(ok = wait(&sh->empty_x[xs], ph ^ 1u, sh, 1))) break;
+        if (!(ok = wait(&sh->empty_x[xs], ph ^ 1u, sh, p, 1))) break;
         if (elect_one()) {
           const uint32_t bar = smem_u32(&sh->full_x[xs]);
           mbar_arrive_expect_tx(bar, x_bytes);
@@ -334,12 +333,12 @@ qmm_wide_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
       uint32_t slot = 0, aph = 0, xph = 0;
       for (; ok && segs.next(p, tile, s0, ns); ++seg) {
         if (seg > 0) {                                      // the epilogue has drained the previous segment's sums
-          if (!(ok = wait(&sh->acc_empty[h], (uint32_t)((seg - 1) & 1), sh, 2))) break;
+          if (!(ok = wait(&sh->acc_empty[h], (uint32_t)((seg - 1) & 1), sh, p, 2))) break;
           tc_fence_after();
         }
         const int nkb = ns * KPS;
         for (int j = 0; j < nkb; ++j) {
-          if (!(ok = wait(&sh->full_x[xs], xph, sh, 2) && wait(&sh->full_a[slot], aph, sh, 2))) break;
+          if (!(ok = wait(&sh->full_x[xs], xph, sh, p, 2) && wait(&sh->full_a[slot], aph, sh, p, 2))) break;
           tc_fence_after();
           if (elect_one()) {
             umma_half_kblock_f16_ts(d, tmem + A_COL0 + slot * 32, xdesc0 + (uint64_t)(xs * (x_bytes >> 4)), idesc, j > 0 ? 1u : 0u);
@@ -376,7 +375,7 @@ qmm_wide_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
     while (ok && segs.next(p, tile, s0, ns)) {
       for (int st = s0; st < s0 + ns; ++st, ++stage_no) {
         if (st == s0 || st % SPG == 0) {                    // scales / biases of this row for the next 8 k-blocks
-          if (!(ok = wait(&sh->sb_full[sbi], sbph, sh, 3))) break;
+          if (!(ok = wait(&sh->sb_full[sbi], sbph, sh, p, 3))) break;
           const uint32_t src = sb_ring + sbi * 2 * SB_TILE_BYTES + (uint32_t)(r * 16);
           s8 = lds128(src);
           b8 = lds128(src + SB_TILE_BYTES);
@@ -388,7 +387,7 @@ qmm_wide_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
         const bool mine = KPS == 4 || (int)(stage_no & 1u) == (grp >> 1);
         if (mine) {
           const int j = KPS == 4 ? grp : (grp & 1);
-          if (!(ok = wait(&sh->full_w[si], ph, sh, 3))) break;
+          if (!(ok = wait(&sh->full_w[si], ph, sh, p, 3))) break;
           constexpr int CPK = PKB / 16;
           uint4 pk[CPK];
           const uint32_t wsrc = w_ring + si * W_STAGE_BYTES + w_row;
@@ -413,7 +412,7 @@ qmm_wide_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
             for (int c = 0; c < 8; ++c) dequant8<T, BITS, XPERM>(pw + c * (BITS / 4), s2, b2, o + 4 * c);
           }
           const uint32_t n = stage_no * KPS + (uint32_t)j, slot = n & (A_SLOTS - 1);
-          if (!(ok = wait(&sh->empty_a[slot], ((n / A_SLOTS) & 1u) ^ 1u, sh, 3))) break;
+          if (!(ok = wait(&sh->empty_a[slot], ((n / A_SLOTS) & 1u) ^ 1u, sh, p, 3))) break;
           tc_fence_after();
           tmem_st32(a_dst + slot * 32, o);
           tmem_st_wait();
@@ -554,6 +553,7 @@ int qmm_wide_launch(const void* x, const uint32_t* w, const void* s, const void*
                 CU_TENSOR_MAP_SWIZZLE_NONE, "y");
   if (rc) return rc;
   Params p;
+  if ((rc = wait_word(WAIT_QMM_WIDE, &p.wait_word))) return rc;
   p.y = y; p.M_tok = (int)M; p.N = (int)N; p.epi = epi; p.y_perm = (flags & B200P_Y_PERM8) ? 1 : 0;
   p.TN = pl.TN; p.H0 = pl.H0; p.H1 = pl.H1; p.ldy = ldy; p.num_st = (int)(row_bytes / 128);
   p.tiles_m = pl.tiles_m; p.row_blocks = pl.row_blocks; p.items = pl.items; p.w_stages = pl.w_stages;
@@ -574,9 +574,4 @@ int qmm_wide_launch(const void* x, const uint32_t* w, const void* s, const void*
 
 // 0, or 1 + the role (0 weight loader, 1 X loader, 2 MMA issuer, 3 dequantiser, 4 epilogue) of the first wait of a wide quantised GEMM
 // that ran out; reading clears it.  Synchronises the device.
-extern "C" int b200p_qmm_wide_fault(void) {
-  int v = 0, zero = 0;
-  if (cudaMemcpyFromSymbol(&v, b200p::wide::g_qmm_wide_fault, sizeof(int)) != cudaSuccess) return -1;
-  if (v) cudaMemcpyToSymbol(b200p::wide::g_qmm_wide_fault, &zero, sizeof(int));
-  return v;
-}
+extern "C" int b200p_qmm_wide_fault(void) { return b200p::wait_take(b200p::WAIT_QMM_WIDE); }

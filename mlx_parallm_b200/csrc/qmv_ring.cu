@@ -42,8 +42,6 @@ bool pdl_enabled_gemm();
 constexpr int QR_STAGES = 2;
 constexpr int QR_UNIT_K = 512;
 
-__device__ int g_qmv_ring_fault;             // 1: a TMA stage never arrived
-
 struct QrParams {
   const void* x;
   void* y;
@@ -52,6 +50,7 @@ struct QrParams {
   int tiles;             // 16-row tiles (SILU_MUL: 8 gate rows and their 8 up rows)
   int chunks;            // K / 512
   int panels;            // k panels of the accumulating epilogue (1: none)
+  int* wait_word;        // where a wait that gives up reports
 };
 
 // unit u of the linear order (panel, tile, chunk within the panel): panel p covers chunks [p * chunks / panels, (p + 1) * chunks / panels)
@@ -237,7 +236,7 @@ qmv_ring_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
   int seg_start = u0;                                      // first unit of the current tile that this warp computed
   bool ok = true;
   for (int u = u0; u < u1; ++u) {
-    if (!(ok = mbar_wait_warp(my_bar + 8 * stage, ph, nullptr, &g_qmv_ring_fault, 0))) break;      // (a warp's stages are its own: it gives up alone)
+    if (!(ok = mbar_wait_warp(my_bar + 8 * stage, ph, nullptr, p.wait_word, 0))) break;      // (a warp's stages are its own: it gives up alone)
     const uint32_t sb = my_ring + stage * CODE_BYTES + g * 128, ss = my_scales + stage * SCALE_BYTES + g * 16;
     const uint8_t* xs = x_mine + ((at.ch * QR_UNIT_K - k0) / STEP_K) * x_step;
 #pragma unroll
@@ -405,6 +404,7 @@ int qmv_ring_launch(const void* x, const uint32_t* w, const void* s, const void*
   QrPlan pl;
   if (!qr_plan(M, p.tiles, p.chunks, bits, epi, &pl)) return 1;
   p.panels = pl.panels;
+  if (const int rc = wait_word(WAIT_QMV_RING, &p.wait_word)) return rc;
   TcEncodeFn enc = tc_get_encode();
   B200P_REQUIRE(enc != nullptr, B200P_ERR_CUDA, "cuTensorMapEncodeTiled entry point not available");
   const CUtensorMapDataType dt16 = dtype == B200P_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
@@ -441,9 +441,4 @@ int qmv_ring_launch(const void* x, const uint32_t* w, const void* s, const void*
 }  // namespace b200p
 
 // 1 after a TMA stage of qmv_ring_kernel failed to arrive in about a second; reading clears it.  Synchronises the device.
-extern "C" int b200p_qmv_fault(void) {
-  int v = 0, zero = 0;
-  if (cudaMemcpyFromSymbol(&v, b200p::g_qmv_ring_fault, sizeof(int)) != cudaSuccess) return -1;
-  if (v) cudaMemcpyToSymbol(b200p::g_qmv_ring_fault, &zero, sizeof(int));
-  return v;
-}
+extern "C" int b200p_qmv_fault(void) { return b200p::wait_take(b200p::WAIT_QMV_RING); }

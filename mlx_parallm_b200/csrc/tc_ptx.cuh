@@ -33,7 +33,7 @@ __device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity) {
       : "memory");
 }
 // ---- bounded waits: they give up after about a second, or as soon as another role of the CTA has (abort; null: the waiter is on its own),
-// and then return false.  A role that gives up leaves through the kernel's common exit.
+// report to the kernel's word (common.cuh) and return false.  A role that gives up leaves through the kernel's common exit.
 __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
@@ -50,15 +50,18 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
 constexpr long long WAIT_CYCLES = 2000000000ll;
 __device__ __forceinline__ void wait_gave_up(volatile int* abort, int* word, int role) {
   if (abort) *abort = 1;
-  atomicCAS(word, 0, 1 + role);
+  // Host memory: a plain store, any of several roles will do, seen when the kernel ends.  (A system fence after it costs the ring GEMV 0.2 to
+  // 0.5 us a launch although it never runs.)
+  *reinterpret_cast<volatile int*>(word) = 1 + role;
 }
 // One thread:
-__device__ __forceinline__ bool mbar_wait_lane(uint32_t bar, uint32_t parity, volatile int* abort, int* word, int role) {
+__device__ __forceinline__ bool mbar_wait_lane(uint32_t bar, uint32_t parity, volatile int* abort, int* word, int role,
+                                               long long cycles = WAIT_CYCLES) {
   const long long t0 = clock64();
   for (;;) {
     if (mbar_try_wait(bar, parity)) return true;
     if (abort && *abort) return false;
-    if (clock64() - t0 > WAIT_CYCLES) {
+    if (clock64() - t0 > cycles) {
       wait_gave_up(abort, word, role);
       return false;
     }
@@ -67,11 +70,12 @@ __device__ __forceinline__ bool mbar_wait_lane(uint32_t bar, uint32_t parity, vo
 // A whole warp, by vote.  Lanes on their own may see the barrier's phase end at different polls, and a loop with two ways out brings them
 // together only where both meet again, but what follows (tcgen05.ld / .st, mma.sync) is for all lanes at once.  Voting at every poll also keeps
 // the loop's branches uniform: one vote after a loop of lanes is 5 to 12 % slower in the wide products (28672 x 4096 at 4096 tokens 930 / 820 us).
-__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort, int* word, int role) {
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort, int* word, int role,
+                                               long long cycles = WAIT_CYCLES) {
   const long long t0 = clock64();
   for (;;) {
     if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
-    if (__any_sync(0xffffffffu, clock64() - t0 > WAIT_CYCLES)) {
+    if (__any_sync(0xffffffffu, clock64() - t0 > cycles)) {
       wait_gave_up(abort, word, role);
       return false;
     }

@@ -64,6 +64,15 @@ def _call(name: str, rc_fn):
     PROFILER.setdefault(key, []).append((s, e))
 
 
+def check_waits() -> None:
+    """Raise if a bounded wait inside an earlier kernel has given up: what has been computed since is incomplete.  A load from
+    host memory, no synchronisation."""
+    code = lib().b200p_wait_fault()
+    if code:
+        raise _lib.B200PError(f"a bounded wait of an earlier launch gave up (kernel {code // 256 - 1}, role {code % 256 - 1}): results since "
+                              "then are incomplete")
+
+
 # ------------------------------------------------------------------------------------------------
 def dequantize(w, scales, biases, group_size=64, bits=4, mode=DQ_F32_MULADD, out=None):
     """mx.dequantize: w int32/uint32 [N, K*bits/32] -> [N, K] in scales.dtype."""

@@ -250,6 +250,7 @@ class _DecodeStep:
         """Consume self.tok (ids of the previous step), leave logits (+ greedy tokens) for this one.  Runs under the
         model's forward lock: the scratch arena and the GEMM workspace belong to one step at a time, and a capture must
         not see another thread's launches (capture_error_mode thread_local: other threads may allocate meanwhile)."""
+        ops.check_waits()                 # a replay passes by the launch functions, which check this themselves
         with self.model._lock:
             rows = self.rows
             if rows is None:
@@ -373,6 +374,7 @@ def generate_step(
         if fx is not None and fx.status() != 0:
             raise RuntimeError("tensor-parallel exchange timed out waiting for a peer rank (status word "
                                f"{fx.status()}): results of this generation are invalid")
+        ops.check_waits()
         # same boundary, same reason: a row appended beyond its cache capacity is dropped by the kernel (it cannot happen
         # through prepare_cache, which grows the buffers first -- this is the loud failure if that invariant ever breaks)
         dropped = ops.kv_overflow_count(reset=True) if model.kernel_units is None else 0

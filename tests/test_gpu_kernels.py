@@ -909,3 +909,31 @@ def test_attention_tensor_matches_generic(ops):
     a, _ = attn_case(ops, 2, 1, 8, 2, 128, [1000, 37], "float16", path=2, seed=9)
     g, _ = attn_case(ops, 2, 1, 8, 2, 128, [1000, 37], "float16", path=1, seed=9)
     assert rel_err(a, g) < 2e-3
+
+
+# ---------------------------------------------------------------- bounded waits that give up
+def test_waits_that_give_up_are_reported(ops):
+    """A wait of a millisecond for an arrival that nothing makes: the host sees it without synchronising on anything but the launch, every
+    launch of a kernel with bounded waits is refused until the report has been taken, and then runs again."""
+    from mlx_parallm_b200 import _lib
+    L = _lib.lib()
+    q, k, v = prefill_inputs("float16", 1, 300, 4, 2, 300, seed=1)
+    before = prefill(ops, q, k, v, [0], 0.1)
+    x, w = torch.ones((200, 64), dtype=torch.float16, device="cuda"), torch.ones((64, 64), dtype=torch.float16, device="cuda")
+    wq, s = torch.zeros((256, 64), dtype=torch.int32, device="cuda"), torch.ones((256, 8), dtype=torch.float16, device="cuda")
+    xq, ws = torch.ones((200, 512), dtype=torch.float16, device="cuda"), torch.zeros(ops.qmm_workspace_bytes(200, 256, 512), dtype=torch.uint8, device="cuda")
+    calls = [lambda: prefill(ops, q, k, v, [0], 0.1), lambda: ops.gemm(x, w, 0), lambda: ops.qmm(xq, wq, s, s, workspace=ws)]
+    assert L.b200p_wait_fault() == 0
+    _lib.check(L.b200p_wait_probe(torch.cuda.current_stream().cuda_stream))
+    torch.cuda.synchronize()
+    assert L.b200p_wait_fault() == 256 * 3 + 1
+    for call in calls:
+        with pytest.raises(_lib.B200PError, match="gave up"):
+            call()
+    with pytest.raises(_lib.B200PError, match="gave up"):
+        ops.check_waits()
+    assert L.b200p_attn_tc_fault() == 0 and L.b200p_qmv_fault() == 1 and L.b200p_qmv_fault() == 0
+    ops.check_waits()
+    assert torch.equal(calls[0](), before)
+    for call in calls[1:]:
+        call()
