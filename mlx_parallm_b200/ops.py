@@ -26,11 +26,14 @@ def dtype_code(dt: torch.dtype) -> int:
 
 
 # The current device's current stream as an integer.  torch.cuda.current_stream() builds a Stream object around the same two
-# numbers: 3.2 us per launch against 0.2, a quarter of what a small call costs on the host.
-_raw_stream, _device_index = torch._C._cuda_getCurrentRawStream, torch._C._cuda_getDevice
+# numbers: 3.2 us per launch against 0.2, a quarter of what a small call costs on the host.  A torch built without CUDA has neither
+# function (and no launch to make); the package still imports there.
+_raw_stream, _device_index = getattr(torch._C, "_cuda_getCurrentRawStream", None), getattr(torch._C, "_cuda_getDevice", None)
 
 
 def _stream() -> int:
+    if _raw_stream is None or _device_index is None:
+        return torch.cuda.current_stream().cuda_stream
     return _raw_stream(_device_index())
 
 

@@ -76,3 +76,17 @@ def test_environment_switches_are_documented_and_exist():
     documented = set(re.findall(r"`(B200P_[A-Z0-9_]+)`", "\n".join(l.split("|")[1] for l in table.splitlines() if l.startswith("| `B200P_"))))
     assert read - documented == set(), f"read but not documented in INTEGRATION.md: {sorted(read - documented)}"
     assert documented - read == set(), f"documented but never read: {sorted(documented - read)}"
+
+
+def test_package_imports_on_a_torch_without_cuda():
+    """The private stream accessors are absent from such builds: importing the ops must not need them."""
+    import subprocess
+    import sys
+    code = ("import torch\n"
+            "for name in ('_cuda_getCurrentRawStream', '_cuda_getDevice'):\n"
+            "    delattr(torch._C, name)\n"
+            "from mlx_parallm_b200 import ops\n"
+            "import mlx_parallm_b200.utils\n"
+            "assert ops._raw_stream is None and ops._device_index is None\n")
+    r = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr[-2000:]
