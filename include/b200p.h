@@ -379,6 +379,11 @@ enum {
 int b200p_delta_scan(const float* qn, const float* kn, const float* v, const float* beta, const float* decay, float* state,
                      const int32_t* cu, const int32_t* rows, const int32_t* lengths, float* o, int nb, int H, int KH, int dk,
                      int dv, int mode, void* stream);
+/* the same, told how many tokens the entries have together (cu[nb], which lies on the device): decode steps take a kernel of their own.
+ * Results do not depend on it. */
+int b200p_delta_scan_tokens(const float* qn, const float* kn, const float* v, const float* beta, const float* decay, float* state,
+                            const int32_t* cu, const int32_t* rows, const int32_t* lengths, float* o, int64_t tokens, int nb, int H, int KH,
+                            int dk, int dv, int mode, void* stream);
 /* step 4: out[t, h, :] (dtype, row stride ld_out) = out_scale * o / sqrt(mean_dv(o^2) + eps) * norm_w * act(gate[t, h, :]);
  * gate fp32 with row stride ldg; gate_act 0 silu, 1 sigmoid.  H == 1 norms the dv values of a row as one group. */
 int b200p_delta_out(const float* o, const float* gate, int64_t ldg, const float* norm_w, void* out, int64_t ld_out, int64_t M,

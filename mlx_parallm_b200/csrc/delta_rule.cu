@@ -207,22 +207,11 @@ __global__ void delta_conv_commit_kernel(const float* __restrict__ proj, int64_t
     if (i < taps - 1) st[(int64_t)i * C] = keep[i];
 }
 
-// lanes that share a state column (lane l keeps rows [l * SEG, (l + 1) * SEG) in registers, SEG = dkp / lanes): 16 rows each, 8 for the
-// smallest keys
-constexpr int ds_lanes(int dkp) { return dkp <= 64 ? 4 : dkp / 16; }
-constexpr int ds_slots(int dkp) { return dkp <= 256 ? 32 : 16; }               // column slots per CTA
-constexpr int ds_threads(int dkp) { return ds_lanes(dkp) * ds_slots(dkp); }
-constexpr int ds_cols(int dkp) { return 2 * ds_slots(dkp); }                   // state columns per CTA: two per column slot
+// Rows of a state column are summed in segments: four interleaved partial sums each (rows i mod 4), combined in a fixed order, then the
+// segments pairwise.  Every kernel below, however many lanes it gives to a column, adds in this one order, so a token's numbers do not
+// depend on whether it arrives in a prompt or alone or on the size of the batch.
+constexpr int ds_segs(int dkp) { return dkp <= 64 ? 4 : dkp <= 128 ? 8 : dkp / 32; }
 
-// dk padded to DKP = 32 ... 512.  A thread owns SEG rows of TWO state columns: every q / k element read from shared memory serves two
-// columns.  The packed fp32 instructions of sm_100 (FMUL2 / FFMA2: both halves rounded like the scalar operation) take two ROWS of a
-// column at once, so that keys, queries and decays are operands as they are read (pairs of columns would need every one of them twice
-// in a register pair: 48 of 187 instructions per token and warp).  The chain of a token (scale and dot with k, reduce over the lanes, update) is what bounds the scan,
-// so each link is kept short: 16 rows per lane at 128-row states and two warps per scheduler that cover each other's latencies; a
-// reduction in which the two lanes of a pair first swap, so that one carries column j0 and the other j1 (1 + log2(lanes) exchanges for
-// two sums instead of 2 log2(lanes)); outputs whose exchanges run beside those of the next token; whole chunks as straight-line code.
-// 4 sequences of 256 to 512 tokens, 16 heads of 128 x 128, decays per channel: 278 -> 237 us, 0.46 us per token.  q and k of CHUNK tokens are staged in shared memory with every lane's part padded by 16 bytes, so the lanes' 128-bit
-// reads fall into different banks.
 // Sums of x and of y over the LANES lanes of a slot: even lanes get the sum of x, odd lanes that of y.
 template <int LANES>
 __device__ __forceinline__ float ds_reduce(float x, float y, bool odd) {
@@ -249,41 +238,137 @@ __device__ __forceinline__ float2 ds_reduce2(float x0, float y0, float x1, float
   return make_float2(r0, r1);
 }
 
+// A thread's SUB segments of SEG rows of two state columns, rows 2 i (.x) and 2 i + 1 (.y) packed: the packed fp32 instructions of sm_100
+// (FMUL2 / FFMA2: both halves rounded like the scalar operation) take two ROWS of a column at once, so that keys, queries and decays are
+// operands as they are read (pairs of columns would need every one of them twice in a register pair).
 // MODE 0: delta rule, one decay per head and token; 1: delta rule, one decay per head, key channel and token (decay
 // [M, H, dk]); 2: no correction, S <- g S + k v^T (one decay per head and token; beta unused).
-template <int DKP, int MODE, int PER_SM = 1>
-__global__ void __launch_bounds__(ds_threads(DKP), PER_SM)
+template <int SEG, int SUB> struct DsCols { float2 c0[SUB][SEG / 2], c1[SUB][SEG / 2]; };
+
+// scale by the decays and, for the delta rule, dot with the key: the thread's share of both sums
+template <int SEG, int SUB, int MODE>
+__device__ __forceinline__ float2 ds_decay_dot(DsCols<SEG, SUB>& S, const float* kp, const float* gp, float g, float2 (&kr)[SUB][SEG / 2]) {
+  float x[SUB], y[SUB];
+#pragma unroll
+  for (int u = 0; u < SUB; ++u) {
+    float2 d0[2], d1[2];
+#pragma unroll
+    for (int a = 0; a < 2; ++a) d0[a] = d1[a] = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int i = 0; i < SEG / 2; i += 2) {
+      const float4 k4 = *reinterpret_cast<const float4*>(kp + u * (SEG + 4) + 2 * i);
+      kr[u][i] = make_float2(k4.x, k4.y);
+      kr[u][i + 1] = make_float2(k4.z, k4.w);
+      float2 gg[2] = {make_float2(g, g), make_float2(g, g)};
+      if constexpr (MODE == 1) {
+        const float4 g4 = *reinterpret_cast<const float4*>(gp + u * (SEG + 4) + 2 * i);
+        gg[0] = make_float2(g4.x, g4.y), gg[1] = make_float2(g4.z, g4.w);
+      }
+#pragma unroll
+      for (int a = 0; a < 2; ++a) {
+        S.c0[u][i + a] = __fmul2_rn(S.c0[u][i + a], gg[a]);
+        S.c1[u][i + a] = __fmul2_rn(S.c1[u][i + a], gg[a]);
+        if constexpr (MODE != 2) {
+          d0[a] = __ffma2_rn(S.c0[u][i + a], kr[u][i + a], d0[a]);
+          d1[a] = __ffma2_rn(S.c1[u][i + a], kr[u][i + a], d1[a]);
+        }
+      }
+    }
+    x[u] = (d0[0].x + d0[0].y) + (d0[1].x + d0[1].y);
+    y[u] = (d1[0].x + d1[0].y) + (d1[1].x + d1[1].y);
+  }
+  if constexpr (SUB == 2) return make_float2(x[0] + x[1], y[0] + y[1]);
+  return make_float2(x[0], y[0]);
+}
+
+// add key times (ux, uy) and dot with the query: the thread's share of both outputs
+template <int SEG, int SUB>
+__device__ __forceinline__ float2 ds_update_dot(DsCols<SEG, SUB>& S, const float* qp, const float2 (&kr)[SUB][SEG / 2], float ux, float uy) {
+  const float2 ux2 = make_float2(ux, ux), uy2 = make_float2(uy, uy);
+  float x[SUB], y[SUB];
+#pragma unroll
+  for (int u = 0; u < SUB; ++u) {
+    float2 p0[2], p1[2];
+#pragma unroll
+    for (int a = 0; a < 2; ++a) p0[a] = p1[a] = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int i = 0; i < SEG / 2; i += 2) {
+      const float4 q4 = *reinterpret_cast<const float4*>(qp + u * (SEG + 4) + 2 * i);
+      const float2 qq[2] = {make_float2(q4.x, q4.y), make_float2(q4.z, q4.w)};
+#pragma unroll
+      for (int a = 0; a < 2; ++a) {
+        S.c0[u][i + a] = __ffma2_rn(kr[u][i + a], ux2, S.c0[u][i + a]);
+        S.c1[u][i + a] = __ffma2_rn(kr[u][i + a], uy2, S.c1[u][i + a]);
+        p0[a] = __ffma2_rn(S.c0[u][i + a], qq[a], p0[a]);
+        p1[a] = __ffma2_rn(S.c1[u][i + a], qq[a], p1[a]);
+      }
+    }
+    x[u] = (p0[0].x + p0[0].y) + (p0[1].x + p0[1].y);
+    y[u] = (p1[0].x + p1[0].y) + (p1[1].x + p1[1].y);
+  }
+  if constexpr (SUB == 2) return make_float2(x[0] + x[1], y[0] + y[1]);
+  return make_float2(x[0], y[0]);
+}
+
+// Prompts, dk padded to DKP = 32 ... 512.  LANES lanes share a column slot of two state columns: every q / k element read from shared
+// memory serves two columns.  The chain of a token (scale and dot with k, reduce over the lanes, update) is what bounds one CTA per SM, so
+// each link is kept short: 16 rows per lane at 128-row states (eight lanes) and two warps per scheduler that cover each other's latencies;
+// a reduction in which the two lanes of a pair first swap, so that one carries column j0 and the other j1 (1 + log2(lanes) exchanges for
+// two sums instead of 2 log2(lanes)); outputs whose exchanges run beside those of the next token; whole chunks as straight-line code.
+// 4 sequences of 512 tokens, 16 heads of 128 x 128, decays per channel: 0.42 us per token.  Where there are more CTAs than SMs the
+// instructions and the state traffic bound it instead, and four lanes of 32 rows, which exchange and read half as often, are faster
+// (delta_scan_launch).  q and k of CHUNK tokens are staged in shared memory with every segment padded by 16 bytes, so the lanes' 128-bit
+// reads fall into different banks.
+constexpr int ds_slots(int dkp) { return dkp <= 128 ? 32 : 4096 / dkp; }       // column slots per CTA, of two state columns each
+template <int DKP, int MODE, int LANES, int PER_SM>
+__global__ void __launch_bounds__(LANES * ds_slots(DKP), PER_SM)
 delta_scan_kernel(const float* __restrict__ qn, const float* __restrict__ kn, const float* __restrict__ v,
                   const float* __restrict__ beta, const float* __restrict__ decay, float* __restrict__ state,
                   const int32_t* __restrict__ cu, const int32_t* __restrict__ rows, const int32_t* __restrict__ lengths,
                   float* __restrict__ o, int H, int KH, int dk, int dv) {
-  constexpr int DS_LANES = ds_lanes(DKP), DS_SLOTS = ds_slots(DKP), DS_COLS = 2 * DS_SLOTS, DS_THREADS = ds_threads(DKP);
-  constexpr int SEG = DKP / DS_LANES;                            // state rows per lane
+  constexpr int SEGS = ds_segs(DKP), SUB = SEGS / LANES, SEG = DKP / SEGS;
+  constexpr int DS_SLOTS = ds_slots(DKP), DS_COLS = 2 * DS_SLOTS, DS_THREADS = LANES * DS_SLOTS;
   constexpr int CHUNK = DKP <= 128 ? 8 : 1024 / DKP;             // tokens staged at a time
-  constexpr int LDK = DKP + 4 * DS_LANES;                        // padded row of the staging buffers
+  // a thread's columns: half a CTA's width apart, or neighbours in one 8-byte access (few slots per warp: 4 x 64 tokens, 8 heads of
+  // 256 x 256: 54 -> 50 us; at 128 rows the same change costs 10 % of a short scan)
+  constexpr int NEXT = DKP <= 128 ? DS_SLOTS : 1, MUL = DKP <= 128 ? 1 : 2;
+  constexpr int LDK = DKP + 4 * SEGS;                            // padded row of the staging buffers
   constexpr int PF = CHUNK * DKP / DS_THREADS;                   // q / k elements each thread stages per chunk
   constexpr int PV = (CHUNK * DS_COLS + DS_THREADS - 1) / DS_THREADS;
   __shared__ __align__(16) float ks[2][CHUNK][LDK], qs[2][CHUNK][LDK];
   __shared__ __align__(16) float gc[MODE == 1 ? 2 : 1][MODE == 1 ? CHUNK : 1][MODE == 1 ? LDK : 4];     // per-channel decays
   __shared__ float vs[2][CHUNK][DS_COLS], gs[2][CHUNK], bs[2][CHUNK];
   const int e = blockIdx.x, h = blockIdx.y;
-  const int l = threadIdx.x & (DS_LANES - 1), slot = threadIdx.x / DS_LANES;
-  const int j0 = blockIdx.z * DS_COLS + slot, j1 = j0 + DS_SLOTS;                // this thread's two state columns
+  const int l = threadIdx.x & (LANES - 1), slot = threadIdx.x / LANES;
+  const int c0 = MUL * slot, j0 = blockIdx.z * DS_COLS + c0, j1 = j0 + NEXT;     // this thread's two state columns
+  const bool pairs = NEXT == 1 && (dv & 1) == 0 && (reinterpret_cast<uintptr_t>(state) & 7) == 0;
   const bool live0 = j0 < dv, live1 = j1 < dv, odd = (l & 1) != 0;
   const int t0 = cu[e], t1 = cu[e + 1];
   if (t1 <= t0) return;
   const int row = rows[e];
   const int kh = h / (H / KH);
-  float2 S0[SEG / 2], S1[SEG / 2];                               // rows 2 i (.x) and 2 i + 1 (.y) of columns j0 and j1
-  float* sp = state + (((int64_t)row * H + h) * dk + l * SEG) * dv;
+  const int r0 = l * SUB * SEG, l0 = l * SUB * (SEG + 4);        // first row of the lane, and where it lies in the staging buffers
+  DsCols<SEG, SUB> S;
+  float* sp = state + (((int64_t)row * H + h) * dk + r0) * dv;
   const bool fresh = lengths[row] == 0;                          // first token of a sequence: the state starts at zero
 #pragma unroll
-  for (int i = 0; i < SEG / 2; ++i) {
-    const bool in0 = !fresh && l * SEG + 2 * i < dk, in1 = !fresh && l * SEG + 2 * i + 1 < dk;
-    const float* s0 = sp + (int64_t)(2 * i) * dv;
-    S0[i] = make_float2(in0 && live0 ? s0[j0] : 0.f, in1 && live0 ? s0[dv + j0] : 0.f);
-    S1[i] = make_float2(in0 && live1 ? s0[j1] : 0.f, in1 && live1 ? s0[dv + j1] : 0.f);
-  }
+  for (int u = 0; u < SUB; ++u)
+#pragma unroll
+    for (int i = 0; i < SEG / 2; ++i) {
+      const int r = u * SEG + 2 * i;
+      const bool in0 = !fresh && r0 + r < dk, in1 = !fresh && r0 + r + 1 < dk;
+      const float* s0 = sp + (int64_t)r * dv;
+      if (NEXT == 1 && pairs) {
+        float2 a = make_float2(0.f, 0.f), b = a;
+        if (in0 && live0) a = *reinterpret_cast<const float2*>(s0 + j0);
+        if (in1 && live0) b = *reinterpret_cast<const float2*>(s0 + dv + j0);
+        S.c0[u][i] = make_float2(a.x, b.x);
+        S.c1[u][i] = make_float2(a.y, b.y);
+        continue;
+      }
+      S.c0[u][i] = make_float2(in0 && live0 ? s0[j0] : 0.f, in1 && live0 ? s0[dv + j0] : 0.f);
+      S.c1[u][i] = make_float2(in0 && live1 ? s0[j1] : 0.f, in1 && live1 ? s0[dv + j1] : 0.f);
+    }
   // The next chunk's inputs are fetched into registers while the current chunk runs out of shared memory, then parked in the
   // other buffer: the recurrence never waits for global memory.
   float pk[PF], pq[PF], pv[PV], pg = 0.f, pb = 0.f;
@@ -325,9 +410,9 @@ delta_scan_kernel(const float* __restrict__ qn, const float* __restrict__ kn, co
     if (threadIdx.x < CHUNK) { gs[buf][threadIdx.x] = pg; bs[buf][threadIdx.x] = pb; }
   };
   // a token's output leaves one token later: its exchanges run beside those of the next token's dot product
-  float px = 0.f, py = 0.f;
-  auto put = [&](int tok, float v) {
-    if (l < 2 && tok >= t0 && (odd ? live1 : live0)) o[((int64_t)tok * H + h) * dv + (odd ? j1 : j0)] = v;
+  float2 out = make_float2(0.f, 0.f);
+  auto put = [&](int tok, float val) {
+    if (l < 2 && tok >= t0 && (odd ? live1 : live0)) o[((int64_t)tok * H + h) * dv + (odd ? j1 : j0)] = val;
   };
   fetch(t0);
   park(0);
@@ -338,67 +423,19 @@ delta_scan_kernel(const float* __restrict__ qn, const float* __restrict__ kn, co
     const bool more = tc + CHUNK < t1;
     if (more) fetch(tc + CHUNK);
     auto step = [&](int tt) {
-      const float v1 = vs[buf][tt][slot + (odd ? DS_SLOTS : 0)];      // of the column this lane sums up
-      const float g = gs[buf][tt], b = bs[buf][tt];
-      const float2 g2 = make_float2(g, g);
-      const float* kp = &ks[buf][tt][l * (SEG + 4)];
-      const float* qp = &qs[buf][tt][l * (SEG + 4)];
-      // both reductions run as four interleaved partial sums per lane (rows i mod 4), combined in a fixed order and then across
-      // the lanes by exchanges: short dependency chains, and the same numbers whether a token arrives in a prompt or
-      // alone
-      float2 d0[2], d1[2];
-#pragma unroll
-      for (int a = 0; a < 2; ++a) d0[a] = d1[a] = make_float2(0.f, 0.f);
-      float2 kr[SEG / 2];                                        // the keys stay in registers for the update below
-#pragma unroll
-      for (int i = 0; i < SEG / 2; i += 2) {
-        const float4 k4 = *reinterpret_cast<const float4*>(kp + 2 * i);
-        kr[i] = make_float2(k4.x, k4.y);
-        kr[i + 1] = make_float2(k4.z, k4.w);
-        float2 gg[2] = {g2, g2};
-        if constexpr (MODE == 1) {
-          const float4 g4 = *reinterpret_cast<const float4*>(&gc[buf][tt][l * (SEG + 4) + 2 * i]);
-          gg[0] = make_float2(g4.x, g4.y), gg[1] = make_float2(g4.z, g4.w);
-        }
-#pragma unroll
-        for (int a = 0; a < 2; ++a) {
-          S0[i + a] = __fmul2_rn(S0[i + a], gg[a]);
-          S1[i + a] = __fmul2_rn(S1[i + a], gg[a]);
-          if constexpr (MODE != 2) {
-            d0[a] = __ffma2_rn(S0[i + a], kr[i + a], d0[a]);
-            d1[a] = __ffma2_rn(S1[i + a], kr[i + a], d1[a]);
-          }
-        }
-      }
+      const float v1 = vs[buf][tt][c0 + (odd ? NEXT : 0)];      // of the column this lane sums up
+      float2 kr[SUB][SEG / 2];                                   // the keys stay in registers for the update
+      const float2 d = ds_decay_dot<SEG, SUB, MODE>(S, &ks[buf][tt][l0], MODE == 1 ? &gc[buf][tt][l0] : nullptr, gs[buf][tt], kr);
       float u1 = v1;
       if constexpr (MODE != 2) {
-        const float dx = (d0[0].x + d0[0].y) + (d0[1].x + d0[1].y), dy = (d1[0].x + d1[0].y) + (d1[1].x + d1[1].y);
-        const float2 r = ds_reduce2<DS_LANES>(dx, dy, px, py, odd);
-        u1 = b * (v1 - r.x);
+        const float2 r = ds_reduce2<LANES>(d.x, d.y, out.x, out.y, odd);
+        u1 = bs[buf][tt] * (v1 - r.x);
         put(tc + tt - 1, r.y);
       } else {
-        put(tc + tt - 1, ds_reduce<DS_LANES>(px, py, odd));
+        put(tc + tt - 1, ds_reduce<LANES>(out.x, out.y, odd));
       }
       const float u_other = __shfl_xor_sync(0xffffffffu, u1, 1);
-      const float ux = odd ? u_other : u1, uy = odd ? u1 : u_other;
-      const float2 ux2 = make_float2(ux, ux), uy2 = make_float2(uy, uy);
-      float2 p0[2], p1[2];
-#pragma unroll
-      for (int a = 0; a < 2; ++a) p0[a] = p1[a] = make_float2(0.f, 0.f);
-#pragma unroll
-      for (int i = 0; i < SEG / 2; i += 2) {
-        const float4 q4 = *reinterpret_cast<const float4*>(qp + 2 * i);
-        const float2 qq[2] = {make_float2(q4.x, q4.y), make_float2(q4.z, q4.w)};
-#pragma unroll
-        for (int a = 0; a < 2; ++a) {
-          S0[i + a] = __ffma2_rn(kr[i + a], ux2, S0[i + a]);
-          S1[i + a] = __ffma2_rn(kr[i + a], uy2, S1[i + a]);
-          p0[a] = __ffma2_rn(S0[i + a], qq[a], p0[a]);
-          p1[a] = __ffma2_rn(S1[i + a], qq[a], p1[a]);
-        }
-      }
-      px = (p0[0].x + p0[0].y) + (p0[1].x + p0[1].y);
-      py = (p1[0].x + p1[0].y) + (p1[1].x + p1[1].y);
+      out = ds_update_dot<SEG, SUB>(S, &qs[buf][tt][l0], kr, odd ? u_other : u1, odd ? u1 : u_other);
     };
     if (nt == CHUNK) {                // straight-line: the next token's operands are read while this one's sums are exchanged
 #pragma unroll
@@ -409,17 +446,128 @@ delta_scan_kernel(const float* __restrict__ qn, const float* __restrict__ kn, co
     if (more) park(buf ^ 1);          // the other buffer was last read in the previous iteration, before its closing barrier
     __syncthreads();
   }
-  put(t1 - 1, ds_reduce<DS_LANES>(px, py, odd));
+  put(t1 - 1, ds_reduce<LANES>(out.x, out.y, odd));
+#pragma unroll
+  for (int u = 0; u < SUB; ++u)
+#pragma unroll
+    for (int i = 0; i < SEG / 2; ++i) {
+      const int r = u * SEG + 2 * i;
+      float* s0 = sp + (int64_t)r * dv;
+      if (NEXT == 1 && pairs) {
+        if (r0 + r < dk && live0) *reinterpret_cast<float2*>(s0 + j0) = make_float2(S.c0[u][i].x, S.c1[u][i].x);
+        if (r0 + r + 1 < dk && live0) *reinterpret_cast<float2*>(s0 + dv + j0) = make_float2(S.c0[u][i].y, S.c1[u][i].y);
+        continue;
+      }
+      if (r0 + r < dk) {
+        if (live0) s0[j0] = S.c0[u][i].x;
+        if (live1) s0[j1] = S.c1[u][i].x;
+      }
+      if (r0 + r + 1 < dk) {
+        if (live0) s0[dv + j0] = S.c0[u][i].y;
+        if (live1) s0[dv + j1] = S.c1[u][i].y;
+      }
+    }
+}
+
+// Decode steps (few tokens per entry).  Reading and writing the state is nearly all of it, so: small CTAs (16 KB of state at 128 rows,
+// in the registers of four warps), as many per SM as fit, so that some load while others compute and store; the token's inputs are asked
+// for first, so that they are staged while the state is on its way; neighbouring columns per thread, one 8-byte access where the
+// alignment allows.  64 entries of one token, us, beside the kernel above: 32 heads of 128 x 128 78 / 80 (3.4 TB/s), of 64 x 64 15 / 24, 8 heads
+// of 256 x 256 79 / 132.
+constexpr int DT_THREADS = 128;
+constexpr int dt_cols(int dkp) { return 2 * DT_THREADS / ds_segs(dkp); }
+template <int DKP, int MODE>
+__global__ void __launch_bounds__(DT_THREADS)
+delta_step_kernel(const float* __restrict__ qn, const float* __restrict__ kn, const float* __restrict__ v,
+                  const float* __restrict__ beta, const float* __restrict__ decay, float* __restrict__ state,
+                  const int32_t* __restrict__ cu, const int32_t* __restrict__ rows, const int32_t* __restrict__ lengths,
+                  float* __restrict__ o, int H, int KH, int dk, int dv) {
+  constexpr int LANES = ds_segs(DKP), SEG = DKP / LANES, LDK = DKP + 4 * LANES;
+  constexpr int PF = (DKP + DT_THREADS - 1) / DT_THREADS;
+  __shared__ __align__(16) float ks[LDK], qs[LDK], gc[MODE == 1 ? LDK : 4];
+  const int e = blockIdx.x, h = blockIdx.y;
+  const int l = threadIdx.x & (LANES - 1), slot = threadIdx.x / LANES;
+  const int j0 = blockIdx.z * dt_cols(DKP) + 2 * slot, j1 = j0 + 1;
+  const bool live0 = j0 < dv, live1 = j1 < dv, odd = (l & 1) != 0;
+  const bool pairs = (dv & 1) == 0 && (reinterpret_cast<uintptr_t>(state) & 7) == 0;
+  const int t0 = cu[e], t1 = cu[e + 1], row = rows[e];
+  if (t1 <= t0) return;
+  const int kh = h / (H / KH);
+  float pk[PF], pq[PF], pg[MODE == 1 ? PF : 1], pv, g = 1.f, b = 0.f;
+  auto fetch = [&](int t) {
+#pragma unroll
+    for (int r = 0; r < PF; ++r) {
+      const int i = threadIdx.x + r * DT_THREADS;
+      const bool ok = i < dk;
+      pk[r] = ok ? kn[((int64_t)t * KH + kh) * dk + i] : 0.f;
+      pq[r] = ok ? qn[((int64_t)t * KH + kh) * dk + i] : 0.f;
+      if constexpr (MODE == 1) pg[r] = ok ? decay[((int64_t)t * H + h) * dk + i] : 1.f;
+    }
+    const int j = odd ? j1 : j0;
+    pv = j < dv ? v[((int64_t)t * H + h) * dv + j] : 0.f;
+    if constexpr (MODE != 1) g = decay[(int64_t)t * H + h];
+    if constexpr (MODE != 2) b = beta[(int64_t)t * H + h];
+  };
+  fetch(t0);
+  const bool fresh = lengths[row] == 0;                          // first token of a sequence: the state starts at zero
+  float* sp = state + (((int64_t)row * H + h) * dk + l * SEG) * dv + j0;
+  DsCols<SEG, 1> S;
 #pragma unroll
   for (int i = 0; i < SEG / 2; ++i) {
-    float* s0 = sp + (int64_t)(2 * i) * dv;
-    if (l * SEG + 2 * i < dk) {
-      if (live0) s0[j0] = S0[i].x;
-      if (live1) s0[j1] = S1[i].x;
+    const bool in0 = l * SEG + 2 * i < dk, in1 = l * SEG + 2 * i + 1 < dk;
+    const float* s0 = sp + (int64_t)(2 * i) * dv;
+    float2 a = make_float2(0.f, 0.f), c = a;
+    if (pairs) {
+      if (in0 && live0) a = *reinterpret_cast<const float2*>(s0);
+      if (in1 && live0) c = *reinterpret_cast<const float2*>(s0 + dv);
+    } else {
+      if (in0 && live0) a.x = s0[0];
+      if (in0 && live1) a.y = s0[1];
+      if (in1 && live0) c.x = s0[dv];
+      if (in1 && live1) c.y = s0[dv + 1];
     }
-    if (l * SEG + 2 * i + 1 < dk) {
-      if (live0) s0[dv + j0] = S0[i].y;
-      if (live1) s0[dv + j1] = S1[i].y;
+    S.c0[0][i] = make_float2(a.x, c.x);
+    S.c1[0][i] = make_float2(a.y, c.y);
+  }
+  for (int t = t0; t < t1; ++t) {
+    if (t > t0) __syncthreads();                                 // the previous token's rows have been read
+#pragma unroll
+    for (int r = 0; r < PF; ++r) {
+      const int i = threadIdx.x + r * DT_THREADS;
+      if (i < DKP) {
+        ks[i + (i / SEG) * 4] = pk[r];
+        qs[i + (i / SEG) * 4] = pq[r];
+        if constexpr (MODE == 1) gc[i + (i / SEG) * 4] = pg[r];
+      }
+    }
+    const float v1 = pv, b1 = b, g1 = g;
+    __syncthreads();
+    if (t + 1 < t1) fetch(t + 1);
+    if (t == t0 && fresh) {
+#pragma unroll
+      for (int i = 0; i < SEG / 2; ++i) S.c0[0][i] = S.c1[0][i] = make_float2(0.f, 0.f);
+    }
+    float2 kr[1][SEG / 2];
+    const float2 d = ds_decay_dot<SEG, 1, MODE>(S, &ks[l * (SEG + 4)], &gc[MODE == 1 ? l * (SEG + 4) : 0], g1, kr);
+    float u1 = v1;
+    if constexpr (MODE != 2) u1 = b1 * (v1 - ds_reduce<LANES>(d.x, d.y, odd));
+    const float u_other = __shfl_xor_sync(0xffffffffu, u1, 1);
+    const float2 p = ds_update_dot<SEG, 1>(S, &qs[l * (SEG + 4)], kr, odd ? u_other : u1, odd ? u1 : u_other);
+    const float out = ds_reduce<LANES>(p.x, p.y, odd);
+    if (l < 2 && (odd ? live1 : live0)) o[((int64_t)t * H + h) * dv + (odd ? j1 : j0)] = out;
+  }
+#pragma unroll
+  for (int i = 0; i < SEG / 2; ++i) {
+    const bool in0 = l * SEG + 2 * i < dk, in1 = l * SEG + 2 * i + 1 < dk;
+    float* s0 = sp + (int64_t)(2 * i) * dv;
+    if (pairs) {
+      if (in0 && live0) *reinterpret_cast<float2*>(s0) = make_float2(S.c0[0][i].x, S.c1[0][i].x);
+      if (in1 && live0) *reinterpret_cast<float2*>(s0 + dv) = make_float2(S.c0[0][i].y, S.c1[0][i].y);
+    } else {
+      if (in0 && live0) s0[0] = S.c0[0][i].x;
+      if (in0 && live1) s0[1] = S.c1[0][i].x;
+      if (in1 && live0) s0[dv] = S.c0[0][i].y;
+      if (in1 && live1) s0[dv + 1] = S.c1[0][i].y;
     }
   }
 }
@@ -510,41 +658,57 @@ extern "C" int b200p_delta_conv_commit(const float* proj, int64_t ldp, float* co
   return B200P_OK;
 }
 
+// tokens: of all entries together; 0 if the caller does not say.
 template <int MODE>
-static void delta_scan_launch(dim3 grid, cudaStream_t st, const float* qn, const float* kn, const float* v, const float* beta,
+static void delta_scan_launch(int64_t tokens, int nb, cudaStream_t st, const float* qn, const float* kn, const float* v, const float* beta,
                               const float* decay, float* state, const int32_t* cu, const int32_t* rows, const int32_t* lengths,
                               float* o, int H, int KH, int dk, int dv) {
-  if (dk <= 32) delta_scan_kernel<32, MODE><<<grid, ds_threads(32), 0, st>>>(qn, kn, v, beta, decay, state, cu, rows, lengths, o, H, KH, dk, dv);
-  else if (dk <= 64) delta_scan_kernel<64, MODE><<<grid, ds_threads(64), 0, st>>>(qn, kn, v, beta, decay, state, cu, rows, lengths, o, H, KH, dk, dv);
-  else if (dk <= 128) {
-    // One CTA per SM may have 170 registers a thread and the shortest chain.  More CTAs than SMs are better run in pairs of 128
-    // registers (a few words spilled): a whole layer pass at 16 sequences of 16 tokens 139 -> 134 us with 16 heads and 193 -> 185 with
-    // 32, of 250 tokens 636 -> 583 and 1185 -> 1054.  The instances share their source and so the order of every sum.
-    if ((int64_t)grid.x * grid.y * grid.z > sm_count())
-      delta_scan_kernel<128, MODE, 2><<<grid, ds_threads(128), 0, st>>>(qn, kn, v, beta, decay, state, cu, rows, lengths, o, H, KH, dk, dv);
-    else
-      delta_scan_kernel<128, MODE><<<grid, ds_threads(128), 0, st>>>(qn, kn, v, beta, decay, state, cu, rows, lengths, o, H, KH, dk, dv);
-  }
-  else if (dk <= 256) delta_scan_kernel<256, MODE><<<grid, ds_threads(256), 0, st>>>(qn, kn, v, beta, decay, state, cu, rows, lengths, o, H, KH, dk, dv);
-  else delta_scan_kernel<512, MODE><<<grid, ds_threads(512), 0, st>>>(qn, kn, v, beta, decay, state, cu, rows, lengths, o, H, KH, dk, dv);
+#define DELTA_STEP(DKP)                                                                                                          \
+  delta_step_kernel<DKP, MODE><<<dim3((unsigned)nb, (unsigned)H, (unsigned)((dv + dt_cols(DKP) - 1) / dt_cols(DKP))), DT_THREADS, 0, st>>>( \
+      qn, kn, v, beta, decay, state, cu, rows, lengths, o, H, KH, dk, dv)
+#define DELTA_SCAN(DKP, LANES, PER_SM)                                                                                           \
+  delta_scan_kernel<DKP, MODE, LANES, PER_SM>                                                                                     \
+      <<<dim3((unsigned)nb, (unsigned)H, (unsigned)((dv + 2 * ds_slots(DKP) - 1) / (2 * ds_slots(DKP)))), LANES * ds_slots(DKP), 0, st>>>( \
+          qn, kn, v, beta, decay, state, cu, rows, lengths, o, H, KH, dk, dv)
+  // The step kernel for decode steps, and for as many tokens per entry as it keeps up with the scan (us, step / scan): 128 x 128, 16
+  // entries of 1 / 2 / 4 tokens, 32 heads, 21.7 / 23.1, 27.1 / 25.3, 32.0 / 29.2; 64 x 64, 32 heads, of 2 / 4 / 8, 6.8 / 8.8, 7.9 / 9.6,
+  // 10.2 / 11.4, but with 16 heads 4.3 / 4.6, 5.1 / 5.0, 7.3 / 6.4; 32 x 64, 16 heads, of 2 / 4, 3.4 / 3.5, 4.2 / 3.9; 256 x 256, 8 heads,
+  // 4 entries of 16 / 64, 20 / 20, 58 / 50.
+  // The plain accumulation of keys above 128 takes it at any length (16 x 250 tokens of 256 x 256: 407 / 678; 4 x 512: 315 / 309).
+  const int most = dk > 128 ? 8 : dk > 64 ? 1 : dk > 32 ? 4 : 2;
+  const bool few = (tokens > 0 && tokens <= most * (int64_t)nb) || (MODE == 2 && dk > 128);
+  // 128 rows: one CTA per SM takes eight lanes per column and the shortest chain (4 x 512 tokens, 16 heads, decays per channel / per
+  // head: 220 / 193 us, the former four-lane kernel 280 / 206); more CTAs than SMs take four (32 heads 379 / 346 -> 356 / 317; 16 x 250
+  // tokens 672 / 594 -> 637 / 544).
+  const bool crowded = (int64_t)nb * H * ((dv + 63) / 64) > sm_count();
+  if (dk > 256) { if (few) DELTA_STEP(512); else DELTA_SCAN(512, 16, 1); }
+  else if (dk > 128) { if (few) DELTA_STEP(256); else DELTA_SCAN(256, 8, 1); }
+  else if (dk > 64) { if (few) DELTA_STEP(128); else if (crowded) DELTA_SCAN(128, 4, 2); else DELTA_SCAN(128, 8, 1); }
+  else if (dk > 32) { if (few) DELTA_STEP(64); else DELTA_SCAN(64, 4, 1); }
+  else { if (few) DELTA_STEP(32); else DELTA_SCAN(32, 4, 1); }
+#undef DELTA_STEP
+#undef DELTA_SCAN
 }
 
-extern "C" int b200p_delta_scan(const float* qn, const float* kn, const float* v, const float* beta, const float* decay,
-                                float* state, const int32_t* cu, const int32_t* rows, const int32_t* lengths, float* o, int nb,
-                                int H, int KH, int dk, int dv, int mode, void* stream) {
+extern "C" int b200p_delta_scan_tokens(const float* qn, const float* kn, const float* v, const float* beta, const float* decay,
+                                       float* state, const int32_t* cu, const int32_t* rows, const int32_t* lengths, float* o, int64_t tokens,
+                                       int nb, int H, int KH, int dk, int dv, int mode, void* stream) {
   B200P_REQUIRE(qn && kn && v && decay && state && cu && rows && lengths && o, B200P_ERR_ARG, "null pointer");
   B200P_REQUIRE(mode >= B200P_SCAN_DELTA && mode <= B200P_SCAN_ACCUMULATE, B200P_ERR_ARG, "unknown scan mode %d", mode);
   B200P_REQUIRE(beta || mode == B200P_SCAN_ACCUMULATE, B200P_ERR_ARG, "the delta rule needs beta");
   B200P_REQUIRE(nb > 0 && H > 0 && KH > 0 && H % KH == 0 && H < 65536 && dk > 0 && dv > 0, B200P_ERR_ARG, "bad head geometry");
   B200P_REQUIRE(dk <= 512, B200P_ERR_ARG, "key size %d > 512 is not built", dk);
-  const int dkp = dk <= 32 ? 32 : dk <= 64 ? 64 : dk <= 128 ? 128 : dk <= 256 ? 256 : 512, cols = ds_cols(dkp);
-  dim3 grid((unsigned)nb, (unsigned)H, (unsigned)((dv + cols - 1) / cols));
   cudaStream_t st = (cudaStream_t)stream;
-  if (mode == B200P_SCAN_DELTA) delta_scan_launch<0>(grid, st, qn, kn, v, beta, decay, state, cu, rows, lengths, o, H, KH, dk, dv);
-  else if (mode == B200P_SCAN_DELTA_CHANNEL) delta_scan_launch<1>(grid, st, qn, kn, v, beta, decay, state, cu, rows, lengths, o, H, KH, dk, dv);
-  else delta_scan_launch<2>(grid, st, qn, kn, v, beta, decay, state, cu, rows, lengths, o, H, KH, dk, dv);
+  const auto launch = mode == B200P_SCAN_DELTA ? delta_scan_launch<0> : mode == B200P_SCAN_DELTA_CHANNEL ? delta_scan_launch<1> : delta_scan_launch<2>;
+  launch(tokens, nb, st, qn, kn, v, beta, decay, state, cu, rows, lengths, o, H, KH, dk, dv);
   B200P_LAUNCH_CHECK("delta_scan_kernel");
   return B200P_OK;
+}
+
+extern "C" int b200p_delta_scan(const float* qn, const float* kn, const float* v, const float* beta, const float* decay,
+                                float* state, const int32_t* cu, const int32_t* rows, const int32_t* lengths, float* o, int nb,
+                                int H, int KH, int dk, int dv, int mode, void* stream) {
+  return b200p_delta_scan_tokens(qn, kn, v, beta, decay, state, cu, rows, lengths, o, 0, nb, H, KH, dk, dv, mode, stream);
 }
 
 extern "C" int b200p_linear_attn_prep(const float* proj, int64_t ldp, const float* head_decay, float* q, float* k, float* v,

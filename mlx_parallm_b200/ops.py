@@ -361,8 +361,8 @@ def delta_scan(qn, kn, v, beta, decay, state, cu, rows, lengths, o, nb, H, KH, d
     the plain decayed accumulation without the delta correction)."""
     _dev(qn, kn, v, beta, decay, state, cu, rows, lengths, o)
     assert state.dtype == torch.float32 and state.is_contiguous()
-    _call("b200p_delta_scan", lambda: lib().b200p_delta_scan(_p(qn), _p(kn), _p(v), _p(beta), _p(decay), _p(state), _p(cu), _p(rows),
-                                                            _p(lengths), _p(o), nb, H, KH, dk, dv, int(mode), _stream()))
+    _call("b200p_delta_scan", lambda: lib().b200p_delta_scan_tokens(_p(qn), _p(kn), _p(v), _p(beta), _p(decay), _p(state), _p(cu), _p(rows),
+                                                                   _p(lengths), _p(o), qn.shape[0], nb, H, KH, dk, dv, int(mode), _stream()))
 
 
 def delta_out(o, gate, norm_w, out, H, dv, eps, gate_act=_lib.GATE_SILU, out_scale=1.0):

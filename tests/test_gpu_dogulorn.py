@@ -647,6 +647,33 @@ def test_delta_scan_of_more_ctas_than_sms_equals_its_parts(mode, dk):
     assert torch.equal(o[0], o[1]) and torch.equal(states[0], states[1])
 
 
+@pytest.mark.parametrize("mode", [0, 1, 2])
+@pytest.mark.parametrize("dk,dv,H,KH,shift", [(16, 31, 2, 1, 0), (32, 64, 4, 4, 1), (50, 66, 2, 2, 0), (64, 64, 3, 1, 0), (100, 96, 4, 2, 0), (128, 128, 20, 4, 1)])
+def test_delta_scan_of_decode_steps_equals_the_scan_of_prompts(mode, dk, dv, H, KH, shift):
+    """Told that an entry has few tokens, the call runs another kernel than it does for prompts: the same bits, whatever the entries hold in
+    fact (none, one, a whole prompt), states of odd widths and at odd addresses (shift), carried and fresh ones."""
+    from mlx_parallm_b200 import _lib
+    lens, nb = [1, 0, 1, 19, 8, 1], 6
+    g, M = torch.Generator(device="cuda").manual_seed(dk + mode), sum(lens)
+    rnd = lambda *sh: torch.randn(*sh, generator=g, device="cuda")
+    qn, kn, v = rnd(M, KH * dk) / dk, torch.nn.functional.normalize(rnd(M, KH, dk), dim=-1).reshape(M, -1).contiguous(), rnd(M, H * dv)
+    beta, decay = torch.rand(M, H, generator=g, device="cuda"), 0.5 + 0.5 * torch.rand(M, H * (dk if mode == 1 else 1), generator=g, device="cuda")
+    state0 = rnd(nb + 1, H, dk, dv) * 0.3
+    i32 = dict(dtype=torch.int32, device="cuda")
+    cu, rows = torch.tensor([0] + torch.tensor(lens).cumsum(0).tolist(), **i32), torch.tensor([4, 6, 1, 0, 5, 2], **i32)
+    lengths, got = torch.tensor([3, 7, 0, 2, 5, 0, 1], **i32), []
+    for tokens in (0, 1, M):
+        state = torch.empty(state0.numel() + 2, device="cuda")[shift:shift + state0.numel()]
+        state.copy_(state0.reshape(-1))
+        o = torch.zeros(M, H * dv, device="cuda")
+        p = lambda t: t.data_ptr()
+        _lib.check(_lib.lib().b200p_delta_scan_tokens(p(qn), p(kn), p(v), p(beta), p(decay), p(state), p(cu), p(rows), p(lengths), p(o), tokens, nb, H, KH,
+                                                      dk, dv, mode, torch.cuda.current_stream().cuda_stream))
+        got.append((o, state.clone()))
+    assert all(torch.equal(got[0][i], other[i]) for other in got[1:] for i in (0, 1))
+    assert torch.equal(got[0][1].view_as(state0)[3], state0[3])             # a row that no entry names is not touched
+
+
 @pytest.mark.parametrize("lens,H,KH,dv,channel", [([257], 1, 1, 128, False), ([1, 300, 2], 3, 1, 256, True), ([130, 3, 129, 9], 4, 2, 128, True)])
 def test_delta_prep_rows_equals_the_per_token_kernel(lens, H, KH, dv, channel):
     """Prompts of more than 256 tokens with 128-channel heads (one warp per 128 channels and 8 tokens) against the per-token kernel fed
