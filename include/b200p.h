@@ -123,7 +123,7 @@ int b200p_wait_probe(void* stream);
 int b200p_qmv_fault(void);
 /* the same for the wide tiles of more than 128 tokens (csrc/qmm_wide.cu): 0, or 1 + the role that gave up */
 int b200p_qmm_wide_fault(void);
-/* smallest M routed to the tensor path in auto mode (default 1: measured, scripts/qmm_sweep.py, profiles/r1_run11_qmm_sweep_gemv_vs_tensor.txt) */
+/* smallest M routed to the tensor path in auto mode (default 1: measured) */
 int b200p_qmm_set_min_tensor_m(int m);
 
 /* mx.fast.rms_norm(x, w, eps)                                      [nn.RMSNorm: models/llama.py:187,

@@ -51,12 +51,12 @@ static int g_qmm_path = 0;   // 0 auto, 1 CUDA-core gemv, 2 tcgen05 tiles, 3 mma
 // pipeline-free mma.sync GEMM (qmm_mma.cu) for the accumulate epilogue above the GEMV's rows: matrices up to this many weights
 // (q|k|v 25 M and o_proj 17 M of Llama-3-8B, every tensor-parallel shard; down_proj 59 M and gate|up stay on the tile kernels)
 static long long g_mma_max_weights = [] { const char* e = getenv("B200P_MMA_MAX_WEIGHTS"); return e ? atoll(e) : (1ll << 25); }();
-// ... and up to this many rows: measured against the tile kernels (profiles/r2_run35_small_gemm_paths.txt) it wins at 8 and 16
+// ... and up to this many rows: measured against the tile kernels it wins at 8 and 16
 // rows (q|k|v 6.2 vs 7.2 us, o_proj 4.3 vs 5.7, TP=8 shards 2.6-4.1 vs 3.8-5.3), ties at 32 and loses at 64, where it is bound
 // by the mma.sync rate (q|k|v 14.6 vs 8.9 us)
 static int g_gemv_silu_max_m = [] { const char* e = getenv("B200P_GEMV_SILU_MAX_M"); return e ? atoi(e) : 0; }();
 static int g_mma_max_m = [] { const char* e = getenv("B200P_MMA_MAX_M"); return e ? atoi(e) : 16; }();
-// Auto rule for the mma.sync GEMV, from the measured three-way sweep (profiles/r1_run12_qmm_sweep_three_paths.txt, us per
+// Auto rule for the mma.sync GEMV, from the measured three-way sweep (us per
 // launch in a CUDA graph): it wins where the tile kernel's fixed cost dominates -- M <= 4 and matrices up to ~32 M weights
 // (q|k|v 6.4 vs 8.4 us, o_proj 5.2 vs 6.5 us at M = 1) -- and loses on the big streams (gate|up 23.9 vs 22.4 us) and as M
 // grows (its activation loads are per 16-row warp, not shared through shared memory).  The CUDA-core GEMV loses everywhere.
@@ -148,10 +148,10 @@ extern "C" int b200p_qmm(const void* x, const uint32_t* w, const void* scales, c
   const bool mma_ok = qmv_mma_supported(M, N, K, group_size, bits, dtype, epilogue) && aligned(w, 32) &&
                       (epilogue == B200P_EPI_SILU_MUL ? aligned(y, 2) : (aligned(y, 4) && !(flags & B200P_Y_PERM8)));
   if (g_qmm_path == 3) B200P_REQUIRE(mma_ok, B200P_ERR_ARG, "mma.sync GEMV forced but unsupported for this call");
-  // up to two rows the GEMV also wins on matrices of twice that size (down_proj 4096 x 14336: 12.8 vs 14.1 us at M = 1,
-  // profiles/r1_run34_gemv_splits.txt); gate|up (117 M weights) stays on the tile kernel
+  // up to two rows the GEMV also wins on matrices of twice that size (down_proj 4096 x 14336: 12.8 vs 14.1 us at M = 1);
+  // gate|up (117 M weights) stays on the tile kernel
   // gate|up with the fused silu(gate) * up epilogue through the GEMV (rows paired gate / up, no K split): up to
-  // B200P_GEMV_SILU_MAX_M rows, any size; 0 = never (the default: see profiles/r2_run39_*)
+  // B200P_GEMV_SILU_MAX_M rows, any size; 0 = never (the default)
   if (mma_ok && epilogue == B200P_EPI_SILU_MUL && g_qmm_path == 0 && M <= g_gemv_silu_max_m)
     return qmv_mma_launch(x, w, scales, biases, y, M, N, K, ldx, ldy, dtype, epilogue, flags, st);
   if (mma_ok && (g_qmm_path == 3 || (g_qmm_path == 0 && epilogue != B200P_EPI_SILU_MUL && M <= g_gemv_max_m &&

@@ -328,10 +328,10 @@ extern "C" int b200p_rmsnorm(const float* x, const void* w, void* y, int64_t M, 
                 "rmsnorm needs 16-byte aligned rows (H %% 4 == 0)");
   if (M == 0) return B200P_OK;
   // Which norm.  The one-pass cluster form (16-bit rows of 2048 * C elements, C in {1, 2, 4, 8}, at most one CTA per SM) is an
-  // "early" kernel and wins at every row count (B=1 T=8192 2.29 -> 2.22 ms, B=8 3.46 -> 3.41, B=64 T=256 2.88 -> 2.86:
-  // profiles/r2_run33_*, r2_run37_*).  Where it does not apply, the two-pass early kernel pays from 16 rows on (the next kernel
+  // "early" kernel and wins at every row count (B=1 T=8192 2.29 -> 2.22 ms, B=8 3.46 -> 3.41, B=64 T=256 2.88 -> 2.86).
+  // Where it does not apply, the two-pass early kernel pays from 16 rows on (the next kernel
   // is then a tile GEMM that streams weights while it waits: B=64 T=256 2.91 -> 2.87 ms) and loses below (a 128-thread CTA is
-  // the slower norm and the GEMV after it gains nothing: B=1 T=8192 2.38 -> 2.43 ms, profiles/r2_run29_*).
+  // the slower norm and the GEMV after it gains nothing: B=1 T=8192 2.38 -> 2.43 ms).
   static const int early_env = [] { const char* e = getenv("B200P_RMS_EARLY"); return e ? atoi(e) : -1; }();
   static const int cluster_env = [] { const char* e = getenv("B200P_RMS_CLUSTER"); return e ? atoi(e) : 1; }();
   const int64_t C = H / 2048;
@@ -447,7 +447,7 @@ __global__ void rope_kv_append_kernel(TIN* __restrict__ qkv, T* __restrict__ q_o
 // position load and its four 8-byte value loads at once and finishes after one round trip; the per-head RMSNorm of Qwen3 is a
 // warp reduction (no block barrier); 8-byte (fp32 input) / 4-byte (16-bit) accesses per lane, whole lines per warp.
 // (A warp looping over 6 heads to reuse its sincos was tried first: 6 dependent round trips, slower -- 18 us cold in ncu
-// against 14.6 us for the generic kernel above, profiles/r1_run37_small_kernels_ncu.txt.)
+// against 14.6 us for the generic kernel above.)
 template <typename T, typename TIN>
 __global__ void __launch_bounds__(256)
 rope_kv_append_d128_kernel(TIN* __restrict__ qkv, T* __restrict__ q_out, T* __restrict__ kc, T* __restrict__ vc,

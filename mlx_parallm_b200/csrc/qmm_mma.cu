@@ -11,8 +11,8 @@
 // rows is the B operand: 8 n-tiles of 8 tokens would be 32 KB of activations per warp and step from L2, so the CTA's 8 warps
 // share ONE [8*NT tokens x 256 k] tile per step in shared memory (cp.async, double-buffered, 16-byte chunks XOR-swizzled so
 // that the fragment loads of a quarter warp hit 8 different bank groups).
-// Legacy mma.sync runs at 1020 MAC/cycle/SM on sm_100a (scripts/probe_hmma.cu, profiles/r2_run34_probe_hmma.txt): 128 weights
-// per cycle and SM at 8 rows, 16 at 64 rows.  Measured against the tile kernels (profiles/r2_run35_small_gemm_paths.txt, us per
+// Legacy mma.sync runs at 1020 MAC/cycle/SM on sm_100a (measured): 128 weights
+// per cycle and SM at 8 rows, 16 at 64 rows.  Measured against the tile kernels (us per
 // launch in a CUDA graph over weight copies larger than L2): q|k|v 6144 x 4096 6.2 vs 7.2 at 8 rows, 6.9 vs 7.3 at 16, 9.0 vs
 // 7.9 at 32, 14.6 vs 8.9 at 64 (640 MAC/cycle/SM: bound by the mma.sync rate and the fragment loads); o_proj 4.3 vs 5.7 at 8
 // rows; TP=8 shards 2.6-4.1 vs 3.8-5.3.  The auto rule in c_api.cu therefore gives it 5..16 rows on matrices up to 32 M weights

@@ -11,7 +11,7 @@
 //   * every segment (whole tile or not) leaves through shared memory and ONE cp.reduce.async.bulk.tensor (.add.f32) per
 //     [16 tokens x 128 rows] staging tile: partial tiles of different CTAs are summed by the L2 atomic units, nothing is
 //     waited for, there is no workspace and no tail.  Sums are NOT taken in a fixed order (fp32 adds of <= 148 partials).
-// Measured against the whole-tile kernel's K split through the workspace (profiles/r2_run11_*): o_proj M=64 8.5 vs 13.4 us,
+// Measured against the whole-tile kernel's K split through the workspace: o_proj M=64 8.5 vs 13.4 us,
 // down_proj 16.7 vs 20.3 us.  The model also sends q|k|v through this epilogue at decode sizes (fp32 accumulator that
 // rope_kv_append rounds and re-zeroes).
 //

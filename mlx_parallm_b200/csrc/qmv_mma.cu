@@ -4,7 +4,7 @@
 //
 // Why this shape of kernel.  At M <= 16 the step is a pure weight stream (AI = 3.56*M flop/B).  The ALU budget at HBM speed is
 // ~2.8 lane-ops per weight (148 SMs x 128 lanes x 1.9 GHz / 13e12 weights/s); a CUDA-core GEMV needs >= 2 ops to unpack a
-// code to fp32 plus M FMAs (the old qmv kernel: 1.4-2.2 TB/s at M = 1, collapsing with M -- profiles/r1_run11_*), while the
+// code to fp32 plus M FMAs (the old qmv kernel: 1.4-2.2 TB/s at M = 1, collapsing with M), while the
 // dequant itself costs 1.5 ops per weight when done on packed half2 (LOP3 + exponent magic + one HFMA2 for q*s+b).  So the
 // dot products go to the tensor cores -- but with NO shared-memory / TMEM / mbarrier pipeline in front of them: every warp
 // streams its own 16 weight rows global -> registers with 128-bit no-allocate loads, dequantises in registers and feeds
@@ -188,8 +188,7 @@ static int launch_qmv_mma(const void* x, const uint32_t* w, const void* s, const
   // Split-K so that every SM holds ~16 warps, but never a grid that spills a few CTAs into a second wave (4096 x 14336 at ten
   // splits was 640 CTAs on 592 slots: 1.08 waves, 30 % slower than 8 splits in one wave): among the split counts pick the
   // one with the lowest waves x (steps per warp + ~1.5 steps of fixed latency); ties go to fewer splits (fewer red.adds).  Plain stores cannot
-  // be split.  (More weights in flight per lane instead of more warps was tried and is slower:
-  // profiles/r1_run33_gemv_prefetch_depth_experiment.txt.)
+  // be split.  (More weights in flight per lane instead of more warps was tried and is slower.)
   int64_t splits = 1;
   if (epi == B200P_EPI_ADD_RESIDUAL) {
     const int64_t capacity = (int64_t)sm_count() * 4;            // resident CTAs: 4 per SM at 121 registers x 128 threads
@@ -201,7 +200,7 @@ static int launch_qmv_mma(const void* x, const uint32_t* w, const void* s, const
       const int64_t ctas = (row_groups * sp_eff + QM_WARPS - 1) / QM_WARPS;
       // a partly filled wave after the first costs its fill fraction, but never less than half a wave (measured: 28672 x 4096 runs
       // 24.1 us as 1.51 waves of 8 steps against 25.5 us as 0.76 wave of 16; 4096 x 14336 16.9 us as 1.08 waves of 6 steps
-      // against 12.9 us as 0.86 wave of 7 -- profiles/r1_run34_gemv_splits.txt)
+      // against 12.9 us as 0.86 wave of 7)
       const int64_t full = ctas / capacity;
       const double frac = (double)(ctas - full * capacity) / (double)capacity;
       const double waves = full == 0 ? 1.0 : (double)full + (frac > 0.0 ? (frac > 0.5 ? frac : 0.5) : 0.0);

@@ -145,7 +145,7 @@ __device__ __forceinline__ void umma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, ui
 //   (16-byte units: 32 bytes = 16 k per MMA).  acc = 0 clears D on the first slice of each block.
 // The two blocks' MMAs ALTERNATE: consecutive tcgen05.mma into the SAME accumulator are a dependent chain (one every
 // 64 cycles at M=128, K=16 whatever N <= 128), two independent accumulators interleaved retire one MMA every 32 cycles at
-// N=64 = the full rate of the pipe (scripts/probe_mma2.cu, profiles/r2_run22_probe_mma2.txt); four in a row per block, the
+// N=64 = the full rate of the pipe (measured); four in a row per block, the
 // order used before, averaged 51.
 __device__ __forceinline__ void umma_kblock_f16_ts(uint32_t d0, uint32_t d1, uint32_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
   asm volatile(
@@ -180,7 +180,7 @@ __device__ __forceinline__ void umma_kblock_f16_ts(uint32_t d0, uint32_t d1, uin
 // The four MMAs of ONE block of a k-block (A slices a, a+8, a+16, a+24; B descriptors b, b+2, b+4, b+6).  The GEMM kernels run
 // TWO issuing warps, one per 128-row block: a single thread issues one tcgen05.mma (M=128, K=16, N <= 64) every 51-64 cycles
 // whatever the order of its accumulators, two threads of different warps together retire one every 32 cycles = the full rate of
-// the pipe at N=64 (scripts/probe_mma2.cu, profiles/r2_run22_probe_mma2.txt).
+// the pipe at N=64 (measured).
 __device__ __forceinline__ void umma_half_kblock_f16_ts(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
   asm volatile(
       "{\n"

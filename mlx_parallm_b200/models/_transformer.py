@@ -34,13 +34,13 @@ from .base import BatchedKVCache, PagedKVCache
 MAX_TOKENS_PER_FORWARD = 8192     # chunk size (B*L) of one prefill pass through the layers
 # Up to this many rows the fused q|k|v projection accumulates in an fp32 buffer through the stream-K kernel (csrc/qmm_sk.cu:
 # partial tiles summed by TMA reduce-adds, no tail; rope_kv_append rounds to the storage type and re-zeroes the buffer).
-# q|k|v has 24 output tiles for 148 SMs, so it must split K; measured at 64 rows (profiles/r2_run11_*): 16.8 us through the
+# q|k|v has 24 output tiles for 148 SMs, so it must split K; measured at 64 rows: 16.8 us through the
 # whole-tile kernel's workspace split against 8-10 us this way.  Above it (prefill) whole 16-bit tiles are stored directly.
 ACC32_MAX_ROWS = 128
 # gate|up: one GPU's full matrix (117 M weights on Llama-3-8B) goes through the whole-tile kernel with the fused silu*mul
 # epilogue (27.9 us at 64 rows; stream-K into fp32 + the silu_mul kernel: 22.7 + 5.9 us, and 22 MB of fp32 round trip).  A
 # tensor-parallel SHARD of it has too few rows to fill 148 SMs with whole tiles and is latency-bound there, so up to this
-# many weights it takes the stream-K accumulate path + silu_mul (profiles/r2_run17_*, r2_run18_*, 64 rows: TP=2 shard
+# many weights it takes the stream-K accumulate path + silu_mul (64 rows: TP=2 shard
 # 14.9 + 4.2 vs 23.5 us, TP=4 10.8 + 3.5 vs 17.3, TP=8 7.4 + 3.1 vs 13.7).
 GATE_UP_ACC32_MAX_WEIGHTS = 100 * 1000 * 1000
 USE_PERM8 = True                  # 4-bit 16-bit models: GEMM inputs in the PERM8 column order (include/b200p.h)

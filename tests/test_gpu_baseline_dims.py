@@ -101,7 +101,7 @@ def test_greedy_32_tokens_on_128_sequences(pair):
     name, dtype, cfg, om, gm = pair
     if (name, dtype) not in GREEDY_DEFAULT and os.environ.get("B200P_FULL_PARITY", "0") != "1":
         pytest.skip("the oracle needs 1.5-4.5 min for this slice (128 x 32 full-vocabulary steps on the host cores): run with "
-                    "B200P_FULL_PARITY=1; the last full run is profiles/r2_baseline_dims_parity.txt")
+                    "B200P_FULL_PARITY=1; a full run is kept as profiles/r2_baseline_dims_parity.txt")
     B, L, S = 128, 16, 32
     ids = np.random.default_rng(9).integers(0, cfg["vocab_size"], (B, L)).astype(np.int64)
     exp, exp_logits = [], []
