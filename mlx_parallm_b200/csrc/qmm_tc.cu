@@ -85,47 +85,6 @@ constexpr int SB_SLOT_BYTES = 4 * SB_TILE_BYTES; // block 0 scales, block 0 bias
 constexpr int MAX_STAGES = 8;                    // weight ring stages / X ring slots (upper bounds)
 constexpr int X_RING_BYTES = 64 * 1024;
 constexpr int EPI_TOK = 8;                       // tokens per epilogue step = work item of the shared split-tile reduction
-// Profiling build only (-DB200P_TC_DEBUG=mask): 1 no X loads, 2 no MMA issue, 4 no epilogue, 8 no A stores, 32 no
-// scale/bias loads.  The shipped kernel is compiled with 0: every branch below folds away.
-#ifndef B200P_TC_DEBUG
-#define B200P_TC_DEBUG 0
-#endif
-constexpr int kDebug = B200P_TC_DEBUG;
-// Profiling build only (-DB200P_TC_TIMING=1): CTA 0 accumulates the cycles each role spends in each barrier wait into
-// g_tc_timing (read back with b200p_debug_tc_timing); slots are listed in scripts/tc_timing.py.
-#ifndef B200P_TC_TIMING
-#define B200P_TC_TIMING 0
-#endif
-#if B200P_TC_TIMING
-__device__ unsigned long long g_tc_timing[32];
-#define TWAIT(slot, bar, par)                                   \
-  do {                                                          \
-    const long long t0_ = clock64();                            \
-    mbar_wait(bar, par);                                        \
-    tacc[slot] += (unsigned long long)(clock64() - t0_);        \
-  } while (0)
-#define TDECL unsigned long long tacc[4] = {0ull, 0ull, 0ull, 0ull}; const long long tstart_ = clock64()
-// section timers of the dequant warps (slots 16..19: LDS fetch, math, TMEM store + wait::st, fence + publish)
-#define TSEC_DECL unsigned long long tsec[4] = {0ull, 0ull, 0ull, 0ull}; long long tmark_ = 0
-#define TSEC_BEGIN() tmark_ = clock64()
-#define TSEC_END(i) do { const long long n_ = clock64(); tsec[i] += (unsigned long long)(n_ - tmark_); tmark_ = n_; } while (0)
-#define TSEC_FLUSH(cond) do { if (blockIdx.x == 0 && (cond)) for (int i_ = 0; i_ < 4; ++i_) g_tc_timing[16 + i_] = tsec[i_]; } while (0)
-#define TFLUSH(base, n, cond)                                                                                   \
-  do {                                                                                                          \
-    if (blockIdx.x == 0 && (cond)) {                                                                            \
-      for (int i_ = 0; i_ < (n); ++i_) g_tc_timing[(base) + i_] = tacc[i_];                                     \
-      g_tc_timing[(base) + (n)] = (unsigned long long)(clock64() - tstart_);                                    \
-    }                                                                                                           \
-  } while (0)
-#else
-#define TWAIT(slot, bar, par) mbar_wait(bar, par)
-#define TDECL
-#define TFLUSH(base, n, cond)
-#define TSEC_DECL
-#define TSEC_BEGIN()
-#define TSEC_END(i)
-#define TSEC_FLUSH(cond)
-#endif
 
 struct TcParams {
   const void* scales;
@@ -315,7 +274,6 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
     // Weights and scale/bias tiles do not depend on the previous kernel: no griddepcontrol.wait here, so under
     // programmatic dependent launch the HBM stream of this kernel starts while the previous kernel drains.
     int si = 0, ph = 0, sbi = 0, sbph = 0;
-    TDECL;
     for (int item = cta; item < p.items; item += G) {
      const TcSeg sg = seg_of(p, item);
      const int pair = sg.tile / p.tiles_m;
@@ -324,24 +282,20 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
      for (int i = 0; i < sg.ns; ++i) {
       const int st = seg_stage(sg, i);
       if (p.sb_tma && (i == 0 || st == sg.s0 || (st % SPG) == 0)) {     // a new group of 8 k-blocks starts with this stage
-        TWAIT(1, sb_empty(sbi), sbph ^ 1);
+        mbar_wait(sb_empty(sbi), sbph ^ 1);
         if (elect_one()) {
           const uint32_t sdst = sb_ring + sbi * SB_SLOT_BYTES;
           const int kb0 = (st / SPG) * 8;
-          if (kDebug & 32) {
-            mbar_arrive(sb_full(sbi));
-          } else {
-            mbar_arrive_expect_tx(sb_full(sbi), (uint32_t)(4 * p.R * 16));
-            tma_load_2d(sdst, &tm_s, kb0, rowA0, sb_full(sbi));
-            tma_load_2d(sdst + SB_TILE_BYTES, &tm_b, kb0, rowA0, sb_full(sbi));
-            tma_load_2d(sdst + 2 * SB_TILE_BYTES, &tm_s, kb0, rowB0, sb_full(sbi));
-            tma_load_2d(sdst + 3 * SB_TILE_BYTES, &tm_b, kb0, rowB0, sb_full(sbi));
-          }
+          mbar_arrive_expect_tx(sb_full(sbi), (uint32_t)(4 * p.R * 16));
+          tma_load_2d(sdst, &tm_s, kb0, rowA0, sb_full(sbi));
+          tma_load_2d(sdst + SB_TILE_BYTES, &tm_b, kb0, rowA0, sb_full(sbi));
+          tma_load_2d(sdst + 2 * SB_TILE_BYTES, &tm_s, kb0, rowB0, sb_full(sbi));
+          tma_load_2d(sdst + 3 * SB_TILE_BYTES, &tm_b, kb0, rowB0, sb_full(sbi));
         }
         __syncwarp();
         if (++sbi == NSB) { sbi = 0; sbph ^= 1; }
       }
-      TWAIT(0, empty_w(si), ph ^ 1);
+      mbar_wait(empty_w(si), ph ^ 1);
       if (elect_one()) {
         const uint32_t dst = w_ring + si * w_stage_bytes;
         mbar_arrive_expect_tx(full_w(si), w_stage_bytes);
@@ -352,12 +306,10 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
       if (++si == S) { si = 0; ph ^= 1; }
      }
     }
-    TFLUSH(0, 2, lane == 0);                         // 0 empty_w, 1 sb_empty, 2 total
   } else if (warp == WARP_X) {
     // ===================================== activation producer ==============================
     pdl_wait();                                      // X is the previous kernel's output
     uint32_t it = 0;
-    TDECL;
     for (int item = cta; item < p.items; item += G) {
      const TcSeg sg = seg_of(p, item);
      const int tm = sg.tile % p.tiles_m;
@@ -366,20 +318,15 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
 #pragma unroll
       for (int jj = 0; jj < KPS; ++jj, ++it) {
         const uint32_t xs = it & x_mask;
-        TWAIT(0, empty_x(xs), ((it >> x_shift) & 1u) ^ 1u);
+        mbar_wait(empty_x(xs), ((it >> x_shift) & 1u) ^ 1u);
         if (elect_one()) {
-          if (kDebug & 1) {
-            mbar_arrive(full_x(xs));
-          } else {
-            mbar_arrive_expect_tx(full_x(xs), x_slot_bytes);
-            tma_load_2d(x_ring + xs * x_slot_bytes, &tm_x, (st * KPS + jj) * 64, tm * TN, full_x(xs));
-          }
+          mbar_arrive_expect_tx(full_x(xs), x_slot_bytes);
+          tma_load_2d(x_ring + xs * x_slot_bytes, &tm_x, (st * KPS + jj) * 64, tm * TN, full_x(xs));
         }
         __syncwarp();
       }
      }
     }
-    TFLUSH(3, 1, lane == 0);                         // 3 empty_x, 4 total
   } else if (warp >= WARP_MMA) {
     // ===================================== MMA issuers (warp WARP_MMA + b: block b of the pair) =====================
     // instruction descriptor (cute::UMMA::InstrDescriptor): c_format F32 (1<<4), a/b format (0 f16, 1 bf16) at
@@ -388,7 +335,6 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
     const uint32_t idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(TN >> 3) << 17) | ((128u >> 4) << 24);
     int seg = 0;
     uint32_t slot = 0, aph = 0, xs = 0, xph = 0;
-    TDECL;
     const uint64_t xdesc0 = make_desc_sw128(x_ring);            // X slot 0, first 16 k; slot s adds s * (slot bytes >> 4)
     const uint32_t xdesc_step = x_slot_bytes >> 4;
     const int mw = warp - WARP_MMA;                    // block of the pair this warp issues for
@@ -398,18 +344,17 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
       const int ns = seg_of(p, item).ns;
       const int buf = NBUF == 2 ? (seg & 1) : 0;
       if (seg >= NBUF) {                               // the epilogue of the segment that last used this D buffer has drained it
-        TWAIT(2, accum_empty(buf), (uint32_t)(((seg / NBUF) - 1) & 1));
+        mbar_wait(accum_empty(buf), (uint32_t)(((seg / NBUF) - 1) & 1));
         tc_fence_after();
       }
       const uint32_t dmine = tmem_base + d_col(buf, mw);
       const int nkb = ns * KPS;
       for (int j = 0; j < nkb; ++j) {
-        TWAIT(0, full_x(xs), xph);
-        TWAIT(1, full_a(slot), aph);
+        mbar_wait(full_x(xs), xph);
+        mbar_wait(full_a(slot), aph);
         tc_fence_after();
         if (elect_one()) {
-          if (!(kDebug & 2))
-            umma_half_kblock_f16_ts(dmine, a_base + slot * 64, xdesc0 + (uint64_t)(xs * xdesc_step), idesc, j > 0 ? 1u : 0u);
+          umma_half_kblock_f16_ts(dmine, a_base + slot * 64, xdesc0 + (uint64_t)(xs * xdesc_step), idesc, j > 0 ? 1u : 0u);
           umma_commit(empty_a(slot));
           umma_commit(empty_x(xs));
           if (j == nkb - 1) umma_commit(accum_full(buf));
@@ -419,7 +364,6 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
         if (++xs == x_slots) { xs = 0; xph ^= 1u; }
       }
     }
-    TFLUSH(5, 3, lane == 0 && mw == 0);              // 5 full_x, 6 full_a, 7 accum_empty, 8 total
   } else if (warp < DQ_WARPS) {
     // ===================================== dequantisers =====================================
     const int grp = warp >> 2;                         // 0..3
@@ -439,8 +383,6 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
     int si = 0, ph = 0, sbi = 0, sbph = 0;
     uint32_t slot = (uint32_t)kpar, aph = 0;         // A ring slot of this thread's next k-block (it advances by 2) + phase
     uint4 s8 = make_uint4(0u, 0u, 0u, 0u), b8 = s8;
-    TDECL;
-    TSEC_DECL;
 
     constexpr int CPK = PKB / 16;                    // 16-byte chunks of packed codes per k-block
     constexpr int KPT = KPS / 2;                     // k-blocks per thread per stage
@@ -448,8 +390,7 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
     // wait for the stage's weights, pull this thread's codes into registers and hand the slot straight back to the
     // producer: the HBM stream then only waits for LDS, not for the dequant math or the MMAs
     auto fetch_stage = [&]() {
-      TWAIT(0, full_w(si), (uint32_t)ph);
-      TSEC_BEGIN();
+      mbar_wait(full_w(si), (uint32_t)ph);
       const uint32_t wsrc = w_ring + si * w_stage_bytes + w_row_off;
 #pragma unroll
       for (int j2 = 0; j2 < KPT; ++j2)
@@ -458,13 +399,11 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
           pk[j2 * CPK + c] = lds128(wsrc + ((((uint32_t)((kpar + 2 * j2) * CPK + c)) ^ w_xor) << 4));
       __syncwarp();
       if (lane == 0) mbar_arrive(empty_w(si));
-      TSEC_END(0);
       if (++si == S) { si = 0; ph ^= 1; }
     };
     // one k-block: 64 codes of row r -> 32 packed 16-bit pairs -> A ring slot
     auto kblock = [&](int j2, uint32_t s2, uint32_t b2) {
       uint32_t o[32];
-      TSEC_BEGIN();
       const uint32_t* pw = reinterpret_cast<const uint32_t*>(pk + j2 * CPK);
       if constexpr (FAST) {
         const SmallScale sc = small_scale_prep<T>(s2, b2);
@@ -474,19 +413,13 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
 #pragma unroll
         for (int c = 0; c < 8; ++c) dequant8<T, BITS, XPERM>(pw + c * (BITS / 4), s2, b2, o + 4 * c);
       }
-      TSEC_END(1);
-      TWAIT(2, empty_a(slot), aph ^ 1u);
-      TSEC_BEGIN();
+      mbar_wait(empty_a(slot), aph ^ 1u);
       tc_fence_after();
-      if (!(kDebug & 8)) {
-        tmem_st32(a_dst + slot * 64, o);
-        tmem_st_wait();
-      }
-      TSEC_END(2);
+      tmem_st32(a_dst + slot * 64, o);
+      tmem_st_wait();
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(full_a(slot));
-      TSEC_END(3);
       slot += 2;
       if (slot >= a_slots) { slot -= a_slots; aph ^= 1u; }
     };
@@ -524,7 +457,7 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
         for (int i = 0; i < ns; ++i) {
           const int st = seg_stage(sg, i);
           if (i == 0 || st == s0 || (st % SPG) == 0) {   // next group of 8 k-blocks: scales / biases of this row
-            TWAIT(1, sb_full(sbi), (uint32_t)sbph);
+            mbar_wait(sb_full(sbi), (uint32_t)sbph);
             const uint32_t src = sb_ring + sbi * SB_SLOT_BYTES + sb_off;
             s8 = lds128(src);
             b8 = lds128(src + SB_TILE_BYTES);
@@ -572,10 +505,8 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
         }
       }
     }
-    TFLUSH(9, 3, threadIdx.x == 0);                  // 9 full_w, 10 sb_full, 11 empty_a, 12 total (dequant warp 0)
-    TSEC_FLUSH(threadIdx.x == 0);
     // ---- help the epilogue warp of this lane quarter drain the CTA's LAST whole tile (see tc_drain_tile)
-    if (p.S == 1 && warp_active && cta < p.items && !(kDebug & 4)) {
+    if (p.S == 1 && warp_active && cta < p.items) {
       const int n_seg = (p.items - cta + G - 1) / G, seg = n_seg - 1, item = cta + seg * G;
       const TcSeg sg = seg_of(p, item);
       const int pair = sg.tile / p.tiles_m, tm = sg.tile % p.tiles_m;
@@ -589,7 +520,6 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
     }
   } else {
     // ===================================== epilogue warps ===================================
-    TDECL;
     // Thread = one output column n (weight row r of block A and of block B), EPI_TOK tokens per step: every warp-level
     // load / store below touches one contiguous line per token (32 lanes x 4 B, or x 2 B for 16-bit outputs -- whole
     // sectors either way), so nothing is staged through shared memory and no store is atomic.
@@ -613,36 +543,33 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
       const int buf = NBUF == 2 ? (seg & 1) : 0;
       const bool full = p.S == 1;
 
-      TWAIT(0, accum_full(buf), (uint32_t)((seg / NBUF) & 1));
+      mbar_wait(accum_full(buf), (uint32_t)((seg / NBUF) & 1));
       tc_fence_after();
       const uint32_t dA = lane_base + d_col(buf, 0), dB = lane_base + d_col(buf, 1);
-      if (!(kDebug & 4)) {
-        if (full) {
-          const bool last = item + G >= p.items;       // the dequant warps help with this CTA's last tile
-          tc_drain_tile<T, FAST>(p, silu, r, dA, dB, TN, rowA0, rowB0, tok0, 0, last ? 1 + DQ_WARPS / 4 : 1);
-        } else {
-          // partial tile of a K split: one slot per CTA (the host plans S > 1 only with one item per CTA)
-          float* part = p.ws_part + (int64_t)cta * slot_elems;
-          for (int t0 = 0; t0 < TN; t0 += EPI_TOK) {
-            float a[EPI_TOK], b[EPI_TOK];
-            tmem_ld8(dA + (uint32_t)t0, a);
-            tmem_ld8(dB + (uint32_t)t0, b);
-            tmem_ld_wait();
+      if (full) {
+        const bool last = item + G >= p.items;       // the dequant warps help with this CTA's last tile
+        tc_drain_tile<T, FAST>(p, silu, r, dA, dB, TN, rowA0, rowB0, tok0, 0, last ? 1 + DQ_WARPS / 4 : 1);
+      } else {
+        // partial tile of a K split: one slot per CTA (the host plans S > 1 only with one item per CTA)
+        float* part = p.ws_part + (int64_t)cta * slot_elems;
+        for (int t0 = 0; t0 < TN; t0 += EPI_TOK) {
+          float a[EPI_TOK], b[EPI_TOK];
+          tmem_ld8(dA + (uint32_t)t0, a);
+          tmem_ld8(dB + (uint32_t)t0, b);
+          tmem_ld_wait();
 #pragma unroll
-            for (int j = 0; j < EPI_TOK; ++j) {
-              __stcg(part + (int64_t)(t0 + j) * 128 + r, a[j] * DSCALE);
-              __stcg(part + (int64_t)(TN + t0 + j) * 128 + r, b[j] * DSCALE);
-            }
+          for (int j = 0; j < EPI_TOK; ++j) {
+            __stcg(part + (int64_t)(t0 + j) * 128 + r, a[j] * DSCALE);
+            __stcg(part + (int64_t)(TN + t0 + j) * 128 + r, b[j] * DSCALE);
           }
-          def0 = tile;
         }
+        def0 = tile;
       }
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(accum_empty(buf));    // this D buffer may be overwritten by a later segment's MMAs
     }
 
-    TFLUSH(13, 1, et == 0);                          // 13 accum_full, 14 total up to the end of the tile epilogues
     // ---- split tile: meet the S - 1 other contributors (CTAs tile*S .. tile*S + S - 1: equal work, they arrive together),
     // then reduce and finish a share of the tile
     if (def0 >= 0) {
@@ -721,7 +648,7 @@ constexpr int SMEM_BUDGET = 227 * 1024;
 constexpr int SMEM_FIXED = 1024 /*align*/ + NSB * SB_SLOT_BYTES + 512 /*barriers*/;
 static_assert(8 * (4 * MAX_STAGES + 2 * NSLOT + 2 * NSB + 4) + 8 <= 512, "barrier block overflows its slot");
 // smallest M that may take the tensor path.  1: the tile kernel beats the CUDA-core GEMV at EVERY M (8.4 vs 10.2 us at
-// M = 1 on q|k|v, 22.5 vs 33.0 us on gate|up: profiles/r1_run11_qmm_sweep_gemv_vs_tensor.txt), so the CUDA-core GEMV only
+// M = 1 on q|k|v, 22.5 vs 33.0 us on gate|up), so the CUDA-core GEMV only
 // serves float32 models, group sizes != 64 and odd shapes.
 // B200P_MIN_TC_M / b200p_qmm_set_min_tensor_m override it.
 static int g_min_tc_m = [] { const char* e = getenv("B200P_MIN_TC_M"); return e ? atoi(e) : 1; }();
@@ -959,9 +886,3 @@ int qmm_tc_launch(const void* x, const uint32_t* w, const void* s, const void* b
 }
 
 }  // namespace b200p
-
-#if B200P_TC_TIMING
-extern "C" int b200p_debug_tc_timing(unsigned long long* out32) {
-  return cudaMemcpyFromSymbol(out32, b200p::g_tc_timing, sizeof(unsigned long long) * 32) == cudaSuccess ? 0 : -1;
-}
-#endif
