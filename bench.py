@@ -1,10 +1,10 @@
 #!/usr/bin/env python
-"""bench.py -- decode tok/s of the batched decode step (BASELINE.json metric), one JSON line on rank 0.
+"""bench.py -- decode tok/s of the batched decode step, one JSON line on rank 0.
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl ours|reference] [--workload ...]
 
-N == 1: Llama-3-8B architecture, MLX 4-bit group-64, batch 64, 8192-token KV context (BASELINE.json
-configs[2], the configuration the metric is quoted on), random-init weights + synthetic KV (no network).
+N == 1: Llama-3-8B architecture, MLX 4-bit group-64, batch 64, 8192-token KV context (the
+configuration the metric is quoted on), random-init weights + synthetic KV (no network).
 N  > 1: the same workload tensor-parallel over N ranks (strong scaling), launched by torch.distributed.run.
 
 A "step" = one decode step of the whole batch: embed -> 32 blocks -> head -> argmax, KV append included.
@@ -12,7 +12,7 @@ A "step" = one decode step of the whole batch: embed -> 32 blocks -> head -> arg
   e2e     the same step driven with HOST token buffers: pinned H2D of the step's ids + D2H of its result
   roofline  dominant kernel (by bytes) timed with CUDA events in an eager instrumented pass
   cpu_baseline  the oracle (numpy port of the reference path) on a bounded sample, rank 0, N == 1 only
---impl reference times that CPU port alone (MLX itself is not installable here: see DESIGN.md).
+--impl reference times that CPU port alone (MLX itself is not installable here).
 """
 from __future__ import annotations
 
@@ -36,11 +36,11 @@ WORKLOADS = {
     "llama3-8b-4bit-b64-t256": ("llama-3-8b", 64, 256),
     "llama3-8b-4bit-b8-t8192": ("llama-3-8b", 8, 8192),
     "llama3-8b-4bit-b1-t8192": ("llama-3-8b", 1, 8192),
-    # configs[2]'s B=256 point: 256 x 8192 tokens of 16-bit KV are 275 GB and do not fit one GPU; context capped at 4096 (137 GB)
+    # the B=256 point: 256 x 8192 tokens of 16-bit KV are 275 GB and do not fit one GPU; context capped at 4096 (137 GB)
     "llama3-8b-4bit-b256-t4096": ("llama-3-8b", 256, 4096),
     "mistral-7b-4bit-b8-t256": ("mistral-7b", 8, 256),
     "qwen3-14b-4bit-b64-t256": ("qwen3-14b", 64, 256),
-    # configs[4]: Llama-3-70B-class 8-bit, batch 128, TP=8.  The quoted 32k context needs 171.8 GB of 16-bit KV per GPU next
+    # Llama-3-70B-class 8-bit, batch 128, TP=8.  The quoted 32k context needs 171.8 GB of 16-bit KV per GPU next
     # to 9.2 GB of weights and does not fit 180 GB; 24 576 tokens (128.8 GB of KV per GPU) is the largest 8k multiple that does
     "llama3-70b-8bit-b128-t24576": ("llama-3-70b", 128, 24576),
     "llama3-70b-8bit-b128-t256": ("llama-3-70b", 128, 256),
@@ -68,11 +68,11 @@ def peaks():
     if os.path.exists(p):
         d = json.load(open(p))
         return float(d["hbm_gbs"]), "measured (MEASURED_PEAKS.json)"
-    return 6650.0, "fallback (B200_PROFILING.md)"
+    return 6650.0, "fallback"
 
 
 class ClockSampler:
-    """nvidia-smi clocks / throttle reasons during the timed region (B200_PROFILING.md recipe)."""
+    """nvidia-smi clocks / throttle reasons during the timed region."""
 
     def __init__(self, gpu_index: int):
         self.rows, self.proc, self.idx = [], None, gpu_index
@@ -718,7 +718,7 @@ def main():
             sweep.append({"workload": name, "error": str(ex)[:200]})
     prefill = None
     if not args.no_prefill:
-        # configs[2] says "8k-token KV context, prefill + decode": short prompts (GEMM-bound) and 2k / 8k prompts (where the
+        # 8k-token KV context, prefill + decode: short prompts (GEMM-bound) and 2k / 8k prompts (where the
         # causal attention grows quadratically), one sequence and eight
         prefill = []
         for pb, pl in ((8, 256), (1, 2048), (8, 2048), (1, 8192), (8, 8192)):

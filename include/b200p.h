@@ -40,7 +40,7 @@ extern "C" {
 
 enum { B200P_F32 = 0, B200P_F16 = 1, B200P_BF16 = 2 };
 
-/* dequantize rounding (SURVEY Appendix A.2; oracle/mlx_ops.py MODE_*) */
+/* dequantize rounding (oracle/mlx_ops.py MODE_*) */
 enum { B200P_DQ_F32_MULADD = 0, B200P_DQ_FMA = 1, B200P_DQ_T_MULADD = 2 };
 
 /* b200p_qmm epilogues */
@@ -84,7 +84,7 @@ int b200p_dequantize(const uint32_t* w, const void* scales, const void* biases, 
 
 /* mx.quantize(w, group_size, bits)                                  [nn.quantize, utils.py:886-905; convert, utils.py:934-981]
  * w `dtype` [N,K] -> wq uint32 [N, K*bits/32], scales / biases `dtype` [N, K/group_size]; every step rounded to `dtype`
- * where MLX's composed ops round it (SURVEY Appendix A.1): bit-exact against oracle/mlx_ops.py quantize.
+ * where MLX's composed ops round it: bit-exact against oracle/mlx_ops.py quantize.
  * group_size 32, 64 or 128. */
 int b200p_quantize(const void* w, uint32_t* wq, void* scales, void* biases, int64_t N, int64_t K, int group_size,
                    int bits, int dtype, void* stream);
@@ -152,7 +152,7 @@ int b200p_rope_kv_append(void* qkv, void* q_out, void* kcache, void* vcache,
 int b200p_silu_mul(float* gu, void* out, int64_t M, int64_t I, int64_t ldg, int64_t ldo, int dtype, int flags,
                    void* stream);
 /* LoRA low-rank update (mlx_lm LoRALinear: y = linear(x) + (scale * (x @ lora_a) @ lora_b).astype(x.dtype))
- *                                       [adapters on q_proj / v_proj: lora_init.py:63-73; SURVEY A.9, row f4]
+ *                                       [adapters on q_proj / v_proj: lora_init.py:63-73]
  * x `dtype` [M,K] (ldx); At `dtype` [16, K] = lora_a transposed, rank padded to 16 with zero rows (k axis permuted like x
  * when x is PERM8); Bt `dtype` [N, 16] = lora_b transposed, padded likewise; y[m, col0 + n] += update for n < N:
  * out_f32 = 1 -> y is the float accumulation buffer of the projection (ldy floats), else its `dtype` output (the update
@@ -230,7 +230,7 @@ int b200p_sample_top_p(const float* logits, int32_t* tokens, float* probs_out, i
                        int64_t V, int64_t ldl, float temperature, float top_p, uint64_t seed,
                        uint64_t offset, void* stream);
 
-/* ---- tensor-parallel exchange over NVLink peer memory (new; the reference is single-device) -----------------
+/* ---- tensor-parallel exchange over NVLink peer memory (new; the reference is single-device) ----------------------------
  * Setup calls (host side, synchronous, NOT graph-capturable; the only entry points that allocate):
  *   b200p_symm_alloc   cudaMalloc + zero a buffer peers may map;   b200p_symm_free releases it
  *   b200p_ipc_export   64-byte cudaIpcMemHandle of such a buffer (ship it to the peers with any host transport)

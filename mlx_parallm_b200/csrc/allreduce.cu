@@ -1,4 +1,4 @@
-// Tensor-parallel exchange over NVLink peer memory (new: the reference is single-device, SURVEY 8e).
+// Tensor-parallel exchange over NVLink peer memory (new: the reference is single-device).
 //
 // b200p_allreduce_residual_rmsnorm fuses what follows every row-parallel projection (o_proj, down_proj) under TP:
 //

@@ -442,7 +442,7 @@ __global__ void rope_kv_append_kernel(TIN* __restrict__ qkv, T* __restrict__ q_o
   }
 }
 
-// head_dim 128 (every BASELINE model): a WARP per (token, head), 8 heads of a token per CTA; lane = pairs (2*lane, 2*lane + 1)
+// head_dim 128: a WARP per (token, head), 8 heads of a token per CTA; lane = pairs (2*lane, 2*lane + 1)
 // of the first half and their partners 64 further.  The kernel is pure latency (4 MB of traffic): every warp issues its
 // position load and its four 8-byte value loads at once and finishes after one round trip; the per-head RMSNorm of Qwen3 is a
 // warp reduction (no block barrier); 8-byte (fp32 input) / 4-byte (16-bit) accesses per lane, whole lines per warp.

@@ -1,5 +1,5 @@
 // mx.quantize(w, group_size, bits): dense 16/32-bit weights -> MLX affine codes + per-group scales / biases
-// (nn.quantize at utils.py:886-905, the converter at utils.py:934-981).  Row f3 of the scope table.
+// (nn.quantize at utils.py:886-905, the converter at utils.py:934-981).
 //
 // HBM-bound byte work: N*K*sizeof(T) in, N*K*bits/8 + 2*N*(K/gs)*sizeof(T) out, one pass.  One thread owns the codes of
 // one output word (8 at 4 bits, 4 at 8 bits: one 16- or 8-byte load); the gs/8 (gs/4) threads of a group reduce min / max

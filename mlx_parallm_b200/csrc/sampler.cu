@@ -371,7 +371,7 @@ top_p_kernel(const float* __restrict__ logits, int32_t* __restrict__ tokens, flo
       __syncthreads();
     }
     thr_bits = s_thr;
-    if (!s_done && s_above <= 0.f) empty = true;   // even the largest p exceeds top_p (reference: 0/0, SURVEY B6)
+    if (!s_done && s_above <= 0.f) empty = true;   // even the largest p exceeds top_p (reference: 0/0)
   }
 
   if (empty) {                                     // documented deviation: the argmax (lowest index among ties)

@@ -16,7 +16,7 @@ sm_100a kernels of libb200parallm.so:
     final RMSNorm + lm_head (float32 logits)                 b200p_rmsnorm, b200p_qmm (EPI_STORE_F32)
 
 The residual stream is float32 (the reference's stream is float32 from layer 0 on because
-PagedKVCache promotes, SURVEY B3); GEMM inputs and the KV cache are the model's 16-bit storage
+PagedKVCache promotes); GEMM inputs and the KV cache are the model's 16-bit storage
 type.  Tensor parallelism (column-split q/k/v/gate/up, row-split o/down, vocab-split head) is
 applied at load time by ``tp.shard_*`` and adds one all-reduce after each row-split projection.
 """
@@ -175,7 +175,7 @@ class DecoderModel:
         self.dtype: Optional[torch.dtype] = None
         self.device: Optional[torch.device] = None
         self._arenas: Dict[int, dict] = {}
-        # One forward at a time per model instance (SURVEY 8b "Threading"): the scratch arenas, the self-cleaning qmm
+        # One forward at a time per model instance: the scratch arenas, the self-cleaning qmm
         # workspace and the fp32 accumulators are shared by every caller of this model, and the reference server runs
         # generate_step from an executor thread and from the event loop at once (utils.py:1345 vs server/main.py:1358).
         # Held around every eager forward, every decode-step replay and every graph capture.
@@ -495,7 +495,7 @@ class DecoderModel:
 
     def __call__(self, inputs, cache: Optional[List[BatchedKVCache]] = None, last_only: bool = False):
         """inputs int [B, L] -> logits float32 [B, L, V] (or [B, 1, V] with last_only, the only rows
-        generate_step reads, utils.py:404 / SURVEY B10).  Under TP the vocab axis is this rank's shard."""
+        generate_step reads, utils.py:404).  Under TP the vocab axis is this rank's shard."""
         with self._lock:
             return self._forward_locked(inputs, cache, last_only)
 

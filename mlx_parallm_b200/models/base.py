@@ -10,7 +10,7 @@ Mirrors mlx_parallm/models/base.py (reference):
                           (latent attention, gated delta rule, previous-token embedding) under the same row protocol
 
 B200 design: one dense device buffer [B, Hkv, Tcap, D] per layer in the model's 16-bit storage type
-(the reference allocates float32, base.py:111-112 -- deliberate deviation, SURVEY B3), plus a device
+(the reference allocates float32, base.py:111-112 -- deliberate deviation), plus a device
 int32 ``lengths[B]`` the kernels read, so that a captured decode graph stays valid while rows
 advance.  The model's fused kernels (b200p_rope_kv_append / b200p_attn) write and read the buffers
 directly; ``update_and_fetch`` is kept for API compatibility with callers that poke the cache.

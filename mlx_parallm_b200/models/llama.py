@@ -42,7 +42,7 @@ class ModelArgs(BaseModelArgs):
                 if self.rope_scaling["rope_type"] not in ["llama3", "linear"]:
                     raise ValueError(f"rope_scaling 'rope_type' {self.rope_scaling['rope_type']} not supported")
         if self.attention_bias or self.mlp_bias:
-            raise NotImplementedError("projection biases are not on the hot path of any BASELINE config")
+            raise NotImplementedError("projection biases are not on the hot path of any supported configuration")
         if self.rope_traditional:
             raise NotImplementedError("rope_traditional=True is not used by Llama/Mistral checkpoints")
 

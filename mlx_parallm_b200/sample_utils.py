@@ -30,7 +30,7 @@ def top_p_sampling(logits: torch.Tensor, top_p: float, temperature: float, axis:
     """softmax(logits/temperature) -> keep the sorted prefix whose inclusive cumulative mass <= top_p ->
     renormalise -> draw (sample_utils.py:15-37).  One kernel (b200p_sample_top_p): radix-select of the
     nucleus threshold + inverse-CDF draw, no sort.  Returns token ids [B, 1] like the reference.
-    Deviation (SURVEY B6): if even the most likely token exceeds top_p the reference divides 0/0; here the
+    Deviation: if even the most likely token exceeds top_p the reference divides 0/0; here the
     argmax is returned."""
     assert axis in (-1, logits.dim() - 1)
     l2 = logits.reshape(-1, logits.shape[-1]).float().contiguous()

@@ -1,7 +1,7 @@
-"""Deterministic synthetic checkpoints in the reference's on-disk format (SURVEY 8d).
+"""Deterministic synthetic checkpoints in the reference's on-disk format.
 
 There is no network for real checkpoints and MLX's threefry PRNG is not reproducible outside MLX
-(scripts/build_tiny_model.py:123 in the reference), so every BASELINE config is instantiated from
+(scripts/build_tiny_model.py:123 in the reference), so every benchmark configuration is instantiated from
 numpy / torch generators with fixed seeds, in MLX layout: ``*.weight`` uint32 packed codes,
 ``*.scales`` / ``*.biases`` [N, K/64], norm weights, ``config.json`` with a ``quantization`` block
 (utils.py:679), ``model.safetensors`` with metadata {"format": "mlx"} (utils.py:870).
@@ -16,7 +16,7 @@ from typing import Dict, Optional
 import numpy as np
 import torch
 
-# HF-style configs of the five BASELINE.json configs (+ tiny variants for tests).  Dims: SURVEY 8.
+# HF-style configs of the five benchmark models (+ tiny variants for tests).
 CONFIGS: Dict[str, dict] = {
     # scripts/build_tiny_model.py:70-101 (hidden 64, 8 layers, 4 heads, inter 128, tied, 4-bit g64)
     "tiny": dict(model_type="llama", hidden_size=64, num_hidden_layers=8, intermediate_size=128,
@@ -95,7 +95,7 @@ def norm_names(cfg: dict):
 
 
 def weight_bytes_per_step(cfg: dict, scale_bytes: int = 2) -> int:
-    """Algorithmic weight bytes of one decode step (SURVEY 8d / BASELINE.md section 3): every linear
+    """Algorithmic weight bytes of one decode step: every linear
     except the embedding table (B gathered rows only) + norm weights."""
     q = cfg["quantization"]
     total = 0
@@ -124,7 +124,7 @@ def _stable_seed(seed: int, name: str) -> int:
 
 def random_weights(cfg: dict, seed: int = 1234, dtype: str = "float16", device="cpu",
                    only: Optional[callable] = None) -> Dict[str, torch.Tensor]:
-    """Config-2 style generator: uniform random codes, scales = +-U(0.5,1.5)*(2/(2^bits-1))/sqrt(K)
+    """Generator of random checkpoints: uniform random codes, scales = +-U(0.5,1.5)*(2/(2^bits-1))/sqrt(K)
     (random sign exercises MLX's signed scales), biases = -scale*(2^bits-1)/2 + N(0, 0.01/sqrt(K)),
     norm weights 1 + N(0, 0.02).  One torch.Generator per tensor, seeded from (seed, name), so any subset or
     any TP shard of the same model can be regenerated independently on any device type... but NOT across

@@ -1,5 +1,5 @@
 """Tensor parallelism for the decode step (new work mandated by the north star; the reference is
-single-device, SURVEY 2.3 / 8e).
+single-device).
 
 One process per GPU (torchrun), ranks share a ``torch.distributed`` group (NCCL on the GPUs, gloo in
 the CPU tests).  Partitioning, applied to MLX-layout tensors at load time so no re-quantisation is

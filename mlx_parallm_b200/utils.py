@@ -130,7 +130,7 @@ def apply_chat_template_cached(tokenizer: TokenizerWrapper, messages: List[Dict[
 # --------------------------------------------------------------------------------- KV pool
 class _KVPool:
     """utils.py:199-223.  Keyed additionally by model identity and thread so two generations never share
-    cache objects (the reference's pool is a documented race)."""
+    cache objects (the reference's pool is a race)."""
 
     def __init__(self):
         self._pool: Dict[tuple, List[BatchedKVCache]] = {}
@@ -331,7 +331,7 @@ def generate_step(
     Same contract as the reference: prefill on the whole (left-padded) prompt batch, greedy if temp == 0
     else top-p / categorical sampling, repetition_penalty raises NotImplementedError (utils.py:366-367),
     and the step for token n+1 is already in flight when token n is yielded (utils.py:420-427).
-    ``probs`` is per row (the reference gathers row 0 only, SURVEY B7).  ``prompt_lengths`` (models with ``supports_ragged``
+    ``probs`` is per row (the reference gathers row 0 only).  ``prompt_lengths`` (models with ``supports_ragged``
     only): row b's last prompt_lengths[b] ids are its prompt, the ids before them are left padding and are not fed at all, so a
     row's tokens do not depend on the other rows of the batch."""
     if repetition_penalty:
@@ -469,7 +469,7 @@ def generate(model, tokenizer, prompt: str, max_tokens: int = 100, verbose: bool
 def batch_generate(model, tokenizer, prompts: List[str], max_tokens: int = 100, verbose: bool = False,
                    format_prompts: bool = True, formatter: Optional[Callable] = None, **kwargs) -> List[str]:
     """utils.py:473-543: chat-template, left-pad (pad = eos if unset), run max_tokens steps with no early
-    stop (SURVEY B8), decode and cut at the eos / pad strings."""
+    stop, decode and cut at the eos / pad strings."""
     if not isinstance(tokenizer, TokenizerWrapper):
         tokenizer = TokenizerWrapper(tokenizer)
     if verbose:

@@ -1,8 +1,7 @@
 """TEST INFRASTRUCTURE -- the hook that pins this oracle against the real reference the day MLX is importable.
 
-The reference's arithmetic lives in ``mlx==0.25.2`` / ``mlx-lm==0.24.1`` (pyproject.toml:38-39), which are installed on
-neither this container nor the GPU box (no wheel, no network), so parity is "unpinned" today.  This
-module is what closes that gap without a code change: when ``import mlx.core`` works AND the reference tree is on disk,
+The reference's arithmetic lives in ``mlx==0.25.2`` / ``mlx-lm==0.24.1`` (pyproject.toml:38-39), which are not
+installed here, so parity is "unpinned" until they are.  This module is what closes that gap without a code change: when ``import mlx.core`` works AND the reference tree is on disk,
 ``available()`` turns true and ``tests/test_mlx_adapter.py`` stops skipping.  It then
 
   * runs the reference's OWN ``load_model`` (mlx_parallm/utils.py:630-708) and ``generate_step`` (utils.py:315-427) on
@@ -106,7 +105,7 @@ class ReferenceRun:
 
 
 def compare_all(checkpoint_dir: str, prompts: np.ndarray, steps: int = 32) -> Dict[str, object]:
-    """Everything SURVEY 8c asks of the adapter in one call (used by tests/test_mlx_adapter.py): reference logits and
+    """Everything the adapter is asked for in one call (used by tests/test_mlx_adapter.py): reference logits and
     greedy transcript for ``prompts`` from the real MLX path."""
     run = ReferenceRun(checkpoint_dir)
     toks: List[np.ndarray] = [t for t, _ in run.greedy(prompts, steps)]

@@ -2,8 +2,8 @@
 
 TEST INFRASTRUCTURE ONLY (see oracle/__init__.py).  PARITY UNPINNED vs real MLX.
 
-Every function cites the reference call site it stands in for (paths relative to
-/root/reference) and the SURVEY.md appendix item that states the MLX semantics.
+Every function cites the reference call site it stands in for (paths within
+the reference project).
 
 dtype convention: arrays are carried as numpy float32 (or float16) and a ``dtype``
 string in {"float32", "float16", "bfloat16"} says which storage type MLX would
@@ -15,7 +15,7 @@ import numpy as np
 
 DTYPES = ("float32", "float16", "bfloat16")
 
-# dequantize rounding modes (SURVEY Appendix A.2 -- unverifiable without MLX, so all
+# dequantize rounding modes (unverifiable without MLX, so all
 # candidates are implemented; the CUDA kernel must match whichever is selected, bit for bit)
 MODE_F32_MULADD = 0   # p = fl32(q*s); r = fl32(p + b); out = round_T(r)      (MLX CPU-backend style)
 MODE_FMA = 1          # out = round_T(fma32(q, s, b))
@@ -47,7 +47,7 @@ def bf16_from_bits(b: np.ndarray) -> np.ndarray:
 def e4m3_round(x: np.ndarray) -> np.ndarray:
     """float32 -> nearest OCP FP8 E4M3 value (round-half-even, 3 mantissa bits, normals 2^-6 .. 448, subnormals in steps
     of 2^-9, saturating), returned as float32.  Not a reference format: the reference stores K/V in float32 (base.py:111-112);
-    this exists to QUANTIFY what an fp8 KV cache would cost against the 1e-2 logits budget."""
+    this exists to QUANTIFY what an fp8 KV cache would cost against the 1e-2 logits tolerance."""
     x = np.asarray(x, dtype=np.float32)
     a = np.abs(x).astype(np.float64)
     with np.errstate(divide="ignore"):
@@ -279,7 +279,7 @@ def top_p_distribution(logits, top_p: float, temperature: float) -> np.ndarray:
     """The categorical distribution top_p_sampling (sample_utils.py:3-39) draws from, as a dense
     [B, V] probability table: softmax(logits/T) -> sort desc -> keep tokens whose INCLUSIVE
     cumulative mass <= top_p -> renormalise.  If nothing is kept (p_1 > top_p; the reference then
-    divides 0/0) the build's documented deviation applies: all mass on the argmax."""
+    divides 0/0) the documented deviation applies: all mass on the argmax."""
     p = softmax(np.asarray(logits, np.float32) / np.float32(temperature))
     B, V = p.shape
     out = np.zeros_like(p)

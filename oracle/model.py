@@ -2,14 +2,14 @@
 
 TEST INFRASTRUCTURE ONLY (see oracle/__init__.py).  PARITY UNPINNED vs real MLX.
 
-Follows (paths relative to /root/reference):
+Follows (paths within the reference project):
   mlx_parallm/models/llama.py:49-271   Attention / MLP / TransformerBlock / LlamaModel / Model
   mlx_parallm/models/qwen3.py:23-226   same with per-head q_norm/k_norm before RoPE (65-70)
   mlx_parallm/models/base.py:42-149    BatchedKVCache / PagedKVCache
   mlx_parallm/utils.py:315-427         generate_step (greedy + sampling dispatch)
 
 ``numerics``:
-  "reference"  MLX type promotion as the reference actually runs (SURVEY B3): storage dtype T up
+  "reference"  MLX type promotion as the reference actually runs: storage dtype T up
                to the first cache fetch, PagedKVCache holds float32 (base.py:111-112), SDPA output
                and everything after it is float32.
   "mirror"     the rounding points of the CUDA path (GEMM inputs / KV in T, fp32 residual stream);
@@ -38,7 +38,7 @@ class OracleConfig:
     head_dim: Optional[int] = None
     rope_theta: float = 10000.0
     rope_scale: float = 1.0
-    tie_word_embeddings: bool = True      # llama.py:30 default (SURVEY B9)
+    tie_word_embeddings: bool = True      # llama.py:30 default
     group_size: int = 64
     bits: int = 4
     dtype: str = "float16"
@@ -238,7 +238,7 @@ class OracleModel:
             else:
                 kf, vf = k, v
             if kv is not None and self.numerics == "reference":
-                cur = "float32"                                          # SURVEY B3 promotion
+                cur = "float32"                                          # MLX's promotion
             odt = cur if self.numerics == "reference" else T
             o = ops.sdpa(q, kf, vf, D ** -0.5, mask, odt)
             o = o.transpose(0, 2, 1, 3).reshape(B, L, H * D)

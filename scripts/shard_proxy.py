@@ -2,8 +2,8 @@
 
 builds rank 0's shard of a world-W model (weights generated tensor by tensor on the device and sharded as they come, so
 the unsharded model never has to exist), fills a synthetic KV context and times the captured decode step.  What it
-measures is the per-GPU compute + HBM part of BASELINE configs[4] (Llama-3-70B-class 8-bit, TP=8), which does not fit
-a box budget as an 8-GPU run: step time under TP = this + 2 exchanges per layer.
+measures is the per-GPU compute + HBM part of a Llama-3-70B-class 8-bit model at TP=8:
+step time under TP = this + 2 exchanges per layer.
 Partial sums are NOT reduced, so the tokens are meaningless; the cost of a step does not depend on the values.
 
     python scripts/shard_proxy.py --config llama-3-70b --world 8 --batch 128 --context 16384

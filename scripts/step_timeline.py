@@ -19,7 +19,7 @@ import bench
 
 def main():
     wl = sys.argv[1] if len(sys.argv) > 1 else "llama3-8b-4bit-b64-t256"
-    out = sys.argv[2] if len(sys.argv) > 2 else "gpurun_out/timeline_" + wl
+    out = sys.argv[2] if len(sys.argv) > 2 else "timeline_" + wl
     cfg_name, B, T = bench.WORKLOADS[wl]
     dev = torch.device("cuda:0")
     torch.cuda.set_device(dev)

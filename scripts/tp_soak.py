@@ -1,7 +1,7 @@
 """Value-checking soak of the peer-memory TP exchange on real GPUs (torchrun, one rank per GPU).
 
 The exchange kernels (csrc/allreduce.cu) publish their arrival with a relaxed flag and read the peers' partial buffers with
-system-scope relaxed loads, relying on the kernel boundary before them for the writes to be performed (VERDICT r1, weak 5).
+system-scope relaxed loads, relying on the kernel boundary before them for the writes to be performed.
 This does not argue that; it measures it: >= 100 000 exchanges with random partial sums, every one of which must deliver
 
   * the bit-identical result on every rank (one-shot: the whole residual stream h and the normalised y; rows: the

@@ -34,7 +34,7 @@ def transcript(name, dtype, B, Lp, steps, **ov):
 
 
 def main():
-    # 1. greedy transcripts: config 1 "tiny" (f32, V=151936, B=8, 16-token prompts, 32 tokens)
+    # 1. greedy transcripts: config "tiny" (f32, V=151936, B=8, 16-token prompts, 32 tokens)
     np.savez_compressed(os.path.join(OUT, "tiny_f32_greedy.npz"), **transcript("tiny", "float32", 8, 16, 32))
     np.savez_compressed(os.path.join(OUT, "tiny_llama_f16_greedy.npz"), **transcript("tiny-llama", "float16", 4, 12, 32))
     np.savez_compressed(os.path.join(OUT, "tiny_qwen3_bf16_greedy.npz"), **transcript("tiny-qwen3", "bfloat16", 4, 12, 32))

@@ -1,5 +1,5 @@
 """The oracle against the committed fixtures (tests/golden/make_golden.py): regression pin for the
-restatement, and for the sizes the reference's own fixture uses (BASELINE config 1 'tiny')."""
+restatement, and for the sizes the reference's own fixture uses ('tiny')."""
 import os
 
 import numpy as np

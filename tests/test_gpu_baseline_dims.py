@@ -1,5 +1,5 @@
-"""Parity against the CPU oracle AT THE DIMENSIONS THE BENCHMARK IS QUOTED ON (VERDICT r1, item 1): two-layer, full-width,
-full-vocabulary slices of every BASELINE.json architecture -- Mistral-7B, Llama-3-8B, Qwen3-14B (4-bit) and Llama-3-70B-class
+"""Parity against the CPU oracle AT THE DIMENSIONS THE BENCHMARK IS QUOTED ON: two-layer, full-width,
+full-vocabulary slices of every benchmark architecture -- Mistral-7B, Llama-3-8B, Qwen3-14B (4-bit) and Llama-3-70B-class
 (8-bit) -- with ``synth.random_weights``, compared with ``OracleModel(numerics="reference")`` (what MLX would compute: fp32 KV
 cache, fp32 residual stream):
 

@@ -1,8 +1,8 @@
-"""The reference's text front-ends on the CUDA engine (SURVEY 8 rows a12-a14): batch_generate, batch_generate_text (LCP split,
+"""The reference's text front-ends on the CUDA engine: batch_generate, batch_generate_text (LCP split,
 shared-prefix prefill), batch_stream_generate_text, generate / stream_generate, the KV pool and two threads on one model.
 
-Expected transcripts come from the CPU oracle fed the SAME padded ids (left pads are attended and take RoPE positions,
-SURVEY B1), with the reference's bookkeeping (utils.py:520-531, 1028-1068, 1296-1340) restated on the oracle's tokens."""
+Expected transcripts come from the CPU oracle fed the SAME padded ids (left pads are attended and take RoPE positions),
+with the reference's bookkeeping (utils.py:520-531, 1028-1068, 1296-1340) restated on the oracle's tokens."""
 import asyncio
 import threading
 
@@ -69,7 +69,7 @@ def test_batch_generate_left_pads_and_matches_the_oracle(pair):
 
 
 def test_batch_generate_runs_max_tokens_steps_and_cuts_at_the_eos_string(pair):
-    """No early stop on EOS (SURVEY B8): every row runs max_tokens steps, the text is cut at the eos string afterwards."""
+    """No early stop on EOS: every row runs max_tokens steps, the text is cut at the eos string afterwards."""
     from mlx_parallm_b200.tokenizer_utils import TokenizerWrapper
     from mlx_parallm_b200.utils import batch_generate
     cfg, om, gm = pair
@@ -220,7 +220,7 @@ def test_kv_pool_reuses_buffers_and_the_decode_graph(pair):
 
 
 def test_two_threads_generate_on_one_model(pair):
-    """SURVEY 8b 'Threading': the reference server runs generate_step from an executor thread and from the event loop at once
+    """Threads: the reference server runs generate_step from an executor thread and from the event loop at once
     (utils.py:1345 vs server/main.py:1358).  Same batch size on purpose: both threads use the same scratch arena."""
     from mlx_parallm_b200 import utils
     cfg, om, gm = pair

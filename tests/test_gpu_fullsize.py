@@ -1,4 +1,4 @@
-"""BASELINE-size checks through size-independent properties (the oracle cannot run these shapes in seconds):
+"""Full-size checks through size-independent properties (the oracle cannot run these shapes in seconds):
 agreement between independent kernels of the library, linearity, permutation invariance, idempotence."""
 import numpy as np
 import pytest

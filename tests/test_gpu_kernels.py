@@ -94,7 +94,7 @@ def test_quantize_bit_exact(ops, bits, dtype, gs):
 
 
 def test_quantize_dequantize_roundtrip_full_size(ops):
-    """Size-independent property at a BASELINE shape (down_proj of Llama-3-8B): dequantize(quantize(w)) is within half a
+    """Size-independent property at a full-size shape (down_proj of Llama-3-8B): dequantize(quantize(w)) is within half a
     quantisation step (+ storage rounding) of w, group by group, and quantising the dequantised matrix again reproduces
     the codes (idempotence)."""
     g = torch.Generator(device="cuda").manual_seed(4)
@@ -529,7 +529,7 @@ def test_top_p_sampling_distribution(ops, top_p, temp):
 
 @pytest.mark.parametrize("V,top_p,temp", [(128256, 0.9, 0.7), (151937, 0.6, 1.0), (32000, 0.95, 1.2)])
 def test_top_p_large_vocab_stays_in_the_oracle_nucleus(ops, V, top_p, temp):
-    """BASELINE vocab sizes (151 937 = unaligned rows -> scalar loads): LM-like logits (a gaussian body, a few large values,
+    """Full vocabulary sizes (151 937 = unaligned rows -> scalar loads): LM-like logits (a gaussian body, a few large values,
     a block of exactly equal logits as untrained vocab slots have), 1500 draws: every token inside the oracle's nucleus,
     frequencies of the heavy tokens as the oracle's renormalised distribution says."""
     rng = np.random.default_rng(V)

@@ -1,5 +1,5 @@
 """LoRA at inference (row f4): b200p_lora_add against numpy, the adapted model against the oracle with the same adapters
-(mlx_lm LoRALinear semantics, SURVEY A.9), adapters loaded from the reference's on-disk format."""
+(mlx_lm LoRALinear semantics), adapters loaded from the reference's on-disk format."""
 import json
 
 import numpy as np

@@ -88,7 +88,7 @@ def test_greedy_tokens_match_golden_transcript(golden_dir, fixture, name, dtype)
         logits = [lg for _, (_, lg) in zip(range(32), oracle_generate_step(g["prompts"], om))]
         frac, near, real = greedy_report(got, g["tokens"], logits, LOGIT_TOL)
         assert not real, real
-    if dtype != "bfloat16":            # bf16 (8 mantissa bits) is held to the logits bar and the near-tie rule, see DESIGN 2
+    if dtype != "bfloat16":            # bf16 (8 mantissa bits) is held to the logits bar and the near-tie rule
         assert same.mean() >= 0.99, same
 
 

@@ -1,6 +1,6 @@
-"""SURVEY 8c plan: the day ``import mlx.core`` works next to a reference checkout, these tests pin the oracle -- and through
+"""The day ``import mlx.core`` works next to a reference checkout, these tests pin the oracle -- and through
 it the CUDA path -- against the reference's own MLX run on the same synthetic checkpoint.  Skipped (with the reason) on
-machines without MLX: parity stays "unpinned" there, as DESIGN.md section 2 states."""
+machines without MLX: parity stays "unpinned" there."""
 import numpy as np
 import pytest
 

@@ -1,4 +1,4 @@
-"""Known-answer tests that pin the oracle (SURVEY 8c): hand-derived, independent of the oracle's own code path."""
+"""Known-answer tests that pin the oracle: hand-derived, independent of the oracle's own code path."""
 import numpy as np
 import pytest
 
@@ -209,7 +209,7 @@ def test_prefill_then_decode_equals_full_forward(name, dtype):
     assert rel_err(inc, full) < 2e-3 if dtype == "bfloat16" else rel_err(inc, full) < 5e-4
 
 
-def test_reference_and_mirror_numerics_agree_within_north_star_tolerance():
+def test_reference_and_mirror_numerics_agree_within_logits_tolerance():
     cfg, om_ref, _ = make_pair("tiny-llama", dtype="float16", device=None, numerics="reference")
     _, om_mir, _ = make_pair("tiny-llama", dtype="float16", device=None, numerics="mirror")
     ids = prompts_for(cfg, 3, 10)

@@ -1,6 +1,6 @@
-"""the reference's UNMODIFIED server module imports on this engine.
+"""The reference's UNMODIFIED server module imports on this engine.
 
-Runs where the reference tree exists (this container: /root/reference; the GPU box has no copy, and reference sources are
+Runs where the reference tree exists (reference sources are
 never vendored into this repo).  ``compat.install(shim_mlx=True)`` makes ``mlx_parallm.utils / .sample_utils / .models.*``
 resolve to this package and registers stand-ins for the handful of ``mlx.core`` names the server calls itself
 (mlx_parallm_b200/mx_shim.py); the server's own code -- FastAPI app, schemas, batching queues, log-prob arithmetic -- is the
