@@ -19,7 +19,9 @@
 // Schedule.  A unit is (16-row tile, 512 k).  Epilogues that need whole sums deal whole tiles to the CTAs; the accumulating epilogue
 // deals units (panel of k, tile, chunk) evenly whatever N and K are, a panel being as much k as x fits shared memory.  Inside a
 // CTA every warp takes an equal contiguous run of units; runs that end inside a tile meet in shared memory once, at the end, and are
-// added in a fixed order.  Only the accumulating epilogue of a tile that two CTAs share depends on the order of two red.adds.
+// added in a fixed order.  The accumulating epilogue adds one piece of a tile per CTA and panel that holds units of it (a CTA's run is often shorter
+// than a tile), in order of arrival: its results are reproducible up to the order of fp32 sums.  (The dispatch takes at most 8 tokens;
+// 9 to 16 run when the path is forced.)
 //
 // Measured (CUDA graph over weight copies larger than L2, us; before: the tile kernel and the register GEMV): gate|up 28672 x 4096 4-bit
 // f16 at M = 1 / 4 / 6: 16.2 / 17.9 / 18.5 (21.7 / 22.0 / 22.1), = 4.1 TB/s at M = 1; 34816 x 5120 at M = 1: 22.0 (26.8), = 4.6 TB/s;
