@@ -22,7 +22,7 @@
 // ranges of (tile, K stage) and adds its sums with cp.reduce.async.bulk.tensor (as qmm_sk.cu does).  Every mbarrier wait is bounded; one that runs out is reported.
 //
 // Measured (bf16 or f16, us, before / after): gate|up 28672 x 4096 4-bit 62 / 51 at 201 tokens, 64 / 57 at 256, 235 / 208 at 1000, 500 / 390 at
-// 2048, 1261 / 780 at 4096 (1.2 PFLOP/s); 57344 x 8192 8-bit (bf16, with the fp32 dequantisation of dequant.cuh) 356 / 214 at 201, 1201 / 790 at 1000; down 4096 x 14336 405 / 359 at 4096.
+// 2048, 1261 / 780 at 4096 (1.2 PFLOP/s); 57344 x 8192 8-bit (bf16, with the fp32 dequantisation of dequant.cuh) 356 / 206 at 201, 1201 / 790 at 1000; down 4096 x 14336 405 / 359 at 4096.
 //
 // warp roles (768 threads): 0..15 dequantisers (group g = 4 warps takes k-blocks g, g + 4, ...; thread = weight row), 16..19 epilogue,
 // 20 TMA producer of weights, scales and biases, 21 TMA producer of X, 22 / 23 MMA issuers.
