@@ -13,7 +13,7 @@ cache, fp32 residual stream):
 Why not "identical on >= 99 % of sequences" as a raw count: a random-init model with V = 128 256 has a top-2 logit margin of
 ~0.2 sigma on average, so a 4e-4 relative logits difference flips the argmax on ~0.1 % of the STEPS and 2-5 % of all 32-token
 transcripts pass through at least one such near-tie (measured: 95.3-97.7 % identical in f16, profiles/
-r2_baseline_dims_parity.txt); trained checkpoints are peaked and do not.  The margin-qualified rule below is the same statement
+v02_baseline_dims_parity.txt); trained checkpoints are peaked and do not.  The margin-qualified rule below is the same statement
 without that artefact, and the raw fraction is printed for the record."""
 import os
 
@@ -101,7 +101,7 @@ def test_greedy_32_tokens_on_128_sequences(pair):
     name, dtype, cfg, om, gm = pair
     if (name, dtype) not in GREEDY_DEFAULT and os.environ.get("B200P_FULL_PARITY", "0") != "1":
         pytest.skip("the oracle needs 1.5-4.5 min for this slice (128 x 32 full-vocabulary steps on the host cores): run with "
-                    "B200P_FULL_PARITY=1; a full run is kept as profiles/r2_baseline_dims_parity.txt")
+                    "B200P_FULL_PARITY=1; a full run is kept as profiles/v02_baseline_dims_parity.txt")
     B, L, S = 128, 16, 32
     ids = np.random.default_rng(9).integers(0, cfg["vocab_size"], (B, L)).astype(np.int64)
     exp, exp_logits = [], []
