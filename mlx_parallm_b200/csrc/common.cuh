@@ -117,6 +117,17 @@ __device__ __forceinline__ float glu_unit(float gate, float up, int epi, float2 
   return gate / (1.f + expf(-gate)) * up;                          // B200P_GEMM_GLU_SILU
 }
 
+// The same where the result is rounded to 16 bits: the unit's exponential and quotient from the approximate instructions (2e-6 of the
+// result over gates of -20 .. 20, against half a unit of 4.9e-4 in f16).  The exact quotient's slow path bounded the prompts' epilogues.
+__device__ __forceinline__ float glu_unit16(float gate, float up, int epi, float2 act) {
+  if (epi == B200P_GEMM_GLU_SILU) return __fdividef(gate, 1.f + __expf(-gate)) * up;
+  if (epi == B200P_GEMM_GLU_CLAMP) {
+    const float g = fminf(gate, act.x), u = fminf(fmaxf(up, -act.x), act.x);
+    return __fdividef(g, 1.f + __expf(-1.702f * g)) * (u + 1.f);
+  }
+  return gelu_tanh_unit(gate) * up;
+}
+
 // streaming 128-bit load that does not pollute L1 (weights / KV are read once)
 __device__ __forceinline__ uint4 ldg_stream(const void* p) {
   uint4 r;

@@ -1,24 +1,19 @@
-// Dense 16-bit GEMM on tcgen05: y[M,N] = x[M,K] . w[N,K]^T (+ batch), both operands in shared memory, accumulators in TMEM.
+// Dense 16-bit GEMM on tcgen05: y[M,N] = x[M,K] . w[N,K]^T (+ batch, or grouped), both operands in shared memory, accumulators in TMEM.
 //
-//   A = x tile  [128 tokens x 64 k]  K-major, SWIZZLE_128B, filled by TMA          (the M side of the MMA)
-//   B = w tile  [BN rows    x 64 k]  K-major, SWIZZLE_128B, filled by TMA          (the N side; BN = 256, 128 or 64)
-//   D = [128 x BN] fp32 in TMEM, two buffers: the epilogue of one tile overlaps the main loop of the next
+// Two kernels, both with the WEIGHTS on the MMA's M side and the tokens on the N side: the accumulator holds y transposed (lane = output
+// column, TMEM column = token) and the epilogue stores it back transposed, a warp writing 32 consecutive outputs of one token.  Both are
+// persistent (CTA or pair c takes tiles c, c + grid, ...) with two accumulators, so that the epilogue of one tile overlaps the main
+// loop of the next.
 //
-// Persistent: CTA c takes tiles c, c + grid, ...; tiles are numbered with the token tile fastest, so the CTAs that run at the
-// same time share one weight tile through L2 and the activations (a few tens of MB) stay L2-resident across weight tiles.
-//
-// warp roles (192 threads):
-//   warp 0      TMA producer: x and w tiles of one 64-wide k-block per ring stage (3-d tensor maps: k, row, batch index)
-//   warp 1      MMA issuer (one elected lane): four tcgen05.mma (M=128, N=BN, K=16) per stage, tcgen05.commit frees the
-//               stage; owns the TMEM allocation
-//   warps 2..5  epilogue: tcgen05.ld (thread = token row, 32 columns at a time) -> store / store fp32 / clamped gated unit
-//
-// Decode batches (17..64 tokens) swap the operands: the weight tile is the 128-row M side, the tokens are the narrow N side
-// (BN = 32 or 64), because the MMA reads all 128 rows of its A operand from shared memory whatever they hold, and with the
-// tokens there that read (not HBM) bounded the weight stream.  The accumulator then holds y transposed (lane = output column,
-// TMEM column = token) and the epilogue stores it back transposed, a warp writing 32 consecutive outputs of one token.  Where
+// gemm_tc_kernel, up to 64 tokens (decode batches): a CTA takes 128 weight rows against 32 or 64 tokens.  (With the tokens on the M side the
+// MMA would read 128 rows of them from shared memory whatever they hold, and that read, not HBM, bounded the weight stream.)  Where
 // the weight matrix has too few 128-row tiles to fill the GPU (narrow outputs with long K), K is split over several CTAs that
 // add their partial sums into the zeroed fp32 output with red.global.add.
+//   warp 0      TMA producer: w and x tiles of one 64-wide k-block per ring stage (3-d tensor maps: k, row, batch index), K-major, SWIZZLE_128B
+//   warp 1      MMA issuer: four tcgen05.mma (M=128, N=BN, K=16) per stage, tcgen05.commit frees the stage; owns the TMEM allocation
+//   warps 2..5  epilogue: tcgen05.ld (thread = output column, 32 tokens at a time) -> store / store fp32 / gated unit
+//
+// gemm_tc_pair_kernel, prompts: two CTAs on one tile (below).
 //
 // Rows, columns and k outside the tensors are zero-filled by the TMA unit and masked in the epilogue.  Every mbarrier wait is
 // bounded: a wait that runs out raises a device flag (reported by the next launch) and the CTA leaves through the common exit,
@@ -33,17 +28,17 @@
 namespace b200p {
 
 int sm_count();
+bool pdl_enabled_gemm();
 
-constexpr int GT_BM = 128, GT_BK = 64, GT_THREADS = 192, GT_EPI_WARP0 = 2;
+constexpr int GT_BM = 128, GT_BK = 64, GT_THREADS = 192;
 constexpr int GT_A_BYTES = GT_BM * GT_BK * 2;
 
 struct GemmTcParams {
   void* y;
-  int64_t M, N, K, ldy, sy;
-  int tiles_m, tiles_n, num_tiles, num_kb;
-  int splits, kb_per_split;      // K split over `splits` CTAs per output tile (transposed fp32 store only)
-  int trans;                     // operands swapped: accumulator row = output column, accumulator column = token
-  int epi, vec_ok;
+  int64_t R, tokens, ldy, sy;    // output columns (weight rows); tokens (of the largest group)
+  int tiles_r, tiles_t, num_tiles, num_kb;
+  int splits, kb_per_split;      // K split over `splits` CTAs per output tile (fp32 store only)
+  int epi;
   float2 act;
   // grouped products: batch index z owns the rows [seg[z], seg[z+1]) of x and y; seg (device, groups + 1 offsets) is copied to shared
   // memory first, every CTA counts the groups' tiles there
@@ -65,99 +60,24 @@ __device__ __forceinline__ void umma_f16_ss(uint32_t d_tmem, uint64_t a_desc, ui
       : "memory");
 }
 
-template <typename T> __device__ __forceinline__ uint32_t pack2(float a, float b);
-template <> __device__ __forceinline__ uint32_t pack2<__half>(float a, float b) {
-  const __half2 h = __floats2half2_rn(a, b);
-  return *reinterpret_cast<const uint32_t*>(&h);
-}
-template <> __device__ __forceinline__ uint32_t pack2<__nv_bfloat16>(float a, float b) {
-  const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
-  return *reinterpret_cast<const uint32_t*>(&h);
-}
-
-// 32 consecutive accumulator columns of one token row -> y
+// This thread owns output column `n` (a weight row) and holds it for 32 consecutive tokens from `tok0`, of those below `tokens`.
+// Gate / up pairs sit in neighbouring lanes.
 template <typename T>
-__device__ __forceinline__ void gemm_tc_store32(const GemmTcParams& p, int64_t row_off, int64_t n0, const float (&v)[32]) {
-  if (p.epi == B200P_GEMM_CAP_F32) {
-    float* dst = reinterpret_cast<float*>(p.y) + row_off + n0;
-#pragma unroll
-    for (int i = 0; i < 32; ++i)
-      if (n0 + i < p.N) dst[i] = gemm_f32_act(v[i], p.epi, p.act);
-  } else if (p.epi == B200P_GEMM_STORE_F32) {
-    float* dst = reinterpret_cast<float*>(p.y) + row_off + n0;
-    if (p.vec_ok && n0 + 32 <= p.N) {
-#pragma unroll
-      for (int i = 0; i < 32; i += 4) *reinterpret_cast<float4*>(dst + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
-    } else {
-#pragma unroll
-      for (int i = 0; i < 32; ++i)
-        if (n0 + i < p.N) dst[i] = v[i];
-    }
-  } else if (!gemm_epi_is_glu(p.epi)) {
-    float a[32];
-#pragma unroll
-    for (int i = 0; i < 32; ++i) a[i] = v[i];
-    if (p.epi == B200P_GEMM_XIELU) {               // one uniform branch for all elements
-#pragma unroll
-      for (int i = 0; i < 32; ++i) a[i] = xielu_unit(v[i], p.act);
-    } else if (p.epi != B200P_GEMM_STORE) {
-#pragma unroll
-      for (int i = 0; i < 32; ++i) a[i] = gemm_store_act(v[i], p.epi, p.act);
-    }
-    T* dst = reinterpret_cast<T*>(p.y) + row_off + n0;
-    if (p.vec_ok && n0 + 32 <= p.N) {
-#pragma unroll
-      for (int i = 0; i < 32; i += 8) {
-        uint4 u;
-        u.x = pack2<T>(a[i], a[i + 1]);
-        u.y = pack2<T>(a[i + 2], a[i + 3]);
-        u.z = pack2<T>(a[i + 4], a[i + 5]);
-        u.w = pack2<T>(a[i + 6], a[i + 7]);
-        *reinterpret_cast<uint4*>(dst + i) = u;
-      }
-    } else {
-#pragma unroll
-      for (int i = 0; i < 32; ++i)
-        if (n0 + i < p.N) dst[i] = Tr<T>::from_f(a[i]);
-    }
-  } else {  // gated units: columns 2i / 2i+1 are gate_i / up_i
-    float a[16];
-#pragma unroll
-    for (int i = 0; i < 16; ++i) a[i] = glu_unit(v[2 * i], v[2 * i + 1], p.epi, p.act);
-    T* dst = reinterpret_cast<T*>(p.y) + row_off + (n0 >> 1);
-    if (p.vec_ok && n0 + 32 <= p.N) {
-#pragma unroll
-      for (int i = 0; i < 16; i += 8) {
-        uint4 u;
-        u.x = pack2<T>(a[i], a[i + 1]);
-        u.y = pack2<T>(a[i + 2], a[i + 3]);
-        u.z = pack2<T>(a[i + 4], a[i + 5]);
-        u.w = pack2<T>(a[i + 6], a[i + 7]);
-        *reinterpret_cast<uint4*>(dst + i) = u;
-      }
-    } else {
-#pragma unroll
-      for (int i = 0; i < 16; ++i)
-        if (n0 + 2 * i + 1 < p.N) dst[i] = Tr<T>::from_f(a[i]);
-    }
-  }
-}
-
-// Swapped operands: this thread owns output column `n` (a weight row) and holds it for 32 consecutive tokens from `tok0`.
-// p.M counts output columns here; `tokens` of this batch index (group) exist.  Gate / up pairs sit in neighbouring lanes.
-template <typename T>
-__device__ __forceinline__ void gemm_tc_store32_trans(const GemmTcParams& p, int64_t z_off, int64_t n, int64_t tok0, int64_t tokens,
+__device__ __forceinline__ void gemm_tc_store32(const GemmTcParams& p, int64_t z_off, int64_t n, int64_t tok0, int64_t tokens,
                                                       const float (&v)[32]) {
   if (gemm_epi_is_glu(p.epi)) {
+    // the even lane of a pair holds the gate, the odd one the up row: the former finishes even tokens, the latter odd ones
+    const bool odd = (threadIdx.x & 1) != 0;
+    T* dst = reinterpret_cast<T*>(p.y) + z_off + (tok0 + odd) * p.ldy + (n >> 1);
 #pragma unroll
-    for (int i = 0; i < 32; ++i) {
-      const float other = __shfl_xor_sync(0xffffffffu, v[i], 1);
-      if (!(threadIdx.x & 1) && n + 1 < p.M && tok0 + i < tokens)
-        reinterpret_cast<T*>(p.y)[z_off + (tok0 + i) * p.ldy + (n >> 1)] = Tr<T>::from_f(glu_unit(v[i], other, p.epi, p.act));
+    for (int i = 0; i < 32; i += 2) {
+      const float other = __shfl_xor_sync(0xffffffffu, odd ? v[i] : v[i + 1], 1);
+      if ((n | 1) < p.R && tok0 + i + odd < tokens)
+        dst[i * p.ldy] = Tr<T>::from_f(glu_unit16(odd ? other : v[i], odd ? v[i + 1] : other, p.epi, p.act));
     }
     return;
   }
-  if (n >= p.M) return;
+  if (n >= p.R) return;
   if (p.epi == B200P_GEMM_STORE_F32) {
     float* dst = reinterpret_cast<float*>(p.y) + z_off + n;
     if (p.splits > 1) {
@@ -176,9 +96,17 @@ __device__ __forceinline__ void gemm_tc_store32_trans(const GemmTcParams& p, int
       if (tok0 + i < tokens) dst[(tok0 + i) * p.ldy] = gemm_f32_act(v[i], p.epi, p.act);
   } else {
     T* dst = reinterpret_cast<T*>(p.y) + z_off + n;
+    float a[32];                                   // one uniform branch for all elements
+    if (p.epi == B200P_GEMM_XIELU) {
+#pragma unroll
+      for (int i = 0; i < 32; ++i) a[i] = xielu_unit(v[i], p.act);
+    } else {
+#pragma unroll
+      for (int i = 0; i < 32; ++i) a[i] = p.epi == B200P_GEMM_RELU_SQ ? gemm_store_act(v[i], B200P_GEMM_RELU_SQ, p.act) : v[i];
+    }
 #pragma unroll
     for (int i = 0; i < 32; ++i)
-      if (tok0 + i < tokens) dst[(tok0 + i) * p.ldy] = Tr<T>::from_f(gemm_store_act(v[i], p.epi, p.act));
+      if (tok0 + i < tokens) dst[(tok0 + i) * p.ldy] = Tr<T>::from_f(a[i]);
   }
 }
 
@@ -187,39 +115,29 @@ struct GemmTcShared {            // lives behind the ring stages (8-byte aligned
   uint32_t tmem_base;
   volatile int abort;
   int seg[GT_MAX_GROUPS + 1];
-  int live[GT_MAX_GROUPS + 1];   // grouped prompts: row tiles of all groups before this one that hold rows
+  int live[GT_MAX_GROUPS + 1];   // grouped products: row tiles of all groups before this one that hold rows
 };
 
-// Tile t of the launch: batch index (group) z, tile column nt, tile row mt; first row of the group in x / y and how many rows it has.
-// Grouped products number only the tiles that hold rows (with swapped operands: the tiles of groups that have any), so that the CTAs
-// share them evenly whatever the routing; numbering max_rows rows for every group and skipping left a CTA 8 to 15 live tiles of 12000 x
-// 4096 (16 groups) where 10.4 is the mean.
-struct GemmTcTile { int z, nt, mt, first, len; };
-__device__ __forceinline__ int gemm_tc_num_tiles(const GemmTcParams& p, const GemmTcShared* sh) {
-  return p.seg ? sh->live[p.groups] * (p.trans ? 1 : p.tiles_n) : p.num_tiles;
-}
+// Tile t of the launch: batch index (group) z, row tile rt; first token of the group in x / y and how many it has.  Grouped products
+// number only the tiles of groups that hold tokens, so that the CTAs share them evenly whatever the routing.
+struct GemmTcTile { int z, rt, first, len; };
 __device__ __forceinline__ GemmTcTile gemm_tc_tile(const GemmTcParams& p, const GemmTcShared* sh, int t) {
   GemmTcTile r;
   if (!p.seg) {
-    const int ts = t / p.splits, per_batch = p.tiles_m * p.tiles_n;
-    r.z = ts / per_batch;
-    const int in = ts - r.z * per_batch;
-    r.nt = in / p.tiles_m;
-    r.mt = in - r.nt * p.tiles_m;
+    const int ts = t / p.splits;
+    r.z = ts / p.tiles_r;
+    r.rt = ts - r.z * p.tiles_r;
     r.first = 0;
-    r.len = p.trans ? (int)p.N : (int)p.M;
+    r.len = (int)p.tokens;
     return r;
   }
-  const int width = p.trans ? 1 : p.tiles_n;
-  int lo = 0, hi = p.groups - 1;                  // last group z with live[z] * width <= t (groups without tiles share their start)
+  int lo = 0, hi = p.groups - 1;                  // last group z with live[z] <= t (groups without tiles share their start)
   while (lo < hi) {
     const int mid = (lo + hi + 1) >> 1;
-    if (sh->live[mid] * width <= t) lo = mid; else hi = mid - 1;
+    if (sh->live[mid] <= t) lo = mid; else hi = mid - 1;
   }
   r.z = lo;
-  const int in = t - sh->live[lo] * width, rows = sh->live[lo + 1] - sh->live[lo];
-  r.nt = p.trans ? 0 : in / rows;
-  r.mt = in - r.nt * rows;
+  r.rt = t - sh->live[lo];
   r.first = sh->seg[lo];
   r.len = sh->seg[lo + 1] - r.first;
   return r;
@@ -227,10 +145,10 @@ __device__ __forceinline__ GemmTcTile gemm_tc_tile(const GemmTcParams& p, const 
 
 template <typename T, int BN, int STAGES>
 __global__ void __launch_bounds__(GT_THREADS, 1)
-gemm_tc_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constant__ CUtensorMap tmw, const GemmTcParams p) {
+gemm_tc_kernel(const __grid_constant__ CUtensorMap tmw, const __grid_constant__ CUtensorMap tmx, const GemmTcParams p) {
   constexpr int B_BYTES = BN * GT_BK * 2, STAGE_BYTES = GT_A_BYTES + B_BYTES;
-  constexpr uint32_t TMEM_COLS = 2 * BN;           // 64 .. 512: a power of two >= 32
-  static_assert(STAGES <= 10 && (BN == 32 || BN == 64 || BN == 128 || BN == 256), "ring / tile shape");
+  constexpr uint32_t TMEM_COLS = 2 * BN;           // 64 or 128: a power of two >= 32
+  static_assert(STAGES <= 10 && (BN == 32 || BN == 64), "ring / tile shape");
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;    // SWIZZLE_128B tiles start on 1024-byte boundaries
@@ -261,7 +179,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constant__ 
       int run = 0;
       for (int z0 = 0; z0 < p.groups; z0 += 32) {
         const int z = z0 + lane, len = z < p.groups ? sh->seg[z + 1] - sh->seg[z] : 0;
-        const int mine = p.trans ? (len > 0 ? p.tiles_m : 0) : (len + GT_BM - 1) / GT_BM;
+        const int mine = len > 0 ? p.tiles_r : 0;
         int sum = mine;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -278,60 +196,56 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constant__ 
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = sh->tmem_base;
-  const int num_tiles = gemm_tc_num_tiles(p, sh);
+  const int num_tiles = p.seg ? sh->live[p.groups] : p.num_tiles;
 
+  // (whole warps walk the loops and one elected lane issues: operands of warp-uniform code need no uniformising)
   if (warp == 0) {
-    if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0;
-      bool ok = true;
-      for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
-        const int kb0 = (t % p.splits) * p.kb_per_split, kb1 = min(p.num_kb, kb0 + p.kb_per_split);
-        const GemmTcTile tl = gemm_tc_tile(p, sh, t);
-        const int z = tl.z, nt = tl.nt, mt = tl.mt, first = tl.first;
-        for (int kb = kb0; kb < kb1; ++kb) {
-          if (!(ok = mbar_wait_lane(smem_u32(&sh->empty[stage]), phase ^ 1u, &sh->abort, p.wait_word, 0))) break;
+    int stage = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
+      const int kb0 = (t % p.splits) * p.kb_per_split, kb1 = min(p.num_kb, kb0 + p.kb_per_split);
+      const GemmTcTile tl = gemm_tc_tile(p, sh, t);
+      for (int kb = kb0; kb < kb1; ++kb) {
+        if (!(ok = mbar_wait_warp(smem_u32(&sh->empty[stage]), phase ^ 1u, &sh->abort, p.wait_word, 0))) break;
+        if (elect_one()) {
           const uint32_t bar = smem_u32(&sh->full[stage]);
           const uint32_t dst = base + stage * STAGE_BYTES;
           mbar_arrive_expect_tx(bar, STAGE_BYTES);
-          if (p.trans) {                            // A = weights, B = tokens
-            tma_load_3d(dst, &tmx, kb * GT_BK, mt * GT_BM, z, bar);
-            tma_load_3d(dst + GT_A_BYTES, &tmw, kb * GT_BK, first + nt * BN, p.seg ? 0 : z, bar);
-          } else {
-            tma_load_3d(dst, &tmx, kb * GT_BK, first + mt * GT_BM, p.seg ? 0 : z, bar);
-            tma_load_3d(dst + GT_A_BYTES, &tmw, kb * GT_BK, nt * BN, z, bar);
-          }
-          if (++stage == STAGES) { stage = 0; phase ^= 1u; }
+          tma_load_3d(dst, &tmw, kb * GT_BK, tl.rt * GT_BM, tl.z, bar);
+          tma_load_3d(dst + GT_A_BYTES, &tmx, kb * GT_BK, tl.first, p.seg ? 0 : tl.z, bar);
         }
+        __syncwarp();
+        if (++stage == STAGES) { stage = 0; phase ^= 1u; }
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t fmt = std::is_same<T, __nv_bfloat16>::value ? 1u : 0u;
-      constexpr uint32_t idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(GT_BM >> 4) << 24);
-      int stage = 0, acc = 0;
-      uint32_t phase = 0, acc_phase = 0;
-      bool ok = true;
-      for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
-        if (!(ok = mbar_wait_lane(smem_u32(&sh->acc_empty[acc]), acc_phase ^ 1u, &sh->abort, p.wait_word, 1))) break;
+    constexpr uint32_t fmt = std::is_same<T, __nv_bfloat16>::value ? 1u : 0u;
+    constexpr uint32_t idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(GT_BM >> 4) << 24);
+    int stage = 0, acc = 0;
+    uint32_t phase = 0, acc_phase = 0;
+    bool ok = true;
+    for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
+      if (!(ok = mbar_wait_warp(smem_u32(&sh->acc_empty[acc]), acc_phase ^ 1u, &sh->abort, p.wait_word, 1))) break;
+      tc_fence_after();
+      const uint32_t d = tmem_base + (uint32_t)(acc * BN);
+      const int kb0 = (t % p.splits) * p.kb_per_split, kb1 = min(p.num_kb, kb0 + p.kb_per_split);
+      for (int kb = kb0; kb < kb1; ++kb) {
+        if (!(ok = mbar_wait_warp(smem_u32(&sh->full[stage]), phase, &sh->abort, p.wait_word, 1))) break;
         tc_fence_after();
-        const uint32_t d = tmem_base + (uint32_t)(acc * BN);
-        const int kb0 = (t % p.splits) * p.kb_per_split, kb1 = min(p.num_kb, kb0 + p.kb_per_split);
-        for (int kb = kb0; kb < kb1; ++kb) {
-          if (!(ok = mbar_wait_lane(smem_u32(&sh->full[stage]), phase, &sh->abort, p.wait_word, 1))) break;
-          tc_fence_after();
+        if (elect_one()) {
           const uint64_t ad = make_desc_sw128(base + stage * STAGE_BYTES);
           const uint64_t bd = make_desc_sw128(base + stage * STAGE_BYTES + GT_A_BYTES);
 #pragma unroll
-          for (int k = 0; k < GT_BK / 16; ++k)     // 16 k = 32 bytes = 2 descriptor units inside the swizzle atom
+          for (int k = 0; k < GT_BK / 16; ++k)       // 16 k = 32 bytes = 2 descriptor units inside the swizzle atom
             umma_f16_ss(d, ad + 2u * k, bd + 2u * k, idesc, ((kb - kb0) | k) ? 1u : 0u);
           umma_commit(smem_u32(&sh->empty[stage]));
-          if (++stage == STAGES) { stage = 0; phase ^= 1u; }
+          if (kb == kb1 - 1) umma_commit(smem_u32(&sh->acc_full[acc]));
         }
-        if (!ok) break;
-        umma_commit(smem_u32(&sh->acc_full[acc]));
-        if (++acc == 2) { acc = 0; acc_phase ^= 1u; }
+        __syncwarp();
+        if (++stage == STAGES) { stage = 0; phase ^= 1u; }
       }
+      if (++acc == 2) { acc = 0; acc_phase ^= 1u; }
     }
   } else {
     const int lg = warp & 3;                       // the TMEM lane quarter this warp may read
@@ -339,22 +253,19 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constant__ 
     uint32_t acc_phase = 0;
     for (int t = blockIdx.x; t < num_tiles; t += gridDim.x) {
       const GemmTcTile tl = gemm_tc_tile(p, sh, t);
-      const int z = tl.z, nt = tl.nt, mt = tl.mt, first = tl.first, len = tl.len;
       if (!mbar_wait_warp(smem_u32(&sh->acc_full[acc]), acc_phase, &sh->abort, p.wait_word, 2)) break;
       tc_fence_after();
-      const int64_t row = (int64_t)mt * GT_BM + lg * 32 + lane;               // within the batch index's (group's) rows
-      const int64_t row_off = p.seg ? (first + row) * p.ldy : (int64_t)z * p.sy + row * p.ldy;
+      const int64_t n = (int64_t)tl.rt * GT_BM + lg * 32 + lane;              // output column
+      const int64_t z_off = p.seg ? tl.first * p.ldy : (int64_t)tl.z * p.sy;
       const uint32_t tsrc = tmem_base + ((uint32_t)(lg * 32) << 16) + (uint32_t)(acc * BN);
 #pragma unroll 1
       for (int c = 0; c < BN; c += 32) {
-        const int64_t n0 = (int64_t)nt * BN + c;
-        if (n0 >= p.N) break;                      // warp-uniform
+        if (c >= p.tokens) break;                  // warp-uniform
         float v[32];
         tmem_ld16(tsrc + c, *reinterpret_cast<float(*)[16]>(&v[0]));
         tmem_ld16(tsrc + c + 16, *reinterpret_cast<float(*)[16]>(&v[16]));
         tmem_ld_wait();
-        if (p.trans) gemm_tc_store32_trans<T>(p, p.seg ? first * p.ldy : (int64_t)z * p.sy, row, n0, len, v);
-        else if (row < len) gemm_tc_store32<T>(p, row_off, n0, v);
+        gemm_tc_store32<T>(p, z_off, n, c, tl.len, v);
       }
       tc_fence_before();
       __syncwarp();
@@ -370,6 +281,265 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constant__ 
     tmem_dealloc(tmem_base, TMEM_COLS);
   }
 }
+
+// ---------------------------------------------------------------------------------------------------------------- two CTAs on one tile
+// Prompts.  A pair of CTAs (a cluster of two, neighbouring SMs) computes 256 weight rows x up to 256 tokens with tcgen05.mma.cta_group::2:
+//
+//   A = w tile  [256 rows   x 64 k], CTA r stages rows [128 r, 128 r + 128)        (the M side; accumulator lane = output column)
+//   B = x tile  [tn tokens  x 64 k], CTA r stages tokens [r tn / 2, (r + 1) tn / 2)  (the N side; accumulator column = token)
+//   D = CTA r: its 128 rows x tn fp32 in its own TMEM, two buffers
+//
+// One CTA per tile is bounded by operand traffic: 128 x 256 x 64 k are 48 KB through L2 for 512 tensor cycles.  A CTA of a pair fetches 32 KB
+// for the same cycles and each operand byte serves both (bf16, fp32 store, us, one CTA / pair: 6000 x 8192 x 2048 179 / 146, 1664 x 2048 x
+// 2048 31 / 17, 1024 x 4096 x 3584 67 / 31, 200 x 7168 x 4096 37 / 22, 65 x 2048 x 4096 20.7 / 18.8; 16 groups of 375 rows, gated, 4096 x
+// 2048, 77 / 74, of 125 rows 65 / 55; 1.3 to 1.4 PFLOP/s at the large end).  Weights are the M side because the N side may be any multiple of 32 tokens: row counts that fill no 128 or 256 rows (an
+// expert's share of a prompt, a portion) are cut evenly, and the host narrows the tile where that fills the last wave.  The stores of a warp
+// are then runs of 32 neighbouring outputs of one token.
+//
+// warp 0: TMA of its CTA's halves (completion counted on the leader's barriers); warp 1 of the leader: MMA issue, commits go to both
+// CTAs; warps 2..9: epilogue, two per lane quarter, alternate pieces of 32 tokens.
+namespace pair {
+
+constexpr int EPI_WARPS = 8, THREADS = 64 + 32 * EPI_WARPS, STAGES = 6, MAX_TN = 256, TN_STEP = 32;
+constexpr int A_BYTES = 128 * GT_BK * 2, B_BYTES = MAX_TN / 2 * GT_BK * 2, STAGE_BYTES = A_BYTES + B_BYTES;
+
+struct Params {
+  GemmTcParams g;
+  int tn;                        // tokens per tile (plain products; a group's own are cut evenly)
+  int box;                       // tokens per TMA box
+};
+struct Shared {
+  uint64_t full[STAGES], empty[STAGES], acc_full[2], acc_empty[2];
+  uint32_t tmem_base;
+  volatile int abort;
+  int seg[GT_MAX_GROUPS + 1], live[GT_MAX_GROUPS + 1];       // group offsets; token tiles of all groups before this one
+};
+
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t map_to_leader(uint32_t addr) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(addr));
+  return r;
+}
+__device__ __forceinline__ void arrive_cluster(uint32_t addr) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(addr) : "memory");
+}
+// this CTA's tile part, its bytes counted on a barrier of either CTA of the pair
+__device__ __forceinline__ void load_3d(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(dst),
+      "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(bar)
+      : "memory");
+}
+__device__ __forceinline__ void umma_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accum) {
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "setp.ne.b32 p, %4, 0;\n"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n"
+      "}\n" ::"r"(d_tmem),
+      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accum)
+      : "memory");
+}
+__device__ __forceinline__ void commit_pair(uint32_t bar) {  // arrives at this offset in both CTAs
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"((uint16_t)3)
+               : "memory");
+}
+
+// token tiles of a group of `len` tokens and their width
+__device__ __forceinline__ int even_tn(int len) {
+  const int nt = (len + MAX_TN - 1) / MAX_TN;
+  return nt == 0 ? TN_STEP : ((len + nt - 1) / nt + TN_STEP - 1) / TN_STEP * TN_STEP;
+}
+
+struct Tile { int z, rt, tok0, first, len, tn; };            // batch index (group), row tile, first token within it, ...
+__device__ __forceinline__ Tile tile_of(const Params& p, const Shared* sh, int t) {
+  Tile r;
+  int in, nt;
+  if (!p.g.seg) {
+    nt = p.g.tiles_t;
+    const int per = p.g.tiles_r * nt;
+    r.z = t / per;
+    in = t - r.z * per;
+    r.first = 0;
+    r.len = (int)p.g.tokens;
+    r.tn = p.tn;
+  } else {
+    int lo = 0, hi = p.g.groups - 1;                         // last group with live * tiles_r <= t
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if (sh->live[mid] * p.g.tiles_r <= t) lo = mid; else hi = mid - 1;
+    }
+    r.z = lo;
+    nt = sh->live[lo + 1] - sh->live[lo];
+    in = t - sh->live[lo] * p.g.tiles_r;
+    r.first = sh->seg[lo];
+    r.len = sh->seg[lo + 1] - r.first;
+    r.tn = even_tn(r.len);
+  }
+  r.rt = in / nt;                                            // token tile fastest: pairs that run together share weights
+  r.tok0 = (in - r.rt * nt) * r.tn;
+  return r;
+}
+
+template <typename T>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
+gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmw, const __grid_constant__ CUtensorMap tmx, const Params p) {
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t raw = smem_u32(smem_raw);
+  const uint32_t base = (raw + 1023u) & ~1023u;              // the same offset in both CTAs
+  Shared* sh = reinterpret_cast<Shared*>(smem_raw + (base - raw) + STAGES * STAGE_BYTES);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t rank = cluster_rank();
+  const int pair0 = (int)(blockIdx.x >> 1), pairs = (int)(gridDim.x >> 1);
+  int* word = p.g.wait_word;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < STAGES; ++s) {
+      mbar_init(smem_u32(&sh->full[s]), 1);                  // used in the leader
+      mbar_init(smem_u32(&sh->empty[s]), 1);
+    }
+    for (int a = 0; a < 2; ++a) {
+      mbar_init(smem_u32(&sh->acc_full[a]), 1);
+      mbar_init(smem_u32(&sh->acc_empty[a]), 2 * EPI_WARPS); // used in the leader: the epilogue warps of both CTAs
+    }
+    sh->abort = 0;
+    fence_barrier_init();
+    tma_prefetch_desc(&tmw);
+    tma_prefetch_desc(&tmx);
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&sh->tmem_base)), "r"(512u) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+  }
+  pdl_launch_dependents();
+  pdl_wait();                                                // x, seg and y belong to the previous kernels until here
+  if (p.g.seg) {
+    for (int i = threadIdx.x; i <= p.g.groups; i += THREADS) sh->seg[i] = p.g.seg[i];
+    __syncthreads();
+    if (warp == 2) {                                         // running count of the groups' token tiles
+      int run = 0;
+      for (int z0 = 0; z0 < p.g.groups; z0 += 32) {
+        const int z = z0 + lane, len = z < p.g.groups ? sh->seg[z + 1] - sh->seg[z] : 0, tn = even_tn(len);
+        const int mine = (len + tn - 1) / tn;
+        int sum = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int v = __shfl_up_sync(0xffffffffu, sum, o);
+          if (lane >= o) sum += v;
+        }
+        if (z < p.g.groups) sh->live[z] = run + sum - mine;
+        run += __shfl_sync(0xffffffffu, sum, 31);
+      }
+      if (lane == 0) sh->live[p.g.groups] = run;
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync();                                            // both CTAs' barriers exist
+  tc_fence_after();
+  const uint32_t tmem_base = sh->tmem_base;
+  const int num_tiles = p.g.seg ? sh->live[p.g.groups] * p.g.tiles_r : p.g.num_tiles;
+
+  // (whole warps walk the loops and one elected lane issues: operands of warp-uniform code need no uniformising)
+  if (warp == 0) {
+    int stage = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    for (int t = pair0; t < num_tiles && ok; t += pairs) {
+      const Tile tl = tile_of(p, sh, t);
+      const int half = tl.tn / 2, boxes = (half + p.box - 1) / p.box;
+      const int row = tl.rt * 256 + (int)rank * 128, tok = tl.first + tl.tok0 + (int)rank * half, zx = p.g.seg ? 0 : tl.z;
+      const uint32_t box_bytes = (uint32_t)p.box * GT_BK * 2, bytes = 2u * (uint32_t)(A_BYTES + boxes * box_bytes);
+      for (int kb = 0; kb < p.g.num_kb; ++kb) {
+        if (!(ok = mbar_wait_warp(smem_u32(&sh->empty[stage]), phase ^ 1u, &sh->abort, word, 0))) break;
+        if (elect_one()) {
+          const uint32_t bar = map_to_leader(smem_u32(&sh->full[stage])), dst = base + stage * STAGE_BYTES;
+          if (rank == 0) mbar_arrive_expect_tx(smem_u32(&sh->full[stage]), bytes);
+          load_3d(dst, &tmw, kb * GT_BK, row, tl.z, bar);
+          for (int b = 0; b < boxes; ++b) load_3d(dst + A_BYTES + b * box_bytes, &tmx, kb * GT_BK, tok + b * p.box, zx, bar);
+        }
+        __syncwarp();
+        if (++stage == STAGES) { stage = 0; phase ^= 1u; }
+      }
+    }
+    // the pair's last commits have arrived here before this CTA may leave
+    for (int s = 0; s < STAGES && ok; ++s) {
+      ok = mbar_wait_warp(smem_u32(&sh->empty[stage]), phase ^ 1u, &sh->abort, word, 0);
+      if (++stage == STAGES) { stage = 0; phase ^= 1u; }
+    }
+  } else if (warp == 1) {
+    if (rank == 0) {
+      constexpr uint32_t fmt = std::is_same<T, __nv_bfloat16>::value ? 1u : 0u;
+      int stage = 0, acc = 0;
+      uint32_t phase = 0, acc_phase = 0;
+      bool ok = true;
+      for (int t = pair0; t < num_tiles && ok; t += pairs) {
+        const int tn = p.g.seg ? tile_of(p, sh, t).tn : p.tn;
+        const uint32_t idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(tn >> 3) << 17) | ((256u >> 4) << 24);
+        if (!(ok = mbar_wait_warp(smem_u32(&sh->acc_empty[acc]), acc_phase ^ 1u, &sh->abort, word, 1))) break;
+        tc_fence_after();
+        const uint32_t d = tmem_base + (uint32_t)(acc * MAX_TN);
+        for (int kb = 0; kb < p.g.num_kb; ++kb) {
+          if (!(ok = mbar_wait_warp(smem_u32(&sh->full[stage]), phase, &sh->abort, word, 1))) break;
+          tc_fence_after();
+          if (elect_one()) {
+            const uint64_t ad = make_desc_sw128(base + stage * STAGE_BYTES), bd = make_desc_sw128(base + stage * STAGE_BYTES + A_BYTES);
+#pragma unroll
+            for (int k = 0; k < GT_BK / 16; ++k) umma_pair(d, ad + 2u * k, bd + 2u * k, idesc, (kb | k) ? 1u : 0u);
+            commit_pair(smem_u32(&sh->empty[stage]));
+            if (kb == p.g.num_kb - 1) commit_pair(smem_u32(&sh->acc_full[acc]));
+          }
+          __syncwarp();
+          if (++stage == STAGES) { stage = 0; phase ^= 1u; }
+        }
+        if (++acc == 2) { acc = 0; acc_phase ^= 1u; }
+      }
+    }
+  } else {
+    const int lg = warp & 3, part = (warp - 2) >> 2;         // TMEM lane quarter; which pieces of 32 tokens
+    int acc = 0;
+    uint32_t acc_phase = 0;
+    for (int t = pair0; t < num_tiles; t += pairs) {
+      const Tile tl = tile_of(p, sh, t);
+      if (!mbar_wait_warp(smem_u32(&sh->acc_full[acc]), acc_phase, &sh->abort, word, 2)) break;
+      tc_fence_after();
+      const int64_t n = (int64_t)tl.rt * 256 + rank * 128 + lg * 32 + lane;
+      const int64_t z_off = p.g.seg ? (int64_t)tl.first * p.g.ldy : (int64_t)tl.z * p.g.sy;
+      const uint32_t src = tmem_base + ((uint32_t)(lg * 32) << 16) + (uint32_t)(acc * MAX_TN);
+      const int most = min(tl.tn, tl.len - tl.tok0);         // tokens of this tile
+#pragma unroll 1
+      for (int c = 32 * part; c < most; c += 64) {
+        float v[32];
+        tmem_ld16(src + c, *reinterpret_cast<float(*)[16]>(&v[0]));
+        tmem_ld16(src + c + 16, *reinterpret_cast<float(*)[16]>(&v[16]));
+        tmem_ld_wait();
+        gemm_tc_store32<T>(p.g, z_off, n, tl.tok0 + c, tl.tok0 + most, v);
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) arrive_cluster(map_to_leader(smem_u32(&sh->acc_empty[acc])));
+      if (++acc == 2) { acc = 0; acc_phase ^= 1u; }
+    }
+  }
+  if (sh->abort) wait_settle();
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync();                                            // neither CTA's memory is read or signalled any more
+  if (warp == 1) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
+  }
+}
+
+}  // namespace pair
 
 // ------------------------------------------------------------------------------------------------ host
 static TcEncodeFn gemm_tc_encode_fn() {
@@ -395,7 +565,7 @@ static bool gemm_tc_map(TcEncodeFn enc, CUtensorMap* tm, CUtensorMapDataType dt,
 }
 
 template <typename T, int BN, int STAGES>
-static int gemm_tc_run(const CUtensorMap& tmx, const CUtensorMap& tmw, GemmTcParams p, cudaStream_t st) {
+static int gemm_tc_run(const CUtensorMap& tmw, const CUtensorMap& tmx, GemmTcParams p, cudaStream_t st) {
   constexpr size_t smem = 1024 + (size_t)STAGES * (GT_A_BYTES + BN * GT_BK * 2) + sizeof(GemmTcShared);
   auto kern = gemm_tc_kernel<T, BN, STAGES>;
   static bool attr_set = false;
@@ -406,10 +576,74 @@ static int gemm_tc_run(const CUtensorMap& tmx, const CUtensorMap& tmw, GemmTcPar
   }
   if (const int rc = wait_word(WAIT_GEMM_TC, &p.wait_word)) return rc;
   const int grid = p.num_tiles < sm_count() ? p.num_tiles : sm_count();
-  kern<<<grid, GT_THREADS, smem, st>>>(tmx, tmw, p);
+  kern<<<grid, GT_THREADS, smem, st>>>(tmw, tmx, p);
   B200P_LAUNCH_CHECK("gemm_tc_kernel");
   return B200P_OK;
 }
+
+namespace pair {
+
+template <typename T>
+static int run(const CUtensorMap& tmw, const CUtensorMap& tmx, Params p, int64_t tiles, cudaStream_t st) {
+  constexpr size_t smem = 1024 + (size_t)STAGES * STAGE_BYTES + sizeof(Shared);
+  auto kern = gemm_tc_pair_kernel<T>;
+  static bool attr_set = false;
+  if (!attr_set) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(gemm_tc_pair_kernel)");
+    attr_set = true;
+  }
+  if (const int rc = wait_word(WAIT_GEMM_TC, &p.g.wait_word)) return rc;
+  const int64_t pairs = sm_count() / 2;
+  const unsigned grid = 2u * (unsigned)(tiles < pairs ? tiles : pairs);
+  cudaError_t e = launch_pdl_opt(pdl_enabled_gemm(), kern, dim3(grid), dim3(THREADS), smem, st, tmw, tmx, p);
+  if (e != cudaSuccess) return cuda_fail(e, "gemm_tc_pair_kernel launch");
+  return B200P_OK;
+}
+
+// Width and number of the token tiles: whole waves of pairs, each as long as the slower of tensor core (2 cycles per token and k-block) and
+// operand fetch (16 KB of weights and half the tokens per CTA, at about 70 bytes per cycle).
+static void plan(int64_t tokens, int64_t R, int64_t batch, int& tn, int64_t& tiles_t) {
+  const int64_t pairs = sm_count() / 2, tiles_r = (R + 255) / 256 * batch, t0 = (tokens + MAX_TN - 1) / MAX_TN, one_wave = pairs / tiles_r;
+  double best = 1e300;
+  for (int64_t i = 0; i <= 9; ++i) {
+    const int64_t n = i < 9 ? t0 + i : one_wave > t0 ? one_wave : t0;
+    const int w = (int)(((tokens + n - 1) / n + TN_STEP - 1) / TN_STEP * TN_STEP);
+    const int64_t nt = (tokens + w - 1) / w, waves = (tiles_r * nt + pairs - 1) / pairs;
+    const double mma = 2.0 * w, fetch = (16384.0 + 64.0 * w) / 70.0, c = (double)waves * (mma > fetch ? mma : fetch);
+    if (c < best * 0.999) { best = c; tn = w; tiles_t = nt; }
+  }
+}
+
+template <typename T>
+static int launch(TcEncodeFn enc, const T* x, const T* w, void* y, const int32_t* seg, int64_t x_rows, int64_t tokens, int tn, int64_t tiles_t, int64_t R,
+                  int64_t K, int64_t ldx, int64_t ldw, int64_t ldy, int64_t batch, int64_t sx, int64_t sw, int64_t sy, int epi, float2 act,
+                  cudaStream_t st) {
+  const CUtensorMapDataType dt = std::is_same<T, __nv_bfloat16>::value ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
+  CUtensorMap tmw, tmx;
+  if (!gemm_tc_map(enc, &tmw, dt, w, K, R, batch, ldw, sw, 128)) return 1;
+  Params p;
+  p.box = seg ? 64 : tn / 2;
+  if (!gemm_tc_map(enc, &tmx, dt, x, K, x_rows, seg ? 1 : batch, ldx, sx, p.box)) return 1;
+  GemmTcParams& g = p.g;
+  g.y = y;
+  g.R = R; g.tokens = tokens; g.ldy = ldy; g.sy = seg ? 0 : sy;
+  g.tiles_r = (int)((R + 255) / 256);
+  g.tiles_t = (int)tiles_t;
+  const int64_t tiles = (int64_t)g.tiles_r * tiles_t * batch;
+  if (tiles >= (1ll << 30)) return 1;
+  g.num_tiles = (int)tiles;
+  g.num_kb = (int)((K + GT_BK - 1) / GT_BK);
+  g.splits = 1; g.kb_per_split = g.num_kb;
+  g.seg = seg;
+  g.groups = seg ? (int)batch : 0;
+  g.epi = epi;
+  g.act = act;
+  p.tn = tn;
+  return run<T>(tmw, tmx, p, tiles, st);
+}
+
+}  // namespace pair
 
 // Up to 64 tokens: weights on the M side, tokens on the N side, transposed store, K split where the output is narrow.
 template <typename T>
@@ -422,11 +656,11 @@ static int gemm_tc_launch_decode(TcEncodeFn enc, const T* x, const T* w, void* y
   if (!gemm_tc_map(enc, &tmb, dt, x, K, M, batch, ldx, sx, bn)) return 1;
   GemmTcParams p;
   p.y = y;
-  p.M = N; p.N = M; p.K = K; p.ldy = ldy; p.sy = sy;
-  p.tiles_m = (int)((N + GT_BM - 1) / GT_BM);
-  p.tiles_n = 1;
+  p.R = N; p.tokens = M; p.ldy = ldy; p.sy = sy;
+  p.tiles_r = (int)((N + GT_BM - 1) / GT_BM);
+  p.tiles_t = 1;
   p.num_kb = (int)((K + GT_BK - 1) / GT_BK);
-  const int64_t tiles = (int64_t)p.tiles_m * batch;
+  const int64_t tiles = (int64_t)p.tiles_r * batch;
   if (tiles >= (1ll << 24)) return 1;
   // few weight tiles and a long K: split K so that about one CTA per SM streams weights, at least 4 k-blocks each
   int splits = 1;
@@ -437,12 +671,10 @@ static int gemm_tc_launch_decode(TcEncodeFn enc, const T* x, const T* w, void* y
   p.kb_per_split = (p.num_kb + splits - 1) / splits;
   p.splits = (p.num_kb + p.kb_per_split - 1) / p.kb_per_split;          // no empty split
   p.num_tiles = (int)(tiles * p.splits);
-  p.trans = 1;
   p.seg = nullptr;
   p.groups = 0;
   p.epi = epi;
   p.act = act;
-  p.vec_ok = 0;
   if (p.splits > 1) {
     cudaError_t e = cudaMemsetAsync(y, 0, (size_t)M * N * sizeof(float), st);
     if (e != cudaSuccess) return cuda_fail(e, "cudaMemsetAsync(split-K output)");
@@ -459,43 +691,16 @@ int gemm_tc_launch(const T* x, const T* w, void* y, int64_t M, int64_t N, int64_
   TcEncodeFn enc = gemm_tc_encode_fn();
   if (!enc) return 1;
   if (M <= 64) return gemm_tc_launch_decode<T>(enc, x, w, y, M, N, K, ldx, ldw, ldy, batch, sx, sw, sy, epi, act, st);
-  const int tiles_m = (int)((M + GT_BM - 1) / GT_BM);
-  // widest weight tile that still gives every SM about two tiles
-  const int64_t want = 2ll * sm_count();
-  int bn = 256;
-  if (N <= 64 || tiles_m * ((N + 127) / 128) * batch < want) bn = 64;
-  else if (N <= 128 || tiles_m * ((N + 255) / 256) * batch < want) bn = 128;
-  const CUtensorMapDataType dt = std::is_same<T, __nv_bfloat16>::value ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
-  CUtensorMap tmx, tmw;
-  if (!gemm_tc_map(enc, &tmx, dt, x, K, M, batch, ldx, sx, GT_BM)) return 1;
-  if (!gemm_tc_map(enc, &tmw, dt, w, K, N, batch, ldw, sw, bn)) return 1;
-  GemmTcParams p;
-  p.y = y;
-  p.M = M; p.N = N; p.K = K; p.ldy = ldy; p.sy = sy;
-  p.tiles_m = tiles_m;
-  p.tiles_n = (int)((N + bn - 1) / bn);
-  const int64_t nt = (int64_t)p.tiles_m * p.tiles_n * batch;
-  if (nt >= (1ll << 31)) return 1;
-  p.num_tiles = (int)nt;
-  p.num_kb = (int)((K + GT_BK - 1) / GT_BK);
-  p.splits = 1;
-  p.kb_per_split = p.num_kb;
-  p.trans = 0;
-  p.seg = nullptr;
-  p.groups = 0;
-  p.epi = epi;
-  p.act = act;
-  const int64_t eb = (epi == B200P_GEMM_STORE_F32 || epi == B200P_GEMM_CAP_F32) ? 4 : 2;
-  p.vec_ok = aligned(y, 16) && (ldy * eb) % 16 == 0 && (sy * eb) % 16 == 0;
-  if (bn == 256) return gemm_tc_run<T, 256, 4>(tmx, tmw, p, st);
-  if (bn == 128) return gemm_tc_run<T, 128, 6>(tmx, tmw, p, st);
-  return gemm_tc_run<T, 64, 8>(tmx, tmw, p, st);
+  int tn = 0;
+  int64_t tiles_t = 0;
+  pair::plan(M, N, batch, tn, tiles_t);
+  return pair::launch<T>(enc, x, w, y, nullptr, M, M, tn, tiles_t, N, K, ldx, ldw, ldy, batch, sx, sw, sy, epi, act, st);
 }
 
 // Grouped product: x [total_rows, K] holds the groups' rows back to back (group z: rows [seg[z], seg[z+1]), at most max_rows of
-// them), w [groups][N][K].  The grid is sized for max_rows rows in every group, the kernel numbers the tiles that exist.  A tile's 128-row box may reach into the next group's rows (or past the tensor, which reads zeros): those accumulator
-// rows are not stored.  Groups of at most 64 rows (decode steps) swap the operands: tiles of 128 weight rows against a group's tokens;
-// declined when the groups that can have rows are too few to occupy the SMs.
+// them), w [groups][N][K].  The grid is sized for the tiles that total_rows rows can make, the kernel numbers those that exist.  A tile's
+// box may reach into the next group's rows (or past the tensor, which reads zeros): those accumulator columns are not stored.  Groups of at
+// most 64 rows (decode steps) take the one-CTA tiles; declined when the groups that can have rows are too few to occupy the SMs.
 template <typename T>
 int gemm_tc_launch_grouped(const T* x, const T* w, void* y, const int32_t* seg, int64_t total_rows, int64_t max_rows, int64_t N,
                            int64_t K, int64_t ldx, int64_t ldw, int64_t ldy, int64_t groups, int64_t sw, int epi, float2 act,
@@ -503,35 +708,32 @@ int gemm_tc_launch_grouped(const T* x, const T* w, void* y, const int32_t* seg, 
   if (K < GT_BK || total_rows >= (1ll << 31) || N >= (1ll << 31) || K >= (1ll << 31) || groups > GT_MAX_GROUPS) return 1;
   TcEncodeFn enc = gemm_tc_encode_fn();
   if (!enc) return 1;
-  const bool trans = max_rows <= 64;
-  if (trans && min(groups, total_rows) * ((N + GT_BM - 1) / GT_BM) < sm_count()) return 1;
-  const int bn = trans ? (max_rows <= 32 ? 32 : 64) : N <= 64 ? 64 : N <= 128 ? 128 : 256;
+  if (max_rows > 64) {
+    const int64_t tiles_t = min(groups, total_rows) + total_rows / pair::MAX_TN;
+    return pair::launch<T>(enc, x, w, y, seg, total_rows, max_rows, 0, (tiles_t + groups - 1) / groups, N, K, ldx, ldw, ldy, groups, 0, sw, 0, epi, act, st);
+  }
+  if (min(groups, total_rows) * ((N + GT_BM - 1) / GT_BM) < sm_count()) return 1;
+  const int bn = max_rows <= 32 ? 32 : 64;
   const CUtensorMapDataType dt = std::is_same<T, __nv_bfloat16>::value ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
   CUtensorMap tmx, tmw;
-  if (!gemm_tc_map(enc, &tmx, dt, x, K, total_rows, 1, ldx, 0, trans ? bn : GT_BM)) return 1;
-  if (!gemm_tc_map(enc, &tmw, dt, w, K, N, groups, ldw, sw, trans ? GT_BM : bn)) return 1;
+  if (!gemm_tc_map(enc, &tmx, dt, x, K, total_rows, 1, ldx, 0, bn)) return 1;
+  if (!gemm_tc_map(enc, &tmw, dt, w, K, N, groups, ldw, sw, GT_BM)) return 1;
   GemmTcParams p;
   p.y = y;
-  p.M = trans ? N : max_rows; p.N = trans ? max_rows : N; p.K = K; p.ldy = ldy; p.sy = 0;
-  p.tiles_m = (int)((p.M + GT_BM - 1) / GT_BM);
-  p.tiles_n = (int)((p.N + bn - 1) / bn);
-  const int64_t nt = (int64_t)p.tiles_m * p.tiles_n * groups;
+  p.R = N; p.tokens = max_rows; p.ldy = ldy; p.sy = 0;
+  p.tiles_r = (int)((N + GT_BM - 1) / GT_BM);
+  p.tiles_t = 1;
+  const int64_t nt = (int64_t)p.tiles_r * groups;
   if (nt >= (1ll << 31)) return 1;
   p.num_tiles = (int)nt;
   p.num_kb = (int)((K + GT_BK - 1) / GT_BK);
   p.splits = 1;
   p.kb_per_split = p.num_kb;
-  p.trans = trans;
   p.seg = seg;
   p.groups = (int)groups;
   p.epi = epi;
   p.act = act;
-  const int64_t eb = (epi == B200P_GEMM_STORE_F32 || epi == B200P_GEMM_CAP_F32) ? 4 : 2;
-  p.vec_ok = aligned(y, 16) && (ldy * eb) % 16 == 0;
-  if (trans) return bn == 32 ? gemm_tc_run<T, 32, 10>(tmw, tmx, p, st) : gemm_tc_run<T, 64, 8>(tmw, tmx, p, st);
-  if (bn == 256) return gemm_tc_run<T, 256, 4>(tmx, tmw, p, st);
-  if (bn == 128) return gemm_tc_run<T, 128, 6>(tmx, tmw, p, st);
-  return gemm_tc_run<T, 64, 8>(tmx, tmw, p, st);
+  return bn == 32 ? gemm_tc_run<T, 32, 10>(tmw, tmx, p, st) : gemm_tc_run<T, 64, 8>(tmw, tmx, p, st);
 }
 template int gemm_tc_launch_grouped<__half>(const __half*, const __half*, void*, const int32_t*, int64_t, int64_t, int64_t, int64_t, int64_t,
                                             int64_t, int64_t, int64_t, int64_t, int, float2, cudaStream_t);

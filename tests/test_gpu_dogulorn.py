@@ -133,6 +133,37 @@ def test_gemm_tcgen05_tiles(dtype, M, N, K):
         assert glu.shape == (M, N // 2) and (glu.double() - a * torch.sigmoid(1.702 * a) * (u + 1)).abs().max() < 0.02
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("M,N,K,batch", [(65, 2, 64, 1), (96, 256, 72, 1), (257, 300, 200, 1), (512, 257, 448, 1), (777, 1030, 136, 1), (1000, 640, 64, 3),
+                                         (4100, 5000, 320, 1)])
+def test_gemm_pairs_of_ctas(dtype, M, N, K, batch):
+    """Two CTAs on one tile of 256 output columns x up to 256 tokens (more than 64 rows): ragged edges in all three dimensions, columns
+    that end in the first CTA's half, one tile for a pair and several, batches, all kinds of stores."""
+    from mlx_parallm_b200 import _lib, ops
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    x = (torch.randn(batch, M, K, generator=g, device="cuda") / 4).to(dtype)
+    w = (torch.randn(batch, N, K, generator=g, device="cuda") / 4).to(dtype)
+    want = torch.einsum("bmk,bnk->mbn", x.double(), w.double())
+    for epi in (_lib.GEMM_STORE_F32, _lib.GEMM_STORE, _lib.GEMM_RELU_SQ, _lib.GEMM_CAP_F32, _lib.GEMM_GLU_SILU):
+        gated = epi == _lib.GEMM_GLU_SILU
+        if gated and N % 2:
+            continue
+        cols = N // 2 if gated else N
+        out = torch.full((M, batch, cols), 7.0, dtype=torch.float32 if _lib.gemm_is_f32(epi) else dtype, device="cuda")
+        ops.gemm(x, w, epi, out=out, act=(3.0, 0.0), batch=batch, strides=(M * K, N * K, cols), M=M, N=N, K=K, ldx=K, ldw=K, ldy=batch * cols)
+        ref, tol = want, 2e-5 * math.sqrt(K)                        # sums of K products of about 1 / 16 in fp32
+        if epi == _lib.GEMM_RELU_SQ:
+            ref = want.clamp(min=0).square()
+        elif epi == _lib.GEMM_CAP_F32:
+            ref = 3.0 * torch.tanh(want / 3.0)
+        elif gated:
+            ref = torch.nn.functional.silu(want[..., 0::2]) * want[..., 1::2]
+        if not _lib.gemm_is_f32(epi):                               # one rounding to 8 or 11 bits of the largest result
+            tol += float(ref.abs().max()) * (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11)
+        assert (out.double() - ref).abs().max() <= tol, epi
+    assert _lib.lib().b200p_gemm_tc_fault() == 0
+
+
 @pytest.mark.parametrize("M", [330, 24, 57])
 def test_gemm_tcgen05_heads_and_strides(M):
     """One weight block per head, operands and outputs strided inside wider rows (3-d tensor maps)."""
