@@ -305,11 +305,19 @@ int b200p_gemm(const void* x, const void* w, void* y, int64_t M, int64_t N, int6
 /* Grouped product (the experts of a mixture): group z < groups multiplies the rows [seg[z], seg[z+1]) of x (and writes the same
  * rows of y) by its own weight block w + z * stride_w ([N, K]); seg is a DEVICE array of groups + 1 ascending offsets and
  * max_rows an upper bound of a group's row count, which sizes the launch (so the launch does not depend on the routing);
- * total_rows = rows of x and y (seg[groups] <= total_rows).  16-bit calls run on tcgen05: more than 64 rows per group with the rows
- * on the MMA's M side, fewer with the weights there (unless the groups that can have rows are too few to occupy the GPU). */
+ * total_rows = rows of x and y (seg[groups] <= total_rows).  16-bit calls run on tcgen05 (up to 64 rows per group unless the groups
+ * that can have rows are too few to occupy the GPU). */
 int b200p_gemm_grouped(const void* x, const void* w, void* y, const int32_t* seg, int64_t total_rows, int64_t max_rows, int64_t N, int64_t K,
                        int64_t ldx, int64_t ldw, int64_t ldy, int64_t groups, int64_t stride_w, int dtype, int epilogue,
                        float act_a, float act_b, void* stream);
+
+/* The same and a plain product y2 [M2, N2] = x2 [M2, K2] . w2 [N2, K2]^T with the same types and epilogue (a shared expert beside the
+ * routed ones; neither may read what the other writes): one launch where both run on tcgen05 and M2 == max_rows, else one after the
+ * other. */
+int b200p_gemm_grouped_with(const void* x, const void* w, void* y, const int32_t* seg, int64_t total_rows, int64_t max_rows, int64_t N,
+                            int64_t K, int64_t ldx, int64_t ldw, int64_t ldy, int64_t groups, int64_t stride_w, const void* x2,
+                            const void* w2, void* y2, int64_t M2, int64_t N2, int64_t K2, int64_t ldx2, int64_t ldw2, int64_t ldy2,
+                            int dtype, int epilogue, float act_a, float act_b, void* stream);
 
 /* 0 (default): calls of 9 rows and more run on tcgen05 (TMA-fed shared-memory operands, TMEM accumulators; up to 64 rows with the
  * weights on the MMA's M side and K split where the output is narrow, which adds fp32 partial sums in no fixed order) and fall

@@ -74,6 +74,13 @@ __device__ __forceinline__ float warp_max(float v) {
   return v;
 }
 
+// a plain product y [M, N] = x [M, K] . w [N, K]^T that rides in the launch of a grouped one (dense_gemm_tc.cu)
+struct GemmTcPlain {
+  const void *x, *w;
+  void* y;
+  int64_t M, N, K, ldx, ldw, ldy;
+};
+
 // ---- gated hidden unit of a feed-forward, computed in the GEMM epilogue from the (gate, up) pair of one unit --------------
 __device__ __forceinline__ float gelu_tanh_unit(float z) {
   return 0.5f * z * (1.f + tanhf(0.7978845608028654f * (z + 0.044715f * z * z * z)));

@@ -20,7 +20,7 @@ int gemm_tc_launch(const T* x, const T* w, void* y, int64_t M, int64_t N, int64_
 template <typename T>
 int gemm_tc_launch_grouped(const T* x, const T* w, void* y, const int32_t* seg, int64_t total_rows, int64_t max_rows, int64_t N,
                            int64_t K, int64_t ldx, int64_t ldw, int64_t ldy, int64_t groups, int64_t sw, int epi, float2 act,
-                           cudaStream_t st);
+                           const GemmTcPlain* two, cudaStream_t st);
 // 0: tcgen05 from 9 rows up (its decode variant streams the weights 1.0-2.3x faster than gemm_stream_kernel at 16 rows, 1.1-2.6x at
 //    32, 1.6-4.4x at 64), the mma.sync kernels where it declines; 1: mma.sync kernels only; 2: the same as 0
 static int g_gemm_path = 0;
@@ -401,14 +401,20 @@ static int gemm_dispatch(const void* x, const void* w, void* y, int64_t M, int64
 template <typename T>
 static int gemm_grouped_dispatch(const void* x, const void* w, void* y, const int32_t* seg, int64_t total_rows, int64_t max_rows, int64_t N, int64_t K,
                                  int64_t ldx, int64_t ldw, int64_t ldy, int64_t groups, int64_t sw, int epi, float2 act, bool fast_ok,
-                                 cudaStream_t st) {
+                                 const GemmTcPlain* two, bool two_fast, cudaStream_t st) {
   const T* xp = (const T*)x;
   const T* wp = (const T*)w;
   if constexpr (!std::is_same<T, float>::value) {
     if (fast_ok && g_gemm_path != 1) {
-      const int rc = gemm_tc_launch_grouped<T>(xp, wp, y, seg, total_rows, max_rows, N, K, ldx, ldw, ldy, groups, sw, epi, act, st);
+      const int rc = gemm_tc_launch_grouped<T>(xp, wp, y, seg, total_rows, max_rows, N, K, ldx, ldw, ldy, groups, sw, epi, act, two_fast ? two : nullptr, st);
+      if (rc == B200P_OK && two && !two_fast)
+        return gemm_dispatch<T>(two->x, two->w, two->y, two->M, two->N, two->K, two->ldx, two->ldw, two->ldy, 1, 0, 0, 0, epi, act, false, st);
       if (rc != 1) return rc;
     }
+  }
+  if (two) {                                     // not together: one after the other
+    const int rc = gemm_dispatch<T>(two->x, two->w, two->y, two->M, two->N, two->K, two->ldx, two->ldw, two->ldy, 1, 0, 0, 0, epi, act, two_fast, st);
+    if (rc) return rc;
   }
   if (fast_ok && max_rows <= 64) {
     dim3 grid((unsigned)((N + 15) / 16), 1, (unsigned)groups);
@@ -429,10 +435,10 @@ static int gemm_grouped_dispatch(const void* x, const void* w, void* y, const in
 
 }  // namespace b200p
 
-extern "C" int b200p_gemm_grouped(const void* x, const void* w, void* y, const int32_t* seg, int64_t total_rows, int64_t max_rows, int64_t N, int64_t K,
-                                  int64_t ldx, int64_t ldw, int64_t ldy, int64_t groups, int64_t stride_w, int dtype, int epilogue,
-                                  float act_a, float act_b, void* stream) {
-  using namespace b200p;
+namespace b200p {
+static int gemm_grouped_call(const void* x, const void* w, void* y, const int32_t* seg, int64_t total_rows, int64_t max_rows, int64_t N, int64_t K,
+                             int64_t ldx, int64_t ldw, int64_t ldy, int64_t groups, int64_t stride_w, const GemmTcPlain* two, int dtype,
+                             int epilogue, float act_a, float act_b, void* stream) {
   B200P_REQUIRE(x && w && y && seg, B200P_ERR_ARG, "null pointer");
   B200P_REQUIRE(total_rows >= max_rows, B200P_ERR_ARG, "x has fewer rows than a group may have");
   B200P_REQUIRE(max_rows >= 0 && N > 0 && K > 0 && groups > 0 && groups < 65536 && ldx >= K && ldw >= K, B200P_ERR_ARG, "bad GEMM shape");
@@ -440,22 +446,47 @@ extern "C" int b200p_gemm_grouped(const void* x, const void* w, void* y, const i
   B200P_REQUIRE(epilogue != B200P_GEMM_CAP_F32 || act_a > 0.f, B200P_ERR_ARG, "the capped epilogue needs a positive cap");
   B200P_REQUIRE(epilogue < B200P_GEMM_GLU_CLAMP || epilogue > B200P_GEMM_GLU_SILU || N % 2 == 0, B200P_ERR_ARG, "the gated epilogue needs gate / up row pairs");
   B200P_REQUIRE((max_rows + 63) / 64 < 65536, B200P_ERR_ARG, "grid too large");
+  if (two) {
+    B200P_REQUIRE(two->x && two->w && two->y, B200P_ERR_ARG, "null pointer");
+    B200P_REQUIRE(two->M >= 0 && two->N > 0 && two->K > 0 && two->ldx >= two->K && two->ldw >= two->K, B200P_ERR_ARG, "bad GEMM shape");
+    B200P_REQUIRE(epilogue < B200P_GEMM_GLU_CLAMP || epilogue > B200P_GEMM_GLU_SILU || two->N % 2 == 0, B200P_ERR_ARG, "the gated epilogue needs gate / up row pairs");
+    B200P_REQUIRE((two->M + 63) / 64 < 65536, B200P_ERR_ARG, "grid too large");
+    if (two->M == 0) two = nullptr;
+    else if (max_rows == 0)
+      return b200p_gemm(two->x, two->w, two->y, two->M, two->N, two->K, two->ldx, two->ldw, two->ldy, 1, 0, 0, 0, dtype, epilogue, act_a, act_b, stream);
+  }
   if (max_rows == 0) return B200P_OK;
   cudaStream_t st = (cudaStream_t)stream;
   const bool fast_ok = dtype != B200P_F32 && K % 8 == 0 && ldx % 8 == 0 && ldw % 8 == 0 && stride_w % 8 == 0 && aligned(x, 16) &&
                        aligned(w, 16);
+  const bool two_fast = two && dtype != B200P_F32 && two->K % 8 == 0 && two->ldx % 8 == 0 && two->ldw % 8 == 0 && aligned(two->x, 16) && aligned(two->w, 16);
   switch (dtype) {
     case B200P_F32:
-      return gemm_grouped_dispatch<float>(x, w, y, seg, total_rows, max_rows, N, K, ldx, ldw, ldy, groups, stride_w, epilogue, {act_a, act_b}, false, st);
+      return gemm_grouped_dispatch<float>(x, w, y, seg, total_rows, max_rows, N, K, ldx, ldw, ldy, groups, stride_w, epilogue, {act_a, act_b}, false, two, two_fast, st);
     case B200P_F16:
-      return gemm_grouped_dispatch<__half>(x, w, y, seg, total_rows, max_rows, N, K, ldx, ldw, ldy, groups, stride_w, epilogue, {act_a, act_b}, fast_ok, st);
+      return gemm_grouped_dispatch<__half>(x, w, y, seg, total_rows, max_rows, N, K, ldx, ldw, ldy, groups, stride_w, epilogue, {act_a, act_b}, fast_ok, two, two_fast, st);
     case B200P_BF16:
       return gemm_grouped_dispatch<__nv_bfloat16>(x, w, y, seg, total_rows, max_rows, N, K, ldx, ldw, ldy, groups, stride_w, epilogue, {act_a, act_b},
-                                                  fast_ok, st);
+                                                  fast_ok, two, two_fast, st);
     default:
       set_error("bad dtype %d", dtype);
       return B200P_ERR_ARG;
   }
+}
+}  // namespace b200p
+
+extern "C" int b200p_gemm_grouped(const void* x, const void* w, void* y, const int32_t* seg, int64_t total_rows, int64_t max_rows, int64_t N, int64_t K,
+                                  int64_t ldx, int64_t ldw, int64_t ldy, int64_t groups, int64_t stride_w, int dtype, int epilogue,
+                                  float act_a, float act_b, void* stream) {
+  return b200p::gemm_grouped_call(x, w, y, seg, total_rows, max_rows, N, K, ldx, ldw, ldy, groups, stride_w, nullptr, dtype, epilogue, act_a, act_b, stream);
+}
+
+extern "C" int b200p_gemm_grouped_with(const void* x, const void* w, void* y, const int32_t* seg, int64_t total_rows, int64_t max_rows, int64_t N,
+                                       int64_t K, int64_t ldx, int64_t ldw, int64_t ldy, int64_t groups, int64_t stride_w, const void* x2,
+                                       const void* w2, void* y2, int64_t M2, int64_t N2, int64_t K2, int64_t ldx2, int64_t ldw2, int64_t ldy2,
+                                       int dtype, int epilogue, float act_a, float act_b, void* stream) {
+  const b200p::GemmTcPlain two = {x2, w2, y2, M2, N2, K2, ldx2, ldw2, ldy2};
+  return b200p::gemm_grouped_call(x, w, y, seg, total_rows, max_rows, N, K, ldx, ldw, ldy, groups, stride_w, &two, dtype, epilogue, act_a, act_b, stream);
 }
 
 extern "C" int b200p_gemm_set_path(int path) {

@@ -33,9 +33,10 @@ bool pdl_enabled_gemm();
 constexpr int GT_BM = 128, GT_BK = 64, GT_THREADS = 192;
 constexpr int GT_A_BYTES = GT_BM * GT_BK * 2;
 
+struct GemmTcOut { void* y; int64_t R, ldy; };     // R: output columns (weight rows)
 struct GemmTcParams {
-  void* y;
-  int64_t R, tokens, ldy, sy;    // output columns (weight rows); tokens (of the largest group)
+  GemmTcOut out[2];              // of the product, and of the second one
+  int64_t tokens, sy;            // tokens (of the largest group)
   int tiles_r, tiles_t, num_tiles, num_kb;
   int splits, kb_per_split;      // K split over `splits` CTAs per output tile (fp32 store only)
   int epi;
@@ -44,6 +45,11 @@ struct GemmTcParams {
   // memory first, every CTA counts the groups' tiles there
   const int32_t* seg;
   int groups;
+  // a plain product in the same launch (a mixture's shared expert beside the routed ones): its tiles come first, its K may be another
+  struct Second {
+    int64_t tokens;
+    int tiles_r, tiles_t, num_tiles, num_kb, tn;
+  } two;
   int* wait_word;                // where a wait that gives up reports
 };
 constexpr int GT_MAX_GROUPS = 1024;
@@ -63,39 +69,39 @@ __device__ __forceinline__ void umma_f16_ss(uint32_t d_tmem, uint64_t a_desc, ui
 // This thread owns output column `n` (a weight row) and holds it for 32 consecutive tokens from `tok0`, of those below `tokens`.
 // Gate / up pairs sit in neighbouring lanes.
 template <typename T>
-__device__ __forceinline__ void gemm_tc_store32(const GemmTcParams& p, int64_t z_off, int64_t n, int64_t tok0, int64_t tokens,
-                                                      const float (&v)[32]) {
+__device__ __forceinline__ void gemm_tc_store32(const GemmTcParams& p, const GemmTcOut& o, int64_t z_off, int64_t n, int64_t tok0, int64_t tokens,
+                                                const float (&v)[32]) {
   if (gemm_epi_is_glu(p.epi)) {
     // the even lane of a pair holds the gate, the odd one the up row: the former finishes even tokens, the latter odd ones
     const bool odd = (threadIdx.x & 1) != 0;
-    T* dst = reinterpret_cast<T*>(p.y) + z_off + (tok0 + odd) * p.ldy + (n >> 1);
+    T* dst = reinterpret_cast<T*>(o.y) + z_off + (tok0 + odd) * o.ldy + (n >> 1);
 #pragma unroll
     for (int i = 0; i < 32; i += 2) {
       const float other = __shfl_xor_sync(0xffffffffu, odd ? v[i] : v[i + 1], 1);
-      if ((n | 1) < p.R && tok0 + i + odd < tokens)
-        dst[i * p.ldy] = Tr<T>::from_f(glu_unit16(odd ? other : v[i], odd ? v[i + 1] : other, p.epi, p.act));
+      if ((n | 1) < o.R && tok0 + i + odd < tokens)
+        dst[i * o.ldy] = Tr<T>::from_f(glu_unit16(odd ? other : v[i], odd ? v[i + 1] : other, p.epi, p.act));
     }
     return;
   }
-  if (n >= p.R) return;
+  if (n >= o.R) return;
   if (p.epi == B200P_GEMM_STORE_F32) {
-    float* dst = reinterpret_cast<float*>(p.y) + z_off + n;
+    float* dst = reinterpret_cast<float*>(o.y) + z_off + n;
     if (p.splits > 1) {
 #pragma unroll
       for (int i = 0; i < 32; ++i)
-        if (tok0 + i < tokens) atomicAdd(dst + (tok0 + i) * p.ldy, v[i]);
+        if (tok0 + i < tokens) atomicAdd(dst + (tok0 + i) * o.ldy, v[i]);
     } else {
 #pragma unroll
       for (int i = 0; i < 32; ++i)
-        if (tok0 + i < tokens) dst[(tok0 + i) * p.ldy] = v[i];
+        if (tok0 + i < tokens) dst[(tok0 + i) * o.ldy] = v[i];
     }
   } else if (p.epi == B200P_GEMM_CAP_F32) {
-    float* dst = reinterpret_cast<float*>(p.y) + z_off + n;
+    float* dst = reinterpret_cast<float*>(o.y) + z_off + n;
 #pragma unroll
     for (int i = 0; i < 32; ++i)
-      if (tok0 + i < tokens) dst[(tok0 + i) * p.ldy] = gemm_f32_act(v[i], p.epi, p.act);
+      if (tok0 + i < tokens) dst[(tok0 + i) * o.ldy] = gemm_f32_act(v[i], p.epi, p.act);
   } else {
-    T* dst = reinterpret_cast<T*>(p.y) + z_off + n;
+    T* dst = reinterpret_cast<T*>(o.y) + z_off + n;
     float a[32];                                   // one uniform branch for all elements
     if (p.epi == B200P_GEMM_XIELU) {
 #pragma unroll
@@ -106,7 +112,7 @@ __device__ __forceinline__ void gemm_tc_store32(const GemmTcParams& p, int64_t z
     }
 #pragma unroll
     for (int i = 0; i < 32; ++i)
-      if (tok0 + i < tokens) dst[(tok0 + i) * p.ldy] = Tr<T>::from_f(a[i]);
+      if (tok0 + i < tokens) dst[(tok0 + i) * o.ldy] = Tr<T>::from_f(a[i]);
   }
 }
 
@@ -120,11 +126,24 @@ struct GemmTcShared {            // lives behind the ring stages (8-byte aligned
 
 // Tile t of the launch: batch index (group) z, row tile rt; first token of the group in x / y and how many it has.  Grouped products
 // number only the tiles of groups that hold tokens, so that the CTAs share them evenly whatever the routing.
-struct GemmTcTile { int z, rt, first, len; };
+struct GemmTcTile { int z, rt, first, len, kb0, kb1, second; };
 __device__ __forceinline__ GemmTcTile gemm_tc_tile(const GemmTcParams& p, const GemmTcShared* sh, int t) {
   GemmTcTile r;
+  r.second = t < p.two.num_tiles;
+  r.kb0 = 0;
+  if (r.second) {
+    r.z = r.first = 0;
+    r.rt = t;
+    r.len = (int)p.two.tokens;
+    r.kb1 = p.two.num_kb;
+    return r;
+  }
+  t -= p.two.num_tiles;
+  r.kb1 = p.num_kb;
   if (!p.seg) {
     const int ts = t / p.splits;
+    r.kb0 = (t - ts * p.splits) * p.kb_per_split;
+    r.kb1 = min(p.num_kb, r.kb0 + p.kb_per_split);
     r.z = ts / p.tiles_r;
     r.rt = ts - r.z * p.tiles_r;
     r.first = 0;
@@ -145,7 +164,8 @@ __device__ __forceinline__ GemmTcTile gemm_tc_tile(const GemmTcParams& p, const 
 
 template <typename T, int BN, int STAGES>
 __global__ void __launch_bounds__(GT_THREADS, 1)
-gemm_tc_kernel(const __grid_constant__ CUtensorMap tmw, const __grid_constant__ CUtensorMap tmx, const GemmTcParams p) {
+gemm_tc_kernel(const __grid_constant__ CUtensorMap tmw, const __grid_constant__ CUtensorMap tmx, const __grid_constant__ CUtensorMap tmw2,
+               const __grid_constant__ CUtensorMap tmx2, const GemmTcParams p) {
   constexpr int B_BYTES = BN * GT_BK * 2, STAGE_BYTES = GT_A_BYTES + B_BYTES;
   constexpr uint32_t TMEM_COLS = 2 * BN;           // 64 or 128: a power of two >= 32
   static_assert(STAGES <= 10 && (BN == 32 || BN == 64), "ring / tile shape");
@@ -172,6 +192,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmw, const __grid_constant__ 
     tma_prefetch_desc(&tmw);
   }
   if (warp == 1) tmem_alloc(smem_u32(&sh->tmem_base), TMEM_COLS);
+  pdl_launch_dependents();
+  pdl_wait();                                      // operands, seg and y belong to the previous kernels until here
   if (p.seg) {
     for (int i = threadIdx.x; i <= p.groups; i += blockDim.x) sh->seg[i] = p.seg[i];
     __syncthreads();
@@ -196,7 +218,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmw, const __grid_constant__ 
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = sh->tmem_base;
-  const int num_tiles = p.seg ? sh->live[p.groups] : p.num_tiles;
+  const int num_tiles = p.two.num_tiles + (p.seg ? sh->live[p.groups] : p.num_tiles);
 
   // (whole warps walk the loops and one elected lane issues: operands of warp-uniform code need no uniformising)
   if (warp == 0) {
@@ -204,16 +226,16 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmw, const __grid_constant__ 
     uint32_t phase = 0;
     bool ok = true;
     for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
-      const int kb0 = (t % p.splits) * p.kb_per_split, kb1 = min(p.num_kb, kb0 + p.kb_per_split);
       const GemmTcTile tl = gemm_tc_tile(p, sh, t);
-      for (int kb = kb0; kb < kb1; ++kb) {
+      const CUtensorMap *mw = tl.second ? &tmw2 : &tmw, *mx = tl.second ? &tmx2 : &tmx;
+      for (int kb = tl.kb0; kb < tl.kb1; ++kb) {
         if (!(ok = mbar_wait_warp(smem_u32(&sh->empty[stage]), phase ^ 1u, &sh->abort, p.wait_word, 0))) break;
         if (elect_one()) {
           const uint32_t bar = smem_u32(&sh->full[stage]);
           const uint32_t dst = base + stage * STAGE_BYTES;
           mbar_arrive_expect_tx(bar, STAGE_BYTES);
-          tma_load_3d(dst, &tmw, kb * GT_BK, tl.rt * GT_BM, tl.z, bar);
-          tma_load_3d(dst + GT_A_BYTES, &tmx, kb * GT_BK, tl.first, p.seg ? 0 : tl.z, bar);
+          tma_load_3d(dst, mw, kb * GT_BK, tl.rt * GT_BM, tl.z, bar);
+          tma_load_3d(dst + GT_A_BYTES, mx, kb * GT_BK, tl.first, p.seg ? 0 : tl.z, bar);
         }
         __syncwarp();
         if (++stage == STAGES) { stage = 0; phase ^= 1u; }
@@ -229,8 +251,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmw, const __grid_constant__ 
       if (!(ok = mbar_wait_warp(smem_u32(&sh->acc_empty[acc]), acc_phase ^ 1u, &sh->abort, p.wait_word, 1))) break;
       tc_fence_after();
       const uint32_t d = tmem_base + (uint32_t)(acc * BN);
-      const int kb0 = (t % p.splits) * p.kb_per_split, kb1 = min(p.num_kb, kb0 + p.kb_per_split);
-      for (int kb = kb0; kb < kb1; ++kb) {
+      const GemmTcTile tl = gemm_tc_tile(p, sh, t);
+      for (int kb = tl.kb0; kb < tl.kb1; ++kb) {
         if (!(ok = mbar_wait_warp(smem_u32(&sh->full[stage]), phase, &sh->abort, p.wait_word, 1))) break;
         tc_fence_after();
         if (elect_one()) {
@@ -238,9 +260,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmw, const __grid_constant__ 
           const uint64_t bd = make_desc_sw128(base + stage * STAGE_BYTES + GT_A_BYTES);
 #pragma unroll
           for (int k = 0; k < GT_BK / 16; ++k)       // 16 k = 32 bytes = 2 descriptor units inside the swizzle atom
-            umma_f16_ss(d, ad + 2u * k, bd + 2u * k, idesc, ((kb - kb0) | k) ? 1u : 0u);
+            umma_f16_ss(d, ad + 2u * k, bd + 2u * k, idesc, ((kb - tl.kb0) | k) ? 1u : 0u);
           umma_commit(smem_u32(&sh->empty[stage]));
-          if (kb == kb1 - 1) umma_commit(smem_u32(&sh->acc_full[acc]));
+          if (kb == tl.kb1 - 1) umma_commit(smem_u32(&sh->acc_full[acc]));
         }
         __syncwarp();
         if (++stage == STAGES) { stage = 0; phase ^= 1u; }
@@ -256,16 +278,17 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmw, const __grid_constant__ 
       if (!mbar_wait_warp(smem_u32(&sh->acc_full[acc]), acc_phase, &sh->abort, p.wait_word, 2)) break;
       tc_fence_after();
       const int64_t n = (int64_t)tl.rt * GT_BM + lg * 32 + lane;              // output column
-      const int64_t z_off = p.seg ? tl.first * p.ldy : (int64_t)tl.z * p.sy;
+      const GemmTcOut out = p.out[tl.second];
+      const int64_t z_off = p.seg ? tl.first * out.ldy : (int64_t)tl.z * p.sy;       // (0 of the second product)
       const uint32_t tsrc = tmem_base + ((uint32_t)(lg * 32) << 16) + (uint32_t)(acc * BN);
 #pragma unroll 1
       for (int c = 0; c < BN; c += 32) {
-        if (c >= p.tokens) break;                  // warp-uniform
+        if (c >= tl.len) break;                    // warp-uniform
         float v[32];
         tmem_ld16(tsrc + c, *reinterpret_cast<float(*)[16]>(&v[0]));
         tmem_ld16(tsrc + c + 16, *reinterpret_cast<float(*)[16]>(&v[16]));
         tmem_ld_wait();
-        gemm_tc_store32<T>(p, z_off, n, c, tl.len, v);
+        gemm_tc_store32<T>(p, out, z_off, n, c, tl.len, v);
       }
       tc_fence_before();
       __syncwarp();
@@ -359,11 +382,20 @@ __device__ __forceinline__ int even_tn(int len) {
   return nt == 0 ? TN_STEP : ((len + nt - 1) / nt + TN_STEP - 1) / TN_STEP * TN_STEP;
 }
 
-struct Tile { int z, rt, tok0, first, len, tn; };            // batch index (group), row tile, first token within it, ...
+struct Tile { int z, rt, tok0, first, len, tn, num_kb, second; };      // batch index (group), row tile, first token within it, ...
 __device__ __forceinline__ Tile tile_of(const Params& p, const Shared* sh, int t) {
   Tile r;
   int in, nt;
-  if (!p.g.seg) {
+  r.second = t < p.g.two.num_tiles;
+  r.num_kb = r.second ? p.g.two.num_kb : p.g.num_kb;
+  if (!r.second) t -= p.g.two.num_tiles;
+  if (r.second) {
+    nt = p.g.two.tiles_t;
+    in = t;
+    r.z = r.first = 0;
+    r.len = (int)p.g.two.tokens;
+    r.tn = p.g.two.tn;
+  } else if (!p.g.seg) {
     nt = p.g.tiles_t;
     const int per = p.g.tiles_r * nt;
     r.z = t / per;
@@ -391,7 +423,8 @@ __device__ __forceinline__ Tile tile_of(const Params& p, const Shared* sh, int t
 
 template <typename T>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
-gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmw, const __grid_constant__ CUtensorMap tmx, const Params p) {
+gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmw, const __grid_constant__ CUtensorMap tmx, const __grid_constant__ CUtensorMap tmw2,
+                    const __grid_constant__ CUtensorMap tmx2, const Params p) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;              // the same offset in both CTAs
@@ -446,7 +479,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmw, const __grid_consta
   cluster_sync();                                            // both CTAs' barriers exist
   tc_fence_after();
   const uint32_t tmem_base = sh->tmem_base;
-  const int num_tiles = p.g.seg ? sh->live[p.g.groups] * p.g.tiles_r : p.g.num_tiles;
+  const int num_tiles = p.g.two.num_tiles + (p.g.seg ? sh->live[p.g.groups] * p.g.tiles_r : p.g.num_tiles);
 
   // (whole warps walk the loops and one elected lane issues: operands of warp-uniform code need no uniformising)
   if (warp == 0) {
@@ -455,16 +488,17 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmw, const __grid_consta
     bool ok = true;
     for (int t = pair0; t < num_tiles && ok; t += pairs) {
       const Tile tl = tile_of(p, sh, t);
-      const int half = tl.tn / 2, boxes = (half + p.box - 1) / p.box;
+      const int box = tl.second ? tl.tn / 2 : p.box, half = tl.tn / 2, boxes = (half + box - 1) / box;
+      const CUtensorMap *mw = tl.second ? &tmw2 : &tmw, *mx = tl.second ? &tmx2 : &tmx;
       const int row = tl.rt * 256 + (int)rank * 128, tok = tl.first + tl.tok0 + (int)rank * half, zx = p.g.seg ? 0 : tl.z;
-      const uint32_t box_bytes = (uint32_t)p.box * GT_BK * 2, bytes = 2u * (uint32_t)(A_BYTES + boxes * box_bytes);
-      for (int kb = 0; kb < p.g.num_kb; ++kb) {
+      const uint32_t box_bytes = (uint32_t)box * GT_BK * 2, bytes = 2u * (uint32_t)(A_BYTES + boxes * box_bytes);
+      for (int kb = 0; kb < tl.num_kb; ++kb) {
         if (!(ok = mbar_wait_warp(smem_u32(&sh->empty[stage]), phase ^ 1u, &sh->abort, word, 0))) break;
         if (elect_one()) {
           const uint32_t bar = map_to_leader(smem_u32(&sh->full[stage])), dst = base + stage * STAGE_BYTES;
           if (rank == 0) mbar_arrive_expect_tx(smem_u32(&sh->full[stage]), bytes);
-          load_3d(dst, &tmw, kb * GT_BK, row, tl.z, bar);
-          for (int b = 0; b < boxes; ++b) load_3d(dst + A_BYTES + b * box_bytes, &tmx, kb * GT_BK, tok + b * p.box, zx, bar);
+          load_3d(dst, mw, kb * GT_BK, row, tl.z, bar);
+          for (int b = 0; b < boxes; ++b) load_3d(dst + A_BYTES + b * box_bytes, mx, kb * GT_BK, tok + b * box, zx, bar);
         }
         __syncwarp();
         if (++stage == STAGES) { stage = 0; phase ^= 1u; }
@@ -482,12 +516,13 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmw, const __grid_consta
       uint32_t phase = 0, acc_phase = 0;
       bool ok = true;
       for (int t = pair0; t < num_tiles && ok; t += pairs) {
-        const int tn = p.g.seg ? tile_of(p, sh, t).tn : p.tn;
+        const Tile tl = tile_of(p, sh, t);
+        const int tn = tl.tn;
         const uint32_t idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(tn >> 3) << 17) | ((256u >> 4) << 24);
         if (!(ok = mbar_wait_warp(smem_u32(&sh->acc_empty[acc]), acc_phase ^ 1u, &sh->abort, word, 1))) break;
         tc_fence_after();
         const uint32_t d = tmem_base + (uint32_t)(acc * MAX_TN);
-        for (int kb = 0; kb < p.g.num_kb; ++kb) {
+        for (int kb = 0; kb < tl.num_kb; ++kb) {
           if (!(ok = mbar_wait_warp(smem_u32(&sh->full[stage]), phase, &sh->abort, word, 1))) break;
           tc_fence_after();
           if (elect_one()) {
@@ -495,7 +530,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmw, const __grid_consta
 #pragma unroll
             for (int k = 0; k < GT_BK / 16; ++k) umma_pair(d, ad + 2u * k, bd + 2u * k, idesc, (kb | k) ? 1u : 0u);
             commit_pair(smem_u32(&sh->empty[stage]));
-            if (kb == p.g.num_kb - 1) commit_pair(smem_u32(&sh->acc_full[acc]));
+            if (kb == tl.num_kb - 1) commit_pair(smem_u32(&sh->acc_full[acc]));
           }
           __syncwarp();
           if (++stage == STAGES) { stage = 0; phase ^= 1u; }
@@ -512,7 +547,8 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmw, const __grid_consta
       if (!mbar_wait_warp(smem_u32(&sh->acc_full[acc]), acc_phase, &sh->abort, word, 2)) break;
       tc_fence_after();
       const int64_t n = (int64_t)tl.rt * 256 + rank * 128 + lg * 32 + lane;
-      const int64_t z_off = p.g.seg ? (int64_t)tl.first * p.g.ldy : (int64_t)tl.z * p.g.sy;
+      const GemmTcOut out = p.g.out[tl.second];
+      const int64_t z_off = p.g.seg ? (int64_t)tl.first * out.ldy : (int64_t)tl.z * p.g.sy;
       const uint32_t src = tmem_base + ((uint32_t)(lg * 32) << 16) + (uint32_t)(acc * MAX_TN);
       const int most = min(tl.tn, tl.len - tl.tok0);         // tokens of this tile
 #pragma unroll 1
@@ -521,7 +557,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmw, const __grid_consta
         tmem_ld16(src + c, *reinterpret_cast<float(*)[16]>(&v[0]));
         tmem_ld16(src + c + 16, *reinterpret_cast<float(*)[16]>(&v[16]));
         tmem_ld_wait();
-        gemm_tc_store32<T>(p.g, z_off, n, tl.tok0 + c, tl.tok0 + most, v);
+        gemm_tc_store32<T>(p.g, out, z_off, n, tl.tok0 + c, tl.tok0 + most, v);
       }
       tc_fence_before();
       __syncwarp();
@@ -564,8 +600,20 @@ static bool gemm_tc_map(TcEncodeFn enc, CUtensorMap* tm, CUtensorMapDataType dt,
              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+static void gemm_tc_set_second(GemmTcParams& p, const GemmTcPlain* two, int rows) {
+  p.two = {};
+  p.out[1] = p.out[0];
+  if (!two) return;
+  p.out[1] = {two->y, two->N, two->ldy};
+  p.two.tokens = two->M;
+  p.two.tiles_r = (int)((two->N + rows - 1) / rows);
+  p.two.tiles_t = 1;
+  p.two.num_tiles = p.two.tiles_r;
+  p.two.num_kb = (int)((two->K + GT_BK - 1) / GT_BK);
+}
+
 template <typename T, int BN, int STAGES>
-static int gemm_tc_run(const CUtensorMap& tmw, const CUtensorMap& tmx, GemmTcParams p, cudaStream_t st) {
+static int gemm_tc_run(const CUtensorMap* tm, GemmTcParams p, cudaStream_t st) {
   constexpr size_t smem = 1024 + (size_t)STAGES * (GT_A_BYTES + BN * GT_BK * 2) + sizeof(GemmTcShared);
   auto kern = gemm_tc_kernel<T, BN, STAGES>;
   static bool attr_set = false;
@@ -575,16 +623,16 @@ static int gemm_tc_run(const CUtensorMap& tmw, const CUtensorMap& tmx, GemmTcPar
     attr_set = true;
   }
   if (const int rc = wait_word(WAIT_GEMM_TC, &p.wait_word)) return rc;
-  const int grid = p.num_tiles < sm_count() ? p.num_tiles : sm_count();
-  kern<<<grid, GT_THREADS, smem, st>>>(tmw, tmx, p);
-  B200P_LAUNCH_CHECK("gemm_tc_kernel");
+  const int tiles = p.num_tiles + p.two.num_tiles, grid = tiles < sm_count() ? tiles : sm_count();
+  cudaError_t e = launch_pdl_opt(pdl_enabled_gemm(), kern, dim3((unsigned)grid), dim3(GT_THREADS), smem, st, tm[0], tm[1], tm[2], tm[3], p);
+  if (e != cudaSuccess) return cuda_fail(e, "gemm_tc_kernel launch");
   return B200P_OK;
 }
 
 namespace pair {
 
 template <typename T>
-static int run(const CUtensorMap& tmw, const CUtensorMap& tmx, Params p, int64_t tiles, cudaStream_t st) {
+static int run(const CUtensorMap* tm, Params p, int64_t tiles, cudaStream_t st) {
   constexpr size_t smem = 1024 + (size_t)STAGES * STAGE_BYTES + sizeof(Shared);
   auto kern = gemm_tc_pair_kernel<T>;
   static bool attr_set = false;
@@ -596,7 +644,7 @@ static int run(const CUtensorMap& tmw, const CUtensorMap& tmx, Params p, int64_t
   if (const int rc = wait_word(WAIT_GEMM_TC, &p.g.wait_word)) return rc;
   const int64_t pairs = sm_count() / 2;
   const unsigned grid = 2u * (unsigned)(tiles < pairs ? tiles : pairs);
-  cudaError_t e = launch_pdl_opt(pdl_enabled_gemm(), kern, dim3(grid), dim3(THREADS), smem, st, tmw, tmx, p);
+  cudaError_t e = launch_pdl_opt(pdl_enabled_gemm(), kern, dim3(grid), dim3(THREADS), smem, st, tm[0], tm[1], tm[2], tm[3], p);
   if (e != cudaSuccess) return cuda_fail(e, "gemm_tc_pair_kernel launch");
   return B200P_OK;
 }
@@ -618,16 +666,16 @@ static void plan(int64_t tokens, int64_t R, int64_t batch, int& tn, int64_t& til
 template <typename T>
 static int launch(TcEncodeFn enc, const T* x, const T* w, void* y, const int32_t* seg, int64_t x_rows, int64_t tokens, int tn, int64_t tiles_t, int64_t R,
                   int64_t K, int64_t ldx, int64_t ldw, int64_t ldy, int64_t batch, int64_t sx, int64_t sw, int64_t sy, int epi, float2 act,
-                  cudaStream_t st) {
+                  const GemmTcPlain* two, cudaStream_t st) {
   const CUtensorMapDataType dt = std::is_same<T, __nv_bfloat16>::value ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
-  CUtensorMap tmw, tmx;
-  if (!gemm_tc_map(enc, &tmw, dt, w, K, R, batch, ldw, sw, 128)) return 1;
+  CUtensorMap tm[4];
+  if (!gemm_tc_map(enc, &tm[0], dt, w, K, R, batch, ldw, sw, 128)) return 1;
   Params p;
   p.box = seg ? 64 : tn / 2;
-  if (!gemm_tc_map(enc, &tmx, dt, x, K, x_rows, seg ? 1 : batch, ldx, sx, p.box)) return 1;
+  if (!gemm_tc_map(enc, &tm[1], dt, x, K, x_rows, seg ? 1 : batch, ldx, sx, p.box)) return 1;
   GemmTcParams& g = p.g;
-  g.y = y;
-  g.R = R; g.tokens = tokens; g.ldy = ldy; g.sy = seg ? 0 : sy;
+  g.out[0] = {y, R, ldy};
+  g.tokens = tokens; g.sy = seg ? 0 : sy;
   g.tiles_r = (int)((R + 255) / 256);
   g.tiles_t = (int)tiles_t;
   const int64_t tiles = (int64_t)g.tiles_r * tiles_t * batch;
@@ -640,7 +688,18 @@ static int launch(TcEncodeFn enc, const T* x, const T* w, void* y, const int32_t
   g.epi = epi;
   g.act = act;
   p.tn = tn;
-  return run<T>(tmw, tmx, p, tiles, st);
+  gemm_tc_set_second(g, two, 256);
+  tm[2] = tm[0];
+  tm[3] = tm[1];
+  if (two) {
+    int64_t tiles_t2 = 0;
+    plan(two->M, two->N, 1, g.two.tn, tiles_t2);
+    g.two.tiles_t = (int)tiles_t2;
+    g.two.num_tiles *= (int)tiles_t2;
+    if (!gemm_tc_map(enc, &tm[2], dt, two->w, two->K, two->N, 1, two->ldw, 0, 128)) return 1;
+    if (!gemm_tc_map(enc, &tm[3], dt, two->x, two->K, two->M, 1, two->ldx, 0, g.two.tn / 2)) return 1;
+  }
+  return run<T>(tm, p, tiles + g.two.num_tiles, st);
 }
 
 }  // namespace pair
@@ -651,12 +710,14 @@ static int gemm_tc_launch_decode(TcEncodeFn enc, const T* x, const T* w, void* y
                                  int64_t ldy, int64_t batch, int64_t sx, int64_t sw, int64_t sy, int epi, float2 act, cudaStream_t st) {
   const CUtensorMapDataType dt = std::is_same<T, __nv_bfloat16>::value ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
   const int bn = M <= 32 ? 32 : 64;
-  CUtensorMap tma, tmb;                            // A = weights (128-row boxes), B = tokens (bn-row boxes)
-  if (!gemm_tc_map(enc, &tma, dt, w, K, N, batch, ldw, sw, GT_BM)) return 1;
-  if (!gemm_tc_map(enc, &tmb, dt, x, K, M, batch, ldx, sx, bn)) return 1;
+  CUtensorMap tm[4];                               // A = weights (128-row boxes), B = tokens (bn-row boxes)
+  if (!gemm_tc_map(enc, &tm[0], dt, w, K, N, batch, ldw, sw, GT_BM)) return 1;
+  if (!gemm_tc_map(enc, &tm[1], dt, x, K, M, batch, ldx, sx, bn)) return 1;
+  tm[2] = tm[0];
+  tm[3] = tm[1];
   GemmTcParams p;
-  p.y = y;
-  p.R = N; p.tokens = M; p.ldy = ldy; p.sy = sy;
+  p.out[0] = {y, N, ldy};
+  p.tokens = M; p.sy = sy;
   p.tiles_r = (int)((N + GT_BM - 1) / GT_BM);
   p.tiles_t = 1;
   p.num_kb = (int)((K + GT_BK - 1) / GT_BK);
@@ -679,8 +740,9 @@ static int gemm_tc_launch_decode(TcEncodeFn enc, const T* x, const T* w, void* y
     cudaError_t e = cudaMemsetAsync(y, 0, (size_t)M * N * sizeof(float), st);
     if (e != cudaSuccess) return cuda_fail(e, "cudaMemsetAsync(split-K output)");
   }
-  if (bn == 32) return gemm_tc_run<T, 32, 10>(tma, tmb, p, st);
-  return gemm_tc_run<T, 64, 8>(tma, tmb, p, st);
+  gemm_tc_set_second(p, nullptr, GT_BM);
+  if (bn == 32) return gemm_tc_run<T, 32, 10>(tm, p, st);
+  return gemm_tc_run<T, 64, 8>(tm, p, st);
 }
 
 // Returns B200P_OK, an error, or 1 when the shape is not one this kernel takes (the caller then runs the mma.sync kernel).
@@ -694,33 +756,40 @@ int gemm_tc_launch(const T* x, const T* w, void* y, int64_t M, int64_t N, int64_
   int tn = 0;
   int64_t tiles_t = 0;
   pair::plan(M, N, batch, tn, tiles_t);
-  return pair::launch<T>(enc, x, w, y, nullptr, M, M, tn, tiles_t, N, K, ldx, ldw, ldy, batch, sx, sw, sy, epi, act, st);
+  return pair::launch<T>(enc, x, w, y, nullptr, M, M, tn, tiles_t, N, K, ldx, ldw, ldy, batch, sx, sw, sy, epi, act, nullptr, st);
 }
 
 // Grouped product: x [total_rows, K] holds the groups' rows back to back (group z: rows [seg[z], seg[z+1]), at most max_rows of
 // them), w [groups][N][K].  The grid is sized for the tiles that total_rows rows can make, the kernel numbers those that exist.  A tile's
 // box may reach into the next group's rows (or past the tensor, which reads zeros): those accumulator columns are not stored.  Groups of at
-// most 64 rows (decode steps) take the one-CTA tiles; declined when the groups that can have rows are too few to occupy the SMs.
+// most 64 rows (decode steps) take the one-CTA tiles.  `two`: a plain product of max_rows tokens in the same
+// launch.  Declined when the groups that can have rows are too few to occupy the SMs.
 template <typename T>
 int gemm_tc_launch_grouped(const T* x, const T* w, void* y, const int32_t* seg, int64_t total_rows, int64_t max_rows, int64_t N,
                            int64_t K, int64_t ldx, int64_t ldw, int64_t ldy, int64_t groups, int64_t sw, int epi, float2 act,
-                           cudaStream_t st) {
+                           const GemmTcPlain* two, cudaStream_t st) {
+  if (two && (two->K < GT_BK || two->M != max_rows || two->N >= (1ll << 31) || two->K >= (1ll << 31))) return 1;
   if (K < GT_BK || total_rows >= (1ll << 31) || N >= (1ll << 31) || K >= (1ll << 31) || groups > GT_MAX_GROUPS) return 1;
   TcEncodeFn enc = gemm_tc_encode_fn();
   if (!enc) return 1;
   if (max_rows > 64) {
     const int64_t tiles_t = min(groups, total_rows) + total_rows / pair::MAX_TN;
-    return pair::launch<T>(enc, x, w, y, seg, total_rows, max_rows, 0, (tiles_t + groups - 1) / groups, N, K, ldx, ldw, ldy, groups, 0, sw, 0, epi, act, st);
+    return pair::launch<T>(enc, x, w, y, seg, total_rows, max_rows, 0, (tiles_t + groups - 1) / groups, N, K, ldx, ldw, ldy, groups, 0, sw, 0, epi, act, two, st);
   }
-  if (min(groups, total_rows) * ((N + GT_BM - 1) / GT_BM) < sm_count()) return 1;
+  if (min(groups, total_rows) * ((N + GT_BM - 1) / GT_BM) + (two ? (two->N + GT_BM - 1) / GT_BM : 0) < sm_count()) return 1;
   const int bn = max_rows <= 32 ? 32 : 64;
   const CUtensorMapDataType dt = std::is_same<T, __nv_bfloat16>::value ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
-  CUtensorMap tmx, tmw;
-  if (!gemm_tc_map(enc, &tmx, dt, x, K, total_rows, 1, ldx, 0, bn)) return 1;
-  if (!gemm_tc_map(enc, &tmw, dt, w, K, N, groups, ldw, sw, GT_BM)) return 1;
+  CUtensorMap tm[4];
+  if (!gemm_tc_map(enc, &tm[0], dt, w, K, N, groups, ldw, sw, GT_BM)) return 1;
+  if (!gemm_tc_map(enc, &tm[1], dt, x, K, total_rows, 1, ldx, 0, bn)) return 1;
+  tm[2] = tm[0];
+  tm[3] = tm[1];
+  if (two && !(gemm_tc_map(enc, &tm[2], dt, two->w, two->K, two->N, 1, two->ldw, 0, GT_BM) &&
+               gemm_tc_map(enc, &tm[3], dt, two->x, two->K, two->M, 1, two->ldx, 0, bn)))
+    return 1;
   GemmTcParams p;
-  p.y = y;
-  p.R = N; p.tokens = max_rows; p.ldy = ldy; p.sy = 0;
+  p.out[0] = {y, N, ldy};
+  p.tokens = max_rows; p.sy = 0;
   p.tiles_r = (int)((N + GT_BM - 1) / GT_BM);
   p.tiles_t = 1;
   const int64_t nt = (int64_t)p.tiles_r * groups;
@@ -733,12 +802,14 @@ int gemm_tc_launch_grouped(const T* x, const T* w, void* y, const int32_t* seg, 
   p.groups = (int)groups;
   p.epi = epi;
   p.act = act;
-  return bn == 32 ? gemm_tc_run<T, 32, 10>(tmw, tmx, p, st) : gemm_tc_run<T, 64, 8>(tmw, tmx, p, st);
+  gemm_tc_set_second(p, two, GT_BM);
+  return bn == 32 ? gemm_tc_run<T, 32, 10>(tm, p, st) : gemm_tc_run<T, 64, 8>(tm, p, st);
 }
 template int gemm_tc_launch_grouped<__half>(const __half*, const __half*, void*, const int32_t*, int64_t, int64_t, int64_t, int64_t, int64_t,
-                                            int64_t, int64_t, int64_t, int64_t, int, float2, cudaStream_t);
+                                            int64_t, int64_t, int64_t, int64_t, int, float2, const GemmTcPlain*, cudaStream_t);
 template int gemm_tc_launch_grouped<__nv_bfloat16>(const __nv_bfloat16*, const __nv_bfloat16*, void*, const int32_t*, int64_t, int64_t,
-                                                   int64_t, int64_t, int64_t, int64_t, int64_t, int64_t, int64_t, int, float2, cudaStream_t);
+                                                   int64_t, int64_t, int64_t, int64_t, int64_t, int64_t, int64_t, int, float2, const GemmTcPlain*,
+                                                   cudaStream_t);
 
 template int gemm_tc_launch<__half>(const __half*, const __half*, void*, int64_t, int64_t, int64_t, int64_t, int64_t, int64_t,
                                     int64_t, int64_t, int64_t, int64_t, int, float2, cudaStream_t);

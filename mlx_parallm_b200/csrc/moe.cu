@@ -12,27 +12,32 @@
 
 namespace b200p {
 
+bool pdl_enabled_gemm();
+// Programmatic launches for decode batches, where the gaps between these kernels are a tenth of the call (32 tokens, 16 experts of 2048 x
+// 2048: 129 -> 100 us with the shared expert's products beside the routed ones').  Prompts launch plainly: the gaps are a hundredth there, and
+// a stream that holds nothing but programmatic launches did not come to its end under CUPTI's kernel tracing.
+static bool moe_pdl(int64_t tokens) { return pdl_enabled_gemm() && tokens <= 64; }
+
 constexpr int MOE_MAX_PER_LANE = 32;    // experts <= 1024
 constexpr int MOE_MAX_TOP = 32;
 
-__global__ void moe_route_kernel(const float* __restrict__ logits, int64_t ldl, const float* __restrict__ bias,
-                                 int32_t* __restrict__ ids, float* __restrict__ wts, int64_t M, int E, int top) {
-  const int lane = threadIdx.x & 31;
-  const int64_t t = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (t >= M) return;
-  float z[MOE_MAX_PER_LANE];
+// One warp's token: the choice k goes to lane k.  PER_LANE * 32 experts at most.
+template <int PER_LANE>
+__device__ __forceinline__ void moe_route_token(const float* __restrict__ logits, int64_t ldl, const float* __restrict__ bias, int64_t t, int E,
+                                                int top, int lane, int& my_id, float& my_wt) {
+  float z[PER_LANE];
 #pragma unroll
-  for (int i = 0; i < MOE_MAX_PER_LANE; ++i) {
+  for (int i = 0; i < PER_LANE; ++i) {
     const int e = i * 32 + lane;
     z[i] = e < E ? logits[t * ldl + e] + (bias ? bias[e] : 0.f) : -INFINITY;
   }
   float first = 0.f, den = 0.f, mine = 0.f;
-  int my_id = 0;
+  my_id = 0;
   for (int k = 0; k < top; ++k) {
     float best = -INFINITY;
     int be = E;
 #pragma unroll
-    for (int i = 0; i < MOE_MAX_PER_LANE; ++i)
+    for (int i = 0; i < PER_LANE; ++i)
       if (z[i] > best) { best = z[i]; be = i * 32 + lane; }          // ascending e within a lane: ties keep the smallest index
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -40,17 +45,32 @@ __global__ void moe_route_kernel(const float* __restrict__ logits, int64_t ldl, 
       const int oe = __shfl_xor_sync(0xffffffffu, be, o);
       if (ob > best || (ob == best && oe < be)) { best = ob; be = oe; }
     }
+    if (be >= E) be = 0;                                             // nothing above -inf is left (NaN logits): the weights come out as NaN
     if (k == 0) first = best;
     const float p = expf(best - first);                              // the first pick is the largest: exponents <= 0
     den += p;
     if (lane == k) { mine = p; my_id = be; }
 #pragma unroll
-    for (int i = 0; i < MOE_MAX_PER_LANE; ++i)
+    for (int i = 0; i < PER_LANE; ++i)
       if (i * 32 + lane == be) z[i] = -INFINITY;
   }
+  my_wt = mine / den;
+}
+
+template <int PER_LANE>
+__global__ void moe_route_kernel(const float* __restrict__ logits, int64_t ldl, const float* __restrict__ bias,
+                                 int32_t* __restrict__ ids, float* __restrict__ wts, int64_t M, int E, int top) {
+  const int lane = threadIdx.x & 31;
+  const int64_t t = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  pdl_launch_dependents();
+  pdl_wait();
+  if (t >= M) return;
+  int id;
+  float wt;
+  moe_route_token<PER_LANE>(logits, ldl, bias, t, E, top, lane, id, wt);
   if (lane < top) {
-    ids[t * top + lane] = my_id;
-    wts[t * top + lane] = mine / den;
+    ids[t * top + lane] = id;
+    wts[t * top + lane] = wt;
   }
 }
 
@@ -65,6 +85,8 @@ __global__ void moe_route_scores_kernel(const float* __restrict__ logits, int64_
   extern __shared__ float mr_sm[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t t = (int64_t)blockIdx.x * (blockDim.x >> 5) + warp;
+  pdl_launch_dependents();
+  pdl_wait();
   if (t >= M) return;
   float* sc = mr_sm + (size_t)warp * (2 * E + count);     // scores
   float* pick = sc + E;                                    // picking scores, -inf once masked or taken
@@ -147,35 +169,92 @@ __global__ void moe_route_scores_kernel(const float* __restrict__ logits, int64_
   }
 }
 
-__global__ void moe_plan_kernel(const int32_t* __restrict__ ids, int32_t* __restrict__ seg, int32_t* __restrict__ slot_of,
-                                int32_t* __restrict__ token_of, int64_t n, int E, int top) {
-  extern __shared__ int32_t cnt[];               // [E] counts, then [E] cursors
+// Segments and slots of n chosen experts, one block.  id_of(i): the expert of (token, choice) i; cnt: [2 E] in shared memory.
+template <typename F>
+__device__ __forceinline__ void moe_plan(F id_of, int32_t* cnt, int32_t* __restrict__ seg, int32_t* __restrict__ slot_of,
+                                         int32_t* __restrict__ token_of, int64_t n, int E, int top) {
+  constexpr int B = 8;                           // reads in flight per thread
   int32_t* cur = cnt + E;
   for (int e = threadIdx.x; e < E; e += blockDim.x) cnt[e] = 0;
   __syncthreads();
-  for (int64_t i = threadIdx.x; i < n; i += blockDim.x) atomicAdd(&cnt[ids[i]], 1);
+  for (int64_t i0 = threadIdx.x; i0 < n; i0 += (int64_t)B * blockDim.x) {
+    int id[B];
+#pragma unroll
+    for (int r = 0; r < B; ++r) id[r] = i0 + r * (int64_t)blockDim.x < n ? id_of(i0 + r * (int64_t)blockDim.x) : -1;
+#pragma unroll
+    for (int r = 0; r < B; ++r)
+      if (id[r] >= 0) atomicAdd(&cnt[id[r]], 1);
+  }
   __syncthreads();
-  if (threadIdx.x == 0) {
+  if (threadIdx.x < 32) {                        // running sum of the counts
     int32_t run = 0;
-    for (int e = 0; e < E; ++e) {
-      seg[e] = run;
-      cur[e] = run;
-      run += cnt[e];
+    for (int e0 = 0; e0 < E; e0 += 32) {
+      const int e = e0 + (int)threadIdx.x, mine = e < E ? cnt[e] : 0;
+      int sum = mine;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, sum, o);
+        if ((int)threadIdx.x >= o) sum += v;
+      }
+      if (e < E) seg[e] = cur[e] = run + sum - mine;
+      run += __shfl_sync(0xffffffffu, sum, 31);
     }
-    seg[E] = run;
+    if (threadIdx.x == 0) seg[E] = run;
   }
   __syncthreads();
   // the order of an expert's rows is whatever the atomics give: every row is computed on its own, so the values do not depend on it
-  for (int64_t i = threadIdx.x; i < n; i += blockDim.x) {
-    const int32_t s = atomicAdd(&cur[ids[i]], 1);
-    slot_of[i] = s;
-    token_of[s] = (int32_t)(i / top);
+  for (int64_t i0 = threadIdx.x; i0 < n; i0 += (int64_t)B * blockDim.x) {
+    int id[B];
+#pragma unroll
+    for (int r = 0; r < B; ++r) id[r] = i0 + r * (int64_t)blockDim.x < n ? id_of(i0 + r * (int64_t)blockDim.x) : -1;
+#pragma unroll
+    for (int r = 0; r < B; ++r) {
+      if (id[r] < 0) continue;
+      const int64_t i = i0 + r * (int64_t)blockDim.x;
+      const int32_t s = atomicAdd(&cur[id[r]], 1);
+      slot_of[i] = s;
+      token_of[s] = (int32_t)(i / top);
+    }
   }
+}
+
+__global__ void moe_plan_kernel(const int32_t* __restrict__ ids, int32_t* __restrict__ seg, int32_t* __restrict__ slot_of,
+                                int32_t* __restrict__ token_of, int64_t n, int E, int top) {
+  extern __shared__ int32_t cnt[];               // [E] counts, then [E] cursors
+  pdl_launch_dependents();
+  pdl_wait();
+  moe_plan([&](int64_t i) { return ids[i]; }, cnt, seg, slot_of, token_of, n, E, top);
+}
+
+// Decode batches: choice and plan in one block (a launch less; 32 tokens, 16 experts, 2 of them each).
+constexpr int MOE_ONE_BLOCK = 1024;              // (token, choice) pairs
+template <int PER_LANE>
+__global__ void __launch_bounds__(1024)
+moe_route_plan_kernel(const float* __restrict__ logits, int64_t ldl, const float* __restrict__ bias, int32_t* __restrict__ ids,
+                      float* __restrict__ wts, int32_t* __restrict__ seg, int32_t* __restrict__ slot_of, int32_t* __restrict__ token_of,
+                      int64_t M, int E, int top) {
+  extern __shared__ int32_t cnt[];               // [E] counts, then [E] cursors
+  __shared__ int32_t chosen[MOE_ONE_BLOCK];
+  const int lane = threadIdx.x & 31;
+  pdl_launch_dependents();
+  pdl_wait();
+  for (int64_t t = threadIdx.x >> 5; t < M; t += blockDim.x >> 5) {
+    int id;
+    float wt;
+    moe_route_token<PER_LANE>(logits, ldl, bias, t, E, top, lane, id, wt);
+    if (lane < top) {
+      ids[t * top + lane] = chosen[t * top + lane] = id;
+      wts[t * top + lane] = wt;
+    }
+  }
+  moe_plan([&](int64_t i) { return chosen[i]; }, cnt, seg, slot_of, token_of, M * top, E, top);      // (its first barrier covers `chosen`)
 }
 
 template <typename T>
 __global__ void moe_gather_kernel(const T* __restrict__ x, const int32_t* __restrict__ token_of, T* __restrict__ xs, int64_t W) {
   const int64_t s = blockIdx.x;
+  pdl_launch_dependents();
+  pdl_wait();
   const T* src = x + (int64_t)token_of[s] * W;
   T* dst = xs + s * W;
   if (W % 8 == 0 && sizeof(T) == 2) {
@@ -192,6 +271,8 @@ __global__ void moe_scatter_scaled_kernel(const T* __restrict__ x, const int32_t
                                           T* __restrict__ xs, int64_t W) {
   const int64_t i = blockIdx.x;                        // (token, choice)
   const int top = gridDim.y;
+  pdl_launch_dependents();
+  pdl_wait();
   const int64_t tk = i * top + blockIdx.y;
   const float w = wts[tk];
   const T* src = x + i * W;
@@ -215,6 +296,8 @@ __global__ void moe_combine_kernel(const float* __restrict__ ye, const int32_t* 
                                    const float* __restrict__ shared_y, const float* __restrict__ shared_gate, int64_t ldg,
                                    float* __restrict__ y, int64_t W, int top) {
   const int64_t t = blockIdx.x;
+  pdl_launch_dependents();
+  pdl_wait();
   const float sg = shared_gate ? 1.f / (1.f + expf(-shared_gate[t * ldg])) : 1.f;
   __shared__ int32_t sl[MOE_MAX_TOP];
   __shared__ float wt[MOE_MAX_TOP];
@@ -247,6 +330,13 @@ __global__ void moe_combine_kernel(const float* __restrict__ ye, const int32_t* 
 
 using namespace b200p;
 
+static int moe_plan_launch(const int32_t* ids, int32_t* seg, int32_t* slot_of, int32_t* token_of, int64_t M, int E, int top, cudaStream_t st) {
+  cudaError_t e = launch_pdl_opt(moe_pdl(M), moe_plan_kernel, dim3(1), dim3(1024), 2 * E * sizeof(int32_t), st, ids, seg, slot_of, token_of,
+                                 M * top, E, top);
+  if (e != cudaSuccess) return cuda_fail(e, "moe_plan_kernel launch");
+  return B200P_OK;
+}
+
 extern "C" int b200p_moe_route(const float* logits, int64_t ldl, const float* bias, int32_t* ids, float* wts, int32_t* seg,
                                int32_t* slot_of, int32_t* token_of, int64_t M, int E, int top, void* stream) {
   B200P_REQUIRE(logits && ids && wts && seg && slot_of && token_of, B200P_ERR_ARG, "null pointer");
@@ -254,11 +344,18 @@ extern "C" int b200p_moe_route(const float* logits, int64_t ldl, const float* bi
                 "experts in [1, %d] and top in [1, min(experts, %d)]", 32 * MOE_MAX_PER_LANE, MOE_MAX_TOP);
   if (M == 0) return B200P_OK;
   cudaStream_t st = (cudaStream_t)stream;
-  moe_route_kernel<<<(unsigned)((M + 3) / 4), 128, 0, st>>>(logits, ldl, bias, ids, wts, M, E, top);
-  B200P_LAUNCH_CHECK("moe_route_kernel");
-  moe_plan_kernel<<<1, 1024, 2 * E * sizeof(int32_t), st>>>(ids, seg, slot_of, token_of, M * top, E, top);
-  B200P_LAUNCH_CHECK("moe_plan_kernel");
-  return B200P_OK;
+  const bool pdl = moe_pdl(M);
+  cudaError_t e;
+  if (M * top <= MOE_ONE_BLOCK && M <= 64) {
+    auto kern = E <= 32 ? moe_route_plan_kernel<1> : E <= 128 ? moe_route_plan_kernel<4> : moe_route_plan_kernel<MOE_MAX_PER_LANE>;
+    e = launch_pdl_opt(pdl, kern, dim3(1), dim3(1024), 2 * E * sizeof(int32_t), st, logits, ldl, bias, ids, wts, seg, slot_of, token_of, M, E, top);
+    if (e != cudaSuccess) return cuda_fail(e, "moe_route_plan_kernel launch");
+    return B200P_OK;
+  }
+  auto kern = E <= 32 ? moe_route_kernel<1> : E <= 128 ? moe_route_kernel<4> : moe_route_kernel<MOE_MAX_PER_LANE>;
+  e = launch_pdl_opt(pdl, kern, dim3((unsigned)((M + 3) / 4)), dim3(128), 0, st, logits, ldl, bias, ids, wts, M, E, top);
+  if (e != cudaSuccess) return cuda_fail(e, "moe_route_kernel launch");
+  return moe_plan_launch(ids, seg, slot_of, token_of, M, E, top, st);
 }
 
 extern "C" int b200p_moe_route_sigmoid(const float* logits, int64_t ldl, const float* correction, int32_t* ids, float* wts,
@@ -277,12 +374,10 @@ extern "C" int b200p_moe_route_sigmoid(const float* logits, int64_t ldl, const f
     cudaError_t e = cudaFuncSetAttribute(moe_route_scores_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(moe_route_scores_kernel)");
   }
-  moe_route_scores_kernel<<<(unsigned)((M + warps - 1) / warps), warps * 32, smem, st>>>(logits, ldl, correction, ids, wts, M, E, top,
-                                                                                           count, keep, scale, 1, 0, 0);
-  B200P_LAUNCH_CHECK("moe_route_scores_kernel");
-  moe_plan_kernel<<<1, 1024, 2 * E * sizeof(int32_t), st>>>(ids, seg, slot_of, token_of, M * top, E, top);
-  B200P_LAUNCH_CHECK("moe_plan_kernel");
-  return B200P_OK;
+  cudaError_t e = launch_pdl_opt(moe_pdl(M), moe_route_scores_kernel, dim3((unsigned)((M + warps - 1) / warps)), dim3(warps * 32), smem, st, logits,
+                                 ldl, correction, ids, wts, M, E, top, count, keep, scale, 1, 0, 0);
+  if (e != cudaSuccess) return cuda_fail(e, "moe_route_scores_kernel launch");
+  return moe_plan_launch(ids, seg, slot_of, token_of, M, E, top, st);
 }
 
 extern "C" int b200p_moe_route_scores(const float* logits, int64_t ldl, int32_t* ids, float* wts, int32_t* seg, int32_t* slot_of,
@@ -301,12 +396,10 @@ extern "C" int b200p_moe_route_scores(const float* logits, int64_t ldl, int32_t*
     cudaError_t e = cudaFuncSetAttribute(moe_route_scores_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(moe_route_scores_kernel)");
   }
-  moe_route_scores_kernel<<<(unsigned)((M + warps - 1) / warps), warps * 32, smem, st>>>(logits, ldl, nullptr, ids, wts, M, E, top,
-                                                                                          count, keep, 1.f, renorm, softmax, 1);
-  B200P_LAUNCH_CHECK("moe_route_scores_kernel");
-  moe_plan_kernel<<<1, 1024, 2 * E * sizeof(int32_t), st>>>(ids, seg, slot_of, token_of, M * top, E, top);
-  B200P_LAUNCH_CHECK("moe_plan_kernel");
-  return B200P_OK;
+  cudaError_t e = launch_pdl_opt(moe_pdl(M), moe_route_scores_kernel, dim3((unsigned)((M + warps - 1) / warps)), dim3(warps * 32), smem, st, logits,
+                                 ldl, nullptr, ids, wts, M, E, top, count, keep, 1.f, renorm, softmax, 1);
+  if (e != cudaSuccess) return cuda_fail(e, "moe_route_scores_kernel launch");
+  return moe_plan_launch(ids, seg, slot_of, token_of, M, E, top, st);
 }
 
 extern "C" int b200p_moe_scatter_scaled(const void* x, const int32_t* slot_of, const float* wts, void* xs, int64_t M, int64_t W, int top,
@@ -314,18 +407,20 @@ extern "C" int b200p_moe_scatter_scaled(const void* x, const int32_t* slot_of, c
   B200P_REQUIRE(x && slot_of && wts && xs && W > 0 && top > 0 && top <= MOE_MAX_TOP, B200P_ERR_ARG, "null pointer or bad top");
   B200P_REQUIRE(dtype == B200P_F32 || W % 8 != 0 || (aligned(x, 16) && aligned(xs, 16)), B200P_ERR_ALIGN, "x and xs must be 16-byte aligned");
   if (M == 0) return B200P_OK;
-  B200P_DISPATCH_DTYPE(dtype, T, (moe_scatter_scaled_kernel<T><<<dim3((unsigned)M, (unsigned)top), 128, 0, (cudaStream_t)stream>>>(
-      (const T*)x, slot_of, wts, (T*)xs, W)));
-  B200P_LAUNCH_CHECK("moe_scatter_scaled_kernel");
+  cudaError_t e = cudaSuccess;
+  B200P_DISPATCH_DTYPE(dtype, T, (e = launch_pdl_opt(moe_pdl(M), moe_scatter_scaled_kernel<T>, dim3((unsigned)M, (unsigned)top), dim3(128), 0,
+                                                     (cudaStream_t)stream, (const T*)x, slot_of, wts, (T*)xs, W)));
+  if (e != cudaSuccess) return cuda_fail(e, "moe_scatter_scaled_kernel launch");
   return B200P_OK;
 }
 
 extern "C" int b200p_moe_gather(const void* x, const int32_t* token_of, void* xs, int64_t slots, int64_t W, int dtype, void* stream) {
   B200P_REQUIRE(x && token_of && xs && W > 0, B200P_ERR_ARG, "null pointer");
   if (slots == 0) return B200P_OK;
-  B200P_DISPATCH_DTYPE(dtype, T, (moe_gather_kernel<T><<<(unsigned)slots, 128, 0, (cudaStream_t)stream>>>(
-      (const T*)x, token_of, (T*)xs, W)));
-  B200P_LAUNCH_CHECK("moe_gather_kernel");
+  cudaError_t e = cudaSuccess;
+  B200P_DISPATCH_DTYPE(dtype, T, (e = launch_pdl_opt(moe_pdl(slots / 4), moe_gather_kernel<T>, dim3((unsigned)slots), dim3(128), 0, (cudaStream_t)stream,
+                                                     (const T*)x, token_of, (T*)xs, W)));
+  if (e != cudaSuccess) return cuda_fail(e, "moe_gather_kernel launch");
   return B200P_OK;
 }
 
@@ -334,10 +429,9 @@ extern "C" int b200p_moe_combine(const float* ye, const int32_t* slot_of, const 
   B200P_REQUIRE(ye && slot_of && y && W > 0 && top > 0 && top <= MOE_MAX_TOP, B200P_ERR_ARG, "null pointer or bad top");
   if (M == 0) return B200P_OK;
   const unsigned threads = W >= 1024 ? 256 : 128;
-  if (W % 4 == 0 && aligned(ye, 16) && aligned(shared_y, 16) && aligned(y, 16))
-    moe_combine_kernel<4><<<(unsigned)M, threads, 0, (cudaStream_t)stream>>>(ye, slot_of, wts, shared_y, shared_gate, ldg, y, W, top);
-  else
-    moe_combine_kernel<1><<<(unsigned)M, threads, 0, (cudaStream_t)stream>>>(ye, slot_of, wts, shared_y, shared_gate, ldg, y, W, top);
-  B200P_LAUNCH_CHECK("moe_combine_kernel");
+  auto kern = W % 4 == 0 && aligned(ye, 16) && aligned(shared_y, 16) && aligned(y, 16) ? moe_combine_kernel<4> : moe_combine_kernel<1>;
+  cudaError_t e = launch_pdl_opt(moe_pdl(M), kern, dim3((unsigned)M), dim3(threads), 0, (cudaStream_t)stream, ye, slot_of, wts, shared_y,
+                                 shared_gate, ldg, y, W, top);
+  if (e != cudaSuccess) return cuda_fail(e, "moe_combine_kernel launch");
   return B200P_OK;
 }

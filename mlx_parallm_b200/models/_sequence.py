@@ -844,11 +844,16 @@ class RoutedExperts:
             ops.moe_scatter_scaled(x, slot_of, wts, xs, self.top)
         else:
             ops.moe_gather(x, token_of, xs)
-        act = ops.gemm_grouped(xs, self.gate_up, seg, M, self.epilogue, out=s.get("moe_act", dt, n, self.ff), act=(self.limit, 0.0))
-        ye = ops.gemm_grouped(act, self.down, seg, M, GEMM_STORE_F32, out=s.get("moe_y", f32, n, self.width))
-        ysh = None
-        if self.shared is not None:
-            ysh = self.shared(x, s.get("y_shared", f32, M, self.width), s)
+        sh, ysh, also, also_down = self.shared, None, None, None
+        if sh is not None:
+            ysh = s.get("y_shared", f32, M, self.width)
+            if sh.epilogue == self.epilogue and sh.limit == self.limit:      # the shared expert's products beside the routed ones'
+                act_sh = s.get("act", dt, M, sh.ff)
+                also, also_down = (x, sh.gate_up.weight, act_sh), (act_sh, sh.down.weight, ysh)
+            else:
+                sh(x, ysh, s)
+        act = ops.gemm_grouped(xs, self.gate_up, seg, M, self.epilogue, out=s.get("moe_act", dt, n, self.ff), act=(self.limit, 0.0), also=also)
+        ye = ops.gemm_grouped(act, self.down, seg, M, GEMM_STORE_F32, out=s.get("moe_y", f32, n, self.width), also=also_down)
         ops.moe_combine(ye, slot_of, None if on_input else wts, ysh, y_out, self.top, shared_gate=logits[:, self.experts:self.experts + 1] if self.shared_gate else None)
         return y_out
 

@@ -384,8 +384,10 @@ def linear_attn_prep(proj, head_decay, q, k, v, decay, H, dk, dv):
                                                                         _p(decay), M, H, dk, dv, _stream()))
 
 
-def gemm_grouped(x, w, seg, max_rows: int, epilogue=_lib.GEMM_STORE, out=None, act=(0.0, 0.0)):
-    """Rows [seg[z], seg[z+1]) of x times the z-th block of w [groups, N, K] (b200p_gemm_grouped); ``seg`` int32 on the device."""
+def gemm_grouped(x, w, seg, max_rows: int, epilogue=_lib.GEMM_STORE, out=None, act=(0.0, 0.0), also=None):
+    """Rows [seg[z], seg[z+1]) of x times the z-th block of w [groups, N, K] (b200p_gemm_grouped); ``seg`` int32 on the device.
+    ``also`` = (x2 [M2, K2], w2 [N2, K2], out2): a plain product with the same epilogue beside them, in the same launch where that
+    is possible (b200p_gemm_grouped_with)."""
     _dev(x, w, seg, out)
     groups, N, K = w.shape
     assert x.dtype == w.dtype and x.stride(-1) == 1 and w.is_contiguous() and x.shape[1] == K and seg.dtype == torch.int32
@@ -394,9 +396,20 @@ def gemm_grouped(x, w, seg, max_rows: int, epilogue=_lib.GEMM_STORE, out=None, a
     if out is None:
         out = torch.empty((x.shape[0], N // 2 if glu else N), dtype=want, device=x.device)
     assert out.dtype == want and out.stride(-1) == 1
-    _call(("b200p_gemm_grouped", N, K, groups), lambda: lib().b200p_gemm_grouped(
-        _p(x), _p(w), _p(out), _p(seg), x.shape[0], int(max_rows), N, K, x.stride(0), K, out.stride(0), groups, N * K, dtype_code(x.dtype),
-        epilogue, float(act[0]), float(act[1]), _stream()))
+    if also is None:
+        _call(("b200p_gemm_grouped", N, K, groups), lambda: lib().b200p_gemm_grouped(
+            _p(x), _p(w), _p(out), _p(seg), x.shape[0], int(max_rows), N, K, x.stride(0), K, out.stride(0), groups, N * K, dtype_code(x.dtype),
+            epilogue, float(act[0]), float(act[1]), _stream()))
+        return out
+    x2, w2, out2 = also
+    _dev(x2, w2, out2)
+    (M2, K2), N2 = x2.shape, w2.shape[0]
+    assert x2.dtype == w2.dtype == x.dtype and x2.stride(1) == 1 and w2.stride(1) == 1 and w2.shape[1] == K2
+    assert out2.dtype == want and out2.stride(1) == 1 and out2.shape == (M2, N2 // 2 if glu else N2)
+    _call(("b200p_gemm_grouped", N, K, groups), lambda: lib().b200p_gemm_grouped_with(
+        _p(x), _p(w), _p(out), _p(seg), x.shape[0], int(max_rows), N, K, x.stride(0), K, out.stride(0), groups, N * K, _p(x2), _p(w2),
+        _p(out2), M2, N2, K2, x2.stride(0), w2.stride(0), out2.stride(0), dtype_code(x.dtype), epilogue, float(act[0]), float(act[1]),
+        _stream()))
     return out
 
 

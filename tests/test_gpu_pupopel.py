@@ -678,3 +678,32 @@ def test_checkpoint_on_disk_and_trace_runner(tmp_path, models):
     assert not (out / "2.f32").exists()
     s3 = torch.from_numpy(np.fromfile(out / "3.f32", dtype="<f4").reshape(1, V))
     assert O.logits_error(s3, wa[11:12]) < F32_TOL
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("E,top,tokens,N,K,N2,K2", [(16, 2, 32, 512, 128, 768, 192), (16, 2, 64, 1300, 128, 2, 64), (8, 4, 65, 264, 200, 1030, 72), (8, 2, 700, 512, 128, 520, 320),
+                                                    (4, 1, 3, 128, 64, 256, 64), (16, 1, 40, 2048, 64, 130, 40)])
+def test_grouped_products_with_a_plain_one(dtype, E, top, tokens, N, K, N2, K2):
+    """The shared expert's product in the launch of the routed ones (and beside it where they cannot share one: few groups, float32, a K of
+    less than 64): both equal what they are alone up to the order of fp32 sums, gated and plain, and nothing else is written."""
+    from mlx_parallm_b200 import _lib, ops
+    g = torch.Generator().manual_seed(tokens + N)
+    cnt = torch.bincount(torch.randint(0, E, (tokens * top,), generator=g), minlength=E).clamp(max=tokens)
+    seg = torch.cat([torch.zeros(1, dtype=torch.long), cnt.cumsum(0)])
+    x, w = torch.randn(tokens * top, K, generator=g).to(dtype), (torch.randn(E, N, K, generator=g) / math.sqrt(K)).to(dtype)
+    x2, w2 = torch.randn(tokens, K2, generator=g).to(dtype), (torch.randn(N2, K2, generator=g) / math.sqrt(K2)).to(dtype)
+    for epi in (_lib.GEMM_STORE_F32, _lib.GEMM_GLU_SILU):
+        gated = epi == _lib.GEMM_GLU_SILU
+        out_t = dtype if gated else torch.float32
+        y = torch.full((tokens * top, N // 2 if gated else N), 5.0, dtype=out_t, device="cuda")
+        y2 = torch.full((tokens + 1, N2 // 2 if gated else N2), 5.0, dtype=out_t, device="cuda")
+        ops.gemm_grouped(x.cuda(), w.cuda(), seg.to(torch.int32).cuda(), tokens, epi, out=y, also=(x2.cuda(), w2.cuda(), y2[:tokens]))
+        tol = 2.0 ** -8 if gated and dtype == torch.bfloat16 else 2.0 ** -11 if gated and dtype == torch.float16 else 2e-6 * math.sqrt(max(K, K2))
+        f = (lambda z: O.silu(z[:, 0::2]) * z[:, 1::2]) if gated else (lambda z: z)
+        want = torch.cat([f(x[int(seg[e]):int(seg[e + 1])].double() @ w[e].double().T) for e in range(E)])
+        assert (y[:int(seg[-1])].double().cpu() - want).abs().max() <= tol * max(1.0, float(want.abs().max())), epi
+        assert int(seg[-1]) == len(y) or float((y[int(seg[-1]):] - 5.0).abs().max()) == 0.0
+        want = f(x2.double() @ w2.double().T)
+        assert (y2[:tokens].double().cpu() - want).abs().max() <= tol * max(1.0, float(want.abs().max())), epi
+        assert float((y2[tokens:] - 5.0).abs().max()) == 0.0
+    assert _lib.lib().b200p_gemm_tc_fault() == 0
