@@ -388,7 +388,8 @@ int b200p_delta_scan(const float* qn, const float* kn, const float* v, const flo
                      const int32_t* cu, const int32_t* rows, const int32_t* lengths, float* o, int nb, int H, int KH, int dk,
                      int dv, int mode, void* stream);
 /* the same, told how many tokens the entries have together (cu[nb], which lies on the device): decode steps take a kernel of their own.
- * Results do not depend on it. */
+ * Results do not depend on it (an entry of 32 tokens and more beside as many empty ones excepted: fp32 rounding).  Entries of 32 tokens and
+ * more with keys of 65 to 128 channels take two tokens at a time in the delta rule: the same sums in another order than token by token. */
 int b200p_delta_scan_tokens(const float* qn, const float* kn, const float* v, const float* beta, const float* decay, float* state,
                             const int32_t* cu, const int32_t* rows, const int32_t* lengths, float* o, int64_t tokens, int nb, int H, int KH,
                             int dk, int dv, int mode, void* stream);

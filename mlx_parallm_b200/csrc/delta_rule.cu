@@ -7,13 +7,15 @@
 // The same kernels carry the variants other designs use: a decay per head AND key channel (a row of S each), a gate that is a
 // sigmoid of a separate tensor, and the plain decayed accumulation S <- g S + k v^T (linear attention with a constant decay,
 // fed by linear_attn_prep_kernel).
-// Prompts and single decoded tokens run the SAME scan kernel in the same summation order, so a prompt cut into portions gives
-// the same numbers as one pass.
+// An entry's numbers depend on its own tokens alone.  Single tokens and entries of less than 32 run in one summation order, whatever kernel takes
+// them; entries of 32 tokens and more (keys of 65 to 128 channels, delta rule) two tokens at a time (delta_pair_kernel), which differs in the last
+// places.
 #include "common.cuh"
 
 namespace b200p {
 
 int sm_count();
+bool pdl_enabled_gemm();
 
 __device__ __forceinline__ float silu_f(float z) { return z / (1.f + __expf(-z)); }
 __device__ __forceinline__ float softplus_f(float z) { return z > 20.f ? z : log1pf(expf(z)); }
@@ -325,7 +327,7 @@ __global__ void __launch_bounds__(LANES * ds_slots(DKP), PER_SM)
 delta_scan_kernel(const float* __restrict__ qn, const float* __restrict__ kn, const float* __restrict__ v,
                   const float* __restrict__ beta, const float* __restrict__ decay, float* __restrict__ state,
                   const int32_t* __restrict__ cu, const int32_t* __restrict__ rows, const int32_t* __restrict__ lengths,
-                  float* __restrict__ o, int H, int KH, int dk, int dv) {
+                  float* __restrict__ o, int H, int KH, int dk, int dv, int most) {
   constexpr int SEGS = ds_segs(DKP), SUB = SEGS / LANES, SEG = DKP / SEGS;
   constexpr int DS_SLOTS = ds_slots(DKP), DS_COLS = 2 * DS_SLOTS, DS_THREADS = LANES * DS_SLOTS;
   constexpr int CHUNK = DKP <= 128 ? 8 : 1024 / DKP;             // tokens staged at a time
@@ -344,7 +346,10 @@ delta_scan_kernel(const float* __restrict__ qn, const float* __restrict__ kn, co
   const bool pairs = NEXT == 1 && (dv & 1) == 0 && (reinterpret_cast<uintptr_t>(state) & 7) == 0;
   const bool live0 = j0 < dv, live1 = j1 < dv, odd = (l & 1) != 0;
   const int t0 = cu[e], t1 = cu[e + 1];
-  if (t1 <= t0) return;
+  if (t1 <= t0 || t1 - t0 > most) {                              // (longer entries: delta_pair_kernel, launched before)
+    pdl_wait();
+    return;
+  }
   const int row = rows[e];
   const int kh = h / (H / KH);
   const int r0 = l * SUB * SEG, l0 = l * SUB * (SEG + 4);        // first row of the lane, and where it lies in the staging buffers
@@ -447,6 +452,7 @@ delta_scan_kernel(const float* __restrict__ qn, const float* __restrict__ kn, co
     __syncthreads();
   }
   put(t1 - 1, ds_reduce<LANES>(out.x, out.y, odd));
+  pdl_wait();                         // (see delta_scan_launch: ends no earlier than the launch before)
 #pragma unroll
   for (int u = 0; u < SUB; ++u)
 #pragma unroll
@@ -465,6 +471,240 @@ delta_scan_kernel(const float* __restrict__ qn, const float* __restrict__ kn, co
       if (r0 + r + 1 < dk) {
         if (live0) s0[dv + j0] = S.c0[u][i].y;
         if (live1) s0[dv + j1] = S.c1[u][i].y;
+      }
+    }
+}
+
+// Prompts of keys of 65 to 128 channels, two tokens at a time.  In the kernels above the chain of one token (dot, reduction over the lanes,
+// update, dot) and the reads of shared memory for it are what bounds a CTA.  With g1, k1, q1, v1 and g2, k2, q2, v2 of two tokens and the
+// state S before them,
+//     u1 = b1 (v1 - S^T (g1 k1))                 o1 = S^T (g1 q1) + (q1 . k1) u1
+//     u2 = b2 (v2 - S^T (g1 g2 k2) - (k2 . g2 k1) u1)      o2 = S^T (g1 g2 q2) + (q2 . g2 k1) u1 + (q2 . k2) u2
+//     S <- g1 g2 S + (g2 k1) u1 + k2 u2
+// so that four dot products with one state share a pass and a reduction, and 7 instead of 8 operations per element and pair are left.  The scaled
+// vectors and the four scalars are the same for all columns: the threads that stage a token's row compute them.  All of it stays fp32.
+// A thread holds 16 rows of FOUR columns: a 16-byte read of shared memory (four cycles of its port for a warp) serves 16 packed products; eight
+// lanes share a column slot.  The exchanges for u run beside the products with the queries, those for o beside the update.
+// An entry takes this path if it has at least DP_MIN tokens, whatever the others have, so its bits do not depend on its batch; a prompt
+// whose portions are shorter has the bits of single tokens, which differ in the last places.
+// Bound: FFMA2 with three distinct operands, one in about four cycles per scheduler (measured; scalar FFMA, two in 2.5, needs registers that are
+// not there: 274 us).  us before -> now, heads of 128 x 128, decays per channel / per head: 4 x 512 tokens, 16 heads 221 -> 156 / 193 -> 152, 32
+// heads 357 -> 266 / 315 -> 260 (two CTAs per SM; one: 304 / 298); 16 x 250, 32 heads 635 -> 449 / 542 -> 441; 1 x 32, 16 heads 18.6 -> 14.5.
+constexpr int DP_MIN = 32, DP_CHUNK = 8, DP_COLS = 64, DP_LDK = 160;
+// warps 0 .. 3 compute, 4 .. 7 stage; two CTAs per SM: registers at launch 256 x 128 = 128 x 168 + 128 x 88
+constexpr int DP_TEAM = 128, DP_THREADS = 2 * DP_TEAM, DP_REGS_COMPUTE = 168, DP_REGS_STAGE = 88;
+template <int MODE, int PER_SM>
+__global__ void __launch_bounds__(DP_THREADS, PER_SM)
+delta_pair_kernel(const float* __restrict__ qn, const float* __restrict__ kn, const float* __restrict__ v, const float* __restrict__ beta,
+                  const float* __restrict__ decay, float* __restrict__ state, const int32_t* __restrict__ cu, const int32_t* __restrict__ rows,
+                  const int32_t* __restrict__ lengths, float* __restrict__ o, int H, int KH, int dk, int dv) {
+  enum { K1, K2, Q1, Q2, GG, KD, KU, VECS };                   // g1 k1, g1 g2 k2, g1 q1, g1 g2 q2, g1 g2, g2 k1, k2
+  constexpr int PAIRS = DP_CHUNK / 2;
+  __shared__ __align__(16) float vec[2][PAIRS][VECS][DP_LDK];  // 16 rows per lane, padded by 16 bytes: the lanes' reads fall into different banks
+  __shared__ __align__(16) float dots[2][PAIRS][4][4];         // k2 . kd, q1 . k1, q2 . kd, q2 . k2: a share per warp
+  __shared__ __align__(16) float vs[2][DP_CHUNK][DP_COLS];
+  __shared__ float bs[2][DP_CHUNK];
+  const int e = blockIdx.x, h = blockIdx.y, tid = threadIdx.x & (DP_TEAM - 1), lane = tid & 31, warp = tid >> 5;
+  pdl_launch_dependents();
+  const int t0 = cu[e], t1 = cu[e + 1];
+  if (t1 - t0 < DP_MIN) return;
+  const int row = rows[e], kh = h / (H / KH);
+  if (threadIdx.x >= DP_TEAM) {
+    if constexpr (PER_SM == 2) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(DP_REGS_STAGE));
+    // ===================================== staging =====================================
+    // Inputs travel to registers a chunk ahead; tokens past the end are ones that change nothing.
+    float pk[DP_CHUNK], pq[DP_CHUNK], pg[DP_CHUNK], pv[4], pb = 0.f;
+    auto fetch = [&](int tc) {
+#pragma unroll
+      for (int t = 0; t < DP_CHUNK; ++t) {
+        const bool ok = tc + t < t1 && tid < dk;
+        const int64_t src = ((int64_t)(tc + t) * KH + kh) * dk + tid;
+        pk[t] = ok ? kn[src] : 0.f;
+        pq[t] = ok ? qn[src] : 0.f;
+        if constexpr (MODE == 1) pg[t] = ok ? decay[((int64_t)(tc + t) * H + h) * dk + tid] : 1.f;
+        else pg[t] = tc + t < t1 ? decay[(int64_t)(tc + t) * H + h] : 1.f;
+      }
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const int idx = tid + r * DP_TEAM, t = idx / DP_COLS, c = blockIdx.z * DP_COLS + idx % DP_COLS;
+        pv[r] = tc + t < t1 && c < dv ? v[((int64_t)(tc + t) * H + h) * dv + c] : 0.f;
+      }
+      if (tid < DP_CHUNK) pb = tc + tid < t1 ? beta[(int64_t)(tc + tid) * H + h] : 0.f;
+    };
+    auto park = [&](int buf) {
+      const int at = tid + (tid >> 4) * 4;
+      float d[4 * PAIRS];
+#pragma unroll
+      for (int p = 0; p < PAIRS; ++p) {
+        const float g1 = pg[2 * p], g2 = pg[2 * p + 1], k1 = pk[2 * p], k2 = pk[2 * p + 1], q1 = pq[2 * p], q2 = pq[2 * p + 1];
+        const float gg = g1 * g2, kd = g2 * k1;
+        float (*w)[DP_LDK] = vec[buf][p];
+        w[K1][at] = g1 * k1;
+        w[K2][at] = gg * k2;
+        w[Q1][at] = g1 * q1;
+        w[Q2][at] = gg * q2;
+        w[GG][at] = gg;
+        w[KD][at] = kd;
+        w[KU][at] = k2;
+        d[4 * p] = k2 * kd;
+        d[4 * p + 1] = q1 * k1;
+        d[4 * p + 2] = q2 * kd;
+        d[4 * p + 3] = q2 * k2;
+      }
+      // 16 sums over 32 lanes: halve the values with every exchange, lane l ends up with sum (l >> 1)
+#pragma unroll
+      for (int n = 8, m = 16; n >= 1; n >>= 1, m >>= 1) {
+        const bool up = (lane & m) != 0;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          if (i >= n) continue;
+          const float give = up ? d[i] : d[n + i], keep = up ? d[n + i] : d[i];
+          d[i] = keep + __shfl_xor_sync(0xffffffffu, give, m);
+        }
+      }
+      d[0] += __shfl_xor_sync(0xffffffffu, d[0], 1);
+      if (!(lane & 1)) dots[buf][lane >> 3][(lane >> 1) & 3][warp] = d[0];
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const int idx = tid + r * DP_TEAM;
+        vs[buf][idx / DP_COLS][idx % DP_COLS] = pv[r];
+      }
+      if (tid < DP_CHUNK) bs[buf][tid] = pb;
+    };
+    fetch(t0);
+    park(0);
+    fetch(t0 + DP_CHUNK);
+    __syncthreads();
+    int buf = 0;
+    for (int tc = t0; tc < t1; tc += DP_CHUNK, buf ^= 1) {      // (the other buffer was last read in the previous iteration)
+      if (tc + DP_CHUNK < t1) park(buf ^ 1);
+      if (tc + 2 * DP_CHUNK < t1) fetch(tc + 2 * DP_CHUNK);
+      __syncthreads();
+    }
+    return;
+  }
+  if constexpr (PER_SM == 2) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(DP_REGS_COMPUTE));
+  // ===================================== recurrence ==================================
+  const int l = tid & 7, slot = tid >> 3, j0 = blockIdx.z * DP_COLS + 4 * slot;    // this thread's columns j0 .. j0 + 3, rows 16 l .. 16 l + 15
+  const bool vec4 = (dv & 3) == 0 && (reinterpret_cast<uintptr_t>(state) & 15) == 0 && j0 + 3 < dv;
+  float* sp = state + (((int64_t)row * H + h) * dk + 16 * l) * dv + j0;
+  const bool fresh = lengths[row] == 0;
+  float2 S[4][8];                                              // [column][row pair]
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int b = 0; b < 2; ++b) {
+      const int r = 2 * i + b;
+      float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (!fresh && 16 * l + r < dk) {
+        const float* s0 = sp + (int64_t)r * dv;
+        if (vec4) x = *reinterpret_cast<const float4*>(s0);
+        else {
+          if (j0 < dv) x.x = s0[0];
+          if (j0 + 1 < dv) x.y = s0[1];
+          if (j0 + 2 < dv) x.z = s0[2];
+          if (j0 + 3 < dv) x.w = s0[3];
+        }
+      }
+      (b ? S[0][i].y : S[0][i].x) = x.x;
+      (b ? S[1][i].y : S[1][i].x) = x.y;
+      (b ? S[2][i].y : S[2][i].x) = x.z;
+      (b ? S[3][i].y : S[3][i].x) = x.w;
+    }
+  const int jo = j0 + (l & 3);                                 // the column whose outputs this lane writes
+  __syncthreads();
+  int buf = 0;
+  for (int tc = t0; tc < t1; tc += DP_CHUNK, buf ^= 1) {
+    auto step = [&](int p) {
+      const float* w = &vec[buf][p][0][20 * l];
+      // this thread's rows of two dot products with the four columns
+      auto dot2 = [&](int s0, float (&r1)[4], float (&r2)[4]) {
+        float2 a[2][4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) a[0][c] = a[1][c] = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int s = 0; s < 2; ++s) {
+            const float4 x = *reinterpret_cast<const float4*>(w + (s0 + s) * DP_LDK + 4 * i);
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+              a[s][c] = __ffma2_rn(S[c][2 * i], make_float2(x.x, x.y), a[s][c]);
+              a[s][c] = __ffma2_rn(S[c][2 * i + 1], make_float2(x.z, x.w), a[s][c]);
+            }
+          }
+#pragma unroll
+        for (int c = 0; c < 4; ++c) r1[c] = a[0][c].x + a[0][c].y, r2[c] = a[1][c].x + a[1][c].y;
+      };
+      // over the eight lanes: lane l < 4 gets the first product's sum of column l, lane l + 4 the second's
+      auto reduce = [&](const float (&r1)[4], const float (&r2)[4]) {
+        const bool b4 = (l & 4) != 0, b2 = (l & 2) != 0, b1 = (l & 1) != 0;
+        float r[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) r[c] = (b4 ? r2[c] : r1[c]) + __shfl_xor_sync(0xffffffffu, b4 ? r1[c] : r2[c], 4);
+#pragma unroll
+        for (int c = 0; c < 2; ++c) r[c] = (b2 ? r[c + 2] : r[c]) + __shfl_xor_sync(0xffffffffu, b2 ? r[c] : r[c + 2], 2);
+        return (b1 ? r[1] : r[0]) + __shfl_xor_sync(0xffffffffu, b1 ? r[0] : r[1], 1);
+      };
+      float r1[4], r2[4], y1[4], y2[4];
+      dot2(K1, r1, r2);
+      const float sk = reduce(r1, r2);
+      dot2(Q1, y1, y2);                                        // (beside the exchanges of the sums for u)
+      auto dot_of = [&](int d) {
+        const float4 x = *reinterpret_cast<const float4*>(dots[buf][p][d]);
+        return (x.x + x.y) + (x.z + x.w);
+      };
+      const float k2kd = dot_of(0), q1k1 = dot_of(1), q2kd = dot_of(2), q2k2 = dot_of(3), b1 = bs[buf][2 * p], b2 = bs[buf][2 * p + 1];
+      const float4 v1 = *reinterpret_cast<const float4*>(&vs[buf][2 * p][4 * slot]), v2 = *reinterpret_cast<const float4*>(&vs[buf][2 * p + 1][4 * slot]);
+      const float va[4] = {v1.x, v1.y, v1.z, v1.w}, vb[4] = {v2.x, v2.y, v2.z, v2.w};
+      float u1[4], u2[4];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const float s1 = __shfl_sync(0xffffffffu, sk, c, 8), s2 = __shfl_sync(0xffffffffu, sk, c + 4, 8);
+        u1[c] = b1 * (va[c] - s1);
+        u2[c] = b2 * (vb[c] - fmaf(k2kd, u1[c], s2));
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float4 g = *reinterpret_cast<const float4*>(w + GG * DP_LDK + 4 * i), kd = *reinterpret_cast<const float4*>(w + KD * DP_LDK + 4 * i);
+        const float4 ku = *reinterpret_cast<const float4*>(w + KU * DP_LDK + 4 * i);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          const float2 ua = make_float2(u1[c], u1[c]), ub = make_float2(u2[c], u2[c]);
+          S[c][2 * i] = __ffma2_rn(make_float2(ku.x, ku.y), ub, __ffma2_rn(make_float2(kd.x, kd.y), ua, __fmul2_rn(S[c][2 * i], make_float2(g.x, g.y))));
+          S[c][2 * i + 1] = __ffma2_rn(make_float2(ku.z, ku.w), ub, __ffma2_rn(make_float2(kd.z, kd.w), ua, __fmul2_rn(S[c][2 * i + 1], make_float2(g.z, g.w))));
+        }
+      }
+      const float sq = reduce(y1, y2);                         // (beside the update)
+      const bool c2 = (l & 2) != 0, c1 = (l & 1) != 0;
+      const float ua = c2 ? (c1 ? u1[3] : u1[2]) : (c1 ? u1[1] : u1[0]), ub = c2 ? (c1 ? u2[3] : u2[2]) : (c1 ? u2[1] : u2[0]);
+      const float out = l < 4 ? fmaf(q1k1, ua, sq) : fmaf(q2k2, ub, fmaf(q2kd, ua, sq));
+      const int t = tc + 2 * p + (l >> 2);
+      if (jo < dv && t < t1) o[((int64_t)t * H + h) * dv + jo] = out;
+    };
+    if (t1 - tc >= DP_CHUNK) {
+#pragma unroll
+      for (int p = 0; p < PAIRS; ++p) step(p);
+    } else {
+#pragma unroll 1
+      for (int p = 0; tc + 2 * p < t1; ++p) step(p);
+    }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int b = 0; b < 2; ++b) {
+      const int r = 2 * i + b;
+      if (16 * l + r >= dk) continue;
+      const float4 x = b ? make_float4(S[0][i].y, S[1][i].y, S[2][i].y, S[3][i].y) : make_float4(S[0][i].x, S[1][i].x, S[2][i].x, S[3][i].x);
+      float* s0 = sp + (int64_t)r * dv;
+      if (vec4) *reinterpret_cast<float4*>(s0) = x;
+      else {
+        if (j0 < dv) s0[0] = x.x;
+        if (j0 + 1 < dv) s0[1] = x.y;
+        if (j0 + 2 < dv) s0[2] = x.z;
+        if (j0 + 3 < dv) s0[3] = x.w;
       }
     }
 }
@@ -667,9 +907,9 @@ static void delta_scan_launch(int64_t tokens, int nb, cudaStream_t st, const flo
   delta_step_kernel<DKP, MODE><<<dim3((unsigned)nb, (unsigned)H, (unsigned)((dv + dt_cols(DKP) - 1) / dt_cols(DKP))), DT_THREADS, 0, st>>>( \
       qn, kn, v, beta, decay, state, cu, rows, lengths, o, H, KH, dk, dv)
 #define DELTA_SCAN(DKP, LANES, PER_SM)                                                                                           \
-  delta_scan_kernel<DKP, MODE, LANES, PER_SM>                                                                                     \
-      <<<dim3((unsigned)nb, (unsigned)H, (unsigned)((dv + 2 * ds_slots(DKP) - 1) / (2 * ds_slots(DKP)))), LANES * ds_slots(DKP), 0, st>>>( \
-          qn, kn, v, beta, decay, state, cu, rows, lengths, o, H, KH, dk, dv)
+  launch_pdl_opt(pairs && pdl_enabled_gemm(), delta_scan_kernel<DKP, MODE, LANES, PER_SM>,                                        \
+                 dim3((unsigned)nb, (unsigned)H, (unsigned)((dv + 2 * ds_slots(DKP) - 1) / (2 * ds_slots(DKP)))), dim3(LANES * ds_slots(DKP)), 0, st, \
+                 qn, kn, v, beta, decay, state, cu, rows, lengths, o, H, KH, dk, dv, pairs ? DP_MIN - 1 : INT32_MAX)
   // The step kernel for decode steps, and for as many tokens per entry as it keeps up with the scan (us, step / scan): 128 x 128, 16
   // entries of 1 / 2 / 4 tokens, 32 heads, 21.7 / 23.1, 27.1 / 25.3, 32.0 / 29.2; 64 x 64, 32 heads, of 2 / 4 / 8, 6.8 / 8.8, 7.9 / 9.6,
   // 10.2 / 11.4, but with 16 heads 4.3 / 4.6, 5.1 / 5.0, 7.3 / 6.4; 32 x 64, 16 heads, of 2 / 4, 3.4 / 3.5, 4.2 / 3.9; 256 x 256, 8 heads,
@@ -681,6 +921,15 @@ static void delta_scan_launch(int64_t tokens, int nb, cudaStream_t st, const flo
   // head: 220 / 193 us, the former four-lane kernel 280 / 206); more CTAs than SMs take four (32 heads 379 / 346 -> 356 / 317; 16 x 250
   // tokens 672 / 594 -> 637 / 544).
   const bool crowded = (int64_t)nb * H * ((dv + 63) / 64) > sm_count();
+  // Entries of DP_MIN tokens and more two tokens at a time, the shorter ones by the launch behind it, which needs nothing of it: it may start
+  // at once (its inputs were complete when the first began) and waits for it only at its end, so that what follows waits for both.
+  const bool pairs = MODE != 2 && dk > 64 && dk <= 128 && !few && (tokens == 0 || tokens >= DP_MIN);
+  if constexpr (MODE != 2) {
+    const auto pair_kernel = crowded ? delta_pair_kernel<MODE, 2> : delta_pair_kernel<MODE, 1>;
+    if (pairs)
+      pair_kernel<<<dim3((unsigned)nb, (unsigned)H, (unsigned)((dv + DP_COLS - 1) / DP_COLS)), DP_THREADS, 0, st>>>(
+          qn, kn, v, beta, decay, state, cu, rows, lengths, o, H, KH, dk, dv);
+  }
   if (dk > 256) { if (few) DELTA_STEP(512); else DELTA_SCAN(512, 16, 1); }
   else if (dk > 128) { if (few) DELTA_STEP(256); else DELTA_SCAN(256, 8, 1); }
   else if (dk > 64) { if (few) DELTA_STEP(128); else if (crowded) DELTA_SCAN(128, 4, 2); else DELTA_SCAN(128, 8, 1); }

@@ -705,6 +705,49 @@ def test_delta_scan_of_decode_steps_equals_the_scan_of_prompts(mode, dk, dv, H, 
     assert torch.equal(got[0][1].view_as(state0)[3], state0[3])             # a row that no entry names is not touched
 
 
+@pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("dk,dv,H,KH,shift", [(128, 128, 4, 2, 0), (65, 31, 2, 1, 0), (100, 66, 4, 4, 1), (128, 192, 2, 2, 1)])
+def test_delta_scan_of_long_entries(mode, dk, dv, H, KH, shift):
+    """Entries of 32 tokens and more go two tokens at a time: against a float64 loop, odd lengths, lengths around the border, carried and fresh
+    states, widths and addresses that forbid 16-byte accesses; an entry's bits are the same alone and among others, short and long."""
+    from mlx_parallm_b200 import _lib
+    lens = [32, 33, 31, 1, 71, 0]
+    g, nb, M = torch.Generator(device="cuda").manual_seed(dk + mode), len(lens), sum(lens)
+    rnd = lambda *sh: torch.randn(*sh, generator=g, device="cuda")
+    qn, kn, v = rnd(M, KH * dk) / dk ** 0.5, torch.nn.functional.normalize(rnd(M, KH, dk), dim=-1).reshape(M, -1).contiguous(), rnd(M, H * dv)
+    beta, decay = torch.rand(M, H, generator=g, device="cuda"), 0.5 + 0.5 * torch.rand(M, H * (dk if mode else 1), generator=g, device="cuda")
+    state0 = rnd(nb + 1, H, dk, dv) * 0.3
+    i32 = dict(dtype=torch.int32, device="cuda")
+    cu, rows, lengths = torch.tensor([0] + torch.tensor(lens).cumsum(0).tolist(), **i32), torch.tensor([4, 6, 1, 0, 5, 2], **i32), torch.tensor([3, 7, 0, 2, 0, 9, 1], **i32)
+
+    def scan(tokens, cu, rows, n):
+        state = torch.empty(state0.numel() + 2, device="cuda")[shift:shift + state0.numel()]
+        state.copy_(state0.reshape(-1))
+        o = torch.zeros(M, H * dv, device="cuda")
+        p = lambda t: t.data_ptr()
+        _lib.check(_lib.lib().b200p_delta_scan_tokens(p(qn), p(kn), p(v), p(beta), p(decay), p(state), p(cu), p(rows), p(lengths), p(o), tokens, n, H, KH,
+                                                      dk, dv, mode, torch.cuda.current_stream().cuda_stream))
+        return o, state.view_as(state0)
+
+    o, state = scan(0, cu, rows, nb)
+    for e, n in enumerate(lens):
+        lo, r = int(cu[e]), int(rows[e])
+        if n:
+            alone = scan(n, cu[e:e + 2].contiguous(), rows[e:e + 1].contiguous(), 1)
+            assert torch.equal(alone[0][lo:lo + n], o[lo:lo + n]) and torch.equal(alone[1][r], state[r]), e
+        S = (state0[r] * (int(lengths[r]) > 0)).double() if n else state0[r].double()
+        out = []
+        for t in range(lo, lo + n):
+            k, q_ = (x[t].double().view(KH, dk).repeat_interleave(H // KH, 0) for x in (kn, qn))
+            S = S * decay[t].double().view(H, -1, 1)
+            u = beta[t].double().unsqueeze(1) * (v[t].double().view(H, dv) - torch.einsum("hkv,hk->hv", S, k))
+            S = S + k.unsqueeze(2) * u.unsqueeze(1)
+            out.append(torch.einsum("hkv,hk->hv", S, q_).reshape(-1))
+        assert (state[r].double() - S).abs().max() < 2e-5                # 71 tokens of fp32 sums over 128 rows of about 0.3, unit keys
+        assert not out or (o[lo:lo + n].double() - torch.stack(out)).abs().max() < 2e-5
+    assert torch.equal(state[3], state0[3])                              # a row that no entry names is not touched
+
+
 @pytest.mark.parametrize("lens,H,KH,dv,channel", [([257], 1, 1, 128, False), ([1, 300, 2], 3, 1, 256, True), ([130, 3, 129, 9], 4, 2, 128, True)])
 def test_delta_prep_rows_equals_the_per_token_kernel(lens, H, KH, dv, channel):
     """Prompts of more than 256 tokens with 128-channel heads (one warp per 128 channels and 8 tokens) against the per-token kernel fed
