@@ -17,7 +17,7 @@ namespace b200p {
 int sm_count();
 bool pdl_enabled_gemm();
 
-__device__ __forceinline__ float silu_f(float z) { return z / (1.f + __expf(-z)); }
+__device__ __forceinline__ float silu_f(float z) { return __fdividef(z, 1.f + __expf(-z)); }
 __device__ __forceinline__ float softplus_f(float z) { return z > 20.f ? z : log1pf(expf(z)); }
 
 constexpr int DELTA_MAX_TAPS = 16;
@@ -70,74 +70,82 @@ delta_prep_kernel(const float* __restrict__ proj, int64_t ldp, int64_t col_b, co
     decay[t * (int64_t)nd + i] = expf(-expf(A_log[i / dper]) * softplus_f(at[i] + dt_bias[i]));
 }
 
-// The same for prompts whose heads are runs of 128 channels: a warp takes 128 channels (one q or k head, a piece of v, of the decays or
-// of beta) through `tt` consecutive tokens, lane l the channels l, l + 32, l + 64, l + 96, and keeps the last TAPS - 1 inputs in
+// The same for heads that are runs of 128 channels: a warp takes 128 channels (one q or k head, a piece of v, of the decays or
+// of beta) through TT consecutive tokens, lane l the channels l, l + 32, l + 64, l + 96, and keeps the last TAPS - 1 inputs in
 // registers, so the fp32 projection is read once instead of TAPS times.  Same operations in the same order per value as above: the
-// results are bit for bit those of delta_prep_kernel.  Bound: HBM / L2 traffic.
-template <int TAPS>
+// results are bit for bit those of delta_prep_kernel.  Bound: instructions (two exponentials and a logarithm per decay) and the latency of a warp's
+// reads, which are asked for together; four tokens keep code and registers small (eight ran out of the instruction cache).  16 + 16 heads of
+// 128, decays per channel, us: 1664 tokens 38 -> 29 (one token ahead, eight tokens per warp, before), 400 15.5 -> 11.2, 4 tokens (a block per token
+// before) 10.4 -> 4.2.
+template <int TAPS, int TT>
 __global__ void __launch_bounds__(128)
 delta_prep_rows_kernel(const float* __restrict__ proj, int64_t ldp, int64_t col_b, const float* __restrict__ a, int64_t lda, int dper,
                        const float* __restrict__ conv_w, const float* __restrict__ conv_state, const float* __restrict__ A_log,
                        const float* __restrict__ dt_bias, const int32_t* __restrict__ t_row, const int32_t* __restrict__ t_pos,
                        const int32_t* __restrict__ t_off, float* __restrict__ qn, float* __restrict__ kn, float* __restrict__ vout,
-                       float* __restrict__ beta, float* __restrict__ decay, int M, int H, int KH, int dv, int tt) {
+                       float* __restrict__ beta, float* __restrict__ decay, int M, int H, int KH, int dv) {
   constexpr int DK = 128;
   const int lane = threadIdx.x & 31, unit = blockIdx.y * 4 + (threadIdx.x >> 5);
-  const int t0 = blockIdx.x * tt, t1 = min(M, t0 + tt);
+  const int t0 = blockIdx.x * TT, nt = min(TT, M - t0);
   const int nv = H * dv / 128, nd = H * dper, u_conv = 2 * KH + nv, u_dec = (nd + 127) / 128, u_beta = (H + 127) / 128;
   if (unit >= u_conv + u_dec + u_beta) return;
   if (unit >= u_conv) {                                       // decays, then betas: one value per token and entry
     const bool dec = unit < u_conv + u_dec;
     const int base = (dec ? unit - u_conv : unit - u_conv - u_dec) * 128 + lane, n = dec ? nd : H;
-    float ea[4], bias[4];
+    const float* src = dec ? a : proj + col_b;
+    const int64_t ld = dec ? lda : ldp;
+#pragma unroll 1
+    for (int c = base; c < n && c < base + 128; c += 32) {
+      float x[TT];
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      const int i = base + 32 * r;
-      const bool in = dec && i < n;
-      ea[r] = in ? -expf(A_log[i / dper]) : 0.f;
-      bias[r] = in ? dt_bias[i] : 0.f;
-    }
-#pragma unroll 2
-    for (int t = t0; t < t1; ++t) {
+      for (int i = 0; i < TT; ++i) x[i] = i < nt ? src[(int64_t)(t0 + i) * ld + c] : 0.f;
+      const float ea = dec ? -expf(A_log[c / dper]) : 0.f, bias = dec ? dt_bias[c] : 0.f;
 #pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        const int i = base + 32 * r;
-        if (i >= n) continue;
-        if (dec) decay[(int64_t)t * nd + i] = expf(ea[r] * softplus_f(a[(int64_t)t * lda + i] + bias[r]));
-        else beta[(int64_t)t * H + i] = 1.f / (1.f + expf(-proj[(int64_t)t * ldp + col_b + i]));
+      for (int i = 0; i < TT; ++i) {
+        if (i >= nt) break;
+        if (dec) decay[(int64_t)(t0 + i) * nd + c] = expf(ea * softplus_f(x[i] + bias));
+        else beta[(int64_t)(t0 + i) * H + c] = 1.f / (1.f + expf(-x[i]));
       }
     }
     return;
   }
+  float in[TT][4];
   const int C = 2 * KH * DK + H * dv, c0 = unit * 128 + lane;
+  int off[TT];
+  const int row0 = t_row[t0], pos0 = t_pos[t0];
+#pragma unroll
+  for (int i = 0; i < TT; ++i) {
+    off[i] = i < nt ? t_off[t0 + i] : 0;
+#pragma unroll
+    for (int r = 0; r < 4; ++r) in[i][r] = i < nt ? proj[(int64_t)(t0 + i) * ldp + c0 + 32 * r] : 0.f;
+  }
   float w[4][TAPS], win[4][TAPS];                             // win[r][j]: input of tap j
+  const bool w16 = TAPS == 4 && (reinterpret_cast<uintptr_t>(conv_w) & 15) == 0;
 #pragma unroll
-  for (int r = 0; r < 4; ++r)
+  for (int r = 0; r < 4; ++r) {
+    if (w16) {
+      const float4 q = *reinterpret_cast<const float4*>(conv_w + (int64_t)(c0 + 32 * r) * TAPS);
+      w[r][0] = q.x, w[r][1] = q.y, w[r][2] = q.z, w[r][3] = q.w;
+    } else {
 #pragma unroll
-    for (int j = 0; j < TAPS; ++j) w[r][j] = conv_w[(int64_t)(c0 + 32 * r) * TAPS + j];
-  float next[4];
-#pragma unroll
-  for (int r = 0; r < 4; ++r) next[r] = proj[(int64_t)t0 * ldp + c0 + 32 * r];
-  for (int t = t0; t < t1; ++t) {
-    const int off = t_off[t];
-    float cur[4];
-#pragma unroll
-    for (int r = 0; r < 4; ++r) cur[r] = next[r];
-    if (t + 1 < t1) {
-#pragma unroll
-      for (int r = 0; r < 4; ++r) next[r] = proj[(int64_t)(t + 1) * ldp + c0 + 32 * r];
+      for (int j = 0; j < TAPS; ++j) w[r][j] = conv_w[(int64_t)(c0 + 32 * r) * TAPS + j];
     }
-    if (t == t0 || off == 0) {                                // the inputs before this token: of the portion, carried, or none
-      const int row = t_row[t], pos = t_pos[t];
+  }
+#pragma unroll
+  for (int i = 0; i < TT; ++i) {
+    if (i >= nt) break;
+    const int t = t0 + i;
+    if (i == 0 || off[i] == 0) {                              // the inputs before this token: of the portion, carried, or none
+      const int row = i == 0 ? row0 : t_row[t], pos = i == 0 ? pos0 : t_pos[t];
 #pragma unroll
       for (int j = 0; j < TAPS - 1; ++j) {
         const int d = TAPS - 1 - j;
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
           const int c = c0 + 32 * r;
-          float in = 0.f;
-          if (d <= pos) in = d <= off ? proj[(int64_t)(t - d) * ldp + c] : conv_state[((int64_t)row * (TAPS - 1) + (TAPS - 1 + off - d)) * C + c];
-          win[r][j] = in;
+          float x = 0.f;
+          if (d <= pos) x = d <= off[i] ? proj[(int64_t)(t - d) * ldp + c] : conv_state[((int64_t)row * (TAPS - 1) + (TAPS - 1 + off[i] - d)) * C + c];
+          win[r][j] = x;
         }
       }
     } else {
@@ -149,7 +157,7 @@ delta_prep_rows_kernel(const float* __restrict__ proj, int64_t ldp, int64_t col_
     float act[4];
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
-      win[r][TAPS - 1] = cur[r];
+      win[r][TAPS - 1] = in[i][r];
       float acc = 0.f;
 #pragma unroll
       for (int j = 0; j < TAPS; ++j) acc = fmaf(w[r][j], win[r][j], acc);
@@ -850,6 +858,40 @@ __global__ void delta_out_kernel(const float* __restrict__ o, const float* __res
   }
 }
 
+// The same for groups of 128 * NV values in 16-byte pieces: a warp per (token, head), its values in registers between the sum and the
+// output.  1664 tokens, 16 heads of 128, bf16, us: 15.2 -> 8.4.
+template <typename T, int NV>
+__global__ void __launch_bounds__(256)
+delta_out_rows_kernel(const float* __restrict__ o, const float* __restrict__ gate, int64_t ldg, const float* __restrict__ norm_w,
+                      T* __restrict__ out, int64_t ld_out, int64_t pairs, int H, float eps, int act, float out_scale) {
+  constexpr int DV = 128 * NV;
+  const int64_t i = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  if (i >= pairs) return;
+  const int64_t t = i / H;
+  const int h = (int)(i - t * H);
+  float4 x[NV], g[NV], w[NV];
+#pragma unroll
+  for (int k = 0; k < NV; ++k) {
+    const int c = 128 * k + 4 * lane;
+    x[k] = *reinterpret_cast<const float4*>(o + i * DV + c);
+    g[k] = *reinterpret_cast<const float4*>(gate + t * ldg + (int64_t)h * DV + c);
+    w[k] = *reinterpret_cast<const float4*>(norm_w + c);
+  }
+  float ss = 0.f;
+#pragma unroll
+  for (int k = 0; k < NV; ++k) ss = fmaf(x[k].x, x[k].x, fmaf(x[k].y, x[k].y, fmaf(x[k].z, x[k].z, fmaf(x[k].w, x[k].w, ss))));
+  const float inv = out_scale / sqrtf(warp_sum(ss) / (float)DV + eps);
+#pragma unroll
+  for (int k = 0; k < NV; ++k) {
+    __align__(16) T r[4] = {Tr<T>::from_f(x[k].x * inv * w[k].x * gate_act_f(g[k].x, act)), Tr<T>::from_f(x[k].y * inv * w[k].y * gate_act_f(g[k].y, act)),
+                            Tr<T>::from_f(x[k].z * inv * w[k].z * gate_act_f(g[k].z, act)), Tr<T>::from_f(x[k].w * inv * w[k].w * gate_act_f(g[k].w, act))};
+    T* dst = out + t * ld_out + (int64_t)h * DV + 128 * k + 4 * lane;
+    if constexpr (sizeof(T) == 4) *reinterpret_cast<float4*>(dst) = *reinterpret_cast<const float4*>(r);
+    else *reinterpret_cast<uint2*>(dst) = *reinterpret_cast<const uint2*>(r);
+  }
+}
+
 }  // namespace b200p
 
 using namespace b200p;
@@ -866,13 +908,12 @@ extern "C" int b200p_delta_prep(const float* proj, int64_t ldp, int64_t col_b, c
   if (M == 0) return B200P_OK;
   const size_t smem = (size_t)2 * KH * dk * sizeof(float);
   B200P_REQUIRE(smem <= 48 * 1024, B200P_ERR_ARG, "q and k of one token must fit 48 KB of shared memory");
-  // prompts of designs with 128-channel heads (1664 tokens of 4096 + 2048 channels: 81 -> 37 us)
-  if (M > 256 && M < (1ll << 30) && dk == 128 && dv % 128 == 0 && taps == 4) {
-    const int tt = M >= 4096 ? 16 : 8, nd = H * decay_per_head;
+  if (M < (1ll << 30) && dk == 128 && dv % 128 == 0 && taps == 4) {             // heads of 128 channels; fewer tokens, shorter runs of them per warp
+    const int tt = M > 128 ? 4 : 1, nd = H * decay_per_head;
     const int units = 2 * KH + H * dv / 128 + (nd + 127) / 128 + (H + 127) / 128;
-    delta_prep_rows_kernel<4><<<dim3((unsigned)((M + tt - 1) / tt), (unsigned)((units + 3) / 4)), 128, 0, (cudaStream_t)stream>>>(
-        proj, ldp, col_b, a, lda, decay_per_head, conv_w, conv_state, A_log, dt_bias, t_row, t_pos, t_off, qn, kn, v, beta, decay, (int)M, H, KH,
-        dv, tt);
+    const auto kern = tt == 4 ? delta_prep_rows_kernel<4, 4> : delta_prep_rows_kernel<4, 1>;
+    kern<<<dim3((unsigned)((M + tt - 1) / tt), (unsigned)((units + 3) / 4)), 128, 0, (cudaStream_t)stream>>>(
+        proj, ldp, col_b, a, lda, decay_per_head, conv_w, conv_state, A_log, dt_bias, t_row, t_pos, t_off, qn, kn, v, beta, decay, (int)M, H, KH, dv);
     B200P_LAUNCH_CHECK("delta_prep_rows_kernel");
     return B200P_OK;
   }
@@ -975,6 +1016,17 @@ extern "C" int b200p_delta_out(const float* o, const float* gate, int64_t ldg, c
   B200P_REQUIRE(gate_act == 0 || gate_act == 1, B200P_ERR_ARG, "gate activation: 0 silu, 1 sigmoid");
   B200P_REQUIRE(ld_out >= (int64_t)H * dv, B200P_ERR_ARG, "output rows are shorter than the heads");
   if (M == 0) return B200P_OK;
+  const int nv = dv % 128 == 0 ? dv / 128 : 0, piece = dtype == B200P_F32 ? 16 : 8;
+  if (H > 1 && (nv == 1 || nv == 2 || nv == 4) && aligned(o, 16) && aligned(gate, 16) && ldg % 4 == 0 && aligned(norm_w, 16) && aligned(out, piece) &&
+      ld_out % 4 == 0) {
+    const int64_t pairs = M * H;
+    B200P_DISPATCH_DTYPE(dtype, T, {
+      const auto kern = nv == 1 ? delta_out_rows_kernel<T, 1> : nv == 2 ? delta_out_rows_kernel<T, 2> : delta_out_rows_kernel<T, 4>;
+      kern<<<(unsigned)((pairs + 7) / 8), 256, 0, (cudaStream_t)stream>>>(o, gate, ldg, norm_w, (T*)out, ld_out, pairs, H, eps, gate_act, out_scale);
+    });
+    B200P_LAUNCH_CHECK("delta_out_rows_kernel");
+    return B200P_OK;
+  }
   const unsigned threads = H == 1 ? (dv >= 1024 ? 256 : 128) : H >= 8 ? 256 : 32 * (unsigned)H;
   B200P_DISPATCH_DTYPE(dtype, T, (delta_out_kernel<T><<<(unsigned)M, threads, 0, (cudaStream_t)stream>>>(
       o, gate, ldg, norm_w, (T*)out, ld_out, H, dv, eps, gate_act, out_scale)));

@@ -225,7 +225,8 @@ static int gemm_mma_launch(const T* x, const T* w, void* y, int64_t M, int64_t N
 // ---- few rows (decode): the weights stream once, every warp owns two weight rows ---------------------------------------------
 constexpr int GEMV_MAX_M = 8;
 
-template <typename T, int MR>
+// STAGED: x lies in shared memory (M * K values, the M rows one after the other): with one L1 access per row and piece the time grew with M.
+template <typename T, int MR, bool STAGED>
 __global__ void __launch_bounds__(256)
 gemv_rows_kernel(const T* __restrict__ x, const T* __restrict__ w, void* __restrict__ y, int M, int64_t N, int64_t K, int64_t ldx,
                  int64_t ldw, int64_t ldy, int64_t sx, int64_t sw, int64_t sy, int epi, float2 act) {
@@ -234,33 +235,57 @@ gemv_rows_kernel(const T* __restrict__ x, const T* __restrict__ w, void* __restr
   w += z * sw;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t n = ((int64_t)blockIdx.x * 8 + warp) * 2;
-  if (n >= N) return;
-  const bool two = n + 1 < N;
+  extern __shared__ uint4 gv_x[];
+  const int pieces = (int)(K / 8);                 // (16-byte pieces of a row: the caller has checked K % 8)
+  if constexpr (STAGED) {
+    for (int m = 0; m < M; ++m)
+      for (int c = threadIdx.x; c < pieces; c += 256) gv_x[m * pieces + c] = *reinterpret_cast<const uint4*>(x + (int64_t)m * ldx + 8 * c);
+  }
+  if (!STAGED && n >= N) return;
+  const bool live = n < N, two = n + 1 < N;
   float a0[MR], a1[MR];
 #pragma unroll
   for (int m = 0; m < MR; ++m) a0[m] = a1[m] = 0.f;
   const T* w0 = w + n * ldw;
   const T* w1 = w + (two ? n + 1 : n) * ldw;
-  for (int64_t k = (int64_t)lane * 8; k < K; k += 256) {
-    const uint4 u0 = ldg_stream(w0 + k), u1 = ldg_stream(w1 + k);
-    const T* p0 = reinterpret_cast<const T*>(&u0);
-    const T* p1 = reinterpret_cast<const T*>(&u1);
-    float f0[8], f1[8];
+  bool first = true;
+  // Bound: the weights' way from HBM.  A warp asks for four pieces of each row at a time and x comes from shared memory (us, bf16, one piece at
+  // a time and x from L1 -> now, 1 / 4 / 8 rows: 2048 x 2048 9.9 -> 6.7 / 15.2 -> 8.3 / 22 -> 12.3; 4368 x 2048 10.2 -> 8.2 / 16.3 -> 10.3 / 23.7 ->
+  // 15.8; 4096 x 4096 16.4 -> 12.3 / 28.6 -> 16.4 / 43 -> 24.7; 512 x 8192 25 -> 16 / 49 -> 20 / 76 -> 65, not staged).
+  constexpr int AHEAD = 4;
+  const int64_t k_end = STAGED ? (K + 255) / 256 * 256 : K;          // (staged: every lane takes part in the barrier)
+  for (int64_t k0 = (int64_t)lane * 8; k0 < k_end; k0 += 256 * AHEAD) {
+    uint4 u0[AHEAD], u1[AHEAD];
 #pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      f0[e] = Tr<T>::to_f(p0[e]);
-      f1[e] = Tr<T>::to_f(p1[e]);
+    for (int j = 0; j < AHEAD; ++j)
+      if (live && k0 + 256 * j < K) u0[j] = ldg_stream(w0 + k0 + 256 * j), u1[j] = ldg_stream(w1 + k0 + 256 * j);
+    if (STAGED && first) {                         // x arrives while the first pieces of the weights are on their way
+      __syncthreads();
+      first = false;
     }
 #pragma unroll
-    for (int m = 0; m < MR; ++m) {
-      if (m < M) {
-        const uint4 ux = *reinterpret_cast<const uint4*>(x + (int64_t)m * ldx + k);
-        const T* px = reinterpret_cast<const T*>(&ux);
+    for (int j = 0; j < AHEAD; ++j) {
+      const int64_t k = k0 + 256 * j;
+      if (k >= K) break;
+      const T* p0 = reinterpret_cast<const T*>(&u0[j]);
+      const T* p1 = reinterpret_cast<const T*>(&u1[j]);
+      float f0[8], f1[8];
 #pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          const float xv = Tr<T>::to_f(px[e]);
-          a0[m] = fmaf(xv, f0[e], a0[m]);
-          a1[m] = fmaf(xv, f1[e], a1[m]);
+      for (int e = 0; e < 8; ++e) {
+        f0[e] = Tr<T>::to_f(p0[e]);
+        f1[e] = Tr<T>::to_f(p1[e]);
+      }
+#pragma unroll
+      for (int m = 0; m < MR; ++m) {
+        if (m < M) {
+          const uint4 ux = STAGED ? gv_x[m * pieces + (int)(k >> 3)] : *reinterpret_cast<const uint4*>(x + (int64_t)m * ldx + k);
+          const T* px = reinterpret_cast<const T*>(&ux);
+#pragma unroll
+          for (int e = 0; e < 8; ++e) {
+            const float xv = Tr<T>::to_f(px[e]);
+            a0[m] = fmaf(xv, f0[e], a0[m]);
+            a1[m] = fmaf(xv, f1[e], a1[m]);
+          }
         }
       }
     }
@@ -270,7 +295,7 @@ gemv_rows_kernel(const T* __restrict__ x, const T* __restrict__ w, void* __restr
     a0[m] = warp_sum(a0[m]);
     a1[m] = warp_sum(a1[m]);
   }
-  if (lane == 0) {
+  if (lane == 0 && live) {
 #pragma unroll
     for (int m = 0; m < MR; ++m)
       if (m < M) gemm_store_pair<T>(y, z * sy + (int64_t)m * ldy, n, N, a0[m], a1[m], epi, act);
@@ -358,9 +383,21 @@ static int gemm_dispatch(const void* x, const void* w, void* y, int64_t M, int64
   const T* wp = (const T*)w;
   if (fast_ok && M <= GEMV_MAX_M) {
     dim3 grid((unsigned)((N + 15) / 16), 1, (unsigned)batch);
-    if (M <= 2) gemv_rows_kernel<T, 2><<<grid, 256, 0, st>>>(xp, wp, y, (int)M, N, K, ldx, ldw, ldy, sx, sw, sy, epi, act);
-    else if (M <= 4) gemv_rows_kernel<T, 4><<<grid, 256, 0, st>>>(xp, wp, y, (int)M, N, K, ldx, ldw, ldy, sx, sw, sy, epi, act);
-    else gemv_rows_kernel<T, 8><<<grid, 256, 0, st>>>(xp, wp, y, (int)M, N, K, ldx, ldw, ldy, sx, sw, sy, epi, act);
+    const size_t smem = (size_t)M * K * sizeof(T);
+    if (M > 1 && K >= 512 && smem <= 96 * 1024) {       // (short rows: the copy costs more than it spares, 2048 x 128, 4 rows: 5.2 / 4.2 us)
+      const auto kern = M <= 2 ? gemv_rows_kernel<T, 2, true> : M <= 4 ? gemv_rows_kernel<T, 4, true> : gemv_rows_kernel<T, 8, true>;
+      static bool attr_set[3] = {false, false, false};
+      bool& set = attr_set[M <= 2 ? 0 : M <= 4 ? 1 : 2];
+      if (smem > 48 * 1024 && !set) {
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
+        if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(gemv_rows_kernel)");
+        set = true;
+      }
+      kern<<<grid, 256, smem, st>>>(xp, wp, y, (int)M, N, K, ldx, ldw, ldy, sx, sw, sy, epi, act);
+    } else {
+      const auto kern = M <= 2 ? gemv_rows_kernel<T, 2, false> : M <= 4 ? gemv_rows_kernel<T, 4, false> : gemv_rows_kernel<T, 8, false>;
+      kern<<<grid, 256, 0, st>>>(xp, wp, y, (int)M, N, K, ldx, ldw, ldy, sx, sw, sy, epi, act);
+    }
     B200P_LAUNCH_CHECK("gemv_rows_kernel");
     return B200P_OK;
   }

@@ -133,6 +133,24 @@ def test_gemm_tcgen05_tiles(dtype, M, N, K):
         assert glu.shape == (M, N // 2) and (glu.double() - a * torch.sigmoid(1.702 * a) * (u + 1)).abs().max() < 0.02
 
 
+@pytest.mark.parametrize("M,N,K,batch", [(1, 35, 520, 1), (2, 16, 504, 2), (2, 17, 512, 3), (3, 50, 1032, 1), (4, 31, 2056, 2), (8, 40, 6144, 1), (8, 16, 6152, 1), (5, 3, 4096, 2)])
+def test_gemv_of_few_rows(M, N, K, batch):
+    """Up to eight rows: x staged in shared memory (512 <= K, up to 96 KB) or read in place, pieces of K that end inside a warp's four, odd
+    numbers of columns and warps without any, rows and products strided; a row's bits do not depend on how many others there are."""
+    from mlx_parallm_b200 import _lib, ops
+    g = torch.Generator(device="cuda").manual_seed(M + K)
+    x = (torch.randn(M, batch, K, generator=g, device="cuda") / 4).to(torch.bfloat16)
+    w = (torch.randn(batch, N, K, generator=g, device="cuda") / 4).to(torch.bfloat16)
+    out = torch.full((M, batch, N), 7.0, device="cuda")
+    args = dict(batch=batch, strides=(K, N * K, N), N=N, K=K, ldx=batch * K, ldw=K, ldy=batch * N)
+    ops.gemm(x, w, _lib.GEMM_STORE_F32, out=out, M=M, **args)
+    want = torch.einsum("mbk,bnk->mbn", x.double(), w.double())
+    assert (out.double() - want).abs().max() <= 2e-5 * math.sqrt(K)
+    one = torch.empty((1, batch, N), device="cuda")
+    ops.gemm(x[M - 1:], w, _lib.GEMM_STORE_F32, out=one, M=1, **args)
+    assert torch.equal(one[0], out[M - 1])
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("M,N,K,batch", [(65, 2, 64, 1), (96, 256, 72, 1), (257, 300, 200, 1), (512, 257, 448, 1), (777, 1030, 136, 1), (1000, 640, 64, 3),
                                          (4100, 5000, 320, 1)])
@@ -778,3 +796,48 @@ def test_delta_prep_rows_equals_the_per_token_kernel(lens, H, KH, dv, channel):
     cuts = list(range(0, M, 200)) + [M]
     for w, p in zip(whole, run(list(zip(cuts[:-1], cuts[1:])))):
         assert torch.equal(w, p)
+
+
+@pytest.mark.parametrize("M,H,KH,dv,channel", [(1, 3, 1, 128, True), (128, 2, 2, 256, False), (131, 2, 1, 128, True), (1025, 2, 1, 128, True)])
+def test_delta_prep_of_128_channel_heads(M, H, KH, dv, channel):
+    """A warp per 128 channels and 1, 4 or 8 tokens (by their number), one sequence that carries inputs: against float64."""
+    from mlx_parallm_b200 import ops
+    dk, taps, C = 128, 4, 2 * KH * 128 + H * dv
+    g = torch.Generator(device="cuda").manual_seed(M)
+    rnd = lambda *s: torch.randn(s, generator=g, device="cuda")        # noqa: E731
+    nd, i32 = H * (dk if channel else 1), dict(dtype=torch.int32, device="cuda")
+    proj, a, conv_w, state, A_log, dt_bias = rnd(M, C + H + 1), rnd(M, nd), rnd(C, taps), rnd(1, taps - 1, C), rnd(H), rnd(nd)
+    pos = torch.arange(M, **i32)
+    out = [torch.zeros((M, n), device="cuda") for n in (KH * dk, KH * dk, H * dv, H, nd)]
+    ops.delta_prep(proj, C, a, conv_w, state, A_log, dt_bias, torch.zeros(M, **i32), pos + 2, pos, *out, H, KH, dk, dv, taps)
+    past = torch.cat([state[0].double(), proj[:, :C].double()])
+    past[0] = 0                                                         # position 2: two inputs lie before the portion, not three
+    act = torch.nn.functional.silu(sum(conv_w.double()[:, j] * past[j:j + M] for j in range(taps)))
+    q, k = act[:, :KH * dk].view(M, KH, dk), act[:, KH * dk:2 * KH * dk].view(M, KH, dk)
+    unit = lambda z: z * torch.rsqrt(z.square().sum(-1, keepdim=True) + 1e-6)        # noqa: E731
+    step = torch.nn.functional.softplus(a.double() + dt_bias.double())
+    want = [(unit(q) * dk ** -0.5).reshape(M, -1), unit(k).reshape(M, -1), act[:, 2 * KH * dk:], torch.sigmoid(proj[:, C:C + H].double()),
+            torch.exp(-A_log.double().exp().repeat_interleave(nd // H) * step)]
+    for got, ref in zip(out, want):
+        assert (got.double() - ref).abs().max() <= 4e-6 * max(1.0, float(ref.abs().max()))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("H,dv,col", [(3, 128, 0), (2, 256, 4), (5, 512, 0), (3, 384, 0), (3, 128, 1), (2, 100, 0)])
+def test_delta_out_widths(dtype, H, dv, col):
+    """Norm, weight and gate per head: 16-byte pieces for groups of 128, 256 and 512 values, the general kernel for other widths and for
+    gates that start between 16-byte boundaries."""
+    from mlx_parallm_b200 import ops
+    M = 7
+    g = torch.Generator(device="cuda").manual_seed(dv)
+    o, gate = torch.randn(M, H * dv, generator=g, device="cuda"), torch.randn(M, H * dv + 8, generator=g, device="cuda")
+    w = 1 + 0.1 * torch.randn(dv, generator=g, device="cuda")
+    for act in (0, 1):
+        out = torch.zeros(M, H * dv, dtype=dtype, device="cuda")
+        gt = gate[:, col:col + H * dv]
+        ops.delta_out(o, gt, w, out, H, dv, 1e-5, act)
+        x, z = o.double().view(M, H, dv), gt.double()
+        s = z * torch.sigmoid(z) if act == 0 else torch.sigmoid(z)
+        want = (x * torch.rsqrt(x.square().mean(-1, keepdim=True) + 1e-5) * w.double()).reshape(M, -1) * s
+        tol = {torch.float32: 4e-6, torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11}[dtype]      # one rounding
+        assert (out.double() - want).abs().max() <= tol * float(want.abs().max())
