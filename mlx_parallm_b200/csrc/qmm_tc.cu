@@ -108,6 +108,8 @@ struct TcParams {
   int sb_tma;          // 1: scale/bias tiles come through TMA (num_kb % 8 == 0)
   int w_stages;        // weight ring depth
   int x_slots;         // X ring depth (4 or 8; one slot = the [TN x 64] tile of one k-block)
+  uint32_t zero;       // 0, which the compiler does not know: a slot is handed back (and overwritten by the copy engine) only when what was read
+                       // from it has arrived in registers, the address of the arrival depends on it (what happens otherwise: qmm_wide.cu)
 };
 
 // work item -> (output tile, stage range): item = tile * S + split, split covers stages [split*num_st/S, (split+1)*num_st/S)
@@ -397,8 +399,12 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
 #pragma unroll
         for (int c = 0; c < CPK; ++c)
           pk[j2 * CPK + c] = lds128(wsrc + ((((uint32_t)((kpar + 2 * j2) * CPK + c)) ^ w_xor) << 4));
+      uint32_t all = 0;
+#pragma unroll
+      for (int c = 0; c < KPT * CPK; ++c) all |= pk[c].w;
+      const uint32_t done = empty_w(si) + (all & p.zero);          // (see TcParams::zero)
       __syncwarp();
-      if (lane == 0) mbar_arrive(empty_w(si));
+      if (lane == 0) mbar_arrive(done);
       if (++si == S) { si = 0; ph ^= 1; }
     };
     // one k-block: 64 codes of row r -> 32 packed 16-bit pairs -> A ring slot
@@ -461,8 +467,9 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
             const uint32_t src = sb_ring + sbi * SB_SLOT_BYTES + sb_off;
             s8 = lds128(src);
             b8 = lds128(src + SB_TILE_BYTES);
+            const uint32_t done = sb_empty(sbi) + ((s8.w | b8.w) & p.zero);
             __syncwarp();
-            if (lane == 0) mbar_arrive(sb_empty(sbi));
+            if (lane == 0) mbar_arrive(done);
             if (++sbi == NSB) { sbi = 0; sbph ^= 1; }
           }
           fetch_stage();
@@ -857,6 +864,7 @@ int qmm_tc_launch(const void* x, const uint32_t* w, const void* s, const void* b
     tms[3] = tms[0];
   }
   TcParams p;
+  p.zero = 0;
   p.scales = s; p.biases = b; p.y = y;
   const size_t counters = ws_counter_bytes(M, N);
   const size_t need = counters + (pl.S > 1 ? (size_t)pl.grid * 2 * pl.TN * 128 * sizeof(float) : 0);

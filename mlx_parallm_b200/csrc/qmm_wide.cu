@@ -64,6 +64,11 @@ struct Params {
   int tiles_m, row_blocks, items, row_fast;       // token tiles, row blocks, all tiles and their order (tile_of)
   int w_stages;
   int* wait_word;                                 // where a wait that gives up reports
+  // 0, which the compiler does not know.  A slot is handed back (and overwritten by the copy engine) only when what was read from it has arrived in
+  // registers: the address of the arrival depends on it.  Reads that are merely issued before the arrival may still wait their turn behind another
+  // kernel's memory instructions on the same SM, and rows 0 to 23 of a stage then came from the next one (5 to 8 columns in 3000 launches of
+  // 18944 x 1024, 8 bits, 250 tokens, between elementwise kernels).
+  uint32_t zero;
 };
 struct Shared {
   uint64_t full_w[MAX_STAGES], empty_w[MAX_STAGES], full_x[X_SLOTS], empty_x[X_SLOTS], full_a[A_SLOTS], empty_a[A_SLOTS];
@@ -379,8 +384,9 @@ qmm_wide_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
           const uint32_t src = sb_ring + sbi * 2 * SB_TILE_BYTES + (uint32_t)(r * 16);
           s8 = lds128(src);
           b8 = lds128(src + SB_TILE_BYTES);
+          const uint32_t done = smem_u32(&sh->sb_empty[sbi]) + ((s8.w | b8.w) & p.zero);
           __syncwarp();
-          if (lane == 0) mbar_arrive(smem_u32(&sh->sb_empty[sbi]));
+          if (lane == 0) mbar_arrive(done);
           if (++sbi == NSB) { sbi = 0; sbph ^= 1u; }
         }
         // 4 bits: group g takes k-block g of every stage; 8 bits: k-block g & 1 of every second stage
@@ -393,8 +399,12 @@ qmm_wide_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
           const uint32_t wsrc = w_ring + si * W_STAGE_BYTES + w_row;
 #pragma unroll
           for (int c = 0; c < CPK; ++c) pk[c] = lds128(wsrc + ((((uint32_t)(j * CPK + c)) ^ w_xor) << 4));
+          uint32_t all = 0;
+#pragma unroll
+          for (int c = 0; c < CPK; ++c) all |= pk[c].w;
+          const uint32_t done = smem_u32(&sh->empty_w[si]) + (all & p.zero);          // (see Params::zero)
           __syncwarp();
-          if (lane == 0) mbar_arrive(smem_u32(&sh->empty_w[si]));
+          if (lane == 0) mbar_arrive(done);
           const int e = (st % SPG) * KPS + j;               // k-block within the group: half e & 1 of word e >> 1
           const int we = e >> 1;
           const uint32_t sw = we == 0 ? s8.x : we == 1 ? s8.y : we == 2 ? s8.z : s8.w;
@@ -553,6 +563,7 @@ int qmm_wide_launch(const void* x, const uint32_t* w, const void* s, const void*
                 CU_TENSOR_MAP_SWIZZLE_NONE, "y");
   if (rc) return rc;
   Params p;
+  p.zero = 0;
   if ((rc = wait_word(WAIT_QMM_WIDE, &p.wait_word))) return rc;
   p.y = y; p.M_tok = (int)M; p.N = (int)N; p.epi = epi; p.y_perm = (flags & B200P_Y_PERM8) ? 1 : 0;
   p.TN = pl.TN; p.H0 = pl.H0; p.H1 = pl.H1; p.ldy = ldy; p.num_st = (int)(row_bytes / 128);

@@ -53,6 +53,8 @@ struct QrParams {
   int chunks;            // K / 512
   int panels;            // k panels of the accumulating epilogue (1: none)
   int* wait_word;        // where a wait that gives up reports
+  uint32_t zero;         // 0, which the compiler does not know: a stage is refilled only when what was read from it has arrived in registers, the
+                         // addresses of the copies depend on it (what happens otherwise: qmm_wide.cu)
 };
 
 // unit u of the linear order (panel, tile, chunk within the panel): panel p covers chunks [p * chunks / panels, (p + 1) * chunks / panels)
@@ -181,9 +183,9 @@ qmv_ring_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
   __syncwarp();
   QrPos pr = qr_locate(p, u0 < u1 ? u0 : c0);              // position of the next unit to fetch
   int pu = u0;
-  auto fetch = [&](uint32_t stage) {
+  auto fetch = [&](uint32_t stage, uint32_t after) {        // (after: 0, known when the stage has been read: QrParams::zero)
     if (lane == 0) {
-      const uint32_t bar = my_bar + 8 * stage, dst = my_ring + stage * CODE_BYTES, sdst = my_scales + stage * SCALE_BYTES;
+      const uint32_t bar = my_bar + 8 * stage + after, dst = my_ring + stage * CODE_BYTES + after, sdst = my_scales + stage * SCALE_BYTES + after;
       const int ra = silu ? pr.tile * 8 : pr.tile * 16, rb = silu ? p.N / 2 + ra : ra + 8;
       mbar_arrive_expect_tx(bar, CODE_BYTES + SCALE_BYTES);
       tma_load_3d(dst, &tm_w, 0, ra, pr.ch * STEPS, bar);
@@ -197,7 +199,7 @@ qmv_ring_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
     qr_next(p, pr);
   };
   QrPos at = pr;                                           // position of the unit being computed
-  for (uint32_t s = 0; s < S && pu < u1; ++s) fetch(s);
+  for (uint32_t s = 0; s < S && pu < u1; ++s) fetch(s, 0);
   pdl_launch_dependents();
   pdl_wait();                                              // x is the previous kernel's output; y its accumulator
 
@@ -261,8 +263,12 @@ qmv_ring_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
         bvb[c2] = lds_u16(ss + 384 + 2 * grp);
       }
       if (half == STEPS / 2 - 1) {
+        uint32_t all = 0;
+#pragma unroll
+        for (int c2 = 0; c2 < 2; ++c2) all |= qa[c2][0].w | qa[c2][1].w | qb[c2][0].w | qb[c2][1].w | sva[c2] | bva[c2] | svb[c2] | bvb[c2];
+        all &= p.zero;
         __syncwarp();                                      // the stage sits in registers: hand it back to the stream
-        if (pu < u1) fetch(stage);
+        if (pu < u1) fetch(stage, all);
       }
 #pragma unroll
       for (int c2 = 0; c2 < 2; ++c2) {
@@ -398,6 +404,7 @@ static int qr_run(const CUtensorMap* tm, const QrParams& p, const QrPlan& pl, cu
 int qmv_ring_launch(const void* x, const uint32_t* w, const void* s, const void* b, void* y, int64_t M, int64_t N, int64_t K, int64_t ldx,
                     int64_t ldy, int bits, int dtype, int epi, int flags, cudaStream_t st) {
   QrParams p;
+  p.zero = 0;
   p.x = x; p.y = y; p.M = (int)M; p.N = (int)N; p.K = (int)K; p.epi = epi; p.ldx = ldx; p.ldy = ldy;
   p.x_perm = (flags & B200P_X_PERM8) ? 1 : 0;
   p.y_perm = (flags & B200P_Y_PERM8) ? 1 : 0;

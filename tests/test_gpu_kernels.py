@@ -787,6 +787,24 @@ def test_qmm_wide_tiles_repeat_bit_for_bit(ops, M, N, K, bits, dtype):
     assert int(bad) == 0
 
 
+@pytest.mark.parametrize("M,N,K,bits,dtype", [(250, 18944, 1024, 8, "bfloat16"), (64, 8192, 4096, 4, "float16"), (40, 4096, 8192, 8, "bfloat16"), (1, 8192, 8192, 4, "bfloat16")])
+def test_qmm_between_memory_bound_kernels(ops, M, N, K, bits, dtype):
+    """A product that starts while an elementwise kernel still fills the SM's memory pipeline: the weights' slots must not be refilled
+    while reads from them wait their turn (before, about one launch in 500 of the first case had a column that differed)."""
+    g = torch.Generator(device="cuda").manual_seed(M)
+    dt = TD[dtype]
+    w = torch.randint(-2 ** 31, 2 ** 31, (N, K * bits // 32), generator=g, device="cuda", dtype=torch.int64).to(torch.int32)
+    s = ((torch.rand((N, K // 64), generator=g, device="cuda") + 0.5) * 2 / (2 ** bits - 1) / K ** 0.5).to(dt)
+    b = (-s.float() * (2 ** bits - 1) / 2).to(dt)
+    x, ws = torch.randn((M, K), generator=g, device="cuda").to(dt), torch.zeros(ops.qmm_workspace_bytes(M, N, K), dtype=torch.uint8, device="cuda")
+    first, bad = ops.qmm(x, w, s, b, 64, bits, 1, workspace=ws, small_scale=True), torch.zeros((), dtype=torch.int64, device="cuda")
+    other = torch.zeros(1 << 21, device="cuda")
+    for _ in range(2000):
+        other.add_(1.0)
+        bad += (ops.qmm(x, w, s, b, 64, bits, 1, workspace=ws, small_scale=True) != first).sum()
+    assert int(bad) == 0
+
+
 # ---------------------------------------------------------------- TMA-ring GEMV of b200p_qmm (M <= 16)
 @pytest.mark.parametrize("M,N,K,bits,dtype,epi,small", [
     (1, 16, 512, 4, "float16", 1, True),          # one unit: seven of eight warps have nothing to do
