@@ -184,7 +184,7 @@ qmv_ring_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
   QrPos pr = qr_locate(p, u0 < u1 ? u0 : c0);              // position of the next unit to fetch
   int pu = u0;
   auto fetch = [&](uint32_t stage, uint32_t after) {        // (after: 0, known when the stage has been read: QrParams::zero)
-    if (lane == 0) {
+    if (elect_one()) {                                       // (not `lane == 0`: operands of warp-uniform code need no uniformising)
       const uint32_t bar = my_bar + 8 * stage + after, dst = my_ring + stage * CODE_BYTES + after, sdst = my_scales + stage * SCALE_BYTES + after;
       const int ra = silu ? pr.tile * 8 : pr.tile * 16, rb = silu ? p.N / 2 + ra : ra + 8;
       mbar_arrive_expect_tx(bar, CODE_BYTES + SCALE_BYTES);
@@ -195,6 +195,7 @@ qmv_ring_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
       tma_load_2d(sdst + 256, &tm_s, pr.ch * 8, rb, bar);
       tma_load_2d(sdst + 384, &tm_b, pr.ch * 8, rb, bar);
     }
+    __syncwarp();
     ++pu;
     qr_next(p, pr);
   };
