@@ -533,10 +533,12 @@ rope_kv_append_d128_kernel(TIN* __restrict__ qkv, T* __restrict__ q_out, T* __re
 
 // The same for prompts of 16-bit models (head_dim 128): 8 threads per (token, head) with 16-byte loads and stores, and a thread keeps
 // its token and its 8 angles while it walks over heads, so the 16 sines and cosines of a thread serve every head it visits instead of
-// one.  Bound: HBM / L2 traffic (read and write every projected value once).  A CTA holds 2^tpc_log2 tokens x (32 >> tpc_log2) walkers
-// per token.  4096 tokens, 40 + 16 heads with norms, bf16: 57 -> 35 us (117 MB); 4 x 777 tokens, 32 + 16 heads: 31 -> 18 us.
+// one.  Bound: HBM / L2 traffic (read and write every projected value once) and the bytes in flight for it: two heads are asked for at a time, four
+// CTAs per SM.  A CTA holds 2^tpc_log2 tokens x (32 >> tpc_log2) walkers per token.  us, one head at a time -> now (four heads and fewer CTAs are no
+// better): 4096 tokens, 40 + 16 heads with norms, bf16 37 -> 28.5 (117 MB); 4 x 777 tokens, 32 + 16 heads 18.5 -> 16.6; 8 x 1000, 64 + 16 heads 67 ->
+// 57.5 (5.7 TB/s).
 template <typename T>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 4)
 rope_kv_append_rows_kernel(const T* __restrict__ qkv, T* __restrict__ q_out, T* __restrict__ kc, T* __restrict__ vc,
                            const int32_t* __restrict__ lengths, const T* __restrict__ qn_w, const T* __restrict__ kn_w, int M, int L,
                            int Hq, int Hkv, int64_t Tcap, float log2_base, float rope_scale, float eps, int tpc_log2) {
@@ -550,33 +552,34 @@ rope_kv_append_rows_kernel(const T* __restrict__ qkv, T* __restrict__ q_out, T* 
   const int b = tok / L, l = tok - b * L, H = Hq + 2 * Hkv, i0 = 8 * c;
   const int pos_i = lengths[b] + l;
   const T* row = qkv + (int64_t)tok * H * D + i0;
+  constexpr int AHEAD = 2;                                  // heads asked for together
   int head = slot >> tpc_log2;
-  uint4 a = make_uint4(0u, 0u, 0u, 0u), p = a;
-  if (head < H) {
-    a = *reinterpret_cast<const uint4*>(row + head * D);
-    p = *reinterpret_cast<const uint4*>(row + head * D + HALF);
-  }
+  uint4 a[AHEAD], p[AHEAD];
+  auto fetch = [&]() {
+#pragma unroll
+    for (int k = 0; k < AHEAD; ++k)
+      if (head + k * step < H) {
+        a[k] = *reinterpret_cast<const uint4*>(row + (head + k * step) * D);
+        p[k] = *reinterpret_cast<const uint4*>(row + (head + k * step) * D + HALF);
+      }
+  };
+  fetch();
   float sn[8], cs[8];
 #pragma unroll
   for (int j = 0; j < 8; ++j) {                             // theta = pos * scale * base^(-i/half)
     const float inv_freq = exp2f(-(float)(i0 + j) * (log2_base / (float)HALF));
     sincosf((float)pos_i * rope_scale * inv_freq, &sn[j], &cs[j]);
   }
-  for (; head < H; head += step) {
-    const uint4 ca = a, cp = p;
-    if (head + step < H) {                                  // the next head's values are on their way while this one is rotated
-      a = *reinterpret_cast<const uint4*>(row + (head + step) * D);
-      p = *reinterpret_cast<const uint4*>(row + (head + step) * D + HALF);
-    }
+  auto one = [&](int head, const uint4& ca, const uint4& cp) {
     if (head >= Hq + Hkv) {                                 // V head: plain append
       if (pos_i >= Tcap) {
         if (c == 0) atomicAdd(&g_kv_overflow, 1u);
-        continue;
+        return;
       }
       T* dst = vc + (((int64_t)b * Hkv + (head - Hq - Hkv)) * Tcap + pos_i) * D + i0;
       *reinterpret_cast<uint4*>(dst) = ca;
       *reinterpret_cast<uint4*>(dst + HALF) = cp;
-      continue;
+      return;
     }
     float x1[8], x2[8];
     const T* va = reinterpret_cast<const T*>(&ca);
@@ -605,7 +608,7 @@ rope_kv_append_rows_kernel(const T* __restrict__ qkv, T* __restrict__ q_out, T* 
     if (is_q) {
       dst = q_out + ((int64_t)tok * Hq + head) * D + i0;
     } else {
-      if (pos_i >= Tcap) continue;
+      if (pos_i >= Tcap) return;
       dst = kc + (((int64_t)b * Hkv + (head - Hq)) * Tcap + pos_i) * D + i0;
     }
     __align__(16) T o1[8], o2[8];
@@ -616,6 +619,14 @@ rope_kv_append_rows_kernel(const T* __restrict__ qkv, T* __restrict__ q_out, T* 
     }
     *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(o1);
     *reinterpret_cast<uint4*>(dst + HALF) = *reinterpret_cast<const uint4*>(o2);
+  };
+  for (;;) {
+#pragma unroll
+    for (int k = 0; k < AHEAD; ++k)
+      if (head + k * step < H) one(head + k * step, a[k], p[k]);
+    head += AHEAD * step;
+    if (head >= H) break;
+    fetch();
   }
 }
 
