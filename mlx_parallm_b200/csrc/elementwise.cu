@@ -455,6 +455,7 @@ rope_kv_append_d128_kernel(TIN* __restrict__ qkv, T* __restrict__ q_out, T* __re
                            int L, int Hq, int Hkv, int64_t Tcap, float log2_base, float rope_scale, float eps) {
   constexpr int D = 128, HALF = 64;
   constexpr bool ACC_IN = std::is_same<TIN, float>::value && !std::is_same<T, float>::value;
+  pdl_launch_dependents();
   pdl_wait();
   const int tok = blockIdx.x;  // b*L + l
   const int b = tok / L, l = tok - b * L;
@@ -543,6 +544,7 @@ rope_kv_append_rows_kernel(const T* __restrict__ qkv, T* __restrict__ q_out, T* 
                            const int32_t* __restrict__ lengths, const T* __restrict__ qn_w, const T* __restrict__ kn_w, int M, int L,
                            int Hq, int Hkv, int64_t Tcap, float log2_base, float rope_scale, float eps, int tpc_log2) {
   constexpr int D = 128, HALF = 64;
+  pdl_launch_dependents();                                  // (the attention behind it sets itself up meanwhile)
   pdl_wait();
   const int c = threadIdx.x & 7, slot = threadIdx.x >> 3;
   const int tok = (int)(blockIdx.x << tpc_log2) + (slot & ((1 << tpc_log2) - 1));
