@@ -167,6 +167,14 @@ GATE_SILU, GATE_SIGMOID = 0, 1
 
 _lib = None
 
+# Functions that return an int and take only numbers and addresses are called through a small extension (csrc/fastcall.c) where that has been
+# built, the others and all calls without it through ctypes: the same functions with the same arguments.
+try:
+    from . import _fastcall
+except ImportError:
+    _fastcall = None
+_LETTERS = {_vp: "p", _i64: "i", _i32: "i", _u64: "i", _sz: "i", _f32: "f"}
+
 
 class B200PError(RuntimeError):
     pass
@@ -182,6 +190,9 @@ def _bind(path: str, partial: bool) -> C.CDLL:
                 raise
             continue
         fn.restype, fn.argtypes = res, args
+        sig = "".join(_LETTERS.get(a, "?") for a in args)
+        if _fastcall is not None and res is _i32 and "?" not in sig:
+            setattr(L, name, _fastcall.bind(C.cast(fn, C.c_void_p).value, sig, fn))
     return L
 
 

@@ -88,6 +88,7 @@ class Scratch:
         self._bufs: Dict[tuple, torch.Tensor] = {}
         self._need: Dict[tuple, int] = {}
         self._flat: Dict[tuple, int] = {}
+        self._views: Dict[tuple, torch.Tensor] = {}         # get(): a slice and a view cost 3 us, a layer of a decode step asks for ten
 
     def reserve(self, name: str, dtype, cols: int):
         key = (name, dtype)
@@ -101,6 +102,7 @@ class Scratch:
     def allocate(self):
         for key, cols in self._need.items():
             self._bufs[key] = torch.empty((self.rows * cols,), dtype=key[1], device=self.device)
+        self._views.clear()
         for key, n in self._flat.items():
             self._bufs[key] = torch.zeros((n,), dtype=key[1], device=self.device)
 
@@ -108,7 +110,13 @@ class Scratch:
         return self._bufs[(name, dtype)]
 
     def get(self, name: str, dtype, M: int, cols: int) -> torch.Tensor:
-        return self._bufs[(name, dtype)][:M * cols].view(M, cols)
+        key = (name, dtype, M, cols)
+        v = self._views.get(key)
+        if v is None:
+            if len(self._views) >= 512:                     # (numbers of rows that come and go)
+                self._views.clear()
+            v = self._views[key] = self._bufs[(name, dtype)][:M * cols].view(M, cols)
+        return v
 
 
 def _round8(n: int) -> int:
