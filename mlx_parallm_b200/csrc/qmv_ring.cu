@@ -6,7 +6,7 @@
 // weight to spend on them (60 % of its issue slots, so it needs four warps per scheduler to cover their latencies).  What else
 // bounds the stream is bytes in flight (a microsecond of latency times 44 KB per microsecond and SM) and the start: every kernel of a
 // decode step begins with an empty pipe.  Hence
-//   * every warp owns a ring of TMA stages (16 rows x 512 k: codes, scales, biases) that it refills itself, lane 0 issuing, as soon
+//   * every warp owns a ring of TMA stages (16 rows x 512 k: codes, scales, biases) that it refills itself, an elected lane issuing, as soon
 //     as a stage sits in registers: no producer warp, no barrier between warps, no register spent on loads in flight;
 //   * the rings are filled BEFORE griddepcontrol.wait (weights depend on no previous kernel), so under programmatic dependent launch
 //     a matrix starts to stream in while its predecessor still computes;
@@ -24,8 +24,8 @@
 // 9 to 16 run when the path is forced.)
 //
 // Measured (CUDA graph over weight copies larger than L2, us; before: the tile kernel and the register GEMV): gate|up 28672 x 4096 4-bit
-// f16 at M = 1 / 4 / 6: 16.2 / 17.9 / 18.5 (21.7 / 22.0 / 22.1), = 4.1 TB/s at M = 1; 34816 x 5120 at M = 1: 22.0 (26.8), = 4.6 TB/s;
-// 57344 x 8192 8-bit: 82 (92), = 6.1 TB/s; down 4096 x 14336 at M = 1: 11.2 (13.2).  Two warps per scheduler instead of four: 19.1.
+// f16 at M = 1 / 4: 16.0 / 17.2 (21.7 / 22.0; with the copies issued under lane == 0 16.5 / 17.9), = 4.1 TB/s at M = 1; 34816 x 5120 at M = 1: 21.4
+// (26.8), = 4.7 TB/s; 57344 x 8192 8-bit: 78.5 (92), = 6.3 TB/s; down 4096 x 14336 at M = 1: 11.0 (13.2).  Two warps per scheduler instead of four: 19.1.
 //
 // Algorithmic HBM bytes per launch: N*K*bits/8 + 2*N*(K/64)*2.
 #include <cuda.h>
