@@ -17,7 +17,8 @@ namespace b200p {
 int sm_count();
 bool pdl_enabled_gemm();
 
-__device__ __forceinline__ float silu_f(float z) { return __fdividef(z, 1.f + __expf(-z)); }
+// (a true quotient: __fdividef is 0 where the divisor is above 2^126, and float32 models round nothing away behind it)
+__device__ __forceinline__ float silu_f(float z) { return z / (1.f + __expf(-z)); }
 __device__ __forceinline__ float softplus_f(float z) { return z > 20.f ? z : log1pf(expf(z)); }
 
 constexpr int DELTA_MAX_TAPS = 16;

@@ -841,3 +841,28 @@ def test_delta_out_widths(dtype, H, dv, col):
         want = (x * torch.rsqrt(x.square().mean(-1, keepdim=True) + 1e-5) * w.double()).reshape(M, -1) * s
         tol = {torch.float32: 4e-6, torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11}[dtype]      # one rounding
         assert (out.double() - want).abs().max() <= tol * float(want.abs().max())
+
+
+def test_silu_of_the_delta_kernels_keeps_its_fp32_range():
+    """silu(z) for z = -88.5 .. 88.5 wherever the recurrent mixers apply it (convolved q, k, v, the plain accumulation's inputs, the head norm's
+    gate of a float32 model) against float64, relative to each value: the smallest, -88 e^-88 = -5e-37, is a normal fp32 number.  Bound:
+    __expf's documented error of 2 + 1.173 * 88.5 units in the last place of 2^-23, and two more roundings."""
+    from mlx_parallm_b200 import ops
+    H, KH, dk, dv, taps, M, bound = 1, 1, 128, 128, 4, 3, 1.3e-5
+    z = torch.linspace(-88.5, 88.5, 2 * dk + dv, dtype=torch.float64).float().cuda().repeat(M, 1)
+    want = z.double() * torch.sigmoid(z.double())
+    rel = lambda got, ref: float(((got.double() - ref).abs() / ref.abs().clamp(min=1e-300)).max())        # noqa: E731
+    f32, i32 = dict(dtype=torch.float32, device="cuda"), dict(dtype=torch.int32, device="cuda")
+    q, k, v, decay = (torch.zeros(M, n, **f32) for n in (dk, dk, dv, H))
+    ops.linear_attn_prep(z, torch.ones(H, **f32), q, k, v, decay, H, dk, dv)
+    assert rel(torch.cat([q, k, v], 1), want) < bound
+    conv_w = torch.zeros(2 * dk + dv, taps, **f32)
+    conv_w[:, -1] = 1                                                  # the convolution hands its newest input through
+    proj, beta, pos = torch.cat([z, z[:, :H]], 1), torch.zeros(M, H, **f32), torch.arange(M, **i32)
+    ops.delta_prep(proj, 2 * dk + dv, z[:, :H], conv_w, torch.zeros(1, taps - 1, 2 * dk + dv, **f32), torch.zeros(H, **f32), torch.zeros(H, **f32),
+                   torch.zeros(M, **i32), pos, pos, q, k, v, beta, decay, H, KH, dk, dv, taps)
+    assert rel(v, want[:, 2 * dk:]) < bound                            # (q and k are made unit vectors)
+    for heads in (3, 1):                                               # heads of 128 values in 16-byte pieces; one group of all
+        gate, o, out = z[:, :dv * 3].contiguous(), torch.ones(M, 3 * dv, **f32), torch.zeros(M, 3 * dv, **f32)
+        ops.delta_out(o, gate, torch.ones(3 * dv // heads, **f32), out, heads, 3 * dv // heads, 0.0)
+        assert rel(out, want) < bound
