@@ -124,14 +124,17 @@ __device__ __forceinline__ float glu_unit(float gate, float up, int epi, float2 
   return gate / (1.f + expf(-gate)) * up;                          // B200P_GEMM_GLU_SILU
 }
 
-// The same where the result is rounded to 16 bits: the unit's exponential and quotient from the approximate instructions (2e-6 of the
-// result over gates of -20 .. 20, against half a unit of 4.9e-4 in f16).  The exact quotient's slow path bounded the prompts' epilogues.
+// z * sigmoid(c z) with the approximate exponential and quotient.  The exponent is never positive and the divisor lies in 1 .. 2, so neither
+// overflows and nothing is lost where z / (1 + e^(-c z)) would divide by more than 2^126 (__fdividef gives 0 there).
+__device__ __forceinline__ float z_sigmoid_approx(float z, float c) {
+  const float t = __expf(-fabsf(c * z));
+  return __fdividef(z < 0.f ? z * t : z, 1.f + t);
+}
+// The same where the result is rounded to 16 bits: __expf's error, 2 + 1.17 |z| units of 2^-23 (1.3e-5 of the result at gates of -88, 3e-6 at
+// -20), against half a unit of 4.9e-4 in f16, 3.9e-3 in bf16.  The exact quotient's slow path bounded the prompts' epilogues.
 __device__ __forceinline__ float glu_unit16(float gate, float up, int epi, float2 act) {
-  if (epi == B200P_GEMM_GLU_SILU) return __fdividef(gate, 1.f + __expf(-gate)) * up;
-  if (epi == B200P_GEMM_GLU_CLAMP) {
-    const float g = fminf(gate, act.x), u = fminf(fmaxf(up, -act.x), act.x);
-    return __fdividef(g, 1.f + __expf(-1.702f * g)) * (u + 1.f);
-  }
+  if (epi == B200P_GEMM_GLU_SILU) return z_sigmoid_approx(gate, 1.f) * up;
+  if (epi == B200P_GEMM_GLU_CLAMP) return z_sigmoid_approx(fminf(gate, act.x), 1.702f) * (fminf(fmaxf(up, -act.x), act.x) + 1.f);
   return gelu_tanh_unit(gate) * up;
 }
 

@@ -866,3 +866,25 @@ def test_silu_of_the_delta_kernels_keeps_its_fp32_range():
         gate, o, out = z[:, :dv * 3].contiguous(), torch.ones(M, 3 * dv, **f32), torch.zeros(M, 3 * dv, **f32)
         ops.delta_out(o, gate, torch.ones(3 * dv // heads, **f32), out, heads, 3 * dv // heads, 0.0)
         assert rel(out, want) < bound
+
+
+@pytest.mark.parametrize("M", [9, 33, 65, 300])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_gated_units_of_the_tcgen05_products_keep_their_range(dtype, M):
+    """Gates of -88 .. 88 (silu) and -51 .. 51 (clamped, whose sigmoid has 1.702 z) beside an up value of 2^100 in bf16, 1 in f16: each result
+    against float64, relative to itself: half a unit of the storage type, and __expf's documented error (2 + 1.17 * 88 units of 2^-23) with
+    the few roundings of the unit."""
+    from mlx_parallm_b200 import _lib, ops
+    up = 2.0 ** 100 if dtype == torch.bfloat16 else 1.0
+    half, tiny = (2.0 ** -8, 2.0 ** -126) if dtype == torch.bfloat16 else (2.0 ** -11, 2.0 ** -14)
+    for epi, c, most, add in ((_lib.GEMM_GLU_SILU, 1.0, 88.0, 0.0), (_lib.GEMM_GLU_CLAMP, 1.702, 51.0, 1.0)):
+        gates = torch.linspace(-most, most, 200, dtype=torch.float64).to(dtype).cuda()
+        w = torch.zeros(400, 64, dtype=dtype, device="cuda")
+        w[0::2, 0], w[1::2, 0] = gates, up
+        x = torch.zeros(M, 64, dtype=dtype, device="cuda")
+        x[:, 0] = 1
+        got = ops.gemm(x, w, epi, act=(2.0 ** 101, 0.0)).double()
+        z = gates.double()
+        want = (z * torch.sigmoid(c * z) * (up + add)).expand(M, -1)
+        err = (got - want).abs() / want.abs().clamp(min=tiny)          # (below the normal numbers: of the smallest of them)
+        assert float(err.max()) <= half + 1.4e-5
