@@ -19,6 +19,16 @@ bool pdl_enabled_gemm();
 
 // (a true quotient: __fdividef is 0 where the divisor is above 2^126, and float32 models round nothing away behind it)
 __device__ __forceinline__ float silu_f(float z) { return z / (1.f + __expf(-z)); }
+// The same bits without the division's branch to its special cases (of all 2^32 arguments two subnormal ones differ by a unit, and -0 gives 0):
+// approximate reciprocal, then one step on the residual (Markstein, IBM J. Res. Dev. 34, 1990).  An infinite divisor or z has no residual (NaN);
+// the first product is the result then: -0, infinity or NaN, as for the division.
+__device__ __forceinline__ float silu_straight_f(float z) {
+  const float d = 1.f + __expf(-z);
+  float r;
+  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(d));
+  const float q = z * r, rest = fmaf(-d, q, z);
+  return rest == rest ? fmaf(rest, r, q) : q;
+}
 __device__ __forceinline__ float softplus_f(float z) { return z > 20.f ? z : log1pf(expf(z)); }
 
 constexpr int DELTA_MAX_TAPS = 16;
@@ -74,10 +84,11 @@ delta_prep_kernel(const float* __restrict__ proj, int64_t ldp, int64_t col_b, co
 // The same for heads that are runs of 128 channels: a warp takes 128 channels (one q or k head, a piece of v, of the decays or
 // of beta) through TT consecutive tokens, lane l the channels l, l + 32, l + 64, l + 96, and keeps the last TAPS - 1 inputs in
 // registers, so the fp32 projection is read once instead of TAPS times.  Same operations in the same order per value as above: the
-// results are bit for bit those of delta_prep_kernel.  Bound: instructions (two exponentials and a logarithm per decay) and the latency of a warp's
-// reads, which are asked for together; four tokens keep code and registers small (eight ran out of the instruction cache).  16 + 16 heads of
-// 128, decays per channel, us: 1664 tokens 38 -> 29 (one token ahead, eight tokens per warp, before), 400 15.5 -> 11.2, 4 tokens (a block per token
-// before) 10.4 -> 4.2.
+// results are bit for bit those of delta_prep_kernel.  Bound: instructions (two exponentials and a logarithm per decay, an exponential and a
+// quotient per channel) and the latency of a warp's reads, which are asked for together; longer runs of tokens read the inputs before the first
+// fewer times, shorter ones give a small call more warps.  16 + 16 heads of 128, us, decays per head / per channel, 1 (up to 128 tokens), 4 (to
+// 512), 8 tokens at a time: 64 tokens 2.9 / 4.0, 496 8.7 / 13.1, 1664 24.7 / 42.2 (a block per token 10.5 / 11.1, the loop before, one token ahead,
+// 9.7 / 15.1 and 26.6 / 50.0; four at a time 26.7 / 41.9; with the quotient's special cases 29.7 / 44.3).
 template <int TAPS, int TT>
 __global__ void __launch_bounds__(128)
 delta_prep_rows_kernel(const float* __restrict__ proj, int64_t ldp, int64_t col_b, const float* __restrict__ a, int64_t lda, int dper,
@@ -162,7 +173,7 @@ delta_prep_rows_kernel(const float* __restrict__ proj, int64_t ldp, int64_t col_
       float acc = 0.f;
 #pragma unroll
       for (int j = 0; j < TAPS; ++j) acc = fmaf(w[r][j], win[r][j], acc);
-      act[r] = silu_f(acc);
+      act[r] = silu_straight_f(acc);
     }
     if (unit >= 2 * KH) {
 #pragma unroll
@@ -910,9 +921,9 @@ extern "C" int b200p_delta_prep(const float* proj, int64_t ldp, int64_t col_b, c
   const size_t smem = (size_t)2 * KH * dk * sizeof(float);
   B200P_REQUIRE(smem <= 48 * 1024, B200P_ERR_ARG, "q and k of one token must fit 48 KB of shared memory");
   if (M < (1ll << 30) && dk == 128 && dv % 128 == 0 && taps == 4) {             // heads of 128 channels; fewer tokens, shorter runs of them per warp
-    const int tt = M > 128 ? 4 : 1, nd = H * decay_per_head;
+    const int tt = M > 512 ? 8 : M > 128 ? 4 : 1, nd = H * decay_per_head;
     const int units = 2 * KH + H * dv / 128 + (nd + 127) / 128 + (H + 127) / 128;
-    const auto kern = tt == 4 ? delta_prep_rows_kernel<4, 4> : delta_prep_rows_kernel<4, 1>;
+    const auto kern = tt == 8 ? delta_prep_rows_kernel<4, 8> : tt == 4 ? delta_prep_rows_kernel<4, 4> : delta_prep_rows_kernel<4, 1>;
     kern<<<dim3((unsigned)((M + tt - 1) / tt), (unsigned)((units + 3) / 4)), 128, 0, (cudaStream_t)stream>>>(
         proj, ldp, col_b, a, lda, decay_per_head, conv_w, conv_state, A_log, dt_bias, t_row, t_pos, t_off, qn, kn, v, beta, decay, (int)M, H, KH, dv);
     B200P_LAUNCH_CHECK("delta_prep_rows_kernel");
