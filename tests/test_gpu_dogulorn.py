@@ -766,10 +766,11 @@ def test_delta_scan_of_long_entries(mode, dk, dv, H, KH, shift):
     assert torch.equal(state[3], state0[3])                              # a row that no entry names is not touched
 
 
-@pytest.mark.parametrize("lens,H,KH,dv,channel", [([257], 1, 1, 128, False), ([1, 300, 2], 3, 1, 256, True), ([130, 3, 129, 9], 4, 2, 128, True)])
+@pytest.mark.parametrize("lens,H,KH,dv,channel", [([3, 1, 20], 2, 1, 128, True), ([257], 1, 1, 128, False), ([1, 300, 2], 3, 1, 256, True),
+                                                  ([130, 3, 129, 9], 4, 2, 128, True), ([5, 600, 2, 30], 2, 2, 128, False)])
 def test_delta_prep_rows_equals_the_per_token_kernel(lens, H, KH, dv, channel):
-    """Prompts of more than 256 tokens with 128-channel heads (one warp per 128 channels and 8 tokens) against the per-token kernel fed
-    the same portions in two halves: bit for bit, entries that begin inside a warp's tokens and carried inputs among them."""
+    """Heads of 128 channels and four taps (a warp per 128 channels and 1, 4 or 8 tokens) against the kernel of a block per token, which takes the
+    same convolution as five taps, the oldest of weight zero: bit for bit, entries that begin inside a warp's tokens and carried inputs among them."""
     from mlx_parallm_b200 import ops
     dk, taps, M, nb = 128, 4, sum(lens), len(lens)
     C, f32, i32 = 2 * KH * dk + H * dv, torch.float32, torch.int32
@@ -784,21 +785,18 @@ def test_delta_prep_rows_equals_the_per_token_kernel(lens, H, KH, dv, channel):
     t = [torch.zeros(M, dtype=i32, device="cuda") for _ in range(3)]
     ops.ragged_plan(cu, rows, lengths, *t, nb, M)
 
-    def run(parts):
+    def run(conv_w, state, taps):
         out = [torch.zeros((M, n), dtype=f32, device="cuda") for n in (KH * dk, KH * dk, H * dv, H, n_dec)]
-        for lo, hi in parts:
-            # the per-token kernel reads earlier inputs of a portion from the rows before its own: give it the whole tensors' slices
-            ops.delta_prep(proj[lo:hi], C, a[lo:hi], conv_w, state, A_log, dt_bias, *(x[lo:hi].contiguous() for x in t), *(o[lo:hi] for o in out),
-                           H, KH, dk, dv, taps)
+        ops.delta_prep(proj, C, a, conv_w, state, A_log, dt_bias, *t, *out, H, KH, dk, dv, taps)
         return out
 
-    whole = run([(0, M)])
-    cuts = list(range(0, M, 200)) + [M]
-    for w, p in zip(whole, run(list(zip(cuts[:-1], cuts[1:])))):
+    per_token = run(torch.cat([torch.zeros(C, 1, device="cuda"), conv_w], 1), torch.cat([rnd(nb, 1, C), state], 1), taps + 1)
+    for w, p in zip(run(conv_w, state, taps), per_token):
         assert torch.equal(w, p)
 
 
-@pytest.mark.parametrize("M,H,KH,dv,channel", [(1, 3, 1, 128, True), (128, 2, 2, 256, False), (131, 2, 1, 128, True), (1025, 2, 1, 128, True)])
+@pytest.mark.parametrize("M,H,KH,dv,channel", [(1, 3, 1, 128, True), (128, 2, 2, 256, False), (131, 2, 1, 128, True), (512, 1, 1, 128, False), (513, 1, 1, 128, False),
+                                                 (1025, 2, 1, 128, True)])
 def test_delta_prep_of_128_channel_heads(M, H, KH, dv, channel):
     """A warp per 128 channels and 1, 4 or 8 tokens (by their number), one sequence that carries inputs: against float64."""
     from mlx_parallm_b200 import ops
