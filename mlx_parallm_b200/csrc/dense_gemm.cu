@@ -443,9 +443,16 @@ static int gemm_grouped_dispatch(const void* x, const void* w, void* y, const in
   const T* wp = (const T*)w;
   if constexpr (!std::is_same<T, float>::value) {
     if (fast_ok && g_gemm_path != 1) {
-      const int rc = gemm_tc_launch_grouped<T>(xp, wp, y, seg, total_rows, max_rows, N, K, ldx, ldw, ldy, groups, sw, epi, act, two_fast ? two : nullptr, st);
-      if (rc == B200P_OK && two && !two_fast)
-        return gemm_dispatch<T>(two->x, two->w, two->y, two->M, two->N, two->K, two->ldx, two->ldw, two->ldy, 1, 0, 0, 0, epi, act, false, st);
+      // a plain product that cannot ride along, or whose launch together is declined, leaves the grouped one on tcgen05
+      const bool ride = two && two_fast && two->M == max_rows && two->K >= 64;
+      auto run = [&](const GemmTcPlain* with) {
+        return gemm_tc_launch_grouped<T>(xp, wp, y, seg, total_rows, max_rows, N, K, ldx, ldw, ldy, groups, sw, epi, act, with, st);
+      };
+      int rc = run(ride ? two : nullptr);
+      const bool alone = two && (!ride || rc == 1);
+      if (ride && rc == 1) rc = run(nullptr);
+      if (rc == B200P_OK && alone)
+        return gemm_dispatch<T>(two->x, two->w, two->y, two->M, two->N, two->K, two->ldx, two->ldw, two->ldy, 1, 0, 0, 0, epi, act, two_fast, st);
       if (rc != 1) return rc;
     }
   }

@@ -707,3 +707,19 @@ def test_grouped_products_with_a_plain_one(dtype, E, top, tokens, N, K, N2, K2):
         assert (y2[:tokens].double().cpu() - want).abs().max() <= tol * max(1.0, float(want.abs().max())), epi
         assert float((y2[tokens:] - 5.0).abs().max()) == 0.0
     assert _lib.lib().b200p_gemm_tc_fault() == 0
+
+
+@pytest.mark.parametrize("tokens,M2,K2", [(40, 40, 40), (40, 12, 128), (200, 200, 56), (200, 190, 128)])
+def test_grouped_product_keeps_its_kernel_beside_one_that_cannot_share_its_launch(tokens, M2, K2):
+    """A plain product of fewer than 64 channels, or of another number of rows than a group may have, is launched by itself: both results have
+    the bits that they have alone (another kernel sums the 2048 products in another order)."""
+    from mlx_parallm_b200 import _lib, ops
+    E, top, N, N2, K = 16, 2, 2048, 264, 2048
+    g = torch.Generator(device="cuda").manual_seed(tokens + K2)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()        # noqa: E731
+    x, w, x2, w2 = rnd(tokens * top, K), rnd(E, N, K), rnd(M2, K2), rnd(N2, K2)
+    seg = torch.arange(E + 1, dtype=torch.int32, device="cuda") * (tokens * top // E)
+    y2 = torch.zeros(M2, N2, device="cuda")
+    y = ops.gemm_grouped(x, w, seg, tokens, _lib.GEMM_STORE_F32, also=(x2, w2, y2))
+    assert torch.equal(y[:seg[-1]], ops.gemm_grouped(x, w, seg, tokens, _lib.GEMM_STORE_F32)[:seg[-1]])
+    assert torch.equal(y2, ops.gemm(x2, w2, _lib.GEMM_STORE_F32))
