@@ -71,8 +71,9 @@ const char* b200p_last_error(void);
 /* 0 iff the current device is compute capability 10.x */
 int b200p_arch_check(void);
 int b200p_sm_count(void);
-/* Programmatic dependent launch for every kernel of the library (default on): kernel N+1's prologue and weight
- * prefetch overlap kernel N's tail; each kernel executes griddepcontrol.wait before touching its inputs. */
+/* Programmatic dependent launch, 0 off: kernel N+1's prologue and weight prefetch overlap kernel N's tail; each kernel executes
+ * griddepcontrol.wait before touching its inputs.  Default (2): the quantised products, the early norms, attention, the delta rule's second
+ * launch, a mixture's kernels except its last (routing and gather up to 64 tokens); 1: every kernel that can be. */
 int b200p_set_pdl(int enabled);
 
 /* mx.dequantize(w, scales, biases, group_size, bits)            [nn.QuantizedEmbedding.__call__,
@@ -432,6 +433,8 @@ int b200p_moe_route(const float* logits, int64_t ldl, const float* bias, int32_t
                     int32_t* token_of, int64_t M, int E, int top, void* stream);
 /* xs[s, :] = x[token_of[s], :], rows of W elements in `dtype` */
 int b200p_moe_gather(const void* x, const int32_t* token_of, void* xs, int64_t slots, int64_t W, int dtype, void* stream);
+/* the same for M tokens of `top` slots each (slots = M * top): told the tokens, a decode batch launches it programmatically like the routing */
+int b200p_moe_gather_tokens(const void* x, const int32_t* token_of, void* xs, int64_t M, int top, int64_t W, int dtype, void* stream);
 /* The same outputs from sigmoid scores s = sigmoid(logits): experts are picked by s + correction (NULL: none) among the experts of
  * the `keep` best of `count` equal groups of neighbouring experts (a group's score = the sum of its two largest picking scores);
  * wts = the picked experts' s divided by their sum (+ 1e-20), times `scale`.  count == 1 or keep == count: no group limit. */

@@ -168,9 +168,9 @@ __host__ __device__ __forceinline__ int perm8_pos(int n) { return (n & ~7) | (((
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
-// Every kernel of the library is launched with programmatic stream serialization (unless b200p_set_pdl(0)): the
-// next kernel's CTAs may be scheduled as soon as this one's have all passed griddepcontrol.launch_dependents or
-// exited, and each kernel executes griddepcontrol.wait before it touches anything a predecessor reads or writes.
+// Programmatic stream serialization (unless b200p_set_pdl(0); which launches carry it by default: include/b200p.h): the launch's CTAs may be
+// scheduled as soon as those of the kernel before have all passed griddepcontrol.launch_dependents or exited, and each such kernel executes
+// griddepcontrol.wait before it touches anything a predecessor reads or writes.
 bool pdl_enabled();
 // kernel class of the C-ABI call being executed (B200P_PDL_MASK selects, per class, which launches carry the PDL attribute):
 // 2 rmsnorm, 4 rope+append, 8 attention, 16 silu_mul, 32 embed / dequantize / advance / samplers, 64 GEMV paths

@@ -191,8 +191,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmw, const __grid_constant__ 
     tma_prefetch_desc(&tmx);
     tma_prefetch_desc(&tmw);
   }
-  if (warp == 1) tmem_alloc(smem_u32(&sh->tmem_base), TMEM_COLS);
-  pdl_launch_dependents();
+  if (warp == 1) {
+    tmem_alloc(smem_u32(&sh->tmem_base), TMEM_COLS);
+    pdl_launch_dependents();                       // (behind the allocation: no successor's CTA can take the columns first and then wait for us)
+  }
   pdl_wait();                                      // operands, seg and y belong to the previous kernels until here
   if (p.seg) {
     for (int i = threadIdx.x; i <= p.groups; i += blockDim.x) sh->seg[i] = p.seg[i];
@@ -451,8 +453,8 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmw, const __grid_consta
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&sh->tmem_base)), "r"(512u) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    pdl_launch_dependents();                                 // (behind the allocation, as above)
   }
-  pdl_launch_dependents();
   pdl_wait();                                                // x, seg and y belong to the previous kernels until here
   if (p.g.seg) {
     for (int i = threadIdx.x; i <= p.g.groups; i += THREADS) sh->seg[i] = p.g.seg[i];
@@ -612,8 +614,10 @@ static void gemm_tc_set_second(GemmTcParams& p, const GemmTcPlain* two, int rows
   p.two.num_kb = (int)((two->K + GT_BK - 1) / GT_BK);
 }
 
+// pdl: launched programmatically.  A mixture's products are, between its other kernels; a plain product, of which a program may issue any
+// number in a row, is not (moe.cu: streams of nothing but programmatic launches).
 template <typename T, int BN, int STAGES>
-static int gemm_tc_run(const CUtensorMap* tm, GemmTcParams p, cudaStream_t st) {
+static int gemm_tc_run(const CUtensorMap* tm, GemmTcParams p, bool pdl, cudaStream_t st) {
   constexpr size_t smem = 1024 + (size_t)STAGES * (GT_A_BYTES + BN * GT_BK * 2) + sizeof(GemmTcShared);
   auto kern = gemm_tc_kernel<T, BN, STAGES>;
   static bool attr_set = false;
@@ -624,7 +628,7 @@ static int gemm_tc_run(const CUtensorMap* tm, GemmTcParams p, cudaStream_t st) {
   }
   if (const int rc = wait_word(WAIT_GEMM_TC, &p.wait_word)) return rc;
   const int tiles = p.num_tiles + p.two.num_tiles, grid = tiles < sm_count() ? tiles : sm_count();
-  cudaError_t e = launch_pdl_opt(pdl_enabled_gemm(), kern, dim3((unsigned)grid), dim3(GT_THREADS), smem, st, tm[0], tm[1], tm[2], tm[3], p);
+  cudaError_t e = launch_pdl_opt(pdl && pdl_enabled_gemm(), kern, dim3((unsigned)grid), dim3(GT_THREADS), smem, st, tm[0], tm[1], tm[2], tm[3], p);
   if (e != cudaSuccess) return cuda_fail(e, "gemm_tc_kernel launch");
   return B200P_OK;
 }
@@ -632,7 +636,7 @@ static int gemm_tc_run(const CUtensorMap* tm, GemmTcParams p, cudaStream_t st) {
 namespace pair {
 
 template <typename T>
-static int run(const CUtensorMap* tm, Params p, int64_t tiles, cudaStream_t st) {
+static int run(const CUtensorMap* tm, Params p, int64_t tiles, bool pdl, cudaStream_t st) {
   constexpr size_t smem = 1024 + (size_t)STAGES * STAGE_BYTES + sizeof(Shared);
   auto kern = gemm_tc_pair_kernel<T>;
   static bool attr_set = false;
@@ -644,7 +648,7 @@ static int run(const CUtensorMap* tm, Params p, int64_t tiles, cudaStream_t st) 
   if (const int rc = wait_word(WAIT_GEMM_TC, &p.g.wait_word)) return rc;
   const int64_t pairs = sm_count() / 2;
   const unsigned grid = 2u * (unsigned)(tiles < pairs ? tiles : pairs);
-  cudaError_t e = launch_pdl_opt(pdl_enabled_gemm(), kern, dim3(grid), dim3(THREADS), smem, st, tm[0], tm[1], tm[2], tm[3], p);
+  cudaError_t e = launch_pdl_opt(pdl && pdl_enabled_gemm(), kern, dim3(grid), dim3(THREADS), smem, st, tm[0], tm[1], tm[2], tm[3], p);
   if (e != cudaSuccess) return cuda_fail(e, "gemm_tc_pair_kernel launch");
   return B200P_OK;
 }
@@ -699,7 +703,7 @@ static int launch(TcEncodeFn enc, const T* x, const T* w, void* y, const int32_t
     if (!gemm_tc_map(enc, &tm[2], dt, two->w, two->K, two->N, 1, two->ldw, 0, 128)) return 1;
     if (!gemm_tc_map(enc, &tm[3], dt, two->x, two->K, two->M, 1, two->ldx, 0, g.two.tn / 2)) return 1;
   }
-  return run<T>(tm, p, tiles + g.two.num_tiles, st);
+  return run<T>(tm, p, tiles + g.two.num_tiles, seg != nullptr, st);
 }
 
 }  // namespace pair
@@ -741,8 +745,8 @@ static int gemm_tc_launch_decode(TcEncodeFn enc, const T* x, const T* w, void* y
     if (e != cudaSuccess) return cuda_fail(e, "cudaMemsetAsync(split-K output)");
   }
   gemm_tc_set_second(p, nullptr, GT_BM);
-  if (bn == 32) return gemm_tc_run<T, 32, 10>(tm, p, st);
-  return gemm_tc_run<T, 64, 8>(tm, p, st);
+  if (bn == 32) return gemm_tc_run<T, 32, 10>(tm, p, false, st);
+  return gemm_tc_run<T, 64, 8>(tm, p, false, st);
 }
 
 // Returns B200P_OK, an error, or 1 when the shape is not one this kernel takes (the caller then runs the mma.sync kernel).
@@ -803,7 +807,7 @@ int gemm_tc_launch_grouped(const T* x, const T* w, void* y, const int32_t* seg, 
   p.epi = epi;
   p.act = act;
   gemm_tc_set_second(p, two, GT_BM);
-  return bn == 32 ? gemm_tc_run<T, 32, 10>(tm, p, st) : gemm_tc_run<T, 64, 8>(tm, p, st);
+  return bn == 32 ? gemm_tc_run<T, 32, 10>(tm, p, true, st) : gemm_tc_run<T, 64, 8>(tm, p, true, st);
 }
 template int gemm_tc_launch_grouped<__half>(const __half*, const __half*, void*, const int32_t*, int64_t, int64_t, int64_t, int64_t, int64_t,
                                             int64_t, int64_t, int64_t, int64_t, int, float2, const GemmTcPlain*, cudaStream_t);

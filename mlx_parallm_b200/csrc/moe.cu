@@ -13,9 +13,12 @@
 namespace b200p {
 
 bool pdl_enabled_gemm();
-// Programmatic launches for decode batches, where the gaps between these kernels are a tenth of the call (32 tokens, 16 experts of 2048 x
-// 2048: 129 -> 100 us with the shared expert's products beside the routed ones').  Prompts launch plainly: the gaps are a hundredth there, and
-// a stream that holds nothing but programmatic launches did not come to its end under CUPTI's kernel tracing.
+// Programmatic launches for decode batches of up to 64 tokens, where the gaps between these kernels are a tenth of the call (32 tokens, 16
+// experts of 2048 x 2048: 129 -> 102 us with the shared expert's products beside the routed ones').  Prompts launch plainly (the gaps are a
+// hundredth there), and moe_combine, which ends every mixture, always does: a stream that held nothing but programmatic launches of these kernels
+// and the products did not come to its end under CUPTI's kernel tracing, for a reason that the kernels do not show (each waits for its predecessor,
+// allows its successor only once it holds its TMEM, and every other wait is bounded), so no chain of mixtures or of
+// plain dense products is one.
 static bool moe_pdl(int64_t tokens) { return pdl_enabled_gemm() && tokens <= 64; }
 
 constexpr int MOE_MAX_PER_LANE = 32;    // experts <= 1024
@@ -296,8 +299,6 @@ __global__ void moe_combine_kernel(const float* __restrict__ ye, const int32_t* 
                                    const float* __restrict__ shared_y, const float* __restrict__ shared_gate, int64_t ldg,
                                    float* __restrict__ y, int64_t W, int top) {
   const int64_t t = blockIdx.x;
-  pdl_launch_dependents();
-  pdl_wait();
   const float sg = shared_gate ? 1.f / (1.f + expf(-shared_gate[t * ldg])) : 1.f;
   __shared__ int32_t sl[MOE_MAX_TOP];
   __shared__ float wt[MOE_MAX_TOP];
@@ -414,14 +415,23 @@ extern "C" int b200p_moe_scatter_scaled(const void* x, const int32_t* slot_of, c
   return B200P_OK;
 }
 
-extern "C" int b200p_moe_gather(const void* x, const int32_t* token_of, void* xs, int64_t slots, int64_t W, int dtype, void* stream) {
+static int moe_gather_call(const void* x, const int32_t* token_of, void* xs, int64_t slots, bool pdl, int64_t W, int dtype, void* stream) {
   B200P_REQUIRE(x && token_of && xs && W > 0, B200P_ERR_ARG, "null pointer");
   if (slots == 0) return B200P_OK;
   cudaError_t e = cudaSuccess;
-  B200P_DISPATCH_DTYPE(dtype, T, (e = launch_pdl_opt(moe_pdl(slots / 4), moe_gather_kernel<T>, dim3((unsigned)slots), dim3(128), 0, (cudaStream_t)stream,
+  B200P_DISPATCH_DTYPE(dtype, T, (e = launch_pdl_opt(pdl, moe_gather_kernel<T>, dim3((unsigned)slots), dim3(128), 0, (cudaStream_t)stream,
                                                      (const T*)x, token_of, (T*)xs, W)));
   if (e != cudaSuccess) return cuda_fail(e, "moe_gather_kernel launch");
   return B200P_OK;
+}
+
+extern "C" int b200p_moe_gather(const void* x, const int32_t* token_of, void* xs, int64_t slots, int64_t W, int dtype, void* stream) {
+  return moe_gather_call(x, token_of, xs, slots, false, W, dtype, stream);
+}
+
+extern "C" int b200p_moe_gather_tokens(const void* x, const int32_t* token_of, void* xs, int64_t M, int top, int64_t W, int dtype, void* stream) {
+  B200P_REQUIRE(M >= 0 && top > 0 && top <= MOE_MAX_TOP, B200P_ERR_ARG, "bad token count or top");
+  return moe_gather_call(x, token_of, xs, M * top, moe_pdl(M), W, dtype, stream);
 }
 
 extern "C" int b200p_moe_combine(const float* ye, const int32_t* slot_of, const float* wts, const float* shared_y,
@@ -430,8 +440,7 @@ extern "C" int b200p_moe_combine(const float* ye, const int32_t* slot_of, const 
   if (M == 0) return B200P_OK;
   const unsigned threads = W >= 1024 ? 256 : 128;
   auto kern = W % 4 == 0 && aligned(ye, 16) && aligned(shared_y, 16) && aligned(y, 16) ? moe_combine_kernel<4> : moe_combine_kernel<1>;
-  cudaError_t e = launch_pdl_opt(moe_pdl(M), kern, dim3((unsigned)M), dim3(threads), 0, (cudaStream_t)stream, ye, slot_of, wts, shared_y,
-                                 shared_gate, ldg, y, W, top);
-  if (e != cudaSuccess) return cuda_fail(e, "moe_combine_kernel launch");
+  kern<<<(unsigned)M, threads, 0, (cudaStream_t)stream>>>(ye, slot_of, wts, shared_y, shared_gate, ldg, y, W, top);
+  B200P_LAUNCH_CHECK("moe_combine_kernel");
   return B200P_OK;
 }

@@ -481,8 +481,12 @@ def moe_route(logits, bias, ids, wts, seg, slot_of, token_of, top: int):
 def moe_gather(x, token_of, xs):
     _dev(x, token_of, xs)
     assert x.is_contiguous() and xs.is_contiguous() and x.dtype == xs.dtype and x.shape[1] == xs.shape[1]
-    _call("b200p_moe_gather", lambda: lib().b200p_moe_gather(_p(x), _p(token_of), _p(xs), xs.shape[0], x.shape[1], dtype_code(x.dtype),
-                                                            _stream()))
+    M, slots = x.shape[0], xs.shape[0]
+    if M and slots and slots % M == 0 and slots // M <= 32:
+        _call("b200p_moe_gather", lambda: lib().b200p_moe_gather_tokens(_p(x), _p(token_of), _p(xs), M, slots // M, x.shape[1], dtype_code(x.dtype),
+                                                                       _stream()))
+    else:
+        _call("b200p_moe_gather", lambda: lib().b200p_moe_gather(_p(x), _p(token_of), _p(xs), slots, x.shape[1], dtype_code(x.dtype), _stream()))
 
 
 def moe_route_sigmoid(logits, correction, ids, wts, seg, slot_of, token_of, top: int, groups: int = 1, keep: int = 1, scale: float = 1.0,

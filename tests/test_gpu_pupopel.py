@@ -723,3 +723,48 @@ def test_grouped_product_keeps_its_kernel_beside_one_that_cannot_share_its_launc
     y = ops.gemm_grouped(x, w, seg, tokens, _lib.GEMM_STORE_F32, also=(x2, w2, y2))
     assert torch.equal(y[:seg[-1]], ops.gemm_grouped(x, w, seg, tokens, _lib.GEMM_STORE_F32)[:seg[-1]])
     assert torch.equal(y2, ops.gemm(x2, w2, _lib.GEMM_STORE_F32))
+
+
+def captured_edges(fn):
+    """Kinds of the edges between the launches of fn() in issue order: True programmatic, False full."""
+    import ctypes as C
+    g = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(g):
+        fn()
+    rt, n = C.CDLL("libcudart.so.12"), C.c_size_t(0)
+    graph = C.c_void_p(g.raw_cuda_graph())
+    assert rt.cudaGraphGetEdges_v2(graph, None, None, None, C.byref(n)) == 0
+    a, b, data = (C.c_void_p * n.value)(), (C.c_void_p * n.value)(), (C.c_ubyte * (8 * n.value))()
+    assert rt.cudaGraphGetEdges_v2(graph, a, b, data, C.byref(n)) == 0
+    kind = {a[i]: (b[i], data[8 * i + 2] == 1) for i in range(n.value)}          # (cudaGraphEdgeData: from_port, to_port, type)
+    at, out = next(iter(set(kind) - {b for b, _ in kind.values()})), []
+    while at in kind:
+        at, programmatic = kind[at]
+        out.append(programmatic)
+    assert len(out) == n.value                                                   # one chain
+    return out
+
+
+@pytest.mark.parametrize("tokens,top", [(32, 2), (40, 8), (64, 1), (65, 1), (100, 1), (300, 2)])
+def test_every_mixture_and_chain_of_products_holds_a_plain_launch(tokens, top):
+    """Streams of nothing but programmatic launches have hung a tracer: the last kernel of a mixture is launched plainly, a prompt's routing and
+    gather are too (by its tokens, whatever the number of choices), and plain dense products always."""
+    from mlx_parallm_b200 import _lib, ops
+    E, K, N = 16, 128, 2048
+    i32, bf = dict(dtype=torch.int32, device="cuda"), dict(dtype=torch.bfloat16, device="cuda")
+    logits, x, w, xs = torch.randn(tokens, E, device="cuda"), torch.randn(tokens, K, **bf), torch.randn(E, N, K, **bf), torch.empty(tokens * top, K, **bf)
+    ids, slot_of, token_of, seg = (torch.zeros(n, **i32) for n in ((tokens, top), (tokens, top), (tokens * top,), (E + 1,)))
+    wts, ye, y = torch.zeros(tokens, top, device="cuda"), torch.zeros(tokens * top, N, device="cuda"), torch.zeros(tokens, N, device="cuda")
+
+    def mixture():
+        ops.moe_route(logits, None, ids, wts, seg, slot_of, token_of, top)
+        ops.moe_gather(x, token_of, xs)
+        ops.gemm_grouped(xs, w, seg, tokens, _lib.GEMM_STORE_F32, out=ye)
+        ops.moe_combine(ye, slot_of, wts, None, y, top)
+
+    mixture()
+    torch.cuda.synchronize()
+    gather_to_products, products_to_combine = captured_edges(mixture)[-2:]
+    assert gather_to_products and not products_to_combine
+    assert captured_edges(mixture)[-3] == (tokens <= 64)
+    assert captured_edges(lambda: [ops.gemm(x, w[0], _lib.GEMM_STORE_F32, out=y) for _ in range(3)]) == [False, False]
