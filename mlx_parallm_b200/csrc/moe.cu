@@ -230,7 +230,7 @@ __global__ void moe_plan_kernel(const int32_t* __restrict__ ids, int32_t* __rest
 }
 
 // Decode batches: choice and plan in one block (a launch less; 32 tokens, 16 experts, 2 of them each).
-constexpr int MOE_ONE_BLOCK = 1024;              // (token, choice) pairs
+constexpr int MOE_ONE_BLOCK = 64;                // (token, choice) pairs
 template <int PER_LANE>
 __global__ void __launch_bounds__(1024)
 moe_route_plan_kernel(const float* __restrict__ logits, int64_t ldl, const float* __restrict__ bias, int32_t* __restrict__ ids,
@@ -331,6 +331,11 @@ __global__ void moe_combine_kernel(const float* __restrict__ ye, const int32_t* 
 
 using namespace b200p;
 
+// One block for as few choices as its 32 warps make beside each other.  us, one block / two launches: 16 experts, 2 choices, 16 and 32 tokens 3.0 /
+// 3.65, 3.6 / 3.65, 4 choices of 32 tokens 4.4 / 3.9, 8 of 64 10 / 4.6; 128 experts, 4 choices of 16 tokens 4.2 / 4.3, of 32 5.3 / 4.3; above 128
+// a lane has up to 32 logits: 129 experts, 2 choices of 8 and 16 tokens 5.2 / 5.4, 6.1 / 5.4, 160 experts, 16 choices of 64 tokens 71 / 12.
+static bool moe_one_block(int64_t M, int E, int top) { return E <= 128 ? M <= 32 && M * top <= MOE_ONE_BLOCK : M * top <= 16; }
+
 static int moe_plan_launch(const int32_t* ids, int32_t* seg, int32_t* slot_of, int32_t* token_of, int64_t M, int E, int top, cudaStream_t st) {
   cudaError_t e = launch_pdl_opt(moe_pdl(M), moe_plan_kernel, dim3(1), dim3(1024), 2 * E * sizeof(int32_t), st, ids, seg, slot_of, token_of,
                                  M * top, E, top);
@@ -347,7 +352,7 @@ extern "C" int b200p_moe_route(const float* logits, int64_t ldl, const float* bi
   cudaStream_t st = (cudaStream_t)stream;
   const bool pdl = moe_pdl(M);
   cudaError_t e;
-  if (M * top <= MOE_ONE_BLOCK && M <= 64) {
+  if (moe_one_block(M, E, top)) {
     auto kern = E <= 32 ? moe_route_plan_kernel<1> : E <= 128 ? moe_route_plan_kernel<4> : moe_route_plan_kernel<MOE_MAX_PER_LANE>;
     e = launch_pdl_opt(pdl, kern, dim3(1), dim3(1024), 2 * E * sizeof(int32_t), st, logits, ldl, bias, ids, wts, seg, slot_of, token_of, M, E, top);
     if (e != cudaSuccess) return cuda_fail(e, "moe_route_plan_kernel launch");

@@ -768,3 +768,22 @@ def test_every_mixture_and_chain_of_products_holds_a_plain_launch(tokens, top):
     assert gather_to_products and not products_to_combine
     assert captured_edges(mixture)[-3] == (tokens <= 64)
     assert captured_edges(lambda: [ops.gemm(x, w[0], _lib.GEMM_STORE_F32, out=y) for _ in range(3)]) == [False, False]
+
+
+@pytest.mark.parametrize("E,top,M", [(16, 2, 32), (16, 2, 33), (128, 4, 16), (128, 5, 16), (128, 1, 33), (129, 2, 8), (129, 2, 9), (1024, 16, 1), (1024, 32, 1)])
+def test_routing_in_one_block_and_in_two_launches(E, top, M):
+    """On both sides of the line between them: the chosen experts, their weights, and every choice's slot inside its expert's segment."""
+    from mlx_parallm_b200 import ops
+    g = torch.Generator().manual_seed(E + M)
+    logits = torch.randn(M, E, generator=g)
+    i32 = dict(dtype=torch.int32, device="cuda")
+    ids, slot_of, token_of, seg = (torch.zeros(n, **i32) for n in ((M, top), (M, top), (M * top,), (E + 1,)))
+    wts = torch.zeros(M, top, device="cuda")
+    ops.moe_route(logits.cuda(), None, ids, wts, seg, slot_of, token_of, top)
+    tv, ti = torch.topk(logits.double(), top, -1)
+    assert torch.equal(ids.cpu().long(), ti) and (wts.cpu().double() - torch.softmax(tv, -1)).abs().max() < 1e-6
+    flat, slots = ti.reshape(-1), slot_of.cpu().long().reshape(-1)
+    assert torch.equal(seg.cpu().long(), torch.cat([torch.zeros(1, dtype=torch.long), torch.bincount(flat, minlength=E).cumsum(0)]))
+    assert torch.equal(slots.sort().values, torch.arange(M * top))
+    assert bool((seg.cpu().long()[flat] <= slots).all()) and bool((slots < seg.cpu().long()[flat + 1]).all())
+    assert torch.equal(token_of.cpu().long()[slots], torch.arange(M * top) // top)
