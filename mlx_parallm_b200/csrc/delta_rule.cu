@@ -19,14 +19,16 @@ bool pdl_enabled_gemm();
 
 // (a true quotient: __fdividef is 0 where the divisor is above 2^126, and float32 models round nothing away behind it)
 __device__ __forceinline__ float silu_f(float z) { return z / (1.f + __expf(-z)); }
-// The same bits without the division's branch to its special cases (of all 2^32 arguments two subnormal ones differ by a unit, and -0 gives 0):
-// approximate reciprocal, then one step on the residual (Markstein, IBM J. Res. Dev. 34, 1990).  An infinite divisor or z has no residual (NaN);
-// the first product is the result then: -0, infinity or NaN, as for the division.
+// The same bits without the division's branch to its special cases (of all 2^32 arguments two differ by a unit, and some below 2^-100 in magnitude
+// by a few subnormal ones): approximate reciprocal, then one step on the residual (Markstein, IBM J. Res. Dev. 34, 1990).  Both sides of the quotient
+// carry a factor of 1/4, so that the reciprocal of the largest divisor is a normal number.  An infinite divisor or z has no residual (NaN); the
+// first product is the result then: -0, infinity or NaN, as for the division.
 __device__ __forceinline__ float silu_straight_f(float z) {
-  const float d = 1.f + __expf(-z);
-  float r;
-  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(d));
-  const float q = z * r, rest = fmaf(-d, q, z);
+  float e, r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(z * -1.4426950408889634f));
+  const float d = fmaf(0.25f, e, 0.25f), n = 0.25f * z;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
+  const float q = n * r, rest = fmaf(-d, q, n);
   return rest == rest ? fmaf(rest, r, q) : q;
 }
 __device__ __forceinline__ float softplus_f(float z) { return z > 20.f ? z : log1pf(expf(z)); }
@@ -87,8 +89,8 @@ delta_prep_kernel(const float* __restrict__ proj, int64_t ldp, int64_t col_b, co
 // results are bit for bit those of delta_prep_kernel.  Bound: instructions (two exponentials and a logarithm per decay, an exponential and a
 // quotient per channel) and the latency of a warp's reads, which are asked for together; longer runs of tokens read the inputs before the first
 // fewer times, shorter ones give a small call more warps.  16 + 16 heads of 128, us, decays per head / per channel, 1 (up to 128 tokens), 4 (to
-// 512), 8 tokens at a time: 64 tokens 2.9 / 4.0, 496 8.7 / 13.1, 1664 24.7 / 42.2 (a block per token 10.5 / 11.1, the loop before, one token ahead,
-// 9.7 / 15.1 and 26.6 / 50.0; four at a time 26.7 / 41.9; with the quotient's special cases 29.7 / 44.3).
+// 512), 8 tokens at a time: 64 tokens 2.9 / 4.0, 496 8.3 / 13.0, 1664 22.7 / 40.5 (a block per token 10.5 / 11.1, the loop before, one token ahead,
+// 9.7 / 15.2 and 26.6 / 50.1; with the quotient's special cases, four at a time, 29.7 / 44.3).
 template <int TAPS, int TT>
 __global__ void __launch_bounds__(128)
 delta_prep_rows_kernel(const float* __restrict__ proj, int64_t ldp, int64_t col_b, const float* __restrict__ a, int64_t lda, int dper,
