@@ -389,11 +389,17 @@ int b200p_delta_scan(const float* qn, const float* kn, const float* v, const flo
                      const int32_t* cu, const int32_t* rows, const int32_t* lengths, float* o, int nb, int H, int KH, int dk,
                      int dv, int mode, void* stream);
 /* the same, told how many tokens the entries have together (cu[nb], which lies on the device): decode steps take a kernel of their own.
- * Results do not depend on it (an entry of 32 tokens and more beside as many empty ones excepted: fp32 rounding).  Entries of 32 tokens and
- * more with keys of 65 to 128 channels take two tokens at a time in the delta rule: the same sums in another order than token by token. */
+ * Entries of 32 tokens and more with keys of 65 to 128 channels take two tokens at a time in the delta rule: the same sums in another order
+ * than token by token, so a prompt's portions give its results up to fp32 rounding and not bit for bit.  Otherwise an entry's bits depend on
+ * its own tokens alone, unless it has 32 or more beside at least that many empty entries and the call does not say so (longest). */
 int b200p_delta_scan_tokens(const float* qn, const float* kn, const float* v, const float* beta, const float* decay, float* state,
                             const int32_t* cu, const int32_t* rows, const int32_t* lengths, float* o, int64_t tokens, int nb, int H, int KH,
                             int dk, int dv, int mode, void* stream);
+/* the same, told also how many tokens the longest entry has (0: not known): without one of 32 tokens a launch less.  A number that is too
+ * small costs nothing but the other order of the sums. */
+int b200p_delta_scan_entries(const float* qn, const float* kn, const float* v, const float* beta, const float* decay, float* state,
+                             const int32_t* cu, const int32_t* rows, const int32_t* lengths, float* o, int64_t tokens, int64_t longest, int nb,
+                             int H, int KH, int dk, int dv, int mode, void* stream);
 /* step 4: out[t, h, :] (dtype, row stride ld_out) = out_scale * o / sqrt(mean_dv(o^2) + eps) * norm_w * act(gate[t, h, :]);
  * gate fp32 with row stride ldg; gate_act 0 silu, 1 sigmoid.  H == 1 norms the dv values of a row as one group. */
 int b200p_delta_out(const float* o, const float* gate, int64_t ldg, const float* norm_w, void* out, int64_t ld_out, int64_t M,

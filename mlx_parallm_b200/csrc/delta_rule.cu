@@ -368,8 +368,9 @@ delta_scan_kernel(const float* __restrict__ qn, const float* __restrict__ kn, co
   const bool pairs = NEXT == 1 && (dv & 1) == 0 && (reinterpret_cast<uintptr_t>(state) & 7) == 0;
   const bool live0 = j0 < dv, live1 = j1 < dv, odd = (l & 1) != 0;
   const int t0 = cu[e], t1 = cu[e + 1];
-  if (t1 <= t0 || t1 - t0 > most) {                              // (longer entries: delta_pair_kernel, launched before)
-    pdl_wait();
+  const bool waits = (blockIdx.x | blockIdx.y | blockIdx.z) == 0;        // (see delta_scan_launch: the grid ends no earlier than the launch before)
+  if (t1 <= t0 || t1 - t0 > most) {                              // (longer entries: delta_pair_kernel)
+    if (waits) pdl_wait();
     return;
   }
   const int row = rows[e];
@@ -474,7 +475,6 @@ delta_scan_kernel(const float* __restrict__ qn, const float* __restrict__ kn, co
     __syncthreads();
   }
   put(t1 - 1, ds_reduce<LANES>(out.x, out.y, odd));
-  pdl_wait();                         // (see delta_scan_launch: ends no earlier than the launch before)
 #pragma unroll
   for (int u = 0; u < SUB; ++u)
 #pragma unroll
@@ -495,6 +495,7 @@ delta_scan_kernel(const float* __restrict__ qn, const float* __restrict__ kn, co
         if (live1) s0[dv + j1] = S.c1[u][i].y;
       }
     }
+  if (waits) pdl_wait();
 }
 
 // Prompts of keys of 65 to 128 channels, two tokens at a time.  In the kernels above the chain of one token (dot, reduction over the lanes,
@@ -953,9 +954,9 @@ extern "C" int b200p_delta_conv_commit(const float* proj, int64_t ldp, float* co
   return B200P_OK;
 }
 
-// tokens: of all entries together; 0 if the caller does not say.
+// tokens: of all entries together, longest: of the longest; 0 if the caller does not say.
 template <int MODE>
-static void delta_scan_launch(int64_t tokens, int nb, cudaStream_t st, const float* qn, const float* kn, const float* v, const float* beta,
+static void delta_scan_launch(int64_t tokens, int64_t longest, int nb, cudaStream_t st, const float* qn, const float* kn, const float* v, const float* beta,
                               const float* decay, float* state, const int32_t* cu, const int32_t* rows, const int32_t* lengths,
                               float* o, int H, int KH, int dk, int dv) {
 #define DELTA_STEP(DKP)                                                                                                          \
@@ -971,14 +972,19 @@ static void delta_scan_launch(int64_t tokens, int nb, cudaStream_t st, const flo
   // 4 entries of 16 / 64, 20 / 20, 58 / 50.
   // The plain accumulation of keys above 128 takes it at any length (16 x 250 tokens of 256 x 256: 407 / 678; 4 x 512: 315 / 309).
   const int most = dk > 128 ? 8 : dk > 64 ? 1 : dk > 32 ? 4 : 2;
-  const bool few = (tokens > 0 && tokens <= most * (int64_t)nb) || (MODE == 2 && dk > 128);
+  const bool by_pairs = MODE != 2 && dk > 64 && dk <= 128;                   // entries of DP_MIN tokens and more
+  const bool few = (tokens > 0 && tokens <= most * (int64_t)nb && !(by_pairs && longest >= DP_MIN)) || (MODE == 2 && dk > 128);
   // 128 rows: one CTA per SM takes eight lanes per column and the shortest chain (4 x 512 tokens, 16 heads, decays per channel / per
   // head: 220 / 193 us, the former four-lane kernel 280 / 206); more CTAs than SMs take four (32 heads 379 / 346 -> 356 / 317; 16 x 250
   // tokens 672 / 594 -> 637 / 544).
   const bool crowded = (int64_t)nb * H * ((dv + 63) / 64) > sm_count();
-  // Entries of DP_MIN tokens and more two tokens at a time, the shorter ones by the launch behind it, which needs nothing of it: it may start
-  // at once (its inputs were complete when the first began) and waits for it only at its end, so that what follows waits for both.
-  const bool pairs = MODE != 2 && dk > 64 && dk <= 128 && !few && (tokens == 0 || tokens >= DP_MIN);
+  // Entries of DP_MIN tokens and more two tokens at a time, the shorter ones by the launch behind it, which needs nothing of it: it may start at
+  // once (its inputs were complete when the first began), and one of its CTAs waits for the first launch, so that what follows waits for both.
+  // (Only one: with every CTA waiting, those that do not fit beside the first launch started when it had ended: 15 entries of one token and one
+  // of 40, 32 heads, decays per head / channel 43.7 / 45.7 -> 30 / 30.5 us, the scan alone 38 / 42.)  The long ones first: the short ones of such a
+  // batch come with their tail.  A call that knows its longest entry to be short is spared the first launch: 16 entries of 4 tokens, 16 heads 14.4 ->
+  // 13.3 us.
+  const bool pairs = by_pairs && !few && (tokens == 0 || tokens >= DP_MIN) && (longest == 0 || longest >= DP_MIN);
   if constexpr (MODE != 2) {
     const auto pair_kernel = crowded ? delta_pair_kernel<MODE, 2> : delta_pair_kernel<MODE, 1>;
     if (pairs)
@@ -994,19 +1000,26 @@ static void delta_scan_launch(int64_t tokens, int nb, cudaStream_t st, const flo
 #undef DELTA_SCAN
 }
 
-extern "C" int b200p_delta_scan_tokens(const float* qn, const float* kn, const float* v, const float* beta, const float* decay,
+extern "C" int b200p_delta_scan_entries(const float* qn, const float* kn, const float* v, const float* beta, const float* decay,
                                        float* state, const int32_t* cu, const int32_t* rows, const int32_t* lengths, float* o, int64_t tokens,
-                                       int nb, int H, int KH, int dk, int dv, int mode, void* stream) {
+                                       int64_t longest, int nb, int H, int KH, int dk, int dv, int mode, void* stream) {
   B200P_REQUIRE(qn && kn && v && decay && state && cu && rows && lengths && o, B200P_ERR_ARG, "null pointer");
   B200P_REQUIRE(mode >= B200P_SCAN_DELTA && mode <= B200P_SCAN_ACCUMULATE, B200P_ERR_ARG, "unknown scan mode %d", mode);
   B200P_REQUIRE(beta || mode == B200P_SCAN_ACCUMULATE, B200P_ERR_ARG, "the delta rule needs beta");
   B200P_REQUIRE(nb > 0 && H > 0 && KH > 0 && H % KH == 0 && H < 65536 && dk > 0 && dv > 0, B200P_ERR_ARG, "bad head geometry");
+  B200P_REQUIRE(tokens >= 0 && longest >= 0, B200P_ERR_ARG, "negative token count");
   B200P_REQUIRE(dk <= 512, B200P_ERR_ARG, "key size %d > 512 is not built", dk);
   cudaStream_t st = (cudaStream_t)stream;
   const auto launch = mode == B200P_SCAN_DELTA ? delta_scan_launch<0> : mode == B200P_SCAN_DELTA_CHANNEL ? delta_scan_launch<1> : delta_scan_launch<2>;
-  launch(tokens, nb, st, qn, kn, v, beta, decay, state, cu, rows, lengths, o, H, KH, dk, dv);
+  launch(tokens, longest, nb, st, qn, kn, v, beta, decay, state, cu, rows, lengths, o, H, KH, dk, dv);
   B200P_LAUNCH_CHECK("delta_scan_kernel");
   return B200P_OK;
+}
+
+extern "C" int b200p_delta_scan_tokens(const float* qn, const float* kn, const float* v, const float* beta, const float* decay,
+                                       float* state, const int32_t* cu, const int32_t* rows, const int32_t* lengths, float* o, int64_t tokens,
+                                       int nb, int H, int KH, int dk, int dv, int mode, void* stream) {
+  return b200p_delta_scan_entries(qn, kn, v, beta, decay, state, cu, rows, lengths, o, tokens < 0 ? 0 : tokens, 0, nb, H, KH, dk, dv, mode, stream);
 }
 
 extern "C" int b200p_delta_scan(const float* qn, const float* kn, const float* v, const float* beta, const float* decay,

@@ -214,7 +214,7 @@ class GatedDeltaMixer:
                        plan["t_off"], qn, kn, v, beta, decay, self.heads, self.kv_heads, self.dim, self.vdim, self.taps)
         ops.delta_conv_commit(proj, st.conv, plan["cu"], plan["rows"], plan["nb"], self.conv_channels, self.taps)
         ops.delta_scan(qn, kn, v, beta, decay, st.state, plan["cu"], plan["rows"], plan["lengths"], o, plan["nb"], self.heads,
-                       self.kv_heads, self.dim, self.vdim, SCAN_DELTA_CHANNEL if self.channel_decay else SCAN_DELTA)
+                       self.kv_heads, self.dim, self.vdim, SCAN_DELTA_CHANNEL if self.channel_decay else SCAN_DELTA, longest=plan.get("max_n", 0))
         mix = s.get("mix", dt, M, self.c_v)
         ops.delta_out(o, gate, self.norm_w, mix, self.heads, self.vdim, self.eps, self.gate_act)
         return self.o_proj(mix, GEMM_STORE_F32, out=y_out)

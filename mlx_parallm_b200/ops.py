@@ -356,13 +356,14 @@ def delta_conv_commit(proj, conv_state, cu, rows, nb: int, C: int, taps: int):
                                                                           C, taps, _stream()))
 
 
-def delta_scan(qn, kn, v, beta, decay, state, cu, rows, lengths, o, nb, H, KH, dk, dv, mode=_lib.SCAN_DELTA):
+def delta_scan(qn, kn, v, beta, decay, state, cu, rows, lengths, o, nb, H, KH, dk, dv, mode=_lib.SCAN_DELTA, longest: int = 0):
     """The recurrence over every entry's tokens; ``mode`` one of _lib.SCAN_* (decay per head, per head and key channel, or
-    the plain decayed accumulation without the delta correction)."""
+    the plain decayed accumulation without the delta correction); ``longest``: tokens of the longest entry (0: not known)."""
     _dev(qn, kn, v, beta, decay, state, cu, rows, lengths, o)
     assert state.dtype == torch.float32 and state.is_contiguous()
-    _call("b200p_delta_scan", lambda: lib().b200p_delta_scan_tokens(_p(qn), _p(kn), _p(v), _p(beta), _p(decay), _p(state), _p(cu), _p(rows),
-                                                                   _p(lengths), _p(o), qn.shape[0], nb, H, KH, dk, dv, int(mode), _stream()))
+    _call("b200p_delta_scan", lambda: lib().b200p_delta_scan_entries(_p(qn), _p(kn), _p(v), _p(beta), _p(decay), _p(state), _p(cu), _p(rows),
+                                                                    _p(lengths), _p(o), qn.shape[0], int(longest), nb, H, KH, dk, dv, int(mode),
+                                                                    _stream()))
 
 
 def delta_out(o, gate, norm_w, out, H, dv, eps, gate_act=_lib.GATE_SILU, out_scale=1.0):

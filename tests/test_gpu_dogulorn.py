@@ -886,3 +886,27 @@ def test_gated_units_of_the_tcgen05_products_keep_their_range(dtype, M):
         want = (z * torch.sigmoid(c * z) * (up + add)).expand(M, -1)
         err = (got - want).abs() / want.abs().clamp(min=tiny)          # (below the normal numbers: of the smallest of them)
         assert float(err.max()) <= half + 1.4e-5
+
+
+@pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("lens,H", [([40, 1, 1, 3, 0, 33, 2], 3), ([1] * 40 + [32], 8), ([5, 9, 20], 20), ([0] * 30 + [50] + [0] * 40, 2)])
+def test_delta_scan_of_long_entries_among_short_ones(mode, lens, H):
+    """The two launches of such a batch overlap, with more CTAs than fit and without; what reads the results behind them sees both.  A call that is
+    told its tokens and its longest entry gives the bits of one that is not (which takes both launches), also beside as many empty entries as a
+    decode step would have; a length that is told too small changes no more than the order of the sums."""
+    from mlx_parallm_b200 import _lib
+    g, nb, M, KH, dk, dv = torch.Generator(device="cuda").manual_seed(H + mode), len(lens), sum(lens), 1, 128, 128
+    rnd = lambda *sh: torch.randn(*sh, generator=g, device="cuda")        # noqa: E731
+    qn, kn, v = rnd(M, KH * dk) / dk ** 0.5, torch.nn.functional.normalize(rnd(M, KH, dk), dim=-1).reshape(M, -1).contiguous(), rnd(M, H * dv)
+    beta, decay = torch.rand(M, H, generator=g, device="cuda"), 0.5 + 0.5 * torch.rand(M, H * (dk if mode else 1), generator=g, device="cuda")
+    i32 = dict(dtype=torch.int32, device="cuda")
+    cu, rows, lengths = torch.tensor([0] + np.cumsum(lens).tolist(), **i32), torch.arange(nb, **i32), torch.full((nb,), 3, **i32)
+    state0, got = rnd(nb, H, dk, dv) * 0.3, []
+    for tokens, longest in ((0, 0), (M, max(lens)), (M, 1)):
+        state, o = state0.clone(), torch.zeros(M, H * dv, device="cuda")
+        _lib.check(_lib.lib().b200p_delta_scan_entries(*(t.data_ptr() for t in (qn, kn, v, beta, decay, state, cu, rows, lengths, o)), tokens, longest, nb,
+                                                       H, KH, dk, dv, mode, torch.cuda.current_stream().cuda_stream))
+        got.append((o * 1, state * 1))
+        state.zero_()
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+    assert (got[0][0] - got[2][0]).abs().max() < 4e-5 and (got[0][1] - got[2][1]).abs().max() < 4e-5        # (2e-5 each: the test above)
