@@ -13,6 +13,8 @@
 
 namespace b200p {
 
+int sm_count();
+
 // dense_gemm_tc.cu: B200P_OK, an error, or 1 = "not a shape for the tcgen05 kernel"
 template <typename T>
 int gemm_tc_launch(const T* x, const T* w, void* y, int64_t M, int64_t N, int64_t K, int64_t ldx, int64_t ldw, int64_t ldy,
@@ -226,7 +228,7 @@ static int gemm_mma_launch(const T* x, const T* w, void* y, int64_t M, int64_t N
 constexpr int GEMV_MAX_M = 8;
 
 // STAGED: x lies in shared memory (M * K values, the M rows one after the other): with one L1 access per row and piece the time grew with M.
-template <typename T, int MR, bool STAGED>
+template <typename T, int MR, bool STAGED, int AHEAD>
 __global__ void __launch_bounds__(256)
 gemv_rows_kernel(const T* __restrict__ x, const T* __restrict__ w, void* __restrict__ y, int M, int64_t N, int64_t K, int64_t ldx,
                  int64_t ldw, int64_t ldy, int64_t sx, int64_t sw, int64_t sy, int epi, float2 act) {
@@ -252,7 +254,6 @@ gemv_rows_kernel(const T* __restrict__ x, const T* __restrict__ w, void* __restr
   // Bound: the weights' way from HBM.  A warp asks for four pieces of each row at a time and x comes from shared memory (us, bf16, one piece at
   // a time and x from L1 -> now, 1 / 4 / 8 rows: 2048 x 2048 9.9 -> 6.7 / 15.2 -> 8.3 / 22 -> 12.3; 4368 x 2048 10.2 -> 8.2 / 16.3 -> 10.3 / 23.7 ->
   // 15.8; 4096 x 4096 16.4 -> 12.3 / 28.6 -> 16.4 / 43 -> 24.7; 512 x 8192 25 -> 16 / 49 -> 20 / 76 -> 65, not staged).
-  constexpr int AHEAD = 4;
   const int64_t k_end = STAGED ? (K + 255) / 256 * 256 : K;          // (staged: every lane takes part in the barrier)
   for (int64_t k0 = (int64_t)lane * 8; k0 < k_end; k0 += 256 * AHEAD) {
     uint4 u0[AHEAD], u1[AHEAD];
@@ -384,8 +385,12 @@ static int gemm_dispatch(const void* x, const void* w, void* y, int64_t M, int64
   if (fast_ok && M <= GEMV_MAX_M) {
     dim3 grid((unsigned)((N + 15) / 16), 1, (unsigned)batch);
     const size_t smem = (size_t)M * K * sizeof(T);
-    if (M > 1 && K >= 512 && smem <= 96 * 1024) {       // (short rows: the copy costs more than it spares, 2048 x 128, 4 rows: 5.2 / 4.2 us)
-      const auto kern = M <= 2 ? gemv_rows_kernel<T, 2, true> : M <= 4 ? gemv_rows_kernel<T, 4, true> : gemv_rows_kernel<T, 8, true>;
+    // Short rows in more CTAs than the GPU holds twice (the per-head products of a decode step): registers for the pieces ahead and the copy of x
+    // cost more than they spare.  us, one piece at a time / four: 128 heads of 512 x 128, 1 / 4 / 8 rows 10.3 / 14.9, 18.5 / 24.7, 37 / 51; 64 of 128 x
+    // 512 3.6 / 4.5, 5.7 / 7.2, 11.9 / 11.8; 64 of 512 x 1024 14.7 / 15.1, 24.5 / 24.3, 53 / 50.
+    const bool many = (N + 15) / 16 * batch > 2 * sm_count(), deep = K >= 512 && !(many && (K < 1024 || (K < 2048 && M <= 2)));
+    if (M > 1 && deep && smem <= 96 * 1024) {
+      const auto kern = M <= 2 ? gemv_rows_kernel<T, 2, true, 4> : M <= 4 ? gemv_rows_kernel<T, 4, true, 4> : gemv_rows_kernel<T, 8, true, 4>;
       static bool attr_set[3] = {false, false, false};
       bool& set = attr_set[M <= 2 ? 0 : M <= 4 ? 1 : 2];
       if (smem > 48 * 1024 && !set) {
@@ -394,8 +399,11 @@ static int gemm_dispatch(const void* x, const void* w, void* y, int64_t M, int64
         set = true;
       }
       kern<<<grid, 256, smem, st>>>(xp, wp, y, (int)M, N, K, ldx, ldw, ldy, sx, sw, sy, epi, act);
+    } else if (deep) {
+      const auto kern = M <= 2 ? gemv_rows_kernel<T, 2, false, 4> : M <= 4 ? gemv_rows_kernel<T, 4, false, 4> : gemv_rows_kernel<T, 8, false, 4>;
+      kern<<<grid, 256, 0, st>>>(xp, wp, y, (int)M, N, K, ldx, ldw, ldy, sx, sw, sy, epi, act);
     } else {
-      const auto kern = M <= 2 ? gemv_rows_kernel<T, 2, false> : M <= 4 ? gemv_rows_kernel<T, 4, false> : gemv_rows_kernel<T, 8, false>;
+      const auto kern = M <= 2 ? gemv_rows_kernel<T, 2, false, 1> : M <= 4 ? gemv_rows_kernel<T, 4, false, 1> : gemv_rows_kernel<T, 8, false, 1>;
       kern<<<grid, 256, 0, st>>>(xp, wp, y, (int)M, N, K, ldx, ldw, ldy, sx, sw, sy, epi, act);
     }
     B200P_LAUNCH_CHECK("gemv_rows_kernel");

@@ -910,3 +910,17 @@ def test_delta_scan_of_long_entries_among_short_ones(mode, lens, H):
         state.zero_()
     assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
     assert (got[0][0] - got[2][0]).abs().max() < 4e-5 and (got[0][1] - got[2][1]).abs().max() < 4e-5        # (2e-5 each: the test above)
+
+
+@pytest.mark.parametrize("M,N,K,batch", [(1, 64, 128, 9), (2, 512, 128, 16), (5, 128, 512, 64), (8, 130, 512, 3), (3, 128, 1024, 40), (1, 128, 520, 64)])
+def test_gemv_of_short_rows(M, N, K, batch):
+    """Few rows over many short weight rows (per-head products): one piece of a row at a time; from 512 channels, where the CTAs fit the GPU
+    twice, and from 1024 four of them and staged x."""
+    from mlx_parallm_b200 import _lib, ops
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    x = (torch.randn(M, batch, K, generator=g, device="cuda") / 4).bfloat16()
+    w = (torch.randn(batch, N, K, generator=g, device="cuda") / 4).bfloat16()
+    out = torch.full((M, batch, N), 7.0, device="cuda")
+    ops.gemm(x, w, _lib.GEMM_STORE_F32, out=out, batch=batch, strides=(K, N * K, N), M=M, N=N, K=K, ldx=batch * K, ldw=K, ldy=batch * N)
+    want = torch.einsum("mbk,bnk->mbn", x.double(), w.double())
+    assert (out.double() - want).abs().max() <= 2e-5 * math.sqrt(K)
