@@ -1,6 +1,6 @@
 // Dense (unquantised) linear layers: y[M,N] = x[M,K] . w[N,K]^T with fp32 accumulation, optionally batched over a leading
-// index (one weight block per attention head).  Six kernels behind b200p_gemm:
-//   gemm_tc_pair_kernel, gemm_tc_kernel  16-bit operands, tcgen05 / TMA / TMEM (dense_gemm_tc.cu)           (more than 64 rows; 9 to 64)
+// index (one weight block per attention head).  Seven kernels behind b200p_gemm:
+//   gemm_tc_pair_kernel, gemm_tc_rows_kernel, gemm_tc_kernel  16-bit operands, tcgen05 / TMA / TMEM (dense_gemm_tc.cu)   (more than 64 rows; 9 to 64)
 //   gemm_mma_kernel    16-bit operands, mma.sync m16n8k16 over cp.async-staged tiles, two tile shapes      (K < 64, or on request)
 //   gemm_stream_kernel 16-bit operands, weights streamed from global memory straight into MMA fragments    (9..64 rows where tcgen05 declines)
 //   gemv_rows_kernel   16-bit operands, a warp per pair of weight rows, 128-bit streaming                  (up to 8 rows)

@@ -1,7 +1,7 @@
 // Dense 16-bit GEMM on tcgen05: y[M,N] = x[M,K] . w[N,K]^T (+ batch, or grouped), both operands in shared memory, accumulators in TMEM.
 //
-// Two kernels, both with the WEIGHTS on the MMA's M side and the tokens on the N side: the accumulator holds y transposed (lane = output
-// column, TMEM column = token) and the epilogue stores it back transposed, a warp writing 32 consecutive outputs of one token.  Both are
+// Three kernels.  Two have the WEIGHTS on the MMA's M side and the tokens on the N side: the accumulator holds y transposed (lane = output
+// column, TMEM column = token) and the epilogue stores it back transposed, a warp writing 32 consecutive outputs of one token.  All are
 // persistent (CTA or pair c takes tiles c, c + grid, ...) with two accumulators, so that the epilogue of one tile overlaps the main
 // loop of the next.
 //
@@ -13,7 +13,7 @@
 //   warp 1      MMA issuer: four tcgen05.mma (M=128, N=BN, K=16) per stage, tcgen05.commit frees the stage; owns the TMEM allocation
 //   warps 2..5  epilogue: tcgen05.ld (thread = output column, 32 tokens at a time) -> store / store fp32 / gated unit
 //
-// gemm_tc_pair_kernel, prompts: two CTAs on one tile (below).
+// gemm_tc_pair_kernel, prompts: two CTAs on one tile; gemm_tc_rows_kernel, prompts with a short K or a narrow output: tokens on the M side.
 //
 // Rows, columns and k outside the tensors are zero-filled by the TMA unit and masked in the epilogue.  Every mbarrier wait is
 // bounded: a wait that runs out raises a device flag (reported by the next launch) and the CTA leaves through the common exit,
@@ -291,6 +291,163 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmw, const __grid_constant__ 
         tmem_ld16(tsrc + c + 16, *reinterpret_cast<float(*)[16]>(&v[16]));
         tmem_ld_wait();
         gemm_tc_store32<T>(p, out, z_off, n, c, tl.len, v);
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&sh->acc_empty[acc]));
+      if (++acc == 2) { acc = 0; acc_phase ^= 1u; }
+    }
+  }
+  if (sh->abort) wait_settle();
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, TMEM_COLS);
+  }
+}
+
+// ---------------------------------------------------------------------------------------------------------- short K, narrow outputs
+// More than 64 tokens where the pair kernel below has little to multiply: one CTA on a tile of 128 tokens (the M side) x BN weight rows.  The
+// set-up is half of the pair's (no cluster, fewer TMEM columns), a narrow output pads no 256 rows, and a thread owns a token's row, so that its
+// outputs leave as 16-byte pieces: at a short K the store is what bounds the call.  Bound: the output's way to HBM (64 x 1500 x 128 x 128 to
+// bf16: 3.6 TB/s) or, in small calls, latency.  Where the line lies: gemm_tc_rows_better.
+template <typename T> __device__ __forceinline__ uint32_t pack2(float a, float b);
+template <> __device__ __forceinline__ uint32_t pack2<__half>(float a, float b) {
+  const __half2 h = __floats2half2_rn(a, b);
+  return *reinterpret_cast<const uint32_t*>(&h);
+}
+template <> __device__ __forceinline__ uint32_t pack2<__nv_bfloat16>(float a, float b) {
+  const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+  return *reinterpret_cast<const uint32_t*>(&h);
+}
+
+// outputs n0 .. n0 + 31 of one token's row (at element row_off of y); vec: whole pieces may leave as 16 bytes
+template <typename T>
+__device__ __forceinline__ void gemm_tc_store_row32(const GemmTcParams& p, int64_t row_off, int64_t n0, bool vec, const float (&v)[32]) {
+  const int64_t R = p.out[0].R;
+  if (p.epi == B200P_GEMM_STORE_F32) {
+    float* dst = reinterpret_cast<float*>(p.out[0].y) + row_off + n0;
+    if (vec && n0 + 32 <= R) {
+#pragma unroll
+      for (int i = 0; i < 32; i += 4) *reinterpret_cast<float4*>(dst + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+    } else {
+#pragma unroll
+      for (int i = 0; i < 32; ++i)
+        if (n0 + i < R) dst[i] = v[i];
+    }
+    return;
+  }
+  float a[32];
+#pragma unroll
+  for (int i = 0; i < 32; ++i) a[i] = p.epi == B200P_GEMM_RELU_SQ ? gemm_store_act(v[i], B200P_GEMM_RELU_SQ, p.act) : v[i];
+  T* dst = reinterpret_cast<T*>(p.out[0].y) + row_off + n0;
+  if (vec && n0 + 32 <= R) {
+#pragma unroll
+    for (int i = 0; i < 32; i += 8)
+      *reinterpret_cast<uint4*>(dst + i) = make_uint4(pack2<T>(a[i], a[i + 1]), pack2<T>(a[i + 2], a[i + 3]), pack2<T>(a[i + 4], a[i + 5]), pack2<T>(a[i + 6], a[i + 7]));
+  } else {
+#pragma unroll
+    for (int i = 0; i < 32; ++i)
+      if (n0 + i < R) dst[i] = Tr<T>::from_f(a[i]);
+  }
+}
+
+template <typename T, int BN, int STAGES>
+__global__ void __launch_bounds__(GT_THREADS, 1)
+gemm_tc_rows_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constant__ CUtensorMap tmw, const GemmTcParams p, const bool vec) {
+  constexpr int B_BYTES = BN * GT_BK * 2, STAGE_BYTES = GT_A_BYTES + B_BYTES;
+  constexpr uint32_t TMEM_COLS = 2 * BN;           // 128, 256 or 512
+  static_assert(STAGES <= 10 && (BN == 64 || BN == 128 || BN == 256), "ring / tile shape");
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t raw = smem_u32(smem_raw);
+  const uint32_t base = (raw + 1023u) & ~1023u;
+  GemmTcShared* sh = reinterpret_cast<GemmTcShared*>(smem_raw + (base - raw) + STAGES * STAGE_BYTES);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < STAGES; ++s) {
+      mbar_init(smem_u32(&sh->full[s]), 1);
+      mbar_init(smem_u32(&sh->empty[s]), 1);
+    }
+    for (int a = 0; a < 2; ++a) {
+      mbar_init(smem_u32(&sh->acc_full[a]), 1);
+      mbar_init(smem_u32(&sh->acc_empty[a]), 4);   // one arrival per epilogue warp
+    }
+    sh->abort = 0;
+    fence_barrier_init();
+    tma_prefetch_desc(&tmx);
+    tma_prefetch_desc(&tmw);
+  }
+  if (warp == 1) tmem_alloc(smem_u32(&sh->tmem_base), TMEM_COLS);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = sh->tmem_base;
+  const int per = p.tiles_t * p.tiles_r;           // tiles of a batch index, token tile fastest
+
+  if (warp == 0) {
+    int stage = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    for (int t = blockIdx.x; t < p.num_tiles && ok; t += gridDim.x) {
+      const int z = t / per, rt = (t - z * per) / p.tiles_t, tt = (t - z * per) - rt * p.tiles_t;
+      for (int kb = 0; kb < p.num_kb; ++kb) {
+        if (!(ok = mbar_wait_warp(smem_u32(&sh->empty[stage]), phase ^ 1u, &sh->abort, p.wait_word, 0))) break;
+        if (elect_one()) {
+          const uint32_t bar = smem_u32(&sh->full[stage]), dst = base + stage * STAGE_BYTES;
+          mbar_arrive_expect_tx(bar, STAGE_BYTES);
+          tma_load_3d(dst, &tmx, kb * GT_BK, tt * GT_BM, z, bar);
+          tma_load_3d(dst + GT_A_BYTES, &tmw, kb * GT_BK, rt * BN, z, bar);
+        }
+        __syncwarp();
+        if (++stage == STAGES) { stage = 0; phase ^= 1u; }
+      }
+    }
+  } else if (warp == 1) {
+    constexpr uint32_t fmt = std::is_same<T, __nv_bfloat16>::value ? 1u : 0u;
+    constexpr uint32_t idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(GT_BM >> 4) << 24);
+    int stage = 0, acc = 0;
+    uint32_t phase = 0, acc_phase = 0;
+    bool ok = true;
+    for (int t = blockIdx.x; t < p.num_tiles && ok; t += gridDim.x) {
+      if (!(ok = mbar_wait_warp(smem_u32(&sh->acc_empty[acc]), acc_phase ^ 1u, &sh->abort, p.wait_word, 1))) break;
+      tc_fence_after();
+      const uint32_t d = tmem_base + (uint32_t)(acc * BN);
+      for (int kb = 0; kb < p.num_kb; ++kb) {
+        if (!(ok = mbar_wait_warp(smem_u32(&sh->full[stage]), phase, &sh->abort, p.wait_word, 1))) break;
+        tc_fence_after();
+        if (elect_one()) {
+          const uint64_t ad = make_desc_sw128(base + stage * STAGE_BYTES), bd = make_desc_sw128(base + stage * STAGE_BYTES + GT_A_BYTES);
+#pragma unroll
+          for (int k = 0; k < GT_BK / 16; ++k) umma_f16_ss(d, ad + 2u * k, bd + 2u * k, idesc, (kb | k) ? 1u : 0u);
+          umma_commit(smem_u32(&sh->empty[stage]));
+          if (kb == p.num_kb - 1) umma_commit(smem_u32(&sh->acc_full[acc]));
+        }
+        __syncwarp();
+        if (++stage == STAGES) { stage = 0; phase ^= 1u; }
+      }
+      if (++acc == 2) { acc = 0; acc_phase ^= 1u; }
+    }
+  } else {
+    const int lg = warp & 3;                       // the TMEM lane quarter this warp may read
+    int acc = 0;
+    uint32_t acc_phase = 0;
+    for (int t = blockIdx.x; t < p.num_tiles; t += gridDim.x) {
+      const int z = t / per, rt = (t - z * per) / p.tiles_t, tt = (t - z * per) - rt * p.tiles_t;
+      if (!mbar_wait_warp(smem_u32(&sh->acc_full[acc]), acc_phase, &sh->abort, p.wait_word, 2)) break;
+      tc_fence_after();
+      const int64_t row = (int64_t)tt * GT_BM + lg * 32 + lane, row_off = (int64_t)z * p.sy + row * p.out[0].ldy;
+      const uint32_t tsrc = tmem_base + ((uint32_t)(lg * 32) << 16) + (uint32_t)(acc * BN);
+#pragma unroll 1
+      for (int c = 0; c < BN; c += 32) {
+        const int64_t n0 = (int64_t)rt * BN + c;
+        if (n0 >= p.out[0].R) break;               // warp-uniform
+        float v[32];
+        tmem_ld16(tsrc + c, *reinterpret_cast<float(*)[16]>(&v[0]));
+        tmem_ld16(tsrc + c + 16, *reinterpret_cast<float(*)[16]>(&v[16]));
+        tmem_ld_wait();
+        if (row < p.tokens) gemm_tc_store_row32<T>(p, row_off, n0, vec, v);
       }
       tc_fence_before();
       __syncwarp();
@@ -749,6 +906,68 @@ static int gemm_tc_launch_decode(TcEncodeFn enc, const T* x, const T* w, void* y
   return gemm_tc_run<T, 64, 8>(tm, p, false, st);
 }
 
+// Which of the two kernels of more than 64 tokens (us, one CTA / pair, bf16).  tiles: of 128 tokens x 64 outputs.
+//   16-bit stores: 2048 x 2048 x 128 8.1 / 11.0, x 512 13.4 / 12.9, 4096 x 2048 x 512 16.2 / 20.4, 64 x 1500 x 512 x 128 43 / 85; up to K = 1024 while
+//     one wave holds the tiles (512 x 2048 x 1024 8.5 / 9.4; 1024 x 2048 x 1024 13.2 / 11.1);
+//   fp32: up to K = 256 (512 x 2048 x 128 4.9 / 5.8, 64 x 512 x 512 x 128 28 / 31, 2048 x 8192 x 256 29.8 / 31.4) unless the output is large (4096 x 8192 x
+//     256 59 / 52); up to K = 768 in one wave (512 x 2048 x 512 6.7 / 7.1; 1024 x 2048 x 512 9.2 / 8.5);
+//   outputs that fill half of the pair's 256 rows: up to K = 512 (64 x 1500 x 128 x 512 33 / 44), and the narrowest of many tokens at any K
+//     (4096 x 16 x 2048 12.1 / 14.4, x 64 12.3 / 11.9).
+// Gated units and the activations with exponentials stay with the pair, whose epilogue has twice the warps (128 x 2048 x 128 gated 7.5 / 6.5).
+static bool gemm_tc_rows_better(int64_t M, int64_t N, int64_t K, int64_t batch, int epi) {
+  if (epi != B200P_GEMM_STORE && epi != B200P_GEMM_RELU_SQ && epi != B200P_GEMM_STORE_F32) return false;
+  const int64_t sms = sm_count(), tiles = (M + GT_BM - 1) / GT_BM * ((N + 63) / 64) * batch;
+  if ((N <= 128 && K <= 512) || (N <= 32 && M > 1024)) return true;
+  if (epi != B200P_GEMM_STORE_F32) return K <= 512 || (K <= 1024 && tiles <= sms);
+  return (K <= 256 && tiles <= 14 * sms) || (K <= 768 && tiles <= sms);
+}
+
+template <typename T, int BN, int STAGES>
+static int gemm_tc_rows_run(const CUtensorMap& tmx, const CUtensorMap& tmw, GemmTcParams p, bool vec, cudaStream_t st) {
+  constexpr size_t smem = 1024 + (size_t)STAGES * (GT_A_BYTES + BN * GT_BK * 2) + sizeof(GemmTcShared);
+  auto kern = gemm_tc_rows_kernel<T, BN, STAGES>;
+  static bool attr_set = false;
+  if (!attr_set) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(gemm_tc_rows_kernel)");
+    attr_set = true;
+  }
+  if (const int rc = wait_word(WAIT_GEMM_TC, &p.wait_word)) return rc;
+  kern<<<(unsigned)(p.num_tiles < sm_count() ? p.num_tiles : sm_count()), GT_THREADS, smem, st>>>(tmx, tmw, p, vec);
+  B200P_LAUNCH_CHECK("gemm_tc_rows_kernel");
+  return B200P_OK;
+}
+
+template <typename T>
+static int gemm_tc_launch_rows(TcEncodeFn enc, const T* x, const T* w, void* y, int64_t M, int64_t N, int64_t K, int64_t ldx, int64_t ldw,
+                               int64_t ldy, int64_t batch, int64_t sx, int64_t sw, int64_t sy, int epi, float2 act, cudaStream_t st) {
+  // widest weight tile that still gives every SM about two tiles
+  const int64_t tiles_t = (M + GT_BM - 1) / GT_BM, want = 2ll * sm_count();
+  int bn = 256;
+  if (N <= 64 || tiles_t * ((N + 127) / 128) * batch < want) bn = 64;
+  else if (N <= 128 || tiles_t * ((N + 255) / 256) * batch < want) bn = 128;
+  const int64_t tiles_r = (N + bn - 1) / bn, tiles = tiles_t * tiles_r * batch;
+  if (tiles >= (1ll << 30)) return 1;
+  const CUtensorMapDataType dt = std::is_same<T, __nv_bfloat16>::value ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
+  CUtensorMap tmx, tmw;
+  if (!gemm_tc_map(enc, &tmx, dt, x, K, M, batch, ldx, sx, GT_BM)) return 1;
+  if (!gemm_tc_map(enc, &tmw, dt, w, K, N, batch, ldw, sw, bn)) return 1;
+  GemmTcParams p = {};
+  p.out[0] = {y, N, ldy};
+  p.tokens = M; p.sy = sy;
+  p.tiles_r = (int)tiles_r;
+  p.tiles_t = (int)tiles_t;
+  p.num_tiles = (int)tiles;
+  p.num_kb = (int)((K + GT_BK - 1) / GT_BK);
+  p.epi = epi;
+  p.act = act;
+  const int64_t eb = epi == B200P_GEMM_STORE_F32 ? 4 : 2;
+  const bool vec = aligned(y, 16) && (ldy * eb) % 16 == 0 && (batch == 1 || (sy * eb) % 16 == 0);
+  if (bn == 256) return gemm_tc_rows_run<T, 256, 4>(tmx, tmw, p, vec, st);
+  if (bn == 128) return gemm_tc_rows_run<T, 128, 6>(tmx, tmw, p, vec, st);
+  return gemm_tc_rows_run<T, 64, 8>(tmx, tmw, p, vec, st);
+}
+
 // Returns B200P_OK, an error, or 1 when the shape is not one this kernel takes (the caller then runs the mma.sync kernel).
 template <typename T>
 int gemm_tc_launch(const T* x, const T* w, void* y, int64_t M, int64_t N, int64_t K, int64_t ldx, int64_t ldw, int64_t ldy,
@@ -757,6 +976,7 @@ int gemm_tc_launch(const T* x, const T* w, void* y, int64_t M, int64_t N, int64_
   TcEncodeFn enc = gemm_tc_encode_fn();
   if (!enc) return 1;
   if (M <= 64) return gemm_tc_launch_decode<T>(enc, x, w, y, M, N, K, ldx, ldw, ldy, batch, sx, sw, sy, epi, act, st);
+  if (gemm_tc_rows_better(M, N, K, batch, epi)) return gemm_tc_launch_rows<T>(enc, x, w, y, M, N, K, ldx, ldw, ldy, batch, sx, sw, sy, epi, act, st);
   int tn = 0;
   int64_t tiles_t = 0;
   pair::plan(M, N, batch, tn, tiles_t);

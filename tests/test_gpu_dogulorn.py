@@ -153,10 +153,12 @@ def test_gemv_of_few_rows(M, N, K, batch):
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("M,N,K,batch", [(65, 2, 64, 1), (96, 256, 72, 1), (257, 300, 200, 1), (512, 257, 448, 1), (777, 1030, 136, 1), (1000, 640, 64, 3),
-                                         (4100, 5000, 320, 1)])
+                                         (4100, 5000, 320, 1), (65, 2, 1032, 1), (257, 300, 1096, 1), (513, 257, 1032, 1), (777, 1030, 1032, 1), (300, 640, 1032, 3),
+                                         (1030, 31, 1032, 1), (129, 200, 768, 2), (200, 130, 1024, 1), (2100, 128, 512, 2)])
 def test_gemm_pairs_of_ctas(dtype, M, N, K, batch):
-    """Two CTAs on one tile of 256 output columns x up to 256 tokens (more than 64 rows): ragged edges in all three dimensions, columns
-    that end in the first CTA's half, one tile for a pair and several, batches, all kinds of stores."""
+    """More than 64 rows: two CTAs on one tile of 256 output columns x up to 256 tokens, or one on 128 tokens x 64 to 256 columns (stores and the
+    squared relu at a short K or a narrow output): ragged edges in all three dimensions, columns that end in the first CTA's half, one tile for
+    a pair and several, batches, all kinds of stores."""
     from mlx_parallm_b200 import _lib, ops
     g = torch.Generator(device="cuda").manual_seed(M + N + K)
     x = (torch.randn(batch, M, K, generator=g, device="cuda") / 4).to(dtype)
@@ -924,3 +926,21 @@ def test_gemv_of_short_rows(M, N, K, batch):
     ops.gemm(x, w, _lib.GEMM_STORE_F32, out=out, batch=batch, strides=(K, N * K, N), M=M, N=N, K=K, ldx=batch * K, ldw=K, ldy=batch * N)
     want = torch.einsum("mbk,bnk->mbn", x.double(), w.double())
     assert (out.double() - want).abs().max() <= 2e-5 * math.sqrt(K)
+
+
+@pytest.mark.parametrize("M,N,K,ld,shift", [(130, 96, 64, 96, 1), (130, 96, 128, 97, 0), (200, 33, 256, 40, 4), (129, 64, 72, 200, 8), (1025, 32, 1032, 32, 2)])
+def test_gemm_rows_at_any_output_address(M, N, K, ld, shift):
+    """Short K and narrow outputs store a token's outputs as 16-byte pieces where address and row stride allow it: others, and columns that are
+    not theirs, stay right."""
+    from mlx_parallm_b200 import _lib, ops
+    g = torch.Generator(device="cuda").manual_seed(M + N + ld)
+    x, w = (torch.randn(n, K, generator=g, device="cuda").bfloat16() for n in (M, N))
+    want = x.double() @ w.double().T
+    for epi, dt in ((_lib.GEMM_STORE_F32, torch.float32), (_lib.GEMM_STORE, torch.bfloat16)):
+        buf = torch.full((M * ld + 16,), 7.0, dtype=dt, device="cuda")
+        ops.gemm(x, w, epi, out=buf[shift:shift + M * ld].view(M, ld)[:, :N], ldy=ld)
+        rows = buf[shift:shift + M * ld].view(M, ld)
+        tol = 2e-5 * math.sqrt(K) + (2.0 ** -8 * float(want.abs().max()) if dt == torch.bfloat16 else 0.0)
+        assert (rows[:, :N].double() - want).abs().max() <= tol and bool((rows[:, N:] == 7).all())
+        assert bool((buf[:shift] == 7).all()) and bool((buf[shift + M * ld:] == 7).all())
+    assert _lib.lib().b200p_gemm_tc_fault() == 0
