@@ -73,7 +73,8 @@ int b200p_arch_check(void);
 int b200p_sm_count(void);
 /* Programmatic dependent launch, 0 off: kernel N+1's prologue and weight prefetch overlap kernel N's tail; each kernel executes
  * griddepcontrol.wait before touching its inputs.  Default (2): the quantised products, the early norms, attention, the delta rule's second
- * launch, a mixture's kernels except its last (routing and gather up to 64 tokens); 1: every kernel that can be. */
+ * launch, dense products between other kernels (B200P_GEMM_CHAINED), a mixture's kernels except its last (routing and gather up to 64
+ * tokens); 1: every kernel that can be. */
 int b200p_set_pdl(int enabled);
 
 /* mx.dequantize(w, scales, biases, group_size, bits)            [nn.QuantizedEmbedding.__call__,
@@ -294,6 +295,10 @@ enum {
   B200P_GEMM_XIELU = 6,      /* y[M,N] (dtype) = act_a z^2 + z / 2 (z > 0), act_b (e^z - 1 - z) + z / 2 (z <= 0), z = acc */
   B200P_GEMM_CAP_F32 = 7     /* y[M,N] (float) = act_a tanh(acc / act_a): capped logits                              */
 };
+/* OR-ed into b200p_gemm's epilogue: other kernels of the caller surround the product, so it may be launched programmatically (saves 1 to 1.5 us).
+ * Without it the launch is plain: a program may issue any number of products in a row, and a stream of nothing but programmatic launches once
+ * did not come to its end under a tracer. */
+#define B200P_GEMM_CHAINED 0x100
 /* act_a / act_b: the epilogue's constants (0 where it has none).
  * y = x . w^T, x [M,K] and w [N,K] in `dtype` (row strides ldx / ldw elements), fp32 accumulation; `batch` independent
  * products at element strides stride_x / stride_w / stride_y.  B200P_F32 runs true fp32 FMAs in ascending k.  16-bit calls

@@ -152,6 +152,7 @@ UNIT_SETS = {
     "sequence_rows": ("runtime", "dense_gemm", "dense_gemm_tc", "ragged", "row_attn_prep", "sink_attn", "moe", "sampler"),
 }
 GEMM_STORE, GEMM_STORE_F32, GEMM_GLU_CLAMP, GEMM_GLU_GELU_TANH, GEMM_GLU_SILU, GEMM_RELU_SQ, GEMM_XIELU, GEMM_CAP_F32 = 0, 1, 2, 3, 4, 5, 6, 7
+GEMM_CHAINED = 0x100                                # b200p_gemm: other kernels surround the product (include/b200p.h)
 
 
 def gemm_is_gated(epilogue: int) -> bool:

@@ -173,7 +173,8 @@ __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepc
 // griddepcontrol.wait before it touches anything a predecessor reads or writes.
 bool pdl_enabled();
 // kernel class of the C-ABI call being executed (B200P_PDL_MASK selects, per class, which launches carry the PDL attribute):
-// 2 rmsnorm, 4 rope+append, 8 attention, 16 silu_mul, 32 embed / dequantize / advance / samplers, 64 GEMV paths
+// 2 rmsnorm, 4 rope+append, 8 attention, 16 silu_mul, 32 embed / dequantize / advance / samplers, 64 GEMV paths; 128 dense products between
+// other kernels (programmatic unless everything is off)
 void pdl_set_class(int cls);
 struct PdlClass {
   explicit PdlClass(int c) { pdl_set_class(c); }

@@ -508,6 +508,7 @@ static int gemm_grouped_call(const void* x, const void* w, void* y, const int32_
       return b200p_gemm(two->x, two->w, two->y, two->M, two->N, two->K, two->ldx, two->ldw, two->ldy, 1, 0, 0, 0, dtype, epilogue, act_a, act_b, stream);
   }
   if (max_rows == 0) return B200P_OK;
+  PdlClass pdl_cls(128);
   cudaStream_t st = (cudaStream_t)stream;
   const bool fast_ok = dtype != B200P_F32 && K % 8 == 0 && ldx % 8 == 0 && ldw % 8 == 0 && stride_w % 8 == 0 && aligned(x, 16) &&
                        aligned(w, 16);
@@ -550,6 +551,8 @@ extern "C" int b200p_gemm(const void* x, const void* w, void* y, int64_t M, int6
                           int64_t ldy, int64_t batch, int64_t stride_x, int64_t stride_w, int64_t stride_y, int dtype,
                           int epilogue, float act_a, float act_b, void* stream) {
   using namespace b200p;
+  PdlClass pdl_cls(epilogue >= 0 && (epilogue & B200P_GEMM_CHAINED) ? 128 : 0);
+  if (epilogue >= 0) epilogue &= ~B200P_GEMM_CHAINED;
   B200P_REQUIRE(x && w && y, B200P_ERR_ARG, "null pointer");
   B200P_REQUIRE(M >= 0 && N > 0 && K > 0 && batch > 0 && ldx >= K && ldw >= K, B200P_ERR_ARG, "bad GEMM shape");
   B200P_REQUIRE(epilogue >= B200P_GEMM_STORE && epilogue <= B200P_GEMM_CAP_F32, B200P_ERR_ARG, "unknown epilogue %d", epilogue);

@@ -28,7 +28,7 @@
 namespace b200p {
 
 int sm_count();
-bool pdl_enabled_gemm();
+bool pdl_chained();
 
 constexpr int GT_BM = 128, GT_BK = 64, GT_THREADS = 192;
 constexpr int GT_A_BYTES = GT_BM * GT_BK * 2;
@@ -379,7 +379,11 @@ gemm_tc_rows_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_consta
     tma_prefetch_desc(&tmx);
     tma_prefetch_desc(&tmw);
   }
-  if (warp == 1) tmem_alloc(smem_u32(&sh->tmem_base), TMEM_COLS);
+  if (warp == 1) {
+    tmem_alloc(smem_u32(&sh->tmem_base), TMEM_COLS);
+    pdl_launch_dependents();                       // (as above)
+  }
+  pdl_wait();                                      // operands and y belong to the previous kernels until here
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -771,10 +775,10 @@ static void gemm_tc_set_second(GemmTcParams& p, const GemmTcPlain* two, int rows
   p.two.num_kb = (int)((two->K + GT_BK - 1) / GT_BK);
 }
 
-// pdl: launched programmatically.  A mixture's products are, between its other kernels; a plain product, of which a program may issue any
-// number in a row, is not (moe.cu: streams of nothing but programmatic launches).
+// (pdl_chained: launched programmatically in a mixture and where the caller says that other kernels surround the product; a program may issue any
+// number of other products in a row, and streams of nothing but programmatic launches are avoided, moe.cu)
 template <typename T, int BN, int STAGES>
-static int gemm_tc_run(const CUtensorMap* tm, GemmTcParams p, bool pdl, cudaStream_t st) {
+static int gemm_tc_run(const CUtensorMap* tm, GemmTcParams p, cudaStream_t st) {
   constexpr size_t smem = 1024 + (size_t)STAGES * (GT_A_BYTES + BN * GT_BK * 2) + sizeof(GemmTcShared);
   auto kern = gemm_tc_kernel<T, BN, STAGES>;
   static bool attr_set = false;
@@ -785,7 +789,7 @@ static int gemm_tc_run(const CUtensorMap* tm, GemmTcParams p, bool pdl, cudaStre
   }
   if (const int rc = wait_word(WAIT_GEMM_TC, &p.wait_word)) return rc;
   const int tiles = p.num_tiles + p.two.num_tiles, grid = tiles < sm_count() ? tiles : sm_count();
-  cudaError_t e = launch_pdl_opt(pdl && pdl_enabled_gemm(), kern, dim3((unsigned)grid), dim3(GT_THREADS), smem, st, tm[0], tm[1], tm[2], tm[3], p);
+  cudaError_t e = launch_pdl_opt(pdl_chained(), kern, dim3((unsigned)grid), dim3(GT_THREADS), smem, st, tm[0], tm[1], tm[2], tm[3], p);
   if (e != cudaSuccess) return cuda_fail(e, "gemm_tc_kernel launch");
   return B200P_OK;
 }
@@ -793,7 +797,7 @@ static int gemm_tc_run(const CUtensorMap* tm, GemmTcParams p, bool pdl, cudaStre
 namespace pair {
 
 template <typename T>
-static int run(const CUtensorMap* tm, Params p, int64_t tiles, bool pdl, cudaStream_t st) {
+static int run(const CUtensorMap* tm, Params p, int64_t tiles, cudaStream_t st) {
   constexpr size_t smem = 1024 + (size_t)STAGES * STAGE_BYTES + sizeof(Shared);
   auto kern = gemm_tc_pair_kernel<T>;
   static bool attr_set = false;
@@ -805,7 +809,7 @@ static int run(const CUtensorMap* tm, Params p, int64_t tiles, bool pdl, cudaStr
   if (const int rc = wait_word(WAIT_GEMM_TC, &p.g.wait_word)) return rc;
   const int64_t pairs = sm_count() / 2;
   const unsigned grid = 2u * (unsigned)(tiles < pairs ? tiles : pairs);
-  cudaError_t e = launch_pdl_opt(pdl && pdl_enabled_gemm(), kern, dim3(grid), dim3(THREADS), smem, st, tm[0], tm[1], tm[2], tm[3], p);
+  cudaError_t e = launch_pdl_opt(pdl_chained(), kern, dim3(grid), dim3(THREADS), smem, st, tm[0], tm[1], tm[2], tm[3], p);
   if (e != cudaSuccess) return cuda_fail(e, "gemm_tc_pair_kernel launch");
   return B200P_OK;
 }
@@ -860,7 +864,7 @@ static int launch(TcEncodeFn enc, const T* x, const T* w, void* y, const int32_t
     if (!gemm_tc_map(enc, &tm[2], dt, two->w, two->K, two->N, 1, two->ldw, 0, 128)) return 1;
     if (!gemm_tc_map(enc, &tm[3], dt, two->x, two->K, two->M, 1, two->ldx, 0, g.two.tn / 2)) return 1;
   }
-  return run<T>(tm, p, tiles + g.two.num_tiles, seg != nullptr, st);
+  return run<T>(tm, p, tiles + g.two.num_tiles, st);
 }
 
 }  // namespace pair
@@ -902,8 +906,8 @@ static int gemm_tc_launch_decode(TcEncodeFn enc, const T* x, const T* w, void* y
     if (e != cudaSuccess) return cuda_fail(e, "cudaMemsetAsync(split-K output)");
   }
   gemm_tc_set_second(p, nullptr, GT_BM);
-  if (bn == 32) return gemm_tc_run<T, 32, 10>(tm, p, false, st);
-  return gemm_tc_run<T, 64, 8>(tm, p, false, st);
+  if (bn == 32) return gemm_tc_run<T, 32, 10>(tm, p, st);
+  return gemm_tc_run<T, 64, 8>(tm, p, st);
 }
 
 // Which of the two kernels of more than 64 tokens (us, one CTA / pair, bf16).  tiles: of 128 tokens x 64 outputs.
@@ -933,8 +937,9 @@ static int gemm_tc_rows_run(const CUtensorMap& tmx, const CUtensorMap& tmw, Gemm
     attr_set = true;
   }
   if (const int rc = wait_word(WAIT_GEMM_TC, &p.wait_word)) return rc;
-  kern<<<(unsigned)(p.num_tiles < sm_count() ? p.num_tiles : sm_count()), GT_THREADS, smem, st>>>(tmx, tmw, p, vec);
-  B200P_LAUNCH_CHECK("gemm_tc_rows_kernel");
+  const unsigned grid = (unsigned)(p.num_tiles < sm_count() ? p.num_tiles : sm_count());
+  cudaError_t e = launch_pdl_opt(pdl_chained(), kern, dim3(grid), dim3(GT_THREADS), smem, st, tmx, tmw, p, vec);
+  if (e != cudaSuccess) return cuda_fail(e, "gemm_tc_rows_kernel launch");
   return B200P_OK;
 }
 
@@ -1027,7 +1032,7 @@ int gemm_tc_launch_grouped(const T* x, const T* w, void* y, const int32_t* seg, 
   p.epi = epi;
   p.act = act;
   gemm_tc_set_second(p, two, GT_BM);
-  return bn == 32 ? gemm_tc_run<T, 32, 10>(tm, p, true, st) : gemm_tc_run<T, 64, 8>(tm, p, true, st);
+  return bn == 32 ? gemm_tc_run<T, 32, 10>(tm, p, st) : gemm_tc_run<T, 64, 8>(tm, p, st);
 }
 template int gemm_tc_launch_grouped<__half>(const __half*, const __half*, void*, const int32_t*, int64_t, int64_t, int64_t, int64_t, int64_t,
                                             int64_t, int64_t, int64_t, int64_t, int, float2, const GemmTcPlain*, cudaStream_t);

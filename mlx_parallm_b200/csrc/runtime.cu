@@ -51,6 +51,7 @@ static thread_local int g_pdl_class = 0;
 void pdl_set_class(int cls) { g_pdl_class = cls; }
 bool pdl_enabled() { return g_pdl == 1 || (g_pdl != 0 && (g_pdl_mask & g_pdl_class) != 0); }
 bool pdl_enabled_gemm() { return g_pdl != 0; }
+bool pdl_chained() { return g_pdl != 0 && g_pdl_class == 128; }
 
 int sm_count() {
   query_device();

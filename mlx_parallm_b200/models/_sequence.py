@@ -77,7 +77,7 @@ class Linear:
         self.weight: Optional[torch.Tensor] = None
 
     def __call__(self, x, epilogue=GEMM_STORE, out=None, act=(0.0, 0.0)):
-        return ops.gemm(x, self.weight, epilogue, out=out, act=act)
+        return ops.gemm(x, self.weight, epilogue, out=out, act=act, chained=True)
 
 
 class Scratch:
@@ -556,27 +556,27 @@ class LatentAttention:
                                  plan["t_row"], plan["t_pos"])
             q = self.uq(cq, GEMM_STORE, out=s.get("q", dt, M, H * (dk + dr)))
             qlat = s.get("qlat", f32, M, H * row)
-            ops.gemm(q, self.uk_t, GEMM_STORE_F32, out=qlat, batch=H, strides=(dk + dr, R * dk, row), M=M, N=R, K=dk, ldx=H * (dk + dr),
+            ops.gemm(q, self.uk_t, GEMM_STORE_F32, chained=True, out=qlat, batch=H, strides=(dk + dr, R * dk, row), M=M, N=R, K=dk, ldx=H * (dk + dr),
                      ldw=dk, ldy=H * row)
             ops.latent_q_rope(q, H, dk, dr, R, self.rates, self.mag, plan["t_pos"], qlat)
             olat = s.get("olat", dt, M, H * row)
             ops.latent_attn(qlat, st.latent, plan["t_row"], plan["t_pos"], olat, H, row, self.window, self.scale, cu=plan["cu"],
                             rows=plan["rows"], nb=plan["nb"], max_n=plan["max_n"])
             mix = s.get("mix", dt, M, H * dv)
-            ops.gemm(olat, self.uv, GEMM_STORE, out=mix, batch=H, strides=(row, dv * R, dv), M=M, N=dv, K=R, ldx=H * row, ldw=R, ldy=H * dv)
+            ops.gemm(olat, self.uv, GEMM_STORE, chained=True, out=mix, batch=H, strides=(row, dv * R, dv), M=M, N=dv, K=R, ldx=H * row, ldw=R, ldy=H * dv)
             return self.o_proj(mix, GEMM_STORE_F32, out=y_out)
         cache = st if self.own_kv else caches[self.kv_from]
         ops.latent_prep(proj, self.q_rank, R, self.q_norm_w, self.kv_norm_w, self.eps, cq, cache.latent if self.own_kv else None,
                         plan["t_row"], plan["t_pos"])
         q = self.uq(cq, GEMM_STORE, out=s.get("q", dt, M, H * dk))
         qlat = s.get("qlat", f32, M, H * R)
-        ops.gemm(q, self.uk_t, GEMM_STORE_F32, out=qlat, batch=H, strides=(dk, R * dk, R), M=M, N=R, K=dk, ldx=H * dk, ldw=dk,
+        ops.gemm(q, self.uk_t, GEMM_STORE_F32, chained=True, out=qlat, batch=H, strides=(dk, R * dk, R), M=M, N=R, K=dk, ldx=H * dk, ldw=dk,
                  ldy=H * R)
         olat = s.get("olat", dt, M, H * R)
         ops.latent_attn(qlat, cache.latent, plan["t_row"], plan["t_pos"], olat, H, R, self.window, self.scale, cu=plan["cu"],
                         rows=plan["rows"], nb=plan["nb"], max_n=plan["max_n"])
         mix = s.get("mix", dt, M, H * dv)
-        ops.gemm(olat, self.uv, GEMM_STORE, out=mix, batch=H, strides=(R, dv * R, dv), M=M, N=dv, K=R, ldx=H * R, ldw=R, ldy=H * dv)
+        ops.gemm(olat, self.uv, GEMM_STORE, chained=True, out=mix, batch=H, strides=(R, dv * R, dv), M=M, N=dv, K=R, ldx=H * R, ldw=R, ldy=H * dv)
         return self.o_proj(mix, GEMM_STORE_F32, out=y_out)
 
 

@@ -270,11 +270,11 @@ def sample_top_p(logits, temperature, top_p, seed, offset, out=None, probs_out=N
 
 # ---- dense linear layers, ragged batches, gated delta rule, latent attention ------------------------------------------
 def gemm(x, w, epilogue=_lib.GEMM_STORE, out=None, act=(0.0, 0.0), batch=1, strides=(0, 0, 0), M=None, N=None, K=None,
-         ldx=None, ldw=None, ldy=None):
+         ldx=None, ldw=None, ldy=None, chained=False):
     """y = x . w^T with fp32 accumulation (b200p_gemm).  Plain call: x [M, K], w [N, K] of one dtype.  Batched call (one
     weight block per head): pass M, N, K, the row strides and ``strides`` = element strides of x, w, y between products.
     ``act``: the epilogue's constants (the clamp of GEMM_GLU_CLAMP, the two factors of GEMM_XIELU,
-    the cap of GEMM_CAP_F32)."""
+    the cap of GEMM_CAP_F32).  ``chained``: a model's layer calls it, between other kernels (_lib.GEMM_CHAINED)."""
     _dev(x, w, out)
     assert x.dtype == w.dtype and x.stride(-1) == 1 and w.stride(-1) == 1
     if M is None:
@@ -290,7 +290,7 @@ def gemm(x, w, epilogue=_lib.GEMM_STORE, out=None, act=(0.0, 0.0), batch=1, stri
     want = torch.float32 if _lib.gemm_is_f32(epilogue) else x.dtype
     assert out.dtype == want and out.stride(-1) == 1, (out.dtype, want)
     _call(("b200p_gemm", N, K, batch), lambda: lib().b200p_gemm(_p(x), _p(w), _p(out), M, N, K, ldx, ldw, ldy, batch, strides[0], strides[1],
-                                                        strides[2], dtype_code(x.dtype), epilogue, float(act[0]), float(act[1]), _stream()))
+                                                        strides[2], dtype_code(x.dtype), epilogue | (_lib.GEMM_CHAINED if chained else 0), float(act[0]), float(act[1]), _stream()))
     return out
 
 

@@ -768,6 +768,7 @@ def test_every_mixture_and_chain_of_products_holds_a_plain_launch(tokens, top):
     assert gather_to_products and not products_to_combine
     assert captured_edges(mixture)[-3] == (tokens <= 64)
     assert captured_edges(lambda: [ops.gemm(x, w[0], _lib.GEMM_STORE_F32, out=y) for _ in range(3)]) == [False, False]
+    assert captured_edges(lambda: [ops.gemm(x, w[0], _lib.GEMM_STORE_F32, out=y, chained=True) for _ in range(2)]) == [True]      # (a layer's)
 
 
 @pytest.mark.parametrize("E,top,M", [(16, 2, 32), (16, 2, 33), (128, 4, 16), (128, 5, 16), (128, 1, 33), (129, 2, 8), (129, 2, 9), (1024, 16, 1), (1024, 32, 1)])
