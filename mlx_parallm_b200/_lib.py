@@ -8,6 +8,7 @@ from __future__ import annotations
 
 import ctypes as C
 import os
+import sys
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "libb200parallm.so")
@@ -224,7 +225,7 @@ def ensure_built(unit_set: str, verbose: bool = False) -> C.CDLL:
     import subprocess
     units = UNIT_SETS[unit_set]
     part = os.path.join(_HERE, f"libb200parallm_{unit_set}.so")
-    cmd = ["make", "-C", os.path.join(_HERE, "csrc"), f"-j{min(8, os.cpu_count() or 1)}",
+    cmd = ["make", "-C", os.path.join(_HERE, "csrc"), f"-j{min(8, os.cpu_count() or 1)}", "PYTHON=" + sys.executable,
            "SRCS=" + " ".join(u + ".cu" for u in units), "LIB=" + part]
     r = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
     if r.returncode != 0 or not os.path.exists(part):

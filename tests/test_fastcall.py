@@ -1,15 +1,47 @@
 """The extension that calls the library without ctypes' conversions hands over what ctypes would: every signature of the binding, called
 through both into a recorder (no device needed)."""
 import ctypes as C
+import os
+import platform
+import shutil
+import subprocess
+import sys
+import sysconfig
 
 import pytest
 
 from mlx_parallm_b200 import _lib
 
-fast = pytest.importorskip("mlx_parallm_b200._fastcall")
+fast = _lib._fastcall
+needs_fast = pytest.mark.skipif(fast is None, reason="the extension is not built for this interpreter")
+CSRC = os.path.join(os.path.dirname(_lib.__file__), "csrc")
+BUILDABLE = os.path.exists(os.path.join(sysconfig.get_paths()["include"], "Python.h")) and platform.machine() == "x86_64" and sys.platform == "linux"
 BOUND = sorted(n for n, (res, args) in _lib.SIGNATURES.items() if res is C.c_int and all(a in _lib._LETTERS for a in args))
 
 
+@pytest.mark.skipif(not BUILDABLE or not os.path.exists(os.path.join(os.path.dirname(_lib.__file__), "libb200parallm.so")), reason="nothing built, or no headers")
+def test_a_built_tree_has_the_extension_of_this_interpreter():
+    assert fast is not None and fast.__file__.endswith(sysconfig.get_config_var("EXT_SUFFIX"))
+
+
+@pytest.mark.skipif(not BUILDABLE, reason="no Python headers, or another platform")
+def test_the_build_reports_what_it_does_not_build(tmp_path):
+    """A compile error fails the build, a missing header is said, and the file carries the interpreter's suffix (another one does not load it)."""
+    os.mkdir(tmp_path / "csrc")
+    for f in ("Makefile", "fastcall.c"):
+        shutil.copy(os.path.join(CSRC, f), tmp_path / "csrc" / f)
+    make = lambda *a: subprocess.run(["make", "-C", str(tmp_path / "csrc"), "fast", *a], capture_output=True, text=True)        # noqa: E731
+    skipped = make("PYTHON=/nonexistent/python")
+    assert skipped.returncode == 0 and "not built" in skipped.stdout
+    assert make("PYTHON=" + sys.executable).returncode == 0
+    assert [f for f in os.listdir(tmp_path) if f.startswith("_fastcall")] == ["_fastcall" + sysconfig.get_config_var("EXT_SUFFIX")]
+    with open(tmp_path / "csrc" / "fastcall.c", "a") as f:
+        f.write("int broken(void) { return undeclared; }\n")
+    os.utime(tmp_path / "csrc" / "fastcall.c", (2 ** 31, 2 ** 31))
+    assert make("PYTHON=" + sys.executable).returncode != 0
+
+
+@needs_fast
 @pytest.mark.parametrize("name", BOUND)
 def test_arguments_arrive(name):
     args = _lib.SIGNATURES[name][1]
@@ -31,6 +63,7 @@ def test_arguments_arrive(name):
     assert seen[0] == seen[1] and len(seen[0]) == len(args)
 
 
+@needs_fast
 def test_other_arguments_go_through_ctypes():
     seen = []
     target = C.CFUNCTYPE(C.c_int, C.c_void_p, C.c_int, C.c_float)(lambda *a: (seen.append(a), 0)[1])
