@@ -100,9 +100,9 @@ class Scratch:
         self._flat[key] = max(self._flat.get(key, 0), n)
 
     def allocate(self):
+        self._views.clear()                                 # (they would keep the buffers that are replaced)
         for key, cols in self._need.items():
             self._bufs[key] = torch.empty((self.rows * cols,), dtype=key[1], device=self.device)
-        self._views.clear()
         for key, n in self._flat.items():
             self._bufs[key] = torch.zeros((n,), dtype=key[1], device=self.device)
 

@@ -85,7 +85,7 @@ def test_error_codes_and_messages():
         _lib.check(L.b200p_gemm(None, None, None, *[1] * 10, 0, 0, 0.0, 0.0, None), "b200p_gemm")
 
 
-def test_scratch_views_are_kept_and_follow_a_new_allocation():
+def test_scratch_views_are_kept_and_follow_a_new_allocation(monkeypatch):
     import torch
     from mlx_parallm_b200.models._sequence import Scratch
     s = Scratch(torch.device("cpu"), 700)
@@ -96,5 +96,10 @@ def test_scratch_views_are_kept_and_follow_a_new_allocation():
     for m in range(1, 700):
         assert s.get("a", torch.float32, m, 4).shape == (m, 4)
     assert len(s._views) <= 512
+    del v
+    s.reserve("b", torch.float32, 4)
+    make, held = torch.empty, []
+    monkeypatch.setattr(torch, "empty", lambda *args, **kw: (held.append(len(s._views)), make(*args, **kw))[1])
     s.allocate()
+    assert held == [0, 0]                                    # no view keeps a buffer that is being replaced
     assert s.get("a", torch.float32, 3, 4).data_ptr() == s._bufs[("a", torch.float32)].data_ptr()
