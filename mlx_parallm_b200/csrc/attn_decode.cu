@@ -284,11 +284,16 @@ static int launch_attn_decode_w(const void* q, const void* kc, const void* vc, c
     attr_set = true;
   }
   dim3 grid((unsigned)splits, (unsigned)Hkv, (unsigned)B);
-  launch_pdl(kern, grid, WARPS * 32, SMEM, st, (const T*)q, (const T*)kc, (const T*)vc, lengths, (T*)out, (float*)ws, Hq, Hkv,
+  // Programmatic launches spare 0.2 to 0.3 us each, but CTAs that are more than the SMs and do not fill their slots take longer to get under way than
+  // those of a plain launch (us, plain / programmatic, attention alone so, behind rope and append: 8 key heads, 2 warps, 128 CTAs 7.2 / 6.9, 256 7.4 / 8.1
+  // and 9.5 / 11.1, 384 11.0 / 11.3, 512 10.8 / 10.5), the reduction's small ones already below (so many rows: 64 7.1 / 6.9, 96 7.6 / 7.6, 128 7.9 /
+  // 8.4, 256 7.9 / 9.4, 512 9.0 / 10.7, 1024 11.2 / 12.3, 3072 the same).
+  const int64_t ctas = (int64_t)splits * Hkv * B, sms = sm_count();
+  launch_pdl_opt(pdl_enabled() && (WARPS == 8 || ctas <= sms || ctas >= 3 * sms), kern, grid, WARPS * 32, SMEM, st, (const T*)q, (const T*)kc, (const T*)vc, lengths, (T*)out, (float*)ws, Hq, Hkv,
              Tcap, scale * 1.4426950408889634f, splits, out_perm);
   B200P_LAUNCH_CHECK("attn_decode_kernel");
   if (splits > 1) {
-    launch_pdl(attn_reduce_kernel<T>, (unsigned)(B * Hq), AD_D, 0, st, (const float*)ws, (T*)out, splits, out_perm);
+    launch_pdl_opt(pdl_enabled() && B * Hq <= 96, attn_reduce_kernel<T>, (unsigned)(B * Hq), AD_D, 0, st, (const float*)ws, (T*)out, splits, out_perm);
     B200P_LAUNCH_CHECK("attn_reduce_kernel");
   }
   return B200P_OK;
