@@ -1,4 +1,4 @@
-"""What would an fp8 (E4M3) KV cache cost against the north star's 1e-2 relative logits tolerance?  CPU study with the oracle:
+"""What would an fp8 (E4M3) KV cache cost against the 1e-2 relative logits tolerance?  CPU study with the oracle:
 the same model and prompts with the K/V cache stored as float32 (the reference, base.py:111-112), float16 (this build) and
 E4M3 without / with one fp32 scale per (token, kv head) -- logits of the last position and of 8 greedy decode steps.
 

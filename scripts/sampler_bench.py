@@ -1,4 +1,4 @@
-"""Time the sampling head (north star kernel 3): argmax, categorical (top_p = 1) and nucleus sampling on [B, V] float32 logits."""
+"""Time the sampling head (kernel 3): argmax, categorical (top_p = 1) and nucleus sampling on [B, V] float32 logits."""
 import os
 import sys
 
