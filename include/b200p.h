@@ -78,7 +78,7 @@ int b200p_sm_count(void);
 int b200p_set_pdl(int enabled);
 
 /* mx.dequantize(w, scales, biases, group_size, bits)            [nn.QuantizedEmbedding.__call__,
- * models/llama.py:212, models/qwen3.py:166; bit-exactness target of the north star]
+ * models/llama.py:212, models/qwen3.py:166; held bit-exact]
  * out[N,K] in `dtype`. */
 int b200p_dequantize(const uint32_t* w, const void* scales, const void* biases, void* out,
                      int64_t N, int64_t K, int group_size, int bits, int dtype, int mode,

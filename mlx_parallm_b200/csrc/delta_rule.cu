@@ -2,14 +2,15 @@
 // current value along the current key and read with the current query), as four kernels over a ragged batch:
 //   delta_prep_kernel         short causal convolution + silu of q, k, v; unit q / k per head; beta and decay   (per token)
 //   delta_conv_commit_kernel  the convolution's carried inputs                                                   (per entry)
-//   delta_scan_kernel         the recurrence, fp32, token by token; four lanes per pair of state columns           (per entry, head)
+//   delta_scan_kernel         the recurrence, fp32, token by token; decode steps: delta_step_kernel, long entries: delta_pair_kernel  (per entry, head)
 //   delta_out_kernel          per-head rms norm * weight * silu(gate)                                            (per token)
 // The same kernels carry the variants other designs use: a decay per head AND key channel (a row of S each), a gate that is a
 // sigmoid of a separate tensor, and the plain decayed accumulation S <- g S + k v^T (linear attention with a constant decay,
 // fed by linear_attn_prep_kernel).
-// An entry's numbers depend on its own tokens alone.  Single tokens and entries of less than 32 run in one summation order, whatever kernel takes
-// them; entries of 32 tokens and more (keys of 65 to 128 channels, delta rule) two tokens at a time (delta_pair_kernel), which differs in the last
-// places.
+// Single tokens and entries of less than 32 run in one summation order, whatever kernel takes them; entries of 32 tokens and more (keys of 65 to 128
+// channels, delta rule) two tokens at a time (delta_pair_kernel), which differs in the last places, so a prompt and its portions agree to rounding.
+// An entry's bits depend on its own tokens alone, with one exception: beside at least as many empty entries as it has tokens, in a call that
+// does not say how long its longest entry is, it goes token by token (delta_step_kernel).
 #include "common.cuh"
 
 namespace b200p {
@@ -232,8 +233,8 @@ __global__ void delta_conv_commit_kernel(const float* __restrict__ proj, int64_t
 }
 
 // Rows of a state column are summed in segments: four interleaved partial sums each (rows i mod 4), combined in a fixed order, then the
-// segments pairwise.  Every kernel below, however many lanes it gives to a column, adds in this one order, so a token's numbers do not
-// depend on whether it arrives in a prompt or alone or on the size of the batch.
+// segments pairwise.  The kernels that go token by token, however many lanes they give to a column, add in this one order, so a token's numbers do
+// not depend on whether it arrives in a short prompt or alone or on the size of the batch.
 constexpr int ds_segs(int dkp) { return dkp <= 64 ? 4 : dkp <= 128 ? 8 : dkp / 32; }
 
 // Sums of x and of y over the LANES lanes of a slot: even lanes get the sum of x, odd lanes that of y.
@@ -508,8 +509,8 @@ delta_scan_kernel(const float* __restrict__ qn, const float* __restrict__ kn, co
 // vectors and the four scalars are the same for all columns: the threads that stage a token's row compute them.  All of it stays fp32.
 // A thread holds 16 rows of FOUR columns: a 16-byte read of shared memory (four cycles of its port for a warp) serves 16 packed products; eight
 // lanes share a column slot.  The exchanges for u run beside the products with the queries, those for o beside the update.
-// An entry takes this path if it has at least DP_MIN tokens, whatever the others have, so its bits do not depend on its batch; a prompt
-// whose portions are shorter has the bits of single tokens, which differ in the last places.
+// An entry takes this path if it has at least DP_MIN tokens, whatever the others have (the exception: top of the file); a prompt whose portions are
+// shorter has the bits of single tokens, which differ in the last places.
 // Bound: FFMA2 with three distinct operands, one in about four cycles per scheduler (measured; scalar FFMA, two in 2.5, needs registers that are
 // not there: 274 us).  us before -> now, heads of 128 x 128, decays per channel / per head: 4 x 512 tokens, 16 heads 221 -> 156 / 193 -> 152, 32
 // heads 357 -> 266 / 315 -> 260 (two CTAs per SM; one: 304 / 298); 16 x 250, 32 heads 635 -> 449 / 542 -> 441; 1 x 32, 16 heads 18.6 -> 14.5.

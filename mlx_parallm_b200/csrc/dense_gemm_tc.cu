@@ -310,8 +310,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmw, const __grid_constant__ 
 // ---------------------------------------------------------------------------------------------------------- short K, narrow outputs
 // More than 64 tokens where the pair kernel below has little to multiply: one CTA on a tile of 128 tokens (the M side) x BN weight rows.  The
 // set-up is half of the pair's (no cluster, fewer TMEM columns), a narrow output pads no 256 rows, and a thread owns a token's row, so that its
-// outputs leave as 16-byte pieces: at a short K the store is what bounds the call.  Bound: the output's way to HBM (64 x 1500 x 128 x 128 to
-// bf16: 3.6 TB/s) or, in small calls, latency.  Where the line lies: gemm_tc_rows_better.
+// outputs leave as 16-byte pieces: at a short K the store is what bounds the call.  Bound: the output's way through L2 (64 x 1500 x 512 x 128 to
+// bf16: L2 at 67 % of its peak, tensor pipe 16 %) or, in small calls, latency.  Where the line lies: gemm_tc_rows_better.
 template <typename T> __device__ __forceinline__ uint32_t pack2(float a, float b);
 template <> __device__ __forceinline__ uint32_t pack2<__half>(float a, float b) {
   const __half2 h = __floats2half2_rn(a, b);

@@ -1,4 +1,4 @@
-"""Tensor parallelism for the decode step (new work mandated by the north star; the reference is
+"""Tensor parallelism for the decode step (new work; the reference is
 single-device).
 
 One process per GPU (torchrun), ranks share a ``torch.distributed`` group (NCCL on the GPUs, gloo in

@@ -174,7 +174,7 @@ def quantized_matmul(x, w_q, scales, biases, group_size: int = 64, bits: int = 4
     b = np.asarray(biases, np.float32)
     # grouped form, but evaluated with one BLAS call: W = q*s + b exactly in fp32-ish
     # (sum_g s_g * (x_g . q_g)) == x . (q * s_rep); the difference to the per-group order is
-    # fp32 reassociation only, far inside the 1e-2 tolerance the north star states.
+    # fp32 reassociation only, far inside the 1e-2 tolerance of the logits.
     wf = q * np.repeat(s, group_size, -1) + np.repeat(b, group_size, -1)
     y = x2 @ wf.T
     del ng, n

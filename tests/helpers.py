@@ -21,7 +21,7 @@ def make_pair(name, dtype="float16", seed=1234, numerics="reference", device="cu
 
 
 def rel_err(a, b):
-    """max |a-b| / max |b| -- the 'relative' of the north star's 1e-2 logits tolerance."""
+    """max |a-b| / max |b| -- the 'relative' of the 1e-2 logits tolerance."""
     a = np.asarray(a, np.float64)
     b = np.asarray(b, np.float64)
     return float(np.abs(a - b).max() / max(np.abs(b).max(), 1e-30))

@@ -3,7 +3,7 @@ full-vocabulary slices of every benchmark architecture -- Mistral-7B, Llama-3-8B
 (8-bit) -- with ``synth.random_weights``, compared with ``OracleModel(numerics="reference")`` (what MLX would compute: fp32 KV
 cache, fp32 residual stream):
 
-  * decode logits at B = 64 over a synthetic 2048-token context          <= 1e-2 relative (north star)
+  * decode logits at B = 64 over a synthetic 2048-token context          <= 1e-2 relative
   * prefill logits (last position) at B x L = 4 x 64 = 256 tokens         <= 1e-2 relative
   * 32 greedy tokens on 128 sequences: every decision the oracle makes with a top-2 margin above the logits tolerance is
     reproduced; a sequence may leave the oracle's transcript only at a near-tie (see ``greedy_report``)

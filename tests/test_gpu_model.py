@@ -1,4 +1,4 @@
-"""Model-level parity: logits within the north star's 1e-2 relative, greedy ids against the oracle and the
+"""Model-level parity: logits within the 1e-2 relative, greedy ids against the oracle and the
 committed golden transcripts, and the reference-API behaviours of generate_step."""
 import os
 
@@ -11,7 +11,7 @@ from oracle.model import generate_step as oracle_generate_step
 
 pytestmark = pytest.mark.gpu
 
-LOGIT_TOL = 1e-2          # north star: per-step logits within 1e-2 relative (fp32 accumulate)
+LOGIT_TOL = 1e-2          # per-step logits within 1e-2 relative (fp32 accumulate)
 
 
 @pytest.mark.parametrize("name,dtype", [("tiny-llama", "float16"), ("tiny-qwen3", "bfloat16"),
