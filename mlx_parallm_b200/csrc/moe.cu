@@ -24,6 +24,18 @@ static bool moe_pdl(int64_t tokens) { return pdl_enabled_gemm() && tokens <= 64;
 constexpr int MOE_MAX_PER_LANE = 32;    // experts <= 1024
 constexpr int MOE_MAX_TOP = 32;
 
+// Choices that found nothing above -inf (logits that are NaN or -inf) hold E: they get the first experts that the token has not chosen, so that it
+// never gives an expert two rows and no group grows beyond the batch.  Whole warps; lane k holds choice k.
+__device__ __forceinline__ void moe_fill_choices(int lane, int E, int top, int& my_id) {
+  if (!__any_sync(0xffffffffu, lane < top && my_id >= E)) return;
+  for (int k = 0; k < top; ++k) {
+    if (__shfl_sync(0xffffffffu, my_id, k) < E) continue;
+    int e = 0;
+    while (__any_sync(0xffffffffu, lane < top && my_id == e)) ++e;
+    if (lane == k) my_id = e;
+  }
+}
+
 // One warp's token: the choice k goes to lane k.  PER_LANE * 32 experts at most.
 template <int PER_LANE>
 __device__ __forceinline__ void moe_route_token(const float* __restrict__ logits, int64_t ldl, const float* __restrict__ bias, int64_t t, int E,
@@ -48,7 +60,6 @@ __device__ __forceinline__ void moe_route_token(const float* __restrict__ logits
       const int oe = __shfl_xor_sync(0xffffffffu, be, o);
       if (ob > best || (ob == best && oe < be)) { best = ob; be = oe; }
     }
-    if (be >= E) be = 0;                                             // nothing above -inf is left (NaN logits): the weights come out as NaN
     if (k == 0) first = best;
     const float p = expf(best - first);                              // the first pick is the largest: exponents <= 0
     den += p;
@@ -57,7 +68,8 @@ __device__ __forceinline__ void moe_route_token(const float* __restrict__ logits
     for (int i = 0; i < PER_LANE; ++i)
       if (i * 32 + lane == be) z[i] = -INFINITY;
   }
-  my_wt = mine / den;
+  my_wt = mine / den;                                                // (a filled choice: 0, or NaN where no logit is a number)
+  moe_fill_choices(lane, E, top, my_id);
 }
 
 template <int PER_LANE>
@@ -158,14 +170,14 @@ __global__ void moe_route_scores_kernel(const float* __restrict__ logits, int64_
       const int oe = __shfl_xor_sync(0xffffffffu, be, o);
       if (ob > best || (ob == best && oe < be)) { best = ob; be = oe; }
     }
-    if (be >= E) be = 0;                                               // fewer candidates than picks: cannot happen with keep * per >= top
-    const float s = sc[be];
+    const float s = be < E ? sc[be] : sc[0];                            // (E: scores that are NaN; otherwise keep * per >= top)
     den += s;
     if (lane == k) { mine = s; my_id = be; }
     __syncwarp();
-    if (lane == 0) pick[be] = -INFINITY;
+    if (lane == 0 && be < E) pick[be] = -INFINITY;
     __syncwarp();
   }
+  moe_fill_choices(lane, E, top, my_id);
   if (lane < top) {
     ids[t * top + lane] = my_id;
     wts[t * top + lane] = renorm ? mine / (den + 1e-20f) * scale : mine * scale;       // renorm 0: the scores as they are
@@ -333,8 +345,11 @@ using namespace b200p;
 
 // One block for as few choices as its 32 warps make beside each other.  us, one block / two launches: 16 experts, 2 choices, 16 and 32 tokens 3.0 /
 // 3.65, 3.6 / 3.65, 4 choices of 32 tokens 4.4 / 3.9, 8 of 64 10 / 4.6; 128 experts, 4 choices of 16 tokens 4.2 / 4.3, of 32 5.3 / 4.3; above 128
-// a lane has up to 32 logits: 129 experts, 2 choices of 8 and 16 tokens 5.2 / 5.4, 6.1 / 5.4, 160 experts, 16 choices of 64 tokens 71 / 12.
-static bool moe_one_block(int64_t M, int E, int top) { return E <= 128 ? M <= 32 && M * top <= MOE_ONE_BLOCK : M * top <= 16; }
+// a lane has up to 32 logits: 129 experts, 6 choices of 4 tokens 6.4 / 6.8, 2 of 8 and 16 5.2 / 5.4, 6.1 / 5.4, 160 experts, 16 choices of 64 tokens
+// 71 / 12.
+static bool moe_one_block(int64_t M, int E, int top) {
+  return E <= 128 ? M <= 32 && M * top <= MOE_ONE_BLOCK : M * top <= (M <= 4 ? 32 : 16);
+}
 
 static int moe_plan_launch(const int32_t* ids, int32_t* seg, int32_t* slot_of, int32_t* token_of, int64_t M, int E, int top, cudaStream_t st) {
   cudaError_t e = launch_pdl_opt(moe_pdl(M), moe_plan_kernel, dim3(1), dim3(1024), 2 * E * sizeof(int32_t), st, ids, seg, slot_of, token_of,

@@ -771,7 +771,7 @@ def test_every_mixture_and_chain_of_products_holds_a_plain_launch(tokens, top):
     assert captured_edges(lambda: [ops.gemm(x, w[0], _lib.GEMM_STORE_F32, out=y, chained=True) for _ in range(2)]) == [True]      # (a layer's)
 
 
-@pytest.mark.parametrize("E,top,M", [(16, 2, 32), (16, 2, 33), (128, 4, 16), (128, 5, 16), (128, 1, 33), (129, 2, 8), (129, 2, 9), (1024, 16, 1), (1024, 32, 1)])
+@pytest.mark.parametrize("E,top,M", [(16, 2, 32), (16, 2, 33), (128, 4, 16), (128, 5, 16), (128, 1, 33), (129, 2, 8), (129, 2, 9), (129, 8, 4), (129, 9, 4), (1024, 32, 1), (1024, 32, 2)])
 def test_routing_in_one_block_and_in_two_launches(E, top, M):
     """On both sides of the line between them: the chosen experts, their weights, and every choice's slot inside its expert's segment."""
     from mlx_parallm_b200 import ops
@@ -788,3 +788,39 @@ def test_routing_in_one_block_and_in_two_launches(E, top, M):
     assert torch.equal(slots.sort().values, torch.arange(M * top))
     assert bool((seg.cpu().long()[flat] <= slots).all()) and bool((slots < seg.cpu().long()[flat + 1]).all())
     assert torch.equal(token_of.cpu().long()[slots], torch.arange(M * top) // top)
+
+
+@pytest.mark.parametrize("M,E,top", [(32, 16, 8), (4, 16, 8), (100, 40, 4), (9, 200, 3)])
+@pytest.mark.parametrize("how", ["softmax", "sigmoid", "scores"])
+def test_logits_without_enough_numbers_choose_distinct_experts(how, M, E, top):
+    """Rows of NaN, of -inf and with fewer numbers than choices: every choice is an expert, none twice, so no expert gets more rows than there are
+    tokens (which sizes the grouped products: a surplus row would push out another sequence's), and the other rows choose as they do alone."""
+    from mlx_parallm_b200 import ops
+    g = torch.Generator().manual_seed(M + E)
+    logits = torch.randn(M, E, generator=g)
+    logits[:, 0] = 4.0                                                   # everyone's choice
+    logits[1], logits[2] = float("nan"), float("-inf")
+    logits[3, 2:] = float("nan")
+    i32 = dict(dtype=torch.int32, device="cuda")
+
+    def route(z):
+        m = z.shape[0]
+        ids, slot_of, token_of, seg = (torch.zeros(n, **i32) for n in ((m, top), (m, top), (m * top,), (E + 1,)))
+        wts = torch.zeros(m, top, device="cuda")
+        if how == "softmax":
+            ops.moe_route(z.cuda(), None, ids, wts, seg, slot_of, token_of, top)
+        elif how == "sigmoid":
+            ops.moe_route_sigmoid(z.cuda(), None, ids, wts, seg, slot_of, token_of, top)
+        else:
+            ops.moe_route_scores(z.cuda(), ids, wts, seg, slot_of, token_of, top, softmax=True)
+        return ids.cpu(), wts.cpu(), seg.cpu(), slot_of.cpu()
+
+    ids, wts, seg, slots = route(logits)
+    assert bool((ids >= 0).all()) and bool((ids < E).all()) and all(len(set(r.tolist())) == top for r in ids)
+    assert int(seg.diff().max()) <= M and int(seg[-1]) == M * top and torch.equal(slots.reshape(-1).sort().values, torch.arange(M * top, dtype=torch.int32))
+    for t in range(M):
+        if t not in (1, 2, 3):
+            alone = route(logits[t:t + 1])
+            assert torch.equal(alone[0][0], ids[t]) and torch.equal(alone[1][0], wts[t])
+    if how == "softmax":
+        assert set(ids[3, :2].tolist()) == {0, 1} and bool((wts[3, 2:] == 0).all()) and bool(wts[1].isnan().all())
