@@ -45,7 +45,7 @@ static int query_device() {
 
 // per-class PDL mask for the non-GEMM kernels (see common.cuh).  Attention by default: its launch and set-up hide behind rope and append, and its
 // reduction behind it (us, off / on: decode steps 16 x 8192 77.3 / 75.0, prompts 4 x 777 61.9 / 59.4, decode step of one sequence 257.5 / 252.7);
-// rope as well gives nothing more in captured steps (255.1).
+// rope as well gives nothing more in captured steps (255.1).  Which sizes of decode attention are launched plainly all the same: attn_decode.cu.
 static int g_pdl_mask = [] { const char* e = getenv("B200P_PDL_MASK"); return e ? atoi(e) : 8; }();
 static thread_local int g_pdl_class = 0;
 void pdl_set_class(int cls) { g_pdl_class = cls; }
