@@ -40,7 +40,7 @@ template <typename T, int AD_WARPS>
 __global__ void __launch_bounds__(AD_WARPS * 32, AD_WARPS == 8 ? 1 : 4)
 attn_decode_kernel(const T* __restrict__ q, const T* __restrict__ kc, const T* __restrict__ vc,
                    const int32_t* __restrict__ lengths, T* __restrict__ out, float* __restrict__ ws, int Hq, int Hkv,
-                   int64_t Tcap, float scale_log2e, int splits, int out_perm) {
+                   int64_t Tcap, float scale_log2e, int splits, int out_perm, int early) {
   extern __shared__ __align__(128) uint8_t smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int split = blockIdx.x, kvh = blockIdx.y, b = blockIdx.z;
@@ -175,7 +175,7 @@ attn_decode_kernel(const T* __restrict__ q, const T* __restrict__ kc, const T* _
   // ---- finish row sums across the quad, publish this warp's partial ---------------------------------
   l0 += __shfl_xor_sync(0xffffffffu, l0, 1); l0 += __shfl_xor_sync(0xffffffffu, l0, 2);
   l1 += __shfl_xor_sync(0xffffffffu, l1, 1); l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
-  pdl_launch_dependents();
+  if (early) pdl_launch_dependents();               // (launch_attn_decode_w)
   __syncthreads();                                  // everyone is past its K/V smem: reuse it for the merge
   float* wo = reinterpret_cast<float*>(smem) + warp * (16 * (AD_D + 4));   // [16 rows][m, l, pad, pad, O[128]]
   {
@@ -286,14 +286,15 @@ static int launch_attn_decode_w(const void* q, const void* kc, const void* vc, c
   dim3 grid((unsigned)splits, (unsigned)Hkv, (unsigned)B);
   // Programmatic launches spare 0.2 to 0.3 us each, but CTAs that are more than the SMs and do not fill their slots take longer to get under way than
   // those of a plain launch (us, plain / programmatic, attention alone so, behind rope and append: 8 key heads, 2 warps, 128 CTAs 7.2 / 6.9, 256 7.4 / 8.1
-  // and 9.5 / 11.1, 384 11.0 / 11.3, 512 10.8 / 10.5), the reduction's small ones already below (so many rows: 64 7.1 / 6.9, 96 7.6 / 7.6, 128 7.9 /
-  // 8.4, 256 7.9 / 9.4, 512 9.0 / 10.7, 1024 11.2 / 12.3, 3072 the same).
+  // and 9.5 / 11.1, 384 11.0 / 11.3, 512 10.8 / 10.5).  The reduction is programmatic at any size, but let in early, while the attention still runs,
+  // only where it is small or fills the GPU several times over (so many rows, plain / let in / at the attention's end: 32 6.4 / 6.1 / 6.4, 128 7.9 / 8.4 /
+  // 7.7, 256 7.9 / 9.7 / 7.4, 512 10.8 / 12.3 / 10.6, 1024 11.0 / 12.2 / 10.7, 1536 16.6 / 17.0 / 16.5, 3072 20.2 / 20.0 / 20.2).
   const int64_t ctas = (int64_t)splits * Hkv * B, sms = sm_count();
   launch_pdl_opt(pdl_enabled() && (WARPS == 8 || ctas <= sms || ctas >= 3 * sms), kern, grid, WARPS * 32, SMEM, st, (const T*)q, (const T*)kc, (const T*)vc, lengths, (T*)out, (float*)ws, Hq, Hkv,
-             Tcap, scale * 1.4426950408889634f, splits, out_perm);
+             Tcap, scale * 1.4426950408889634f, splits, out_perm, splits == 1 || B * Hq <= 96 || B * Hq >= 2048 ? 1 : 0);
   B200P_LAUNCH_CHECK("attn_decode_kernel");
   if (splits > 1) {
-    launch_pdl_opt(pdl_enabled() && B * Hq <= 96, attn_reduce_kernel<T>, (unsigned)(B * Hq), AD_D, 0, st, (const float*)ws, (T*)out, splits, out_perm);
+    launch_pdl(attn_reduce_kernel<T>, (unsigned)(B * Hq), AD_D, 0, st, (const float*)ws, (T*)out, splits, out_perm);
     B200P_LAUNCH_CHECK("attn_reduce_kernel");
   }
   return B200P_OK;
