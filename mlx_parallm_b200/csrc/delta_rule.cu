@@ -2,15 +2,16 @@
 // current value along the current key and read with the current query), as four kernels over a ragged batch:
 //   delta_prep_kernel         short causal convolution + silu of q, k, v; unit q / k per head; beta and decay   (per token)
 //   delta_conv_commit_kernel  the convolution's carried inputs                                                   (per entry)
-//   delta_scan_kernel         the recurrence, fp32, token by token; decode steps: delta_step_kernel, long entries: delta_pair_kernel  (per entry, head)
+//   delta_scan_kernel         the recurrence, fp32, token by token; decode steps: delta_step_kernel, long entries: delta_chunk_kernel  (per entry, head)
 //   delta_out_kernel          per-head rms norm * weight * silu(gate)                                            (per token)
 // The same kernels carry the variants other designs use: a decay per head AND key channel (a row of S each), a gate that is a
 // sigmoid of a separate tensor, and the plain decayed accumulation S <- g S + k v^T (linear attention with a constant decay,
 // fed by linear_attn_prep_kernel).
 // Single tokens and entries of less than 32 run in one summation order, whatever kernel takes them; entries of 32 tokens and more (keys of 65 to 128
-// channels, delta rule) two tokens at a time (delta_pair_kernel), which differs in the last places, so a prompt and its portions agree to rounding.
-// An entry's bits depend on its own tokens alone, with one exception: beside at least as many empty entries as it has tokens, in a call that
-// does not say how long its longest entry is, it goes token by token (delta_step_kernel).
+// channels, delta rule) 16 tokens at a time (delta_chunk_kernel), which differs in the last places, so a prompt and its portions agree to rounding.
+// An entry's bits depend on its own tokens alone, with two exceptions: beside at least as many empty entries as it has tokens, in a call that
+// does not say how long its longest entry is, it goes token by token (delta_step_kernel); with 16 to 31 tokens, in a call that says that its longest entry
+// has 32 or more, it goes with that one.
 #include "common.cuh"
 
 namespace b200p {
@@ -370,7 +371,7 @@ delta_scan_kernel(const float* __restrict__ qn, const float* __restrict__ kn, co
   const bool live0 = j0 < dv, live1 = j1 < dv, odd = (l & 1) != 0;
   const int t0 = cu[e], t1 = cu[e + 1];
   const bool waits = (blockIdx.x | blockIdx.y | blockIdx.z) == 0;        // (see delta_scan_launch: the grid ends no earlier than the launch before)
-  if (t1 <= t0 || t1 - t0 > most) {                              // (longer entries: delta_pair_kernel)
+  if (t1 <= t0 || t1 - t0 > most) {                              // (longer entries: delta_chunk_kernel)
     if (waits) pdl_wait();
     return;
   }
@@ -499,237 +500,545 @@ delta_scan_kernel(const float* __restrict__ qn, const float* __restrict__ kn, co
   if (waits) pdl_wait();
 }
 
-// Prompts of keys of 65 to 128 channels, two tokens at a time.  In the kernels above the chain of one token (dot, reduction over the lanes,
-// update, dot) and the reads of shared memory for it are what bounds a CTA.  With g1, k1, q1, v1 and g2, k2, q2, v2 of two tokens and the
-// state S before them,
-//     u1 = b1 (v1 - S^T (g1 k1))                 o1 = S^T (g1 q1) + (q1 . k1) u1
-//     u2 = b2 (v2 - S^T (g1 g2 k2) - (k2 . g2 k1) u1)      o2 = S^T (g1 g2 q2) + (q2 . g2 k1) u1 + (q2 . k2) u2
-//     S <- g1 g2 S + (g2 k1) u1 + k2 u2
-// so that four dot products with one state share a pass and a reduction, and 7 instead of 8 operations per element and pair are left.  The scaled
-// vectors and the four scalars are the same for all columns: the threads that stage a token's row compute them.  All of it stays fp32.
-// A thread holds 16 rows of FOUR columns: a 16-byte read of shared memory (four cycles of its port for a warp) serves 16 packed products; eight
-// lanes share a column slot.  The exchanges for u run beside the products with the queries, those for o beside the update.
-// An entry takes this path if it has at least DP_MIN tokens, whatever the others have (the exception: top of the file); a prompt whose portions are
-// shorter has the bits of single tokens, which differ in the last places.
-// Bound: FFMA2 with three distinct operands, one in about four cycles per scheduler (measured; scalar FFMA, two in 2.5, needs registers that are
-// not there: 274 us).  us before -> now, heads of 128 x 128, decays per channel / per head: 4 x 512 tokens, 16 heads 221 -> 156 / 193 -> 152, 32
-// heads 357 -> 266 / 315 -> 260 (two CTAs per SM; one: 304 / 298); 16 x 250, 32 heads 635 -> 449 / 542 -> 441; 1 x 32, 16 heads 18.6 -> 14.5.
-constexpr int DP_MIN = 32, DP_CHUNK = 8, DP_COLS = 64, DP_LDK = 160;
-// warps 0 .. 3 compute, 4 .. 7 stage; two CTAs per SM: registers at launch 256 x 128 = 128 x 168 + 128 x 88
-constexpr int DP_TEAM = 128, DP_THREADS = 2 * DP_TEAM, DP_REGS_COMPUTE = 168, DP_REGS_STAGE = 88;
-template <int MODE, int PER_SM>
-__global__ void __launch_bounds__(DP_THREADS, PER_SM)
-delta_pair_kernel(const float* __restrict__ qn, const float* __restrict__ kn, const float* __restrict__ v, const float* __restrict__ beta,
-                  const float* __restrict__ decay, float* __restrict__ state, const int32_t* __restrict__ cu, const int32_t* __restrict__ rows,
-                  const int32_t* __restrict__ lengths, float* __restrict__ o, int H, int KH, int dk, int dv) {
-  enum { K1, K2, Q1, Q2, GG, KD, KU, VECS };                   // g1 k1, g1 g2 k2, g1 q1, g1 g2 q2, g1 g2, g2 k1, k2
-  constexpr int PAIRS = DP_CHUNK / 2;
-  __shared__ __align__(16) float vec[2][PAIRS][VECS][DP_LDK];  // 16 rows per lane, padded by 16 bytes: the lanes' reads fall into different banks
-  __shared__ __align__(16) float dots[2][PAIRS][4][4];         // k2 . kd, q1 . k1, q2 . kd, q2 . k2: a share per warp
-  __shared__ __align__(16) float vs[2][DP_CHUNK][DP_COLS];
-  __shared__ float bs[2][DP_CHUNK];
-  const int e = blockIdx.x, h = blockIdx.y, tid = threadIdx.x & (DP_TEAM - 1), lane = tid & 31, warp = tid >> 5;
+// Prompts of keys of 65 to 128 channels, 16 tokens (a chunk) at a time, the products on the tensor cores.  With G_t the product of the decays of the
+// chunk's tokens up to t and S the state before it,
+//     X_t = v_t - S^T (G_t k_t)          A_tj = k_t . (G_t / G_j) k_j  (j < t)       P_tj = q_t . (G_t / G_j) k_j  (j <= t)
+//     U = T X,  T = (I + diag(b) A)^-1 diag(b)       O = S^T (G_t q_t) + P U         S <- G S + sum_j (G / G_j) k_j u_j
+// so the chain from state to state is two products per 16 tokens instead of two dot products per token, and T and P, which need no state, are made
+// beforehand for all chunks at once (delta_triangle_kernel).  Every quotient of decays is a product of the decays in between: never above one, no
+// division.
+//
+// All of it keeps fp32's accuracy: an operand is the sum of two tf32 numbers (the nearest one and the rest), a product three MMAs (high . high,
+// low . high, high . low; what is left out is below 2^-22 of it), and as an MMA cuts its sum off instead of rounding it, the large products are
+// summed over 32 channels at most before a rounding addition takes over.  Relative error of o / the state against 64 bits, 512 tokens, 128 x 128: 1.7e-7 / 1.5e-7
+// with decays as a layer has them, 1.9e-7 / 2.1e-7 with decays of 0.98 to 1 (token by token 0.8e-7 / 0.8e-7 and 1.6e-7 / 2.2e-7; sums left to the MMA alone
+// 7e-7 and 1.1e-6).
+constexpr int DC_MIN = 32, DC_CHUNK = 16, DC_COLS = 64, DC_TEAM = 128;
+constexpr int DC_MIN_DV = DC_CHUNK + 1;                        // a chunk of m tokens keeps T and P, m (m + 1) numbers, in its m rows of o until o is written
+
+__device__ __forceinline__ void dc_mma(float (&d)[4], const float (&a)[4], float b0, float b1) {
+  asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+      : "r"(__float_as_uint(a[0])), "r"(__float_as_uint(a[1])), "r"(__float_as_uint(a[2])), "r"(__float_as_uint(a[3])), "r"(__float_as_uint(b0)),
+        "r"(__float_as_uint(b1)));
+}
+__device__ __forceinline__ void dc_mma0(float (&d)[4], const float (&a)[4], float b0, float b1) {
+  asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+      : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+      : "r"(__float_as_uint(a[0])), "r"(__float_as_uint(a[1])), "r"(__float_as_uint(a[2])), "r"(__float_as_uint(a[3])), "r"(__float_as_uint(b0)),
+        "r"(__float_as_uint(b1)), "f"(0.f));
+}
+// x = high + low: the nearest tf32 number and what is left (the MMA drops the last two of its 13 bits)
+__device__ __forceinline__ float dc_high(float x) { return __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xffffe000u); }
+__device__ __forceinline__ void dc_split(float2 x, float2& hi, float2& lo) {
+  hi = make_float2(dc_high(x.x), dc_high(x.y));
+  lo = make_float2(x.x - hi.x, x.y - hi.y);
+}
+// an accumulator's columns 2 t, 2 t + 1 as the A operand's t, t + 4 (the MMA's k index is a label: B is laid out for it)
+__device__ __forceinline__ void dc_operand(const float (&c)[4], float (&hi)[4], float (&lo)[4]) {
+  float2 h0, h1, l0, l1;
+  dc_split(make_float2(c[0], c[1]), h0, l0);
+  dc_split(make_float2(c[2], c[3]), h1, l1);
+  hi[0] = h0.x, hi[1] = h1.x, hi[2] = h0.y, hi[3] = h1.y;
+  lo[0] = l0.x, lo[1] = l1.x, lo[2] = l0.y, lo[3] = l1.y;
+}
+
+// channel d of a chunk's keys, queries and decays; tokens past the end are ones that change nothing
+template <int MODE>
+__device__ __forceinline__ void dc_fetch(const float* __restrict__ qn, const float* __restrict__ kn, const float* __restrict__ decay, int tc, int t1, int h, int kh,
+                                         int d, int H, int KH, int dk, float (&k)[DC_CHUNK], float (&q)[DC_CHUNK], float (&gg)[DC_CHUNK]) {
+  const float* ks = kn + ((int64_t)tc * KH + kh) * dk + d;
+  const float* qs = qn + ((int64_t)tc * KH + kh) * dk + d;
+  const float* gs = MODE == 1 ? decay + ((int64_t)tc * H + h) * dk + d : decay + (int64_t)tc * H + h;
+  const int64_t k_step = (int64_t)KH * dk, g_step = MODE == 1 ? (int64_t)H * dk : H;
+  if (tc + DC_CHUNK <= t1 && dk == 128) {
+#pragma unroll
+    for (int i = 0; i < DC_CHUNK; ++i) k[i] = ks[i * k_step], q[i] = qs[i * k_step], gg[i] = gs[i * g_step];
+  } else {
+#pragma unroll
+    for (int i = 0; i < DC_CHUNK; ++i) {
+      const bool in = tc + i < t1, ok = in && d < dk;
+      k[i] = ok ? ks[i * k_step] : 0.f;
+      q[i] = ok ? qs[i * k_step] : 0.f;
+      gg[i] = (MODE == 1 ? ok : in) ? gs[i * g_step] : 1.f;
+    }
+  }
+}
+
+// T and P of every chunk of the entries of DC_MIN tokens and more, a CTA each, a thread per key channel: left in the chunk's rows of o, one copy per
+// slice of columns, row by row (T's part, then P's).  A and P of two tokens in different halves of the chunk, or different quarters of a half, are a
+// product of rows scaled from the border on and of rows scaled up to it (12 MMAs per warp); those of one quarter are summed over the channels directly.
+// Bound: instructions (5500 per chunk and head, issue slots half used) and the latency of a CTA's reads: 104 chunks x 16 heads 15 us, six CTAs per SM; four 18 us.
+template <int MODE>
+__global__ void __launch_bounds__(DC_TEAM, 6)
+delta_triangle_kernel(const float* __restrict__ qn, const float* __restrict__ kn, const float* __restrict__ beta, const float* __restrict__ decay,
+                      const int32_t* __restrict__ cu, float* __restrict__ o, int H, int KH, int dk, int dv, int slices, int least) {
+  constexpr int LDR = 40, LDP = 17;                            // padded rows: a half warp's 8-byte reads fall into different banks
+  __shared__ __align__(16) float scratch_all[4][24 * LDR], part[4][2][16 * LDP], tri[16 * 20];
+  __shared__ float out[16 * 17];
+  const int h = blockIdx.y, d = threadIdx.x, w = d >> 5, lane = d & 31, g = lane >> 2, t = lane & 3;
   pdl_launch_dependents();
-  const int t0 = cu[e], t1 = cu[e + 1];
-  if (t1 - t0 < DP_MIN) return;
-  const int row = rows[e], kh = h / (H / KH);
-  if (threadIdx.x >= DP_TEAM) {
-    if constexpr (PER_SM == 2) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(DP_REGS_STAGE));
-    // ===================================== staging =====================================
-    // Inputs travel to registers a chunk ahead; tokens past the end are ones that change nothing.
-    float pk[DP_CHUNK], pq[DP_CHUNK], pg[DP_CHUNK], pv[4], pb = 0.f;
-    auto fetch = [&](int tc) {
+  const int t0 = cu[blockIdx.x], t1 = cu[blockIdx.x + 1];
+  if (t1 - t0 < least) return;
+  const int kh = h / (H / KH), wide = (dv + slices - 1) / slices, last = dv - (slices - 1) * wide, tok = lane & 15;
+  const int per_wide = 65535 / wide + 1, per_last = 65535 / last + 1;          // i / w = (i * per) >> 16 for i < 272, w <= 64
+  float* scratch = scratch_all[w];
+  // where this lane's two sums of tokens of one quarter go: lane = 16 * (quarter of two) + (0 .. 5: A of pairs, 6 .. 11: P of them, 12 .. 15: P of the diagonal)
+  const int idx = lane & 15, pair = idx < 6 ? idx : idx - 6;
+  const int pt = idx < 12 ? (0x332321 >> (4 * pair)) & 15 : idx - 12, pj = idx < 12 ? (0x211000 >> (4 * pair)) & 15 : idx - 12;
+  const int sum_at = ((lane >> 4) * 4 + pt) * LDP + (lane >> 4) * 4 + pj;
+  for (int tc = t0 + (int)blockIdx.z * DC_CHUNK; tc < t1; tc += (int)gridDim.z * DC_CHUNK) {
+    float k[DC_CHUNK], q[DC_CHUNK], gg[DC_CHUNK];              // tokens past the end are ones that change nothing
+    dc_fetch<MODE>(qn, kn, decay, tc, t1, h, kh, d, H, KH, dk, k, q, gg);
+    const float b = w == 0 && tc + tok < t1 ? beta[(int64_t)(tc + tok) * H + h] : 0.f;
+    // ---- quarters: 32 sums over 32 lanes at a time (halve the values with every exchange)
 #pragma unroll
-      for (int t = 0; t < DP_CHUNK; ++t) {
-        const bool ok = tc + t < t1 && tid < dk;
-        const int64_t src = ((int64_t)(tc + t) * KH + kh) * dk + tid;
-        pk[t] = ok ? kn[src] : 0.f;
-        pq[t] = ok ? qn[src] : 0.f;
-        if constexpr (MODE == 1) pg[t] = ok ? decay[((int64_t)(tc + t) * H + h) * dk + tid] : 1.f;
-        else pg[t] = tc + t < t1 ? decay[(int64_t)(tc + t) * H + h] : 1.f;
+    for (int half = 0; half < 2; ++half) {
+      float s[32];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int a = 8 * half + 4 * u;
+        const float w01 = k[a] * gg[a + 1], w02 = w01 * gg[a + 2], w03 = w02 * gg[a + 3], w12 = k[a + 1] * gg[a + 2], w13 = w12 * gg[a + 3],
+                    w23 = k[a + 2] * gg[a + 3];
+        const float ws[6] = {w01, w02, w03, w12, w13, w23};
+        const int to[6] = {1, 2, 3, 2, 3, 3};
+#pragma unroll
+        for (int i = 0; i < 6; ++i) s[16 * u + i] = k[a + to[i]] * ws[i], s[16 * u + 6 + i] = q[a + to[i]] * ws[i];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) s[16 * u + 12 + i] = q[a + i] * k[a + i];
       }
 #pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        const int idx = tid + r * DP_TEAM, t = idx / DP_COLS, c = blockIdx.z * DP_COLS + idx % DP_COLS;
-        pv[r] = tc + t < t1 && c < dv ? v[((int64_t)(tc + t) * H + h) * dv + c] : 0.f;
-      }
-      if (tid < DP_CHUNK) pb = tc + tid < t1 ? beta[(int64_t)(tc + tid) * H + h] : 0.f;
-    };
-    auto park = [&](int buf) {
-      const int at = tid + (tid >> 4) * 4;
-      float d[4 * PAIRS];
-#pragma unroll
-      for (int p = 0; p < PAIRS; ++p) {
-        const float g1 = pg[2 * p], g2 = pg[2 * p + 1], k1 = pk[2 * p], k2 = pk[2 * p + 1], q1 = pq[2 * p], q2 = pq[2 * p + 1];
-        const float gg = g1 * g2, kd = g2 * k1;
-        float (*w)[DP_LDK] = vec[buf][p];
-        w[K1][at] = g1 * k1;
-        w[K2][at] = gg * k2;
-        w[Q1][at] = g1 * q1;
-        w[Q2][at] = gg * q2;
-        w[GG][at] = gg;
-        w[KD][at] = kd;
-        w[KU][at] = k2;
-        d[4 * p] = k2 * kd;
-        d[4 * p + 1] = q1 * k1;
-        d[4 * p + 2] = q2 * kd;
-        d[4 * p + 3] = q2 * k2;
-      }
-      // 16 sums over 32 lanes: halve the values with every exchange, lane l ends up with sum (l >> 1)
-#pragma unroll
-      for (int n = 8, m = 16; n >= 1; n >>= 1, m >>= 1) {
+      for (int m = 16; m >= 1; m >>= 1) {
         const bool up = (lane & m) != 0;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          if (i >= n) continue;
-          const float give = up ? d[i] : d[n + i], keep = up ? d[n + i] : d[i];
-          d[i] = keep + __shfl_xor_sync(0xffffffffu, give, m);
+        for (int i = 0; i < 16; ++i) {
+          if (i >= m) continue;
+          const float give = up ? s[i] : s[m + i], keep = up ? s[m + i] : s[i];
+          s[i] = keep + __shfl_xor_sync(0xffffffffu, give, m);
         }
       }
-      d[0] += __shfl_xor_sync(0xffffffffu, d[0], 1);
-      if (!(lane & 1)) dots[buf][lane >> 3][(lane >> 1) & 3][warp] = d[0];
+      part[w][idx < 6 ? 0 : 1][sum_at + half * (8 * LDP + 8)] = s[0];
+    }
+    // ---- halves of the chunk, then the quarters of both halves: rows of k and q from the border on, rows of k up to it
 #pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        const int idx = tid + r * DP_TEAM;
-        vs[buf][idx / DP_COLS][idx % DP_COLS] = pv[r];
+    for (int level = 0; level < 2; ++level) {
+#pragma unroll
+      for (int u = 0; u < (level ? 2 : 1); ++u) {
+        const int len = level ? 4 : 8, at = level ? 8 * u + 4 : 8, r0 = level ? 4 * u : 0;
+        float c = 1.f;
+#pragma unroll
+        for (int i = 0; i < len; ++i) {
+          c *= gg[at + i];
+          scratch[(r0 + i) * LDR + lane] = k[at + i] * c;
+          scratch[(8 + r0 + i) * LDR + lane] = q[at + i] * c;
+        }
+        c = 1.f;
+#pragma unroll
+        for (int i = len - 1; i >= 0; --i) {
+          scratch[(16 + r0 + i) * LDR + lane] = k[at - len + i] * c;
+          c *= gg[at - len + i];
+        }
       }
-      if (tid < DP_CHUNK) bs[buf][tid] = pb;
-    };
-    fetch(t0);
-    park(0);
-    fetch(t0 + DP_CHUNK);
+      __syncwarp();
+      float acc[4] = {0.f, 0.f, 0.f, 0.f}, rest[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int ks = 0; ks < 4; ++ks) {
+        const float2 ak = *reinterpret_cast<const float2*>(scratch + g * LDR + 8 * ks + 2 * t);
+        const float2 aq = *reinterpret_cast<const float2*>(scratch + (8 + g) * LDR + 8 * ks + 2 * t);
+        const float2 bk = *reinterpret_cast<const float2*>(scratch + (16 + g) * LDR + 8 * ks + 2 * t);
+        const float r[4] = {ak.x, ak.y, aq.x, aq.y};
+        float hi[4], lo[4];
+        dc_operand(r, hi, lo);
+        float2 bh, bl;
+        dc_split(bk, bh, bl);
+        dc_mma(rest, lo, bh.x, bh.y);
+        dc_mma(acc, hi, bh.x, bh.y);
+        dc_mma(rest, hi, bl.x, bl.y);
+      }
+      const int i0 = g, j0 = 2 * t;                            // row of both kinds, columns j0, j0 + 1
+      if (level == 0 || (i0 >> 2) == (j0 >> 2)) {
+        const int at = level ? ((i0 >> 2) * 8 + 4 + (i0 & 3)) * LDP + (j0 >> 2) * 8 + (j0 & 3) : (8 + i0) * LDP + j0;
+        part[w][0][at] = acc[0] + rest[0];
+        part[w][0][at + 1] = acc[1] + rest[1];
+        part[w][1][at] = acc[2] + rest[2];
+        part[w][1][at + 1] = acc[3] + rest[3];
+      }
+      __syncwarp();
+    }
     __syncthreads();
-    int buf = 0;
-    for (int tc = t0; tc < t1; tc += DP_CHUNK, buf ^= 1) {      // (the other buffer was last read in the previous iteration)
-      if (tc + DP_CHUNK < t1) park(buf ^ 1);
-      if (tc + 2 * DP_CHUNK < t1) fetch(tc + 2 * DP_CHUNK);
-      __syncthreads();
+    if (w == 0) {                                              // lane: row of A (0 .. 15) or of P (16 .. 31), then column of the inverse
+      float r[16];
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        const int at = tok * LDP + j, kind = lane >> 4;
+        r[j] = (part[0][kind][at] + part[1][kind][at]) + (part[2][kind][at] + part[3][kind][at]);
+      }
+      if (lane >= 16) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j)
+          if (j <= tok) out[(tok + 1) * (tok + 1) + j] = r[j];
+      } else {
+#pragma unroll
+        for (int j = 0; j < 16; j += 4)
+          *reinterpret_cast<float4*>(tri + tok * 20 + j) = make_float4(j < tok ? b * r[j] : 0.f, j + 1 < tok ? b * r[j + 1] : 0.f,
+                                                                       j + 2 < tok ? b * r[j + 2] : 0.f, j + 3 < tok ? b * r[j + 3] : 0.f);
+      }
+      __syncwarp();
+      float x[16];                                             // column tok of (I + diag(b) A)^-1, by rows
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        float s[4] = {i == tok ? 1.f : 0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int j = 0; j < i; j += 4) {
+          const float4 l = *reinterpret_cast<const float4*>(tri + i * 20 + j);
+          s[0] = fmaf(-l.x, x[j], s[0]);
+          if (j + 1 < i) s[1] = fmaf(-l.y, x[j + 1], s[1]);
+          if (j + 2 < i) s[2] = fmaf(-l.z, x[j + 2], s[2]);
+          if (j + 3 < i) s[3] = fmaf(-l.w, x[j + 3], s[3]);
+        }
+        x[i] = (s[0] + s[1]) + (s[2] + s[3]);
+        if (lane <= i) out[i * (i + 1) + lane] = x[i] * b;     // (lane 16 .. 31: not below 16)
+      }
+    }
+    __syncthreads();
+    const int m = min(DC_CHUNK, t1 - tc), numbers = m * (m + 1);
+    for (int z = 0; z < slices; ++z) {
+      const int wz = z + 1 < slices ? wide : last;
+      float* dst = o + ((int64_t)tc * H + h) * dv + z * wide;
+      for (int i = d; i < numbers; i += DC_TEAM) {
+        const int r = (i * (z + 1 < slices ? per_wide : per_last)) >> 16;
+        dst[(int64_t)r * H * dv + (i - r * wz)] = out[i];
+      }
+    }
+    __syncthreads();
+  }
+}
+
+// The chain.  A CTA has up to 64 columns of a head.  Two warps keep S^T of 16 columns, half of the channels each, in the accumulators of m16n8k8 (rows: columns of
+// the state), which are the A operand of the next products as they are; nothing of the state passes through shared memory, the two exchange
+// their shares of the products with it.  Four more warps, a thread per key channel, scale the next chunks' vectors, split them and store them in the
+// order in which the MMAs read them; three buffers, named barriers, so that pairs of warps may drift apart and cover each other's latencies.
+// Bound: the tf32 MMAs (315 per chunk and scheduler, 8 cycles each: 2520 of about 4900) and the fp32 instructions, which sm_100 does not issue beside them:
+// a warp of mma.sync and one of FFMA on the same scheduler take the sum of their times (measured; integer instructions overlap by half).  So what
+// is left counts: vectors split once by the warps that scale them instead of by the four pairs that read them, 3 %; scalar subtractions instead of
+// packed ones, which hold the pipe for 2.4 cycles, 3 %; all channels in one warp (nothing beside its MMAs), 3.1 instead of 2.6 us per chunk; making T and P
+// here too, in both CTAs of a head, 12000 instructions per chunk, 4.4 us.
+// us, two tokens at a time in fp32 (the kernel before) -> now with the triangles, heads of 128 x 128, decays per channel / per head: 4 x 320 to 512 tokens, 16
+// heads 156 -> 101 / 153 -> 100, 32 heads 267 -> 191 / 261 -> 190; 16 x 250, 32 heads 464 -> 379 / 456 -> 375; 1 x 1000, 16 heads 290 -> 174; 1 x 32 16 -> 12.
+// An entry takes this path if it has at least DC_MIN tokens, whatever the others have (the exceptions: top of the file); a prompt whose portions are
+// shorter has the bits of single tokens, which differ in the last places.
+// One buffer, in floats: K~ and Q~ as [16 k steps][4 tiles of 8 tokens][8 tokens][8 channels] (k steps padded), K- as [16 tiles of 8 channels][2 k steps]
+// [8 channels][8 tokens] (halves of 4 tokens swapped in the upper 4 channels), blocks (0, 0), (1, 0), (1, 1) of T and of P as [8 tokens][8 tokens], and the
+// decays over the whole chunk
+constexpr int DC_STATE_WARPS = 8, DC_THREADS = 32 * DC_STATE_WARPS + DC_TEAM, DC_NBUF = 3;
+constexpr int DC_KS = 4 * 64 + 8, DC_KB = 16 * DC_KS, DC_LOW = DC_KB + 32 * 64, DC_TP = 2 * DC_LOW, DC_G = DC_TP + 6 * 64, DC_BUF = DC_G + 128;
+constexpr int DC_SWAP = DC_NBUF * DC_BUF;                      // [2][8 warps][3 pieces][32 lanes][4]
+constexpr int DC_SMEM = (DC_SWAP + 2 * DC_STATE_WARPS * 3 * 128) * 4;
+enum { DC_BAR_FULL = 1, DC_BAR_FREE = DC_BAR_FULL + DC_NBUF, DC_BAR_PAIR = DC_BAR_FREE + DC_NBUF };       // + buffer, + pair of warps
+
+__device__ __forceinline__ void dc_sync(int bar, int n) { asm volatile("barrier.cta.sync %0, %1;" ::"r"(bar), "r"(n) : "memory"); }
+__device__ __forceinline__ void dc_arrive(int bar, int n) { asm volatile("barrier.cta.arrive %0, %1;" ::"r"(bar), "r"(n) : "memory"); }
+struct DcTile { float x[2][4]; };                              // 16 columns of the state x 16 tokens, accumulator layout
+__device__ __forceinline__ float dc_nonfinite(const DcTile& a) {             // 0, or NaN if an element is not finite
+  float s[2] = {0.f, 0.f};
+#pragma unroll
+  for (int n = 0; n < 2; ++n)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) s[n] = fmaf(a.x[n][i], 0.f, s[n]);
+  return s[0] + s[1];
+}
+// columns 8 n .. 8 n + 7 of in . M^T, added to out, with the lower triangle M [16, 16]
+template <int N>
+__device__ __forceinline__ void dc_triangle(float (&out)[4], const float (&hi)[2][4], const float (&lo)[2][4], const float* m, int lane) {
+  float2 h0, l0;
+  dc_split(*reinterpret_cast<const float2*>(m + 64 * N + 2 * lane), h0, l0);
+  float s[4];                                                  // (chains of two or three)
+  dc_mma0(s, lo[0], h0.x, h0.y);
+  if constexpr (N == 1) {
+    float2 h1, l1;
+    float r[4];
+    dc_split(*reinterpret_cast<const float2*>(m + 128 + 2 * lane), h1, l1);
+    dc_mma0(r, lo[1], h1.x, h1.y);
+    dc_mma(s, hi[0], l0.x, l0.y);
+    dc_mma(r, hi[1], l1.x, l1.y);
+    dc_mma(s, hi[0], h0.x, h0.y);
+    dc_mma(r, hi[1], h1.x, h1.y);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) out[i] += s[i] + r[i];
+  } else {
+    dc_mma(s, hi[0], l0.x, l0.y);
+    dc_mma(s, hi[0], h0.x, h0.y);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) out[i] += s[i];
+  }
+}
+// The same for inputs that are not all finite: no product with the zeros above the diagonal, so a token's NaN or infinity reaches none before it.
+__device__ __noinline__ DcTile dc_triangle_masked(DcTile in, const float* m, int lane) {
+  const int t = lane & 3;
+  DcTile out = {};
+  for (int j = 0; j < 16; ++j) {
+    const int from = (lane & ~3) | ((j & 7) >> 1);
+    float x[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) x[i] = __shfl_sync(0xffffffffu, j < 8 ? in.x[0][i] : in.x[1][i], from);
+    const float xr[2] = {j & 1 ? x[1] : x[0], j & 1 ? x[3] : x[2]};
+#pragma unroll
+    for (int n = 0; n < 2; ++n)
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        const int tok = 8 * n + 2 * t + c;
+        if (tok < j) continue;
+        const float w = m[(n + (j >> 3)) * 64 + (tok & 7) * 8 + (j & 7)];
+        out.x[n][c] = fmaf(w, xr[0], out.x[n][c]);
+        out.x[n][c + 2] = fmaf(w, xr[1], out.x[n][c + 2]);
+      }
+  }
+  return out;
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(DC_THREADS, 1)
+delta_chunk_kernel(const float* __restrict__ qn, const float* __restrict__ kn, const float* __restrict__ v, const float* __restrict__ decay,
+                   float* __restrict__ state, const int32_t* __restrict__ cu, const int32_t* __restrict__ rows, const int32_t* __restrict__ lengths,
+                   float* o, int H, int KH, int dk, int dv, int least) {
+  extern __shared__ __align__(16) float dc_smem[];
+  const int e = blockIdx.x, h = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  pdl_launch_dependents();
+  const int t0 = cu[e], t1 = cu[e + 1];
+  if (t1 - t0 < least) return;
+  const int row = rows[e], kh = h / (H / KH), chunks = (t1 - t0 + DC_CHUNK - 1) / DC_CHUNK;
+  const int z0 = (int)blockIdx.z * ((dv + (int)gridDim.z - 1) / (int)gridDim.z), z1 = min(dv, z0 + (dv + (int)gridDim.z - 1) / (int)gridDim.z);
+  if (warp >= DC_STATE_WARPS) {
+    // ===================================== vectors =====================================
+    const int d = threadIdx.x - 32 * DC_STATE_WARPS;           // key channel
+    float k[DC_CHUNK], q[DC_CHUNK], gg[DC_CHUNK], tp[3];
+    // T and P: this thread's numbers d, d + 128, d + 256 of the packed rows
+    const float* tp_src[3];
+    int tp_dst[3], tp_tok[3];
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+      const int i = d + r * DC_TEAM, wz = z1 - z0;
+      int tt = 0;
+      while ((tt + 1) * (tt + 2) <= i) ++tt;                   // rows below tt have tt (tt + 1) numbers
+      const int in = i - tt * (tt + 1), p = in > tt ? 1 : 0, j = in - p * (tt + 1);
+      tp_tok[r] = i < DC_CHUNK * (DC_CHUNK + 1) ? tt : 1 << 30;
+      tp_dst[r] = DC_TP + (3 * p + (tt >> 3) + (j >> 3)) * 64 + (tt & 7) * 8 + (j & 7);
+      tp_src[r] = o + ((int64_t)(t0 + i / wz) * H + h) * dv + z0 + i % wz;
+    }
+    auto fetch = [&](int tc) {
+      dc_fetch<MODE>(qn, kn, decay, tc, t1, h, kh, d, H, KH, dk, k, q, gg);
+#pragma unroll
+      for (int r = 0; r < 3; ++r) tp[r] = tc + tp_tok[r] < t1 ? tp_src[r][(int64_t)(tc - t0) * H * dv] : 0.f;
+    };
+    for (int i = d; i < DC_NBUF * 6 * 64; i += DC_TEAM) dc_smem[(i / 384) * DC_BUF + DC_TP + i % 384] = 0.f;       // (above the diagonal it stays so)
+    pdl_wait();                                                // T and P
+    fetch(t0);
+    dc_sync(DC_BAR_FREE, DC_TEAM);                             // (the zeros before the numbers)
+    for (int n = 0; n < chunks; ++n) {
+      const int buf = n % DC_NBUF;
+      float* b = dc_smem + buf * DC_BUF;
+      if (n >= DC_NBUF) dc_sync(DC_BAR_FREE + buf, DC_THREADS);
+      {                                                        // K~ = -G_t k_t and Q~ = G_t q_t
+        float c = 1.f;
+        float* dst = b + (d >> 3) * DC_KS + (d & 7);
+#pragma unroll
+        for (int i = 0; i < DC_CHUNK; ++i) {
+          c *= gg[i];
+          const float x = -k[i] * c, y = q[i] * c, hx = dc_high(x), hy = dc_high(y);
+          dst[i * 8] = hx, dst[DC_LOW + i * 8] = x - hx;
+          dst[128 + i * 8] = hy, dst[DC_LOW + 128 + i * 8] = y - hy;
+        }
+        b[DC_G + d] = c;
+      }
+      {                                                        // K- = (G / G_j) k_j
+        float c = 1.f;
+        float* dst = b + DC_KB + (d >> 3) * 128 + (d & 7) * 8;
+#pragma unroll
+        for (int i = DC_CHUNK - 4; i >= 0; i -= 4) {
+          float4 x;
+          x.w = k[i + 3] * c, c *= gg[i + 3];
+          x.z = k[i + 2] * c, c *= gg[i + 2];
+          x.y = k[i + 1] * c, c *= gg[i + 1];
+          x.x = k[i] * c, c *= gg[i];
+          const float4 xh = make_float4(dc_high(x.x), dc_high(x.y), dc_high(x.z), dc_high(x.w));
+          float* at = dst + (i >> 3) * 64 + 4 * (((i >> 2) & 1) ^ ((d >> 2) & 1));
+          *reinterpret_cast<float4*>(at) = xh;
+          *reinterpret_cast<float4*>(at + DC_LOW) = make_float4(x.x - xh.x, x.y - xh.y, x.z - xh.z, x.w - xh.w);
+        }
+      }
+#pragma unroll
+      for (int r = 0; r < 3; ++r)
+        if (tp_tok[r] < DC_CHUNK) b[tp_dst[r]] = tp[r];
+      dc_arrive(DC_BAR_FULL + buf, DC_THREADS);
+      if (n + 1 < chunks) fetch(t0 + (n + 1) * DC_CHUNK);
     }
     return;
   }
-  if constexpr (PER_SM == 2) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(DP_REGS_COMPUTE));
-  // ===================================== recurrence ==================================
-  const int l = tid & 7, slot = tid >> 3, j0 = blockIdx.z * DP_COLS + 4 * slot;    // this thread's columns j0 .. j0 + 3, rows 16 l .. 16 l + 15
-  const bool vec4 = (dv & 3) == 0 && (reinterpret_cast<uintptr_t>(state) & 15) == 0 && j0 + 3 < dv;
-  float* sp = state + (((int64_t)row * H + h) * dk + 16 * l) * dv + j0;
-  const bool fresh = lengths[row] == 0;
-  float2 S[4][8];                                              // [column][row pair]
+  // ===================================== state =======================================
+  const int half = warp & 1, pair = warp >> 1;                 // 64 of the channels, 16 of the columns
+  const int ja = z0 + 16 * pair + g, jb = ja + 8;              // this lane's columns of the state (rows of the fragments)
+  const bool la = ja < z1, lb = jb < z1;
+  float* sp = state + (((int64_t)row * H + h) * dk + 64 * half) * dv;
+  const bool fresh = lengths[row] == 0;                        // first token of a sequence: the state starts at zero
+  float S[8][4];                                               // [8 channels][(column a, channels 2 t, 2 t + 1), (column b, the same)]
 #pragma unroll
-  for (int i = 0; i < 8; ++i)
+  for (int n = 0; n < 8; ++n)
 #pragma unroll
-    for (int b = 0; b < 2; ++b) {
-      const int r = 2 * i + b;
-      float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (!fresh && 16 * l + r < dk) {
-        const float* s0 = sp + (int64_t)r * dv;
-        if (vec4) x = *reinterpret_cast<const float4*>(s0);
-        else {
-          if (j0 < dv) x.x = s0[0];
-          if (j0 + 1 < dv) x.y = s0[1];
-          if (j0 + 2 < dv) x.z = s0[2];
-          if (j0 + 3 < dv) x.w = s0[3];
-        }
-      }
-      (b ? S[0][i].y : S[0][i].x) = x.x;
-      (b ? S[1][i].y : S[1][i].x) = x.y;
-      (b ? S[2][i].y : S[2][i].x) = x.z;
-      (b ? S[3][i].y : S[3][i].x) = x.w;
+    for (int c = 0; c < 2; ++c) {
+      const int r = 8 * n + 2 * t + c;
+      const bool in = !fresh && 64 * half + r < dk;
+      S[n][c] = in && la ? sp[(int64_t)r * dv + ja] : 0.f;
+      S[n][2 + c] = in && lb ? sp[(int64_t)r * dv + jb] : 0.f;
     }
-  const int jo = j0 + (l & 3);                                 // the column whose outputs this lane writes
-  __syncthreads();
-  int buf = 0;
-  for (int tc = t0; tc < t1; tc += DP_CHUNK, buf ^= 1) {
-    auto step = [&](int p) {
-      const float* w = &vec[buf][p][0][20 * l];
-      // this thread's rows of two dot products with the four columns
-      auto dot2 = [&](int s0, float (&r1)[4], float (&r2)[4]) {
-        float2 a[2][4];
+  DcTile vn;                                                   // the next chunk's values
+  auto fetch_v = [&](int tc) {
 #pragma unroll
-        for (int c = 0; c < 4; ++c) a[0][c] = a[1][c] = make_float2(0.f, 0.f);
+    for (int n = 0; n < 2; ++n)
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-          for (int s = 0; s < 2; ++s) {
-            const float4 x = *reinterpret_cast<const float4*>(w + (s0 + s) * DP_LDK + 4 * i);
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-              a[s][c] = __ffma2_rn(S[c][2 * i], make_float2(x.x, x.y), a[s][c]);
-              a[s][c] = __ffma2_rn(S[c][2 * i + 1], make_float2(x.z, x.w), a[s][c]);
-            }
-          }
-#pragma unroll
-        for (int c = 0; c < 4; ++c) r1[c] = a[0][c].x + a[0][c].y, r2[c] = a[1][c].x + a[1][c].y;
-      };
-      // over the eight lanes: lane l < 4 gets the first product's sum of column l, lane l + 4 the second's
-      auto reduce = [&](const float (&r1)[4], const float (&r2)[4]) {
-        const bool b4 = (l & 4) != 0, b2 = (l & 2) != 0, b1 = (l & 1) != 0;
-        float r[4];
-#pragma unroll
-        for (int c = 0; c < 4; ++c) r[c] = (b4 ? r2[c] : r1[c]) + __shfl_xor_sync(0xffffffffu, b4 ? r1[c] : r2[c], 4);
-#pragma unroll
-        for (int c = 0; c < 2; ++c) r[c] = (b2 ? r[c + 2] : r[c]) + __shfl_xor_sync(0xffffffffu, b2 ? r[c] : r[c + 2], 2);
-        return (b1 ? r[1] : r[0]) + __shfl_xor_sync(0xffffffffu, b1 ? r[0] : r[1], 1);
-      };
-      float r1[4], r2[4], y1[4], y2[4];
-      dot2(K1, r1, r2);
-      const float sk = reduce(r1, r2);
-      dot2(Q1, y1, y2);                                        // (beside the exchanges of the sums for u)
-      auto dot_of = [&](int d) {
-        const float4 x = *reinterpret_cast<const float4*>(dots[buf][p][d]);
-        return (x.x + x.y) + (x.z + x.w);
-      };
-      const float k2kd = dot_of(0), q1k1 = dot_of(1), q2kd = dot_of(2), q2k2 = dot_of(3), b1 = bs[buf][2 * p], b2 = bs[buf][2 * p + 1];
-      const float4 v1 = *reinterpret_cast<const float4*>(&vs[buf][2 * p][4 * slot]), v2 = *reinterpret_cast<const float4*>(&vs[buf][2 * p + 1][4 * slot]);
-      const float va[4] = {v1.x, v1.y, v1.z, v1.w}, vb[4] = {v2.x, v2.y, v2.z, v2.w};
-      float u1[4], u2[4];
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        const float s1 = __shfl_sync(0xffffffffu, sk, c, 8), s2 = __shfl_sync(0xffffffffu, sk, c + 4, 8);
-        u1[c] = b1 * (va[c] - s1);
-        u2[c] = b2 * (vb[c] - fmaf(k2kd, u1[c], s2));
+      for (int c = 0; c < 2; ++c) {
+        const int tok = tc + 8 * n + 2 * t + c;
+        const float* src = v + ((int64_t)tok * H + h) * dv;
+        vn.x[n][c] = tok < t1 && la ? src[ja] : 0.f;
+        vn.x[n][2 + c] = tok < t1 && lb ? src[jb] : 0.f;
       }
+  };
+  fetch_v(t0);
+  for (int n = 0; n < chunks; ++n) {
+    const int buf = n % DC_NBUF, tc = t0 + n * DC_CHUNK;
+    const float* b = dc_smem + buf * DC_BUF;
+    float4* swap = reinterpret_cast<float4*>(dc_smem + DC_SWAP) + (n & 1) * (DC_STATE_WARPS * 3 * 32) + lane;
+    float sum[4][4], rest[4][4];                               // -S^T K~ of tokens 0 .. 7, 8 .. 15, S^T Q~ of both
+#pragma unroll
+    for (int m = 0; m < 4; ++m)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) sum[m][i] = rest[m][i] = 0.f;
+    dc_sync(DC_BAR_FULL + buf, DC_THREADS);
+#pragma unroll
+    for (int k4 = 0; k4 < 2; ++k4) {
+      float acc[4][4];
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        const float4 g = *reinterpret_cast<const float4*>(w + GG * DP_LDK + 4 * i), kd = *reinterpret_cast<const float4*>(w + KD * DP_LDK + 4 * i);
-        const float4 ku = *reinterpret_cast<const float4*>(w + KU * DP_LDK + 4 * i);
+        const int ks = 4 * k4 + i;
+        float hi[4], lo[4];
+        float2 bh[4], bl[4];
+        dc_operand(S[ks], hi, lo);
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          const float2 ua = make_float2(u1[c], u1[c]), ub = make_float2(u2[c], u2[c]);
-          S[c][2 * i] = __ffma2_rn(make_float2(ku.x, ku.y), ub, __ffma2_rn(make_float2(kd.x, kd.y), ua, __fmul2_rn(S[c][2 * i], make_float2(g.x, g.y))));
-          S[c][2 * i + 1] = __ffma2_rn(make_float2(ku.z, ku.w), ub, __ffma2_rn(make_float2(kd.z, kd.w), ua, __fmul2_rn(S[c][2 * i + 1], make_float2(g.z, g.w))));
+        for (int m = 0; m < 4; ++m) {
+          const float* at = b + (8 * half + ks) * DC_KS + m * 64 + 2 * lane;
+          bh[m] = *reinterpret_cast<const float2*>(at), bl[m] = *reinterpret_cast<const float2*>(at + DC_LOW);
         }
-      }
-      const float sq = reduce(y1, y2);                         // (beside the update)
-      const bool c2 = (l & 2) != 0, c1 = (l & 1) != 0;
-      const float ua = c2 ? (c1 ? u1[3] : u1[2]) : (c1 ? u1[1] : u1[0]), ub = c2 ? (c1 ? u2[3] : u2[2]) : (c1 ? u2[1] : u2[0]);
-      const float out = l < 4 ? fmaf(q1k1, ua, sq) : fmaf(q2k2, ub, fmaf(q2kd, ua, sq));
-      const int t = tc + 2 * p + (l >> 2);
-      if (jo < dv && t < t1) o[((int64_t)t * H + h) * dv + jo] = out;
-    };
-    if (t1 - tc >= DP_CHUNK) {
 #pragma unroll
-      for (int p = 0; p < PAIRS; ++p) step(p);
-    } else {
-#pragma unroll 1
-      for (int p = 0; tc + 2 * p < t1; ++p) step(p);
+        for (int m = 0; m < 4; ++m)
+          if (i == 0) dc_mma0(acc[m], hi, bh[m].x, bh[m].y);
+          else dc_mma(acc[m], hi, bh[m].x, bh[m].y);
+#pragma unroll
+        for (int m = 0; m < 4; ++m) dc_mma(rest[m], hi, bl[m].x, bl[m].y);
+#pragma unroll
+        for (int m = 0; m < 4; ++m) dc_mma(rest[m], lo, bh[m].x, bh[m].y);
+      }
+#pragma unroll
+      for (int m = 0; m < 4; ++m)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) sum[m][i] += acc[m][i];
     }
-    __syncthreads();
+#pragma unroll
+    for (int m = 0; m < 4; ++m)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) sum[m][i] += rest[m][i];
+    // ---- the other half of the channels; this warp writes the outputs of tokens 8 half .. 8 half + 7
+    float4* mine = swap + warp * 96;
+    const float4* theirs = swap + (warp ^ 1) * 96;
+    const float (&give)[4] = half ? sum[2] : sum[3];
+    mine[0] = make_float4(sum[0][0], sum[0][1], sum[0][2], sum[0][3]);
+    mine[32] = make_float4(sum[1][0], sum[1][1], sum[1][2], sum[1][3]);
+    mine[64] = make_float4(give[0], give[1], give[2], give[3]);
+    dc_sync(DC_BAR_PAIR + pair, 64);
+    DcTile X, U;
+    float out[4];
+#pragma unroll
+    for (int m = 0; m < 2; ++m) {
+      const float4 x = theirs[32 * m];
+      X.x[m][0] = vn.x[m][0] + (sum[m][0] + x.x), X.x[m][1] = vn.x[m][1] + (sum[m][1] + x.y);
+      X.x[m][2] = vn.x[m][2] + (sum[m][2] + x.z), X.x[m][3] = vn.x[m][3] + (sum[m][3] + x.w);
+      U.x[m][0] = U.x[m][1] = U.x[m][2] = U.x[m][3] = 0.f;
+    }
+    {
+      const float4 x = theirs[64];
+      out[0] = (half ? sum[3][0] : sum[2][0]) + x.x, out[1] = (half ? sum[3][1] : sum[2][1]) + x.y;
+      out[2] = (half ? sum[3][2] : sum[2][2]) + x.z, out[3] = (half ? sum[3][3] : sum[2][3]) + x.w;
+    }
+    if (n + 1 < chunks) fetch_v(tc + DC_CHUNK);
+    // ---- U = T X, O += P U
+    float hi[2][4], lo[2][4];
+    if (__any_sync(0xffffffffu, dc_nonfinite(X) != 0.f)) {
+      U = dc_triangle_masked(X, b + DC_TP, lane);
+    } else {
+      dc_operand(X.x[0], hi[0], lo[0]);
+      dc_operand(X.x[1], hi[1], lo[1]);
+      dc_triangle<0>(U.x[0], hi, lo, b + DC_TP, lane);
+      dc_triangle<1>(U.x[1], hi, lo, b + DC_TP, lane);
+    }
+    dc_operand(U.x[0], hi[0], lo[0]);
+    dc_operand(U.x[1], hi[1], lo[1]);
+    if (__any_sync(0xffffffffu, dc_nonfinite(U) != 0.f)) {
+      const DcTile m = dc_triangle_masked(U, b + DC_TP + 3 * 64, lane);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) out[i] += half ? m.x[1][i] : m.x[0][i];
+    } else if (half) {
+      dc_triangle<1>(out, hi, lo, b + DC_TP + 3 * 64, lane);
+    } else {
+      dc_triangle<0>(out, hi, lo, b + DC_TP + 3 * 64, lane);
+    }
+    // ---- S <- G S + K- U
+    const float* kb = b + DC_KB + half * (8 * 128) + g * 8 + 4 * ((t >> 1) ^ (g >> 2)) + 2 * (t & 1);
+#pragma unroll
+    for (int m0 = 0; m0 < 8; m0 += 4) {                        // (four sums at a time cover each other's latencies)
+      float acc[4][4];
+      float2 h0[4], l0[4], h1[4], l1[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float* at = kb + (m0 + i) * 128;
+        h0[i] = *reinterpret_cast<const float2*>(at), l0[i] = *reinterpret_cast<const float2*>(at + DC_LOW);
+        h1[i] = *reinterpret_cast<const float2*>(at + 64), l1[i] = *reinterpret_cast<const float2*>(at + DC_LOW + 64);
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) dc_mma0(acc[i], lo[0], h0[i].x, h0[i].y);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) dc_mma(acc[i], hi[0], l0[i].x, l0[i].y);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) dc_mma(acc[i], lo[1], h1[i].x, h1[i].y);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) dc_mma(acc[i], hi[1], l1[i].x, l1[i].y);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) dc_mma(acc[i], hi[0], h0[i].x, h0[i].y);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) dc_mma(acc[i], hi[1], h1[i].x, h1[i].y);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float2 c = *reinterpret_cast<const float2*>(b + DC_G + 64 * half + 8 * (m0 + i) + 2 * t);
+        float (&x)[4] = S[m0 + i];
+        const float2 p = __ffma2_rn(make_float2(x[0], x[1]), c, make_float2(acc[i][0], acc[i][1]));
+        const float2 r = __ffma2_rn(make_float2(x[2], x[3]), c, make_float2(acc[i][2], acc[i][3]));
+        x[0] = p.x, x[1] = p.y, x[2] = r.x, x[3] = r.y;
+      }
+    }
+    if (n + DC_NBUF < chunks) dc_arrive(DC_BAR_FREE + buf, DC_THREADS);
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      const int tok = tc + 8 * half + 2 * t + c;
+      float* dst = o + ((int64_t)tok * H + h) * dv;
+      if (tok < t1 && la) dst[ja] = out[c];
+      if (tok < t1 && lb) dst[jb] = out[2 + c];
+    }
   }
 #pragma unroll
-  for (int i = 0; i < 8; ++i)
+  for (int n = 0; n < 8; ++n)
 #pragma unroll
-    for (int b = 0; b < 2; ++b) {
-      const int r = 2 * i + b;
-      if (16 * l + r >= dk) continue;
-      const float4 x = b ? make_float4(S[0][i].y, S[1][i].y, S[2][i].y, S[3][i].y) : make_float4(S[0][i].x, S[1][i].x, S[2][i].x, S[3][i].x);
-      float* s0 = sp + (int64_t)r * dv;
-      if (vec4) *reinterpret_cast<float4*>(s0) = x;
-      else {
-        if (j0 < dv) s0[0] = x.x;
-        if (j0 + 1 < dv) s0[1] = x.y;
-        if (j0 + 2 < dv) s0[2] = x.z;
-        if (j0 + 3 < dv) s0[3] = x.w;
-      }
+    for (int c = 0; c < 2; ++c) {
+      const int r = 8 * n + 2 * t + c;
+      if (64 * half + r >= dk) continue;
+      if (la) sp[(int64_t)r * dv + ja] = S[n][c];
+      if (lb) sp[(int64_t)r * dv + jb] = S[n][2 + c];
     }
 }
 
@@ -957,40 +1266,50 @@ extern "C" int b200p_delta_conv_commit(const float* proj, int64_t ldp, float* co
 
 // tokens: of all entries together, longest: of the longest; 0 if the caller does not say.
 template <int MODE>
-static void delta_scan_launch(int64_t tokens, int64_t longest, int nb, cudaStream_t st, const float* qn, const float* kn, const float* v, const float* beta,
+static cudaError_t delta_scan_launch(int64_t tokens, int64_t longest, int nb, cudaStream_t st, const float* qn, const float* kn, const float* v, const float* beta,
                               const float* decay, float* state, const int32_t* cu, const int32_t* rows, const int32_t* lengths,
                               float* o, int H, int KH, int dk, int dv) {
 #define DELTA_STEP(DKP)                                                                                                          \
   delta_step_kernel<DKP, MODE><<<dim3((unsigned)nb, (unsigned)H, (unsigned)((dv + dt_cols(DKP) - 1) / dt_cols(DKP))), DT_THREADS, 0, st>>>( \
       qn, kn, v, beta, decay, state, cu, rows, lengths, o, H, KH, dk, dv)
 #define DELTA_SCAN(DKP, LANES, PER_SM)                                                                                           \
-  launch_pdl_opt(pairs && pdl_enabled_gemm(), delta_scan_kernel<DKP, MODE, LANES, PER_SM>,                                        \
+  launch_pdl_opt(chunks && pdl_enabled_gemm(), delta_scan_kernel<DKP, MODE, LANES, PER_SM>,                                        \
                  dim3((unsigned)nb, (unsigned)H, (unsigned)((dv + 2 * ds_slots(DKP) - 1) / (2 * ds_slots(DKP)))), dim3(LANES * ds_slots(DKP)), 0, st, \
-                 qn, kn, v, beta, decay, state, cu, rows, lengths, o, H, KH, dk, dv, pairs ? DP_MIN - 1 : INT32_MAX)
+                 qn, kn, v, beta, decay, state, cu, rows, lengths, o, H, KH, dk, dv, chunks ? least - 1 : INT32_MAX)
   // The step kernel for decode steps, and for as many tokens per entry as it keeps up with the scan (us, step / scan): 128 x 128, 16
   // entries of 1 / 2 / 4 tokens, 32 heads, 21.7 / 23.1, 27.1 / 25.3, 32.0 / 29.2; 64 x 64, 32 heads, of 2 / 4 / 8, 6.8 / 8.8, 7.9 / 9.6,
   // 10.2 / 11.4, but with 16 heads 4.3 / 4.6, 5.1 / 5.0, 7.3 / 6.4; 32 x 64, 16 heads, of 2 / 4, 3.4 / 3.5, 4.2 / 3.9; 256 x 256, 8 heads,
   // 4 entries of 16 / 64, 20 / 20, 58 / 50.
   // The plain accumulation of keys above 128 takes it at any length (16 x 250 tokens of 256 x 256: 407 / 678; 4 x 512: 315 / 309).
   const int most = dk > 128 ? 8 : dk > 64 ? 1 : dk > 32 ? 4 : 2;
-  const bool by_pairs = MODE != 2 && dk > 64 && dk <= 128;                   // entries of DP_MIN tokens and more
-  const bool few = (tokens > 0 && tokens <= most * (int64_t)nb && !(by_pairs && longest >= DP_MIN)) || (MODE == 2 && dk > 128);
+  const bool by_chunks = MODE != 2 && dk > 64 && dk <= 128 && dv >= DC_MIN_DV && o != v;                   // entries of DC_MIN tokens and more
+  const bool few = (tokens > 0 && tokens <= most * (int64_t)nb && !(by_chunks && longest >= DC_MIN)) || (MODE == 2 && dk > 128);
   // 128 rows: one CTA per SM takes eight lanes per column and the shortest chain (4 x 512 tokens, 16 heads, decays per channel / per
   // head: 220 / 193 us, the former four-lane kernel 280 / 206); more CTAs than SMs take four (32 heads 379 / 346 -> 356 / 317; 16 x 250
   // tokens 672 / 594 -> 637 / 544).
   const bool crowded = (int64_t)nb * H * ((dv + 63) / 64) > sm_count();
-  // Entries of DP_MIN tokens and more two tokens at a time, the shorter ones by the launch behind it, which needs nothing of it: it may start at
+  // Entries of DC_MIN tokens and more in chunks (into values of more than 16 columns, other than v's own memory: o holds T and P), the shorter ones by the launch behind it, which needs nothing of it: it may start at
   // once (its inputs were complete when the first began), and one of its CTAs waits for the first launch, so that what follows waits for both.
   // (Only one: with every CTA waiting, those that do not fit beside the first launch started when it had ended: 15 entries of one token and one
   // of 40, 32 heads, decays per head / channel 43.7 / 45.7 -> 30 / 30.5 us, the scan alone 38 / 42.)  The long ones first: the short ones of such a
   // batch come with their tail.  A call that knows its longest entry to be short is spared the first launch: 16 entries of 4 tokens, 16 heads 14.4 ->
   // 13.3 us.
-  const bool pairs = by_pairs && !few && (tokens == 0 || tokens >= DP_MIN) && (longest == 0 || longest >= DP_MIN);
+  const bool chunks = by_chunks && !few && (tokens == 0 || tokens >= DC_MIN) && (longest == 0 || longest >= DC_MIN);
+  // Beside the chunk kernel's CTAs, which take an SM's registers, the token-by-token ones find no room: a call that knows of an entry of DC_MIN tokens
+  // takes those down to one chunk along (us, start / one launch behind the other / along: 40, 35, 30, 25 tokens, 32 heads 28.4 / 40.8 / 28.0, 48 to 27 tokens,
+  // eight entries of 16 heads 32 / 41.6 / 28.5); below that a single entry gains nothing (20 tokens 12.6 / 12.9).
+  const int least = longest >= DC_MIN ? DC_CHUNK : DC_MIN;
   if constexpr (MODE != 2) {
-    const auto pair_kernel = crowded ? delta_pair_kernel<MODE, 2> : delta_pair_kernel<MODE, 1>;
-    if (pairs)
-      pair_kernel<<<dim3((unsigned)nb, (unsigned)H, (unsigned)((dv + DP_COLS - 1) / DP_COLS)), DP_THREADS, 0, st>>>(
-          qn, kn, v, beta, decay, state, cu, rows, lengths, o, H, KH, dk, dv);
+    if (chunks) {
+      static const cudaError_t ready = cudaFuncSetAttribute(delta_chunk_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, DC_SMEM);
+      if (ready != cudaSuccess) return ready;
+      const unsigned slices = (unsigned)((dv + DC_COLS - 1) / DC_COLS), most = (unsigned)(longest ? (longest + DC_CHUNK - 1) / DC_CHUNK : 16);
+      delta_triangle_kernel<MODE><<<dim3((unsigned)nb, (unsigned)H, most < 1024 ? most : 1024), DC_TEAM, 0, st>>>(qn, kn, beta, decay, cu, o, H, KH, dk, dv, (int)slices,
+                                                                                                                 least);
+      const cudaError_t e = launch_pdl_opt(pdl_enabled_gemm(), delta_chunk_kernel<MODE>, dim3((unsigned)nb, (unsigned)H, slices), dim3(DC_THREADS), DC_SMEM, st,
+                                           qn, kn, v, decay, state, cu, rows, lengths, o, H, KH, dk, dv, least);
+      if (e != cudaSuccess) return e;
+    }
   }
   if (dk > 256) { if (few) DELTA_STEP(512); else DELTA_SCAN(512, 16, 1); }
   else if (dk > 128) { if (few) DELTA_STEP(256); else DELTA_SCAN(256, 8, 1); }
@@ -999,6 +1318,7 @@ static void delta_scan_launch(int64_t tokens, int64_t longest, int nb, cudaStrea
   else { if (few) DELTA_STEP(32); else DELTA_SCAN(32, 4, 1); }
 #undef DELTA_STEP
 #undef DELTA_SCAN
+  return cudaSuccess;
 }
 
 extern "C" int b200p_delta_scan_entries(const float* qn, const float* kn, const float* v, const float* beta, const float* decay,
@@ -1012,7 +1332,8 @@ extern "C" int b200p_delta_scan_entries(const float* qn, const float* kn, const 
   B200P_REQUIRE(dk <= 512, B200P_ERR_ARG, "key size %d > 512 is not built", dk);
   cudaStream_t st = (cudaStream_t)stream;
   const auto launch = mode == B200P_SCAN_DELTA ? delta_scan_launch<0> : mode == B200P_SCAN_DELTA_CHANNEL ? delta_scan_launch<1> : delta_scan_launch<2>;
-  launch(tokens, longest, nb, st, qn, kn, v, beta, decay, state, cu, rows, lengths, o, H, KH, dk, dv);
+  if (const cudaError_t e = launch(tokens, longest, nb, st, qn, kn, v, beta, decay, state, cu, rows, lengths, o, H, KH, dk, dv))
+    return cuda_fail(e, "delta_chunk_kernel");
   B200P_LAUNCH_CHECK("delta_scan_kernel");
   return B200P_OK;
 }

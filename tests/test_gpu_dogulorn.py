@@ -728,7 +728,7 @@ def test_delta_scan_of_decode_steps_equals_the_scan_of_prompts(mode, dk, dv, H, 
 @pytest.mark.parametrize("mode", [0, 1])
 @pytest.mark.parametrize("dk,dv,H,KH,shift", [(128, 128, 4, 2, 0), (65, 31, 2, 1, 0), (100, 66, 4, 4, 1), (128, 192, 2, 2, 1)])
 def test_delta_scan_of_long_entries(mode, dk, dv, H, KH, shift):
-    """Entries of 32 tokens and more go two tokens at a time: against a float64 loop, odd lengths, lengths around the border, carried and fresh
+    """Entries of 32 tokens and more go in chunks: against a float64 loop, odd lengths, lengths around the border, carried and fresh
     states, widths and addresses that forbid 16-byte accesses; an entry's bits are the same alone and among others, short and long."""
     from mlx_parallm_b200 import _lib
     lens = [32, 33, 31, 1, 71, 0]
@@ -912,6 +912,48 @@ def test_delta_scan_of_long_entries_among_short_ones(mode, lens, H):
         state.zero_()
     assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
     assert (got[0][0] - got[2][0]).abs().max() < 4e-5 and (got[0][1] - got[2][1]).abs().max() < 4e-5        # (2e-5 each: the test above)
+
+
+@pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("dk,dv,in_place", [(128, 16, False), (128, 17, False), (72, 64, False), (128, 129, False), (128, 128, True)])
+def test_delta_scan_in_chunks(mode, dk, dv, in_place):
+    """Entries of 32 tokens and more, 16 at a time, against float64 with the recurrence's fp32 bound (the test of long entries): last chunks of 1, 15 and 16
+    tokens, the narrowest outputs that hold a chunk's intermediate numbers and the widest that do not, outputs in the memory of v, decays of zero and
+    of 1e-30 (quotients of decays would be infinite); a key of NaN reaches no token before it and no other entry."""
+    from mlx_parallm_b200 import ops
+    H, KH, lens, bad = 2, 1, [33, 48, 63, 47], 20
+    g, nb, M = torch.Generator(device="cuda").manual_seed(dk + dv + mode), len(lens), sum(lens)
+    rnd = lambda *sh: torch.randn(*sh, generator=g, device="cuda")        # noqa: E731
+    nd = dk if mode else 1
+    qn, kn, v = rnd(M, KH * dk) / dk ** 0.5, torch.nn.functional.normalize(rnd(M, KH, dk), dim=-1).reshape(M, -1).contiguous(), rnd(M, H * dv)
+    beta, decay = torch.rand(M, H, generator=g, device="cuda"), 0.5 + 0.5 * torch.rand(M, H * nd, generator=g, device="cuda")
+    decay[5::11, ::3], decay[7::13, ::2] = 0.0, 1e-30
+    i32, off = dict(dtype=torch.int32, device="cuda"), [0]
+    for n in lens:
+        off.append(off[-1] + n)
+    cu, rows, lengths, state0 = torch.tensor(off, **i32), torch.arange(nb, **i32), torch.full((nb,), 3, **i32), rnd(nb, H, dk, dv) * 0.3
+
+    def scan(kn):
+        state, vals = state0.clone(), v.clone()
+        o = vals if in_place else torch.empty(M, H * dv, device="cuda")
+        ops.delta_scan(qn, kn, vals, beta, decay, state, cu, rows, lengths, o, nb, H, KH, dk, dv, mode, longest=max(lens))
+        return o, state
+
+    o, state = scan(kn)
+    for e in range(nb):
+        S = state0[e].double()
+        for t in range(off[e], off[e + 1]):
+            S = S * decay[t].double().view(H, -1, 1)
+            u = beta[t].double().unsqueeze(1) * (v[t].double().view(H, dv) - torch.einsum("hkv,k->hv", S, kn[t].double()))
+            S = S + kn[t].double().view(1, dk, 1) * u.unsqueeze(1)
+            assert (o[t].double() - torch.einsum("hkv,k->hv", S, qn[t].double()).reshape(-1)).abs().max() < 2e-5
+        assert (state[e].double() - S).abs().max() < 2e-5
+    spoilt = kn.clone()
+    spoilt[off[1] + bad, 3] = float("nan")
+    o2, state2 = scan(spoilt)
+    keep = [t for t in range(M) if not off[1] + bad <= t < off[2]]
+    assert (o2[keep] - o[keep]).abs().max() < 2e-5 and o2[off[1] + bad:off[2]].isnan().all()
+    assert torch.equal(state2[[0, 2, 3]], state[[0, 2, 3]]) and state2[1].isnan().any()
 
 
 @pytest.mark.parametrize("M,N,K,batch", [(1, 64, 128, 9), (2, 512, 128, 16), (5, 128, 512, 64), (8, 130, 512, 3), (3, 128, 1024, 40), (1, 128, 520, 64)])
