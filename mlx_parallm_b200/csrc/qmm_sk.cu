@@ -11,6 +11,8 @@
 //   * every segment (whole tile or not) leaves through shared memory and ONE cp.reduce.async.bulk.tensor (.add.f32) per
 //     [16 tokens x 128 rows] staging tile: partial tiles of different CTAs are summed by the L2 atomic units, nothing is
 //     waited for, there is no workspace and no tail.  Sums are NOT taken in a fixed order (fp32 adds of <= 148 partials).
+// Up to 96 tokens the roles hand over units of two k-blocks at 4 bits, as there (us at 24 / 64 tokens: 5120 x 17408 17.2 -> 15.4 / 17.7 -> 16.3, 4096 x 14336
+// 12.9 -> 11.8 / 14.1 -> 13.4).
 // Measured against the whole-tile kernel's K split through the workspace: o_proj M=64 8.5 vs 13.4 us,
 // down_proj 16.7 vs 20.3 us.  The model also sends q|k|v through this epilogue at decode sizes (fp32 accumulator that
 // rope_kv_append rounds and re-zeroes).
@@ -46,8 +48,8 @@ constexpr int TMEM_COLS = 512;
 constexpr int MAX_TN = 128;
 constexpr int W_TILE_BYTES = 128 * 128;          // one weight block of one stage: 128 rows x 128 packed bytes
 constexpr int W_STAGE_BYTES = 2 * W_TILE_BYTES;
-constexpr int NSLOT = 4;                         // A ring slots (each: 2 blocks x 32 TMEM columns)
-constexpr uint32_t A_COL0 = 256;                 // TMEM columns [0,256) hold D, [256,512) the A ring
+constexpr int NSLOT = 8;                         // upper bound of A ring slots (each: a unit of 1 or 2 k-blocks x 2 blocks x 32 TMEM columns); a
+                                                 // launch uses p.a_slots = what the D buffers leave of the 512 TMEM columns
 constexpr int NSB = 2;                           // scale/bias ring slots
 constexpr int SB_TILE_BYTES = 128 * 16;          // 128 rows x 8 k-blocks x 2 bytes
 constexpr int SB_SLOT_BYTES = 4 * SB_TILE_BYTES; // block 0 scales, block 0 biases, block 1 scales, block 1 biases
@@ -71,14 +73,15 @@ struct TcParams {
   long long U;         // total units = pairs * tiles_m * num_st
   int sb_tma;          // 1: scale/bias tiles come through TMA (num_kb % 8 == 0)
   int w_stages;        // weight ring depth
-  int x_slots;         // X ring depth (4 or 8; one slot = the [TN x 64] tile of one k-block)
+  int a_slots;         // A ring depth in units: (512 - D columns) / (64 x k-blocks per unit)
+  int x_slots;         // X ring depth (2, 4 or 8; one slot = the [TN x 64] tiles of one unit)
   uint32_t zero;       // 0, which the compiler does not know: a slot is handed back (and overwritten by the copy engine) only when what was read
                        // from it has arrived in registers, the address of the arrival depends on it (what happens otherwise: qmm_wide.cu)
 };
 
 
 // FAST: the small-scale dequant of dequant.cuh (caller promised B200P_W_SMALLSCALE): A and D are produced at 1 / SmallScaleOut<T>.
-template <typename T, int BITS, bool XPERM, bool FAST>
+template <typename T, int BITS, bool XPERM, bool FAST, int UKB>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 qmm_sk_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x,
               const __grid_constant__ CUtensorMap tm_s, const __grid_constant__ CUtensorMap tm_b,
@@ -86,18 +89,23 @@ qmm_sk_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
   constexpr int PKB = 64 * BITS / 8;            // packed bytes per row per k-block
   constexpr int KPS = 128 / PKB;                // k-blocks per stage (a stage row is one 128-byte line)
   constexpr int SPG = 8 / KPS;                  // stages per scale/bias group of 8 k-blocks
+  constexpr int NU = KPS / (2 * UKB);           // units (of UKB k-blocks) that a group of dequantisers makes of a stage
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   const uint32_t w_ring = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const int S = p.w_stages;
   const int TN = p.TN;
   const uint32_t x_ring = w_ring + S * W_STAGE_BYTES;
-  const uint32_t x_slot_bytes = (uint32_t)(TN * 128);
+  const uint32_t x_slot_bytes = (uint32_t)(UKB * TN * 128);
   const uint32_t x_mask = (uint32_t)(p.x_slots - 1);
-  const int x_shift = p.x_slots == 8 ? 3 : 2;
+  const int x_shift = p.x_slots == 8 ? 3 : p.x_slots == 4 ? 2 : 1;
   const uint32_t sb_ring = x_ring + p.x_slots * x_slot_bytes;
   const uint32_t epi_ring = sb_ring + NSB * SB_SLOT_BYTES;
   const uint32_t bar_base = epi_ring + EPI_NBUF * EPI_BUF_BYTES;
-  const int NBUF = TN > 64 ? 1 : 2;              // D buffers: buffer d, block b at columns d*128 + b*64 (TN <= 64) / b*128
+  const int NBUF = TN > 64 ? 1 : 2;              // D buffers: buffer d, block b at columns (2d + b) * d_stride
+  const uint32_t d_stride = TN <= 32 ? 32u : (TN <= 64 ? 64u : 128u);
+  constexpr uint32_t A_SLOT = UKB * 64;          // columns: [k-block][weight block][32]
+  const uint32_t A_COL0 = 512u - (uint32_t)p.a_slots * A_SLOT;   // the A ring sits at the top of TMEM
+  const uint32_t a_slots = (uint32_t)p.a_slots;
   auto full_w = [&](int s) { return bar_base + 8u * s; };
   auto empty_w = [&](int s) { return bar_base + 8u * (MAX_STAGES + s); };
   auto full_x = [&](int s) { return bar_base + 8u * (2 * MAX_STAGES + s); };
@@ -109,7 +117,7 @@ qmm_sk_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
   auto accum_full = [&](int d) { return bar_base + 8u * (4 * MAX_STAGES + 2 * NSLOT + 2 * NSB + d); };
   auto accum_empty = [&](int d) { return bar_base + 8u * (4 * MAX_STAGES + 2 * NSLOT + 2 * NSB + 2 + d); };
   const uint32_t tmem_slot = bar_base + 8u * (4 * MAX_STAGES + 2 * NSLOT + 2 * NSB + 4);
-  auto d_col = [&](int d, int b) { return (uint32_t)(TN > 64 ? b * 128 : d * 128 + b * 64); };
+  auto d_col = [&](int d, int b) { return (uint32_t)(2 * d + b) * d_stride; };
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int G = (int)gridDim.x, cta = (int)blockIdx.x;
@@ -118,7 +126,7 @@ qmm_sk_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
   if (threadIdx.x == 0) {
     for (int s = 0; s < S; ++s) { mbar_init(full_w(s), 1); mbar_init(empty_w(s), DQ_WARPS); }
     for (int s = 0; s < p.x_slots; ++s) { mbar_init(full_x(s), 1); mbar_init(empty_x(s), MMA_WARPS); }
-    for (int s = 0; s < NSLOT; ++s) { mbar_init(full_a(s), 8); mbar_init(empty_a(s), MMA_WARPS); }
+    for (int s = 0; s < p.a_slots; ++s) { mbar_init(full_a(s), 8); mbar_init(empty_a(s), MMA_WARPS); }
     for (int s = 0; s < NSB; ++s) { mbar_init(sb_full(s), 1); mbar_init(sb_empty(s), DQ_WARPS); }
     for (int d = 0; d < 2; ++d) { mbar_init(accum_full(d), MMA_WARPS); mbar_init(accum_empty(d), EPI_WARPS); }
     fence_barrier_init();
@@ -140,11 +148,9 @@ qmm_sk_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
     // Weights and scale/bias tiles do not depend on the previous kernel: no griddepcontrol.wait here, so under
     // programmatic dependent launch the HBM stream of this kernel starts while the previous kernel drains.
     int si = 0, ph = 0, sbi = 0, sbph = 0;
+    int tile = (int)(u_begin / p.num_st), st = (int)(u_begin % p.num_st), rowA0 = tile / p.tiles_m * 256;
     for (long long u = u_begin; u < u_end; ++u) {
-      const int tile = (int)(u / p.num_st), st = (int)(u % p.num_st);
-      const int pair = tile / p.tiles_m;
-      const int rowA0 = pair * 256;
-      const int rowB0 = pair * 256 + 128;
+      const int rowB0 = rowA0 + 128;
       if (p.sb_tma && (u == u_begin || (st % SPG) == 0)) {     // a new group of 8 k-blocks starts with this stage
         mbar_wait(sb_empty(sbi), sbph ^ 1);
         if (elect_one()) {
@@ -168,24 +174,27 @@ qmm_sk_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
       }
       __syncwarp();
       if (++si == S) { si = 0; ph ^= 1; }
+      if (++st == p.num_st) { st = 0; rowA0 = ++tile / p.tiles_m * 256; }
     }
   } else if (warp == WARP_X) {
     // ===================================== activation producer ==============================
     pdl_wait();                                      // X is the previous kernel's output
     uint32_t it = 0;
+    int tile = (int)(u_begin / p.num_st), st = (int)(u_begin % p.num_st), tm = tile % p.tiles_m;
     for (long long u = u_begin; u < u_end; ++u) {
-      const int tile = (int)(u / p.num_st), st = (int)(u % p.num_st);
-      const int tm = tile % p.tiles_m;
 #pragma unroll
-      for (int jj = 0; jj < KPS; ++jj, ++it) {
+      for (int jj = 0; jj < 2 * NU; ++jj, ++it) {
         const uint32_t xs = it & x_mask;
         mbar_wait(empty_x(xs), ((it >> x_shift) & 1u) ^ 1u);
         if (elect_one()) {
           mbar_arrive_expect_tx(full_x(xs), x_slot_bytes);
-          tma_load_2d(x_ring + xs * x_slot_bytes, &tm_x, (st * KPS + jj) * 64, tm * TN, full_x(xs));
+#pragma unroll
+          for (int k = 0; k < UKB; ++k)
+            tma_load_2d(x_ring + xs * x_slot_bytes + k * (uint32_t)(TN * 128), &tm_x, (st * KPS + jj * UKB + k) * 64, tm * TN, full_x(xs));
         }
         __syncwarp();
       }
+      if (++st == p.num_st) { st = 0; tm = ++tile % p.tiles_m; }
     }
   } else if (warp >= WARP_MMA) {
     // ===================================== MMA issuers (warp WARP_MMA + b: block b of the pair) =====================
@@ -194,7 +203,8 @@ qmm_sk_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
     const uint32_t fmt = std::is_same<T, __nv_bfloat16>::value ? 1u : 0u;
     const uint32_t idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(TN >> 3) << 17) | ((128u >> 4) << 24);
     int seg = 0;
-    uint32_t it = 0;
+    uint32_t slot = 0, aph = 0, xs = 0, xph = 0;
+    const uint32_t x_slots = (uint32_t)p.x_slots;
     const uint64_t xdesc0 = make_desc_sw128(x_ring);            // X slot 0, first 16 k; slot s adds s * (slot bytes >> 4)
     const uint32_t xdesc_step = x_slot_bytes >> 4;
     const int mw = warp - WARP_MMA;                    // block of the pair this warp issues for
@@ -208,19 +218,23 @@ qmm_sk_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
         tc_fence_after();
       }
       const uint32_t dmine = tmem_base + d_col(buf, mw);
-      const int nkb = ns * KPS;
-      for (int j = 0; j < nkb; ++j, ++it) {
-        const uint32_t slot = it & (NSLOT - 1), xs = it & x_mask;
-        mbar_wait(full_x(xs), (it >> x_shift) & 1u);
-        mbar_wait(full_a(slot), (it >> 2) & 1u);
+      const int nu = ns * 2 * NU;
+      for (int j = 0; j < nu; ++j) {
+        mbar_wait(full_x(xs), xph);
+        mbar_wait(full_a(slot), aph);
         tc_fence_after();
         if (elect_one()) {
-          umma_half_kblock_f16_ts(dmine, a_base + slot * 64, xdesc0 + (uint64_t)(xs * xdesc_step), idesc, j > 0 ? 1u : 0u);
+#pragma unroll
+          for (int k = 0; k < UKB; ++k)
+            umma_half_kblock_f16_ts(dmine, a_base + slot * A_SLOT + k * 64, xdesc0 + (uint64_t)(xs * xdesc_step + k * (uint32_t)(TN * 8)), idesc,
+                                    j > 0 || k > 0 ? 1u : 0u);
           umma_commit(empty_a(slot));
           umma_commit(empty_x(xs));
-          if (j == nkb - 1) umma_commit(accum_full(buf));
+          if (j == nu - 1) umma_commit(accum_full(buf));
         }
         __syncwarp();
+        if (++slot == a_slots) { slot = 0; aph ^= 1u; }
+        if (++xs == x_slots) { xs = 0; xph ^= 1u; }
       }
       u += ns;
     }
@@ -235,56 +249,57 @@ qmm_sk_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
     const uint32_t w_row_off = (uint32_t)(blk * W_TILE_BYTES + (r >> 3) * 1024 + (r & 7) * 128);
     const uint32_t w_xor = (uint32_t)(r & 7);
     const uint32_t sb_off = (uint32_t)(blk * 2 * SB_TILE_BYTES + r * 16);
-    const uint32_t half_sel = kpar ? 0x3232u : 0x1010u;   // which 16-bit half of a scale word is this thread's k-block
 
     int si = 0, ph = 0, sbi = 0, sbph = 0;
-    uint32_t it = (uint32_t)kpar;                    // global k-block counter of this thread (slot = it % 4)
+    uint32_t slot = (uint32_t)kpar, aph = 0;         // A ring slot of this thread's next unit (it advances by 2) + phase
     uint4 s8 = make_uint4(0u, 0u, 0u, 0u), b8 = s8;
 
     constexpr int CPK = PKB / 16;                    // 16-byte chunks of packed codes per k-block
-    constexpr int KPT = KPS / 2;                     // k-blocks per thread per stage
-    uint4 pk[KPT * CPK];
+    uint4 pk[NU * UKB * CPK];                        // units kpar, kpar + 2 of the stage
     // wait for the stage's weights, pull this thread's codes into registers and hand the slot straight back to the
     // producer: the HBM stream then only waits for LDS, not for the dequant math or the MMAs
     auto fetch_stage = [&]() {
       mbar_wait(full_w(si), (uint32_t)ph);
       const uint32_t wsrc = w_ring + si * W_STAGE_BYTES + w_row_off;
 #pragma unroll
-      for (int j2 = 0; j2 < KPT; ++j2)
+      for (int n = 0; n < NU; ++n)
 #pragma unroll
-        for (int c = 0; c < CPK; ++c)
-          pk[j2 * CPK + c] = lds128(wsrc + ((((uint32_t)((kpar + 2 * j2) * CPK + c)) ^ w_xor) << 4));
+        for (int c = 0; c < UKB * CPK; ++c) pk[n * UKB * CPK + c] = lds128(wsrc + (((uint32_t)((kpar + 2 * n) * UKB * CPK + c) ^ w_xor) << 4));
       uint32_t all = 0;
 #pragma unroll
-      for (int c = 0; c < KPT * CPK; ++c) all |= pk[c].w;
+      for (int c = 0; c < NU * UKB * CPK; ++c) all |= pk[c].w;
       const uint32_t done = empty_w(si) + (all & p.zero);          // (see TcParams::zero)
       __syncwarp();
       if (lane == 0) mbar_arrive(done);
       if (++si == S) { si = 0; ph ^= 1; }
     };
-    // one k-block: 64 codes of row r -> 32 packed 16-bit pairs -> A ring slot
-    auto kblock = [&](int j2, uint32_t s2, uint32_t b2) {
-      uint32_t o[32];
-      const uint32_t* pw = reinterpret_cast<const uint32_t*>(pk + j2 * CPK);
-      if constexpr (FAST) {
-        const SmallScale sc = small_scale_prep<T>(s2, b2);
+    // one unit: UKB k-blocks of 64 codes of row r -> 32 packed 16-bit pairs each -> A ring slot.  One wait for the slot and one hand-over per unit: at
+    // one k-block each, waits and hand-overs took the dequantisers and the MMA issuers longer than their work (see the top).
+    auto unit = [&](int n, const uint32_t (&s2)[UKB], const uint32_t (&b2)[UKB]) {
 #pragma unroll
-        for (int c = 0; c < 8; ++c) dequant8_small<T, BITS, XPERM>(pw + c * (BITS / 4), sc, o + 4 * c);
-      } else {
+      for (int j = 0; j < UKB; ++j) {
+        uint32_t o[32];
+        const uint32_t* pw = reinterpret_cast<const uint32_t*>(pk + (n * UKB + j) * CPK);
+        if constexpr (FAST) {
+          const SmallScale sc = small_scale_prep<T>(s2[j], b2[j]);
 #pragma unroll
-        for (int c = 0; c < 8; ++c) dequant8<T, BITS, XPERM>(pw + c * (BITS / 4), s2, b2, o + 4 * c);
+          for (int c = 0; c < 8; ++c) dequant8_small<T, BITS, XPERM>(pw + c * (BITS / 4), sc, o + 4 * c);
+        } else {
+#pragma unroll
+          for (int c = 0; c < 8; ++c) dequant8<T, BITS, XPERM>(pw + c * (BITS / 4), s2[j], b2[j], o + 4 * c);
+        }
+        if (j == 0) {
+          mbar_wait(empty_a(slot), aph ^ 1u);
+          tc_fence_after();
+        }
+        tmem_st32(a_dst + slot * A_SLOT + j * 64, o);
       }
-      const uint32_t slot = it & (NSLOT - 1);
-      mbar_wait(empty_a(slot), ((it >> 2) & 1u) ^ 1u);
-      tc_fence_after();
-      {
-        tmem_st32(a_dst + slot * 64, o);
-        tmem_st_wait();
-      }
+      tmem_st_wait();
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(full_a(slot));
-      it += 2;
+      slot += 2;
+      if (slot >= a_slots) { slot -= a_slots; aph ^= 1u; }
     };
 
     for (long long u = u_begin; u < u_end;) {
@@ -306,16 +321,22 @@ qmm_sk_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
           if constexpr (KPS == 4) {
             // stage st holds k-blocks 4*(st&1) + {0..3} of the group: words 2*(st&1) + {0,1}
             const bool hi = (st & 1) != 0;
-            const uint32_t sw0 = hi ? s8.z : s8.x, sw1 = hi ? s8.w : s8.y;
-            const uint32_t bw0 = hi ? b8.z : b8.x, bw1 = hi ? b8.w : b8.y;
-            kblock(0, prmt(sw0, 0u, half_sel), prmt(bw0, 0u, half_sel));
-            kblock(1, prmt(sw1, 0u, half_sel), prmt(bw1, 0u, half_sel));
+            const uint32_t sw0 = hi ? s8.z : s8.x, sw1 = hi ? s8.w : s8.y, bw0 = hi ? b8.z : b8.x, bw1 = hi ? b8.w : b8.y;
+            if constexpr (UKB == 2) {                    // this thread's two k-blocks are one word
+              const uint32_t sw = kpar ? sw1 : sw0, bw = kpar ? bw1 : bw0;
+              unit(0, {prmt(sw, 0u, 0x1010u), prmt(sw, 0u, 0x3232u)}, {prmt(bw, 0u, 0x1010u), prmt(bw, 0u, 0x3232u)});
+            } else {                                     // half kpar of both
+              const uint32_t half_sel = kpar ? 0x3232u : 0x1010u;
+              unit(0, {prmt(sw0, 0u, half_sel)}, {prmt(bw0, 0u, half_sel)});
+              unit(1, {prmt(sw1, 0u, half_sel)}, {prmt(bw1, 0u, half_sel)});
+            }
           } else {
-            // stage st holds k-blocks 2*(st&3) + {0,1}: word st&3
+            // stage st holds k-blocks 2*(st&3) + {0,1}: word st&3, this thread's is half kpar of it
             const int wsel = st & 3;
+            const uint32_t half_sel = kpar ? 0x3232u : 0x1010u;
             const uint32_t sw = wsel == 0 ? s8.x : (wsel == 1 ? s8.y : (wsel == 2 ? s8.z : s8.w));
             const uint32_t bw = wsel == 0 ? b8.x : (wsel == 1 ? b8.y : (wsel == 2 ? b8.z : b8.w));
-            kblock(0, prmt(sw, 0u, half_sel), prmt(bw, 0u, half_sel));
+            unit(0, {prmt(sw, 0u, half_sel)}, {prmt(bw, 0u, half_sel)});
           }
         }
       } else {
@@ -327,17 +348,19 @@ qmm_sk_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
         const T* bp = reinterpret_cast<const T*>(p.biases) + (int64_t)(row_ok ? grow : 0) * p.num_kb;
         const T zero = Tr<T>::from_f(0.f);
         for (int st = s0; st < s0 + ns; ++st) {
-          T sv[KPS / 2], bv[KPS / 2];
+          uint32_t sv[NU][UKB], bv[NU][UKB];
 #pragma unroll
-          for (int j2 = 0; j2 < KPS / 2; ++j2) {
-            const int kb = st * KPS + kpar + 2 * j2;
-            const bool ok = row_ok && kb < p.num_kb;          // k-blocks past K are zero-filled by TMA: A = 0
-            sv[j2] = ok ? __ldg(sp + kb) : zero;
-            bv[j2] = ok ? __ldg(bp + kb) : zero;
-          }
+          for (int n = 0; n < NU; ++n)
+#pragma unroll
+            for (int j = 0; j < UKB; ++j) {
+              const int kb = st * KPS + (kpar + 2 * n) * UKB + j;
+              const bool ok = row_ok && kb < p.num_kb;        // k-blocks past K are zero-filled by TMA: A = 0
+              sv[n][j] = dup16(ok ? __ldg(sp + kb) : zero);
+              bv[n][j] = dup16(ok ? __ldg(bp + kb) : zero);
+            }
           fetch_stage();
 #pragma unroll
-          for (int j2 = 0; j2 < KPS / 2; ++j2) kblock(j2, dup16(sv[j2]), dup16(bv[j2]));
+          for (int n = 0; n < NU; ++n) unit(n, sv[n], bv[n]);
         }
       }
       u += ns;
@@ -411,7 +434,7 @@ static_assert(8 * (4 * MAX_STAGES + 2 * NSLOT + 2 * NSB + 4) + 8 <= 512, "barrie
 constexpr int MIN_UNITS_PER_CTA = 2;
 
 struct TcPlan {
-  int TN, tiles_m, pairs, grid, w_stages, x_slots, smem_bytes;
+  int TN, tiles_m, pairs, grid, w_stages, x_slots, a_slots, ukb, smem_bytes;
   long long U;
 };
 
@@ -428,17 +451,21 @@ static TcPlan make_plan(int64_t M, int64_t N, int64_t K, int bits) {
   const int sms = sm_count();
   pl.grid = (int)(g > sms ? sms : (g < 1 ? 1 : g));
   // X ring: one [TN x 64] tile per k-block, 8 slots (4 at TN = 128); the weight ring gets the rest of shared memory
-  pl.x_slots = tn * 128 * 8 <= X_RING_BYTES ? 8 : 4;
-  int st = (SMEM_BUDGET - SMEM_FIXED - pl.x_slots * tn * 128) / W_STAGE_BYTES;
+  // k-blocks per unit of the A and X rings.  Above 96 tokens the MMAs take longer than the dequantisation, and what is left of TMEM holds two large
+  // units or four small ones: 4096 x 14336 at 128 tokens 19.3 / 18.8 us.
+  const int ukb = pl.ukb = bits == 4 && tn <= 96 ? 2 : 1;
+  pl.x_slots = (tn * 128 * 8 <= X_RING_BYTES ? 8 : 4) / ukb;
+  pl.a_slots = bits == 4 && tn <= 32 ? 3 : 256 / (64 * ukb);
+  int st = (SMEM_BUDGET - SMEM_FIXED - pl.x_slots * ukb * tn * 128) / W_STAGE_BYTES;
   if (st > MAX_STAGES) st = MAX_STAGES;
   pl.w_stages = st;
-  pl.smem_bytes = SMEM_FIXED + pl.x_slots * tn * 128 + st * W_STAGE_BYTES;
+  pl.smem_bytes = SMEM_FIXED + pl.x_slots * ukb * tn * 128 + st * W_STAGE_BYTES;
   return pl;
 }
 
-template <typename T, int BITS, bool XPERM, bool FAST>
-static int launch_sk(const CUtensorMap* tms, const TcParams& p, const TcPlan& pl, cudaStream_t st) {
-  auto kern = qmm_sk_kernel<T, BITS, XPERM, FAST>;
+template <typename T, int BITS, bool XPERM, bool FAST, int UKB>
+static int launch_sk_u(const CUtensorMap* tms, const TcParams& p, const TcPlan& pl, cudaStream_t st) {
+  auto kern = qmm_sk_kernel<T, BITS, XPERM, FAST, UKB>;
   static bool attr_set = false;
   if (!attr_set) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BUDGET);
@@ -458,6 +485,13 @@ static int launch_sk(const CUtensorMap* tms, const TcParams& p, const TcPlan& pl
   cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tms[0], tms[1], tms[2], tms[3], tms[4], p);
   if (e != cudaSuccess) return cuda_fail(e, "qmm_sk_kernel launch");
   return B200P_OK;
+}
+template <typename T, int BITS, bool XPERM, bool FAST>
+static int launch_sk(const CUtensorMap* tms, const TcParams& p, const TcPlan& pl, cudaStream_t st) {
+  if constexpr (BITS == 4) {
+    if (pl.ukb == 2) return launch_sk_u<T, BITS, XPERM, FAST, 2>(tms, p, pl, st);
+  }
+  return launch_sk_u<T, BITS, XPERM, FAST, 1>(tms, p, pl, st);
 }
 
 }  // namespace sk
@@ -511,7 +545,7 @@ int qmm_sk_launch(const void* x, const uint32_t* w, const void* s, const void* b
   p.num_kb = num_kb; p.pairs = pl.pairs; p.tiles_m = pl.tiles_m; p.U = pl.U;
   p.num_st = (p.num_kb + (bits == 4 ? 4 : 2) - 1) / (bits == 4 ? 4 : 2);
   p.sb_tma = sb_tma ? 1 : 0;
-  p.w_stages = pl.w_stages; p.x_slots = pl.x_slots;
+  p.w_stages = pl.w_stages; p.x_slots = pl.x_slots; p.a_slots = pl.a_slots;
   if (dtype == B200P_F16) {
     if (bits == 8) return fast ? launch_sk<__half, 8, false, true>(tms, p, pl, st) : launch_sk<__half, 8, false, false>(tms, p, pl, st);
     if (fast) return x_perm ? launch_sk<__half, 4, true, true>(tms, p, pl, st) : launch_sk<__half, 4, false, true>(tms, p, pl, st);

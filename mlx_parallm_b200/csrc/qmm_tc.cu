@@ -23,7 +23,7 @@
 // Sums are therefore taken in a fixed order: results are bit-reproducible run to run.
 //
 // warp roles (768 threads):
-//   warps 0..15  dequantisers: 4 groups of 4 warps, group g handles weight block g&1 on k-blocks of parity g>>1;
+//   warps 0..15  dequantisers: 4 groups of 4 warps, group g handles weight block g&1 on half g>>1 of every stage's k-blocks;
 //                a thread owns one weight row: LDS packed codes -> 16-bit q*s+b -> tcgen05.st into the A ring;
 //   warps 16..19 epilogue: TMEM -> registers -> global (thread = output column n: every warp store is one coalesced
 //                line per token), stream-K partial tiles and their final reduction;
@@ -34,12 +34,17 @@
 // rings:  W   (packed weights, 2 x [128 rows x 128 B] per stage) in shared memory, SWIZZLE_128B, filled by TMA and
 //             handed back as soon as the dequant warps hold the codes in registers, so the HBM stream never waits
 //             for dequant math or MMAs;
-//         X   (one [TN x 64] activation tile per k-block, 8 slots) SWIZZLE_128B, filled by TMA, freed by MMA
+//         X   (one [TN x 64] activation tile per k-block, 8 of them in slots of a unit) SWIZZLE_128B, filled by TMA, freed by MMA
 //             completion (tcgen05.commit);
 //         SB  (scales + biases of 8 k-blocks for both blocks, [128 rows x 16 B] tiles) filled by TMA when the
 //             rows of the scale matrix are 16-byte multiples (K % 512 == 0), else the dequantisers read them
 //             from global memory; freed by the dequant warps as soon as the values are in registers;
-//         A   (4 slots x 2 blocks x 32 TMEM columns), filled by the dequantisers, freed by MMA completion.
+//         A   (2 blocks x 32 TMEM columns per k-block, in slots of a unit), filled by the dequantisers, freed by MMA completion.
+// A unit is what one group of dequantisers makes of a stage: two k-blocks at 4 bits, one at 8.  The roles hand over units: a wait on a barrier that
+// is long complete takes about 100 cycles, and with one k-block per hand-over the MMA issuers spent 200 of their 490 cycles per k-block on
+// them, the dequantisers 300 of 1250 (152064 x 5120 bf16, 24 / 64 tokens: 137.6 -> 122.4 / 160 -> 147 us; 34816 x 5120 29.4 -> 26.0 / 32.0 -> 28.8; the same bits).
+// Neither memory, arithmetic nor MMAs bound the loop by themselves (152064 x 5120: all three left out but the hand-overs 72 us, arithmetic alone
+// 123, MMAs alone 97).  Asking for the next stage's codes before this one's arithmetic needs registers that 24 warps do not have: 26 -> 37 us.
 //
 // X layout: B200P_X_PERM8 says the 16-bit activations arrive with every aligned group of 8 k permuted to
 // [0,4,1,5,2,6,3,7] -- the order in which a 4-bit word's nibbles fall out of two masks as packed pairs -- which
@@ -77,8 +82,8 @@ constexpr int MMA_WARPS = 2;                      // one issuing warp per 128-ro
 constexpr int TC_THREADS = (WARP_MMA + MMA_WARPS) * 32;
 constexpr int TMEM_COLS = 512;
 constexpr int MAX_TN = 128;
-constexpr int NSLOT = 8;                         // upper bound of A ring slots (each: 2 blocks x 32 TMEM columns); a launch
-                                                 // uses p.a_slots (even) = what the D buffers leave of the 512 TMEM columns
+constexpr int NSLOT = 8;                         // upper bound of A ring slots (each: a unit of 1 or 2 k-blocks x 2 blocks x 32 TMEM columns);
+                                                 // a launch uses p.a_slots = what the D buffers leave of the 512 TMEM columns
 constexpr int NSB = 2;                           // scale/bias ring slots
 constexpr int SB_TILE_BYTES = 128 * 16;          // 128 rows x 8 k-blocks x 2 bytes
 constexpr int SB_SLOT_BYTES = 4 * SB_TILE_BYTES; // block 0 scales, block 0 biases, block 1 scales, block 1 biases
@@ -104,10 +109,10 @@ struct TcParams {
   int items;           // work items = tiles * S; CTA c takes items c, c + G, c + 2G, ...
   int rotate;          // 1: an item's stages are visited in rotated order (seg_of)
   int nbuf;            // D buffers (2: the epilogue of one item overlaps the main loop of the next; 1 frees TMEM for the A ring)
-  int a_slots;         // A ring depth: (512 - D columns) / 64, even
+  int a_slots;         // A ring depth in units: (512 - D columns) / (64 x k-blocks per unit)
   int sb_tma;          // 1: scale/bias tiles come through TMA (num_kb % 8 == 0)
   int w_stages;        // weight ring depth
-  int x_slots;         // X ring depth (4 or 8; one slot = the [TN x 64] tile of one k-block)
+  int x_slots;         // X ring depth (2, 4 or 8; one slot = the [TN x 64] tiles of one unit)
   uint32_t zero;       // 0, which the compiler does not know: a slot is handed back (and overwritten by the copy engine) only when what was read
                        // from it has arrived in registers, the address of the arrival depends on it (what happens otherwise: qmm_wide.cu)
 };
@@ -212,13 +217,14 @@ __device__ __forceinline__ void tc_drain_tile(const TcParams& p, bool silu, int 
 }
 
 // FAST: the small-scale dequant of dequant.cuh (caller promised B200P_W_SMALLSCALE): A and D are produced at 1 / SmallScaleOut<T>.
-template <typename T, int BITS, bool XPERM, bool FAST>
+template <typename T, int BITS, bool XPERM, bool FAST, int UKB>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 qmm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x,
               const __grid_constant__ CUtensorMap tm_s, const __grid_constant__ CUtensorMap tm_b, const TcParams p) {
   constexpr int PKB = 64 * BITS / 8;            // packed bytes per row per k-block
   constexpr int KPS = 128 / PKB;                // k-blocks per stage (a stage row is one 128-byte line)
   constexpr int SPG = 8 / KPS;                  // stages per scale/bias group of 8 k-blocks
+  constexpr int NU = KPS / (2 * UKB);           // units (of UKB k-blocks) that a group of dequantisers makes of a stage
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   const uint32_t w_ring = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const int S = p.w_stages;
@@ -226,14 +232,15 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
   const uint32_t w_tile_bytes = (uint32_t)p.R * 128u;          // one block of one stage: R rows x 128 packed bytes
   const uint32_t w_stage_bytes = 2u * w_tile_bytes;
   const uint32_t x_ring = w_ring + S * w_stage_bytes;
-  const uint32_t x_slot_bytes = (uint32_t)(TN * 128);
+  const uint32_t x_slot_bytes = (uint32_t)(UKB * TN * 128);
   const uint32_t x_mask = (uint32_t)(p.x_slots - 1);
-  const int x_shift = p.x_slots == 8 ? 3 : 2;
+  const int x_shift = p.x_slots == 8 ? 3 : p.x_slots == 4 ? 2 : 1;
   const uint32_t sb_ring = x_ring + p.x_slots * x_slot_bytes;
   const uint32_t bar_base = sb_ring + NSB * SB_SLOT_BYTES;
   const int NBUF = p.nbuf;                       // D buffers: buffer d, block b at columns (2d + b) * d_stride
   const uint32_t d_stride = TN <= 32 ? 32u : (TN <= 64 ? 64u : 128u);
-  const uint32_t A_COL0 = 512u - (uint32_t)p.a_slots * 64u;   // the A ring sits at the top of TMEM
+  constexpr uint32_t A_SLOT = UKB * 64;          // columns: [k-block][weight block][32]
+  const uint32_t A_COL0 = 512u - (uint32_t)p.a_slots * A_SLOT;   // the A ring sits at the top of TMEM
   const uint32_t a_slots = (uint32_t)p.a_slots;
   auto full_w = [&](int s) { return bar_base + 8u * s; };
   auto empty_w = [&](int s) { return bar_base + 8u * (MAX_STAGES + s); };
@@ -318,12 +325,14 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
      for (int i = 0; i < sg.ns; ++i) {
       const int st = seg_stage(sg, i);
 #pragma unroll
-      for (int jj = 0; jj < KPS; ++jj, ++it) {
+      for (int jj = 0; jj < 2 * NU; ++jj, ++it) {
         const uint32_t xs = it & x_mask;
         mbar_wait(empty_x(xs), ((it >> x_shift) & 1u) ^ 1u);
         if (elect_one()) {
           mbar_arrive_expect_tx(full_x(xs), x_slot_bytes);
-          tma_load_2d(x_ring + xs * x_slot_bytes, &tm_x, (st * KPS + jj) * 64, tm * TN, full_x(xs));
+#pragma unroll
+          for (int k = 0; k < UKB; ++k)
+            tma_load_2d(x_ring + xs * x_slot_bytes + k * (uint32_t)(TN * 128), &tm_x, (st * KPS + jj * UKB + k) * 64, tm * TN, full_x(xs));
         }
         __syncwarp();
       }
@@ -350,16 +359,19 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
         tc_fence_after();
       }
       const uint32_t dmine = tmem_base + d_col(buf, mw);
-      const int nkb = ns * KPS;
-      for (int j = 0; j < nkb; ++j) {
+      const int nu = ns * 2 * NU;
+      for (int j = 0; j < nu; ++j) {
         mbar_wait(full_x(xs), xph);
         mbar_wait(full_a(slot), aph);
         tc_fence_after();
         if (elect_one()) {
-          umma_half_kblock_f16_ts(dmine, a_base + slot * 64, xdesc0 + (uint64_t)(xs * xdesc_step), idesc, j > 0 ? 1u : 0u);
+#pragma unroll
+          for (int k = 0; k < UKB; ++k)
+            umma_half_kblock_f16_ts(dmine, a_base + slot * A_SLOT + k * 64, xdesc0 + (uint64_t)(xs * xdesc_step + k * (uint32_t)(TN * 8)), idesc,
+                                    j > 0 || k > 0 ? 1u : 0u);
           umma_commit(empty_a(slot));
           umma_commit(empty_x(xs));
-          if (j == nkb - 1) umma_commit(accum_full(buf));
+          if (j == nu - 1) umma_commit(accum_full(buf));
         }
         __syncwarp();
         if (++slot == a_slots) { slot = 0; aph ^= 1u; }
@@ -380,48 +392,51 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
     const bool warp_active = q * 32 < p.R;
     const uint32_t w_xor = (uint32_t)(r & 7);
     const uint32_t sb_off = (uint32_t)(blk * 2 * SB_TILE_BYTES + r * 16);
-    const uint32_t half_sel = kpar ? 0x3232u : 0x1010u;   // which 16-bit half of a scale word is this thread's k-block
 
     int si = 0, ph = 0, sbi = 0, sbph = 0;
     uint32_t slot = (uint32_t)kpar, aph = 0;         // A ring slot of this thread's next k-block (it advances by 2) + phase
     uint4 s8 = make_uint4(0u, 0u, 0u, 0u), b8 = s8;
 
     constexpr int CPK = PKB / 16;                    // 16-byte chunks of packed codes per k-block
-    constexpr int KPT = KPS / 2;                     // k-blocks per thread per stage
-    uint4 pk[KPT * CPK];
+    uint4 pk[NU * UKB * CPK];                        // units kpar, kpar + 2 of the stage
     // wait for the stage's weights, pull this thread's codes into registers and hand the slot straight back to the
     // producer: the HBM stream then only waits for LDS, not for the dequant math or the MMAs
     auto fetch_stage = [&]() {
       mbar_wait(full_w(si), (uint32_t)ph);
       const uint32_t wsrc = w_ring + si * w_stage_bytes + w_row_off;
 #pragma unroll
-      for (int j2 = 0; j2 < KPT; ++j2)
+      for (int n = 0; n < NU; ++n)
 #pragma unroll
-        for (int c = 0; c < CPK; ++c)
-          pk[j2 * CPK + c] = lds128(wsrc + ((((uint32_t)((kpar + 2 * j2) * CPK + c)) ^ w_xor) << 4));
+        for (int c = 0; c < UKB * CPK; ++c) pk[n * UKB * CPK + c] = lds128(wsrc + (((uint32_t)((kpar + 2 * n) * UKB * CPK + c) ^ w_xor) << 4));
       uint32_t all = 0;
 #pragma unroll
-      for (int c = 0; c < KPT * CPK; ++c) all |= pk[c].w;
+      for (int c = 0; c < NU * UKB * CPK; ++c) all |= pk[c].w;
       const uint32_t done = empty_w(si) + (all & p.zero);          // (see TcParams::zero)
       __syncwarp();
       if (lane == 0) mbar_arrive(done);
       if (++si == S) { si = 0; ph ^= 1; }
     };
-    // one k-block: 64 codes of row r -> 32 packed 16-bit pairs -> A ring slot
-    auto kblock = [&](int j2, uint32_t s2, uint32_t b2) {
-      uint32_t o[32];
-      const uint32_t* pw = reinterpret_cast<const uint32_t*>(pk + j2 * CPK);
-      if constexpr (FAST) {
-        const SmallScale sc = small_scale_prep<T>(s2, b2);
+    // one unit: UKB k-blocks of 64 codes of row r -> 32 packed 16-bit pairs each -> A ring slot.  One wait for the slot and one hand-over per unit: at
+    // one k-block each, waits and hand-overs took the dequantisers and the MMA issuers longer than their work (see the top).
+    auto unit = [&](int n, const uint32_t (&s2)[UKB], const uint32_t (&b2)[UKB]) {
 #pragma unroll
-        for (int c = 0; c < 8; ++c) dequant8_small<T, BITS, XPERM>(pw + c * (BITS / 4), sc, o + 4 * c);
-      } else {
+      for (int j = 0; j < UKB; ++j) {
+        uint32_t o[32];
+        const uint32_t* pw = reinterpret_cast<const uint32_t*>(pk + (n * UKB + j) * CPK);
+        if constexpr (FAST) {
+          const SmallScale sc = small_scale_prep<T>(s2[j], b2[j]);
 #pragma unroll
-        for (int c = 0; c < 8; ++c) dequant8<T, BITS, XPERM>(pw + c * (BITS / 4), s2, b2, o + 4 * c);
+          for (int c = 0; c < 8; ++c) dequant8_small<T, BITS, XPERM>(pw + c * (BITS / 4), sc, o + 4 * c);
+        } else {
+#pragma unroll
+          for (int c = 0; c < 8; ++c) dequant8<T, BITS, XPERM>(pw + c * (BITS / 4), s2[j], b2[j], o + 4 * c);
+        }
+        if (j == 0) {
+          mbar_wait(empty_a(slot), aph ^ 1u);
+          tc_fence_after();
+        }
+        tmem_st32(a_dst + slot * A_SLOT + j * 64, o);
       }
-      mbar_wait(empty_a(slot), aph ^ 1u);
-      tc_fence_after();
-      tmem_st32(a_dst + slot * 64, o);
       tmem_st_wait();
       tc_fence_before();
       __syncwarp();
@@ -446,7 +461,7 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
           __syncwarp();
           if (lane == 0) mbar_arrive(empty_w(si));
           if (++si == S) { si = 0; ph ^= 1; }
-          for (int j2 = 0; j2 < KPS / 2; ++j2) {
+          for (int n = 0; n < NU; ++n) {
             mbar_wait(empty_a(slot), aph ^ 1u);
             __syncwarp();
             if (lane == 0) mbar_arrive(full_a(slot));
@@ -476,16 +491,22 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
           if constexpr (KPS == 4) {
             // stage st holds k-blocks 4*(st&1) + {0..3} of the group: words 2*(st&1) + {0,1}
             const bool hi = (st & 1) != 0;
-            const uint32_t sw0 = hi ? s8.z : s8.x, sw1 = hi ? s8.w : s8.y;
-            const uint32_t bw0 = hi ? b8.z : b8.x, bw1 = hi ? b8.w : b8.y;
-            kblock(0, prmt(sw0, 0u, half_sel), prmt(bw0, 0u, half_sel));
-            kblock(1, prmt(sw1, 0u, half_sel), prmt(bw1, 0u, half_sel));
+            const uint32_t sw0 = hi ? s8.z : s8.x, sw1 = hi ? s8.w : s8.y, bw0 = hi ? b8.z : b8.x, bw1 = hi ? b8.w : b8.y;
+            if constexpr (UKB == 2) {                    // this thread's two k-blocks are one word
+              const uint32_t sw = kpar ? sw1 : sw0, bw = kpar ? bw1 : bw0;
+              unit(0, {prmt(sw, 0u, 0x1010u), prmt(sw, 0u, 0x3232u)}, {prmt(bw, 0u, 0x1010u), prmt(bw, 0u, 0x3232u)});
+            } else {                                     // half kpar of both
+              const uint32_t half_sel = kpar ? 0x3232u : 0x1010u;
+              unit(0, {prmt(sw0, 0u, half_sel)}, {prmt(bw0, 0u, half_sel)});
+              unit(1, {prmt(sw1, 0u, half_sel)}, {prmt(bw1, 0u, half_sel)});
+            }
           } else {
-            // stage st holds k-blocks 2*(st&3) + {0,1}: word st&3
+            // stage st holds k-blocks 2*(st&3) + {0,1}: word st&3, this thread's is half kpar of it
             const int wsel = st & 3;
+            const uint32_t half_sel = kpar ? 0x3232u : 0x1010u;
             const uint32_t sw = wsel == 0 ? s8.x : (wsel == 1 ? s8.y : (wsel == 2 ? s8.z : s8.w));
             const uint32_t bw = wsel == 0 ? b8.x : (wsel == 1 ? b8.y : (wsel == 2 ? b8.z : b8.w));
-            kblock(0, prmt(sw, 0u, half_sel), prmt(bw, 0u, half_sel));
+            unit(0, {prmt(sw, 0u, half_sel)}, {prmt(bw, 0u, half_sel)});
           }
         }
       } else {
@@ -498,17 +519,19 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
         const T zero = Tr<T>::from_f(0.f);
         for (int i = 0; i < ns; ++i) {
           const int st = seg_stage(sg, i);
-          T sv[KPS / 2], bv[KPS / 2];
+          uint32_t sv[NU][UKB], bv[NU][UKB];
 #pragma unroll
-          for (int j2 = 0; j2 < KPS / 2; ++j2) {
-            const int kb = st * KPS + kpar + 2 * j2;
-            const bool ok = row_ok && kb < p.num_kb;          // k-blocks past K are zero-filled by TMA: A = 0
-            sv[j2] = ok ? __ldg(sp + kb) : zero;
-            bv[j2] = ok ? __ldg(bp + kb) : zero;
-          }
+          for (int n = 0; n < NU; ++n)
+#pragma unroll
+            for (int j = 0; j < UKB; ++j) {
+              const int kb = st * KPS + (kpar + 2 * n) * UKB + j;
+              const bool ok = row_ok && kb < p.num_kb;        // k-blocks past K are zero-filled by TMA: A = 0
+              sv[n][j] = dup16(ok ? __ldg(sp + kb) : zero);
+              bv[n][j] = dup16(ok ? __ldg(bp + kb) : zero);
+            }
           fetch_stage();
 #pragma unroll
-          for (int j2 = 0; j2 < KPS / 2; ++j2) kblock(j2, dup16(sv[j2]), dup16(bv[j2]));
+          for (int n = 0; n < NU; ++n) unit(n, sv[n], bv[n]);
         }
       }
     }
@@ -662,12 +685,12 @@ static int g_min_tc_m = [] { const char* e = getenv("B200P_MIN_TC_M"); return e 
 void qmm_tc_set_min_m(int m) { g_min_tc_m = m < 1 ? 1 : m; }
 // A launch is cut into work items (output tile, K split).  An output tile is a PAIR of row blocks of R <= 128 weight rows
 // each (for SILU_MUL: R gate rows and the matching R up rows) times one token tile; R is chosen per matrix so that the tiles
-// fill the SMs evenly with WHOLE tiles wherever the matrix has enough rows (gate|up of Llama-3-8B: R = 104 -> 138 tiles on
-// 148 SMs; lm_head: R = 88 -> 5 tiles per SM) -- no partial tiles, the fused epilogue goes straight from TMEM to global
+// fill the SMs evenly with WHOLE tiles wherever an 8-bit matrix has enough rows (57344 x 8192: R = 104 -> 276 tiles, two per SM), 128 in 4
+// bits (make_plan) -- no partial tiles, the fused epilogue goes straight from TMEM to global
 // memory.  Only matrices with too few rows for that (o_proj, down_proj, q|k|v at decode) split K S ways, S * tiles <= #SMs,
 // and sum the S partial tiles through the workspace (kernel tail).
 struct TcPlan {
-  int TN, tiles_m, pairs, R, S, items, grid, w_stages, x_slots, smem_bytes, nbuf, a_slots;
+  int TN, tiles_m, pairs, R, S, items, grid, w_stages, x_slots, smem_bytes, nbuf, a_slots, ukb;
 };
 
 static int env_int(const char* name, int dflt) { const char* e = getenv(name); return e ? atoi(e) : dflt; }
@@ -691,7 +714,11 @@ static TcPlan make_plan(int64_t M, int64_t N, int64_t K, int bits, int epi) {
   // partly filled warp still cost issue slots, and a K split pays for writing + re-reading its fp32 partial tile.
   double best = 1e30;
   pl.R = 128; pl.S = 1;
-  for (int R = 8; R <= 128; R += 8) {
+  // 4 bits, matrices of 16 tiles and more (2368 x 3584 lost 4 %): a k-block takes a CTA its handshakes and latencies, about the same for 80 rows as for 128, so whole blocks always (us at 24 / 64 tokens, R
+  // of the cost model / 128: 152064 x 5120 122.3 / 101.2 and 147 / 119 with R = 88, 34816 x 5120 26.2 / 25.9 with 120, 28672 x 4096 21.0 / 20.3 with 104,
+  // 5120 x 5120 12.3 / 11.9).  8 bits stream twice the bytes in that time and gain from even shares (57344 x 8192: 97.5 with 104, 106.7 with 128).
+  const bool whole = bits == 4 && (rows + (silu ? 127 : 255)) / (silu ? 128 : 256) >= 16;
+  for (int R = whole ? 128 : 8; R <= 128; R += 8) {
     if (g_force_R && R != g_force_R) continue;
     const int64_t pairs = silu ? (rows + R - 1) / R : (rows + 2 * R - 1) / (2 * R);
     const int64_t tiles = pairs * pl.tiles_m;
@@ -720,16 +747,20 @@ static TcPlan make_plan(int64_t M, int64_t N, int64_t K, int bits, int epi) {
   const int d_stride = tn <= 32 ? 32 : (tn <= 64 ? 64 : 128);
   pl.nbuf = (tn > 64 || items <= sms) ? 1 : 2;
   if (g_force_nbuf && tn <= 64) pl.nbuf = g_force_nbuf;
-  pl.a_slots = ((512 - pl.nbuf * 2 * d_stride) / 64) & ~1;
+  // k-blocks per unit of the A and X rings.  Above 96 tokens the MMAs take longer than the dequantisation, and what is left of TMEM holds two large
+  // units or four small ones: 4096 x 14336 at 128 tokens 19.3 / 18.8 us.
+  const int ukb = pl.ukb = bits == 4 && tn <= 96 ? 2 : 1;
+  pl.a_slots = (512 - pl.nbuf * 2 * d_stride) / (64 * ukb);
+  if (ukb == 1) pl.a_slots &= ~1;
   if (pl.a_slots > NSLOT) pl.a_slots = NSLOT;
   // X ring: one [TN x 64] tile per k-block, 8 slots (4 at TN = 128) -- about 1 us of MMA work in flight, enough to
   // cover the L2 latency of the tile loads; the weight ring gets the rest of shared memory
-  pl.x_slots = tn * 128 * 8 <= X_RING_BYTES ? 8 : 4;
+  pl.x_slots = (tn * 128 * 8 <= X_RING_BYTES ? 8 : 4) / ukb;
   const int stage_bytes = 2 * pl.R * 128;
-  int st = (SMEM_BUDGET - SMEM_FIXED - pl.x_slots * tn * 128) / stage_bytes;
+  int st = (SMEM_BUDGET - SMEM_FIXED - pl.x_slots * ukb * tn * 128) / stage_bytes;
   if (st > MAX_STAGES) st = MAX_STAGES;
   pl.w_stages = st;
-  pl.smem_bytes = SMEM_FIXED + pl.x_slots * tn * 128 + st * stage_bytes;
+  pl.smem_bytes = SMEM_FIXED + pl.x_slots * ukb * tn * 128 + st * stage_bytes;
   return pl;
 }
 
@@ -756,9 +787,9 @@ size_t qmm_tc_workspace_bytes(int64_t M, int64_t N, int64_t K) {
   return ws_counter_bytes(M, N) + (size_t)sm_count() * 2 * tn * 128 * sizeof(float);
 }
 
-template <typename T, int BITS, bool XPERM, bool FAST>
-static int launch_tc(const CUtensorMap* tms, const TcParams& p, const TcPlan& pl, cudaStream_t st) {
-  auto kern = qmm_tc_kernel<T, BITS, XPERM, FAST>;
+template <typename T, int BITS, bool XPERM, bool FAST, int UKB>
+static int launch_tc_u(const CUtensorMap* tms, const TcParams& p, const TcPlan& pl, cudaStream_t st) {
+  auto kern = qmm_tc_kernel<T, BITS, XPERM, FAST, UKB>;
   static bool attr_set = false;
   if (!attr_set) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BUDGET);
@@ -778,6 +809,13 @@ static int launch_tc(const CUtensorMap* tms, const TcParams& p, const TcPlan& pl
   cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tms[0], tms[1], tms[2], tms[3], p);
   if (e != cudaSuccess) return cuda_fail(e, "qmm_tc_kernel launch");
   return B200P_OK;
+}
+template <typename T, int BITS, bool XPERM, bool FAST>
+static int launch_tc(const CUtensorMap* tms, const TcParams& p, const TcPlan& pl, cudaStream_t st) {
+  if constexpr (BITS == 4) {
+    if (pl.ukb == 2) return launch_tc_u<T, BITS, XPERM, FAST, 2>(tms, p, pl, st);
+  }
+  return launch_tc_u<T, BITS, XPERM, FAST, 1>(tms, p, pl, st);
 }
 
 // Tensor maps are pure functions of (base, dims, stride, box, type, swizzle): encode each distinct one once per process

@@ -787,6 +787,21 @@ def test_qmm_wide_tiles_repeat_bit_for_bit(ops, M, N, K, bits, dtype):
     assert int(bad) == 0
 
 
+@pytest.mark.parametrize("M,N,K,dtype,epi,small", [
+    (8, 4096, 576, "bfloat16", 0, True),          # nine k-blocks: a stage with one, scales that the copy engine cannot fetch, whole row blocks
+    (32, 4112, 2368, "float16", 3, False),        # three slots of the ring; rows past N / 2 in the last block
+    (33, 8200, 1024, "bfloat16", 1, True),        # two slots
+    (64, 40960, 512, "float16", 0, True),         # more tiles than SMs: two accumulators, one unit on each side of the border
+    (96, 4096, 512, "bfloat16", 2, True),         # the largest token tile of two k-blocks ...
+    (97, 4096, 512, "bfloat16", 2, True),         # ... and the smallest of one
+    (20, 2056, 1216, "float16", 2, False),        # ranges of K that end inside a tile
+])
+def test_qmm_units_of_two_k_blocks(ops, M, N, K, dtype, epi, small):
+    """The tile kernels hand over two k-blocks at a time at 4 bits up to 96 tokens: against the oracle, tolerances as for the other 16-bit paths."""
+    got, exp = qmm_case(ops, M, N, K, 4, dtype, epi, seed=M + N, path=2, small_scale=small)
+    assert rel_err(got, exp) < {"float16": 3e-3, "bfloat16": 2e-2}[dtype]
+
+
 @pytest.mark.parametrize("M,N,K,bits,dtype", [(250, 18944, 1024, 8, "bfloat16"), (64, 8192, 4096, 4, "float16"), (40, 4096, 8192, 8, "bfloat16"), (1, 8192, 8192, 4, "bfloat16")])
 def test_qmm_between_memory_bound_kernels(ops, M, N, K, bits, dtype):
     """A product that starts while an elementwise kernel still fills the SM's memory pipeline: the weights' slots must not be refilled
