@@ -13,7 +13,7 @@ int qmv_launch(const void* x, const uint32_t* w, const void* s, const void* b, v
 bool qmm_tc_supported(int64_t M, int64_t N, int64_t K, int gs, int bits, int dtype, int epi);
 int qmm_tc_launch(const void* x, const uint32_t* w, const void* s, const void* b, void* y, int64_t M, int64_t N,
                   int64_t K, int64_t ldx, int64_t ldy, int bits, int dtype, int epi, int flags, void* ws, size_t ws_bytes,
-                  cudaStream_t st);
+                  int64_t row0, cudaStream_t st);
 size_t qmm_tc_workspace_bytes(int64_t M, int64_t N, int64_t K);
 bool qmm_sk_supported(int64_t M, int64_t N, int64_t K, int bits, int epi, const void* y, int64_t ldy);
 int qmm_sk_launch(const void* x, const uint32_t* w, const void* s, const void* b, void* y, int64_t M, int64_t N,
@@ -25,7 +25,7 @@ int qmm_mma_launch(const void* x, const uint32_t* w, const void* s, const void* 
                    int64_t ldx, int64_t ldy, int dtype, int flags, cudaStream_t st);
 bool qmm_wide_supported(int64_t M, int64_t N, int64_t K, int bits, int epi, const void* s, const void* b, const void* y, int64_t ldy);
 int qmm_wide_launch(const void* x, const uint32_t* w, const void* s, const void* b, void* y, int64_t M, int64_t N, int64_t K, int64_t ldx,
-                    int64_t ldy, int bits, int dtype, int epi, int flags, cudaStream_t st);
+                    int64_t ldy, int bits, int dtype, int epi, int flags, void* ws, size_t ws_bytes, cudaStream_t st);
 bool qmv_ring_supported(int64_t M, int64_t N, int64_t K, int gs, int bits, int dtype, int epi);
 int qmv_ring_launch(const void* x, const uint32_t* w, const void* s, const void* b, void* y, int64_t M, int64_t N, int64_t K, int64_t ldx,
                     int64_t ldy, int bits, int dtype, int epi, int flags, cudaStream_t st);
@@ -167,7 +167,8 @@ extern "C" int b200p_qmm(const void* x, const uint32_t* w, const void* scales, c
   }
   // more than 128 tokens: one 128-row weight block against up to 256 tokens (the rule and its figures: qmm_wide.cu)
   if (tc_ok && g_qmm_path != 1 && (tile_args || sk_args) && qmm_wide_supported(M, N, K, bits, epilogue, scales, biases, y, ldy))
-    return qmm_wide_launch(x, w, scales, biases, y, M, N, K, ldx, ldy, bits, dtype, epilogue, flags, st);
+    return qmm_wide_launch(x, w, scales, biases, y, M, N, K, ldx, ldy, bits, dtype, epilogue, flags, tile_args ? workspace : nullptr,
+                           workspace_bytes, st);
   // fp32 accumulate epilogue: the stream-K kernel (partial tiles summed by TMA reduce-adds, no workspace, no tail);
   // B200P_QMM_SK=0 keeps everything on the whole-tile kernel (A/B measurements)
   if (tc_ok && g_qmm_path != 1 && sk_args)
@@ -176,7 +177,7 @@ extern "C" int b200p_qmm(const void* x, const uint32_t* w, const void* scales, c
     B200P_REQUIRE(workspace && workspace_bytes >= qmm_tc_workspace_bytes(M, N, K), B200P_ERR_ARG,
                   "tensor path needs a workspace of %zu bytes", qmm_tc_workspace_bytes(M, N, K));
     return qmm_tc_launch(x, w, scales, biases, y, M, N, K, ldx, ldy, bits, dtype, epilogue, flags, workspace,
-                         workspace_bytes, st);
+                         workspace_bytes, 0, st);
   }
   return qmv_launch(x, w, scales, biases, y, M, N, K, ldx, ldy, group_size, bits, dtype, epilogue, flags, st);
 }

@@ -98,6 +98,7 @@ struct TcParams {
   float* ws_part;      // stream-K partial tiles: [grid][2 slots][2 blocks][TN tokens][128 rows] fp32 (no initial state)
   int* ws_counter;     // {arrived, done} per output tile (zero on entry, left zero)
   int M_tok, N, K, TN;
+  int row0;            // first output row of the launch (SILU_MUL: gate row)
   int64_t ldy;
   int epi;
   int y_perm;          // 1: 16-bit outputs (STORE / SILU_MUL) are written in the PERM8 column order
@@ -286,8 +287,8 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
     for (int item = cta; item < p.items; item += G) {
      const TcSeg sg = seg_of(p, item);
      const int pair = sg.tile / p.tiles_m;
-     const int rowA0 = silu ? pair * p.R : pair * 2 * p.R;
-     const int rowB0 = silu ? p.N / 2 + pair * p.R : pair * 2 * p.R + p.R;
+     const int rowA0 = p.row0 + (silu ? pair * p.R : pair * 2 * p.R);
+     const int rowB0 = p.row0 + (silu ? p.N / 2 + pair * p.R : pair * 2 * p.R + p.R);
      for (int i = 0; i < sg.ns; ++i) {
       const int st = seg_stage(sg, i);
       if (p.sb_tma && (i == 0 || st == sg.s0 || (st % SPG) == 0)) {     // a new group of 8 k-blocks starts with this stage
@@ -512,7 +513,7 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
       } else {
         // scale rows are not 16-byte multiples (K % 512 != 0, e.g. a TP shard): read them from global memory
         const int pair = tile / p.tiles_m;
-        const int grow = (blk ? (silu ? p.N / 2 + pair * p.R : pair * 2 * p.R + p.R) : (silu ? pair * p.R : pair * 2 * p.R)) + r;
+        const int grow = (blk ? (p.row0 + (silu ? p.N / 2 + pair * p.R : pair * 2 * p.R + p.R)) : (p.row0 + (silu ? pair * p.R : pair * 2 * p.R))) + r;
         const bool row_ok = grow < p.N && r < p.R;
         const T* sp = reinterpret_cast<const T*>(p.scales) + (int64_t)(row_ok ? grow : 0) * p.num_kb;
         const T* bp = reinterpret_cast<const T*>(p.biases) + (int64_t)(row_ok ? grow : 0) * p.num_kb;
@@ -545,8 +546,8 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
       mbar_wait(accum_full(buf), (uint32_t)((seg / NBUF) & 1));
       tc_fence_after();
       const uint32_t lane_base = tmem_base + ((uint32_t)(q * 32) << 16);
-      tc_drain_tile<T, FAST>(p, silu, r, lane_base + d_col(buf, 0), lane_base + d_col(buf, 1), TN, silu ? pair * p.R : pair * 2 * p.R,
-                             silu ? p.N / 2 + pair * p.R : pair * 2 * p.R + p.R, tm * TN, 1 + grp, 1 + DQ_WARPS / 4);
+      tc_drain_tile<T, FAST>(p, silu, r, lane_base + d_col(buf, 0), lane_base + d_col(buf, 1), TN, p.row0 + (silu ? pair * p.R : pair * 2 * p.R),
+                             p.row0 + (silu ? p.N / 2 + pair * p.R : pair * 2 * p.R + p.R), tm * TN, 1 + grp, 1 + DQ_WARPS / 4);
     }
   } else {
     // ===================================== epilogue warps ===================================
@@ -567,8 +568,8 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
       const TcSeg sg = seg_of(p, item);
       const int tile = sg.tile;
       const int pair = tile / p.tiles_m, tm = tile % p.tiles_m;
-      const int rowA0 = silu ? pair * p.R : pair * 2 * p.R;
-      const int rowB0 = silu ? p.N / 2 + pair * p.R : pair * 2 * p.R + p.R;
+      const int rowA0 = p.row0 + (silu ? pair * p.R : pair * 2 * p.R);
+      const int rowB0 = p.row0 + (silu ? p.N / 2 + pair * p.R : pair * 2 * p.R + p.R);
       const int tok0 = tm * TN;
       const int buf = NBUF == 2 ? (seg & 1) : 0;
       const bool full = p.S == 1;
@@ -622,8 +623,8 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
       }
       named_bar_sync(2, EPI_THREADS);
       const int pair = tile / p.tiles_m, tm = tile % p.tiles_m;
-      const int rowA0 = silu ? pair * p.R : pair * 2 * p.R;
-      const int rowB0 = silu ? p.N / 2 + pair * p.R : pair * 2 * p.R + p.R;
+      const int rowA0 = p.row0 + (silu ? pair * p.R : pair * 2 * p.R);
+      const int rowB0 = p.row0 + (silu ? p.N / 2 + pair * p.R : pair * 2 * p.R + p.R);
       const int tok0 = tm * TN;
       for (int t0 = me * EPI_TOK; t0 < TN; t0 += S * EPI_TOK) {
         if (tok0 + t0 >= p.M_tok) break;               // padding tokens of the last token tile
@@ -868,12 +869,13 @@ static int encode_2d_raw(TcEncodeFn enc, CUtensorMap* tm, CUtensorMapDataType dt
   return B200P_OK;
 }
 
+// row0: the first output row to compute (SILU_MUL: gate row, with its up row), a multiple of 8
 int qmm_tc_launch(const void* x, const uint32_t* w, const void* s, const void* b, void* y, int64_t M, int64_t N,
                   int64_t K, int64_t ldx, int64_t ldy, int bits, int dtype, int epi, int flags, void* ws, size_t ws_bytes,
-                  cudaStream_t st) {
+                  int64_t row0, cudaStream_t st) {
   TcEncodeFn enc = tc_get_encode();
   B200P_REQUIRE(enc != nullptr, B200P_ERR_CUDA, "cuTensorMapEncodeTiled entry point not available");
-  TcPlan pl = make_plan(M, N, K, bits, epi);
+  TcPlan pl = make_plan(M, N - (epi == B200P_EPI_SILU_MUL ? 2 : 1) * row0, K, bits, epi);
   B200P_REQUIRE(pl.w_stages >= 2, B200P_ERR_ARG, "shared memory too small for the tensor path");
   const bool x_perm = (flags & B200P_X_PERM8) != 0, y_perm = (flags & B200P_Y_PERM8) != 0;
   B200P_REQUIRE(!x_perm || bits == 4, B200P_ERR_ARG, "B200P_X_PERM8 is the 4-bit activation layout");
@@ -914,7 +916,7 @@ int qmm_tc_launch(const void* x, const uint32_t* w, const void* s, const void* b
   }
   p.ws_counter = reinterpret_cast<int*>(ws);
   p.ws_part = reinterpret_cast<float*>(reinterpret_cast<char*>(ws) + counters);
-  p.M_tok = (int)M; p.N = (int)N; p.K = (int)K; p.TN = pl.TN; p.ldy = ldy; p.epi = epi; p.y_perm = y_perm ? 1 : 0;
+  p.M_tok = (int)M; p.N = (int)N; p.K = (int)K; p.TN = pl.TN; p.row0 = (int)row0; p.ldy = ldy; p.epi = epi; p.y_perm = y_perm ? 1 : 0;
   B200P_REQUIRE((int64_t)pl.pairs * pl.tiles_m * pl.S < (1ll << 30), B200P_ERR_ARG, "problem too large for the tensor path");
   p.num_kb = num_kb; p.pairs = pl.pairs; p.tiles_m = pl.tiles_m; p.R = pl.R; p.S = pl.S; p.items = pl.items; p.rotate = g_rotate; p.nbuf = pl.nbuf; p.a_slots = pl.a_slots;
   p.num_st = (p.num_kb + (bits == 4 ? 4 : 2) - 1) / (bits == 4 ? 4 : 2);

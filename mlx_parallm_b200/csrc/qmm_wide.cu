@@ -28,6 +28,7 @@
 // 20 TMA producer of weights, scales and biases, 21 TMA producer of X, 22 / 23 MMA issuers.
 #include <cuda.h>
 
+#include <algorithm>
 #include <type_traits>
 
 #include "common.cuh"
@@ -38,6 +39,8 @@ namespace b200p {
 
 int sm_count();
 bool pdl_enabled_gemm();
+int qmm_tc_launch(const void* x, const uint32_t* w, const void* s, const void* b, void* y, int64_t M, int64_t N, int64_t K, int64_t ldx,
+                  int64_t ldy, int bits, int dtype, int epi, int flags, void* ws, size_t ws_bytes, int64_t row0, cudaStream_t st);
 
 namespace wide {
 
@@ -462,9 +465,23 @@ qmm_wide_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
 }
 
 // ------------------------------------------------------------------------------------------------ host
-struct Plan { int tiles_m, TN, H0, H1, row_blocks, items, grid, w_stages, smem; };
+struct Plan { int tiles_m, TN, H0, H1, row_blocks, left, items, grid, w_stages, smem; };
 
-static Plan make_plan(int64_t M, int64_t N, int64_t K, int bits, int epi) {
+// Row blocks of a short last round of whole tiles that are left to the kernel that splits K (qmm_tc.cu): row_blocks x tiles_m just above a multiple of the
+// SMs is common (57344 gated rows are 448 blocks, three times 148 and four), and the few CTAs of the last round then take as long as all of one before.
+// Behind the other launch the split one costs about 30000 cycles and its share of K; a round takes a k-block about 640 cycles with 8-bit codes, 400 or
+// the MMAs' time with 4.  So only long rounds are worth it (us, whole tiles / left: 57344 x 8192 8 bits at 129 / 201 / 300 / 600 tokens 188 / 172, 207 / 189,
+// 308 / 294, 509 / 497, but 1349 / 1377 at 1300, 13 rounds; 28672 x 4096 4 bits 96.3 / 97.5 at 300, 303 / 350 at 1500).
+static int left_over(int row_blocks, int tiles_m, int tn, int64_t M, int64_t K, int bits) {
+  const int sms = sm_count(), items = row_blocks * tiles_m, whole = items / sms * sms;
+  if (whole == 0 || whole == items || whole > 9 * sms) return 0;
+  const int left = row_blocks - whole / tiles_m;
+  const int64_t tiles = (int64_t)(left + 1) / 2 * ((M + 127) / 128), splits = sms / tiles < 16 ? sms / tiles : 16;
+  const double kb = (double)(K / 64), round = kb * std::max(2.0 * tn, bits == 8 ? 640.0 : 400.0);
+  return splits >= 4 && 30000.0 + 700.0 * kb / (double)splits < 0.6 * round ? left : 0;
+}
+
+static Plan make_plan(int64_t M, int64_t N, int64_t K, int bits, int epi, bool may_leave) {
   Plan pl;
   const bool add = epi == B200P_EPI_ADD_RESIDUAL;
   const int rows = epi == B200P_EPI_SILU_MUL ? 64 : 128;
@@ -483,6 +500,8 @@ static Plan make_plan(int64_t M, int64_t N, int64_t K, int bits, int epi) {
   }
   pl.H0 = (pl.TN / 2 + 15) / 16 * 16;
   pl.H1 = pl.TN - pl.H0;
+  pl.left = add || !may_leave ? 0 : left_over(pl.row_blocks, pl.tiles_m, pl.TN, M, K, bits);
+  pl.row_blocks -= pl.left;
   pl.items = pl.row_blocks * pl.tiles_m;
   const int64_t units = add ? (int64_t)pl.items * (K * bits / 1024) / 2 : pl.items;      // at least two stages per CTA
   pl.grid = (int)(units < 1 ? 1 : units > sms ? sms : units);
@@ -541,13 +560,13 @@ bool qmm_wide_supported(int64_t M, int64_t N, int64_t K, int bits, int epi, cons
 }
 
 int qmm_wide_launch(const void* x, const uint32_t* w, const void* s, const void* b, void* y, int64_t M, int64_t N, int64_t K, int64_t ldx,
-                    int64_t ldy, int bits, int dtype, int epi, int flags, cudaStream_t st) {
+                    int64_t ldy, int bits, int dtype, int epi, int flags, void* ws, size_t ws_bytes, cudaStream_t st) {
   using namespace wide;
   TcEncodeFn enc = tc_get_encode();
   B200P_REQUIRE(enc != nullptr, B200P_ERR_CUDA, "cuTensorMapEncodeTiled entry point not available");
   const bool x_perm = (flags & B200P_X_PERM8) != 0, add = epi == B200P_EPI_ADD_RESIDUAL;
   const bool fast = (flags & B200P_W_SMALLSCALE) != 0;
-  const Plan pl = make_plan(M, N, K, bits, epi);
+  const Plan pl = make_plan(M, N, K, bits, epi, ws != nullptr);
   B200P_REQUIRE(pl.w_stages >= 2, B200P_ERR_ARG, "shared memory too small for the tensor path");
   const CUtensorMapDataType dt16 = dtype == B200P_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
   const uint32_t box_rows = epi == B200P_EPI_SILU_MUL ? 16u : 128u;
@@ -570,15 +589,21 @@ int qmm_wide_launch(const void* x, const uint32_t* w, const void* s, const void*
   p.tiles_m = pl.tiles_m; p.row_blocks = pl.row_blocks; p.items = pl.items; p.w_stages = pl.w_stages;
   p.row_fast = M * K * 2 > N * K * bits / 8 ? 1 : 0;
 #define GO(T_, B_, X_, F_) (add ? run<T_, B_, X_, F_, true>(tm, p, pl, st) : run<T_, B_, X_, F_, false>(tm, p, pl, st))
-  if (dtype == B200P_F16) {
-    if (bits == 8) return fast ? GO(__half, 8, false, true) : GO(__half, 8, false, false);
-    if (fast) return x_perm ? GO(__half, 4, true, true) : GO(__half, 4, false, true);
-    return x_perm ? GO(__half, 4, true, false) : GO(__half, 4, false, false);
-  }
-  if (bits == 8) return fast ? GO(__nv_bfloat16, 8, false, true) : GO(__nv_bfloat16, 8, false, false);
-  if (fast) return x_perm ? GO(__nv_bfloat16, 4, true, true) : GO(__nv_bfloat16, 4, false, true);
-  return x_perm ? GO(__nv_bfloat16, 4, true, false) : GO(__nv_bfloat16, 4, false, false);
+  const auto launch = [&]() -> int {
+    if (dtype == B200P_F16) {
+      if (bits == 8) return fast ? GO(__half, 8, false, true) : GO(__half, 8, false, false);
+      if (fast) return x_perm ? GO(__half, 4, true, true) : GO(__half, 4, false, true);
+      return x_perm ? GO(__half, 4, true, false) : GO(__half, 4, false, false);
+    }
+    if (bits == 8) return fast ? GO(__nv_bfloat16, 8, false, true) : GO(__nv_bfloat16, 8, false, false);
+    if (fast) return x_perm ? GO(__nv_bfloat16, 4, true, true) : GO(__nv_bfloat16, 4, false, true);
+    return x_perm ? GO(__nv_bfloat16, 4, true, false) : GO(__nv_bfloat16, 4, false, false);
+  };
 #undef GO
+  rc = launch();
+  if (rc || !pl.left) return rc;
+  return qmm_tc_launch(x, w, s, b, y, M, N, K, ldx, ldy, bits, dtype, epi, flags, ws, ws_bytes,
+                       (int64_t)pl.row_blocks * (epi == B200P_EPI_SILU_MUL ? 64 : 128), st);
 }
 
 }  // namespace b200p

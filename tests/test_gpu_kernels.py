@@ -769,6 +769,27 @@ def test_qmm_wide_tiles(ops, M, N, K, bits, dtype, epi, small):
     assert rel_err(got, exp) < {"float16": 3e-3, "bfloat16": 2e-2}[dtype]
 
 
+@pytest.mark.parametrize("M,N,K,bits,epi", [(130, 19328, 8192, 8, 3), (300, 9856, 8192, 8, 0), (145, 19001 * 2, 8192, 8, 1)])
+def test_qmm_wide_tiles_leave_a_short_last_round(ops, M, N, K, bits, epi):
+    """Row blocks beyond whole rounds of tiles go to the kernel that splits K: every column against a float64 product (1.5e-2: one bf16 rounding of weights,
+    activations and outputs each), twice with one workspace, whose counters are left as they were found."""
+    g = torch.Generator(device="cuda").manual_seed(N)
+    w = torch.randint(-2 ** 31, 2 ** 31, (N, K // 4), generator=g, device="cuda", dtype=torch.int64).to(torch.int32)
+    s = ((torch.rand((N, K // 64), generator=g, device="cuda") + 0.5) * 2 / 255 / K ** 0.5).bfloat16()
+    b = (-s.float() * 255 / 2).bfloat16()
+    x = torch.randn((M, K), generator=g, device="cuda").bfloat16()
+    ws = torch.zeros(ops.qmm_workspace_bytes(M, N, K), dtype=torch.uint8, device="cuda")
+    for _ in range(2):
+        got = ops.qmm(x, w, s, b, 64, bits, epi, workspace=ws, small_scale=True).double()
+        full = torch.empty(M, N, dtype=torch.float64, device="cuda")
+        for i in range(0, N, 4096):
+            codes = ((w[i:i + 4096].unsqueeze(-1) >> torch.arange(0, 32, 8, device="cuda", dtype=torch.int32)) & 255).reshape(-1, K // 64, 64).double()
+            full[:, i:i + 4096] = x.double() @ (codes * s[i:i + 4096].double().unsqueeze(-1) + b[i:i + 4096].double().unsqueeze(-1)).reshape(-1, K).t()
+        want = torch.nn.functional.silu(full[:, :N // 2]) * full[:, N // 2:] if epi == 3 else full
+        err = (got - want).norm(dim=0) / want.norm(dim=0)
+        assert float(err.max()) < 1.5e-2 and not bool(ws[:4096].any())
+
+
 @pytest.mark.parametrize("M,N,K,bits,dtype", [(201, 2048, 4096, 8, "bfloat16"), (250, 18944, 1024, 8, "bfloat16"), (300, 4096, 2048, 4, "float16")])
 def test_qmm_wide_tiles_repeat_bit_for_bit(ops, M, N, K, bits, dtype):
     """Whole tiles are summed in a fixed order: hundreds of launches over the same operands agree in every bit.  (A k-block of one row that is
