@@ -431,6 +431,29 @@ def prefill_inputs(dtype, B, L, Hq, Hkv, Tcap, seed, spread=1.0):
     return (r(B, L, Hq, 128) * spread).to(TD[dtype]), r(B, Hkv, Tcap, 128).to(TD[dtype]), r(B, Hkv, Tcap, 128).to(TD[dtype])
 
 
+@pytest.mark.parametrize("B,L,Hq,Hkv,T", [(20, 50, 32, 8, 0), (8, 300, 32, 8, 77), (3, 700, 40, 8, 300), (5, 513, 64, 8, 0), (40, 2, 8, 8, 130)])
+def test_attention_tcgen05_prefill_of_more_items_than_sms(ops, B, L, Hq, Hkv, T):
+    """CTAs that take several items in turn (items of one key tile, two to four rounds, the last one partly filled) give the bits of every sequence
+    alone, whose items all have a CTA of their own; sequences of different lengths."""
+    from mlx_parallm_b200 import _lib
+    D, g, dt = 128, torch.Generator(device="cuda").manual_seed(B + L), torch.bfloat16
+    cap = -(-(T + L) // 128) * 128 + 128
+    q = torch.randn(B * L, Hq * D, generator=g, device="cuda").to(dt)
+    kc, vc = (torch.randn(B, Hkv, cap, D, generator=g, device="cuda").to(dt) for _ in range(2))
+    lengths = torch.tensor([T - (i * 7) % (T + 1) for i in range(B)], dtype=torch.int32, device="cuda")
+    out, alone = torch.zeros_like(q), torch.zeros_like(q)
+    _lib.lib().b200p_attn_set_path(3)
+    try:
+        ops.attn(q, kc, vc, lengths, out, B, L, Hq, Hkv, D, D ** -0.5)
+        for b in range(B):
+            rows = slice(b * L, (b + 1) * L)
+            ops.attn(q[rows], kc[b:b + 1], vc[b:b + 1], lengths[b:b + 1], alone[rows], 1, L, Hq, Hkv, D, D ** -0.5)
+    finally:
+        _lib.lib().b200p_attn_set_path(0)
+    assert _lib.lib().b200p_attn_tc_fault() == 0
+    assert torch.equal(out, alone) and bool(out.isfinite().all())
+
+
 @pytest.mark.parametrize("dtype", ["float16", "bfloat16"])
 @pytest.mark.parametrize("scale", [0.0, 1e-44, 1e-39, -0.11, 2e-38])
 @pytest.mark.parametrize("path", [0, 3])
