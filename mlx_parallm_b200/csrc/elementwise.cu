@@ -2,11 +2,7 @@
 // All HBM- or latency-bound byte work: one pass, 128-bit accesses, no tensor cores.
 #include <type_traits>
 
-#include <cooperative_groups.h>
-
 #include "common.cuh"
-
-namespace cg = cooperative_groups;
 
 namespace b200p {
 
@@ -231,53 +227,52 @@ rmsnorm_kernel(const float* __restrict__ x, const T* __restrict__ w, T* __restri
     yr[i] = Tr<T>::from_f(xr[i] * inv * Tr<T>::to_f(w[i]));
 }
 
-// "early" RMSNorm in ONE pass over the row: the row is split over a thread-block cluster of C = H / 2048 CTAs (2 at H = 4096,
-// 4 at 8192), every thread keeps its 16 elements in registers between the sum of squares and the output, and the C partial
-// sums meet through distributed shared memory (each CTA writes its sum into slot [rank] of every CTA, one barrier.cluster).
-// The generic kernel above reads the row twice, and with 32 registers per thread its second read is four dependent round
-// trips to L2 (a resident GEMM CTA leaves no L1).  Same launch contract as the NT = 128 variant: 128 threads x 32 registers,
-// PDL attribute, dependents released before its own wait.  The norm weights do not depend on the previous kernel and are
-// loaded before the wait.  The sum is taken in (warp, CTA rank) order: reproducible, not bit-identical to the generic kernel's.
-template <typename T>
-__global__ void __launch_bounds__(128, 16)
-rmsnorm_cluster_kernel(const float* __restrict__ x, const T* __restrict__ w, T* __restrict__ y, int64_t H, float eps, int perm) {
+// The norm of 16-bit rows in ONE pass: a CTA of 256 threads per row, every thread keeps its NG groups of 8 elements in registers
+// between the sum of squares and the output.  What bounds a norm of a decode step is a chain of latencies, not bytes: launch, one
+// round trip for the row, the block's sum, the store.  So the dependents are released first (the matrix kernel that follows sets
+// itself up and streams its weights meanwhile), the norm's own weights, which no kernel before it writes, are loaded before the
+// wait, and all loads of a row are in flight at once.  256 threads and up to 8 groups: 128 threads are as fast or faster back to
+// back (8192 wide, 64 rows: 1.9 us against 2.6), yet slower in a step, where each norm waits for its row (Qwen3-14B at B=24,
+// 3 layers: 400 us against 389); 512 threads are the same in a step and slower from some 300 rows on (5120 wide, 4096 rows: 32 us
+// against 22).  Back to back, us, before (the two-pass kernel above or, for whole multiples of 2048 and up to one CTA per SM, a
+// row split over a cluster of CTAs) -> now, bf16:
+//   5120 wide:  1 row 2.9 -> 1.8    64 rows 4.6 -> 2.0   300 rows 6.8 -> 3.7   4096 rows 30.2 -> 22.3 (5.6 TB/s)
+//   4096 wide:  1 row 2.0 -> 1.7    64 rows 2.3 -> 1.9   300 rows 5.3 -> 3.5   4096 rows 24.7 -> 18.9
+//   8192 wide:  1 row 2.0 -> 2.1    64 rows 6.7 -> 2.6   300 rows 8.7 -> 4.7   4096 rows 49.2 -> 32.2
+// The sum is taken in (thread, warp) order: reproducible, not bit-identical to the two-pass kernel's.
+constexpr int RMS_NT = 256;
+template <typename T, int NG>
+__global__ void __launch_bounds__(RMS_NT)
+rmsnorm_row_kernel(const float* __restrict__ x, const T* __restrict__ w, T* __restrict__ y, int H, float eps, int perm) {
   static_assert(sizeof(T) == 2, "16-bit outputs only");
-  constexpr int NG = 2;                            // groups of 8 consecutive elements per thread
-  __shared__ float s_warp[4];
-  __shared__ float s_cta[8];
-  cg::cluster_group cluster = cg::this_cluster();
-  const unsigned rank = cluster.block_rank(), C = cluster.num_blocks();
-  const int tid = threadIdx.x;
+  __shared__ float sh[33];
   pdl_launch_dependents();
-  const int64_t row = blockIdx.x / C;
+  const int groups = H / 8;
   uint4 wv[NG];
 #pragma unroll
-  for (int j = 0; j < NG; ++j) wv[j] = reinterpret_cast<const uint4*>(w)[(j * C + rank) * 128 + tid];
+  for (int j = 0; j < NG; ++j) {
+    const int g = j * RMS_NT + threadIdx.x;
+    wv[j] = g < groups ? reinterpret_cast<const uint4*>(w)[g] : make_uint4(0u, 0u, 0u, 0u);
+  }
   pdl_wait();
-  const float4* xr = reinterpret_cast<const float4*>(x + row * H);
+  const float4* xr = reinterpret_cast<const float4*>(x + (int64_t)blockIdx.x * H);
   float4 a[NG], b[NG];
 #pragma unroll
   for (int j = 0; j < NG; ++j) {
-    const int64_t g = (int64_t)(j * C + rank) * 128 + tid;
-    a[j] = xr[2 * g];
-    b[j] = xr[2 * g + 1];
+    const int g = j * RMS_NT + threadIdx.x;
+    a[j] = b[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (g < groups) a[j] = xr[2 * g], b[j] = xr[2 * g + 1];
   }
   float ss = 0.f;
 #pragma unroll
   for (int j = 0; j < NG; ++j)
     ss += a[j].x * a[j].x + a[j].y * a[j].y + a[j].z * a[j].z + a[j].w * a[j].w + b[j].x * b[j].x + b[j].y * b[j].y +
           b[j].z * b[j].z + b[j].w * b[j].w;
-  ss = warp_sum(ss);
-  if ((tid & 31) == 0) s_warp[tid >> 5] = ss;
-  __syncthreads();
-  if (tid < (int)C) *cluster.map_shared_rank(&s_cta[rank], tid) = (s_warp[0] + s_warp[1]) + (s_warp[2] + s_warp[3]);
-  cluster.sync();
-  float tot = 0.f;
-  for (unsigned r = 0; r < C; ++r) tot += s_cta[r];
-  const float inv = 1.0f / sqrtf(tot / (float)H + eps);
-  uint4* yr = reinterpret_cast<uint4*>(y + row * H);
+  const float inv = 1.0f / sqrtf(block_sum(ss, sh) / (float)H + eps);
+  uint4* yr = reinterpret_cast<uint4*>(y + (int64_t)blockIdx.x * H);
 #pragma unroll
   for (int j = 0; j < NG; ++j) {
+    const int g = j * RMS_NT + threadIdx.x;
     const T* wp = reinterpret_cast<const T*>(&wv[j]);
     const float v[8] = {a[j].x, a[j].y, a[j].z, a[j].w, b[j].x, b[j].y, b[j].z, b[j].w};
     __align__(16) T o[8];
@@ -287,30 +282,27 @@ rmsnorm_cluster_kernel(const float* __restrict__ x, const T* __restrict__ w, T* 
       // PERM8: element e of the group sits at position [0,4,1,5,2,6,3,7]^-1 = perm8_pos(e) (compile-time after unrolling)
       if (perm) o[perm8_pos(e)] = r; else o[e] = r;
     }
-    yr[(int64_t)(j * C + rank) * 128 + tid] = *reinterpret_cast<uint4*>(o);
+    if (g < groups) yr[g] = *reinterpret_cast<uint4*>(o);
   }
 }
 
 bool pdl_enabled_gemm();      // the global PDL switch (b200p_set_pdl / B200P_PDL != 0): the early norms follow the GEMM launches
 
 template <typename T>
-static cudaError_t launch_rmsnorm_cluster(int C, int64_t M, cudaStream_t st, const float* x, const void* w, void* y, int64_t H,
-                                          float eps, int perm) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(M * C));
-  cfg.blockDim = dim3(128);
-  cfg.dynamicSmemBytes = 0;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = (unsigned)C;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[1].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = pdl_enabled_gemm() ? 2 : 1;       // without the attribute the griddepcontrol instructions are no-ops
-  return cudaLaunchKernelEx(&cfg, rmsnorm_cluster_kernel<T>, x, (const T*)w, (T*)y, H, eps, perm);
+static cudaError_t launch_rmsnorm_row(int64_t M, cudaStream_t st, const float* x, const void* w, void* y, int H, float eps, int perm) {
+  const auto go = [&](auto kern) {
+    return launch_pdl_opt(pdl_enabled_gemm(), kern, (unsigned)M, RMS_NT, 0, st, x, (const T*)w, (T*)y, H, eps, perm);
+  };
+  switch ((H / 8 + RMS_NT - 1) / RMS_NT) {
+    case 1: return go(rmsnorm_row_kernel<T, 1>);
+    case 2: return go(rmsnorm_row_kernel<T, 2>);
+    case 3: return go(rmsnorm_row_kernel<T, 3>);
+    case 4: return go(rmsnorm_row_kernel<T, 4>);
+    case 5: return go(rmsnorm_row_kernel<T, 5>);
+    case 6: return go(rmsnorm_row_kernel<T, 6>);
+    case 7: return go(rmsnorm_row_kernel<T, 7>);
+    default: return go(rmsnorm_row_kernel<T, 8>);
+  }
 }
 int sm_count();
 
@@ -327,24 +319,21 @@ extern "C" int b200p_rmsnorm(const float* x, const void* w, void* y, int64_t M, 
   B200P_REQUIRE(aligned(x, 16) && aligned(y, 16) && H % 4 == 0, B200P_ERR_ALIGN,
                 "rmsnorm needs 16-byte aligned rows (H %% 4 == 0)");
   if (M == 0) return B200P_OK;
-  // Which norm.  The one-pass cluster form (16-bit rows of 2048 * C elements, C in {1, 2, 4, 8}, at most one CTA per SM) is an
-  // "early" kernel and wins at every row count (B=1 T=8192 2.29 -> 2.22 ms, B=8 3.46 -> 3.41, B=64 T=256 2.88 -> 2.86).
-  // Where it does not apply, the two-pass early kernel pays from 16 rows on (the next kernel
-  // is then a tile GEMM that streams weights while it waits: B=64 T=256 2.91 -> 2.87 ms) and loses below (a 128-thread CTA is
-  // the slower norm and the GEMV after it gains nothing: B=1 T=8192 2.38 -> 2.43 ms).
-  static const int early_env = [] { const char* e = getenv("B200P_RMS_EARLY"); return e ? atoi(e) : -1; }();
-  static const int cluster_env = [] { const char* e = getenv("B200P_RMS_CLUSTER"); return e ? atoi(e) : 1; }();
-  const int64_t C = H / 2048;
-  const bool cluster_ok = cluster_env && dtype != B200P_F32 && H % 2048 == 0 && (C == 1 || C == 2 || C == 4 || C == 8) &&
-                          M * C <= sm_count() && aligned(w, 16);
-  const bool early = early_env >= 0 ? early_env != 0 : (M >= 16 || cluster_ok);
-  if (early && cluster_ok) {
-    cudaError_t e = dtype == B200P_F16
-        ? launch_rmsnorm_cluster<__half>((int)C, M, (cudaStream_t)stream, x, w, y, H, eps, perm)
-        : launch_rmsnorm_cluster<__nv_bfloat16>((int)C, M, (cudaStream_t)stream, x, w, y, H, eps, perm);
-    if (e != cudaSuccess) return cuda_fail(e, "rmsnorm_cluster_kernel");
+  // Which norm.  16-bit rows in whole groups of 8, up to 16384 wide: the one-pass kernel at every row count (a feed-forward of one
+  // row, 4096 wide: 34.2 -> 33.1 us, 5120 wide 48.4 -> 43.0; Qwen3-14B's step, 3 layers, B=8: 413 -> 354, of which the norms are
+  // about half; 4 layers, B=64: 611 us with rows split over clusters wherever the rows allow it, 594 in two passes, 592 so).
+  // Everything else: the two-pass kernel, its early form from 16 rows on (the next kernel is then a tile GEMM that streams weights
+  // while it waits) and not below (a 128-thread CTA is the slower norm and the GEMV after it gains nothing).
+  if (dtype != B200P_F32 && H % 8 == 0 && H > 0 && H <= 16384 && aligned(w, 16)) {
+    cudaStream_t st = (cudaStream_t)stream;
+    cudaError_t e;
+    if (dtype == B200P_F16) e = launch_rmsnorm_row<__half>(M, st, x, w, y, (int)H, eps, perm);
+    else e = launch_rmsnorm_row<__nv_bfloat16>(M, st, x, w, y, (int)H, eps, perm);
+    if (e != cudaSuccess) return cuda_fail(e, "rmsnorm_row_kernel");
     return B200P_OK;
   }
+  static const int early_env = [] { const char* e = getenv("B200P_RMS_EARLY"); return e ? atoi(e) : -1; }();
+  const bool early = early_env >= 0 ? early_env != 0 : M >= 16;
   if (early) {
     B200P_DISPATCH_DTYPE(dtype, T, (launch_pdl_opt(b200p::pdl_enabled_gemm(), rmsnorm_kernel<T, 128>, (unsigned)M, 128, 0, (cudaStream_t)stream,
                                        x, (const T*)w, (T*)y, H, eps, perm)));

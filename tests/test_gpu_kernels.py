@@ -214,6 +214,32 @@ def test_rmsnorm_variants_at_decode_sizes(ops, dtype, M, H, perm):
         assert rel_err(y[r], exp[r]) < {"float16": 1.1e-3, "bfloat16": 8.1e-3}[dtype], r
 
 
+@pytest.mark.parametrize("dtype", ["float16", "bfloat16"])
+@pytest.mark.parametrize("H", [8, 1016, 1024, 1032, 3584, 7176, 8192, 8200, 16384, 16392])   # groups per thread, both CTA sizes, beyond
+@pytest.mark.parametrize("M", [1, 17])
+def test_rmsnorm_one_pass_at_every_width(ops, dtype, H, M):
+    """16-bit rows of any number of whole groups of 8, plain and PERM8, against 64 bits; neighbours of the output stay as they were.
+
+    Tolerance per element: half an ulp of the storage type (relative ``u``), plus the fp32 arithmetic before it: a thread's 64
+    terms, 5 steps of the warp, 8 of the block, halved by the square root, and 5 more roundings, below 64 * 2^-24 together; plus
+    half the smallest subnormal of fp16."""
+    rng = np.random.default_rng(H + M)
+    x = rng.standard_normal((M, H)).astype(np.float32) * 3
+    x[M // 2] *= 50.0
+    w = ref.round_to(1 + 0.1 * rng.standard_normal(H), dtype)
+    want = x.astype(np.float64) / np.sqrt((x.astype(np.float64) ** 2).mean(1, keepdims=True) + 1e-5) * np.asarray(w, np.float64)
+    u = {"float16": 2.0 ** -11, "bfloat16": 2.0 ** -8}[dtype]
+    for perm in (False, True):
+        buf = torch.full((M + 2, H), 7.0, dtype=TD[dtype], device="cuda")
+        ops.rmsnorm(torch.from_numpy(x).cuda(), t_(w, dtype), 1e-5, out_perm=perm, out=buf[1:-1])
+        got = buf.float().cpu().numpy()
+        assert (got[0] == 7).all() and (got[-1] == 7).all()
+        y = got[1:-1]
+        if perm:
+            y = y.reshape(M, H // 8, 8)[:, :, [0, 2, 4, 6, 1, 3, 5, 7]].reshape(M, H)
+        assert (np.abs(y - want) <= np.abs(want) * (u + 64 * 2.0 ** -24) + 2.0 ** -25).all()
+
+
 @pytest.mark.parametrize("dtype,D,qk_norm", [("float16", 128, False), ("bfloat16", 128, True), ("float32", 16, False), ("float16", 64, True)])
 def test_rope_kv_append(ops, dtype, D, qk_norm):
     rng = np.random.default_rng(4)
