@@ -263,6 +263,19 @@ static int pick_splits(int64_t B, int Hkv, int64_t Tcap, int ctas_per_sm) {
   return best;
 }
 
+// Few key heads in all: CTAs of 256 keys leave most SMs without one, and a CTA's chain of tiles is then the kernel's time (1000 keys,
+// 8 key heads: 32 CTAs whose warps each walk 8 tiles).  So the keys are spread over up to 7/8 of the SMs, 64 of them (two tiles per
+// warp) per CTA at least.  Attention and reduction back to back, us, before -> so: B=1, 8 key heads, capacity 256 7.0 -> 5.4,
+// 512 8.4 -> 5.4, 1024 8.6 -> 5.8, 2048 8.7 -> 7.0; one key head, 2048 37 -> 7.6.  The lines: below 256 keys the reduction costs more than the split gives
+// (128 keys 5.3 whole, 5.4 in two); 17 or 18 splits of 8 heads are slower than 15 or 16 (1024 keys 6.5 / 5.8, 2048 7.7 / 7.0).
+static int spread_splits(int s, int64_t B, int Hkv, int64_t Tcap) {
+  if (Tcap < 256) return s;
+  const int64_t most = (int64_t)sm_count() * 7 / 8 / (B * Hkv);
+  int64_t want = Tcap / 64 < most ? Tcap / 64 : most;
+  if (want > AD_MAX_SPLITS) want = AD_MAX_SPLITS;
+  return want > s ? (int)want : s;
+}
+
 bool attn_decode_supported(int64_t L, int Hq, int Hkv, int D, int dtype) {
   return L == 1 && D == AD_D && (dtype == B200P_F16 || dtype == B200P_BF16) && Hq % Hkv == 0 && Hq / Hkv <= 16;
 }
@@ -309,7 +322,7 @@ static int launch_attn_decode(const void* q, const void* kc, const void* vc, con
   const int s8 = pick_splits(B, Hkv, Tcap, 1);
   const bool small = g_ad_warps ? g_ad_warps == 2 : (Tcap / s8 <= AD_SHORT_KEYS);
   if (small) {
-    const int s2 = pick_splits(B, Hkv, Tcap, 4);
+    const int s2 = spread_splits(pick_splits(B, Hkv, Tcap, 4), B, Hkv, Tcap);
     return launch_attn_decode_w<T, 2>(q, kc, vc, lengths, out, B, Hq, Hkv, Tcap, scale, out_perm, ws, s2, st);
   }
   return launch_attn_decode_w<T, 8>(q, kc, vc, lengths, out, B, Hq, Hkv, Tcap, scale, out_perm, ws, s8, st);

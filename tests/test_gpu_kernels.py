@@ -1008,6 +1008,20 @@ def test_attention_tensor_decode(ops, dtype, Hq, Hkv, lengths):
     assert rel_err(got, exp) < {"float16": 2e-3, "bfloat16": 1.2e-2}[dtype]
 
 
+@pytest.mark.parametrize("dtype,Hq,Hkv,lengths", [
+    ("float16", 16, 1, [251]),                  # 255 keys of capacity: whole; 256 and 257: in 64s
+    ("bfloat16", 16, 1, [252]),
+    ("float16", 32, 8, [253]),
+    ("bfloat16", 8, 8, [2040]),                 # as many splits as 7/8 of the SMs hold
+    ("float16", 4, 1, [2047, 0, 63, 64, 1000]), # 25 splits: most of them empty in the short rows
+    ("bfloat16", 4, 4, [700] * 32),             # as many (row, key head) pairs as SMs to spread over: not spread further
+])
+def test_attention_tensor_decode_spread_over_idle_sms(ops, dtype, Hq, Hkv, lengths):
+    """Few key heads in all: more splits of fewer keys, rows that end before most of the splits begin."""
+    got, exp = attn_case(ops, len(lengths), 1, Hq, Hkv, 128, lengths, dtype, path=2)
+    assert rel_err(got, exp) < {"float16": 2e-3, "bfloat16": 1.2e-2}[dtype]
+
+
 def test_attention_tensor_matches_generic(ops):
     a, _ = attn_case(ops, 2, 1, 8, 2, 128, [1000, 37], "float16", path=2, seed=9)
     g, _ = attn_case(ops, 2, 1, 8, 2, 128, [1000, 37], "float16", path=1, seed=9)
