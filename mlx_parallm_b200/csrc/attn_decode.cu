@@ -265,11 +265,13 @@ static int pick_splits(int64_t B, int Hkv, int64_t Tcap, int ctas_per_sm) {
 
 // Few key heads in all: CTAs of 256 keys leave most SMs without one, and a CTA's chain of tiles is then the kernel's time (1000 keys,
 // 8 key heads: 32 CTAs whose warps each walk 8 tiles).  So the keys are spread over up to 7/8 of the SMs, 64 of them (two tiles per
-// warp) per CTA at least.  Attention and reduction back to back, us, before -> so: B=1, 8 key heads, capacity 256 7.0 -> 5.4,
-// 512 8.4 -> 5.4, 1024 8.6 -> 5.8, 2048 8.7 -> 7.0; one key head, 2048 37 -> 7.6.  The lines: below 256 keys the reduction costs more than the split gives
-// (128 keys 5.3 whole, 5.4 in two); 17 or 18 splits of 8 heads are slower than 15 or 16 (1024 keys 6.5 / 5.8, 2048 7.7 / 7.0).
+// warp) per CTA at least.  Attention and reduction back to back, us, before -> so: B=1, 8 key heads, capacity 1024 8.6 -> 5.8,
+// 2048 8.7 -> 7.0; B=2, 512 8.4 -> 5.8; one key head, 2048 37 -> 7.6.  The lines: what ran whole, without a reduction, stays so below 768 keys: in a
+// captured step the split would pay from 256 keys on (256 7.0 / 5.4, 512 8.4 / 5.4, 128 5.3 / 5.4), but a call issued alone is bound by its launches
+// there, and one more of them costs it 2 (4 sequences of 163 keys behind rope and append 10.5 / 12.7).  17 or 18 splits of 8 heads are slower than 15 or
+// 16 (1024 keys 6.5 / 5.8, 2048 7.7 / 7.0).
 static int spread_splits(int s, int64_t B, int Hkv, int64_t Tcap) {
-  if (Tcap < 256) return s;
+  if (s == 1 && Tcap < 768) return s;
   const int64_t most = (int64_t)sm_count() * 7 / 8 / (B * Hkv);
   int64_t want = Tcap / 64 < most ? Tcap / 64 : most;
   if (want > AD_MAX_SPLITS) want = AD_MAX_SPLITS;

@@ -1009,9 +1009,10 @@ def test_attention_tensor_decode(ops, dtype, Hq, Hkv, lengths):
 
 
 @pytest.mark.parametrize("dtype,Hq,Hkv,lengths", [
-    ("float16", 16, 1, [251]),                  # 255 keys of capacity: whole; 256 and 257: in 64s
-    ("bfloat16", 16, 1, [252]),
-    ("float16", 32, 8, [253]),
+    ("float16", 16, 1, [763]),                  # 767 keys of capacity: whole; 768 and 769: in 64s
+    ("bfloat16", 16, 1, [764]),
+    ("float16", 32, 8, [765]),
+    ("float16", 32, 16, [508, 70]),             # 512 keys, two splits become eight
     ("bfloat16", 8, 8, [2040]),                 # as many splits as 7/8 of the SMs hold
     ("float16", 4, 1, [2047, 0, 63, 64, 1000]), # 25 splits: most of them empty in the short rows
     ("bfloat16", 4, 4, [700] * 32),             # as many (row, key head) pairs as SMs to spread over: not spread further
