@@ -556,6 +556,35 @@ def test_argmax_large_vocab_unaligned(ops):
     assert ops.argmax(t).tolist() == lg.argmax(-1).tolist()
 
 
+@pytest.mark.parametrize("B,V", [(1, 1), (2, 3), (1, 32), (3, 4101), (1, 32000), (5, 16384 * 8 + 4), (300, 70)])
+def test_argmax_and_probability_at_segment_edges(ops, B, V):
+    """Segments, loads and warps that are not full, rows that no 16-byte load reads, ties, NaN, rows of -inf and a row with +inf.
+
+    Tolerance of the probability: __expf is right to 2 ulp of its argument's product, here at most 2^-22 * 16, for two of them and two
+    roundings of each of the 20 sums in a chain: 1e-5 of the value."""
+    rng = np.random.default_rng(V)
+    for ld in (V, (V + 3) // 4 * 4, V + 1):
+        lg = (rng.standard_normal((B, V)) * 3).astype(np.float32)
+        lg[0, V // 2] = lg[0, V - 1] = 9.0                  # tie (the lower index wins)
+        if B > 1:
+            lg[1] = -np.inf
+        if B > 2:
+            lg[2, ::2] = np.nan
+        buf = torch.full((B, ld), 50.0, device="cuda")
+        buf[:, :V] = torch.from_numpy(lg)
+        probs = torch.full((B,), -1.0, device="cuda")
+        tok = ops.argmax(buf[:, :V], probs_out=probs).tolist()
+        fin = np.where(np.isnan(lg), -np.inf, lg).astype(np.float64)
+        assert tok == fin.argmax(-1).tolist()
+        with np.errstate(invalid="ignore"):
+            want = 1.0 / np.exp(fin - fin.max(-1, keepdims=True)).sum(-1)
+        want[np.isnan(want)] = 0.0                          # nothing but -inf
+        assert np.allclose(probs.cpu().numpy(), want, rtol=1e-5, atol=0)
+        buf[0, V // 3] = float("inf")
+        tok = ops.argmax(buf[:, :V], probs_out=probs)
+        assert int(tok[0]) == V // 3 and float(probs[0]) == 0.0
+
+
 @pytest.mark.parametrize("top_p,temp", [(0.9, 1.0), (0.5, 0.7), (1.0, 1.3)])
 def test_top_p_sampling_distribution(ops, top_p, temp):
     """Distributional parity (A.7: MLX's threefry stream is not reproducible outside MLX): draws must stay in
