@@ -543,6 +543,14 @@ __device__ __forceinline__ void dc_operand(const float (&c)[4], float (&hi)[4], 
   lo[0] = l0.x, lo[1] = l1.x, lo[2] = l0.y, lo[3] = l1.y;
 }
 
+// Columns of a head are dealt to the slices evenly, the first ones one more: never above DC_COLS (slices = columns / DC_COLS, rounded up), and two slices
+// or more have at least DC_COLS / 2 each.  (A remainder of its own in the last slice could be narrower than DC_MIN_DV: 3088 columns in 49 slices of 63, 64.)
+struct DcSlice { int z0, n; };
+__device__ __forceinline__ DcSlice dc_slice(int dv, int slices, int z) {
+  const int base = dv / slices, more = dv % slices;
+  return {z * base + min(z, more), base + (z < more ? 1 : 0)};
+}
+
 // channel d of a chunk's keys, queries and decays; tokens past the end are ones that change nothing
 template <int MODE>
 __device__ __forceinline__ void dc_fetch(const float* __restrict__ qn, const float* __restrict__ kn, const float* __restrict__ decay, int tc, int t1, int h, int kh,
@@ -580,8 +588,8 @@ delta_triangle_kernel(const float* __restrict__ qn, const float* __restrict__ kn
   pdl_launch_dependents();
   const int t0 = cu[blockIdx.x], t1 = cu[blockIdx.x + 1];
   if (t1 - t0 < least) return;
-  const int kh = h / (H / KH), wide = (dv + slices - 1) / slices, last = dv - (slices - 1) * wide, tok = lane & 15;
-  const int per_wide = 65535 / wide + 1, per_last = 65535 / last + 1;          // i / w = (i * per) >> 16 for i < 272, w <= 64
+  const int kh = h / (H / KH), tok = lane & 15, wide = dc_slice(dv, slices, 0).n, narrow = dc_slice(dv, slices, slices - 1).n;
+  const int per_wide = 65535 / wide + 1, per_narrow = 65535 / narrow + 1;      // i / w = (i * per) >> 16 for i < 272, w <= 64
   float* scratch = scratch_all[w];
   // where this lane's two sums of tokens of one quarter go: lane = 16 * (quarter of two) + (0 .. 5: A of pairs, 6 .. 11: P of them, 12 .. 15: P of the diagonal)
   const int idx = lane & 15, pair = idx < 6 ? idx : idx - 6;
@@ -703,11 +711,11 @@ delta_triangle_kernel(const float* __restrict__ qn, const float* __restrict__ kn
     __syncthreads();
     const int m = min(DC_CHUNK, t1 - tc), numbers = m * (m + 1);
     for (int z = 0; z < slices; ++z) {
-      const int wz = z + 1 < slices ? wide : last;
-      float* dst = o + ((int64_t)tc * H + h) * dv + z * wide;
+      const DcSlice sl = dc_slice(dv, slices, z);
+      float* dst = o + ((int64_t)tc * H + h) * dv + sl.z0;
       for (int i = d; i < numbers; i += DC_TEAM) {
-        const int r = (i * (z + 1 < slices ? per_wide : per_last)) >> 16;
-        dst[(int64_t)r * H * dv + (i - r * wz)] = out[i];
+        const int r = (i * (sl.n == wide ? per_wide : per_narrow)) >> 16;
+        dst[(int64_t)r * H * dv + (i - r * sl.n)] = out[i];
       }
     }
     __syncthreads();
@@ -807,7 +815,8 @@ delta_chunk_kernel(const float* __restrict__ qn, const float* __restrict__ kn, c
   const int t0 = cu[e], t1 = cu[e + 1];
   if (t1 - t0 < least) return;
   const int row = rows[e], kh = h / (H / KH), chunks = (t1 - t0 + DC_CHUNK - 1) / DC_CHUNK;
-  const int z0 = (int)blockIdx.z * ((dv + (int)gridDim.z - 1) / (int)gridDim.z), z1 = min(dv, z0 + (dv + (int)gridDim.z - 1) / (int)gridDim.z);
+  const DcSlice sl = dc_slice(dv, (int)gridDim.z, (int)blockIdx.z);
+  const int z0 = sl.z0, z1 = z0 + sl.n;
   if (warp >= DC_STATE_WARPS) {
     // ===================================== vectors =====================================
     const int d = threadIdx.x - 32 * DC_STATE_WARPS;           // key channel

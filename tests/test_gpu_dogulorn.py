@@ -956,6 +956,32 @@ def test_delta_scan_in_chunks(mode, dk, dv, in_place):
     assert torch.equal(state2[[0, 2, 3]], state[[0, 2, 3]]) and state2[1].isnan().any()
 
 
+@pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("dv", [65, 3088, 4097])                # two slices; a remainder of 16, of 1 beside slices of 64
+def test_delta_scan_in_chunks_of_wide_values(mode, dv):
+    """A chunk's intermediate numbers lie in each slice of its rows of the output, so every slice has to be wide enough for them: against float64 with the
+    recurrence's fp32 bound; rows behind the output stay as they were."""
+    from mlx_parallm_b200 import ops
+    dk, lens = 128, [33, 48]
+    g, nb, M = torch.Generator(device="cuda").manual_seed(dv + mode), len(lens), sum(lens)
+    rnd = lambda *sh: torch.randn(*sh, generator=g, device="cuda")        # noqa: E731
+    qn, kn, v = rnd(M, dk) / dk ** 0.5, torch.nn.functional.normalize(rnd(M, dk), dim=-1), rnd(M, dv)
+    beta, decay = torch.rand(M, 1, generator=g, device="cuda"), 0.5 + 0.5 * torch.rand(M, dk if mode else 1, generator=g, device="cuda")
+    i32 = dict(dtype=torch.int32, device="cuda")
+    cu, rows, lengths, state0 = torch.tensor([0, 33, M], **i32), torch.arange(nb, **i32), torch.full((nb,), 3, **i32), rnd(nb, 1, dk, dv) * 0.3
+    state, buf = state0.clone(), torch.full((M + 300, dv), 7.0, device="cuda")
+    ops.delta_scan(qn, kn, v, beta, decay, state, cu, rows, lengths, buf[:M], nb, 1, 1, dk, dv, mode, longest=max(lens))
+    assert bool((buf[M:] == 7).all())
+    for e, (a, b) in enumerate([(0, 33), (33, M)]):
+        S = state0[e, 0].double()
+        for t in range(a, b):
+            S = S * decay[t].double().view(-1, 1)
+            u = beta[t].double() * (v[t].double() - S.t() @ kn[t].double())
+            S = S + kn[t].double().view(-1, 1) * u
+            assert (buf[t].double() - S.t() @ qn[t].double()).abs().max() < 2e-5
+        assert (state[e, 0].double() - S).abs().max() < 2e-5
+
+
 @pytest.mark.parametrize("M,N,K,batch", [(1, 64, 128, 9), (2, 512, 128, 16), (5, 128, 512, 64), (8, 130, 512, 3), (3, 128, 1024, 40), (1, 128, 520, 64)])
 def test_gemv_of_short_rows(M, N, K, batch):
     """Few rows over many short weight rows (per-head products): one piece of a row at a time; from 512 channels, where the CTAs fit the GPU
