@@ -813,7 +813,10 @@ delta_chunk_kernel(const float* __restrict__ qn, const float* __restrict__ kn, c
   const int e = blockIdx.x, h = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   pdl_launch_dependents();
   const int t0 = cu[e], t1 = cu[e + 1];
-  if (t1 - t0 < least) return;
+  if (t1 - t0 < least) {
+    if ((blockIdx.x | blockIdx.y | blockIdx.z) == 0) pdl_wait();       // (this grid ends no earlier than the launch before, also where no entry is long)
+    return;
+  }
   const int row = rows[e], kh = h / (H / KH), chunks = (t1 - t0 + DC_CHUNK - 1) / DC_CHUNK;
   const DcSlice sl = dc_slice(dv, (int)gridDim.z, (int)blockIdx.z);
   const int z0 = sl.z0, z1 = z0 + sl.n;
