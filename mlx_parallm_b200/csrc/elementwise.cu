@@ -230,8 +230,8 @@ rmsnorm_kernel(const float* __restrict__ x, const T* __restrict__ w, T* __restri
 // The norm of 16-bit rows in ONE pass: a CTA of 256 threads per row, every thread keeps its NG groups of 8 elements in registers
 // between the sum of squares and the output.  What bounds a norm of a decode step is a chain of latencies, not bytes: launch, one
 // round trip for the row, the block's sum, the store.  So the dependents are released first (the matrix kernel that follows sets
-// itself up and streams its weights meanwhile), the norm's own weights, which no kernel before it writes, are loaded before the
-// wait, and all loads of a row are in flight at once.  256 threads and up to 8 groups: 128 threads are as fast or faster back to
+// itself up and streams its weights meanwhile), and all loads of a row are in flight at once, the norm's own weights among them (behind the
+// wait: the kernel before may be the one that writes them; ahead of it, or brought into L2 there, they gain nothing).  256 threads and up to 8 groups: 128 threads are as fast or faster back to
 // back (8192 wide, 64 rows: 1.9 us against 2.6), yet slower in a step, where each norm waits for its row (Qwen3-14B at B=24,
 // 3 layers: 400 us against 389); 512 threads are the same in a step and slower from some 300 rows on (5120 wide, 4096 rows: 32 us
 // against 22).  Back to back, us, before (the two-pass kernel above or, for whole multiples of 2048 and up to one CTA per SM, a
@@ -243,25 +243,25 @@ rmsnorm_kernel(const float* __restrict__ x, const T* __restrict__ w, T* __restri
 constexpr int RMS_NT = 256;
 template <typename T, int NG>
 __global__ void __launch_bounds__(RMS_NT)
-rmsnorm_row_kernel(const float* __restrict__ x, const T* __restrict__ w, T* __restrict__ y, int H, float eps, int perm) {
+rmsnorm_row_kernel(const float* x, const T* w, T* __restrict__ y, int H, float eps, int perm) {
   static_assert(sizeof(T) == 2, "16-bit outputs only");
   __shared__ float sh[33];
   pdl_launch_dependents();
   const int groups = H / 8;
-  uint4 wv[NG];
-#pragma unroll
-  for (int j = 0; j < NG; ++j) {
-    const int g = j * RMS_NT + threadIdx.x;
-    wv[j] = g < groups ? reinterpret_cast<const uint4*>(w)[g] : make_uint4(0u, 0u, 0u, 0u);
-  }
   pdl_wait();
   const float4* xr = reinterpret_cast<const float4*>(x + (int64_t)blockIdx.x * H);
   float4 a[NG], b[NG];
+  uint4 wv[NG];
 #pragma unroll
   for (int j = 0; j < NG; ++j) {
     const int g = j * RMS_NT + threadIdx.x;
     a[j] = b[j] = make_float4(0.f, 0.f, 0.f, 0.f);
     if (g < groups) a[j] = xr[2 * g], b[j] = xr[2 * g + 1];
+  }
+#pragma unroll
+  for (int j = 0; j < NG; ++j) {
+    const int g = j * RMS_NT + threadIdx.x;
+    wv[j] = g < groups ? reinterpret_cast<const uint4*>(w)[g] : make_uint4(0u, 0u, 0u, 0u);
   }
   float ss = 0.f;
 #pragma unroll

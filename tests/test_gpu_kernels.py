@@ -240,6 +240,35 @@ def test_rmsnorm_one_pass_at_every_width(ops, dtype, H, M):
         assert (np.abs(y - want) <= np.abs(want) * (u + 64 * 2.0 ** -24) + 2.0 ** -25).all()
 
 
+@pytest.mark.parametrize("H", [1024, 4096, 5120, 8192, 16384])
+def test_rmsnorm_of_weights_that_the_kernel_before_writes(ops, H):
+    """A norm that starts while the kernel before it still runs reads nothing of its, weights included: chains of two norms, the second's weights an output of the
+    first, give the bits of the same calls one at a time."""
+    g, n = torch.Generator(device="cuda").manual_seed(H), 24
+    x = torch.randn(n, 150, H, generator=g, device="cuda")
+    row, w0 = torch.randn(1, H, generator=g, device="cuda"), torch.randn(H, generator=g, device="cuda").bfloat16()
+
+    def chain(apart):
+        buf, outs = torch.full((150, H), 3.0, dtype=torch.bfloat16, device="cuda"), torch.empty(n, 1, H, dtype=torch.bfloat16, device="cuda")
+        for i in range(n):
+            ops.rmsnorm(x[i], w0, 1e-5, out=buf)
+            if apart:
+                torch.cuda.synchronize()
+            ops.rmsnorm(row, buf[149], 1e-5, out=outs[i])
+            if apart:
+                torch.cuda.synchronize()
+        return outs
+
+    want = chain(True)
+    assert torch.equal(chain(False), want)
+    graph, stream = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    with torch.cuda.graph(graph, stream=stream):
+        got = chain(False)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(got, want)
+
+
 @pytest.mark.parametrize("dtype,D,qk_norm", [("float16", 128, False), ("bfloat16", 128, True), ("float32", 16, False), ("float16", 64, True)])
 def test_rope_kv_append(ops, dtype, D, qk_norm):
     rng = np.random.default_rng(4)
