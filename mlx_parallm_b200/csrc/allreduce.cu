@@ -123,8 +123,8 @@ __device__ __forceinline__ void peer_handshake(const ArPeers& pe, int W, int ran
 // one CTA per row (grid-stride over rows); dynamic shared memory: H floats (the summed row) + 33 reduction slots
 template <typename T, int W>
 __global__ void __launch_bounds__(AR_THREADS)
-allreduce_residual_rmsnorm_kernel(const ArPeers pe, int rank, uint32_t* status, float* __restrict__ h, const T* __restrict__ nw,
-                                  T* __restrict__ y, float* __restrict__ zero_buf, int64_t M, int64_t H, int64_t ldp,
+allreduce_residual_rmsnorm_kernel(const ArPeers pe, int rank, uint32_t* status, float* h, const T* nw,
+                                  T* __restrict__ y, float* zero_buf, int64_t M, int64_t H, int64_t ldp,
                                   float eps, int perm) {
   extern __shared__ __align__(16) float ar_sm[];
   float* row = ar_sm;
@@ -202,8 +202,8 @@ struct ArPeersX {
 
 template <typename T, int W>
 __global__ void __launch_bounds__(AR_THREADS)
-allreduce_rows_rmsnorm_kernel(const ArPeers pe, const ArPeersX px, int rank, uint32_t* status, float* __restrict__ h,
-                              const T* __restrict__ nw, float* __restrict__ zero_buf, int64_t M, int64_t H, int64_t ldp,
+allreduce_rows_rmsnorm_kernel(const ArPeers pe, const ArPeersX px, int rank, uint32_t* status, float* h,
+                              const T* nw, float* zero_buf, int64_t M, int64_t H, int64_t ldp,
                               int64_t rpr, float eps, int perm) {
   extern __shared__ __align__(16) float ar_sm[];
   float* row = ar_sm;

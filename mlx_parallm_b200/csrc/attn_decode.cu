@@ -38,8 +38,8 @@ constexpr int AD_MAX_SPLITS = 32;                                 // at most one
 
 template <typename T, int AD_WARPS>
 __global__ void __launch_bounds__(AD_WARPS * 32, AD_WARPS == 8 ? 1 : 4)
-attn_decode_kernel(const T* __restrict__ q, const T* __restrict__ kc, const T* __restrict__ vc,
-                   const int32_t* __restrict__ lengths, T* __restrict__ out, float* __restrict__ ws, int Hq, int Hkv,
+attn_decode_kernel(const T* q, const T* kc, const T* vc,
+                   const int32_t* lengths, T* __restrict__ out, float* __restrict__ ws, int Hq, int Hkv,
                    int64_t Tcap, float scale_log2e, int splits, int out_perm, int early) {
   extern __shared__ __align__(128) uint8_t smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -222,7 +222,7 @@ attn_decode_kernel(const T* __restrict__ q, const T* __restrict__ kc, const T* _
 // picks factor s up with a shuffle.  (The serial form took 5.5 us for 32 splits at B = 1, T = 8192.)
 template <typename T>
 __global__ void __launch_bounds__(AD_D)
-attn_reduce_kernel(const float* __restrict__ ws, T* __restrict__ out, int splits, int out_perm) {
+attn_reduce_kernel(const float* ws, T* __restrict__ out, int splits, int out_perm) {
   pdl_wait();
   const int64_t bh = blockIdx.x;
   const int d = threadIdx.x, lane = threadIdx.x & 31;

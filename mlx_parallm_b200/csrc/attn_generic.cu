@@ -22,8 +22,8 @@ __device__ __forceinline__ void load_vec(const T* p, float (&v)[EPL], bool act) 
 
 template <typename T, int EPL>
 __global__ void __launch_bounds__(128)
-attn_generic_kernel(const T* __restrict__ q, const T* __restrict__ kc, const T* __restrict__ vc,
-                    const int32_t* __restrict__ lengths, T* __restrict__ out, int L, int Hq, int Hkv, int D,
+attn_generic_kernel(const T* q, const T* kc, const T* vc,
+                    const int32_t* lengths, T* __restrict__ out, int L, int Hq, int Hkv, int D,
                     int64_t Tcap, float scale, int out_perm) {
   __shared__ float sh_m[4], sh_l[4];
   __shared__ float sh_acc[4][32 * EPL];

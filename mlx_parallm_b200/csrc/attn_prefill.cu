@@ -28,8 +28,8 @@ constexpr int AP_SMEM = AP_STAGES * 2 * AP_TILE_BYTES;   // 64 KB
 
 template <typename T>
 __global__ void __launch_bounds__(AP_THREADS)
-attn_prefill_kernel(const T* __restrict__ q, const T* __restrict__ kc, const T* __restrict__ vc,
-                    const int32_t* __restrict__ lengths, T* __restrict__ out, int L, int Hq, int Hkv, int64_t Tcap,
+attn_prefill_kernel(const T* q, const T* kc, const T* vc,
+                    const int32_t* lengths, T* __restrict__ out, int L, int Hq, int Hkv, int64_t Tcap,
                     float scale_log2e, int out_perm) {
   extern __shared__ __align__(128) uint8_t smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;

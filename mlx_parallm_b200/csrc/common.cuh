@@ -165,6 +165,8 @@ __host__ __device__ __forceinline__ int perm8_pos(int n) { return (n & ~7) | (((
 
 // Programmatic dependent launch: wait for the producer grid's memory to be visible / allow the
 // consumer grid to start its prologue.  No-ops when the launch carries no PDL attribute.
+// What a kernel reads behind its wait it does not take through __restrict__ pointers: the promise that nothing else writes there while the kernel
+// runs is not true before the wait, and lets the compiler move the reads above it (a norm in which it did so read the row of the step before).
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

@@ -26,9 +26,9 @@ __device__ __forceinline__ float dq_one(uint32_t q, float s, float b) {
 // so there is no 64-bit division on the index path; the row index comes from `rows` (gather) or is the identity.
 template <typename T, int BITS, int MODE, typename OUT>
 __global__ void __launch_bounds__(256)
-dequant_kernel(const uint32_t* __restrict__ w, const T* __restrict__ scales,
-               const T* __restrict__ biases, OUT* __restrict__ out,
-               const int32_t* __restrict__ rows, int64_t row0, int64_t V, int64_t K, int gs) {
+dequant_kernel(const uint32_t* w, const T* scales,
+               const T* biases, OUT* __restrict__ out,
+               const int32_t* rows, int64_t row0, int64_t V, int64_t K, int gs) {
   constexpr int PER = 32 / BITS;
   const int words_per_row = (int)(K / PER);
   const int w0 = (blockIdx.x * blockDim.x + threadIdx.x) * 4;          // first of this thread's 4 words
@@ -177,7 +177,7 @@ __device__ __forceinline__ float block_sum(float v, float* sh) {
 // waiting for its own producer -- the GEMM that follows the norm is then scheduled while the GEMM before the norm drains.
 template <typename T, int NT>
 __global__ void __launch_bounds__(NT, NT == 128 ? 16 : 1)
-rmsnorm_kernel(const float* __restrict__ x, const T* __restrict__ w, T* __restrict__ y, int64_t H, float eps, int perm) {
+rmsnorm_kernel(const float* x, const T* w, T* __restrict__ y, int64_t H, float eps, int perm) {
   __shared__ float sh[33];
   if constexpr (NT == 128) pdl_launch_dependents();
   pdl_wait();
@@ -361,9 +361,9 @@ __device__ unsigned int g_kv_overflow = 0;
 // projection (b200p_qmm with ADD_RESIDUAL into a zeroed buffer): values are rounded to T first (the rounding the
 // reference's projection output has) and the buffer is re-zeroed behind the read, ready for the next step.
 template <typename T, typename TIN>
-__global__ void rope_kv_append_kernel(TIN* __restrict__ qkv, T* __restrict__ q_out, T* __restrict__ kc,
-                                      T* __restrict__ vc, const int32_t* __restrict__ lengths,
-                                      const T* __restrict__ qn_w, const T* __restrict__ kn_w, int L, int Hq,
+__global__ void rope_kv_append_kernel(TIN* qkv, T* __restrict__ q_out, T* __restrict__ kc,
+                                      T* __restrict__ vc, const int32_t* lengths,
+                                      const T* qn_w, const T* kn_w, int L, int Hq,
                                       int Hkv, int D, int64_t Tcap, float log2_base, float rope_scale,
                                       float eps) {
   __shared__ float sh[33];
@@ -439,8 +439,8 @@ __global__ void rope_kv_append_kernel(TIN* __restrict__ qkv, T* __restrict__ q_o
 // against 14.6 us for the generic kernel above.)
 template <typename T, typename TIN>
 __global__ void __launch_bounds__(256)
-rope_kv_append_d128_kernel(TIN* __restrict__ qkv, T* __restrict__ q_out, T* __restrict__ kc, T* __restrict__ vc,
-                           const int32_t* __restrict__ lengths, const T* __restrict__ qn_w, const T* __restrict__ kn_w,
+rope_kv_append_d128_kernel(TIN* qkv, T* __restrict__ q_out, T* __restrict__ kc, T* __restrict__ vc,
+                           const int32_t* lengths, const T* qn_w, const T* kn_w,
                            int L, int Hq, int Hkv, int64_t Tcap, float log2_base, float rope_scale, float eps) {
   constexpr int D = 128, HALF = 64;
   constexpr bool ACC_IN = std::is_same<TIN, float>::value && !std::is_same<T, float>::value;
@@ -529,8 +529,8 @@ rope_kv_append_d128_kernel(TIN* __restrict__ qkv, T* __restrict__ q_out, T* __re
 // 57.5 (5.7 TB/s).
 template <typename T>
 __global__ void __launch_bounds__(256, 4)
-rope_kv_append_rows_kernel(const T* __restrict__ qkv, T* __restrict__ q_out, T* __restrict__ kc, T* __restrict__ vc,
-                           const int32_t* __restrict__ lengths, const T* __restrict__ qn_w, const T* __restrict__ kn_w, int M, int L,
+rope_kv_append_rows_kernel(const T* qkv, T* __restrict__ q_out, T* __restrict__ kc, T* __restrict__ vc,
+                           const int32_t* lengths, const T* qn_w, const T* kn_w, int M, int L,
                            int Hq, int Hkv, int64_t Tcap, float log2_base, float rope_scale, float eps, int tpc_log2) {
   constexpr int D = 128, HALF = 64;
   pdl_launch_dependents();                                  // (the attention behind it sets itself up meanwhile)
@@ -625,7 +625,7 @@ rope_kv_append_rows_kernel(const T* __restrict__ qkv, T* __restrict__ q_out, T* 
 // (models/llama.py:165); the buffer is re-zeroed behind the read.  One thread per aligned group of 8 outputs.
 template <typename T>
 __global__ void __launch_bounds__(256)
-silu_mul_kernel(float* __restrict__ gu, T* __restrict__ out, int64_t M, int64_t I, int64_t ldg, int64_t ldo, int perm) {
+silu_mul_kernel(float* gu, T* __restrict__ out, int64_t M, int64_t I, int64_t ldg, int64_t ldo, int perm) {
   pdl_wait();
   const int64_t groups = I / 8;
   const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;

@@ -23,7 +23,7 @@ constexpr int LR_NSLICE = 512;                  // output columns per CTA
 
 template <typename T, bool OUT_F32>
 __global__ void __launch_bounds__(LR_THREADS)
-lora_add_kernel(const T* __restrict__ x, const T* __restrict__ At, const T* __restrict__ Bt, void* __restrict__ yv, int M,
+lora_add_kernel(const T* x, const T* At, const T* Bt, void* yv, int M,
                 int64_t N, int64_t K, int64_t ldx, int64_t ldy, int64_t col0, float scale) {
   __shared__ float part[LR_WARPS][16][LR_R + 1];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;

@@ -73,7 +73,7 @@ __device__ __forceinline__ void moe_route_token(const float* __restrict__ logits
 }
 
 template <int PER_LANE>
-__global__ void moe_route_kernel(const float* __restrict__ logits, int64_t ldl, const float* __restrict__ bias,
+__global__ void moe_route_kernel(const float* logits, int64_t ldl, const float* bias,
                                  int32_t* __restrict__ ids, float* __restrict__ wts, int64_t M, int E, int top) {
   const int lane = threadIdx.x & 31;
   const int64_t t = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -94,7 +94,7 @@ __global__ void moe_route_kernel(const float* __restrict__ logits, int64_t ldl, 
 // its largest; only the experts of the `keep` best groups can be picked (the others count as -inf, since picking scores may be
 // negative).  The `top` largest picking scores win, ties to the smaller index; weights w_k = s_k / (sum of the picked s + 1e-20) *
 // scale.  softmax: s = softmax(z) over ALL experts, picked (and groups compared) by z, which orders the experts as s does.
-__global__ void moe_route_scores_kernel(const float* __restrict__ logits, int64_t ldl, const float* __restrict__ correction,
+__global__ void moe_route_scores_kernel(const float* logits, int64_t ldl, const float* correction,
                                          int32_t* __restrict__ ids, float* __restrict__ wts, int64_t M, int E, int top, int count,
                                          int keep, float scale, int renorm, int softmax, int group_best) {
   extern __shared__ float mr_sm[];
@@ -233,7 +233,7 @@ __device__ __forceinline__ void moe_plan(F id_of, int32_t* cnt, int32_t* __restr
   }
 }
 
-__global__ void moe_plan_kernel(const int32_t* __restrict__ ids, int32_t* __restrict__ seg, int32_t* __restrict__ slot_of,
+__global__ void moe_plan_kernel(const int32_t* ids, int32_t* __restrict__ seg, int32_t* __restrict__ slot_of,
                                 int32_t* __restrict__ token_of, int64_t n, int E, int top) {
   extern __shared__ int32_t cnt[];               // [E] counts, then [E] cursors
   pdl_launch_dependents();
@@ -245,7 +245,7 @@ __global__ void moe_plan_kernel(const int32_t* __restrict__ ids, int32_t* __rest
 constexpr int MOE_ONE_BLOCK = 64;                // (token, choice) pairs
 template <int PER_LANE>
 __global__ void __launch_bounds__(1024)
-moe_route_plan_kernel(const float* __restrict__ logits, int64_t ldl, const float* __restrict__ bias, int32_t* __restrict__ ids,
+moe_route_plan_kernel(const float* logits, int64_t ldl, const float* bias, int32_t* __restrict__ ids,
                       float* __restrict__ wts, int32_t* __restrict__ seg, int32_t* __restrict__ slot_of, int32_t* __restrict__ token_of,
                       int64_t M, int E, int top) {
   extern __shared__ int32_t cnt[];               // [E] counts, then [E] cursors
@@ -266,14 +266,23 @@ moe_route_plan_kernel(const float* __restrict__ logits, int64_t ldl, const float
 }
 
 template <typename T>
-__global__ void moe_gather_kernel(const T* __restrict__ x, const int32_t* __restrict__ token_of, T* __restrict__ xs, int64_t W) {
+__global__ void moe_gather_kernel(const T* x, const int32_t* token_of, T* __restrict__ xs, int64_t W) {
   const int64_t s = blockIdx.x;
   pdl_launch_dependents();
   pdl_wait();
   const T* src = x + (int64_t)token_of[s] * W;
   T* dst = xs + s * W;
   if (W % 8 == 0 && sizeof(T) == 2) {
-    for (int64_t c = threadIdx.x * 8; c < W; c += blockDim.x * 8) *reinterpret_cast<uint4*>(dst + c) = *reinterpret_cast<const uint4*>(src + c);
+    const int64_t step = blockDim.x * 8;
+    for (int64_t c = threadIdx.x * 8; c < W; c += 4 * step) {          // (four pieces in flight)
+      uint4 v[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (c + k * step < W) v[k] = *reinterpret_cast<const uint4*>(src + c + k * step);
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (c + k * step < W) *reinterpret_cast<uint4*>(dst + c + k * step) = v[k];
+    }
   } else {
     for (int64_t c = threadIdx.x; c < W; c += blockDim.x) dst[c] = src[c];
   }
@@ -282,7 +291,7 @@ __global__ void moe_gather_kernel(const T* __restrict__ x, const int32_t* __rest
 // xs[slot_of[t, k], :] = wts[t, k] * x[t, :]: designs whose routing weight multiplies the expert's INPUT (the product is
 // formed in fp32 and rounded once to the storage type)
 template <typename T>
-__global__ void moe_scatter_scaled_kernel(const T* __restrict__ x, const int32_t* __restrict__ slot_of, const float* __restrict__ wts,
+__global__ void moe_scatter_scaled_kernel(const T* x, const int32_t* slot_of, const float* wts,
                                           T* __restrict__ xs, int64_t W) {
   const int64_t i = blockIdx.x;                        // (token, choice)
   const int top = gridDim.y;

@@ -63,8 +63,8 @@ __device__ __forceinline__ void bulk_reduce_add_f32(float* dst, uint32_t src_sme
 
 template <typename T, int NT, bool XPERM>
 __global__ void __launch_bounds__(QG_WARPS * 32, 2)
-qmm_mma_kernel(const T* __restrict__ x, const uint32_t* __restrict__ w, const T* __restrict__ scales,
-               const T* __restrict__ biases, float* __restrict__ y, int M, int64_t N, int64_t K, int64_t ldx, int64_t ldy,
+qmm_mma_kernel(const T* x, const uint32_t* __restrict__ w, const T* __restrict__ scales,
+               const T* __restrict__ biases, float* y, int M, int64_t N, int64_t K, int64_t ldx, int64_t ldy,
                int splits, int steps_per_split) {
   extern __shared__ __align__(128) uint8_t smem[];
   constexpr int TOK = NT * 8;

@@ -37,8 +37,8 @@ __device__ __forceinline__ float silu_f(float g) { return g / (1.0f + __expf(-g)
 // grid.x = ceil(pairs / 4) with pairs = N/2 ; block = 128 (4 warps, one row pair each)
 template <typename T, int BITS, int MB, int EPI>
 __global__ void __launch_bounds__(128)
-qmv_kernel(const T* __restrict__ x, const uint32_t* __restrict__ w, const T* __restrict__ scales,
-           const T* __restrict__ biases, void* __restrict__ yv, int m_valid, int64_t N, int64_t K,
+qmv_kernel(const T* x, const uint32_t* __restrict__ w, const T* __restrict__ scales,
+           const T* __restrict__ biases, void* yv, int m_valid, int64_t N, int64_t K,
            int64_t ldx, int64_t ldy, int gs, int flags) {
   constexpr int WPL = (32 / BITS) * 4;  // weights per lane per 128-bit load
   const int lane = threadIdx.x & 31;

@@ -52,8 +52,8 @@ constexpr int QM_STEP_K = 256;
 // silu(g) * u as one 16-bit value, in the PERM8 column order if y_perm; never K-split.
 template <typename T, int NT, bool XPERM, int MODE>
 __global__ void __launch_bounds__(QM_WARPS * 32)
-qmv_mma_kernel(const T* __restrict__ x, const uint32_t* __restrict__ w, const T* __restrict__ scales,
-               const T* __restrict__ biases, float* __restrict__ y, int M, int64_t N, int64_t K, int64_t ldx, int64_t ldy,
+qmv_mma_kernel(const T* x, const uint32_t* __restrict__ w, const T* __restrict__ scales,
+               const T* __restrict__ biases, float* y, int M, int64_t N, int64_t K, int64_t ldx, int64_t ldy,
                int splits, int steps_per_split, int y_perm) {
   constexpr bool ATOMIC = MODE == 1;
   constexpr bool SILU = MODE == 2;

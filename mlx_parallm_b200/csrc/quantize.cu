@@ -13,7 +13,7 @@ template <typename T> __device__ __forceinline__ float rt(float v) { return Tr<T
 
 template <typename T, int BITS>
 __global__ void __launch_bounds__(256)
-quantize_kernel(const T* __restrict__ w, uint32_t* __restrict__ wq, T* __restrict__ scales, T* __restrict__ biases, int64_t N,
+quantize_kernel(const T* w, uint32_t* __restrict__ wq, T* __restrict__ scales, T* __restrict__ biases, int64_t N,
                 int64_t K, int gs) {
   constexpr int PER = 32 / BITS;                       // codes per word = elements per thread
   const int tpg = gs / PER;                            // threads per group: 4..32, a power of two

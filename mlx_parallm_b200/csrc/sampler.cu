@@ -93,7 +93,7 @@ __device__ __forceinline__ void row_visit(const float* __restrict__ row, int64_t
 
 // grid (S, B), cluster (S, 1, 1): CTA `rank` of the cluster takes segment `rank` of row blockIdx.y
 __global__ void __launch_bounds__(SAMP_THREADS)
-argmax_kernel(const float* __restrict__ logits, int32_t* __restrict__ tokens, float* __restrict__ probs_out,
+argmax_kernel(const float* logits, int32_t* __restrict__ tokens, float* __restrict__ probs_out,
               int64_t V, int64_t ldl, float4* __restrict__ rec_out, int vocab_offset) {
   __shared__ float shv[32];
   __shared__ int shi[32];
@@ -184,7 +184,7 @@ argmax_kernel(const float* __restrict__ logits, int32_t* __restrict__ tokens, fl
 
 // merge W per-shard records per row: highest max wins, lowest global index among ties (shards hold
 // ascending vocab ranges, so this is mx.argmax's lowest-index rule); prob = 1 / sum_r s_r exp(m_r - M).
-__global__ void argmax_merge_kernel(const float4* __restrict__ recs, int32_t* __restrict__ tokens,
+__global__ void argmax_merge_kernel(const float4* recs, int32_t* __restrict__ tokens,
                                     float* __restrict__ probs_out, int W, int64_t B) {
   pdl_wait();
   const int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -269,7 +269,7 @@ constexpr int TP_XCH = TP_BINS + 2;               // 64 digit masses + Z + Z1
 
 // grid (S, B), cluster (S, 1, 1): CTA `rank` takes segment `rank` of row blockIdx.y in every pass
 __global__ void __launch_bounds__(TP_THREADS)
-top_p_kernel(const float* __restrict__ logits, int32_t* __restrict__ tokens, float* __restrict__ probs_out,
+top_p_kernel(const float* logits, int32_t* __restrict__ tokens, float* __restrict__ probs_out,
              int64_t V, int64_t ldl, float inv_temp, float top_p, uint64_t seed, uint64_t offset) {
   extern __shared__ float lhist[];                 // [TP_BINS][TP_THREADS]
   __shared__ float sh[32];
