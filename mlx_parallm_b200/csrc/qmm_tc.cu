@@ -97,14 +97,14 @@ struct TcParams {
   void* y;
   float* ws_part;      // stream-K partial tiles: [grid][2 slots][2 blocks][TN tokens][128 rows] fp32 (no initial state)
   int* ws_counter;     // {arrived, done} per output tile (zero on entry, left zero)
-  int M_tok, N, K, TN;
-  int row0;            // first output row of the launch (SILU_MUL: gate row)
-  int64_t ldy;
+  int M_tok, N, TN;
+  int up, rows;        // SILU_MUL: matrix row of the first up row; rows of the matrix (all relative to the launch's first row)
   int epi;
+  int64_t ldy;
   int y_perm;          // 1: 16-bit outputs (STORE / SILU_MUL) are written in the PERM8 column order
   int num_kb;          // K / 64
   int num_st;          // stages along K = ceil(num_kb / KPS)
-  int pairs, tiles_m;  // output tile t = pair * tiles_m + token tile
+  int tiles_m;         // output tile t = pair * tiles_m + token tile
   int R;               // weight rows per MMA block of a tile (multiple of 8, <= 128): a tile is R + R rows
   int S;               // K splits per tile (1: whole tiles; > 1 only when tiles * S <= grid, one item per CTA)
   int items;           // work items = tiles * S; CTA c takes items c, c + G, c + 2G, ...
@@ -117,6 +117,10 @@ struct TcParams {
   uint32_t zero;       // 0, which the compiler does not know: a slot is handed back (and overwritten by the copy engine) only when what was read
                        // from it has arrived in registers, the address of the arrival depends on it (what happens otherwise: qmm_wide.cu)
 };
+
+// Above 128 bytes the compiler keeps the parameters in memory and their values in local copies: 100 to 250 bytes of spills in every variant, 2 to 4 % of
+// the time of all shapes (28672 x 4096 8 bits at 64 tokens 33.7 / 32.9 us).
+static_assert(sizeof(TcParams) <= 128, "kernel parameters that the compiler takes apart");
 
 // work item -> (output tile, stage range): item = tile * S + split, split covers stages [split*num_st/S, (split+1)*num_st/S)
 // The stages of an item are visited in ROTATED order, starting at stage s0 + rot: CTAs that walk K in lockstep (all at the
@@ -287,8 +291,8 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
     for (int item = cta; item < p.items; item += G) {
      const TcSeg sg = seg_of(p, item);
      const int pair = sg.tile / p.tiles_m;
-     const int rowA0 = p.row0 + (silu ? pair * p.R : pair * 2 * p.R);
-     const int rowB0 = p.row0 + (silu ? p.N / 2 + pair * p.R : pair * 2 * p.R + p.R);
+     const int rowA0 = silu ? pair * p.R : pair * 2 * p.R;
+     const int rowB0 = silu ? p.up + pair * p.R : pair * 2 * p.R + p.R;
      for (int i = 0; i < sg.ns; ++i) {
       const int st = seg_stage(sg, i);
       if (p.sb_tma && (i == 0 || st == sg.s0 || (st % SPG) == 0)) {     // a new group of 8 k-blocks starts with this stage
@@ -513,8 +517,8 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
       } else {
         // scale rows are not 16-byte multiples (K % 512 != 0, e.g. a TP shard): read them from global memory
         const int pair = tile / p.tiles_m;
-        const int grow = (blk ? (p.row0 + (silu ? p.N / 2 + pair * p.R : pair * 2 * p.R + p.R)) : (p.row0 + (silu ? pair * p.R : pair * 2 * p.R))) + r;
-        const bool row_ok = grow < p.N && r < p.R;
+        const int grow = (blk ? (silu ? p.up + pair * p.R : pair * 2 * p.R + p.R) : (silu ? pair * p.R : pair * 2 * p.R)) + r;
+        const bool row_ok = grow < p.rows && r < p.R;
         const T* sp = reinterpret_cast<const T*>(p.scales) + (int64_t)(row_ok ? grow : 0) * p.num_kb;
         const T* bp = reinterpret_cast<const T*>(p.biases) + (int64_t)(row_ok ? grow : 0) * p.num_kb;
         const T zero = Tr<T>::from_f(0.f);
@@ -546,8 +550,8 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
       mbar_wait(accum_full(buf), (uint32_t)((seg / NBUF) & 1));
       tc_fence_after();
       const uint32_t lane_base = tmem_base + ((uint32_t)(q * 32) << 16);
-      tc_drain_tile<T, FAST>(p, silu, r, lane_base + d_col(buf, 0), lane_base + d_col(buf, 1), TN, p.row0 + (silu ? pair * p.R : pair * 2 * p.R),
-                             p.row0 + (silu ? p.N / 2 + pair * p.R : pair * 2 * p.R + p.R), tm * TN, 1 + grp, 1 + DQ_WARPS / 4);
+      tc_drain_tile<T, FAST>(p, silu, r, lane_base + d_col(buf, 0), lane_base + d_col(buf, 1), TN, silu ? pair * p.R : pair * 2 * p.R,
+                             silu ? p.up + pair * p.R : pair * 2 * p.R + p.R, tm * TN, 1 + grp, 1 + DQ_WARPS / 4);
     }
   } else {
     // ===================================== epilogue warps ===================================
@@ -568,8 +572,8 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
       const TcSeg sg = seg_of(p, item);
       const int tile = sg.tile;
       const int pair = tile / p.tiles_m, tm = tile % p.tiles_m;
-      const int rowA0 = p.row0 + (silu ? pair * p.R : pair * 2 * p.R);
-      const int rowB0 = p.row0 + (silu ? p.N / 2 + pair * p.R : pair * 2 * p.R + p.R);
+      const int rowA0 = silu ? pair * p.R : pair * 2 * p.R;
+      const int rowB0 = silu ? p.up + pair * p.R : pair * 2 * p.R + p.R;
       const int tok0 = tm * TN;
       const int buf = NBUF == 2 ? (seg & 1) : 0;
       const bool full = p.S == 1;
@@ -623,8 +627,8 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
       }
       named_bar_sync(2, EPI_THREADS);
       const int pair = tile / p.tiles_m, tm = tile % p.tiles_m;
-      const int rowA0 = p.row0 + (silu ? pair * p.R : pair * 2 * p.R);
-      const int rowB0 = p.row0 + (silu ? p.N / 2 + pair * p.R : pair * 2 * p.R + p.R);
+      const int rowA0 = silu ? pair * p.R : pair * 2 * p.R;
+      const int rowB0 = silu ? p.up + pair * p.R : pair * 2 * p.R + p.R;
       const int tok0 = tm * TN;
       for (int t0 = me * EPI_TOK; t0 < TN; t0 += S * EPI_TOK) {
         if (tok0 + t0 >= p.M_tok) break;               // padding tokens of the last token tile
@@ -869,13 +873,20 @@ static int encode_2d_raw(TcEncodeFn enc, CUtensorMap* tm, CUtensorMapDataType dt
   return B200P_OK;
 }
 
-// row0: the first output row to compute (SILU_MUL: gate row, with its up row), a multiple of 8
+// row0: the first output row to compute (SILU_MUL: gate row, with its up row), a multiple of 8.  It goes into the pointers.
 int qmm_tc_launch(const void* x, const uint32_t* w, const void* s, const void* b, void* y, int64_t M, int64_t N,
                   int64_t K, int64_t ldx, int64_t ldy, int bits, int dtype, int epi, int flags, void* ws, size_t ws_bytes,
                   int64_t row0, cudaStream_t st) {
   TcEncodeFn enc = tc_get_encode();
   B200P_REQUIRE(enc != nullptr, B200P_ERR_CUDA, "cuTensorMapEncodeTiled entry point not available");
-  TcPlan pl = make_plan(M, N - (epi == B200P_EPI_SILU_MUL ? 2 : 1) * row0, K, bits, epi);
+  const int64_t up = N / 2;
+  w += row0 * (K * bits / 32);
+  s = reinterpret_cast<const char*>(s) + row0 * (K / 64) * 2;
+  b = reinterpret_cast<const char*>(b) + row0 * (K / 64) * 2;
+  y = reinterpret_cast<char*>(y) + row0 * (epi == B200P_EPI_STORE_F32 || epi == B200P_EPI_ADD_RESIDUAL ? 4 : 2);
+  const int64_t rows = N - row0;
+  N -= (epi == B200P_EPI_SILU_MUL ? 2 : 1) * row0;
+  TcPlan pl = make_plan(M, N, K, bits, epi);
   B200P_REQUIRE(pl.w_stages >= 2, B200P_ERR_ARG, "shared memory too small for the tensor path");
   const bool x_perm = (flags & B200P_X_PERM8) != 0, y_perm = (flags & B200P_Y_PERM8) != 0;
   B200P_REQUIRE(!x_perm || bits == 4, B200P_ERR_ARG, "B200P_X_PERM8 is the 4-bit activation layout");
@@ -886,17 +897,17 @@ int qmm_tc_launch(const void* x, const uint32_t* w, const void* s, const void* b
   const CUtensorMapDataType dt16 = dtype == B200P_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
   const bool fast = (flags & B200P_W_SMALLSCALE) != 0;
   CUtensorMap tms[4];
-  int rc = tc_encode_2d(enc, &tms[0], CU_TENSOR_MAP_DATA_TYPE_UINT8, w, (uint64_t)(K * bits / 8), (uint64_t)N,
+  int rc = tc_encode_2d(enc, &tms[0], CU_TENSOR_MAP_DATA_TYPE_UINT8, w, (uint64_t)(K * bits / 8), (uint64_t)rows,
                      (uint64_t)(K * bits / 8), 128u, (uint32_t)pl.R, CU_TENSOR_MAP_SWIZZLE_128B, "weights");
   if (rc) return rc;
   rc = tc_encode_2d(enc, &tms[1], dt16, x, (uint64_t)K, (uint64_t)M, (uint64_t)(ldx * 2), 64u, (uint32_t)pl.TN,
                  CU_TENSOR_MAP_SWIZZLE_128B, "x");
   if (rc) return rc;
   if (sb_tma) {
-    rc = tc_encode_2d(enc, &tms[2], dt16, s, (uint64_t)num_kb, (uint64_t)N, (uint64_t)num_kb * 2, 8u, (uint32_t)pl.R,
+    rc = tc_encode_2d(enc, &tms[2], dt16, s, (uint64_t)num_kb, (uint64_t)rows, (uint64_t)num_kb * 2, 8u, (uint32_t)pl.R,
                    CU_TENSOR_MAP_SWIZZLE_NONE, "scales");
     if (rc) return rc;
-    rc = tc_encode_2d(enc, &tms[3], dt16, b, (uint64_t)num_kb, (uint64_t)N, (uint64_t)num_kb * 2, 8u, (uint32_t)pl.R,
+    rc = tc_encode_2d(enc, &tms[3], dt16, b, (uint64_t)num_kb, (uint64_t)rows, (uint64_t)num_kb * 2, 8u, (uint32_t)pl.R,
                    CU_TENSOR_MAP_SWIZZLE_NONE, "biases");
     if (rc) return rc;
   } else {
@@ -916,9 +927,9 @@ int qmm_tc_launch(const void* x, const uint32_t* w, const void* s, const void* b
   }
   p.ws_counter = reinterpret_cast<int*>(ws);
   p.ws_part = reinterpret_cast<float*>(reinterpret_cast<char*>(ws) + counters);
-  p.M_tok = (int)M; p.N = (int)N; p.K = (int)K; p.TN = pl.TN; p.row0 = (int)row0; p.ldy = ldy; p.epi = epi; p.y_perm = y_perm ? 1 : 0;
+  p.M_tok = (int)M; p.N = (int)N; p.TN = pl.TN; p.up = (int)up; p.rows = (int)rows; p.ldy = ldy; p.epi = epi; p.y_perm = y_perm ? 1 : 0;
   B200P_REQUIRE((int64_t)pl.pairs * pl.tiles_m * pl.S < (1ll << 30), B200P_ERR_ARG, "problem too large for the tensor path");
-  p.num_kb = num_kb; p.pairs = pl.pairs; p.tiles_m = pl.tiles_m; p.R = pl.R; p.S = pl.S; p.items = pl.items; p.rotate = g_rotate; p.nbuf = pl.nbuf; p.a_slots = pl.a_slots;
+  p.num_kb = num_kb; p.tiles_m = pl.tiles_m; p.R = pl.R; p.S = pl.S; p.items = pl.items; p.rotate = g_rotate; p.nbuf = pl.nbuf; p.a_slots = pl.a_slots;
   p.num_st = (p.num_kb + (bits == 4 ? 4 : 2) - 1) / (bits == 4 ? 4 : 2);
   p.sb_tma = sb_tma ? 1 : 0;
   p.w_stages = pl.w_stages; p.x_slots = pl.x_slots;
