@@ -469,15 +469,17 @@ struct Plan { int tiles_m, TN, H0, H1, row_blocks, left, items, grid, w_stages, 
 
 // Row blocks of a short last round of whole tiles that are left to the kernel that splits K (qmm_tc.cu): row_blocks x tiles_m just above a multiple of the
 // SMs is common (57344 gated rows are 448 blocks, three times 148 and four), and the few CTAs of the last round then take as long as all of one before.
-// Behind the other launch the split one costs about 30000 cycles and its share of K; a round takes a k-block about 640 cycles with 8-bit codes, 400 or
-// the MMAs' time with 4.  So only long rounds are worth it (us, whole tiles / left: 57344 x 8192 8 bits at 129 / 201 / 300 / 600 tokens 188 / 172, 207 / 189,
-// 308 / 294, 509 / 497, but 1349 / 1377 at 1300, 13 rounds; 28672 x 4096 4 bits 96.3 / 97.5 at 300, 303 / 350 at 1500).
+// Behind the other launch the split one costs about 30000 cycles and its share of K; a round takes a k-block about 640 cycles with 8-bit codes.  So only
+// long rounds are worth it (us, whole tiles / left, 8 bits: 57344 x 8192 at 129 / 201 / 300 / 600 tokens 190 / 174, 209 / 192, 319 / 303, 500 / 492, but
+// 1349 / 1377 at 1300, 13 rounds; 19072 x 8192 at 201 / 600 / 1500 119 / 90, 209 / 196, 446 / 433; 22016 x 8192 at 201 115 / 105; 28672 x 8192 at 300
+// 210 / 187), and never at 4 bits, whose rounds are shorter (28672 x 4096 96.3 / 97.5 at 300, 303 / 350 at 1500).
 static int left_over(int row_blocks, int tiles_m, int tn, int64_t M, int64_t K, int bits) {
+  if (bits != 8) return 0;
   const int sms = sm_count(), items = row_blocks * tiles_m, whole = items / sms * sms;
   if (whole == 0 || whole == items || whole > 9 * sms) return 0;
   const int left = row_blocks - whole / tiles_m;
   const int64_t tiles = (int64_t)(left + 1) / 2 * ((M + 127) / 128), splits = sms / tiles < 16 ? sms / tiles : 16;
-  const double kb = (double)(K / 64), round = kb * std::max(2.0 * tn, bits == 8 ? 640.0 : 400.0);
+  const double kb = (double)(K / 64), round = kb * std::max(2.0 * tn, 640.0);
   return splits >= 4 && 30000.0 + 700.0 * kb / (double)splits < 0.6 * round ? left : 0;
 }
 

@@ -897,6 +897,17 @@ def test_qmm_wide_tiles_leave_a_short_last_round(ops, M, N, K, bits, epi):
         assert float(err.max()) < 1.5e-2 and not bool(ws[:4096].any())
 
 
+def test_qmm_wide_tiles_at_4_bits_keep_their_last_round(ops):
+    """Rounds of 4-bit tiles are too short for a second launch: 744 row blocks, five rounds of 148 and four blocks, in one launch that leaves the workspace alone."""
+    M, N, K = 256, 744 * 128, 8192
+    g = torch.Generator(device="cuda").manual_seed(N)
+    w = torch.randint(-2 ** 31, 2 ** 31, (N, K // 8), generator=g, device="cuda", dtype=torch.int64).to(torch.int32)
+    s = ((torch.rand((N, K // 64), generator=g, device="cuda") + 0.5) * 2 / 15 / K ** 0.5).bfloat16()
+    x, ws = torch.randn((M, K), generator=g, device="cuda").bfloat16(), torch.zeros(ops.qmm_workspace_bytes(M, N, K), dtype=torch.uint8, device="cuda")
+    got = ops.qmm(x, w, s, (-s.float() * 15 / 2).bfloat16(), 64, 4, 0, workspace=ws, small_scale=True)
+    assert bool(got.isfinite().all()) and not bool(ws.any())
+
+
 @pytest.mark.parametrize("M,N,K,bits,dtype", [(201, 2048, 4096, 8, "bfloat16"), (250, 18944, 1024, 8, "bfloat16"), (300, 4096, 2048, 4, "float16")])
 def test_qmm_wide_tiles_repeat_bit_for_bit(ops, M, N, K, bits, dtype):
     """Whole tiles are summed in a fixed order: hundreds of launches over the same operands agree in every bit.  (A k-block of one row that is
