@@ -723,7 +723,7 @@ static TcPlan make_plan(int64_t M, int64_t N, int64_t K, int bits, int epi) {
   // of the cost model / 128: 152064 x 5120 122.3 / 101.2 and 147 / 119 with R = 88, 34816 x 5120 26.2 / 25.9 with 120, 28672 x 4096 21.0 / 20.3 with 104,
   // 5120 x 5120 12.3 / 11.9).  8 bits stream twice the bytes in that time and gain from even shares (57344 x 8192: 97.5 with 104, 106.7 with 128).
   const bool whole = bits == 4 && (rows + (silu ? 127 : 255)) / (silu ? 128 : 256) >= 16;
-  for (int R = whole ? 128 : 8; R <= 128; R += 8) {
+  for (int R = whole && !g_force_R ? 128 : 8; R <= 128; R += 8) {
     if (g_force_R && R != g_force_R) continue;
     const int64_t pairs = silu ? (rows + R - 1) / R : (rows + 2 * R - 1) / (2 * R);
     const int64_t tiles = pairs * pl.tiles_m;

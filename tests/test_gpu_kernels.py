@@ -943,6 +943,23 @@ def test_qmm_units_of_two_k_blocks(ops, M, N, K, dtype, epi, small):
     assert rel_err(got, exp) < {"float16": 3e-3, "bfloat16": 2e-2}[dtype]
 
 
+def test_qmm_forced_tiles():
+    """B200P_TC_R and B200P_TC_S force rows per block and K splits, also on 4-bit matrices that take whole blocks by themselves: two splits meet in the workspace."""
+    import os
+    import subprocess
+    import sys
+    code = ("import torch\nfrom mlx_parallm_b200 import ops, _lib\n_lib.lib().b200p_qmm_set_path(2)\n"
+            "w = torch.randint(-2**31, 2**31 - 1, (4096, 512), device='cuda', dtype=torch.int32)\n"
+            "s, x = torch.full((4096, 64), 0.001, device='cuda').half(), torch.randn(24, 4096, device='cuda').half()\n"
+            "ws = torch.zeros(ops.qmm_workspace_bytes(24, 4096, 4096), dtype=torch.uint8, device='cuda')\n"
+            "y = ops.qmm(x, w, s, -s, 64, 4, 0, workspace=ws)\nprint(bool(y.isfinite().all()), bool(ws[4096:].any()))\n")
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    for splits, used in (("1", "False"), ("2", "True")):
+        env = dict(os.environ, PYTHONPATH=root, B200P_TC_R="64", B200P_TC_S=splits)
+        out = subprocess.run([sys.executable, "-c", code], env=env, capture_output=True, text=True, timeout=300)
+        assert out.stdout.split() == ["True", used], out.stdout + out.stderr
+
+
 @pytest.mark.parametrize("M,N,K,bits,dtype", [(250, 18944, 1024, 8, "bfloat16"), (64, 8192, 4096, 4, "float16"), (40, 4096, 8192, 8, "bfloat16"), (1, 8192, 8192, 4, "bfloat16")])
 def test_qmm_between_memory_bound_kernels(ops, M, N, K, bits, dtype):
     """A product that starts while an elementwise kernel still fills the SM's memory pipeline: the weights' slots must not be refilled
