@@ -85,7 +85,7 @@ template <typename T, int BITS, bool XPERM, bool FAST, int UKB>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 qmm_sk_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x,
               const __grid_constant__ CUtensorMap tm_s, const __grid_constant__ CUtensorMap tm_b,
-              const __grid_constant__ CUtensorMap tm_y, const TcParams p) {
+              const __grid_constant__ CUtensorMap tm_y, const __grid_constant__ TcParams p) {
   constexpr int PKB = 64 * BITS / 8;            // packed bytes per row per k-block
   constexpr int KPS = 128 / PKB;                // k-blocks per stage (a stage row is one 128-byte line)
   constexpr int SPG = 8 / KPS;                  // stages per scale/bias group of 8 k-blocks
@@ -104,8 +104,8 @@ qmm_sk_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
   const int NBUF = TN > 64 ? 1 : 2;              // D buffers: buffer d, block b at columns (2d + b) * d_stride
   const uint32_t d_stride = TN <= 32 ? 32u : (TN <= 64 ? 64u : 128u);
   constexpr uint32_t A_SLOT = UKB * 64;          // columns: [k-block][weight block][32]
-  const uint32_t A_COL0 = 512u - (uint32_t)p.a_slots * A_SLOT;   // the A ring sits at the top of TMEM
-  const uint32_t a_slots = (uint32_t)p.a_slots;
+  const uint32_t A_COL0 = UKB == 1 ? 256u : 512u - (uint32_t)p.a_slots * A_SLOT;   // the A ring sits at the top of TMEM
+  const uint32_t a_slots = UKB == 1 ? 4u : (uint32_t)p.a_slots;           // (a constant where the plan has one value: registers)
   auto full_w = [&](int s) { return bar_base + 8u * s; };
   auto empty_w = [&](int s) { return bar_base + 8u * (MAX_STAGES + s); };
   auto full_x = [&](int s) { return bar_base + 8u * (2 * MAX_STAGES + s); };
@@ -348,19 +348,24 @@ qmm_sk_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
         const T* bp = reinterpret_cast<const T*>(p.biases) + (int64_t)(row_ok ? grow : 0) * p.num_kb;
         const T zero = Tr<T>::from_f(0.f);
         for (int st = s0; st < s0 + ns; ++st) {
-          uint32_t sv[NU][UKB], bv[NU][UKB];
+          T sv[NU][UKB], bv[NU][UKB];
 #pragma unroll
           for (int n = 0; n < NU; ++n)
 #pragma unroll
             for (int j = 0; j < UKB; ++j) {
               const int kb = st * KPS + (kpar + 2 * n) * UKB + j;
               const bool ok = row_ok && kb < p.num_kb;        // k-blocks past K are zero-filled by TMA: A = 0
-              sv[n][j] = dup16(ok ? __ldg(sp + kb) : zero);
-              bv[n][j] = dup16(ok ? __ldg(bp + kb) : zero);
+              sv[n][j] = ok ? __ldg(sp + kb) : zero;
+              bv[n][j] = ok ? __ldg(bp + kb) : zero;
             }
           fetch_stage();
 #pragma unroll
-          for (int n = 0; n < NU; ++n) unit(n, sv[n], bv[n]);
+          for (int n = 0; n < NU; ++n) {
+            uint32_t s2[UKB], b2[UKB];
+#pragma unroll
+            for (int j = 0; j < UKB; ++j) s2[j] = dup16(sv[n][j]), b2[j] = dup16(bv[n][j]);
+            unit(n, s2, b2);
+          }
         }
       }
       u += ns;

@@ -524,19 +524,24 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
         const T zero = Tr<T>::from_f(0.f);
         for (int i = 0; i < ns; ++i) {
           const int st = seg_stage(sg, i);
-          uint32_t sv[NU][UKB], bv[NU][UKB];
+          T sv[NU][UKB], bv[NU][UKB];
 #pragma unroll
           for (int n = 0; n < NU; ++n)
 #pragma unroll
             for (int j = 0; j < UKB; ++j) {
               const int kb = st * KPS + (kpar + 2 * n) * UKB + j;
               const bool ok = row_ok && kb < p.num_kb;        // k-blocks past K are zero-filled by TMA: A = 0
-              sv[n][j] = dup16(ok ? __ldg(sp + kb) : zero);
-              bv[n][j] = dup16(ok ? __ldg(bp + kb) : zero);
+              sv[n][j] = ok ? __ldg(sp + kb) : zero;
+              bv[n][j] = ok ? __ldg(bp + kb) : zero;
             }
           fetch_stage();
 #pragma unroll
-          for (int n = 0; n < NU; ++n) unit(n, sv[n], bv[n]);
+          for (int n = 0; n < NU; ++n) {
+            uint32_t s2[UKB], b2[UKB];
+#pragma unroll
+            for (int j = 0; j < UKB; ++j) s2[j] = dup16(sv[n][j]), b2[j] = dup16(bv[n][j]);
+            unit(n, s2, b2);
+          }
         }
       }
     }
@@ -719,9 +724,9 @@ static TcPlan make_plan(int64_t M, int64_t N, int64_t K, int bits, int epi) {
   // partly filled warp still cost issue slots, and a K split pays for writing + re-reading its fp32 partial tile.
   double best = 1e30;
   pl.R = 128; pl.S = 1;
-  // 4 bits, matrices of 16 tiles and more (2368 x 3584 lost 4 %): a k-block takes a CTA its handshakes and latencies, about the same for 80 rows as for 128, so whole blocks always (us at 24 / 64 tokens, R
-  // of the cost model / 128: 152064 x 5120 122.3 / 101.2 and 147 / 119 with R = 88, 34816 x 5120 26.2 / 25.9 with 120, 28672 x 4096 21.0 / 20.3 with 104,
-  // 5120 x 5120 12.3 / 11.9).  8 bits stream twice the bytes in that time and gain from even shares (57344 x 8192: 97.5 with 104, 106.7 with 128).
+  // 4 bits, matrices of 16 tiles and more (2368 x 3584 lost 4 %): a k-block takes a CTA its handshakes and latencies, about the same for 80 rows as for 128,
+  // so whole blocks always (us at 24 / 64 / 128 tokens, R of the cost model / 128: 152064 x 5120 122 / 101, 147 / 119, 247 / 195 with R = 88, 34816 x 5120
+  // 26.2 / 25.9 at 24 and 40.5 / 40.2 at 128 with 120, 28672 x 4096 21.0 / 20.3 and 33.0 / 31.3 with 104, 128256 x 4096 157 / 147 at 128).  8 bits stream twice the bytes in that time and gain from even shares (57344 x 8192: 97.5 with 104, 106.7 with 128).
   const bool whole = bits == 4 && (rows + (silu ? 127 : 255)) / (silu ? 128 : 256) >= 16;
   for (int R = whole && !g_force_R ? 128 : 8; R <= 128; R += 8) {
     if (g_force_R && R != g_force_R) continue;
@@ -753,8 +758,12 @@ static TcPlan make_plan(int64_t M, int64_t N, int64_t K, int bits, int epi) {
   pl.nbuf = (tn > 64 || items <= sms) ? 1 : 2;
   if (g_force_nbuf && tn <= 64) pl.nbuf = g_force_nbuf;
   // k-blocks per unit of the A and X rings.  Above 96 tokens the MMAs take longer than the dequantisation, and what is left of TMEM holds two large
-  // units or four small ones: 4096 x 14336 at 128 tokens 19.3 / 18.8 us.
-  const int ukb = pl.ukb = bits == 4 && tn <= 96 ? 2 : 1;
+  // units or four small ones: 4096 x 14336 at 128 tokens 19.3 / 18.8 us.  Small matrices, whose K is split: units of two pay where a CTA has more than a
+  // stage or so of K, up to 64 tokens (us at 24 / 64 / 96 tokens, one / two k-blocks: 3072 x 8192, 2.7 stages each, 13.1 / 12.7, 14.5 / 14.2, 17.6 / 18.3;
+  // 1536 x 7168, 1.8 stages, 11.8 / 11.7, 13.3 / 13.1, 14.2 / 14.5; one stage each: 2048 x 4096 11.4 / 11.8, 12.5 / 12.6, 13.4 / 13.7).
+  const int64_t stages = (K / 64 + 3) / 4;
+  const bool two = whole ? tn <= 96 : bits == 4 && tn <= 64 && 2 * stages >= 3 * pl.S;
+  const int ukb = pl.ukb = two ? 2 : 1;
   pl.a_slots = (512 - pl.nbuf * 2 * d_stride) / (64 * ukb);
   if (ukb == 1) pl.a_slots &= ~1;
   if (pl.a_slots > NSLOT) pl.a_slots = NSLOT;
