@@ -12,6 +12,8 @@
 // An entry's bits depend on its own tokens alone, with two exceptions: beside at least as many empty entries as it has tokens, in a call that
 // does not say how long its longest entry is, it goes token by token (delta_step_kernel); with 16 to 31 tokens, in a call that says that its longest entry
 // has 32 or more, it goes with that one.
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace b200p {
@@ -508,39 +510,58 @@ delta_scan_kernel(const float* __restrict__ qn, const float* __restrict__ kn, co
 // beforehand for all chunks at once (delta_triangle_kernel).  Every quotient of decays is a product of the decays in between: never above one, no
 // division.
 //
-// All of it keeps fp32's accuracy: an operand is the sum of two tf32 numbers (the nearest one and the rest), a product three MMAs (high . high,
-// low . high, high . low; what is left out is below 2^-22 of it), and as an MMA cuts its sum off instead of rounding it, the large products are
-// summed over 32 channels at most before a rounding addition takes over.  Relative error of o / the state against 64 bits, 512 tokens, 128 x 128: 1.7e-7 / 1.5e-7
-// with decays as a layer has them, 1.9e-7 / 2.1e-7 with decays of 0.98 to 1 (token by token 0.8e-7 / 0.8e-7 and 1.6e-7 / 2.2e-7; sums left to the MMA alone
-// 7e-7 and 1.1e-6).
+// All of it keeps fp32's accuracy.  An operand is the sum of three bf16 numbers, which hold all of its 24 bits, a product six MMAs (what is left out is below
+// 2^-25 of it); the MMAs cut their sums off instead of rounding them, so the leading products of 16 channels, which hardly lose a bit, meet the others in
+// rounding additions.  What a token's output hangs on most, its own value and its own key and query, passes no MMA: the diagonals of both triangles
+// (b_t of U = X + (T - I) X with X = diag(b) (...), and P_tt) are fp32 FMAs.  Relative error of o / the state against 64 bits, 128 x 128, decays per
+// channel, two tokens at a time in fp32 (the kernel before) -> so: decays as a layer has them, 512 tokens 7.9e-8 / 7.8e-8 -> 7.9e-8 / 7.7e-8, 600 tokens 7.9e-8 /
+// 8.3e-8 -> 7.9e-8 / 7.4e-8, 33 to 100 tokens 8.7e-8 / 8.5e-8 -> 8.4e-8 / 7.6e-8; of 0.98 to 1, 512 tokens 1.6e-7 / 2.2e-7 -> 1.2e-7 / 1.4e-7; of 0.9996 to 1
+// 3.5e-7 / 5.2e-7 -> 2.0e-7 / 2.7e-7.  Two tf32 numbers an operand and three MMAs a product take 12 % less time and have twice the error with a layer's
+// decays (1.6e-7 / 1.5e-7): an operand then loses the last of its bits.
 constexpr int DC_MIN = 32, DC_CHUNK = 16, DC_COLS = 64, DC_TEAM = 128;
 constexpr int DC_MIN_DV = DC_CHUNK + 1;                        // a chunk of m tokens keeps T and P, m (m + 1) numbers, in its m rows of o until o is written
 
-__device__ __forceinline__ void dc_mma(float (&d)[4], const float (&a)[4], float b0, float b1) {
-  asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-      : "r"(__float_as_uint(a[0])), "r"(__float_as_uint(a[1])), "r"(__float_as_uint(a[2])), "r"(__float_as_uint(a[3])), "r"(__float_as_uint(b0)),
-        "r"(__float_as_uint(b1)));
+// k = 16: A [16, 16], B [16, 8]; k = 8: the first halves of both
+__device__ __forceinline__ void dc_mma(float (&d)[4], const uint32_t (&a)[4], uint2 b) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b.x), "r"(b.y));
 }
-__device__ __forceinline__ void dc_mma0(float (&d)[4], const float (&a)[4], float b0, float b1) {
-  asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
-      : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
-      : "r"(__float_as_uint(a[0])), "r"(__float_as_uint(a[1])), "r"(__float_as_uint(a[2])), "r"(__float_as_uint(a[3])), "r"(__float_as_uint(b0)),
-        "r"(__float_as_uint(b1)), "f"(0.f));
+__device__ __forceinline__ void dc_mma0(float (&d)[4], const uint32_t (&a)[4], uint2 b) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+      : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b.x), "r"(b.y), "f"(0.f));
 }
-// x = high + low: the nearest tf32 number and what is left (the MMA drops the last two of its 13 bits)
-__device__ __forceinline__ float dc_high(float x) { return __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xffffe000u); }
-__device__ __forceinline__ void dc_split(float2 x, float2& hi, float2& lo) {
-  hi = make_float2(dc_high(x.x), dc_high(x.y));
-  lo = make_float2(x.x - hi.x, x.y - hi.y);
+__device__ __forceinline__ void dc_mma(float (&d)[4], const uint32_t (&a)[4], uint32_t b) {
+  asm("mma.sync.aligned.m16n8k8.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(b));
 }
-// an accumulator's columns 2 t, 2 t + 1 as the A operand's t, t + 4 (the MMA's k index is a label: B is laid out for it)
-__device__ __forceinline__ void dc_operand(const float (&c)[4], float (&hi)[4], float (&lo)[4]) {
-  float2 h0, h1, l0, l1;
-  dc_split(make_float2(c[0], c[1]), h0, l0);
-  dc_split(make_float2(c[2], c[3]), h1, l1);
-  hi[0] = h0.x, hi[1] = h1.x, hi[2] = h0.y, hi[3] = h1.y;
-  lo[0] = l0.x, lo[1] = l1.x, lo[2] = l0.y, lo[3] = l1.y;
+__device__ __forceinline__ void dc_mma0(float (&d)[4], const uint32_t (&a)[4], uint32_t b) {
+  asm("mma.sync.aligned.m16n8k8.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%7,%7,%7,%7};"
+      : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(b), "f"(0.f));
+}
+// x and y (low and high halves of a word) as sums of three bf16 numbers: the nearest one, then the leading 8 bits of what is left, then the rest, which
+// has 8 bits: nothing is lost
+__device__ __forceinline__ void dc_split(float x, float y, uint32_t& w0, uint32_t& w1, uint32_t& w2) {
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(w0) : "f"(y), "f"(x));
+  const float rx = x - __uint_as_float(w0 << 16), ry = y - __uint_as_float(w0 & 0xffff0000u);
+  w1 = __byte_perm(__float_as_uint(rx), __float_as_uint(ry), 0x7632);
+  const float sx = rx - __uint_as_float(__float_as_uint(rx) & 0xffff0000u), sy = ry - __uint_as_float(__float_as_uint(ry) & 0xffff0000u);
+  w2 = __byte_perm(__float_as_uint(sx), __float_as_uint(sy), 0x7632);
+}
+// two accumulators side by side (16 rows, 8 + 8 columns) as an A operand: their layouts are the same
+__device__ __forceinline__ void dc_operand(const float (&c)[4], const float (&d)[4], uint32_t (&a)[3][4]) {
+  dc_split(c[0], c[1], a[0][0], a[1][0], a[2][0]);
+  dc_split(c[2], c[3], a[0][1], a[1][1], a[2][1]);
+  dc_split(d[0], d[1], a[0][2], a[1][2], a[2][2]);
+  dc_split(d[2], d[3], a[0][3], a[1][3], a[2][3]);
+}
+// the five products below the leading one: 2^-16 of it, then 2^-8
+template <typename B, typename F>
+__device__ __forceinline__ void dc_low_terms(const uint32_t (&a)[3][4], const B (&b)[3], F&& mma) {
+  mma(a[2], b[0]);
+  mma(a[0], b[2]);
+  mma(a[1], b[1]);
+  mma(a[1], b[0]);
+  mma(a[0], b[1]);
 }
 
 // Columns of a head are dealt to the slices evenly, the first ones one more: never above DC_COLS (slices = columns / DC_COLS, rounded up), and two slices
@@ -650,18 +671,20 @@ delta_triangle_kernel(const float* __restrict__ qn, const float* __restrict__ kn
       __syncwarp();
       float acc[4] = {0.f, 0.f, 0.f, 0.f}, rest[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-      for (int ks = 0; ks < 4; ++ks) {
-        const float2 ak = *reinterpret_cast<const float2*>(scratch + g * LDR + 8 * ks + 2 * t);
-        const float2 aq = *reinterpret_cast<const float2*>(scratch + (8 + g) * LDR + 8 * ks + 2 * t);
-        const float2 bk = *reinterpret_cast<const float2*>(scratch + (16 + g) * LDR + 8 * ks + 2 * t);
-        const float r[4] = {ak.x, ak.y, aq.x, aq.y};
-        float hi[4], lo[4];
-        dc_operand(r, hi, lo);
-        float2 bh, bl;
-        dc_split(bk, bh, bl);
-        dc_mma(rest, lo, bh.x, bh.y);
-        dc_mma(acc, hi, bh.x, bh.y);
-        dc_mma(rest, hi, bl.x, bl.y);
+      for (int ks = 0; ks < 2; ++ks) {                         // rows of A: keys, queries
+        auto at = [&](int row, int k) { return *reinterpret_cast<const float2*>(scratch + (row + g) * LDR + 16 * ks + k + 2 * t); };
+        const float2 k0 = at(0, 0), q0 = at(8, 0), k1 = at(0, 8), q1 = at(8, 8), b0 = at(16, 0), b1 = at(16, 8);
+        const float lo8[4] = {k0.x, k0.y, q0.x, q0.y}, hi8[4] = {k1.x, k1.y, q1.x, q1.y};
+        uint32_t a[3][4];
+        uint2 b[3];
+        dc_operand(lo8, hi8, a);
+        dc_split(b0.x, b0.y, b[0].x, b[1].x, b[2].x);
+        dc_split(b1.x, b1.y, b[0].y, b[1].y, b[2].y);
+        dc_low_terms(a, b, [&](const uint32_t (&x)[4], uint2 y) { dc_mma(rest, x, y); });
+        float x[4];
+        dc_mma0(x, a[0], b[0]);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc[i] += x[i];
       }
       const int i0 = g, j0 = 2 * t;                            // row of both kinds, columns j0, j0 + 1
       if (level == 0 || (i0 >> 2) == (j0 >> 2)) {
@@ -705,7 +728,7 @@ delta_triangle_kernel(const float* __restrict__ qn, const float* __restrict__ kn
           if (j + 3 < i) s[3] = fmaf(-l.w, x[j + 3], s[3]);
         }
         x[i] = (s[0] + s[1]) + (s[2] + s[3]);
-        if (lane <= i) out[i * (i + 1) + lane] = x[i] * b;     // (lane 16 .. 31: not below 16)
+        if (lane <= i) out[i * (i + 1) + lane] = lane < i ? x[i] : b;          // (lane 16 .. 31: not below 16)
       }
     }
     __syncthreads();
@@ -726,26 +749,28 @@ delta_triangle_kernel(const float* __restrict__ qn, const float* __restrict__ kn
 // the state), which are the A operand of the next products as they are; nothing of the state passes through shared memory, the two exchange
 // their shares of the products with it.  Four more warps, a thread per key channel, scale the next chunks' vectors, split them and store them in the
 // order in which the MMAs read them; three buffers, named barriers, so that pairs of warps may drift apart and cover each other's latencies.
-// Bound: the tf32 MMAs (315 per chunk and scheduler, 8 cycles each: 2520 of about 4900) and the fp32 instructions, which sm_100 does not issue beside them:
-// a warp of mma.sync and one of FFMA on the same scheduler take the sum of their times (measured; integer instructions overlap by half).  So what
-// is left counts: vectors split once by the warps that scale them instead of by the four pairs that read them, 3 %; scalar subtractions instead of
-// packed ones, which hold the pipe for 2.4 cycles, 3 %; all channels in one warp (nothing beside its MMAs), 3.1 instead of 2.6 us per chunk; making T and P
-// here too, in both CTAs of a head, 12000 instructions per chunk, 4.4 us.
+// Bound: the state's warps, by their MMAs (324 per chunk and scheduler, 8 cycles each: 2600 of about 5600) and the fp32 instructions, which sm_100 does not
+// issue beside them: a warp of mma.sync and one of FFMA on the same scheduler take the sum of their times (measured; integer instructions, three quarters
+// of the sum).  Without any of the vectors' work a chunk takes 12 % less, without half of the first products' MMAs 15 % less.  All channels in one warp
+// (nothing beside its MMAs) and making T and P here too, in both CTAs of a head, were slower (3.1 instead of 2.6 us and 4.4 us per chunk, with tf32 numbers).
 // us, two tokens at a time in fp32 (the kernel before) -> now with the triangles, heads of 128 x 128, decays per channel / per head: 4 x 320 to 512 tokens, 16
-// heads 156 -> 101 / 153 -> 100, 32 heads 267 -> 191 / 261 -> 190; 16 x 250, 32 heads 464 -> 379 / 456 -> 375; 1 x 1000, 16 heads 290 -> 174; 1 x 32 16 -> 12.
+// heads 155 -> 108 / 153 -> 108, 32 heads 266 -> 207 / 261 -> 205; 16 x 250, 32 heads 464 -> 413 / 456 -> 410; 1 x 1000, 16 heads 290 -> 187; 1 x 32 16 -> 14;
+// but 8 x 33, 16 heads 26 -> 32 (three chunks for two and a bit).
 // An entry takes this path if it has at least DC_MIN tokens, whatever the others have (the exceptions: top of the file); a prompt whose portions are
 // shorter has the bits of single tokens, which differ in the last places.
-// One buffer, in floats: K~ and Q~ as [16 k steps][4 tiles of 8 tokens][8 tokens][8 channels] (k steps padded), K- as [16 tiles of 8 channels][2 k steps]
-// [8 channels][8 tokens] (halves of 4 tokens swapped in the upper 4 channels), blocks (0, 0), (1, 0), (1, 1) of T and of P as [8 tokens][8 tokens], and the
-// decays over the whole chunk
+// One buffer, in words of two bf16 numbers, three times each (the terms): K~ and Q~ as [8 blocks of 16 channels][4 tiles of 8 tokens][8 tokens][channels 2 t,
+// 2 t + 1, then 8 more, t = 0 .. 3], tiles and blocks padded; K- as [16 tiles of 8 channels][8 channels][tokens 2 t, 2 t + 1, then 8 more] (halves of four words
+// swapped in the upper four channels); T and P as [2 tiles of 8 tokens][8 tokens][columns 2 t, 2 t + 1, then 8 more]; and, in fp32, the decays over the whole chunk
 constexpr int DC_STATE_WARPS = 8, DC_THREADS = 32 * DC_STATE_WARPS + DC_TEAM, DC_NBUF = 3;
-constexpr int DC_KS = 4 * 64 + 8, DC_KB = 16 * DC_KS, DC_LOW = DC_KB + 32 * 64, DC_TP = 2 * DC_LOW, DC_G = DC_TP + 6 * 64, DC_BUF = DC_G + 128;
+constexpr int DC_TILE = 72, DC_BLOCK = 4 * DC_TILE + 16, DC_KQ = 8 * DC_BLOCK, DC_KM = 16 * 64, DC_TRI = 4 * 64;
+constexpr int DC_KM_AT = 3 * DC_KQ, DC_TRI_AT = DC_KM_AT + 3 * DC_KM, DC_G = DC_TRI_AT + 3 * DC_TRI, DC_DIAG = DC_G + 128, DC_BUF = DC_DIAG + 32;
 constexpr int DC_SWAP = DC_NBUF * DC_BUF;                      // [2][8 warps][3 pieces][32 lanes][4]
 constexpr int DC_SMEM = (DC_SWAP + 2 * DC_STATE_WARPS * 3 * 128) * 4;
 enum { DC_BAR_FULL = 1, DC_BAR_FREE = DC_BAR_FULL + DC_NBUF, DC_BAR_PAIR = DC_BAR_FREE + DC_NBUF };       // + buffer, + pair of warps
 
 __device__ __forceinline__ void dc_sync(int bar, int n) { asm volatile("barrier.cta.sync %0, %1;" ::"r"(bar), "r"(n) : "memory"); }
 __device__ __forceinline__ void dc_arrive(int bar, int n) { asm volatile("barrier.cta.arrive %0, %1;" ::"r"(bar), "r"(n) : "memory"); }
+__device__ __forceinline__ int dc_tri_half(int tok, int j) { return 2 * ((tok >> 3) * 64 + (tok & 7) * 8 + ((j & 7) >> 1) * 2 + (j >> 3)) + (j & 1); }
 struct DcTile { float x[2][4]; };                              // 16 columns of the state x 16 tokens, accumulator layout
 __device__ __forceinline__ float dc_nonfinite(const DcTile& a) {             // 0, or NaN if an element is not finite
   float s[2] = {0.f, 0.f};
@@ -755,34 +780,27 @@ __device__ __forceinline__ float dc_nonfinite(const DcTile& a) {             // 
     for (int i = 0; i < 4; ++i) s[n] = fmaf(a.x[n][i], 0.f, s[n]);
   return s[0] + s[1];
 }
-// columns 8 n .. 8 n + 7 of in . M^T, added to out, with the lower triangle M [16, 16]
+// columns 8 N .. 8 N + 7 of in . M^T, added to out, with the lower triangle M [16, 16] (m: its words)
 template <int N>
-__device__ __forceinline__ void dc_triangle(float (&out)[4], const float (&hi)[2][4], const float (&lo)[2][4], const float* m, int lane) {
-  float2 h0, l0;
-  dc_split(*reinterpret_cast<const float2*>(m + 64 * N + 2 * lane), h0, l0);
-  float s[4];                                                  // (chains of two or three)
-  dc_mma0(s, lo[0], h0.x, h0.y);
-  if constexpr (N == 1) {
-    float2 h1, l1;
-    float r[4];
-    dc_split(*reinterpret_cast<const float2*>(m + 128 + 2 * lane), h1, l1);
-    dc_mma0(r, lo[1], h1.x, h1.y);
-    dc_mma(s, hi[0], l0.x, l0.y);
-    dc_mma(r, hi[1], l1.x, l1.y);
-    dc_mma(s, hi[0], h0.x, h0.y);
-    dc_mma(r, hi[1], h1.x, h1.y);
+__device__ __forceinline__ void dc_triangle(float (&out)[4], const uint32_t (&a)[3][4], const uint32_t* m, int lane) {
+  using B = std::conditional_t<N == 0, uint32_t, uint2>;       // (columns 8 .. 15 of the first eight rows are zero)
+  B b[3];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) out[i] += s[i] + r[i];
-  } else {
-    dc_mma(s, hi[0], l0.x, l0.y);
-    dc_mma(s, hi[0], h0.x, h0.y);
+  for (int i = 0; i < 3; ++i) b[i] = *reinterpret_cast<const B*>(m + i * DC_TRI + 64 * N + 2 * lane);
+  float r[4], s[4], u[4];                                      // (short chains)
+  dc_mma0(r, a[0], b[0]);
+  dc_mma0(s, a[2], b[0]);
+  dc_mma0(u, a[0], b[2]);
+  dc_mma(s, a[1], b[1]);
+  dc_mma(u, a[0], b[1]);
+  dc_mma(s, a[1], b[0]);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) out[i] += s[i];
-  }
+  for (int i = 0; i < 4; ++i) out[i] += (s[i] + u[i]) + r[i];
 }
 // The same for inputs that are not all finite: no product with the zeros above the diagonal, so a token's NaN or infinity reaches none before it.
-__device__ __noinline__ DcTile dc_triangle_masked(DcTile in, const float* m, int lane) {
+__device__ __noinline__ DcTile dc_triangle_masked(DcTile in, const uint32_t* m, int lane) {
   const int t = lane & 3;
+  const unsigned short* mh = reinterpret_cast<const unsigned short*>(m);
   DcTile out = {};
   for (int j = 0; j < 16; ++j) {
     const int from = (lane & ~3) | ((j & 7) >> 1);
@@ -795,8 +813,10 @@ __device__ __noinline__ DcTile dc_triangle_masked(DcTile in, const float* m, int
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
         const int tok = 8 * n + 2 * t + c;
-        if (tok < j) continue;
-        const float w = m[(n + (j >> 3)) * 64 + (tok & 7) * 8 + (j & 7)];
+        if (tok <= j) continue;
+        float w = 0.f;
+#pragma unroll
+        for (int i = 0; i < 3; ++i) w += __uint_as_float((uint32_t)mh[2 * i * DC_TRI + dc_tri_half(tok, j)] << 16);
         out.x[n][c] = fmaf(w, xr[0], out.x[n][c]);
         out.x[n][c + 2] = fmaf(w, xr[1], out.x[n][c + 2]);
       }
@@ -834,7 +854,7 @@ delta_chunk_kernel(const float* __restrict__ qn, const float* __restrict__ kn, c
       while ((tt + 1) * (tt + 2) <= i) ++tt;                   // rows below tt have tt (tt + 1) numbers
       const int in = i - tt * (tt + 1), p = in > tt ? 1 : 0, j = in - p * (tt + 1);
       tp_tok[r] = i < DC_CHUNK * (DC_CHUNK + 1) ? tt : 1 << 30;
-      tp_dst[r] = DC_TP + (3 * p + (tt >> 3) + (j >> 3)) * 64 + (tt & 7) * 8 + (j & 7);
+      tp_dst[r] = j == tt ? -(DC_DIAG + p * 16 + tt) : 2 * (DC_TRI_AT + p * 128) + dc_tri_half(tt & 15, j);
       tp_src[r] = o + ((int64_t)(t0 + i / wz) * H + h) * dv + z0 + i % wz;
     }
     auto fetch = [&](int tc) {
@@ -842,45 +862,61 @@ delta_chunk_kernel(const float* __restrict__ qn, const float* __restrict__ kn, c
 #pragma unroll
       for (int r = 0; r < 3; ++r) tp[r] = tc + tp_tok[r] < t1 ? tp_src[r][(int64_t)(tc - t0) * H * dv] : 0.f;
     };
-    for (int i = d; i < DC_NBUF * 6 * 64; i += DC_TEAM) dc_smem[(i / 384) * DC_BUF + DC_TP + i % 384] = 0.f;       // (above the diagonal it stays so)
+    for (int i = d; i < DC_NBUF * 3 * DC_TRI; i += DC_TEAM) dc_smem[(i / (3 * DC_TRI)) * DC_BUF + DC_TRI_AT + i % (3 * DC_TRI)] = 0.f;       // (above the diagonal it stays so)
     pdl_wait();                                                // T and P
     fetch(t0);
     dc_sync(DC_BAR_FREE, DC_TEAM);                             // (the zeros before the numbers)
     for (int n = 0; n < chunks; ++n) {
       const int buf = n % DC_NBUF;
       float* b = dc_smem + buf * DC_BUF;
+      uint32_t* bw = reinterpret_cast<uint32_t*>(b);
       if (n >= DC_NBUF) dc_sync(DC_BAR_FREE + buf, DC_THREADS);
-      {                                                        // K~ = -G_t k_t and Q~ = G_t q_t
-        float c = 1.f;
-        float* dst = b + (d >> 3) * DC_KS + (d & 7);
+      {                                                        // K~ = -G_t k_t and Q~ = G_t q_t: words of two channels, tokens 0 .. 7 in even lanes
+        float c = 1.f, x[DC_CHUNK], y[DC_CHUNK];
 #pragma unroll
-        for (int i = 0; i < DC_CHUNK; ++i) {
-          c *= gg[i];
-          const float x = -k[i] * c, y = q[i] * c, hx = dc_high(x), hy = dc_high(y);
-          dst[i * 8] = hx, dst[DC_LOW + i * 8] = x - hx;
-          dst[128 + i * 8] = hy, dst[DC_LOW + 128 + i * 8] = y - hy;
-        }
+        for (int i = 0; i < DC_CHUNK; ++i) c *= gg[i], x[i] = -k[i] * c, y[i] = q[i] * c;
         b[DC_G + d] = c;
-      }
-      {                                                        // K- = (G / G_j) k_j
-        float c = 1.f;
-        float* dst = b + DC_KB + (d >> 3) * 128 + (d & 7) * 8;
+        const bool odd = (d & 1) != 0;
+        uint32_t* dst = bw + (d >> 4) * DC_BLOCK + (odd ? DC_TILE : 0) + ((d & 7) >> 1) * 2 + ((d >> 3) & 1);
+        auto put = [&](const float (&v)[DC_CHUNK], uint32_t* to) {
 #pragma unroll
-        for (int i = DC_CHUNK - 4; i >= 0; i -= 4) {
-          float4 x;
-          x.w = k[i + 3] * c, c *= gg[i + 3];
-          x.z = k[i + 2] * c, c *= gg[i + 2];
-          x.y = k[i + 1] * c, c *= gg[i + 1];
-          x.x = k[i] * c, c *= gg[i];
-          const float4 xh = make_float4(dc_high(x.x), dc_high(x.y), dc_high(x.z), dc_high(x.w));
-          float* at = dst + (i >> 3) * 64 + 4 * (((i >> 2) & 1) ^ ((d >> 2) & 1));
-          *reinterpret_cast<float4*>(at) = xh;
-          *reinterpret_cast<float4*>(at + DC_LOW) = make_float4(x.x - xh.x, x.y - xh.y, x.z - xh.z, x.w - xh.w);
+          for (int i = 0; i < 8; ++i) {
+            const float other = __shfl_xor_sync(0xffffffffu, odd ? v[i] : v[8 + i], 1), own = odd ? v[8 + i] : v[i];
+            uint32_t w0, w1, w2;
+            dc_split(odd ? other : own, odd ? own : other, w0, w1, w2);
+            to[i * 8] = w0, to[DC_KQ + i * 8] = w1, to[2 * DC_KQ + i * 8] = w2;
+          }
+        };
+        put(x, dst);
+        put(y, dst + 2 * DC_TILE);
+      }
+      {                                                        // K- = (G / G_j) k_j: words of two tokens
+        float c = 1.f, x[DC_CHUNK];
+#pragma unroll
+        for (int i = DC_CHUNK - 1; i >= 0; --i) x[i] = k[i] * c, c *= gg[i];
+        uint32_t* dst = bw + DC_KM_AT + (d >> 3) * 64 + (d & 7) * 8;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {                          // t = 2 h, 2 h + 1
+          uint32_t w[3][4];
+          dc_split(x[4 * h], x[4 * h + 1], w[0][0], w[1][0], w[2][0]);
+          dc_split(x[4 * h + 8], x[4 * h + 9], w[0][1], w[1][1], w[2][1]);
+          dc_split(x[4 * h + 2], x[4 * h + 3], w[0][2], w[1][2], w[2][2]);
+          dc_split(x[4 * h + 10], x[4 * h + 11], w[0][3], w[1][3], w[2][3]);
+          uint32_t* at = dst + 4 * (h ^ ((d >> 2) & 1));
+#pragma unroll
+          for (int i = 0; i < 3; ++i) *reinterpret_cast<uint4*>(at + i * DC_KM) = make_uint4(w[i][0], w[i][1], w[i][2], w[i][3]);
         }
       }
 #pragma unroll
       for (int r = 0; r < 3; ++r)
-        if (tp_tok[r] < DC_CHUNK) b[tp_dst[r]] = tp[r];
+        if (tp_dst[r] < 0 && tp_tok[r] < DC_CHUNK) {
+          b[-tp_dst[r]] = tp[r];
+        } else if (tp_tok[r] < DC_CHUNK) {
+          uint32_t w0, w1, w2;
+          dc_split(tp[r], 0.f, w0, w1, w2);
+          unsigned short* at = reinterpret_cast<unsigned short*>(bw) + tp_dst[r];
+          at[0] = (unsigned short)w0, at[2 * DC_TRI] = (unsigned short)w1, at[4 * DC_TRI] = (unsigned short)w2;
+        }
       dc_arrive(DC_BAR_FULL + buf, DC_THREADS);
       if (n + 1 < chunks) fetch(t0 + (n + 1) * DC_CHUNK);
     }
@@ -918,6 +954,7 @@ delta_chunk_kernel(const float* __restrict__ qn, const float* __restrict__ kn, c
   for (int n = 0; n < chunks; ++n) {
     const int buf = n % DC_NBUF, tc = t0 + n * DC_CHUNK;
     const float* b = dc_smem + buf * DC_BUF;
+    const uint32_t* bw = reinterpret_cast<const uint32_t*>(b);
     float4* swap = reinterpret_cast<float4*>(dc_smem + DC_SWAP) + (n & 1) * (DC_STATE_WARPS * 3 * 32) + lane;
     float sum[4][4], rest[4][4];                               // -S^T K~ of tokens 0 .. 7, 8 .. 15, S^T Q~ of both
 #pragma unroll
@@ -926,28 +963,27 @@ delta_chunk_kernel(const float* __restrict__ qn, const float* __restrict__ kn, c
       for (int i = 0; i < 4; ++i) sum[m][i] = rest[m][i] = 0.f;
     dc_sync(DC_BAR_FULL + buf, DC_THREADS);
 #pragma unroll
-    for (int k4 = 0; k4 < 2; ++k4) {
+    for (int kb = 0; kb < 4; ++kb) {                           // (a block's leading products hardly lose a bit in one MMA; the blocks meet in rounding additions)
       float acc[4][4];
+      uint32_t a[3][4];
+      uint2 bv[4][3];
+      dc_operand(S[2 * kb], S[2 * kb + 1], a);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int ks = 4 * k4 + i;
-        float hi[4], lo[4];
-        float2 bh[4], bl[4];
-        dc_operand(S[ks], hi, lo);
+      for (int m = 0; m < 4; ++m)
 #pragma unroll
-        for (int m = 0; m < 4; ++m) {
-          const float* at = b + (8 * half + ks) * DC_KS + m * 64 + 2 * lane;
-          bh[m] = *reinterpret_cast<const float2*>(at), bl[m] = *reinterpret_cast<const float2*>(at + DC_LOW);
-        }
+        for (int j = 0; j < 3; ++j) bv[m][j] = *reinterpret_cast<const uint2*>(bw + j * DC_KQ + (4 * half + kb) * DC_BLOCK + m * DC_TILE + 2 * lane);
 #pragma unroll
-        for (int m = 0; m < 4; ++m)
-          if (i == 0) dc_mma0(acc[m], hi, bh[m].x, bh[m].y);
-          else dc_mma(acc[m], hi, bh[m].x, bh[m].y);
+      for (int m = 0; m < 4; ++m) dc_mma0(acc[m], a[0], bv[m][0]);
 #pragma unroll
-        for (int m = 0; m < 4; ++m) dc_mma(rest[m], hi, bl[m].x, bl[m].y);
+      for (int m = 0; m < 4; ++m) dc_mma(rest[m], a[2], bv[m][0]);
 #pragma unroll
-        for (int m = 0; m < 4; ++m) dc_mma(rest[m], lo, bh[m].x, bh[m].y);
-      }
+      for (int m = 0; m < 4; ++m) dc_mma(rest[m], a[0], bv[m][2]);
+#pragma unroll
+      for (int m = 0; m < 4; ++m) dc_mma(rest[m], a[1], bv[m][1]);
+#pragma unroll
+      for (int m = 0; m < 4; ++m) dc_mma(rest[m], a[1], bv[m][0]);
+#pragma unroll
+      for (int m = 0; m < 4; ++m) dc_mma(rest[m], a[0], bv[m][1]);
 #pragma unroll
       for (int m = 0; m < 4; ++m)
 #pragma unroll
@@ -965,14 +1001,15 @@ delta_chunk_kernel(const float* __restrict__ qn, const float* __restrict__ kn, c
     mine[32] = make_float4(sum[1][0], sum[1][1], sum[1][2], sum[1][3]);
     mine[64] = make_float4(give[0], give[1], give[2], give[3]);
     dc_sync(DC_BAR_PAIR + pair, 64);
-    DcTile X, U;
+    DcTile X;
+    float2 bt[2];
     float out[4];
 #pragma unroll
     for (int m = 0; m < 2; ++m) {
       const float4 x = theirs[32 * m];
       X.x[m][0] = vn.x[m][0] + (sum[m][0] + x.x), X.x[m][1] = vn.x[m][1] + (sum[m][1] + x.y);
       X.x[m][2] = vn.x[m][2] + (sum[m][2] + x.z), X.x[m][3] = vn.x[m][3] + (sum[m][3] + x.w);
-      U.x[m][0] = U.x[m][1] = U.x[m][2] = U.x[m][3] = 0.f;
+      bt[m] = *reinterpret_cast<const float2*>(b + DC_DIAG + 8 * m + 2 * t);
     }
     {
       const float4 x = theirs[64];
@@ -980,58 +1017,70 @@ delta_chunk_kernel(const float* __restrict__ qn, const float* __restrict__ kn, c
       out[2] = (half ? sum[3][2] : sum[2][2]) + x.z, out[3] = (half ? sum[3][3] : sum[2][3]) + x.w;
     }
     if (n + 1 < chunks) fetch_v(tc + DC_CHUNK);
-    // ---- U = T X, O += P U
-    float hi[2][4], lo[2][4];
-    if (__any_sync(0xffffffffu, dc_nonfinite(X) != 0.f)) {
-      U = dc_triangle_masked(X, b + DC_TP, lane);
-    } else {
-      dc_operand(X.x[0], hi[0], lo[0]);
-      dc_operand(X.x[1], hi[1], lo[1]);
-      dc_triangle<0>(U.x[0], hi, lo, b + DC_TP, lane);
-      dc_triangle<1>(U.x[1], hi, lo, b + DC_TP, lane);
+    // ---- U = b X + (T - I) b X, O += P U: diagonals in fp32 FMAs, the last roundings but those of the large terms beside them
+    DcTile Y, U = {};
+#pragma unroll
+    for (int m = 0; m < 2; ++m) {
+      Y.x[m][0] = X.x[m][0] * bt[m].x, Y.x[m][1] = X.x[m][1] * bt[m].y;
+      Y.x[m][2] = X.x[m][2] * bt[m].x, Y.x[m][3] = X.x[m][3] * bt[m].y;
     }
-    dc_operand(U.x[0], hi[0], lo[0]);
-    dc_operand(U.x[1], hi[1], lo[1]);
+    uint32_t a[3][4];
+    if (__any_sync(0xffffffffu, dc_nonfinite(Y) != 0.f)) {
+      U = dc_triangle_masked(Y, bw + DC_TRI_AT, lane);
+    } else {
+      dc_operand(Y.x[0], Y.x[1], a);
+      dc_triangle<0>(U.x[0], a, bw + DC_TRI_AT, lane);
+      dc_triangle<1>(U.x[1], a, bw + DC_TRI_AT, lane);
+    }
+#pragma unroll
+    for (int m = 0; m < 2; ++m) {
+      U.x[m][0] = fmaf(X.x[m][0], bt[m].x, U.x[m][0]), U.x[m][1] = fmaf(X.x[m][1], bt[m].y, U.x[m][1]);
+      U.x[m][2] = fmaf(X.x[m][2], bt[m].x, U.x[m][2]), U.x[m][3] = fmaf(X.x[m][3], bt[m].y, U.x[m][3]);
+    }
+    dc_operand(U.x[0], U.x[1], a);
     if (__any_sync(0xffffffffu, dc_nonfinite(U) != 0.f)) {
-      const DcTile m = dc_triangle_masked(U, b + DC_TP + 3 * 64, lane);
+      const DcTile m = dc_triangle_masked(U, bw + DC_TRI_AT + 128, lane);
 #pragma unroll
       for (int i = 0; i < 4; ++i) out[i] += half ? m.x[1][i] : m.x[0][i];
     } else if (half) {
-      dc_triangle<1>(out, hi, lo, b + DC_TP + 3 * 64, lane);
+      dc_triangle<1>(out, a, bw + DC_TRI_AT + 128, lane);
     } else {
-      dc_triangle<0>(out, hi, lo, b + DC_TP + 3 * 64, lane);
+      dc_triangle<0>(out, a, bw + DC_TRI_AT + 128, lane);
+    }
+    {
+      const float2 pt = *reinterpret_cast<const float2*>(b + DC_DIAG + 16 + 8 * half + 2 * t);
+      const float (&u)[4] = half ? U.x[1] : U.x[0];
+      out[0] = fmaf(pt.x, u[0], out[0]), out[1] = fmaf(pt.y, u[1], out[1]), out[2] = fmaf(pt.x, u[2], out[2]), out[3] = fmaf(pt.y, u[3], out[3]);
     }
     // ---- S <- G S + K- U
-    const float* kb = b + DC_KB + half * (8 * 128) + g * 8 + 4 * ((t >> 1) ^ (g >> 2)) + 2 * (t & 1);
+    const uint32_t* kb = bw + DC_KM_AT + half * (8 * 64) + g * 8 + 4 * ((t >> 1) ^ (g >> 2)) + 2 * (t & 1);
 #pragma unroll
     for (int m0 = 0; m0 < 8; m0 += 4) {                        // (four sums at a time cover each other's latencies)
-      float acc[4][4];
-      float2 h0[4], l0[4], h1[4], l1[4];
+      float acc[4][4], big[4][4];
+      uint2 bv[4][3];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const float* at = kb + (m0 + i) * 128;
-        h0[i] = *reinterpret_cast<const float2*>(at), l0[i] = *reinterpret_cast<const float2*>(at + DC_LOW);
-        h1[i] = *reinterpret_cast<const float2*>(at + 64), l1[i] = *reinterpret_cast<const float2*>(at + DC_LOW + 64);
-      }
+      for (int i = 0; i < 4; ++i)
 #pragma unroll
-      for (int i = 0; i < 4; ++i) dc_mma0(acc[i], lo[0], h0[i].x, h0[i].y);
+        for (int j = 0; j < 3; ++j) bv[i][j] = *reinterpret_cast<const uint2*>(kb + j * DC_KM + (m0 + i) * 64);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) dc_mma(acc[i], hi[0], l0[i].x, l0[i].y);
+      for (int i = 0; i < 4; ++i) dc_mma0(acc[i], a[2], bv[i][0]);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) dc_mma(acc[i], lo[1], h1[i].x, h1[i].y);
+      for (int i = 0; i < 4; ++i) dc_mma(acc[i], a[0], bv[i][2]);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) dc_mma(acc[i], hi[1], l1[i].x, l1[i].y);
+      for (int i = 0; i < 4; ++i) dc_mma(acc[i], a[1], bv[i][1]);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) dc_mma(acc[i], hi[0], h0[i].x, h0[i].y);
+      for (int i = 0; i < 4; ++i) dc_mma(acc[i], a[1], bv[i][0]);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) dc_mma(acc[i], hi[1], h1[i].x, h1[i].y);
+      for (int i = 0; i < 4; ++i) dc_mma(acc[i], a[0], bv[i][1]);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) dc_mma0(big[i], a[0], bv[i][0]);
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const float2 c = *reinterpret_cast<const float2*>(b + DC_G + 64 * half + 8 * (m0 + i) + 2 * t);
         float (&x)[4] = S[m0 + i];
         const float2 p = __ffma2_rn(make_float2(x[0], x[1]), c, make_float2(acc[i][0], acc[i][1]));
         const float2 r = __ffma2_rn(make_float2(x[2], x[3]), c, make_float2(acc[i][2], acc[i][3]));
-        x[0] = p.x, x[1] = p.y, x[2] = r.x, x[3] = r.y;
+        x[0] = p.x + big[i][0], x[1] = p.y + big[i][1], x[2] = r.x + big[i][2], x[3] = r.y + big[i][3];
       }
     }
     if (n + DC_NBUF < chunks) dc_arrive(DC_BAR_FREE + buf, DC_THREADS);
