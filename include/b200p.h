@@ -398,7 +398,7 @@ int b200p_delta_scan(const float* qn, const float* kn, const float* v, const flo
  * unless o is v: the same sums in another order than token by token (on the tensor cores, every operand as three bf16 numbers that hold all of its
  * bits: as exact as fp32 FMAs; o holds intermediate numbers of an entry's rows), so a prompt's portions give its results up to fp32 rounding and
  * not bit for bit.  Otherwise an entry's bits depend on its own tokens alone, unless it has 32 or more beside at least that many empty entries and
- * the call does not say so (longest), or 16 to 31 beside one of 32 or more and the call says so. */
+ * the call does not say so (longest). */
 int b200p_delta_scan_tokens(const float* qn, const float* kn, const float* v, const float* beta, const float* decay, float* state,
                             const int32_t* cu, const int32_t* rows, const int32_t* lengths, float* o, int64_t tokens, int nb, int H, int KH,
                             int dk, int dv, int mode, void* stream);

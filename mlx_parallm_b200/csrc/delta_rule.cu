@@ -9,9 +9,8 @@
 // fed by linear_attn_prep_kernel).
 // Single tokens and entries of less than 32 run in one summation order, whatever kernel takes them; entries of 32 tokens and more (keys of 65 to 128
 // channels, delta rule) 16 tokens at a time (delta_chunk_kernel), which differs in the last places, so a prompt and its portions agree to rounding.
-// An entry's bits depend on its own tokens alone, with two exceptions: beside at least as many empty entries as it has tokens, in a call that
-// does not say how long its longest entry is, it goes token by token (delta_step_kernel); with 16 to 31 tokens, in a call that says that its longest entry
-// has 32 or more, it goes with that one.
+// An entry's bits depend on its own tokens alone, with one exception: beside at least as many empty entries as it has tokens, in a call that
+// does not say how long its longest entry is, it goes token by token (delta_step_kernel).
 #include <type_traits>
 
 #include "common.cuh"
@@ -601,14 +600,14 @@ __device__ __forceinline__ void dc_fetch(const float* __restrict__ qn, const flo
 template <int MODE>
 __global__ void __launch_bounds__(DC_TEAM, 6)
 delta_triangle_kernel(const float* __restrict__ qn, const float* __restrict__ kn, const float* __restrict__ beta, const float* __restrict__ decay,
-                      const int32_t* __restrict__ cu, float* __restrict__ o, int H, int KH, int dk, int dv, int slices, int least) {
+                      const int32_t* __restrict__ cu, float* __restrict__ o, int H, int KH, int dk, int dv, int slices) {
   constexpr int LDR = 40, LDP = 17;                            // padded rows: a half warp's 8-byte reads fall into different banks
   __shared__ __align__(16) float scratch_all[4][24 * LDR], part[4][2][16 * LDP], tri[16 * 20];
   __shared__ float out[16 * 17];
   const int h = blockIdx.y, d = threadIdx.x, w = d >> 5, lane = d & 31, g = lane >> 2, t = lane & 3;
   pdl_launch_dependents();
   const int t0 = cu[blockIdx.x], t1 = cu[blockIdx.x + 1];
-  if (t1 - t0 < least) return;
+  if (t1 - t0 < DC_MIN) return;
   const int kh = h / (H / KH), tok = lane & 15, wide = dc_slice(dv, slices, 0).n, narrow = dc_slice(dv, slices, slices - 1).n;
   const int per_wide = 65535 / wide + 1, per_narrow = 65535 / narrow + 1;      // i / w = (i * per) >> 16 for i < 272, w <= 64
   float* scratch = scratch_all[w];
@@ -756,7 +755,7 @@ delta_triangle_kernel(const float* __restrict__ qn, const float* __restrict__ kn
 // us, two tokens at a time in fp32 (the kernel before) -> now with the triangles, heads of 128 x 128, decays per channel / per head: 4 x 320 to 512 tokens, 16
 // heads 155 -> 108 / 153 -> 108, 32 heads 266 -> 207 / 261 -> 205; 16 x 250, 32 heads 464 -> 413 / 456 -> 410; 1 x 1000, 16 heads 290 -> 187; 1 x 32 16 -> 14;
 // but 8 x 33, 16 heads 26 -> 32 (three chunks for two and a bit).
-// An entry takes this path if it has at least DC_MIN tokens, whatever the others have (the exceptions: top of the file); a prompt whose portions are
+// An entry takes this path if it has at least DC_MIN tokens, whatever the others have (the exception: top of the file); a prompt whose portions are
 // shorter has the bits of single tokens, which differ in the last places.
 // One buffer, in words of two bf16 numbers, three times each (the terms): K~ and Q~ as [8 blocks of 16 channels][4 tiles of 8 tokens][8 tokens][channels 2 t,
 // 2 t + 1, then 8 more, t = 0 .. 3], tiles and blocks padded; K- as [16 tiles of 8 channels][8 channels][tokens 2 t, 2 t + 1, then 8 more] (halves of four words
@@ -828,12 +827,12 @@ template <int MODE>
 __global__ void __launch_bounds__(DC_THREADS, 1)
 delta_chunk_kernel(const float* __restrict__ qn, const float* __restrict__ kn, const float* __restrict__ v, const float* __restrict__ decay,
                    float* __restrict__ state, const int32_t* __restrict__ cu, const int32_t* __restrict__ rows, const int32_t* __restrict__ lengths,
-                   float* o, int H, int KH, int dk, int dv, int least) {
+                   float* o, int H, int KH, int dk, int dv) {
   extern __shared__ __align__(16) float dc_smem[];
   const int e = blockIdx.x, h = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   pdl_launch_dependents();
   const int t0 = cu[e], t1 = cu[e + 1];
-  if (t1 - t0 < least) {
+  if (t1 - t0 < DC_MIN) {
     if ((blockIdx.x | blockIdx.y | blockIdx.z) == 0) pdl_wait();       // (this grid ends no earlier than the launch before, also where no entry is long)
     return;
   }
@@ -1336,7 +1335,7 @@ static cudaError_t delta_scan_launch(int64_t tokens, int64_t longest, int nb, cu
 #define DELTA_SCAN(DKP, LANES, PER_SM)                                                                                           \
   launch_pdl_opt(chunks && pdl_enabled_gemm(), delta_scan_kernel<DKP, MODE, LANES, PER_SM>,                                        \
                  dim3((unsigned)nb, (unsigned)H, (unsigned)((dv + 2 * ds_slots(DKP) - 1) / (2 * ds_slots(DKP)))), dim3(LANES * ds_slots(DKP)), 0, st, \
-                 qn, kn, v, beta, decay, state, cu, rows, lengths, o, H, KH, dk, dv, chunks ? least - 1 : INT32_MAX)
+                 qn, kn, v, beta, decay, state, cu, rows, lengths, o, H, KH, dk, dv, chunks ? DC_MIN - 1 : INT32_MAX)
   // The step kernel for decode steps, and for as many tokens per entry as it keeps up with the scan (us, step / scan): 128 x 128, 16
   // entries of 1 / 2 / 4 tokens, 32 heads, 21.7 / 23.1, 27.1 / 25.3, 32.0 / 29.2; 64 x 64, 32 heads, of 2 / 4 / 8, 6.8 / 8.8, 7.9 / 9.6,
   // 10.2 / 11.4, but with 16 heads 4.3 / 4.6, 5.1 / 5.0, 7.3 / 6.4; 32 x 64, 16 heads, of 2 / 4, 3.4 / 3.5, 4.2 / 3.9; 256 x 256, 8 heads,
@@ -1356,19 +1355,17 @@ static cudaError_t delta_scan_launch(int64_t tokens, int64_t longest, int nb, cu
   // batch come with their tail.  A call that knows its longest entry to be short is spared the first launch: 16 entries of 4 tokens, 16 heads 14.4 ->
   // 13.3 us.
   const bool chunks = by_chunks && !few && (tokens == 0 || tokens >= DC_MIN) && (longest == 0 || longest >= DC_MIN);
-  // Beside the chunk kernel's CTAs, which take an SM's registers, the token-by-token ones find no room: a call that knows of an entry of DC_MIN tokens
-  // takes those down to one chunk along (us, start / one launch behind the other / along: 40, 35, 30, 25 tokens, 32 heads 28.4 / 40.8 / 28.0, 48 to 27 tokens,
-  // eight entries of 16 heads 32 / 41.6 / 28.5); below that a single entry gains nothing (20 tokens 12.6 / 12.9).
-  const int least = longest >= DC_MIN ? DC_CHUNK : DC_MIN;
+  // An entry's own length alone decides, so that its bits do not depend on the others.  Beside the chunk kernel's CTAs, which take an SM's registers, the
+  // token-by-token ones find little room: batches with entries on both sides of DC_MIN pay for that (us, the two-token kernel before / so / all entries of 16
+  // and more in chunks: 40, 35, 30, 25 tokens, 32 heads 28 / 43 / 31; 60 to 34 tokens, eight entries of 16 heads 38 / 37 / 37; below 64 tokens only).
   if constexpr (MODE != 2) {
     if (chunks) {
       static const cudaError_t ready = cudaFuncSetAttribute(delta_chunk_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, DC_SMEM);
       if (ready != cudaSuccess) return ready;
       const unsigned slices = (unsigned)((dv + DC_COLS - 1) / DC_COLS), most = (unsigned)(longest ? (longest + DC_CHUNK - 1) / DC_CHUNK : 16);
-      delta_triangle_kernel<MODE><<<dim3((unsigned)nb, (unsigned)H, most < 1024 ? most : 1024), DC_TEAM, 0, st>>>(qn, kn, beta, decay, cu, o, H, KH, dk, dv, (int)slices,
-                                                                                                                 least);
+      delta_triangle_kernel<MODE><<<dim3((unsigned)nb, (unsigned)H, most < 1024 ? most : 1024), DC_TEAM, 0, st>>>(qn, kn, beta, decay, cu, o, H, KH, dk, dv, (int)slices);
       const cudaError_t e = launch_pdl_opt(pdl_enabled_gemm(), delta_chunk_kernel<MODE>, dim3((unsigned)nb, (unsigned)H, slices), dim3(DC_THREADS), DC_SMEM, st,
-                                           qn, kn, v, decay, state, cu, rows, lengths, o, H, KH, dk, dv, least);
+                                           qn, kn, v, decay, state, cu, rows, lengths, o, H, KH, dk, dv);
       if (e != cudaSuccess) return e;
     }
   }

@@ -49,9 +49,10 @@ layers mix a recurrent state with windowed attention over a shared low-rank late
 A step is a ragged batch: entry e brings ``counts[e]`` tokens for cache row ``rows[e]``; prompts of different lengths are
 packed back to back (no padding), decode steps bring one token per live row.  Every kernel works from the per-token plan
 (row, position, offset in the portion), so the logits of a position do not depend on how the prompt was cut or on the
-other rows, up to the order of fp32 sums (which the 16-bit products, attention of prompts and steps, and the delta rule's entries of 16 tokens and
+other rows, up to the order of fp32 sums (which the 16-bit products, attention of prompts and steps, and the delta rule's entries of 32 tokens and
 more choose by the size of a call).  Matrix products run in the model's storage type with fp32 accumulation; the residual stream, every norm,
-softmax, the recurrence and what feeds it are fp32.  A float32 model runs true fp32 FMAs throughout.
+softmax, the recurrence and what feeds it are fp32.  A float32 model runs fp32 FMAs throughout, but for the delta rule's entries of 32 tokens and
+more with keys of 65 to 128 channels: their products run on the tensor cores, every operand as three bf16 numbers that hold all of its bits.
 """
 from __future__ import annotations
 

@@ -891,7 +891,7 @@ def test_gated_units_of_the_tcgen05_products_keep_their_range(dtype, M):
 
 
 @pytest.mark.parametrize("mode", [0, 1])
-@pytest.mark.parametrize("lens,H", [([40, 1, 1, 3, 0, 33, 2], 3), ([1] * 40 + [32], 8), ([5, 9, 20], 20), ([0] * 30 + [50] + [0] * 40, 2)])
+@pytest.mark.parametrize("lens,H", [([40, 1, 1, 3, 0, 33, 2], 3), ([1] * 40 + [32], 8), ([5, 9, 20], 20), ([0] * 30 + [50] + [0] * 40, 2), ([16, 31, 32, 20, 70, 15], 6)])
 def test_delta_scan_of_long_entries_among_short_ones(mode, lens, H):
     """The two launches of such a batch overlap, with more CTAs than fit and without; what reads the results behind them sees both.  A call that is
     told its tokens and its longest entry gives the bits of one that is not (which takes both launches), also beside as many empty entries as a
@@ -912,6 +912,13 @@ def test_delta_scan_of_long_entries_among_short_ones(mode, lens, H):
         state.zero_()
     assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
     assert (got[0][0] - got[2][0]).abs().max() < 4e-5 and (got[0][1] - got[2][1]).abs().max() < 4e-5        # (2e-5 each: the test above)
+    for e in [e for e in range(nb) if lens[e]]:              # and each entry those that it has alone
+        a, b = int(cu[e]), int(cu[e + 1])
+        state, o = state0[e:e + 1].clone(), torch.zeros(b - a, H * dv, device="cuda")
+        one, alone = torch.tensor([0, b - a], **i32), [t[a:b].contiguous() for t in (qn, kn, v, beta, decay)]
+        _lib.check(_lib.lib().b200p_delta_scan_entries(*(t.data_ptr() for t in (*alone, state, one, rows, lengths, o)), b - a, b - a, 1, H, KH, dk, dv, mode,
+                                                       torch.cuda.current_stream().cuda_stream))
+        assert torch.equal(o, got[1][0][a:b]) and torch.equal(state[0], got[1][1][e])
 
 
 @pytest.mark.parametrize("mode", [0, 1])
