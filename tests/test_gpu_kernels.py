@@ -190,14 +190,17 @@ def test_rmsnorm(ops, dtype):
 
 
 @pytest.mark.parametrize("dtype,M,H", [
-    ("float16", 8, 4096),       # one-pass cluster kernel at a few rows
+    ("float16", 8, 4096),       # one pass (16-bit rows of up to 16384), two groups of 8 per thread
     ("float16", 1, 4096),
-    ("bfloat16", 8, 5120),      # below 16 rows and no cluster form: the 256-thread kernel
-    ("float16", 64, 4096),      # early one-pass kernel, cluster of 2 (Llama-3-8B decode at B=64)
-    ("bfloat16", 32, 8192),     # cluster of 4 (70B-class)
-    ("float16", 16, 2048),      # cluster of 1
-    ("bfloat16", 64, 5120),     # Qwen3-14B: 5120 is not a multiple of 2048 -> early two-pass kernel
-    ("float16", 100, 4096),     # 100 rows x 2 CTAs exceed the SMs -> early two-pass kernel
+    ("bfloat16", 8, 5120),      # three
+    ("float16", 64, 4096),      # (Llama-3-8B decode at B=64)
+    ("bfloat16", 32, 8192),     # four (70B-class)
+    ("float16", 16, 2048),      # one
+    ("bfloat16", 64, 5120),     # (Qwen3-14B)
+    ("float16", 100, 4096),
+    ("bfloat16", 8, 16392),     # wider: two passes, below 16 rows 256 threads
+    ("float16", 16, 16392),     # from 16 rows on the early kernel of 128
+    ("bfloat16", 40, 20480),
 ])
 @pytest.mark.parametrize("perm", [False, True])
 def test_rmsnorm_variants_at_decode_sizes(ops, dtype, M, H, perm):
@@ -215,7 +218,7 @@ def test_rmsnorm_variants_at_decode_sizes(ops, dtype, M, H, perm):
 
 
 @pytest.mark.parametrize("dtype", ["float16", "bfloat16"])
-@pytest.mark.parametrize("H", [8, 1016, 1024, 1032, 3584, 7176, 8192, 8200, 16384, 16392])   # groups per thread, both CTA sizes, beyond
+@pytest.mark.parametrize("H", [8, 1016, 1024, 1032, 3584, 7176, 8192, 8200, 16384, 16392])   # groups per thread, partly filled ones, beyond
 @pytest.mark.parametrize("M", [1, 17])
 def test_rmsnorm_one_pass_at_every_width(ops, dtype, H, M):
     """16-bit rows of any number of whole groups of 8, plain and PERM8, against 64 bits; neighbours of the output stay as they were.
@@ -1100,7 +1103,8 @@ def test_attention_tensor_decode(ops, dtype, Hq, Hkv, lengths):
     ("float16", 16, 1, [763]),                  # 767 keys of capacity: whole; 768 and 769: in 64s
     ("bfloat16", 16, 1, [764]),
     ("float16", 32, 8, [765]),
-    ("float16", 32, 16, [508, 70]),             # 512 keys, two splits become eight
+    ("float16", 32, 16, [508, 70]),             # 512 keys, two splits become four (32 (row, key head) pairs on 7/8 of 148 SMs)
+    ("float16", 16, 16, [508]),                 # ... eight: 64 keys each
     ("bfloat16", 8, 8, [2040]),                 # as many splits as 7/8 of the SMs hold
     ("float16", 4, 1, [2047, 0, 63, 64, 1000]), # 25 splits: most of them empty in the short rows
     ("bfloat16", 4, 4, [700] * 32),             # as many (row, key head) pairs as SMs to spread over: not spread further
