@@ -72,9 +72,10 @@ const char* b200p_last_error(void);
 int b200p_arch_check(void);
 int b200p_sm_count(void);
 /* Programmatic dependent launch, 0 off: kernel N+1's prologue and weight prefetch overlap kernel N's tail; each kernel executes
- * griddepcontrol.wait before touching its inputs.  Default (2): the quantised products, the early norms, attention, the delta rule's second
- * launch, dense products between other kernels (B200P_GEMM_CHAINED), a mixture's kernels except its last (routing and gather up to 64
- * tokens); 1: every kernel that can be. */
+ * griddepcontrol.wait before touching its inputs, but for the weights, scales and biases of b200p_qmm, which are read before it (the
+ * kernel launched right before must not be one that writes them and lets its dependents start early).  Default (2): the quantised products,
+ * the early norms, attention, the delta rule's second and third launch, dense products between other kernels (B200P_GEMM_CHAINED), a
+ * mixture's kernels except its last (routing and gather up to 64 tokens); 1: every kernel that can be. */
 int b200p_set_pdl(int enabled);
 
 /* mx.dequantize(w, scales, biases, group_size, bits)            [nn.QuantizedEmbedding.__call__,
@@ -103,7 +104,9 @@ int b200p_embed(const int32_t* ids, const uint32_t* w, const void* scales, const
  * x `dtype` [M,K] row-major (ldx elements between rows), y per `epilogue` (ldy elements between
  * rows).  fp32 accumulation.  Internally: the mma.sync register GEMV (4-bit g64, 16-bit, M <= 16, fp32 outputs), the
  * tcgen05 tile path (F16/BF16, group 64) or the generic CUDA-core GEMV (any dtype / shape).  `workspace` (>= b200p_qmm_workspace_bytes) is
- * required by the split-K tensor path; may be NULL for the GEMV path. */
+ * required by the split-K tensor path; may be NULL for the GEMV path.  Its first 4096 bytes are counters that have to be zero when it is first
+ * used; every call leaves them zero, the rest needs no initial state.  One workspace serves one stream at a time.  A call of more than 128 tokens
+ * that could do without uses it where it is given: its last output rows are then sums of parts of K, in another order of fp32 additions. */
 int b200p_qmm(const void* x, const uint32_t* w, const void* scales, const void* biases, void* y,
               int64_t M, int64_t N, int64_t K, int64_t ldx, int64_t ldy, int group_size, int bits,
               int dtype, int epilogue, void* workspace, size_t workspace_bytes, void* stream);

@@ -132,8 +132,8 @@ extern "C" int b200p_qmm(const void* x, const uint32_t* w, const void* scales, c
   cudaStream_t st = (cudaStream_t)stream;
   const bool ring_ok = qmv_ring_supported(M, N, K, group_size, bits, dtype, epilogue) && aligned(scales, 16) && aligned(biases, 16) &&
                        aligned(y, epilogue == B200P_EPI_STORE || epilogue == B200P_EPI_SILU_MUL ? 2 : 4);
-  // The ring and the wide kernel need neither a workspace nor y rows of whole words; a call that the kernels they stand in for would
-  // refuse goes on to those, and is refused there.
+  // The ring and the wide kernel need neither a workspace nor y rows of whole words (the wide one uses a workspace that it is given for a short last
+  // round, whose rows are then summed in parts of K); a call that the kernels they stand in for would refuse goes on to those, and is refused there.
   const bool f32out = epilogue == B200P_EPI_STORE_F32 || epilogue == B200P_EPI_ADD_RESIDUAL;
   const bool tile_args = workspace && workspace_bytes >= qmm_tc_workspace_bytes(M, N, K) && aligned(workspace, 16) && aligned(y, 4) &&
                          (f32out || ldy % 2 == 0);

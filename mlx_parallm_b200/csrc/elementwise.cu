@@ -236,9 +236,9 @@ rmsnorm_kernel(const float* x, const T* w, T* __restrict__ y, int64_t H, float e
 // 3 layers: 400 us against 389); 512 threads are the same in a step and slower from some 300 rows on (5120 wide, 4096 rows: 32 us
 // against 22).  Back to back, us, before (the two-pass kernel above or, for whole multiples of 2048 and up to one CTA per SM, a
 // row split over a cluster of CTAs) -> now, bf16:
-//   5120 wide:  1 row 2.9 -> 1.8    64 rows 4.6 -> 2.0   300 rows 6.8 -> 3.7   4096 rows 30.2 -> 22.3 (5.6 TB/s)
-//   4096 wide:  1 row 2.0 -> 1.7    64 rows 2.3 -> 1.9   300 rows 5.3 -> 3.5   4096 rows 24.7 -> 18.9
-//   8192 wide:  1 row 2.0 -> 2.1    64 rows 6.7 -> 2.6   300 rows 8.7 -> 4.7   4096 rows 49.2 -> 32.2
+//   5120 wide:  1 row 2.9 -> 1.7    64 rows 4.6 -> 2.0   300 rows 6.8 -> 3.7   4096 rows 30.2 -> 22.3 (5.6 TB/s)
+//   4096 wide:  1 row 2.0 -> 1.6    64 rows 2.3 -> 1.9   300 rows 5.3 -> 3.5   4096 rows 24.7 -> 18.9
+//   8192 wide:  1 row 2.0 -> 1.9    64 rows 6.7 -> 2.5   300 rows 8.7 -> 4.7   4096 rows 49.2 -> 32.2
 // The sum is taken in (thread, warp) order: reproducible, not bit-identical to the two-pass kernel's.
 constexpr int RMS_NT = 256;
 template <typename T, int NG>

@@ -41,8 +41,8 @@
 //             from global memory; freed by the dequant warps as soon as the values are in registers;
 //         A   (2 blocks x 32 TMEM columns per k-block, in slots of a unit), filled by the dequantisers, freed by MMA completion.
 // A unit is what one group of dequantisers makes of a stage: two k-blocks at 4 bits, one at 8.  The roles hand over units: a wait on a barrier that
-// is long complete takes about 100 cycles, and with one k-block per hand-over the MMA issuers spent 200 of their 490 cycles per k-block on
-// them, the dequantisers 300 of 1250 (152064 x 5120 bf16, 24 / 64 tokens: 137.6 -> 122.4 / 160 -> 147 us; 34816 x 5120 29.4 -> 26.0 / 32.0 -> 28.8; the same bits).
+// is long complete takes 50 to 100 cycles, and with one k-block per hand-over the MMA issuers spent 200 of their 490 cycles per k-block on
+// them, the dequantisers 300 of 1250 (152064 x 5120 bf16, 24 / 64 tokens: 137.6 -> 122.4 / 160 -> 147 us; 34816 x 5120 29.4 -> 26.0 / 32.0 -> 28.8, with whole row blocks 25.8 / 27.9; the same bits).
 // Neither memory, arithmetic nor MMAs bound the loop by themselves (152064 x 5120: all three left out but the hand-overs 72 us, arithmetic alone
 // 123, MMAs alone 97).  Asking for the next stage's codes before this one's arithmetic needs registers that 24 warps do not have: 26 -> 37 us.
 //
